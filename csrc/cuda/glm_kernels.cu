@@ -348,38 +348,57 @@ extern "C" int skml_glm_validate(const long long* rowptr, const int* cols, const
 }
 
 // ---------------------------------------------------------------------------
-// Compaction of the touched bitmap into a sorted sparse gradient.
-// Each block owns COMPACT_WORDS consecutive bitmap words (each warp 4 groups of 32 words).
-// meta[0] = nnz, meta[1] = kind (1 sparse, 2 dense, 0 empty), meta[2] = touched before filter
+// Compaction of the touched bitmap into a sorted sparse gradient. A warp owns `wpw` consecutive bitmap
+// words, walked 32 at a time; the count pass leaves one count per warp, and every block of the write
+// pass adds up the counts before its own, so there is no scan launch in between.
+// What bounds it is the chain bitmap word -> g and w -> stores of each group of 32 words, so the split is
+// by latency: as few words per warp as the count array allows (wpw = 8 up to 1M coordinates), which spreads
+// 100k coordinates over 49 blocks. (One 1024-thread block per 131,072 coordinates, the split before, put
+// them on one SM: 39 + 2 + 30 us; 1M coordinates on eight: 55 + 2 + 31 us.)
+// meta[0] = nnz, meta[1] = kind (1 sparse, 2 dense, 0 empty)
 // ---------------------------------------------------------------------------
-#define COMPACT_WPT 4
-#define COMPACT_WORDS (SKML_BLOCK * COMPACT_WPT)
-#define COMPACT_SPARSE_BITS 4  // words with at most this many bits are walked by one lane
-#define COMPACT_DENSE_BATCH 8  // dense words whose loads are in flight together
+#define COMPACT_THREADS 256
+#define COMPACT_WARPS (COMPACT_THREADS / 32)
+#define COMPACT_MIN_WPW 8
+#define COMPACT_MAX_COUNTS 4096  // warps at most: every block of the write pass reads all counts (16 KB)
+#define COMPACT_SPARSE_BITS 4    // words with at most this many bits are walked by one lane
+#define COMPACT_DENSE_BATCH 8    // dense words whose loads are in flight together
 
-__global__ void __launch_bounds__(SKML_BLOCK)
+struct CompactShape {
+    int wpw;      // bitmap words per warp: the smallest power of two from COMPACT_MIN_WPW that needs no more than
+                  // COMPACT_MAX_COUNTS warps
+    int nwarps, nblocks;
+};
+
+static CompactShape compact_shape(long long dim) {
+    const long long nwords = (dim + 31) / 32;
+    CompactShape c;
+    c.wpw = COMPACT_MIN_WPW;
+    while (nwords > (long long)c.wpw * COMPACT_MAX_COUNTS) c.wpw *= 2;
+    c.nwarps = (int)((nwords + c.wpw - 1) / c.wpw);
+    c.nblocks = (c.nwarps + COMPACT_WARPS - 1) / COMPACT_WARPS;
+    return c;
+}
+
+__global__ void __launch_bounds__(COMPACT_THREADS)
 compact_count_kernel(float* __restrict__ g, const float* __restrict__ w, unsigned int* __restrict__ bitmap,
-                     long long nwords, int dim, float lambda, unsigned int* __restrict__ block_counts) {
-    // A warp owns COMPACT_WPT groups of 32 consecutive bitmap words. Words with few bits are
-    // walked by their own lane; words with many bits are walked by the whole warp, one bit
-    // per lane, so that the g / w accesses of dense regions are coalesced. Loads are issued in
-    // batches before any of them is consumed (several memory round trips in flight per warp).
+                     long long nwords, int dim, float lambda, int wpw, int nwarps, unsigned int* __restrict__ warp_counts) {
+    // Words with few bits are walked by their own lane; words with many bits are walked by the whole
+    // warp, one bit per lane, so that the g / w accesses of dense regions are coalesced. Loads are issued
+    // in batches before any of them is consumed (several memory round trips in flight per warp).
     // The filtered value g + lambda * w is stored back into g so that the write pass reads one
     // array only.
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long wbase = (long long)blockIdx.x * COMPACT_WORDS + (long long)warp * (32 * COMPACT_WPT);
-    unsigned int bitsv[COMPACT_WPT];
-#pragma unroll
-    for (int grp = 0; grp < COMPACT_WPT; ++grp) {
-        const long long wi = wbase + grp * 32 + lane;
-        bitsv[grp] = wi < nwords ? bitmap[wi] : 0u;
-    }
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * COMPACT_WARPS + (threadIdx.x >> 5);
+    if (gw >= nwarps) return;
+    const long long wbase = (long long)gw * wpw;
+    const long long wend = wbase + wpw < nwords ? wbase + wpw : nwords;
     unsigned int cnt = 0;
-#pragma unroll
-    for (int grp = 0; grp < COMPACT_WPT; ++grp) {
-        const long long gbase = wbase + grp * 32;
+    unsigned int next = wbase + lane < wend ? bitmap[wbase + lane] : 0u;
+    for (long long gbase = wbase; gbase < wend; gbase += 32) {
         const long long wi = gbase + lane;
-        const unsigned int bits = bitsv[grp];
+        const unsigned int bits = next;
+        next = wi + 32 < wend ? bitmap[wi + 32] : 0u;   // one group ahead
         unsigned int keep = bits;
         const int pc = __popc(bits);
         if (pc > 0 && pc <= COMPACT_SPARSE_BITS) {
@@ -447,92 +466,83 @@ compact_count_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
         if (keep != bits) bitmap[wi] = keep;
         cnt += __popc(keep);
     }
-    unsigned int total;
-    block_exclusive_scan<unsigned int>(cnt, &total);
-    if (threadIdx.x == 0) block_counts[blockIdx.x] = total;
+    cnt = warp_sum(cnt);
+    if (lane == 0) warp_counts[gw] = cnt;
 }
 
-__global__ void __launch_bounds__(SKML_BLOCK)
-compact_scan_kernel(unsigned int* __restrict__ block_counts, int nblocks, int dim, int allow_dense,
-                    long long* __restrict__ meta) {
-    __shared__ unsigned int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nblocks; base += SKML_BLOCK) {
-        int i = base + threadIdx.x;
-        unsigned int v = i < nblocks ? block_counts[i] : 0u;
-        unsigned int total;
-        unsigned int ex = block_exclusive_scan<unsigned int>(v, &total);
-        unsigned int c = carry;
-        if (i < nblocks) block_counts[i] = c + ex;
-        __syncthreads();
-        if (threadIdx.x == 0) carry = c + total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        long long nnz = carry;
-        meta[0] = nnz;
-        long long thr = (long long)dim * 2 / 3;
-        meta[1] = nnz == 0 ? 0 : ((allow_dense && nnz > thr) ? 2 : 1);
-    }
-}
-
-__global__ void __launch_bounds__(SKML_BLOCK)
+__global__ void __launch_bounds__(COMPACT_THREADS)
 compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigned int* __restrict__ bitmap,
-                     long long nwords, int dim, float lambda, const unsigned int* __restrict__ block_offsets,
-                     const long long* __restrict__ meta, int* __restrict__ keys, float* __restrict__ vals,
-                     float* __restrict__ dense_vals, long long capacity, unsigned int* status) {
-    __shared__ unsigned int s_warp_off[SKML_WARPS];
-    const int kind = (int)meta[1];
+                     long long nwords, int dim, float lambda, int wpw, int nwarps,
+                     const unsigned int* __restrict__ warp_counts, long long* __restrict__ meta, int* __restrict__ keys,
+                     float* __restrict__ vals, float* __restrict__ dense_vals, long long capacity, unsigned int* status) {
+    __shared__ unsigned int s_before[COMPACT_WARPS], s_total[COMPACT_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long wbase = (long long)blockIdx.x * COMPACT_WORDS + (long long)warp * (32 * COMPACT_WPT);
-    if (kind == 2 && dense_vals != nullptr) {
+    const int gw0 = blockIdx.x * COMPACT_WARPS, gw = gw0 + warp;
+    const long long wbase = (long long)gw * wpw;
+    const long long wend = gw >= nwarps ? wbase : (wbase + wpw < nwords ? wbase + wpw : nwords);
+    unsigned int next = wbase + lane < wend ? bitmap[wbase + lane] : 0u;   // in flight while the counts are added up
+    unsigned int before = 0, total = 0;
+    for (int i = threadIdx.x; i < nwarps; i += COMPACT_THREADS) {
+        const unsigned int c = warp_counts[i];
+        total += c;
+        if (i < gw0) before += c;
+    }
+    before = warp_sum(before);
+    total = warp_sum(total);
+    if (lane == 0) {
+        s_before[warp] = before;
+        s_total[warp] = total;
+    }
+    __syncthreads();
+    before = total = 0;
+#pragma unroll
+    for (int i = 0; i < COMPACT_WARPS; ++i) {
+        before += s_before[i];
+        total += s_total[i];
+    }
+    const int kind = total == 0 ? 0 : ((dense_vals != nullptr && (long long)total > (long long)dim * 2 / 3) ? 2 : 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        meta[0] = total;
+        meta[1] = kind;
+    }
+    if (gw >= nwarps) return;
+    if (kind == 2) {
         // dense kind: every coordinate is shipped. Kept coordinates already hold g + lambda*w
         // (count pass); all others contribute lambda * w alone.
-        for (int grp = 0; grp < COMPACT_WPT; ++grp) {
-            const long long gbase = wbase + grp * 32;
+        for (long long gbase = wbase; gbase < wend; gbase += 32) {
             const long long wi = gbase + lane;
-            const unsigned int bits = wi < nwords ? bitmap[wi] : 0u;
-            if (wi < nwords) bitmap[wi] = 0;
-            for (int j = 0; j < 32; ++j) {
-                const unsigned int wb = __shfl_sync(0xFFFFFFFFu, bits, j);
-                const long long k = (gbase + j) * 32 + lane;
-                if (k < dim) {
-                    dense_vals[k] = ((wb >> lane) & 1u) ? g[k] : lambda * w[k];
-                    g[k] = 0.f;
+            const unsigned int bits = next;
+            next = wi + 32 < wend ? bitmap[wi + 32] : 0u;
+            if (wi < wend) bitmap[wi] = 0;
+            const int words = wend - gbase < 32 ? (int)(wend - gbase) : 32;
+            for (int j0 = 0; j0 < words; j0 += COMPACT_DENSE_BATCH) {
+                float v[COMPACT_DENSE_BATCH];
+#pragma unroll
+                for (int u = 0; u < COMPACT_DENSE_BATCH; ++u) {
+                    const unsigned int wb = __shfl_sync(0xFFFFFFFFu, bits, (j0 + u) & 31);
+                    const long long k = (gbase + j0 + u) * 32 + lane;
+                    v[u] = 0.f;
+                    if (j0 + u < words && k < dim) v[u] = ((wb >> lane) & 1u) ? g[k] : lambda * w[k];
+                }
+#pragma unroll
+                for (int u = 0; u < COMPACT_DENSE_BATCH; ++u) {
+                    const long long k = (gbase + j0 + u) * 32 + lane;
+                    if (j0 + u < words && k < dim) {
+                        dense_vals[k] = v[u];
+                        g[k] = 0.f;
+                    }
                 }
             }
         }
         return;
     }
-    unsigned int words[COMPACT_WPT];
-    unsigned int cnt = 0;
-#pragma unroll
-    for (int grp = 0; grp < COMPACT_WPT; ++grp) {
-        const long long wi = wbase + grp * 32 + lane;
-        words[grp] = wi < nwords ? bitmap[wi] : 0u;
-        cnt += __popc(words[grp]);
-    }
-    const unsigned int warp_total = warp_sum(cnt);
-    if (lane == 0) s_warp_off[warp] = warp_total;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned int v = s_warp_off[lane], inc = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        s_warp_off[lane] = inc - v;
-    }
-    __syncthreads();
-    long long out = (long long)block_offsets[blockIdx.x] + s_warp_off[warp];
+    long long out = before;   // keys in front of this warp's words
+    for (int i = 0; i < warp; ++i) out += warp_counts[gw0 + i];
     bool overflow = false;
-#pragma unroll
-    for (int grp = 0; grp < COMPACT_WPT; ++grp) {
-        const long long gbase = wbase + grp * 32;
+    for (long long gbase = wbase; gbase < wend; gbase += 32) {
         const long long wi = gbase + lane;
-        const unsigned int bits = words[grp];
+        const unsigned int bits = next;
+        next = wi + 32 < wend ? bitmap[wi + 32] : 0u;
         const int pc = __popc(bits);
         unsigned int inc = (unsigned int)pc;
 #pragma unroll
@@ -577,8 +587,9 @@ compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
                 jj[u] = dense ? __ffs(dense) - 1 : -1;
                 dense &= dense - 1;
                 const int src = jj[u] < 0 ? 0 : jj[u];
-                wb[u] = jj[u] < 0 ? 0u : __shfl_sync(0xFFFFFFFFu, bits, src);
+                wb[u] = __shfl_sync(0xFFFFFFFFu, bits, src);
                 exj[u] = __shfl_sync(0xFFFFFFFFu, ex, src);
+                if (jj[u] < 0) wb[u] = 0u;
                 gv[u] = ((wb[u] >> lane) & 1u) ? g[(gbase + src) * 32 + lane] : 0.f;
             }
 #pragma unroll
@@ -601,23 +612,26 @@ compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
     if (overflow) skml_set_status(status, SKML_CAPACITY, 0x20u);
 }
 
-extern "C" int skml_compact(float* g, const float* w, unsigned int* bitmap, int dim, float lambda,
-                            unsigned int* block_counts, long long* meta, int* keys, float* vals, float* dense_vals,
-                            long long capacity, unsigned int* status, void* stream_) {
-    cudaStream_t stream = (cudaStream_t)stream_;
-    long long nwords = ((long long)dim + 31) / 32;
-    int nblocks = (int)((nwords + COMPACT_WORDS - 1) / COMPACT_WORDS);
-    compact_count_kernel<<<nblocks, SKML_BLOCK, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, block_counts);
-    compact_scan_kernel<<<1, SKML_BLOCK, 0, stream>>>(block_counts, nblocks, dim, dense_vals != nullptr, meta);
-    compact_write_kernel<<<nblocks, SKML_BLOCK, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, block_counts, meta,
-                                                            keys, vals, dense_vals, capacity, status);
+static int compact_launch(float* g, const float* w, unsigned int* bitmap, int dim, float lambda, unsigned int* warp_counts,
+                          long long* meta, int* keys, float* vals, float* dense_vals, long long capacity, unsigned int* status,
+                          cudaStream_t stream) {
+    const long long nwords = ((long long)dim + 31) / 32;
+    const CompactShape c = compact_shape(dim);
+    compact_count_kernel<<<c.nblocks, COMPACT_THREADS, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts);
+    compact_write_kernel<<<c.nblocks, COMPACT_THREADS, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts,
+                                                                    meta, keys, vals, dense_vals, capacity, status);
     return (int)cudaGetLastError();
 }
 
-extern "C" long long skml_compact_blocks(int dim) {
-    long long nwords = ((long long)dim + 31) / 32;
-    return (nwords + COMPACT_WORDS - 1) / COMPACT_WORDS;
+extern "C" int skml_compact(float* g, const float* w, unsigned int* bitmap, int dim, float lambda,
+                            unsigned int* block_counts, long long* meta, int* keys, float* vals, float* dense_vals,
+                            long long capacity, unsigned int* status, void* stream_) {
+    return compact_launch(g, w, bitmap, dim, lambda, block_counts, meta, keys, vals, dense_vals, capacity, status,
+                          (cudaStream_t)stream_);
 }
+
+// Entries of the caller's count array.
+extern "C" long long skml_compact_blocks(int dim) { return compact_shape(dim).nwarps; }
 
 // ---------------------------------------------------------------------------
 // Updates for the uncompressed baselines (the compressed path updates inside the
@@ -1284,14 +1298,8 @@ extern "C" int skml_compact_noalloc(float* g, const float* w, unsigned int* bitm
     unsigned int* scratch = nullptr;
     int rc = noalloc_scratch(&scratch);
     if (rc) return rc;
-    cudaStream_t stream = (cudaStream_t)stream_;
-    long long nwords = ((long long)dim + 31) / 32;
-    int nblocks = (int)((nwords + COMPACT_WORDS - 1) / COMPACT_WORDS);
-    // every entry of the scratch that is read (the first nblocks) is rewritten by the count
+    // every entry of the scratch that is read (one per warp, at most COMPACT_MAX_COUNTS) is rewritten by the count
     // kernel of this call, so nothing of an earlier call has to be cleared
-    compact_count_kernel<<<nblocks, SKML_BLOCK, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, scratch);
-    compact_scan_kernel<<<1, SKML_BLOCK, 0, stream>>>(scratch, nblocks, dim, 0, meta);
-    compact_write_kernel<<<nblocks, SKML_BLOCK, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, scratch, meta, keys,
-                                                            vals, nullptr, capacity, status);
-    return (int)cudaGetLastError();
+    static_assert(COMPACT_MAX_COUNTS <= SKML_NOALLOC_MAX_BLOCKS + 64, "the built-in scratch holds one count per warp");
+    return compact_launch(g, w, bitmap, dim, lambda, scratch, meta, keys, vals, nullptr, capacity, status, (cudaStream_t)stream_);
 }

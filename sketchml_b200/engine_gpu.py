@@ -276,7 +276,7 @@ class GpuEngine:
         if lid is not None:
             L.count_launches(len(segs) + 2 + 2)  # gather, gradient segment(s), finalize, compress, decode
         else:
-            L.count_launches((3 if bi is not None else len(segs) + 3) + 1 +
+            L.count_launches((3 if bi is not None else len(segs) + 2) + 1 +
                              (1 if self.st.dense_vals is not None and bi is None else 0) + 1)
 
     # ----------------------------------------------------------------- steps

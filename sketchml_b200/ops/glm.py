@@ -111,7 +111,7 @@ def compact_gradient(st: GlmState, w: torch.Tensor, lam: float) -> None:
     L.check(L.lib().skml_compact(L.ptr(st.g), L.ptr(w), L.ptr(st.bitmap), st.dim, float(lam), L.ptr(st.block_counts),
                                  L.ptr(st.meta), L.ptr(st.keys), L.ptr(st.vals), L.ptr(st.dense_vals), st.n_max,
                                  L.ptr(st.status), L.stream()), "skml_compact")
-    L.count_launches(3)
+    L.count_launches(2)
 
 
 def moment_stride(m, v) -> int:

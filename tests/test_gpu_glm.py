@@ -217,3 +217,41 @@ def test_row_tiled_index_matches_the_per_column_form(binary, tile_rows_max, rows
     assert torch.equal(outs[1], outs[2])
     assert float((outs[0].double() - outs[1].double()).abs().max()) < 2e-6 * max(1.0, float(outs[0].abs().max()))
 
+
+
+@pytest.mark.parametrize("dim", [1, 31, 33, 256, 257, 8 * 256 + 1, 100_000, 4096 * 256, 4096 * 256 + 1, 3_000_001])
+@pytest.mark.parametrize("density", [0.02, 0.6, 0.95])
+def test_compaction_over_its_splits(dim, density):
+    """Edges of the warps' word ranges: one warp, a ragged last warp, the last size with the smallest range and the
+    first with the next one; sparse words, dense words and the dense kind."""
+    from sketchml_b200.ops.glm import GlmState, compact_gradient
+    dev, lam = torch.device("cuda"), 0.5
+    gen = torch.Generator().manual_seed(dim)
+    touched = torch.rand(dim, generator=gen) < density
+    g = torch.where(touched, torch.randn(dim, generator=gen), torch.zeros(dim))
+    g[::9] = torch.where(touched[::9], torch.full_like(g[::9], 1e-9), g[::9])   # falls to the filter where w is zero
+    w = torch.randn(dim, generator=gen)
+    w[::9] = 0.0
+    for allow_dense in (False, True):
+        st = GlmState.create(dim, dim, dev, allow_dense)
+        st.g.copy_(g)
+        words = torch.zeros((dim + 31) // 32 * 32, dtype=torch.int64)
+        words[:dim] = touched.long()
+        bits = (words.view(-1, 32) << torch.arange(32)).sum(1)
+        st.bitmap[:bits.numel()].copy_(torch.where(bits >= 2 ** 31, bits - 2 ** 32, bits).to(torch.int32))
+        compact_gradient(st, w.to(dev), lam)
+        v = (g + lam * w)    # one rounding of the product, one of the sum (or a fused one): 2 ulp
+        keep = touched & (v.abs() > 1e-8)
+        n, kind = int(st.meta[0]), int(st.meta[1])
+        assert int(st.status.item()) == 0 and n == int(keep.sum())
+        dense = allow_dense and n > dim * 2 // 3
+        assert kind == (0 if n == 0 else 2 if dense else 1)
+        if dense:
+            want = torch.where(touched & ~keep, torch.zeros(dim), torch.where(keep, v, lam * w))
+            want = torch.where(touched & ~keep, lam * w, want)
+            assert torch.allclose(st.dense_vals.cpu(), want, rtol=3e-7, atol=3e-7)
+        else:
+            idx = torch.nonzero(keep).flatten()
+            assert torch.equal(st.keys[:n].cpu().long(), idx)
+            assert torch.allclose(st.vals[:n].cpu(), v[idx], rtol=3e-7, atol=3e-7)
+        assert float(st.g.abs().max()) == 0.0 and int(st.bitmap.abs().max()) == 0
