@@ -317,7 +317,7 @@ SKML_HD void skml_pick_hashes(uint64_t seed, uint64_t step, uint32_t rank, uint3
         ids[i] = ids[j];
         ids[j] = t;
     }
-    for (int i = 7; i > 3; --i) {  // Fisher-Yates over the BKDR members ids[3..7]
+    for (int i = 7; i > 3 && rows > 3; --i) {  // Fisher-Yates over the BKDR members ids[3..7]
         uint64_t r = skml_rand(seed, step, ((uint64_t)rank << 32) | group, (uint64_t)i);
         int j = 3 + (int)(r % (uint64_t)(i - 2));
         uint8_t t = ids[i];

@@ -86,6 +86,9 @@ struct CP {
     const float* given_splits;
     int n_given;
     float given_min, given_max;
+    unsigned long long sample_rand;                      // draw behind the sample's offset (host: seed, step, rank)
+    int mixers;                                          // every row of every group uses an integer mixer (<= 3 rows)
+    unsigned char hash_ids[SKML_MAX_GROUPS][SKML_MAX_ROWS];  // hash rows of every group (host: seed, step, rank, group)
 };
 
 struct QInfo {
@@ -110,10 +113,10 @@ struct Layout {
     unsigned long long tbits[SKML_MAX_GROUPS], tstream_off[SKML_MAX_GROUPS], trestart_off[SKML_MAX_GROUPS];
     unsigned long long table_off[SKML_MAX_GROUPS], flag_off[SKML_MAX_GROUPS], delta_off[SKML_MAX_GROUPS],
         restart_off[SKML_MAX_GROUPS], tab32_off[SKML_MAX_GROUPS];
-    unsigned char hash_ids[SKML_MAX_GROUPS][8];
-    unsigned long long col_magic[SKML_MAX_GROUPS];  // ceil(2^64 / col) for the division-free modulo
+    unsigned long long col_magic[SKML_MAX_GROUPS];  // ceil(2^64 / col) for the division-free modulo (other hash rows only)
     unsigned int recip[SKML_MAX_GROUPS];            // floor(2^32 / col) for the mixer-only hash path
-    int mixers;                                     // every row of every group uses an integer mixer (<= 3 rows)
+    unsigned char hash_ids[SKML_MAX_GROUPS][SKML_MAX_ROWS];  // CP's, where the lanes of a warp may differ in the group
+    unsigned long long unit_prefix[SKML_MAX_GROUPS + 1];  // 16-byte units of the narrow tables of the groups before
     unsigned long long off_bv, off_gt, off_flags, off_restart, off_tables, off_deltas, total_bytes;
     int overflow;
 };
@@ -147,7 +150,7 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
     L.tchunk_off = o; o += al256(((rows * ((long long)(col_ratio * (double)n_max) + 2 + G) + 64) / 1024 + SKML_MAX_GROUPS + 8) * 4);
     L.bins = o; o += al256(n_max * 2);
     L.gkeys = o; o += al256((n_max + 4 * SKML_MAX_GROUPS + 8) * 4);
-    L.tables_cap = rows * ((long long)(col_ratio * (double)n_max) + 2 + G) + 64;
+    L.tables_cap = rows * ((long long)(col_ratio * (double)n_max) + 2 + G) + 64 + 4 * G;  // groups' tables start at multiples of 4 cells
     L.tables = o; o += al256(L.tables_cap * 4);
     L.total = o;
     return L;
@@ -234,8 +237,10 @@ struct Smem {
     unsigned long long my_bits[2 * SKML_MAX_GROUPS], pre_bits[2 * SKML_MAX_GROUPS];  // delta_adaptive: flag / delta bits
     unsigned long long my_tbits[SKML_MAX_GROUPS], pre_tbits[SKML_MAX_GROUPS];
     unsigned int sub_part[4][8];                    // scan scratch of the four 256-thread sub-blocks
-    unsigned int sub_total[4];
-    unsigned long long unit_prefix[SKML_MAX_GROUPS + 1];
+    unsigned int sub_total[4], sub_off[4];
+    unsigned long long sums[5];                      // layout_from_counts: totals of its five prefix sums
+    unsigned int scan[2][SKML_WARPS];                // block_rank scratch, alternating
+    alignas(16) SkmlHeader hdr;                      // copied out in 16-byte units
     int flag;
 };
 
@@ -243,6 +248,7 @@ struct Smem {
 // 164 KB is a shared-memory carve-out step of the SM: staying under it (with the block's static shared
 // memory and the 1 KB the system reserves) leaves 92 KB of L1; measured, the scatter + insert stage of
 // 2.3M keys takes 69 us with that L1 and 120 us with the 28 KB that the next step (228 KB) leaves.
+static_assert(offsetof(Smem, hdr) % 16 == 0, "the header is read in 16-byte units");
 static_assert(sizeof(Smem) <= 162 * 1024, "the compress kernels' shared memory must stay below the 164 KB carve-out");
 
 __device__ __forceinline__ unsigned int lanemask_lt() {
@@ -362,7 +368,7 @@ __device__ void summarize_slice(const CP& p, Smem& s, const float* __restrict__ 
             }
             __syncthreads();
             if (st == t0) stage_stamp(p.ctrl, 10);
-            block_sort_2048(s.qs.tile);
+            block_sort_2048(s.qs.tile, s.qs.runs_all);
             if (st == t0) stage_stamp(p.ctrl, 11);
             const unsigned int off = (unsigned int)(skml_rand(p.seed, p.step, ((unsigned long long)p.rank << 32) | blockIdx.x,
                                                               0x7200u + (unsigned long long)((st - t0) / gridDim.x)) & (TILE_W - 1));
@@ -389,7 +395,7 @@ __device__ void summarize_slice(const CP& p, Smem& s, const float* __restrict__ 
             s.qs.tile[t] = chosen;
         }
         __syncthreads();
-        block_sort_2048(s.qs.tile);
+        block_sort_2048(s.qs.tile, s.qs.runs_all);
         int stride = 1;
         while ((ms + stride - 1) / stride > SK_K) stride <<= 1;
         tail_cnt = (ms + stride - 1) / stride;
@@ -604,6 +610,19 @@ __device__ void stage_summary(const CP& p, Smem& s, const float* __restrict__ va
     }
 }
 
+// Warp-wide exclusive prefix sum; `total` = the warp's sum.
+__device__ __forceinline__ unsigned long long warp_prefix(unsigned long long v, unsigned long long& total) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    return inc - v;
+}
+
 // S1, sample form. Every thread-block cluster draws the SAME stratified sample of the values (one value
 // per stride of n / m positions, the offset a function of (seed, step, rank)), so every block ends up with
 // the same split points without a grid barrier and without S2. The two blocks of a cluster sort one half
@@ -613,51 +632,59 @@ __device__ void stage_summary(const CP& p, Smem& s, const float* __restrict__ va
 // The rank error of a split is that of an m-value sample (standard deviation at most 0.8 % of n at
 // m = 4096), the same order as the k = 128 summary's; inputs of up to m values are summarised exactly.
 // Minimum and maximum of ALL values are taken by the count stage, which reads every value anyway.
+// The splits stay in the block's shared memory (raw_splits); block 0 also leaves them in the workspace.
+__device__ __forceinline__ unsigned int* raw_splits(Smem& s) { return s.qs.runs_all + TILE; }
+
 __device__ void stage_sample_splits(const CP& p, Smem& s, const float* __restrict__ vals, long long n) {
     const unsigned int cs = cluster_nctarank(), cr = cluster_ctarank();
-    const int halves = cs >= 2 ? 2 : 1;
+    const int lh = cs >= 2 ? 1 : 0, halves = 1 << lh;
     const long long M = (long long)TILE * halves;
     const long long m = n < M ? n : M;   // sample size
-    const unsigned long long off = n > m ? skml_rand(p.seed, p.step, p.rank, 0x7300u) % (unsigned long long)n : 0ull;
-    const int mine = (int)((m - (long long)(cr % halves) + halves - 1) / halves);   // samples in this block's half
+    __shared__ unsigned long long s_off;
+    if (threadIdx.x == 0) s_off = n > m ? p.sample_rand % (unsigned long long)n : 0ull;
+    __syncthreads();
+    const unsigned long long off = s_off;
+    const int half = (int)cr & (halves - 1);
+    const int mine = (int)((m - half + halves - 1) >> lh);   // samples in this block's half
     for (int t = threadIdx.x; t < TILE; t += blockDim.x) {
-        const long long j = (long long)t * halves + (cr % halves);
+        const long long j = ((long long)t << lh) + half;
         unsigned int key = 0xFFFFFFFFu;
         if (j < m) {
-            const long long pos = n > m ? (long long)(((unsigned long long)j * (unsigned long long)n + off) / (unsigned long long)m) : j;
+            // m is a power of two (TILE * halves) whenever it is not n itself
+            const long long pos = n > m ? (long long)(((unsigned long long)j * (unsigned long long)n + off) >> (11 + lh)) : j;
             key = f2ord(__ldg(vals + pos));
         }
         s.qs.tile[t] = key;
     }
     __syncthreads();
-    block_sort_2048(s.qs.tile);
-    __syncthreads();
+    block_sort_2048(s.qs.tile, s.qs.runs_all);
     const int theirs = (int)(m - mine);
     unsigned int* const their = s.qs.runs_all;   // local copy of the other block's sorted half
     if (halves == 2) {
         cluster_sync_all();   // both halves are sorted and visible in the cluster
-        const unsigned int other = dsmem_addr(s.qs.tile, (cr % halves) ^ 1u);
+        const unsigned int other = dsmem_addr(s.qs.tile, (unsigned int)half ^ 1u);
         for (int t = threadIdx.x; t < theirs; t += blockDim.x) their[t] = ld_dsmem_u32(other + 4u * (unsigned int)t);
-        cluster_sync_all();   // nobody reads the other block's shared memory any more
+        cluster_sync_all();   // nobody reads the other block's shared memory any more; the copy is complete
     }
-    __syncthreads();
     const double inv_q = 1.0 / (double)p.q;
     for (int t = threadIdx.x; t < p.q - 1; t += blockDim.x) {
-        long long k = (long long)((double)m * ((double)(t + 1) * inv_q));   // target rank in the sample
-        if (k > m - 1) k = m - 1;
+        int k = (int)((double)m * ((double)(t + 1) * inv_q));   // target rank in the sample (m <= 4096)
+        if (k > (int)m - 1) k = (int)m - 1;
         // i = how many of the k values before the answer come from this block's half (ties: this half first)
-        int lo = (int)(k - theirs > 0 ? k - theirs : 0), hi = (int)(k < mine ? k : mine);
+        int lo = k - theirs > 0 ? k - theirs : 0, hi = k < mine ? k : mine;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            const long long j = k - mid;
+            const int j = k - mid;
             const bool ok = j >= theirs || s.qs.tile[mid - 1] <= their[j];
             if (ok) lo = mid;
             else hi = mid - 1;
         }
-        const long long j = k - lo;
+        const int j = k - lo;
         const unsigned int a = lo < mine ? s.qs.tile[lo] : 0xFFFFFFFFu;
         const unsigned int b = j < theirs ? their[j] : 0xFFFFFFFFu;
-        p.splits_raw[t] = a < b ? a : b;   // every block stores the same values
+        const unsigned int key = a < b ? a : b;
+        raw_splits(s)[t] = key;
+        if (blockIdx.x == 0) p.splits_raw[t] = key;
     }
     __syncthreads();
 }
@@ -755,70 +782,93 @@ __device__ void stage_query(const CP& p, Smem& s, long long n) {
 // ---------------------------------------------------------------------------
 // S3 prelude: unique splits, zero bucket, group edges (every block, in shared memory)
 // ---------------------------------------------------------------------------
+// Positions of the kept items of one round of blockDim items (thread order), and how many of them are
+// negative: one block barrier. `par` alternates between calls.
+__device__ __forceinline__ unsigned int block_rank(Smem& s, int par, bool keep, bool neg, unsigned int& total, unsigned int& total_neg) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned int km = __ballot_sync(0xFFFFFFFFu, keep), nm = __ballot_sync(0xFFFFFFFFu, keep && neg);
+    if (lane == 0) s.scan[par][warp] = (unsigned int)__popc(km) | ((unsigned int)__popc(nm) << 16);
+    __syncthreads();
+    const unsigned int c = s.scan[par][lane];
+    const unsigned int all = __reduce_add_sync(0xFFFFFFFFu, c), before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? c & 0xFFFFu : 0u);
+    total = all & 0xFFFFu;
+    total_neg = all >> 16;
+    return before + (unsigned int)__popc(km & lanemask_lt());
+}
+
+// Distinct splits, zero bucket and group edges, in the shared memory of every block.
+// in_smem: the raw split points are in raw_splits(s) (sample form, same launch), otherwise in the workspace.
 // minmax_ready = false: the minimum and maximum of the values are not known yet (sample form before the
 // count stage has run); the zero bucket does not need them (see below), refresh_minmax sets them later.
-__device__ void load_quantizer(const CP& p, Smem& s, bool minmax_ready = true) {
+__device__ void load_quantizer(const CP& p, Smem& s, bool in_smem = false, bool minmax_ready = true) {
     const bool given = p.given_splits != nullptr;
     const int nraw = given ? p.n_given : p.q - 1;
-    __shared__ int s_base;
-    if (threadIdx.x == 0) s_base = 0;
-    __syncthreads();
-    for (int b = 0; b < nraw; b += blockDim.x) {
-        int i = b + threadIdx.x;
-        float v = 0.f, prev = 0.f;
+    auto raw = [&](int i) { return given ? p.given_splits[i] : ord2f(in_smem ? raw_splits(s)[i] : __ldcg(p.splits_raw + i)); };
+    unsigned int base = 0, negs = 0;
+    int par = 0;
+    for (int b = 0; b < nraw; b += blockDim.x, par ^= 1) {
+        const int i = b + threadIdx.x;
+        float v = 0.f;
         bool keep = false;
         if (i < nraw) {
-            v = given ? p.given_splits[i] : ord2f(__ldcg(p.splits_raw + i));
-            if (i > 0) prev = given ? p.given_splits[i - 1] : ord2f(__ldcg(p.splits_raw + i - 1));
-            keep = i == 0 || v != prev;
+            v = raw(i);
+            keep = i == 0 || v != raw(i - 1);
         }
-        unsigned int total;
-        unsigned int pos = block_exclusive_scan<unsigned int>(keep ? 1u : 0u, &total);
-        int base = s_base;
+        unsigned int total, total_neg;
+        const unsigned int pos = block_rank(s, par, keep, v < 0.f, total, total_neg);
         if (keep) s.splits[base + pos] = v;
-        __syncthreads();
-        if (threadIdx.x == 0) s_base = base + (int)total;
-        __syncthreads();
+        base += total;
+        negs += total_neg;
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         QInfo& q = s.qi;
-        q.nsplits = s_base;
-        q.bin_num = s_base + 1;
-        q.cell_bits = q.bin_num <= 256 ? 8 : 16;
+        const int lane = threadIdx.x, bin_num = (int)base + 1, G = p.G;
+        float minv = 0.f, maxv = 0.f;
         if (given) {
-            q.minv = p.given_min;
-            q.maxv = p.given_max;
+            minv = p.given_min;
+            maxv = p.given_max;
         } else if (minmax_ready) {
-            q.minv = ord2f(~__ldcg(p.ctrl + 4));
-            q.maxv = ord2f(__ldcg(p.ctrl + 5));
-        } else {
-            q.minv = q.maxv = 0.f;
+            minv = ord2f(~__ldcg(p.ctrl + 4));
+            maxv = ord2f(__ldcg(p.ctrl + 5));
         }
-        // NaN or infinite gradient values cannot be bucketized (the reference's sketch throws on NaN)
-        if (!isfinite(q.minv) || !isfinite(q.maxv)) skml_set_status(p.status, SKML_BAD_INPUT, 0x35u);
-        // With splits taken from the data, min > 0 means every split is positive and max < 0 that every split
-        // is negative, so the search below gives the first two cases' answers too; they stay for given splits.
-        int z;
-        if ((given || minmax_ready) && q.minv > 0.f) z = 0;
-        else if ((given || minmax_ready) && q.maxv < 0.f) z = q.bin_num - 1;
-        else {
-            z = 0;
-            while (z < q.bin_num - 1 && s.splits[z] < 0.f) ++z;
+        // The splits ascend, so the zero bucket (the first whose upper split is not negative) is their number of
+        // negative ones. With splits taken from the data, min > 0 means every split is positive and max < 0 that
+        // every split is negative, so that count gives the first two cases' answers too; they stay for given splits.
+        int z = (int)negs;
+        if ((given || minmax_ready) && minv > 0.f) z = 0;
+        else if ((given || minmax_ready) && maxv < 0.f) z = bin_num - 1;
+        // group edges as skml_group_edges, one lane per group: from the third group on an edge is the one before it
+        // plus a constant, cut at bin_num
+        int edge = bin_num;
+        if (G == 2 && lane == 0) edge = z;
+        if (G > 2 && lane < G - 1) {
+            int bpg = bin_num / G;
+            if (bpg < 1) bpg = 1;
+            const int rem = z % bpg;
+            const int e0 = z < bpg ? z : (rem < bpg / 2 ? bpg + rem : rem);
+            edge = lane == 0 ? e0 : min(e0 + lane * bpg, bin_num);
         }
-        q.zero_idx = z;
-        skml_group_edges(z, q.bin_num, p.G, q.edges);
+        if (lane < G) q.edges[lane] = edge;
+        if (lane == 0) {
+            q.nsplits = (int)base;
+            q.bin_num = bin_num;
+            q.cell_bits = bin_num <= 256 ? 8 : 16;
+            q.minv = minv;
+            q.maxv = maxv;
+            q.zero_idx = z;
+            // NaN or infinite gradient values cannot be bucketized (the reference's sketch throws on NaN)
+            if (!isfinite(minv) || !isfinite(maxv)) skml_set_status(p.status, SKML_BAD_INPUT, 0x35u);
+        }
     }
     __syncthreads();
 }
 
-// Sample form, after the count stage and its grid barrier: minimum and maximum of all values.
+// Sample form, after the count stage and its grid barrier: minimum and maximum of all values (one thread; the
+// caller has a block barrier after it).
 __device__ void refresh_minmax(const CP& p, Smem& s) {
-    if (threadIdx.x == 0) {
-        s.qi.minv = ord2f(~__ldcg(p.ctrl + 4));
-        s.qi.maxv = ord2f(__ldcg(p.ctrl + 5));
-        if (!isfinite(s.qi.minv) || !isfinite(s.qi.maxv)) skml_set_status(p.status, SKML_BAD_INPUT, 0x35u);
-    }
-    __syncthreads();
+    s.qi.minv = ord2f(~__ldcg(p.ctrl + 4));
+    s.qi.maxv = ord2f(__ldcg(p.ctrl + 5));
+    if (!isfinite(s.qi.minv) || !isfinite(s.qi.maxv)) skml_set_status(p.status, SKML_BAD_INPUT, 0x35u);
 }
 
 __device__ __forceinline__ float bucket_value(const Smem& s, int b) {
@@ -839,14 +889,25 @@ __device__ __forceinline__ long long vslice_size(long long n) {
     return (c + 31) / 32 * 32;
 }
 
-__device__ __forceinline__ void build_group_lut(const CP& p, Smem& s) {
-    for (int b = threadIdx.x; b < s.qi.bin_num; b += blockDim.x) s.grp_lut[b] = (unsigned char)skml_group_of(b, s.qi.edges, p.G);
+__device__ __forceinline__ void clear_warp_counts(Smem& s) {
     for (int t = threadIdx.x; t < SKML_WARPS * SKML_MAX_GROUPS; t += blockDim.x) (&s.wcnt[0][0])[t] = 0;
+}
+
+__device__ __forceinline__ void build_group_lut(const CP& p, Smem& s) {
+    for (int b = threadIdx.x; b < s.qi.bin_num; b += blockDim.x) {
+        int g = 0;   // the edges ascend: the group is the number of edges at or below the bucket
+        for (int e = 0; e < p.G - 1; ++e) g += s.qi.edges[e] <= b ? 1 : 0;
+        s.grp_lut[b] = (unsigned char)g;
+    }
+    clear_warp_counts(s);
     __syncthreads();
 }
 
 // S3: bucket of every value; keys of every group in every warp slice.
-__device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax) {
+// `first_val`: the value of this lane's first element where the caller has it in flight already; returns that
+// element's bucket.
+template <bool FUSED>
+__device__ int stage_count(const CP& p, Smem& s, long long n, bool track_minmax, float first_val) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
     build_group_lut(p, s);
@@ -855,8 +916,8 @@ __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax
     long long lo = vb * sub, hi = lo + sub;
     if (lo > n) lo = n;
     if (hi > n) hi = n;
-    float nval = 0.f;
-    if (lo + lane < hi) nval = p.vals[lo + lane];  // one iteration ahead: the load latency stays off the chain
+    int first_bin = 0;
+    float nval = first_val;  // one iteration ahead: the load latency stays off the chain
     for (long long i0 = lo; i0 < hi; i0 += 32) {
         const long long i = i0 + lane;
         const bool valid = i < hi;
@@ -866,6 +927,7 @@ __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax
         if (valid) {
             const int bin = upper_bound_f(s.splits, s.qi.nsplits, val);
             p.bins[i] = (unsigned short)bin;
+            if (i0 == lo) first_bin = bin;
             g = s.grp_lut[bin];
             const unsigned int k = f2ord(val);
             kmin = min(kmin, k);
@@ -875,7 +937,8 @@ __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax
         if (valid && (peers & lanemask_lt()) == 0) s.wcnt[warp][g] += (unsigned int)__popc(peers);  // one leader per group
         __syncwarp();
     }
-    if (lane < p.G) p.warp_cnt[vb * SKML_MAX_GROUPS + lane] = s.wcnt[warp][lane];
+    // (one launch for all stages: the slices' counts stay in shared memory)
+    if (!FUSED && lane < p.G) p.warp_cnt[vb * SKML_MAX_GROUPS + lane] = s.wcnt[warp][lane];
     __syncthreads();
     if (warp < p.G) {  // the block's totals: warp g adds up group g over the 32 slices
         const unsigned int tot = warp_sum(s.wcnt[lane][warp]);
@@ -907,14 +970,17 @@ __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax
             }
         }
     }
+    return first_bin;
 }
 
 // S4 prelude: group sizes, table sizes, hash rows and every section offset that does not depend on
 // the key code (every block computes the same layout); this block's and its warps' starting ranks.
-__device__ void layout_from_counts(const CP& p, Smem& s) {
+template <bool FUSED>
+__device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
     const int G = p.G, nb = gridDim.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Layout& L = s.lay;
+    if (want_minmax && threadIdx.x == SKML_BLOCK - 1) refresh_minmax(p, s);
     if (warp < G) {
         const int g = warp;
         // the blocks' totals (before this block / all blocks), lanes striding over the blocks; this
@@ -925,9 +991,9 @@ __device__ void layout_from_counts(const CP& p, Smem& s) {
             total += c;
             if (b < (int)blockIdx.x) before += c;
         }
-        const unsigned int own = __ldcg(&p.warp_cnt[((long long)blockIdx.x * SKML_WARPS + lane) * SKML_MAX_GROUPS + g]);
-        total = warp_sum(total);
-        before = warp_sum(before);
+        const unsigned int own = FUSED ? s.wcnt[lane][g] : __ldcg(&p.warp_cnt[((long long)blockIdx.x * SKML_WARPS + lane) * SKML_MAX_GROUPS + g]);
+        total = __reduce_add_sync(0xFFFFFFFFu, total);
+        before = __reduce_add_sync(0xFFFFFFFFu, before);
         unsigned int inc = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -939,76 +1005,95 @@ __device__ void layout_from_counts(const CP& p, Smem& s) {
             L.n_g[g] = total;
             L.base_rank[g] = before;
         }
+        if (lane < SKML_MAX_ROWS) L.hash_ids[g][lane] = p.hash_ids[g][lane];
     }
     __syncthreads();
-    if (threadIdx.x < G) {  // per-group divisions and hash draws, one thread each
-        const int g = threadIdx.x;
+    // One lane per group, one warp per quantity: sizes, then prefix sums over the lanes. (One thread that walked the
+    // groups took 3 us of a 62 us launch at 10,000 keys.)
+    const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE;
+    if (warp < 5) {
+        const unsigned int n = lane < G ? L.n_g[lane] : 0u;
+        unsigned long long v = 0;
         unsigned int col = 0;
-        if (L.n_g[g]) {
-            col = (unsigned int)ceil((double)L.n_g[g] * p.col_ratio);
-            if (col < 1) col = 1;
+        if (warp == 2 || warp == 3) {
+            if (n) {
+                col = (unsigned int)ceil((double)n * p.col_ratio);
+                if (col < 1) col = 1;
+            }
+            const unsigned long long cells = (unsigned long long)p.rows * col;
+            v = warp == 2 ? skml_align16(cells * (s.qi.cell_bits / 8)) : (cells + 3ull) & ~3ull;
+        } else if (warp == 0) {
+            v = n && !adaptive ? skml_align16(8ull * ((2ull * n + 63) / 64)) : 0ull;   // flag bytes
+        } else if (warp == 1) {
+            v = ((unsigned long long)((n + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL) << 32) | ((n + 3u) & ~3u);  // chunks | staging entries
+        } else if (lane < G) {
+            // the key code adds at most four bytes per key (delta_adaptive: 49 bits): refuse now what cannot
+            // fit in the worst case
+            v = skml_align16(4ull * n + 8) + (adaptive ? skml_align16(17ull * n / 8 + 8) : 0ull);
         }
-        L.col[g] = col;
-        L.col_magic[g] = col ? skml_fastmod_magic(col) : 0ull;
-        L.recip[g] = skml_recip32(col);
-        skml_pick_hashes(p.seed, p.step, p.rank, (unsigned int)g, p.rows, L.hash_ids[g]);
+        unsigned long long total;
+        const unsigned long long o = warp_prefix(v, total);
+        if (lane < G) {
+            if (warp == 0) L.flag_off[lane] = o;
+            else if (warp == 1) {
+                L.goff[lane] = (unsigned int)o;
+                L.chunk_prefix[lane] = (unsigned int)(o >> 32);
+            } else if (warp == 2) {
+                L.table_off[lane] = o;
+                L.unit_prefix[lane] = o / 16;
+                L.col[lane] = col;
+                L.recip[lane] = skml_recip32(col);
+            } else if (warp == 3) {
+                L.tab32_off[lane] = o;
+                if (!p.mixers) L.col_magic[lane] = col ? skml_fastmod_magic(col) : 0ull;
+            }
+        }
+        if (lane == 0) s.sums[warp] = total;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        bool mix = p.rows <= 3;
-        for (int g = 0; g < G && mix; ++g) mix = skml_rows_are_mixers(L.hash_ids[g], p.rows);
-        L.mixers = mix ? 1 : 0;
-        const int cb = s.qi.cell_bits;
-        L.off_bv = SKML_HEADER_BYTES;
-        L.off_gt = L.off_bv + skml_align16(4ull * p.q);
-        L.off_flags = L.off_gt + (unsigned long long)SKML_GROUP_ENTRY_BYTES * G;
-        const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE;
-        unsigned long long o = L.off_flags;
-        unsigned int go = 0, ch = 0;
-        for (int g = 0; g < G; ++g) {
-            L.flag_off[g] = o;
-            if (L.n_g[g] && !adaptive) o += skml_align16(8ull * ((2ull * L.n_g[g] + 63) / 64));
-            L.goff[g] = go;
-            go += (L.n_g[g] + 3u) & ~3u;
-            L.chunk_prefix[g] = ch;
-            ch += (L.n_g[g] + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL;
+    if (warp == 0) {   // the sections' starts
+        const unsigned long long off_gt = SKML_HEADER_BYTES + skml_align16(4ull * p.q);
+        const unsigned long long off_flags = off_gt + (unsigned long long)SKML_GROUP_ENTRY_BYTES * G;
+        const unsigned int chunks = (unsigned int)(s.sums[1] >> 32);
+        const unsigned long long off_restart = off_flags + s.sums[0], off_tables = off_restart + 16ull * chunks;
+        const unsigned long long off_deltas = off_tables + s.sums[2];
+        if (lane < G) {
+            L.flag_off[lane] += off_flags;
+            L.restart_off[lane] = off_restart + 16ull * L.chunk_prefix[lane];
+            L.table_off[lane] += off_tables;
         }
-        L.chunk_prefix[G] = ch;
-        L.off_restart = o;
-        for (int g = 0; g < G; ++g) {
-            L.restart_off[g] = o;
-            if (L.n_g[g]) o += 16ull * ((L.n_g[g] + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL);
+        if (lane == 0) {
+            L.off_bv = SKML_HEADER_BYTES;
+            L.off_gt = off_gt;
+            L.off_flags = off_flags;
+            L.off_restart = off_restart;
+            L.off_tables = off_tables;
+            L.off_deltas = off_deltas;
+            L.off_keys = off_deltas;  // delta_adaptive: both key sections of every group follow the tables
+            L.chunk_prefix[G] = chunks;
+            L.unit_prefix[G] = s.sums[2] / 16;
+            L.overflow = (off_deltas + s.sums[4] > (unsigned long long)p.slot_capacity) || (s.sums[3] + 4 > (unsigned long long)p.tables_cap);
+            if (L.overflow) skml_set_status(p.status, SKML_CAPACITY, 0x30u);
         }
-        L.off_tables = o;
-        unsigned long long t32 = 0;
-        for (int g = 0; g < G; ++g) {
-            const unsigned int col = L.col[g];
-            L.table_off[g] = o;
-            L.tab32_off[g] = t32;
-            o += skml_align16((unsigned long long)p.rows * col * (cb / 8));
-            t32 += (unsigned long long)p.rows * col;
-        }
-        L.off_deltas = o;
-        L.off_keys = o;  // delta_adaptive: both key sections of every group follow the tables
-        // the key code adds at most four bytes per key (delta_adaptive: 49 bits): refuse now what cannot
-        // fit in the worst case
-        unsigned long long worst = o;
-        for (int g = 0; g < G; ++g)
-            worst += skml_align16(4ull * L.n_g[g] + 8) + (adaptive ? skml_align16(17ull * L.n_g[g] / 8 + 8) : 0ull);
-        L.overflow = (worst > (unsigned long long)p.slot_capacity) || (t32 + 4 > (unsigned long long)p.tables_cap);
-        if (L.overflow) skml_set_status(p.status, SKML_CAPACITY, 0x30u);
     }
     __syncthreads();
 }
 
 // S4: every key goes to its group's staging list (stable, so the lists stay sorted);
 // grouped MinMaxSketch insert.
-__device__ void stage_scatter(const CP& p, Smem& s, long long n) {
+// `nkey`, `nbin`: key and bucket of this lane's first element (one launch for all stages).
+template <bool FUSED>
+__device__ void stage_scatter(const CP& p, Smem& s, long long n, int nkey, int nbin) {
     const int G = p.G;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Layout& L = s.lay;
     if (L.overflow) return;
-    build_group_lut(p, s);  // (also clears the per-iteration counters)
+    if (FUSED) {
+        clear_warp_counts(s);   // the group table is the count stage's
+        __syncthreads();
+    } else {
+        build_group_lut(p, s);
+    }
     const long long sub = vslice_size(n);
     const long long vb = (long long)blockIdx.x * SKML_WARPS + warp;
     long long lo = vb * sub, hi = lo + sub;
@@ -1017,8 +1102,7 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n) {
     const int zero = s.qi.zero_idx;
     unsigned int run = 0;   // lane g: staging position of the next key of group g in this slice
     if (lane < G) run = L.goff[lane] + L.base_rank[lane] + s.wbase[warp][lane];
-    int nkey = 0, nbin = 0;
-    if (lo + lane < hi) {
+    if (!FUSED && lo + lane < hi) {
         nkey = p.keys[lo + lane];
         nbin = p.bins[lo + lane];
     }
@@ -1042,7 +1126,7 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n) {
             const int col = (int)L.col[g];
             unsigned int* tab = p.tables + L.tab32_off[g];
             int pos[SKML_MAX_ROWS];
-            if (L.mixers) {
+            if (p.mixers) {
                 skml_hash_rows_mixers<3>(L.hash_ids[g], p.rows, key, (unsigned int)col, L.recip[g], pos);
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
@@ -1148,128 +1232,161 @@ __device__ __forceinline__ unsigned int sub_scan(Smem& s, unsigned int v, unsign
     return base + inc - v;
 }
 
-// Pass A: byte counts of this block's chunks -> chunk offsets inside the block's part of each group,
-// the block's byte totals per group (published for the blocks after it).
-__device__ void pack_measure(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
+// Group of a group-major chunk (or table chunk) number.
+__device__ __forceinline__ int group_of_chunk(const unsigned int* prefix, int G, unsigned int ch) {
+    int g = 0;
+    while (g + 1 < G && ch >= prefix[g + 1]) ++g;
+    return g;
+}
+
+// Byte counts of one round's four chunks (s.sub_total) -> their offsets inside the block's part of their
+// groups (s.sub_off), the block's running totals. Warp 0, one chunk per lane; the caller has a barrier before.
+__device__ __forceinline__ void round_offsets(const CP& p, Smem& s, unsigned int c0, unsigned int my_end) {
+    if (threadIdx.x >= 32) return;
+    const unsigned int q = threadIdx.x;
+    const bool mine = q < 4 && c0 + q < my_end;
     const Layout& L = s.lay;
+    int g = 0;
+    if (mine) {
+        g = group_of_chunk(L.chunk_prefix, p.G, c0 + q);
+        unsigned int off = (unsigned int)s.my_bytes[g];
+        for (unsigned int k = 0; k < q; ++k)
+            if (c0 + k >= L.chunk_prefix[g]) off += s.sub_total[k];
+        s.sub_off[q] = off;
+    }
+    __syncwarp();
+    if (mine) atomicAdd(&s.my_bytes[g], (unsigned long long)s.sub_total[q]);
+    __syncwarp();
+}
+
+// Pass A: byte counts of this block's chunks -> chunk offsets inside the block's part of each group,
+// the block's byte totals per group (published for the blocks after it). `c`, `boff` and `total` are the
+// last round's: a block with one round of chunks goes on with them and does not read its keys again.
+__device__ void pack_measure(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end, ChunkWork& c, unsigned int& boff,
+                             unsigned int& total) {
     if (threadIdx.x < SKML_MAX_GROUPS) s.my_bytes[threadIdx.x] = 0;
-    __syncthreads();
     for (unsigned int c0 = my_begin; c0 < my_end; c0 += 4) {
-        ChunkWork c;
-        load_chunk(p, L, c0 + (threadIdx.x >> 8), my_end, p.G, c);
-        unsigned int total;
-        sub_scan(s, c.wsum, total);
+        load_chunk(p, s.lay, c0 + (threadIdx.x >> 8), my_end, p.G, c);
+        boff = sub_scan(s, c.wsum, total);
         if ((threadIdx.x & 255) == 0) s.sub_total[threadIdx.x >> 8] = total;
         __syncthreads();
-        if (threadIdx.x == 0) {  // the four chunks of this round, in order
-            for (int q = 0; q < 4 && c0 + q < my_end; ++q) {
-                int g = 0;
-                while (g + 1 < p.G && c0 + q >= L.chunk_prefix[g + 1]) ++g;
-                p.chunk_off[c0 + q] = (unsigned int)s.my_bytes[g];
-                s.my_bytes[g] += s.sub_total[q];
-            }
-        }
-        __syncthreads();
+        round_offsets(p, s, c0, my_end);
+        if (my_end - my_begin > 4 && threadIdx.x < 4 && c0 + threadIdx.x < my_end) p.chunk_off[c0 + threadIdx.x] = s.sub_off[threadIdx.x];
     }
+    __syncthreads();
     if (threadIdx.x < SKML_MAX_GROUPS) p.blk_bytes[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x] = s.my_bytes[threadIdx.x];
 }
 
-// Byte totals of the blocks before this one (they own the chunks before this block's run, so the
-// sums give this block's starting offsets and the sizes of all earlier groups).
-__device__ void pack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch) {
-    if (threadIdx.x < SKML_MAX_GROUPS) s.pre_bytes[threadIdx.x] = 0;
-    __shared__ int s_ok;
-    if (threadIdx.x == 0) s_ok = 1;
-    __syncthreads();
-    if (threadIdx.x < blockIdx.x) {
-        const unsigned int b = threadIdx.x;
-        bool ok = true;
-        if (wait) {
-            const long long t0 = clock64();
-            unsigned int ns = 20;
-            while (ld_acquire_gpu(&p.blk_flag[b]) != epoch) {
-                if (clock64() - t0 > p.budget) {
-                    skml_set_status(p.status, SKML_TIMEOUT_BARRIER, 0x50u);
-                    ok = false;
-                    break;
-                }
-                __nanosleep(ns);
-                if (ns < 400) ns *= 2;
+// Bounded wait for the publications (epoch words) of blocks [0, count); false on every thread when one is missing.
+__device__ bool wait_published(const CP& p, const unsigned int* flags, unsigned int count, unsigned int epoch, unsigned int where) {
+    bool ok = true;
+    if (threadIdx.x < count) {
+        const long long t0 = clock64();
+        unsigned int ns = 0;
+        while (ld_acquire_gpu(&flags[threadIdx.x]) != epoch) {
+            if (clock64() - t0 > p.budget) {
+                skml_set_status(p.status, SKML_TIMEOUT_BARRIER, where);
+                ok = false;
+                break;
             }
-        }
-        if (ok) {
-            for (int g = 0; g < p.G; ++g) {
-                const unsigned long long v = __ldcg(&p.blk_bytes[(long long)b * SKML_MAX_GROUPS + g]);
-                if (v) atomicAdd(&s.pre_bytes[g], v);
-            }
-        } else {
-            s_ok = 0;
+            if (ns) __nanosleep(ns);
+            if (ns < 200) ns += 20;
         }
     }
-    __syncthreads();
+    return __syncthreads_and(ok) != 0;
+}
+
+// Byte totals of the blocks before this one (they own the chunks before this block's run, so the
+// sums give this block's starting offsets and the sizes of all earlier groups); a warp per group.
+__device__ void pack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch) {
+    const bool ok = !wait || wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x50u);
     Layout& L = s.lay;
-    if (threadIdx.x == 0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < p.G) {
+        unsigned long long v = 0;
+        for (unsigned int b = lane; b < blockIdx.x; b += 32) v += __ldcg(&p.blk_bytes[(long long)b * SKML_MAX_GROUPS + warp]);
+        v = warp_sum(v);
+        if (lane == 0) s.pre_bytes[warp] = v;
+    }
+    __syncthreads();
+    if (warp == 0) {
         // section starts of the groups this block can reach: all earlier groups are complete in pre_bytes
         // (plus this block's own part of the group its run starts in)
-        unsigned long long o = L.off_deltas;
-        for (int g = 0; g < p.G; ++g) {
-            L.delta_off[g] = o;
-            const unsigned long long bytes = s.pre_bytes[g] + s.my_bytes[g];
-            if (L.n_g[g]) o += skml_align16(8ull * ((bytes + 7) / 8));
-        }
-        if (!s_ok) L.overflow = 1;
+        unsigned long long size = 0, all;
+        if (lane < p.G && L.n_g[lane]) size = skml_align16(8ull * ((s.pre_bytes[lane] + s.my_bytes[lane] + 7) / 8));
+        const unsigned long long o = warp_prefix(size, all);
+        if (lane < p.G) L.delta_off[lane] = L.off_deltas + o;
+        if (lane == 0 && !ok) L.overflow = 1;
     }
     __syncthreads();
 }
 
-// Pass B: flag bytes, delta bytes and restart points of this block's chunks.
-__device__ void pack_write(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
+// Flag bytes, delta bytes and restart point of one chunk (256 threads, four adjacent keys each).
+__device__ __forceinline__ void pack_emit(const CP& p, const Smem& s, const ChunkWork& c, unsigned int boff, unsigned int total,
+                                          unsigned int off_in_block) {
     const Layout& L = s.lay;
-    if (L.overflow) return;
-    const int t = threadIdx.x & 255;
-    for (unsigned int c0 = my_begin; c0 < my_end; c0 += 4) {
-        ChunkWork c;
-        const unsigned int ch = c0 + (threadIdx.x >> 8);
-        load_chunk(p, L, ch, my_end, p.G, c);
-        unsigned int total;
-        const unsigned int boff = sub_scan(s, c.wsum, total);
-        if (c.g < 0) continue;  // (no barrier follows in this iteration)
-        const int g = c.g;
-        const unsigned int first = c.j * SKML_RESTART_INTERVAL, i0 = 4u * t;
-        const unsigned long long chunk_off = s.pre_bytes[g] + __ldcg(&p.chunk_off[ch]);
-        // flags: (w - 1) most significant bit first at stream bits 2i, 2i+1 -> one byte per four keys
-        // (a group's last chunk also writes the zero padding up to the section's 16-byte end: there the
-        // threads beyond the last key hold widths of zero)
-        const unsigned long long flag_bytes = skml_align16(8ull * ((2ull * L.n_g[g] + 63) / 64));
-        const unsigned long long fbyte = first / 4 + t;
-        if (fbyte < flag_bytes) {
-            unsigned int fb = 0;
+    const int t = threadIdx.x & 255, g = c.g;
+    const unsigned int first = c.j * SKML_RESTART_INTERVAL, i0 = 4u * t;
+    const unsigned long long chunk_off = s.pre_bytes[g] + off_in_block;
+    // flags: (w - 1) most significant bit first at stream bits 2i, 2i+1 -> one byte per four keys
+    // (a group's last chunk also writes the zero padding up to the section's 16-byte end: there the
+    // threads beyond the last key hold widths of zero)
+    const unsigned long long flag_bytes = skml_align16(8ull * ((2ull * L.n_g[g] + 63) / 64));
+    const unsigned long long fbyte = first / 4 + t;
+    if (fbyte < flag_bytes) {
+        unsigned int fb = 0;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const unsigned int fv = c.w[u] ? c.w[u] - 1u : 0u;
-                fb |= (((fv >> 1) & 1u) | ((fv & 1u) << 1)) << (2 * u);
-            }
-            p.payload[L.flag_off[g] + fbyte] = (unsigned char)fb;
+        for (int u = 0; u < 4; ++u) {
+            const unsigned int fv = c.w[u] ? c.w[u] - 1u : 0u;
+            fb |= (((fv >> 1) & 1u) | ((fv & 1u) << 1)) << (2 * u);
         }
-        if (i0 < c.cnt) {
-            unsigned char* dst = p.payload + L.delta_off[g] + chunk_off + boff;
+        p.payload[L.flag_off[g] + fbyte] = (unsigned char)fb;
+    }
+    if (i0 < c.cnt) {
+        unsigned char* dst = p.payload + L.delta_off[g] + chunk_off + boff;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                for (unsigned int j = 0; j < c.w[u]; ++j) dst[j] = skml_delta_stream_byte(c.d[u], (int)c.w[u], (int)j);
-                dst += c.w[u];
+        for (int u = 0; u < 4; ++u) {
+            for (unsigned int j = 0; j < c.w[u]; ++j) dst[j] = skml_delta_stream_byte(c.d[u], (int)c.w[u], (int)j);
+            dst += c.w[u];
+        }
+    }
+    if (t == 0 && c.j + 1 == (L.n_g[g] + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL) {
+        // the group's last chunk: clear the padding between the last delta byte and the section's end
+        const unsigned long long endb = chunk_off + total;
+        for (unsigned long long a = endb; a < skml_align16(8ull * ((endb + 7) / 8)); ++a) p.payload[L.delta_off[g] + a] = 0;
+    }
+    if (t == 0) {
+        SkmlRestart r;
+        r.prev_key = (unsigned int)c.prev0;
+        r.flag_bit_off = 2u * first;
+        r.delta_bit_off = 8ull * chunk_off;
+        *reinterpret_cast<SkmlRestart*>(p.payload + L.restart_off[g] + (unsigned long long)c.j * sizeof(SkmlRestart)) = r;
+    }
+}
+
+// Pass B: the key code of this block's chunks. `c`, `boff`, `total`: pass A's only round, where it had one.
+__device__ void pack_write(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end, bool kept, ChunkWork& c, unsigned int boff,
+                           unsigned int total) {
+    if (s.lay.overflow) return;
+    if (kept) {
+        if (c.g >= 0) pack_emit(p, s, c, boff, total, s.sub_off[threadIdx.x >> 8]);
+    } else {
+        const bool one_round = my_end - my_begin <= 4;
+        for (unsigned int c0 = my_begin; c0 < my_end; c0 += 4) {
+            const unsigned int ch = c0 + (threadIdx.x >> 8);
+            load_chunk(p, s.lay, ch, my_end, p.G, c);
+            boff = sub_scan(s, c.wsum, total);
+            if (one_round) {   // staged launches: pass A's offsets were in another launch's shared memory
+                if ((threadIdx.x & 255) == 0) s.sub_total[threadIdx.x >> 8] = total;
+                __syncthreads();
+                unsigned int off = 0;
+                if (c.g >= 0)
+                    for (unsigned int k = c0; k < ch; ++k)
+                        if (k >= s.lay.chunk_prefix[c.g]) off += s.sub_total[k - c0];
+                if (c.g >= 0) pack_emit(p, s, c, boff, total, off);
+            } else if (c.g >= 0) {
+                pack_emit(p, s, c, boff, total, __ldcg(&p.chunk_off[ch]));
             }
-        }
-        if (t == 0 && c.j + 1 == (L.n_g[g] + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL) {
-            // the group's last chunk: clear the padding between the last delta byte and the section's end
-            const unsigned long long endb = chunk_off + total;
-            for (unsigned long long a = endb; a < skml_align16(8ull * ((endb + 7) / 8)); ++a) p.payload[L.delta_off[g] + a] = 0;
-        }
-        if (t == 0) {
-            SkmlRestart r;
-            r.prev_key = (unsigned int)c.prev0;
-            r.flag_bit_off = 2u * first;
-            r.delta_bit_off = 8ull * chunk_off;
-            *reinterpret_cast<SkmlRestart*>(p.payload + L.restart_off[g] + (unsigned long long)c.j * sizeof(SkmlRestart)) = r;
         }
     }
     __syncthreads();
@@ -1446,37 +1563,15 @@ __device__ void apack_measure(const CP& p, Smem& s, unsigned int my_begin, unsig
 
 // Bit totals of the blocks before this one -> this block's starting bit offsets inside the streams.
 __device__ void apack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch) {
-    if (threadIdx.x < 2 * SKML_MAX_GROUPS) s.pre_bits[threadIdx.x] = 0;
-    __shared__ int s_ok;
-    if (threadIdx.x == 0) s_ok = 1;
-    __syncthreads();
-    if (threadIdx.x < blockIdx.x) {
-        const unsigned int b = threadIdx.x;
-        bool ok = true;
-        if (wait) {
-            const long long t0 = clock64();
-            unsigned int ns = 20;
-            while (ld_acquire_gpu(&p.blk_flag[b]) != epoch) {
-                if (clock64() - t0 > p.budget) {
-                    skml_set_status(p.status, SKML_TIMEOUT_BARRIER, 0x52u);
-                    ok = false;
-                    break;
-                }
-                __nanosleep(ns);
-                if (ns < 400) ns *= 2;
-            }
-        }
-        if (ok) {
-            for (int g = 0; g < 2 * p.G; ++g) {
-                const unsigned long long v = __ldcg(&p.blk_bits[(long long)b * 2 * SKML_MAX_GROUPS + g]);
-                if (v) atomicAdd(&s.pre_bits[g], v);
-            }
-        } else {
-            s_ok = 0;
-        }
+    const bool ok = !wait || wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x52u);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int g = warp; g < 2 * p.G; g += SKML_WARPS) {
+        unsigned long long v = 0;
+        for (unsigned int b = lane; b < blockIdx.x; b += 32) v += __ldcg(&p.blk_bits[(long long)b * 2 * SKML_MAX_GROUPS + g]);
+        v = warp_sum(v);
+        if (lane == 0) s.pre_bits[g] = v;
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && !s_ok) s.lay.overflow = 1;
+    if (threadIdx.x == 0 && !ok) s.lay.overflow = 1;
     __syncthreads();
 }
 
@@ -1552,7 +1647,7 @@ __device__ void apack_write(const CP& p, Smem& s, unsigned int my_begin, unsigne
 }
 
 // The restart points and the 16-byte units of the two bit streams that hold bits of this block only
-// -> the peers' slots. Units that hold a block border are sent by block 0 once every block is done.
+// -> the peers' slots. Units that hold a block border are sent by the last block once every block is done.
 __device__ void apush_own_chunks(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow || my_begin >= my_end) return;
@@ -1571,7 +1666,7 @@ __device__ void apush_own_chunks(const CP& p, Smem& s, unsigned int my_begin, un
     }
 }
 
-// Block 0, after every block has written its chunks: the stream units that hold a block border.
+// The last block, after every block has written its chunks: the stream units that hold a block border.
 __device__ void apush_borders(const CP& p, Smem& s) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow) return;
@@ -1845,13 +1940,12 @@ __device__ void huf_measure(const CP& p, Smem& s, unsigned int t_begin, unsigned
 
 // Table bits of the blocks before this one (the caller has waited for their publications).
 __device__ void huf_prefix(const CP& p, Smem& s) {
-    if (threadIdx.x < SKML_MAX_GROUPS) s.pre_tbits[threadIdx.x] = 0;
-    __syncthreads();
-    if (threadIdx.x < blockIdx.x) {
-        for (int g = 0; g < p.G; ++g) {
-            const unsigned long long v = __ldcg(&p.blk_tbits[(long long)threadIdx.x * SKML_MAX_GROUPS + g]);
-            if (v) atomicAdd(&s.pre_tbits[g], v);
-        }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < p.G) {
+        unsigned long long v = 0;
+        for (unsigned int b = lane; b < blockIdx.x; b += 32) v += __ldcg(&p.blk_tbits[(long long)b * SKML_MAX_GROUPS + warp]);
+        v = warp_sum(v);
+        if (lane == 0) s.pre_tbits[warp] = v;
     }
     __syncthreads();
 }
@@ -1989,35 +2083,39 @@ __device__ void huf_push_borders(const CP& p, Smem& s) {
     }
 }
 
-__device__ __forceinline__ void chunk_run(const Layout& L, int G, unsigned int& my_begin, unsigned int& my_end) {
+// Contiguous run of chunks of this block, a multiple of four (the chunks of one round) per block, and how
+// many blocks have one.
+__device__ __forceinline__ unsigned int chunk_run(const Layout& L, int G, unsigned int& my_begin, unsigned int& my_end) {
     const unsigned int total = L.chunk_prefix[G];
     unsigned int per = (total + gridDim.x - 1) / gridDim.x;
-    per = (per + 3u) & ~3u;  // four chunks per round
+    per = (per + 3u) & ~3u;
     my_begin = min(total, per * blockIdx.x);
     my_end = min(total, my_begin + per);
+    return per ? (total + per - 1) / per : 0u;
 }
 
 // S6 prelude: every group's delta bytes from all blocks' counts -> delta section offsets, total size.
-__device__ void layout_finish(const CP& p, Smem& s) {
+__device__ void layout_finish(const CP& p, Smem& s, unsigned int nactive) {
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < p.G) {
         unsigned long long v = 0;
-        for (int b = lane; b < (int)gridDim.x; b += 32) v += __ldcg(&p.blk_bytes[(long long)b * SKML_MAX_GROUPS + warp]);
+        for (unsigned int b = lane; b < nactive; b += 32) v += __ldcg(&p.blk_bytes[(long long)b * SKML_MAX_GROUPS + warp]);
         v = warp_sum(v);
         if (lane == 0) L.bytes_g[warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long o = L.off_deltas;
-        for (int g = 0; g < p.G; ++g) {
-            L.delta_off[g] = o;
-            if (L.n_g[g]) o += skml_align16(8ull * ((L.bytes_g[g] + 7) / 8));
-        }
-        L.total_bytes = o;
-        if (o > (unsigned long long)p.slot_capacity) {
-            L.overflow = 1;
-            skml_set_status(p.status, SKML_CAPACITY, 0x36u);
+    if (warp == 0) {
+        unsigned long long size = 0, all;
+        if (lane < p.G && L.n_g[lane]) size = skml_align16(8ull * ((L.bytes_g[lane] + 7) / 8));
+        const unsigned long long o = warp_prefix(size, all);
+        if (lane < p.G) L.delta_off[lane] = L.off_deltas + o;
+        if (lane == 0) {
+            L.total_bytes = L.off_deltas + all;
+            if (L.total_bytes > (unsigned long long)p.slot_capacity) {
+                L.overflow = 1;
+                skml_set_status(p.status, SKML_CAPACITY, 0x36u);
+            }
         }
     }
     __syncthreads();
@@ -2026,7 +2124,7 @@ __device__ void layout_finish(const CP& p, Smem& s) {
 // Fill helpers run inside S1 (they do not depend on the summary).
 __device__ void stage_prepare(const CP& p, long long n) {
     // working sketch cells start "empty"
-    long long cells = (long long)p.rows * ((long long)(p.col_ratio * (double)n) + 2 + p.G);
+    long long cells = (long long)p.rows * ((long long)(p.col_ratio * (double)n) + 2 + p.G) + 4 * p.G;
     if (cells > p.tables_cap - 4) cells = p.tables_cap - 4;
     const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
@@ -2044,9 +2142,8 @@ __device__ void stage_prepare(const CP& p, long long n) {
     }
 }
 
-// Header, bucket values and group table (block 0), stored locally and into every peer's slot.
+// Header, bucket values and group table, stored locally and into every peer's slot, by the block that calls it.
 __device__ void write_header(const CP& p, Smem& s, long long n, int kind) {
-    if (blockIdx.x != 0) return;
     const Layout& L = s.lay;
     const QInfo& q = s.qi;
     const bool sparse = kind == SKML_KIND_SPARSE && !L.overflow;
@@ -2055,75 +2152,77 @@ __device__ void write_header(const CP& p, Smem& s, long long n, int kind) {
         const int padded = (int)(skml_align16(4ull * p.q) / 4);
         for (int b = threadIdx.x; b < padded; b += blockDim.x) bv[b] = b < q.bin_num ? bucket_value(s, b) : 0.f;
     }
-    if (sparse) {
-        if (threadIdx.x < p.G) {
-            const int g = threadIdx.x;
-            SkmlGroupEntry e;
-            e.n = L.n_g[g];
-            e.col_num = L.col[g];
-            for (int i = 0; i < 8; ++i) e.hash_ids[i] = L.n_g[g] ? L.hash_ids[g][i] : 0;
-            e.table_off = L.n_g[g] ? L.table_off[g] : 0;
-            e.flag_off = L.n_g[g] ? L.flag_off[g] : 0;
-            e.n_flag_words = (unsigned int)((2ull * L.n_g[g] + 63) / 64);
-            e.num_intervals = 4;
-            e.delta_off = L.n_g[g] ? L.delta_off[g] : 0;
-            e.n_delta_words = (unsigned int)((L.bytes_g[g] + 7) / 8);
-            e.flag_kind = 0;
-            if (p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE) {
-                e.n_flag_words = (unsigned int)((L.flag_bits[g] + 63) / 64);
-                e.n_delta_words = (unsigned int)((L.delta_bits[g] + 63) / 64);
-                e.num_intervals = L.n_g[g] ? L.num_iv[g] : 0;
-                e.flag_kind = L.n_g[g] ? L.flag_kind[g] : 0;
-            }
-            e.restart_off = L.n_g[g] ? L.restart_off[g] : 0;
-            *reinterpret_cast<SkmlGroupEntry*>(p.payload + L.off_gt + (unsigned long long)g * sizeof(SkmlGroupEntry)) = e;
+    if (sparse && threadIdx.x >= 32 && threadIdx.x < 32 + p.G) {
+        const int g = threadIdx.x - 32;
+        const bool any = L.n_g[g] != 0;
+        SkmlGroupEntry e;
+        e.n = L.n_g[g];
+        e.col_num = L.col[g];
+        for (int i = 0; i < 8; ++i) e.hash_ids[i] = any ? p.hash_ids[g][i] : 0;
+        e.table_off = any ? L.table_off[g] : 0;
+        e.flag_off = any ? L.flag_off[g] : 0;
+        e.n_flag_words = (unsigned int)((2ull * L.n_g[g] + 63) / 64);
+        e.num_intervals = 4;
+        e.delta_off = any ? L.delta_off[g] : 0;
+        e.n_delta_words = (unsigned int)((L.bytes_g[g] + 7) / 8);
+        e.flag_kind = 0;
+        if (p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE) {
+            e.n_flag_words = (unsigned int)((L.flag_bits[g] + 63) / 64);
+            e.n_delta_words = (unsigned int)((L.delta_bits[g] + 63) / 64);
+            e.num_intervals = any ? L.num_iv[g] : 0;
+            e.flag_kind = any ? L.flag_kind[g] : 0;
         }
+        e.restart_off = any ? L.restart_off[g] : 0;
+        *reinterpret_cast<SkmlGroupEntry*>(p.payload + L.off_gt + (unsigned long long)g * sizeof(SkmlGroupEntry)) = e;
     }
-    if (threadIdx.x == 0) {
-        SkmlHeader h;
-        unsigned char* hb = reinterpret_cast<unsigned char*>(&h);
-        for (int i = 0; i < SKML_HEADER_BYTES; ++i) hb[i] = 0;
-        h.magic = SKML_MAGIC;
-        h.version = SKML_VERSION;
-        h.kind = (kind == SKML_KIND_SPARSE && L.overflow) ? SKML_KIND_EMPTY : (unsigned int)kind;
-        h.dtype = SKML_F32;
-        h.step = p.step;
-        h.rank = p.rank;
-        h.world = p.world;
-        h.dim = (unsigned long long)p.dim;
-        h.seed = p.seed;
-        if (p.loss_partials)
-            for (int i = 0; i < 4; ++i) h.loss_partials[i] = p.loss_partials[i];
-        h.total_bytes = SKML_HEADER_BYTES;
-        if (h.kind != SKML_KIND_EMPTY) {
-            h.nnz = (unsigned long long)n;
-            h.bin_num = (unsigned int)q.bin_num;
-            h.zero_idx = (unsigned int)q.zero_idx;
-            h.cell_bits = (kind == SKML_KIND_SPARSE && p.huffman) ? 0u : (unsigned int)q.cell_bits;
-            h.min_value = (double)q.minv;
-            h.max_value = (double)q.maxv;
-            h.off_bucket_values = SKML_HEADER_BYTES;
+    if (threadIdx.x < 32) {   // the header is put together in shared memory by one warp
+        const int lane = threadIdx.x;
+        SkmlHeader& h = s.hdr;
+        for (int i = lane; i < SKML_HEADER_BYTES / 4; i += 32) reinterpret_cast<unsigned int*>(&h)[i] = 0u;
+        __syncwarp();
+        if (lane < 4 && p.loss_partials) h.loss_partials[lane] = p.loss_partials[lane];
+        if (lane == 0) {
+            h.magic = SKML_MAGIC;
+            h.version = SKML_VERSION;
+            const unsigned int hk = (kind == SKML_KIND_SPARSE && L.overflow) ? (unsigned int)SKML_KIND_EMPTY : (unsigned int)kind;
+            h.kind = hk;
+            h.dtype = SKML_F32;
+            h.step = p.step;
+            h.rank = p.rank;
+            h.world = p.world;
+            h.dim = (unsigned long long)p.dim;
+            h.seed = p.seed;
+            h.total_bytes = SKML_HEADER_BYTES;
+            if (hk != SKML_KIND_EMPTY) {
+                h.nnz = (unsigned long long)n;
+                h.bin_num = (unsigned int)q.bin_num;
+                h.zero_idx = (unsigned int)q.zero_idx;
+                h.cell_bits = (kind == SKML_KIND_SPARSE && p.huffman) ? 0u : (unsigned int)q.cell_bits;
+                h.min_value = (double)q.minv;
+                h.max_value = (double)q.maxv;
+                h.off_bucket_values = SKML_HEADER_BYTES;
+            }
+            if (hk == SKML_KIND_SPARSE) {
+                h.group_num = (unsigned int)p.G;
+                h.row_num = (unsigned int)p.rows;
+                h.col_ratio = p.col_ratio;
+                h.key_encoder = (unsigned int)p.key_encoder;
+                h.restart_interval = SKML_RESTART_INTERVAL;
+                h.off_group_table = L.off_gt;
+                h.off_key_flags = L.off_flags;
+                h.off_restart = L.off_restart;
+                h.off_tables = L.off_tables;
+                h.off_key_deltas = L.off_deltas;
+                h.total_bytes = L.total_bytes;
+            } else if (hk == SKML_KIND_DENSE) {
+                h.off_dense_codes = SKML_HEADER_BYTES + skml_align16(4ull * p.q);
+                h.total_bytes = skml_align16(h.off_dense_codes + (unsigned long long)p.dim * (q.cell_bits / 8));
+            }
         }
-        if (h.kind == SKML_KIND_SPARSE) {
-            h.group_num = (unsigned int)p.G;
-            h.row_num = (unsigned int)p.rows;
-            h.col_ratio = p.col_ratio;
-            h.key_encoder = (unsigned int)p.key_encoder;
-            h.restart_interval = SKML_RESTART_INTERVAL;
-            h.off_group_table = L.off_gt;
-            h.off_key_flags = L.off_flags;
-            h.off_restart = L.off_restart;
-            h.off_tables = L.off_tables;
-            h.off_key_deltas = L.off_deltas;
-            h.total_bytes = L.total_bytes;
-        } else if (h.kind == SKML_KIND_DENSE) {
-            h.off_dense_codes = SKML_HEADER_BYTES + skml_align16(4ull * p.q);
-            h.total_bytes = skml_align16(h.off_dense_codes + (unsigned long long)p.dim * (q.cell_bits / 8));
-        }
-        h.header_checksum = skml_header_checksum(&h);
-        const uint4* src = reinterpret_cast<const uint4*>(&h);
-        uint4* dst = reinterpret_cast<uint4*>(p.payload);
-        for (int i = 0; i < SKML_HEADER_BYTES / 16; ++i) dst[i] = src[i];
+        __syncwarp();
+        if (lane == 0) h.header_checksum = skml_header_checksum(&h);
+        __syncwarp();
+        if (lane < SKML_HEADER_BYTES / 16) reinterpret_cast<uint4*>(p.payload)[lane] = reinterpret_cast<const uint4*>(&h)[lane];
     }
     // this block wrote the head of the payload (header, bucket values, group table): it also stores it
     // into the peers' slots, so that no other block has to wait for it
@@ -2156,17 +2255,23 @@ __device__ void copy_range_to_peers(const CP& p, unsigned long long lo, unsigned
     }
 }
 
+// The block barrier orders every thread's stores before thread 0's fence, and the fence before the count, so one
+// thread fences for the block (1024 threads fencing at system scope took 7 us); peers' memory needs system scope.
 __device__ void finish_publish(const CP& p) {
     __shared__ int s_last;
-    __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {
+        if (p.world > 1) __threadfence_system();
+        else if (p.peer_flag[0]) __threadfence();   // (alone and without a flag the end of the kernel orders the readers)
         unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
         s_last = prev == gridDim.x - 1;
-        if (s_last) {
+        if (s_last) {       // nobody is in a grid barrier any more
+            p.ctrl[0] = 0;
+            p.ctrl[1] += 1;
             p.ctrl[2] = 0;
             p.ctrl[4] = 0;  // the summary's min / max words go back to "nothing yet"
             p.ctrl[5] = 0;
+            __threadfence();
         }
     }
     __syncthreads();
@@ -2183,34 +2288,30 @@ __device__ void narrow_tables(const CP& p, Smem& s) {
     const Layout& L = s.lay;
     if (L.overflow) return;
     const int G = p.G, cb = s.qi.cell_bits, per = 16 / (cb / 8);  // cells per 16-byte unit
-    if (threadIdx.x == 0) {
-        unsigned long long u = 0;
-        for (int g = 0; g < G; ++g) {
-            s.unit_prefix[g] = u;
-            u += skml_align16((unsigned long long)p.rows * L.col[g] * (cb / 8)) / 16;
-        }
-        s.unit_prefix[G] = u;
-    }
-    __syncthreads();
     const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long units = (long long)s.unit_prefix[G];
+    const long long units = (long long)L.unit_prefix[G];
     const unsigned int zero = (unsigned int)s.qi.zero_idx;
+    auto code_of = [&](unsigned int cell) { return cell == SKML_EMPTY_CELL ? zero : cell; };
     for (long long u = gid; u < units; u += gsz) {
         int g = 0;
-        while (g + 1 < G && (unsigned long long)u >= s.unit_prefix[g + 1]) ++g;
-        const long long j = u - (long long)s.unit_prefix[g];
-        const long long cells = (long long)p.rows * L.col[g];
-        const unsigned int* tab = p.tables + L.tab32_off[g];
+        while (g + 1 < G && (unsigned long long)u >= L.unit_prefix[g + 1]) ++g;
+        const long long j = u - (long long)L.unit_prefix[g];
+        const long long left = (long long)p.rows * L.col[g] - j * per;   // cells from this unit on
+        // a group's working table starts at a multiple of four cells, so the unit is `per / 4` 16-byte loads
+        const uint4* src = reinterpret_cast<const uint4*>(p.tables + L.tab32_off[g]) + j * (per / 4);
         unsigned int words[4] = {0, 0, 0, 0};
-        for (int t = 0; t < per; ++t) {
-            long long c = j * per + t;
-            unsigned int code = 0;
-            if (c < cells) {
-                unsigned int cell = __ldcg(tab + c);
-                code = cell == SKML_EMPTY_CELL ? zero : (cell & 0xFFFFu);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (4 * t >= per) break;
+            uint4 c = make_uint4(0, 0, 0, 0);
+            if (4 * t < left) c = ld_cg_v4(src + t);
+            const unsigned int x0 = 4 * t < left ? code_of(c.x) & 0xFFFFu : 0u, x1 = 4 * t + 1 < left ? code_of(c.y) & 0xFFFFu : 0u;
+            const unsigned int x2 = 4 * t + 2 < left ? code_of(c.z) & 0xFFFFu : 0u, x3 = 4 * t + 3 < left ? code_of(c.w) & 0xFFFFu : 0u;
+            if (cb == 8) words[t] = (x0 & 0xFFu) | ((x1 & 0xFFu) << 8) | ((x2 & 0xFFu) << 16) | (x3 << 24);
+            else if (t < 2) {
+                words[2 * t] = x0 | (x1 << 16);
+                words[2 * t + 1] = x2 | (x3 << 16);
             }
-            if (cb == 8) words[t >> 2] |= (code & 0xFFu) << (8 * (t & 3));
-            else words[t >> 1] |= (code & 0xFFFFu) << (16 * (t & 1));
         }
         uint4 v = make_uint4(words[0], words[1], words[2], words[3]);
         const unsigned long long off = L.table_off[g] + 16ull * j;
@@ -2264,34 +2365,12 @@ __device__ void push_own_chunks(const CP& p, Smem& s, unsigned int my_begin, uns
     }
 }
 
-// Block 0 needs every block's byte counts for the header: bounded wait for their publications.
-__device__ bool wait_all_published(const CP& p, const unsigned int* flags, unsigned int epoch) {
-    __shared__ int s_ok;
-    if (threadIdx.x == 0) s_ok = 1;
-    __syncthreads();
-    if (threadIdx.x < gridDim.x) {
-        const long long t0 = clock64();
-        unsigned int ns = 20;
-        while (ld_acquire_gpu(&flags[threadIdx.x]) != epoch) {
-            if (clock64() - t0 > p.budget) {
-                skml_set_status(p.status, SKML_TIMEOUT_BARRIER, 0x51u);
-                s_ok = 0;
-                break;
-            }
-            __nanosleep(ns);
-            if (ns < 400) ns *= 2;
-        }
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
 #define STAGE_BARRIER(stage_id)                                                           \
     if (FUSED) {                                                                          \
-        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, stage_id)) return; \
+        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, stage_id, passed)) return; \
         stage_stamp(p.ctrl, stage_id);                                                    \
     }
 
@@ -2302,6 +2381,9 @@ template <bool FUSED, bool ADAPTIVE, bool HUFFMAN>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, int stage) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
+    unsigned int passed = 0;   // arrivals of the grid barriers so far
+    // names this launch's publications: one more than the launch before it (see finish_publish)
+    const unsigned int epoch = FUSED ? ld_relaxed_gpu(&p.ctrl[1]) + 1u : 0u;
     const long long kind = p.meta[1];
     if (kind == SKML_KIND_DENSE) return;  // handled by the dense kernel
     long long n = p.meta[0];
@@ -2316,7 +2398,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
                 s.qi.bin_num = 0;
             }
             __syncthreads();
-            write_header(p, s, 0, SKML_KIND_EMPTY);   // block 0 stores it locally and into the peers' slots
+            if (blockIdx.x == 0) write_header(p, s, 0, SKML_KIND_EMPTY);   // locally and into the peers' slots
             finish_publish(p);
         }
         return;
@@ -2325,6 +2407,14 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     if (FUSED) stage_stamp(p.ctrl, 0);
     // sample form of the split search: S1 ends with the splits in every block, S2 and two grid barriers drop out
     const bool sample = p.sample_splits != 0 && !given;
+    // this lane's first element: its value is wanted after S1, its key after S3, both loads start here
+    const long long first_i = vslice_size(n) * ((long long)blockIdx.x * SKML_WARPS + (threadIdx.x >> 5)) + (threadIdx.x & 31);
+    float first_val = 0.f;
+    int first_key = 0, first_bin = 0;
+    if (first_i < n && (FUSED || stage == 3)) {
+        first_val = p.vals[first_i];
+        if (FUSED) first_key = p.keys[first_i];
+    }
     if (FUSED || stage == 1) {
         stage_prepare(p, n);
         stage_stamp(p.ctrl, 8);
@@ -2343,33 +2433,33 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         STAGE_BARRIER(2)
     }
     if (FUSED || stage == 3) {
-        load_quantizer(p, s, !sample);
+        load_quantizer(p, s, FUSED && sample, !sample);
         if (s.qi.bin_num > SKML_GPU_MAX_BINS) {
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x32u);
             return;
         }
-        stage_count(p, s, n, sample);
+        first_bin = stage_count<FUSED>(p, s, n, sample, first_val);
     }
     STAGE_BARRIER(3)
     if (FUSED || stage == 4) {
         if (!FUSED) load_quantizer(p, s);
-        else if (sample) refresh_minmax(p, s);
-        layout_from_counts(p, s);
-        stage_scatter(p, s, n);
+        layout_from_counts<FUSED>(p, s, FUSED && sample);
+        stage_scatter<FUSED>(p, s, n, first_key, first_bin);
     }
     STAGE_BARRIER(4)
     // S5: key code and publication. In one cooperative launch a block waits only for the counts of the
-    // blocks before it (they are resident, and never wait for a later block), and block 0 for all of them
-    // before it writes the header; staged launches split the stage at those points. The delta_adaptive
+    // blocks before it (they are resident, and never wait for a later block), and the last block for all of
+    // them before it writes the header (it has the fewest chunks, none where there are fewer than blocks);
+    // staged launches split the stage at those points. The delta_adaptive
     // code needs the groups' complete histograms of delta widths first: one more grid barrier.
-    unsigned int my_begin = 0, my_end = 0, t_begin = 0, t_end = 0;
+    unsigned int my_begin = 0, my_end = 0, t_begin = 0, t_end = 0, nactive = 0;
     constexpr bool adaptive = ADAPTIVE, huffman = HUFFMAN;
     if (FUSED || stage >= 5) {
         if (!FUSED) {
             load_quantizer(p, s);
-            layout_from_counts(p, s);
+            layout_from_counts<FUSED>(p, s, false);
         }
-        chunk_run(s.lay, p.G, my_begin, my_end);
+        nactive = chunk_run(s.lay, p.G, my_begin, my_end);
         if (huffman) {
             huf_ranges(p, s);
             tchunk_run(s.lay, p.G, t_begin, t_end);
@@ -2378,33 +2468,35 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     if (FUSED || stage == 5) {
         if (huffman) {
             if (!s.lay.overflow) huf_histogram(p, s, t_begin, t_end);
-        } else {
+        } else if (adaptive) {
             narrow_tables(p, s);   // the tables are complete since S4
         }
         if (adaptive && !s.lay.overflow) apack_histogram(p, s, my_begin, my_end);
     }
     if (FUSED && (adaptive || huffman)) {
-        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x15u)) return;
+        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x15u, passed)) return;
     }
     if (FUSED || stage >= 6) {
         // code tables and the layout behind the tables (every block; staged launches repeat it per stage)
         if (huffman && (FUSED || stage >= 6)) huf_build(p, s);
         if (adaptive) apack_choose(p, s);
     }
+    ChunkWork cw;
+    unsigned int boff = 0, btotal = 0;
     if (FUSED || stage == 6) {
         if (adaptive) apack_measure(p, s, my_begin, my_end);
-        else pack_measure(p, s, my_begin, my_end);
+        else if (my_begin < my_end) pack_measure(p, s, my_begin, my_end, cw, boff, btotal);
         if (huffman) huf_measure(p, s, t_begin, t_end);
     }
-    unsigned int epoch = 0;
     if (FUSED) {
-        // every block reads the same barrier generation here: it names this launch's publications
-        epoch = ld_acquire_gpu(&p.ctrl[1]) + 0x40000000u;
-        __threadfence();
         __syncthreads();
-        if (threadIdx.x == 0) st_release_gpu(&p.blk_flag[blockIdx.x], epoch);
+        if (threadIdx.x == 0) {
+            __threadfence();
+            st_relaxed_gpu(&p.blk_flag[blockIdx.x], epoch);
+        }
     }
-    const bool borders = adaptive || huffman;  // stream words shared by two blocks are sent by block 0 at the end
+    if (!huffman && !adaptive && (FUSED || stage == 6)) narrow_tables(p, s);   // while the publications travel
+    const bool borders = adaptive || huffman;  // stream words shared by two blocks are sent by the last block at the end
     if (FUSED || stage == 7) {
         if (!FUSED) {  // the block's own counts again (shared memory does not survive a launch)
             if (threadIdx.x < SKML_MAX_GROUPS) {
@@ -2418,10 +2510,14 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             apack_prefix(p, s, FUSED, epoch);
             apack_write(p, s, my_begin, my_end);
             apush_own_chunks(p, s, my_begin, my_end);
-        } else {
+        } else if (my_begin < my_end) {
             pack_prefix(p, s, FUSED, epoch);
-            pack_write(p, s, my_begin, my_end);
+            pack_write(p, s, my_begin, my_end, FUSED && my_end - my_begin <= 4, cw, boff, btotal);
             push_own_chunks(p, s, my_begin, my_end);
+        } else if (FUSED && huffman) {
+            // no keys here, but huf_prefix below reads the same publications
+            if (!wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x53u) && threadIdx.x == 0) s.lay.overflow = 1;
+            __syncthreads();
         }
         if (huffman) {
             huf_prefix(p, s);   // (the key prefix above has waited for the blocks before this one)
@@ -2429,17 +2525,19 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             huf_push_own(p, s, t_begin, t_end);
         }
         if (FUSED && borders) {
-            __threadfence();
             __syncthreads();
-            if (threadIdx.x == 0) st_release_gpu(&p.blk_done[blockIdx.x], epoch);
+            if (threadIdx.x == 0) {
+                __threadfence();
+                st_relaxed_gpu(&p.blk_done[blockIdx.x], epoch);
+            }
         }
         if (FUSED) stage_stamp(p.ctrl, 5);
     }
     if (FUSED || stage == 8) {
-        if (blockIdx.x == 0) {
-            if (FUSED && !wait_all_published(p, borders ? p.blk_done : p.blk_flag, epoch)) return;
+        if (blockIdx.x == gridDim.x - 1) {
+            if (FUSED && !wait_published(p, borders ? p.blk_done : p.blk_flag, borders ? gridDim.x : nactive, epoch, 0x51u)) return;
             if (adaptive) apush_borders(p, s);
-            else layout_finish(p, s);
+            else layout_finish(p, s, nactive);
             if (huffman) huf_push_borders(p, s);
             write_header(p, s, n, SKML_KIND_SPARSE);
         }
@@ -2454,6 +2552,7 @@ template <bool FUSED>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int stage) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
+    unsigned int passed = 0;   // arrivals of the grid barriers so far
     if (p.meta[1] != SKML_KIND_DENSE) return;
     const long long n = p.dim;
     const bool given = p.given_splits != nullptr;
@@ -2470,7 +2569,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int
         STAGE_BARRIER(2)
     }
     if (FUSED || stage == 3) {
-        load_quantizer(p, s, !sample);
+        load_quantizer(p, s, FUSED && sample, !sample);
         if (s.qi.bin_num > SKML_GPU_MAX_BINS) {
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x33u);
             return;
@@ -2484,7 +2583,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_CAPACITY, 0x34u);
             return;
         }
-        if (!sample) write_header(p, s, n, SKML_KIND_DENSE);
+        if (!sample && blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
         unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
         const long long units = (n + per - 1) / per;
         const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2524,12 +2623,13 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int
     if (FUSED || stage == 4) {
         if (sample) {
             if (!FUSED) load_quantizer(p, s);   // staged launches: the extremes are complete now
-            else refresh_minmax(p, s);
+            else if (threadIdx.x == 0) refresh_minmax(p, s);
+            __syncthreads();
             if (!FUSED) {
                 if (threadIdx.x == 0) s.lay.overflow = 0;
                 __syncthreads();
             }
-            write_header(p, s, n, SKML_KIND_DENSE);
+            if (blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
         }
         finish_publish(p);
     }
@@ -2611,6 +2711,13 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     p.n_given = (int)a->n_given;
     p.given_min = (float)a->given_min;
     p.given_max = (float)a->given_max;
+    // draws that depend on the launch's parameters only are made here, once, instead of by every block
+    p.sample_rand = skml_rand(p.seed, p.step, p.rank, 0x7300u);
+    p.mixers = p.rows <= 3;
+    for (int g = 0; g < p.G; ++g) {
+        skml_pick_hashes(p.seed, p.step, p.rank, (unsigned int)g, p.rows, p.hash_ids[g]);
+        for (int r = 0; r < p.rows && p.mixers; ++r) p.mixers = p.hash_ids[g][r] < 3;
+    }
     return 0;
 }
 

@@ -655,6 +655,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DecSmem& s = *reinterpret_cast<DecSmem*>(smem_raw);
     float dsq = 0.f;  // this thread's share of the change of ||w||^2
+    unsigned int passed = 0;   // arrivals of the grid barriers so far
     if (FUSED && blockIdx.x == 0 && threadIdx.x == 0) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -664,7 +665,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
     if (s.nhuf) {  // tables that arrived Huffman-coded become plain bucket codes first
         if (FUSED || stage == 0) expand_tables(p, s);
         if (FUSED) {
-            if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x2Eu)) return;
+            if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x2Eu, passed)) return;
         }
     }
     if (!FUSED && stage == 0) return;
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
             // Phase 1 (un-fused: stage 1): every payload's keys and values, no ordering needed.
             if (FUSED || stage == 1) decode_accumulate(p, s, 0, s.total_chunks, dsq);
             if (FUSED) {
-                if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x2Fu)) return;
+                if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x2Fu, passed)) return;
                 if (blockIdx.x == 0 && threadIdx.x == 0) {
                     unsigned long long t;
                     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -696,7 +697,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
                     if (s.any_dense) decode_accumulate_dense(p, s, r, r + 1, dsq);
                 }
                 if (FUSED && r + 1 < p.world) {
-                    if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r)) return;
+                    if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r, passed)) return;
                 }
             }
         } else {
@@ -707,7 +708,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
                     if (s.any_dense) decode_accumulate_dense(p, s, r, r + 1, dsq);
                 }
                 if (FUSED && r + 1 < p.world) {
-                    if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r)) return;
+                    if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r, passed)) return;
                 }
             }
         }
@@ -731,6 +732,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
                 const unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
                 if (prev == gridDim.x - 1) {
                     p.ctrl[2] = 0;
+                    p.ctrl[0] = 0;   // nobody is in a grid barrier any more
                     unsigned long long t;
                     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
                     reinterpret_cast<unsigned long long*>(p.ctrl)[16 + (int)(p.step & 1)] = t;
@@ -744,7 +746,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
         if (s.any_dense) decode_accumulate_dense(p, s, 0, p.world, dsq);
     }
     if (FUSED) {
-        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x21u)) return;
+        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x21u, passed)) return;
     }
     if (FUSED && blockIdx.x == 0 && threadIdx.x == 0) {
         unsigned long long t;
@@ -758,6 +760,13 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
         reinterpret_cast<unsigned long long*>(p.ctrl)[11 + 4 * (int)(p.step & 1)] = t;
     }
     finish_norm(p, dsq);
+    if (FUSED) {
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(&p.ctrl[2], 1u) == gridDim.x - 1) {
+            p.ctrl[2] = 0;
+            p.ctrl[0] = 0;
+        }
+    }
 }
 
 extern "C" long long skml_decode_workspace_bytes(long long world, long long group_num) {

@@ -89,49 +89,64 @@ __device__ __forceinline__ void skml_hash_rows_mixers(const unsigned char* ids, 
 }
 
 // ---------------------------------------------------------------------------
-// Grid barrier for cooperative launches. bar[0] = arrival count, bar[1] = generation.
-// Returns false (on every thread of the block) when the wait budget ran out.
+// Grid barrier for cooperative launches. *bar counts arrivals: zero when the kernel starts, nblocks more
+// per barrier, and put back to zero by the kernel's last block. `passed` is the caller's count of arrivals
+// of the barriers before this one. A block adds itself and polls until everyone has: one trip to L2 and
+// one poll, no second word for the last block to release. The status word is polled beside the count, in
+// the same flight: a block that reported an error may have left the kernel and will never arrive, and
+// nobody goes on after an error.
+// Returns false (on every thread of the block) when the wait budget ran out or an error was reported; the
+// host then clears the workspace.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool skml_grid_barrier(unsigned int* bar, unsigned int nblocks, unsigned int* status,
-                                                  long long budget, unsigned int stage) {
+__device__ __forceinline__ unsigned int ld_relaxed_gpu(const unsigned int* p) {
+    unsigned int v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed_gpu(unsigned int* p, unsigned int v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_add_gpu(unsigned int* p, unsigned int v) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+static __device__ __noinline__ bool skml_grid_barrier_at(unsigned int* bar, unsigned int nblocks, unsigned int* status,
+                                                         long long budget, unsigned int stage, unsigned int target) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
+        unsigned int st;
         if (nblocks > 1) {
             __threadfence();
-            unsigned int gen = ld_acquire_gpu(&bar[1]);
-            unsigned int prev = atomicAdd(&bar[0], 1u);
-            if (prev == nblocks - 1) {
-                bar[0] = 0;
-                __threadfence();
-                st_release_gpu(&bar[1], gen + 1);
-            } else {
-                long long t0 = clock64();
-                unsigned int ns = 20, polls = 0;
-                while (ld_acquire_gpu(&bar[1]) == gen) {
-                    if (clock64() - t0 > budget) {
-                        ok = 0;
-                        skml_set_status(status, SKML_TIMEOUT_BARRIER, stage);
-                        break;
-                    }
-                    // a block that reported an error has left the kernel and will never arrive
-                    if ((++polls & 63u) == 0 && (ld_acquire_gpu(status) & 0xFFu) != SKML_OK) {
-                        ok = 0;
-                        break;
-                    }
-                    __nanosleep(ns);
-                    if (ns < 400) ns *= 2;
+            red_add_gpu(bar, 1u);
+            const long long t0 = clock64();
+            unsigned int ns = 0;
+            while (true) {
+                const unsigned int now = ld_relaxed_gpu(bar);
+                st = ld_relaxed_gpu(status);
+                if (now >= target || (st & 0xFFu) != SKML_OK) break;
+                if (clock64() - t0 > budget) {
+                    skml_set_status(status, SKML_TIMEOUT_BARRIER, stage);
+                    ok = 0;
+                    break;
                 }
+                if (ns) __nanosleep(ns);
+                if (ns < 200) ns += 10;
             }
             __threadfence();
+        } else {
+            st = ld_relaxed_gpu(status);
         }
-        // another block may already have failed: leave as well so nobody waits alone
-        if (ok && (ld_acquire_gpu(status) & 0xFFu) != SKML_OK) ok = 0;
-        s_ok = ok;
+        s_ok = ok && (st & 0xFFu) == SKML_OK;
     }
     __syncthreads();
     return s_ok != 0;
+}
+__device__ __forceinline__ bool skml_grid_barrier(unsigned int* bar, unsigned int nblocks, unsigned int* status,
+                                                  long long budget, unsigned int stage, unsigned int& passed) {
+    passed += nblocks;
+    return skml_grid_barrier_at(bar, nblocks, status, budget, stage, passed);
 }
 
 // Waits until *flag == want (system scope). Thread 0 of the block polls.
@@ -257,77 +272,71 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// In-place bitonic sort of N (power of two) unsigned keys in shared memory by the
-// whole block.
-// ---------------------------------------------------------------------------
-template <int N>
-__device__ __forceinline__ void block_bitonic_sort(unsigned int* s) {
-    for (int k = 2; k <= N; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int t = threadIdx.x; t < N / 2; t += blockDim.x) {
-                int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));  // index with bit j cleared
-                int p = i | j;
-                bool up = (i & k) == 0;
-                unsigned int a = s[i], b = s[p];
-                if ((a > b) == up) {
-                    s[i] = b;
-                    s[p] = a;
-                }
-            }
-            __syncthreads();
+// One merge round of sorted runs of LEN keys: an element's place in the merged pair of runs is its place in
+// its own run plus the number of the other run's keys before it (a binary search; the left run wins ties).
+// A warp's 64 elements belong to one run, so its 32 searches run side by side on neighbouring keys.
+template <int LEN>
+__device__ __forceinline__ void merge_round(const unsigned int* __restrict__ src, unsigned int* __restrict__ dst) {
+    const int lane = threadIdx.x & 31, i0 = (threadIdx.x >> 5) * 64 + lane;
+    const int run = i0 / LEN;
+    const unsigned int* other = src + (run ^ 1) * LEN;
+    const unsigned int x0 = src[i0], x1 = src[i0 + 32];
+    int p0 = 0, p1 = 0;
+    if (run & 1) {   // uniform over the warp
+#pragma unroll
+        for (int step = LEN / 2; step > 0; step >>= 1) {
+            if (other[p0 + step - 1] <= x0) p0 += step;
+            if (other[p1 + step - 1] <= x1) p1 += step;
         }
+        p0 += other[p0] <= x0;
+        p1 += other[p1] <= x1;
+    } else {
+#pragma unroll
+        for (int step = LEN / 2; step > 0; step >>= 1) {
+            if (other[p0 + step - 1] < x0) p0 += step;
+            if (other[p1 + step - 1] < x1) p1 += step;
+        }
+        p0 += other[p0] < x0;
+        p1 += other[p1] < x1;
     }
+    const int base = (run & ~1) * LEN + (i0 & (LEN - 1));
+    dst[base + p0] = x0;
+    dst[base + 32 + p1] = x1;
+    __syncthreads();
 }
 
-// Ascending sort of 2048 unsigned keys in shared memory by a block of 1024 threads.
-// Every warp keeps 64 consecutive elements in registers (two per lane), so the bitonic steps
-// with partner distance <= 32 are register / shuffle exchanges without a block barrier; only
-// the steps with distance >= 64 go through shared memory (20 barriers instead of 66).
-__device__ __forceinline__ void block_sort_2048(unsigned int* s) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i0 = warp * 64 + lane, i1 = i0 + 32;
+// Ascending sort of 2048 unsigned keys in shared memory by a block of 1024 threads, `tmp` a second array of
+// that size. Every warp sorts 64 keys in registers (bitonic, shuffles only), five merge rounds by binary
+// search follow with one block barrier each. (A full bitonic network, whose steps of distance 64 and more
+// went through shared memory with 20 barriers and 46 shuffle steps, took 6.9 us of every compress launch.)
+__device__ __forceinline__ void block_sort_2048(unsigned int* s, unsigned int* tmp) {
+    const int lane = threadIdx.x & 31, i0 = (threadIdx.x >> 5) * 64 + lane, i1 = i0 + 32;
     unsigned int a = s[i0], b = s[i1];
-    for (int k = 2; k <= 2048; k <<= 1) {
-        if (k >= 128) {
-            s[i0] = a;
-            s[i1] = b;
-            __syncthreads();
-            for (int j = k >> 1; j >= 64; j >>= 1) {
-                const int t = threadIdx.x;
-                const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-                const int p = i | j;
-                const bool up = (i & k) == 0;
-                const unsigned int x = s[i], y = s[p];
-                if ((x > y) == up) {
-                    s[i] = y;
-                    s[p] = x;
-                }
-                __syncthreads();
-            }
-            a = s[i0];
-            b = s[i1];
+#pragma unroll
+    for (int k = 2; k <= 64; k <<= 1) {
+        if (k == 64 && a > b) {  // distance 32: both elements live in this thread, ascending
+            const unsigned int t = a;
+            a = b;
+            b = t;
         }
-        if (k >= 64) {  // distance 32: both elements live in this thread
-            const bool up = (i0 & k) == 0;
-            if ((a > b) == up) {
-                const unsigned int t = a;
-                a = b;
-                b = t;
-            }
-        }
+#pragma unroll
         for (int j = (k >> 1) < 16 ? (k >> 1) : 16; j > 0; j >>= 1) {
             const unsigned int pa = __shfl_xor_sync(0xFFFFFFFFu, a, j);
             const unsigned int pb = __shfl_xor_sync(0xFFFFFFFFu, b, j);
             const bool low = (lane & j) == 0;
-            const bool up0 = (i0 & k) == 0, up1 = (i1 & k) == 0;
+            const bool up0 = (lane & k) == 0 || k == 64, up1 = ((lane + 32) & k) == 0 || k == 64;
             a = (low == up0) ? min(a, pa) : max(a, pa);
             b = (low == up1) ? min(b, pb) : max(b, pb);
         }
-        __syncwarp();
     }
-    s[i0] = a;
-    s[i1] = b;
+    tmp[i0] = a;
+    tmp[i1] = b;
     __syncthreads();
+    merge_round<64>(tmp, s);
+    merge_round<128>(s, tmp);
+    merge_round<256>(tmp, s);
+    merge_round<512>(s, tmp);
+    merge_round<1024>(tmp, s);
 }
 
 // Number of elements of the ascending array a[0..n) that are <= x (upper bound).
