@@ -86,6 +86,12 @@ struct CP {
     const float* given_splits;
     int n_given;
     float given_min, given_max;
+    const float* dense_vals;                             // values of the dense kind (null: not this launch's business)
+    long long n_value;                                   // count and kind when meta is null
+    int kind_value;
+    int zero_slot;                                       // clear the local slot first
+    unsigned long long* done_word;                       // pinned host word for the status (checked calls)
+    unsigned long long done_seq;
     unsigned long long sample_rand;                      // draw behind the sample's offset (host: seed, step, rank)
     int mixers;                                          // every row of every group uses an integer mixer (<= 3 rows)
     unsigned char hash_ids[SKML_MAX_GROUPS][SKML_MAX_ROWS];  // hash rows of every group (host: seed, step, rank, group)
@@ -265,6 +271,13 @@ __device__ __forceinline__ void stage_stamp(unsigned int* ctrl, int i) {
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         reinterpret_cast<unsigned long long*>(ctrl)[8 + i] = t;
     }
+}
+
+// Clears the local slot (16-byte units; a capacity that is no multiple of 16 keeps its last bytes to the tail).
+__device__ void clear_slot(const CP& p, long long gid, long long gsz) {
+    uint4* z4 = reinterpret_cast<uint4*>(p.payload);
+    for (long long i = gid; i < p.slot_capacity / 16; i += gsz) __stcs(z4 + i, make_uint4(0, 0, 0, 0));
+    if (gid < (p.slot_capacity & 15)) p.payload[(p.slot_capacity & ~15ll) + gid] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2130,6 +2143,7 @@ __device__ void stage_prepare(const CP& p, long long n) {
     uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
     uint4* t4 = reinterpret_cast<uint4*>(p.tables);
     for (long long i = gid; i < (cells + 3) / 4; i += gsz) t4[i] = ones;
+    if (p.zero_slot) clear_slot(p, gid, gsz);
     if (p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE || p.huffman) {
         // the bit streams are completed with atomic ORs where chunks meet: they start from zero
         long long bound = payload_bound(n, 0, p.q, p.G, p.rows, p.col_ratio);
@@ -2272,6 +2286,7 @@ __device__ void finish_publish(const CP& p) {
             p.ctrl[4] = 0;  // the summary's min / max words go back to "nothing yet"
             p.ctrl[5] = 0;
             __threadfence();
+            skml_store_done(p.done_word, p.done_seq, p.status);
         }
     }
     __syncthreads();
@@ -2374,6 +2389,93 @@ __device__ void push_own_chunks(const CP& p, Smem& s, unsigned int my_begin, uns
         stage_stamp(p.ctrl, stage_id);                                                    \
     }
 
+// Dense kind: one narrow bucket code per coordinate, written straight into the local
+// payload and every peer's slot.
+template <bool FUSED>
+__device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ vals, int stage) {
+    unsigned int passed = 0;   // arrivals of the grid barriers so far
+    const long long n = p.dim;
+    const bool given = p.given_splits != nullptr;
+    // sample form: the splits are in every block after S1; the extremes of the values (needed for the bucket
+    // values in the header only) are collected by the code pass, and the header is written after it
+    const bool sample = p.sample_splits != 0 && !given;
+    if (FUSED || stage == 1) {
+        if (p.zero_slot) clear_slot(p, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+        if (sample) stage_sample_splits(p, s, vals, n);
+        else if (!given) stage_summary(p, s, vals, n);
+    }
+    if (!sample) {
+        STAGE_BARRIER(1)
+        if ((FUSED || stage == 2) && !given) stage_query(p, s, n);
+        STAGE_BARRIER(2)
+    }
+    if (FUSED || stage == 3) {
+        load_quantizer(p, s, FUSED && sample, !sample);
+        if (s.qi.bin_num > SKML_GPU_MAX_BINS) {
+            if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x33u);
+            return;
+        }
+        if (threadIdx.x == 0) s.lay.overflow = 0;
+        __syncthreads();
+        const int cb = s.qi.cell_bits, per = 16 / (cb / 8);
+        const unsigned long long off_codes = SKML_HEADER_BYTES + skml_align16(4ull * p.q);
+        const unsigned long long total = skml_align16(off_codes + (unsigned long long)n * (cb / 8));
+        if (total > (unsigned long long)p.slot_capacity) {
+            if (threadIdx.x == 0) skml_set_status(p.status, SKML_CAPACITY, 0x34u);
+            return;
+        }
+        if (!sample && blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
+        unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
+        const long long units = (n + per - 1) / per;
+        const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        for (long long u = gid; u < units; u += gsz) {
+            unsigned int words[4] = {0, 0, 0, 0};
+            for (int t = 0; t < per; ++t) {
+                long long i = u * per + t;
+                unsigned int code = 0;
+                if (i < n) {
+                    const float val = vals[i];
+                    code = (unsigned int)upper_bound_f(s.splits, s.qi.nsplits, val);
+                    const unsigned int k = f2ord(val);
+                    kmin = min(kmin, k);
+                    kmax = max(kmax, k);
+                }
+                if (cb == 8) words[t >> 2] |= (code & 0xFFu) << (8 * (t & 3));
+                else words[t >> 1] |= (code & 0xFFFFu) << (16 * (t & 1));
+            }
+            uint4 v = make_uint4(words[0], words[1], words[2], words[3]);
+            st_v4(reinterpret_cast<uint4*>(p.payload + off_codes) + u, v);
+            for (unsigned int r = 0; r < p.world; ++r)
+                if (r != p.rank && p.peer_payload[r]) st_v4(reinterpret_cast<uint4*>(p.peer_payload[r] + off_codes) + u, v);
+        }
+        if (sample) {   // one pair of atomics per warp
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                kmin = min(kmin, __shfl_xor_sync(0xFFFFFFFFu, kmin, o));
+                kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, o));
+            }
+            if ((threadIdx.x & 31) == 0 && kmin <= kmax) {
+                atomicMax(&p.ctrl[4], ~kmin);
+                atomicMax(&p.ctrl[5], kmax);
+            }
+        }
+    }
+    STAGE_BARRIER(3)
+    if (FUSED || stage == 4) {
+        if (sample) {
+            if (!FUSED) load_quantizer(p, s);   // staged launches: the extremes are complete now
+            else if (threadIdx.x == 0) refresh_minmax(p, s);
+            __syncthreads();
+            if (!FUSED) {
+                if (threadIdx.x == 0) s.lay.overflow = 0;
+                __syncthreads();
+            }
+            if (blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
+        }
+        finish_publish(p);
+    }
+}
+
 // STAGE < 0: all stages in one cooperative launch; otherwise only that stage.
 // ADAPTIVE / HUFFMAN: the key encoder and the table coder are compile-time choices, so that the default
 // path (delta_binary keys, plain tables) carries none of the other coders' registers.
@@ -2384,9 +2486,12 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     unsigned int passed = 0;   // arrivals of the grid barriers so far
     // names this launch's publications: one more than the launch before it (see finish_publish)
     const unsigned int epoch = FUSED ? ld_relaxed_gpu(&p.ctrl[1]) + 1u : 0u;
-    const long long kind = p.meta[1];
-    if (kind == SKML_KIND_DENSE) return;  // handled by the dense kernel
-    long long n = p.meta[0];
+    const long long kind = p.meta ? p.meta[1] : p.kind_value;
+    if (kind == SKML_KIND_DENSE) {  // un-fused launches leave it to the dense kernel's stages
+        if (FUSED && p.dense_vals) dense_stages<FUSED>(p, s, p.dense_vals, stage);
+        return;
+    }
+    long long n = p.meta ? p.meta[0] : p.n_value;
     if (n > p.n_max) {
         if (threadIdx.x == 0) skml_set_status(p.status, SKML_CAPACITY, 0x31u);
         n = 0;
@@ -2398,7 +2503,13 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
                 s.qi.bin_num = 0;
             }
             __syncthreads();
-            if (blockIdx.x == 0) write_header(p, s, 0, SKML_KIND_EMPTY);   // locally and into the peers' slots
+            if (blockIdx.x == 0) {
+                if (p.zero_slot) {   // by this block alone, before its own header
+                    clear_slot(p, threadIdx.x, blockDim.x);
+                    __syncthreads();
+                }
+                write_header(p, s, 0, SKML_KIND_EMPTY);   // locally and into the peers' slots
+            }
             finish_publish(p);
         }
         return;
@@ -2546,93 +2657,11 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     }
 }
 
-// Dense kind: one narrow bucket code per coordinate, written straight into the local
-// payload and every peer's slot.
 template <bool FUSED>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int stage) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-    unsigned int passed = 0;   // arrivals of the grid barriers so far
-    if (p.meta[1] != SKML_KIND_DENSE) return;
-    const long long n = p.dim;
-    const bool given = p.given_splits != nullptr;
-    // sample form: the splits are in every block after S1; the extremes of the values (needed for the bucket
-    // values in the header only) are collected by the code pass, and the header is written after it
-    const bool sample = p.sample_splits != 0 && !given;
-    if (FUSED || stage == 1) {
-        if (sample) stage_sample_splits(p, s, p.vals, n);
-        else if (!given) stage_summary(p, s, p.vals, n);
-    }
-    if (!sample) {
-        STAGE_BARRIER(1)
-        if ((FUSED || stage == 2) && !given) stage_query(p, s, n);
-        STAGE_BARRIER(2)
-    }
-    if (FUSED || stage == 3) {
-        load_quantizer(p, s, FUSED && sample, !sample);
-        if (s.qi.bin_num > SKML_GPU_MAX_BINS) {
-            if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x33u);
-            return;
-        }
-        if (threadIdx.x == 0) s.lay.overflow = 0;
-        __syncthreads();
-        const int cb = s.qi.cell_bits, per = 16 / (cb / 8);
-        const unsigned long long off_codes = SKML_HEADER_BYTES + skml_align16(4ull * p.q);
-        const unsigned long long total = skml_align16(off_codes + (unsigned long long)n * (cb / 8));
-        if (total > (unsigned long long)p.slot_capacity) {
-            if (threadIdx.x == 0) skml_set_status(p.status, SKML_CAPACITY, 0x34u);
-            return;
-        }
-        if (!sample && blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
-        unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
-        const long long units = (n + per - 1) / per;
-        const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-        for (long long u = gid; u < units; u += gsz) {
-            unsigned int words[4] = {0, 0, 0, 0};
-            for (int t = 0; t < per; ++t) {
-                long long i = u * per + t;
-                unsigned int code = 0;
-                if (i < n) {
-                    const float val = p.vals[i];
-                    code = (unsigned int)upper_bound_f(s.splits, s.qi.nsplits, val);
-                    const unsigned int k = f2ord(val);
-                    kmin = min(kmin, k);
-                    kmax = max(kmax, k);
-                }
-                if (cb == 8) words[t >> 2] |= (code & 0xFFu) << (8 * (t & 3));
-                else words[t >> 1] |= (code & 0xFFFFu) << (16 * (t & 1));
-            }
-            uint4 v = make_uint4(words[0], words[1], words[2], words[3]);
-            st_v4(reinterpret_cast<uint4*>(p.payload + off_codes) + u, v);
-            for (unsigned int r = 0; r < p.world; ++r)
-                if (r != p.rank && p.peer_payload[r]) st_v4(reinterpret_cast<uint4*>(p.peer_payload[r] + off_codes) + u, v);
-        }
-        if (sample) {   // one pair of atomics per warp
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                kmin = min(kmin, __shfl_xor_sync(0xFFFFFFFFu, kmin, o));
-                kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, o));
-            }
-            if ((threadIdx.x & 31) == 0 && kmin <= kmax) {
-                atomicMax(&p.ctrl[4], ~kmin);
-                atomicMax(&p.ctrl[5], kmax);
-            }
-        }
-    }
-    STAGE_BARRIER(3)
-    if (FUSED || stage == 4) {
-        if (sample) {
-            if (!FUSED) load_quantizer(p, s);   // staged launches: the extremes are complete now
-            else if (threadIdx.x == 0) refresh_minmax(p, s);
-            __syncthreads();
-            if (!FUSED) {
-                if (threadIdx.x == 0) s.lay.overflow = 0;
-                __syncthreads();
-            }
-            if (blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
-        }
-        finish_publish(p);
-    }
+    if ((p.meta ? p.meta[1] : p.kind_value) != SKML_KIND_DENSE) return;
+    dense_stages<FUSED>(p, *reinterpret_cast<Smem*>(smem_raw), p.vals, stage);
 }
 
 // ---------------------------------------------------------------------------
@@ -2650,7 +2679,7 @@ static int device_sms() {
 }
 
 static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
-    if (!a || !a->meta || !a->payload || !a->workspace || !a->status) return (int)cudaErrorInvalidValue;
+    if (!a || (!a->meta && (a->kind_value < 0 || a->kind_value > 2 || a->n_value < 0)) || !a->payload || !a->workspace || !a->status) return (int)cudaErrorInvalidValue;
     if (a->bin_num < 2 || a->bin_num > SKML_GPU_MAX_BINS) return (int)cudaErrorInvalidValue;
     if (a->group_num < 1 || a->group_num > SKML_MAX_GROUPS) return (int)cudaErrorInvalidValue;
     if (a->row_num < 1 || a->row_num > SKML_MAX_ROWS) return (int)cudaErrorInvalidValue;
@@ -2711,6 +2740,12 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     p.n_given = (int)a->n_given;
     p.given_min = (float)a->given_min;
     p.given_max = (float)a->given_max;
+    p.dense_vals = a->dense_vals;
+    p.n_value = a->n_value;
+    p.kind_value = (int)a->kind_value;
+    p.zero_slot = a->zero_slot != 0;
+    p.done_word = a->done_word;
+    p.done_seq = a->done_seq;
     // draws that depend on the launch's parameters only are made here, once, instead of by every block
     p.sample_rand = skml_rand(p.seed, p.step, p.rank, 0x7300u);
     p.mixers = p.rows <= 3;
@@ -2857,4 +2892,12 @@ extern "C" int skml_compress_dense(const SkmlCompressArgs* a, void* stream) {
     static LaunchCache cache;
     return launch_stages(compress_dense_kernel<true>, compress_dense_kernel<false>, cache, p, grid, a->fused != 0, 4,
                          (cudaStream_t)stream);
+}
+
+extern "C" int skml_compress_checked(SkmlCompressArgs* a, unsigned int* status_out, void* stream) {
+    if (!a || !a->done_word || !a->fused || !status_out) return (int)cudaErrorInvalidValue;
+    a->done_seq = ((*a->done_word >> 32) + 1) & 0xFFFFFFFFull;
+    const int rc = skml_compress_sparse(a, stream);
+    if (rc) return rc;
+    return skml_wait_done(a->done_word, a->done_seq, a->status, status_out, (cudaStream_t)stream);
 }

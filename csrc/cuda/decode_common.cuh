@@ -64,6 +64,8 @@ struct DP {
     double* wsq;       // running sum of squares of the weights (null: not kept)
     double* reg_out;   // receives reg_lambda * sqrt(*wsq) when the launch ends
     double reg_lambda;
+    unsigned long long* done_word;   // pinned host word for the status (checked calls)
+    unsigned long long done_seq;
 };
 
 struct DecItem {  // one (rank, group) key stream

@@ -736,6 +736,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
                     unsigned long long t;
                     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
                     reinterpret_cast<unsigned long long*>(p.ctrl)[16 + (int)(p.step & 1)] = t;
+                    __threadfence();
+                    skml_store_done(p.done_word, p.done_seq, p.status);
                 }
             }
         }
@@ -765,6 +767,8 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
         if (threadIdx.x == 0 && atomicAdd(&p.ctrl[2], 1u) == gridDim.x - 1) {
             p.ctrl[2] = 0;
             p.ctrl[0] = 0;
+            __threadfence();
+            skml_store_done(p.done_word, p.done_seq, p.status);
         }
     }
 }
@@ -810,6 +814,8 @@ extern "C" int skml_decode_update(const SkmlDecodeArgs* a, void* stream_) {
     p.wsq = a->out_sum ? nullptr : a->weight_sumsq;
     p.reg_out = a->reg_out;
     p.reg_lambda = a->reg_lambda;
+    p.done_word = a->done_word;
+    p.done_seq = a->done_seq;
     p.key_capacity = a->key_capacity;
     p.loss_out = a->loss_out;
     p.out_sum = a->out_sum;
@@ -866,6 +872,16 @@ extern "C" int skml_decode_update(const SkmlDecodeArgs* a, void* stream_) {
         if (e != cudaSuccess) return (int)e;
     }
     return 0;
+}
+
+extern "C" int skml_decode_sum_checked(SkmlDecodeArgs* a, unsigned int* status_out, void* stream) {
+    if (!a || !a->done_word || !a->fused || !a->out_sum || !status_out) return (int)cudaErrorInvalidValue;
+    const cudaError_t e = cudaMemsetAsync(a->out_sum, 0, (size_t)a->dim * sizeof(float), (cudaStream_t)stream);
+    if (e != cudaSuccess) return (int)e;
+    a->done_seq = ((*a->done_word >> 32) + 1) & 0xFFFFFFFFull;
+    const int rc = skml_decode_update(a, stream);
+    if (rc) return rc;
+    return skml_wait_done(a->done_word, a->done_seq, a->status, status_out, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -42,6 +42,12 @@ typedef struct SkmlCompressArgs {
     long long quantile_summary;    // 0 = split points from a 4096-value sample that every thread-block cluster
                                    // draws alike (no grid barrier, no query stage), 1 = mergeable k = 128 sketch per block,
                                    // merged per cluster and queried over all runs.
+    const float* dense_vals;       // values of the dense kind: the sparse entry point then serves both kinds in one launch
+                                   // (meta[1] chooses on the device); null = it leaves the dense kind alone
+    long long n_value, kind_value; // count and kind when `meta` is null
+    long long zero_slot;           // 1 = the local slot is cleared up to slot_capacity first
+    unsigned long long* done_word; // pinned host word of the checked call (skml_compress_checked sets done_seq itself)
+    unsigned long long done_seq;
 } SkmlCompressArgs;
 
 long long skml_compress_workspace_bytes(long long n_max, long long bin_num, long long group_num, long long row_num,
@@ -54,6 +60,9 @@ int skml_compress_sparse(const SkmlCompressArgs* args, void* stream);
 // Blocks per thread-block cluster of this process's most recent compress launch (2, 1, or 0 before the first).
 int skml_compress_cluster_size();
 int skml_compress_dense(const SkmlCompressArgs* args, void* stream);
+// skml_compress_sparse that returns once the kernel's status word is known (*status_out; nothing is read back through
+// the stream: the kernel's last block stores it into args->done_word, which the call polls).
+int skml_compress_checked(SkmlCompressArgs* args, unsigned int* status_out, void* stream);
 
 // Arguments of the fused decode + aggregate + update kernel.
 typedef struct SkmlDecodeArgs {
@@ -87,10 +96,14 @@ typedef struct SkmlDecodeArgs {
     long long adam_stride;         // 0 / 1: adam_m and adam_v are plain arrays; 4: both point into one array of
                                    // {m, v, sum, unused} quads (adam_v = adam_m + 1), whose third word the kernel
                                    // uses for the per-coordinate sums of lazy Adam (zero between calls)
+    unsigned long long* done_word; // as in SkmlCompressArgs
+    unsigned long long done_seq;
 } SkmlDecodeArgs;
 
 long long skml_decode_workspace_bytes(long long world, long long group_num);
 int skml_decode_update(const SkmlDecodeArgs* args, void* stream);
+// Clears out_sum, decodes into it and returns once the kernel's status word is known (see skml_compress_checked).
+int skml_decode_sum_checked(SkmlDecodeArgs* args, unsigned int* status_out, void* stream);
 
 // GLM numerics
 int skml_glm_grad(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,

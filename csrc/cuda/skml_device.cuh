@@ -367,3 +367,33 @@ __device__ __forceinline__ int lower_bound_u(const unsigned int* a, int n, unsig
     }
     return lo;
 }
+
+// ---------------------------------------------------------------------------
+// Checked calls: the kernel's last block stores (sequence number, status word) into a pinned host word and
+// the caller polls that word, instead of a device-to-host copy and a stream synchronisation (15 us and more
+// on top of a 35 us kernel). A kernel that reported an error may end without the store: the stream is
+// queried now and then, and once it has drained the status word is read the plain way.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void skml_store_done(unsigned long long* word, unsigned long long seq, const unsigned int* status) {
+    if (word) st_release_sys(word, (seq << 32) | ld_relaxed_gpu(status));
+}
+
+static inline int skml_wait_done(volatile unsigned long long* word, unsigned long long seq, const unsigned int* status,
+                                 unsigned int* status_out, cudaStream_t stream) {
+    for (unsigned long long spins = 1;; ++spins) {
+        const unsigned long long v = *word;
+        if ((v >> 32) == (seq & 0xFFFFFFFFull)) {
+            *status_out = (unsigned int)v;
+            return 0;
+        }
+        if ((spins & 0x3FFF) == 0) {
+            const cudaError_t q = cudaStreamQuery(stream);
+            if (q == cudaErrorNotReady) continue;
+            if (q != cudaSuccess) return (int)q;
+            if ((*word >> 32) == (seq & 0xFFFFFFFFull)) continue;
+            cudaError_t e = cudaMemcpyAsync(status_out, status, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            return (int)e;
+        }
+    }
+}

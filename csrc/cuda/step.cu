@@ -95,14 +95,9 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
     a->compress->keys = a->keys;
     a->compress->meta = a->meta;
     a->compress->vals = a->gvals;
+    a->compress->dense_vals = a->dense_vals;   // one launch serves both kinds
     rc = skml_compress_sparse(a->compress, stream_);
     if (rc) return rc;
-    if (a->dense_vals) {
-        a->compress->vals = a->dense_vals;
-        rc = skml_compress_dense(a->compress, stream_);
-        a->compress->vals = a->gvals;
-        if (rc) return rc;
-    }
     a->decode->step = a->step;
     a->decode->lr = a->lr;
     a->decode->adam_scale = a->adam_scale;

@@ -86,7 +86,11 @@ class GpuEngine:
         if allow_dense and self.mode == "nccl_kv":
             self.mode = "nccl_dense"  # near-dense gradients: the raw key/value list is no smaller
         self.st = GlmState.create(dim, bound, self.device, allow_dense)
-        self.loss_ring = torch.zeros((max(conf.batch_num, 1), 4), dtype=torch.float64, device=self.device)
+        # the loss ring and the status word share one allocation: an epoch's end reads both in one copy
+        ring = max(conf.batch_num, 1) * 4
+        self._report = torch.zeros(ring + 1, dtype=torch.float64, device=self.device)
+        self.loss_ring = self._report[:ring].view(-1, 4)
+        self.st.status = self._report[ring:].view(torch.int32)[:1]
         self.partials_template = torch.tensor([float(self.batch_rows), 0.0, 0.0, 0.0], dtype=torch.float64,
                                               device=self.device)
         self.batch_index = 0
@@ -276,8 +280,7 @@ class GpuEngine:
         if lid is not None:
             L.count_launches(len(segs) + 2 + 2)  # gather, gradient segment(s), finalize, compress, decode
         else:
-            L.count_launches((3 if bi is not None else len(segs) + 2) + 1 +
-                             (1 if self.st.dense_vals is not None and bi is None else 0) + 1)
+            L.count_launches((3 if bi is not None else len(segs) + 2) + 1 + 1)
 
     # ----------------------------------------------------------------- steps
     def _segments(self, count: int):
@@ -384,6 +387,10 @@ class GpuEngine:
         if hi - lo != self.batch_rows or lo % self.batch_rows:
             return None
         return self.tindex[lo // self.batch_rows]
+
+    def defers_gradient(self) -> bool:
+        """Whether `compute_gradient` only notes the batch, for the single-call step to launch everything."""
+        return self._fast_ok()
 
     def _fast_ok(self) -> bool:
         return (self.mode == "sketch" and getattr(self, "depth", 0) == 0 and bool(self.conf.extras.get("single_call_step", True)) and
@@ -559,16 +566,18 @@ class GpuEngine:
 
     def resolve_losses(self, handles) -> List[float]:
         """One device->host read per epoch: batch loss = sum obj / sum batch + reg / world."""
-        self.check()
         m = self.t.model
         if not self.reg_every_step and m.loss.is_l2_reg:
             self.loss_ring[:, 2] = torch.linalg.vector_norm(m.weights).double() * m.loss.lam * self.t.comm.world
-        ring = self.loss_ring.cpu()
+        report = self._report.cpu()
+        if getattr(self, "depth", 0) == 1 or int(report[-1:].view(torch.int32)[0]):
+            self.check()
+        ring = report[:-1].view(-1, 4).tolist()
         world = self.t.comm.world
         out = []
         for h in handles:
-            r = ring[h.index % ring.shape[0]]
-            out.append(float(r[1] / max(float(r[0]), 1.0) + r[2] / world))
+            r = ring[h.index % len(ring)]
+            out.append(r[1] / max(r[0], 1.0) + r[2] / world)
         return out
 
     def validate(self):

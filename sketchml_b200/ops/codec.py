@@ -2,6 +2,8 @@
 from __future__ import annotations
 
 import ctypes as C
+import threading
+import weakref
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -31,6 +33,51 @@ class ExchangeRegionView:
     @staticmethod
     def region_bytes(world: int, slot_capacity: int) -> int:
         return FLAG_BYTES + 2 * world * slot_capacity
+
+
+class _DoneWords:
+    """Pinned host words for checked calls: one page for the process (pinning memory takes milliseconds), a word per
+    codec object, given back with it; an object that finds the page full pins a word of its own."""
+    _WORDS = 512
+    _lock = threading.Lock()
+    _page: Optional[torch.Tensor] = None
+    _free: List[int] = []
+
+    @classmethod
+    def take(cls, owner) -> torch.Tensor:
+        with cls._lock:
+            if cls._page is None:
+                cls._page = torch.zeros(cls._WORDS * 8, dtype=torch.int64).pin_memory()
+                cls._free = list(range(cls._WORDS))
+            if not cls._free:
+                return torch.zeros(1, dtype=torch.int64).pin_memory()
+            i = cls._free.pop()
+        weakref.finalize(owner, cls._give_back, i)
+        return cls._page[8 * i:8 * i + 1]     # 64 bytes apart
+
+    @classmethod
+    def _give_back(cls, i: int) -> None:
+        with cls._lock:
+            cls._free.append(i)
+
+
+class _Checked:
+    """What a checked call needs besides its arguments: a status word, the pinned host word the kernel reports its
+    end in, and room for the status."""
+
+    def __init__(self, device):
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.word = _DoneWords.take(self)
+        self.out = C.c_uint(0)
+        self.out_ref = C.byref(self.out)
+
+    def finish(self, owner, where: str) -> None:
+        st = self.out.value
+        if st:
+            self.status.zero_()
+            owner.reset()
+            from ..parallel.failure import check_status
+            check_status(st, where)
 
 
 def read_status(status: torch.Tensor, reset: bool = True) -> int:
@@ -73,6 +120,8 @@ class GpuCompressor:
         self.dense_possible = self.n_max * 3 > self.dim * 2
         self.capacity = int(self.lib.skml_payload_capacity(self.n_max, self.dim if self.dense_possible else 0, bin_num,
                                                            group_num, row_num, self.col_ratio))
+        self._checked: Optional[_Checked] = None
+        self._local_args = None      # argument block of compress_local, kept between calls
 
     def reset(self) -> None:
         """Clears barrier words, counters and publication marks (needed only after a kernel reported an error)."""
@@ -107,13 +156,14 @@ class GpuCompressor:
                  world: int, payload_ptr: int, slot_capacity: int, peer_payload: Sequence[int],
                  peer_flag: Sequence[Optional[int]], status: torch.Tensor, loss_partials: Optional[torch.Tensor] = None,
                  dense_vals: Optional[torch.Tensor] = None, given=None) -> None:
-        """Launches the sparse-kind kernel (acts iff meta[1] is 0 or 1) and, when ``dense_vals``
-        is given, the dense-kind kernel (acts iff meta[1] == 2)."""
+        """Compresses the sparse kind (meta[1] 0 or 1) and, when ``dense_vals`` is given, the dense kind
+        (meta[1] == 2): one launch serves both; un-fused kernels launch the stages of either."""
         a = self._args(keys, vals, meta, step, rank, world, payload_ptr, slot_capacity, peer_payload, peer_flag,
                        status, loss_partials, given)
+        a.dense_vals = L.ptr(dense_vals)
         L.check(self.lib.skml_compress_sparse(C.byref(a), L.stream()), "skml_compress_sparse")
         L.count_launches(1 if self.fused else 8)
-        if dense_vals is not None:
+        if dense_vals is not None and not self.fused:
             a.vals = L.ptr(dense_vals)
             L.check(self.lib.skml_compress_dense(C.byref(a), L.stream()), "skml_compress_dense")
             L.count_launches(1 if self.fused else 4)
@@ -122,23 +172,36 @@ class GpuCompressor:
                        dense: bool = False, given=None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Single-GPU convenience: compresses into a fresh (or given) byte buffer and returns it."""
         n = vals.numel()
-        meta = torch.tensor([n, 2 if dense else (1 if n else 0), 0, 0], dtype=torch.int64, device=self.device)
+        kind = 2 if dense else (1 if n else 0)
+        ck = self._checked
+        if ck is None:
+            ck = self._checked = _Checked(self.device)
+        if self.fused:   # one launch that also clears the slot; its end and its status come through a host word
+            buf = out if out is not None else torch.empty(self.capacity, dtype=torch.uint8, device=self.device)
+            ptr = buf.data_ptr()
+            a = self._local_args
+            if a is None or given is not None or a.n_given or a.rank != rank or a.world != world:
+                ptrs = [None] * world
+                a = self._local_args = self._args(keys, vals, None, step, rank, world, ptr, buf.numel(), ptrs, ptrs, ck.status,
+                                                  None, given)
+                a.done_word = ck.word.data_ptr()
+            a.keys, a.vals, a.step, a.seed = L.ptr(keys), vals.data_ptr(), step, self.seed
+            a.payload, a.peer_payload[rank], a.slot_capacity = ptr, ptr, buf.numel()
+            a.dense_vals, a.n_value, a.kind_value, a.zero_slot = a.vals if dense else None, n, kind, int(out is None)
+            L.check(self.lib.skml_compress_checked(C.byref(a), ck.out_ref, L.stream()), "skml_compress_checked")
+            L.count_launches(1)
+            ck.finish(self, "in the compress kernel")
+            return buf
+        meta = torch.tensor([n, kind, 0, 0], dtype=torch.int64, device=self.device)
         buf = out if out is not None else torch.zeros(self.capacity, dtype=torch.uint8, device=self.device)
-        status = torch.zeros(1, dtype=torch.int32, device=self.device)
         ptrs = [None] * world
         ptrs[rank] = buf.data_ptr()
-        flags = [None] * world
-        if dense:
-            a = self._args(None, vals, meta, step, rank, world, buf.data_ptr(), buf.numel(), ptrs, flags, status, None, given)
-            L.check(self.lib.skml_compress_dense(C.byref(a), L.stream()), "skml_compress_dense")
-        else:
-            a = self._args(keys, vals, meta, step, rank, world, buf.data_ptr(), buf.numel(), ptrs, flags, status, None, given)
-            L.check(self.lib.skml_compress_sparse(C.byref(a), L.stream()), "skml_compress_sparse")
-        st = read_status(status)
-        if st:
-            self.reset()
-            from ..parallel.failure import check_status
-            check_status(st, "in the compress kernel")
+        a = self._args(None if dense else keys, vals, meta, step, rank, world, buf.data_ptr(), buf.numel(), ptrs, [None] * world,
+                       ck.status, None, given)
+        fn = self.lib.skml_compress_dense if dense else self.lib.skml_compress_sparse
+        L.check(fn(C.byref(a), L.stream()), "skml_compress")
+        ck.out.value = read_status(ck.status)
+        ck.finish(self, "in the compress kernel")
         return buf
 
     def last_splits(self):
@@ -180,6 +243,8 @@ class GpuDecoder:
         self.workspace = torch.zeros(256, dtype=torch.uint8, device=self.device)
         self.table_capacity = int(table_capacity) if table_capacity > 0 else 2 * self.key_capacity + 4096
         self.table_scratch = torch.zeros(self.table_capacity, dtype=torch.uint8, device=self.device)
+        self._checked: Optional[_Checked] = None
+        self._sum_args = None        # argument block of decode_sum, kept between calls
         self.norm_track = None  # (sum of w^2, where lambda * ||w|| goes, lambda): see track_norm
 
     def track_norm(self, sumsq: torch.Tensor, reg_out: torch.Tensor, lam: float) -> None:
@@ -232,13 +297,25 @@ class GpuDecoder:
     def decode_sum(self, payloads: List[torch.Tensor], step: int = 0) -> torch.Tensor:
         """Single-GPU convenience: decodes the given payload buffers (one per rank, rank order)
         and returns the dense fp32 mean over ranks (accumulated into a zeroed buffer)."""
-        out = torch.zeros(self.dim, dtype=torch.float32, device=self.device)
-        status = torch.zeros(1, dtype=torch.int32, device=self.device)
+        ck = self._checked
+        if ck is None:
+            ck = self._checked = _Checked(self.device)
         cap = min(p.numel() for p in payloads)
-        self.decode_update([p.data_ptr() for p in payloads], [None] * len(payloads), cap, step, status, out_sum=out)
-        st = read_status(status)
-        if st:
-            self.reset()
-            from ..parallel.failure import check_status
-            check_status(st, "in the decode kernel")
+        ptrs, flags = [p.data_ptr() for p in payloads], [None] * len(payloads)
+        if self.fused:
+            out = torch.empty(self.dim, dtype=torch.float32, device=self.device)
+            a = self._sum_args
+            if a is None or a.world != len(ptrs):
+                a = self._sum_args = self.make_args(ptrs, flags, cap, step, ck.status, out_sum=out)
+                a.done_word = ck.word.data_ptr()
+            for r, p in enumerate(ptrs):
+                a.payload[r] = p
+            a.slot_capacity, a.step, a.out_sum = cap, step, out.data_ptr()
+            L.check(self.lib.skml_decode_sum_checked(C.byref(a), ck.out_ref, L.stream()), "skml_decode_sum_checked")
+            L.count_launches(1)
+        else:
+            out = torch.zeros(self.dim, dtype=torch.float32, device=self.device)
+            self.decode_update(ptrs, flags, cap, step, ck.status, out_sum=out)
+            ck.out.value = read_status(ck.status)
+        ck.finish(self, "in the decode kernel")
         return out

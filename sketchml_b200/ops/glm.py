@@ -101,7 +101,7 @@ def glm_validate(csr: DeviceCSR, w: torch.Tensor, loss_id: int, status: torch.Te
                                           L.ptr(margins), L.ptr(status), L.budget_cycles(budget_s), L.stream()),
                 "skml_glm_validate")
         L.count_launches(1)
-    acc[5] = csr.rows
+    acc[5:].fill_(float(csr.rows))
     return acc
 
 

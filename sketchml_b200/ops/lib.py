@@ -36,6 +36,8 @@ class CompressArgs(C.Structure):
         ("peer_flag", c_vp * MAX_PEERS), ("workspace", c_vp), ("workspace_bytes", c_ll), ("status", c_vp),
         ("budget_cycles", c_ll), ("given_splits", c_vp), ("n_given", c_ll), ("given_min", c_d),
         ("given_max", c_d), ("fused", c_ll), ("grid", c_ll), ("key_encoder", c_ll), ("cell_bits", c_ll), ("quantile_summary", c_ll),
+        ("dense_vals", c_vp), ("n_value", c_ll), ("kind_value", c_ll), ("zero_slot", c_ll), ("done_word", c_vp),
+        ("done_seq", c_ull),
     ]
 
 
@@ -47,6 +49,7 @@ class DecodeArgs(C.Structure):
         ("out_sum", c_vp), ("workspace", c_vp), ("status", c_vp), ("budget_cycles", c_ll), ("fused", c_ll),
         ("grid", c_ll), ("max_groups", c_ll), ("val_scratch", c_vp), ("table_scratch", c_vp), ("table_capacity", c_ll),
         ("weight_sumsq", c_vp), ("reg_out", c_vp), ("reg_lambda", c_d), ("adam_stride", c_ll),
+        ("done_word", c_vp), ("done_seq", c_ull),
     ]
 
 
@@ -75,6 +78,8 @@ _SIGS = {
     "skml_compress_sparse": (c_int, [C.POINTER(CompressArgs), c_vp]),
     "skml_compress_cluster_size": (c_int, []),
     "skml_compress_dense": (c_int, [C.POINTER(CompressArgs), c_vp]),
+    "skml_compress_checked": (c_int, [C.POINTER(CompressArgs), c_vp, c_vp]),
+    "skml_decode_sum_checked": (c_int, [C.POINTER(DecodeArgs), c_vp, c_vp]),
     "skml_decode_workspace_bytes": (c_ll, [c_ll, c_ll]),
     "skml_decode_update": (c_int, [C.POINTER(DecodeArgs), c_vp]),
     "skml_glm_grad": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_vp, c_vp, c_int, c_f, c_int,

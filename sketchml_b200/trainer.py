@@ -269,7 +269,8 @@ class Trainer:
 
     def compute_gradient(self, epoch: int, batch: int):
         """GeneralizedLinearModel.scala:125-141: batch loss = objLoss/batchSize + regLoss/workerNum."""
-        with self.timer.phase("gradient"):
+        deferred = getattr(self.engine, "defers_gradient", None)
+        with self.timer.phase("gradient", device=not (deferred is not None and deferred())):
             bs, obj, reg = self.engine.compute_gradient()
         if isinstance(bs, (int, float)):
             tot = self.comm.all_reduce_sum([bs, obj, reg])

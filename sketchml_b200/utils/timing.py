@@ -21,11 +21,13 @@ class PhaseTimer:
         self._pending = []
 
     @contextlib.contextmanager
-    def phase(self, name: str):
+    def phase(self, name: str, device: bool = True):
+        """``device=False``: the phase only queues work that another call launches, so it is timed on the host (two
+        event records with nothing between them hold up the stream for several microseconds)."""
         if not self.enabled:
             yield
             return
-        if self.use_cuda:
+        if self.use_cuda and device:
             torch.cuda.nvtx.range_push(name)
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             a.record()
