@@ -11,23 +11,36 @@
 // of every adjacent candidate pair, the thr-th largest error as threshold, pairs at or above it
 // (the first thr of them in index order) stay split. Decode value of a bucket = midpoint of its edges.
 //
-// The split search is one block of 1024 threads: every round is a map over the pairs, a radix select
-// (12-bit digits, shared-memory histogram) and an ordered compaction, and the candidate set halves
-// from round to round, so the whole search reads about two entries per value.
+// The split search is one cooperative launch. A round is a map over the candidate pairs, a selection and
+// an ordered compaction, and the candidate set halves from round to round, so the search reads about two
+// entries per value; what bounds it is the chain of some twenty rounds. While a round has more than
+// Z_ALONE pairs they are cut into one slice per block: every block selects the keys of its slice that can
+// be among the round's largest, publishes them, and after a grid barrier selects among all blocks' lists,
+// which also tells it how many pairs the blocks before it keep split. The rest is block 0's alone, about
+// 2 us a round. (One block for all rounds took 822 us for 330,000 values.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <cub/device/device_radix_sort.cuh>
 
-#include "../common/skml_common.h"
 #include "skml_api.h"
+#include "skml_device.cuh"
 
 namespace {
 
 constexpr int ZT = 1024;           // threads of the split search
-constexpr int ZDIGIT = 12;         // radix-select digit
-constexpr int ZBINS = 1 << ZDIGIT;
 constexpr int Z_MAX_BUCKETS = 8192;     // the split and midpoint tables are staged in shared memory
+constexpr int Z_KPT = 8;                // values a thread handles per tile of the prefix sums
+constexpr int Z_ALONE = ZT * Z_KPT;     // pairs one block handles in shared memory: below, a barrier costs more than it saves
+constexpr int Z_MAX_BLOCKS = 148;
+constexpr int Z_TAIL = 512;             // candidates one warp handles in shared memory and registers, without a barrier
+
+// What the blocks of the split search share (cleared by the pad kernel).
+struct ZShared {
+    unsigned int bar, status, pad[14];
+    double sum_v[Z_MAX_BLOCKS], sum_v2[Z_MAX_BLOCKS];     // sums over the blocks' slices of values
+    unsigned long long cand[Z_ALONE];                     // blocks x kept pairs of a round at most
+};
 
 struct ZScratch {
     float* sorted_in;        // values padded with +inf
@@ -37,6 +50,7 @@ struct ZScratch {
     int* idx_a;              // candidate split positions (double buffered)
     int* idx_b;
     unsigned long long* err; // order-preserving keys of the pair errors
+    ZShared* shared;
     void* cub_temp;
     size_t cub_bytes;
 };
@@ -64,16 +78,18 @@ size_t carve(unsigned char* base, long long n_max, ZScratch* z) {
     int* ia = reinterpret_cast<int*>(take(4 * n));
     int* ib = reinterpret_cast<int*>(take(4 * n));
     unsigned long long* e = reinterpret_cast<unsigned long long*>(take(8 * (n / 2 + 1)));
+    ZShared* sh = reinterpret_cast<ZShared*>(take(sizeof(ZShared)));
     const size_t cb = cub_temp_bytes(n_max);
     void* ct = take(cb);
-    if (z) *z = ZScratch{a, b, r, t, ia, ib, e, ct, cb};
+    if (z) *z = ZScratch{a, b, r, t, ia, ib, e, sh, ct, cb};
     return o;
 }
 
 __global__ void zip_pad_kernel(const float* __restrict__ vals, const long long* __restrict__ n_ptr, long long n_max,
-                               float* __restrict__ out) {
+                               float* __restrict__ out, ZShared* __restrict__ shared) {
     long long n = *n_ptr;
     if (n > n_max) n = n_max;
+    if (blockIdx.x == 0 && threadIdx.x == 0) shared->bar = shared->status = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_max; i += (long long)gridDim.x * blockDim.x)
         out[i] = i < n ? vals[i] : __int_as_float(0x7F800000);
 }
@@ -111,30 +127,166 @@ __device__ __forceinline__ unsigned int zscan(unsigned int v, unsigned int* sh_w
     return sh_warp[warp] + inc - v;
 }
 
-// block-wide inclusive scan of one double per thread (pairwise adds in a fixed order)
-__device__ __forceinline__ double zscan_double(double v, double* sh_warp, double& total) {
+// block-wide exclusive scans of two doubles per thread (pairwise adds in a fixed order)
+__device__ __forceinline__ void zscan_double2(double& va, double& vb, double2* sh_warp, double& total_a, double& total_b) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double inc = v;
+    double a = va, b = vb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const double x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-        if (lane >= o) inc = __dadd_rn(x, inc);
+        const double x = __shfl_up_sync(0xFFFFFFFFu, a, o), y = __shfl_up_sync(0xFFFFFFFFu, b, o);
+        if (lane >= o) {
+            a = __dadd_rn(x, a);
+            b = __dadd_rn(y, b);
+        }
     }
-    __syncthreads();
-    if (lane == 31) sh_warp[warp] = inc;
+    __syncthreads();  // the previous call's readers are done
+    if (lane == 31) sh_warp[warp] = make_double2(a, b);
     __syncthreads();
     if (warp == 0) {
-        double winc = sh_warp[lane];
+        double wa = sh_warp[lane].x, wb = sh_warp[lane].y;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const double x = __shfl_up_sync(0xFFFFFFFFu, winc, o);
-            if (lane >= o) winc = __dadd_rn(x, winc);
+            const double x = __shfl_up_sync(0xFFFFFFFFu, wa, o), y = __shfl_up_sync(0xFFFFFFFFu, wb, o);
+            if (lane >= o) {
+                wa = __dadd_rn(x, wa);
+                wb = __dadd_rn(y, wb);
+            }
         }
-        sh_warp[lane] = winc;
+        sh_warp[lane] = make_double2(wa, wb);
     }
     __syncthreads();
-    total = sh_warp[31];
-    return warp ? __dadd_rn(sh_warp[warp - 1], inc) : inc;
+    total_a = sh_warp[31].x;
+    total_b = sh_warp[31].y;
+    double ea = __shfl_up_sync(0xFFFFFFFFu, a, 1), eb = __shfl_up_sync(0xFFFFFFFFu, b, 1);
+    if (lane == 0) ea = eb = 0.0;
+    if (warp) {
+        ea = __dadd_rn(sh_warp[warp - 1].x, ea);
+        eb = __dadd_rn(sh_warp[warp - 1].y, eb);
+    }
+    va = ea;
+    vb = eb;
+}
+
+// Squared error of merging the values between two prefix sums apart, as a sortable key.
+__device__ __forceinline__ unsigned long long merge_error(double l1, double l2, double cnt) {
+    const double mean = __ddiv_rn(l1, cnt);
+    return zkey(__dadd_rn(__dadd_rn(l2, __dmul_rn(__dmul_rn(mean, mean), cnt)), -__dmul_rn(__dmul_rn(2.0, mean), l1)));
+}
+
+// Squared error of merging candidate pair i (the values from its first candidate up to the next pair's).
+__device__ __forceinline__ unsigned long long pair_error(const ZScratch& z, const int* idx, unsigned int i, unsigned int split_num,
+                                                         unsigned int n) {
+    const unsigned int L = (unsigned int)__ldcg(idx + 2 * i);
+    const unsigned int R = (2 * i + 2 >= split_num ? n : (unsigned int)__ldcg(idx + 2 * i + 2)) - 1u;
+    const double l1 = __dadd_rn(z.r[R], L ? -z.r[L - 1] : 0.0);
+    const double l2 = __dadd_rn(z.t[R], L ? -z.t[L - 1] : 0.0);
+    return merge_error(l1, l2, (double)(R - L + 1u));
+}
+
+struct ZSmem {
+    unsigned long long key[Z_ALONE];   // errors of the block's slice of a round, where they fit
+    unsigned long long all[Z_ALONE];   // the lists of all blocks
+    unsigned int hist[ZT];             // select_largest
+    unsigned int warp[33];
+    double2 dwarp[32];
+    unsigned int digit, above, ncand, fill;
+    // the last rounds (at most Z_TAIL candidates): their positions and the prefix sums in front of them
+    struct Tail {
+        int pos[Z_TAIL];
+        double sum_v[Z_TAIL], sum_v2[Z_TAIL];
+    } tail[2];                         // a round reads one and writes the other
+};
+
+// Threshold for the k largest of keys[0, count), in shared memory or global (0 = no key, k keys at least): the k-th
+// largest, or a value that exactly k keys reach (`exact`). Radix select, ten bits a pass from the top: a
+// shared-memory count per digit, one digit per thread. Two or three passes settle real errors, because it
+// stops as soon as the keys down to a digit's are k. A function of its own: the kernel runs its stages a few
+// times per round, and with everything inlined it spent more time fetching instructions than executing.
+// (Counting against several thresholds per step without a histogram cost 5,000 to 15,000 cycles a selection.)
+__device__ __noinline__ unsigned long long select_largest(ZSmem& sm, const unsigned long long* keys, unsigned int count, unsigned int k,
+                                                          bool& exact) {
+    const unsigned int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long prefix = 0;   // the digits settled so far
+    exact = false;
+    for (int shift = 54;; shift = max(0, shift - 10)) {
+        const int bits = shift == 54 ? 10 : min(10, 54 - shift - ((54 - shift - 1) / 10) * 10);
+        const int top = shift + bits;   // bits from here up are the prefix's
+        sm.hist[tid] = 0;
+        __syncthreads();
+        for (unsigned int i = tid; i < count; i += ZT) {
+            const unsigned long long key = keys[i];
+            if (key && (top == 64 || (key >> top) == (prefix >> top))) atomicAdd(&sm.hist[(unsigned int)(key >> shift) & ((1u << bits) - 1u)], 1u);
+        }
+        __syncthreads();
+        // thread t looks at digit 1023 - t: keys in the digits above it
+        const unsigned int mine = sm.hist[ZT - 1 - tid];
+        unsigned int inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if ((int)lane >= o) inc += x;
+        }
+        if (lane == 31) sm.warp[warp] = inc;
+        __syncthreads();
+        const unsigned int w = sm.warp[lane];
+        const unsigned int above = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? w : 0u) + inc - mine;
+        if (above < k && k <= above + mine) {   // one thread: the k-th largest has this digit
+            sm.digit = ZT - 1 - tid;
+            sm.above = above;
+            sm.ncand = mine;
+        }
+        __syncthreads();
+        prefix |= (unsigned long long)sm.digit << shift;
+        k -= sm.above;
+        exact = sm.ncand == k;
+        if (exact || shift == 0) return prefix;
+    }
+}
+
+// The last rounds: at most Z_TAIL candidates in shared memory, a pair per thread of the first eight warps; the
+// selection is the block's. Every thread keeps count of the set.
+__device__ void tail_rounds(ZSmem& sm, int bin_num, double end_v, double end_v2, int n, unsigned int& split_num, unsigned int& rounds,
+                            unsigned int& which) {
+    const unsigned int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+    while (split_num > (unsigned int)bin_num) {
+        const ZSmem::Tail& in = sm.tail[which];
+        ZSmem::Tail& out = sm.tail[which ^ 1];
+        const unsigned int pairs = split_num / 2, odd = split_num & 1u;
+        int want = bin_num / 2 - (int)odd;
+        if (want < 1) want = 1;
+        const unsigned int thr_num = min((unsigned int)want, pairs);
+        unsigned long long key = 0;
+        if (i < pairs) {
+            const bool last = 2 * i + 2 >= split_num;
+            const double hv = last ? end_v : in.sum_v[2 * i + 2], hv2 = last ? end_v2 : in.sum_v2[2 * i + 2];
+            const int hp = last ? n : in.pos[2 * i + 2];
+            key = merge_error(__dadd_rn(hv, -in.sum_v[2 * i]), __dadd_rn(hv2, -in.sum_v2[2 * i]), (double)(hp - in.pos[2 * i]));
+            sm.key[i] = key;
+        }
+        __syncthreads();
+        bool exact;
+        const unsigned long long thr = thr_num < pairs ? select_largest(sm, sm.key, pairs, thr_num, exact) : 1ull;
+        const unsigned int flags = __ballot_sync(0xFFFFFFFFu, key >= thr);
+        if (lane == 0) sm.warp[warp] = (unsigned int)__popc(flags);
+        __syncthreads();
+        const unsigned int c = sm.warp[lane];
+        const unsigned int all = __reduce_add_sync(0xFFFFFFFFu, c);
+        const unsigned int at = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? c : 0u) + (unsigned int)__popc(flags & ((1u << lane) - 1u));
+        const unsigned int m = pairs + min(all, thr_num) + odd;
+        if (m >= split_num) break;   // no progress: stop with the current set
+        // candidate slots of the next set, thread by thread: first candidates, second ones that stay, an odd last one
+        const unsigned int to = i < pairs ? i + min(at, thr_num) : m - 1;
+        const int copies = i < pairs ? (key >= thr && at < thr_num ? 2 : 1) : (odd && i == pairs ? 1 : 0);
+        for (int q = 0; q < copies; ++q) {
+            out.pos[to + q] = in.pos[2 * i + q];
+            out.sum_v[to + q] = in.sum_v[2 * i + q];
+            out.sum_v2[to + q] = in.sum_v2[2 * i + q];
+        }
+        __syncthreads();
+        split_num = m;
+        which ^= 1;
+        ++rounds;
+    }
 }
 
 // meta_out: [0] buckets, [1] zero bucket, [2] halving rounds run; range_out: min, max of the values.
@@ -142,18 +294,19 @@ __global__ void __launch_bounds__(ZT, 1)
 zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_max, int bin_num,
                   float* __restrict__ splits_out, float* __restrict__ mids_out, int* __restrict__ meta_out,
                   float* __restrict__ range_out) {
-    __shared__ unsigned int hist[ZBINS];
-    __shared__ unsigned long long cand[ZT];   // the last candidates of a selection, ranked directly
-    __shared__ unsigned int sh_warp[33];
-    __shared__ double sh_dwarp[32];
-    __shared__ unsigned int sh_digit, sh_above, sh_ncand;
-    __shared__ unsigned long long sh_thr;
-    const int tid = threadIdx.x;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ZSmem& sm = *reinterpret_cast<ZSmem*>(smem_raw);
+    unsigned int* const sh_warp = sm.warp;
+    ZShared& g = *z.shared;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned int nb = gridDim.x, b = blockIdx.x;
+    unsigned int passed = 0;
+    auto barrier = [&](unsigned int stage) { return skml_grid_barrier(&g.bar, nb, &g.status, 2000000000ll, stage, passed); };
     long long n64 = *n_ptr;
     if (n64 > n_max) n64 = n_max;
     const unsigned int n = (unsigned int)n64;
     if (n == 0) {
-        if (tid == 0) {
+        if (tid == 0 && b == 0) {
             meta_out[0] = 0;
             meta_out[1] = 0;
             meta_out[2] = 0;
@@ -161,23 +314,66 @@ zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_m
         return;
     }
     const float* s = z.sorted;
-    // prefix sums of v and v^2, one tile of ZT values at a time (coalesced), carried from tile to tile
+    // prefix sums of v and v^2: a slice of the values per block, tiles of Z_KPT values per thread carried from
+    // tile to tile; every addition in a fixed order. A slice of one tile stays in registers while the blocks
+    // exchange their sums, a longer one is added up first.
     {
-        double carry_a = 0.0, carry_b = 0.0;
-        for (unsigned int base = 0; base < n; base += ZT) {
-            const unsigned int i = base + tid;
-            const double v = i < n ? (double)s[i] : 0.0;
-            double ta, tb;
-            const double ia = zscan_double(v, sh_dwarp, ta);
-            const double ib = zscan_double(__dmul_rn(v, v), sh_dwarp, tb);
-            if (i < n) {
-                z.r[i] = __dadd_rn(carry_a, ia);
-                z.t[i] = __dadd_rn(carry_b, ib);
-                z.idx_a[i] = (int)i;
+        const unsigned int per = (n + nb - 1) / nb, lo = min(n, per * b), hi = min(n, lo + per);
+        const bool one_tile = per <= (unsigned int)Z_ALONE;
+        double carry_a = 0.0, carry_b = 0.0, ta = 0.0, tb = 0.0;
+        if (nb > 1 && !one_tile) {
+            double a = 0.0, q = 0.0;
+            for (unsigned int i = lo + tid; i < hi; i += ZT) {
+                const double v = (double)s[i];
+                a = __dadd_rn(a, v);
+                q = __dadd_rn(q, __dmul_rn(v, v));
             }
-            carry_a = __dadd_rn(carry_a, ta);
-            carry_b = __dadd_rn(carry_b, tb);
+            zscan_double2(a, q, sm.dwarp, ta, tb);
         }
+        for (unsigned int base = lo; base < hi || base == lo; base += Z_ALONE) {
+            const unsigned int i0 = base + Z_KPT * tid;
+            float v[Z_KPT];
+            double a = 0.0, q = 0.0;
+#pragma unroll
+            for (int j = 0; j < Z_KPT; ++j) {
+                v[j] = i0 + j < hi ? s[i0 + j] : 0.f;
+                a = __dadd_rn(a, (double)v[j]);
+                q = __dadd_rn(q, __dmul_rn((double)v[j], (double)v[j]));
+            }
+            double tile_a, tile_b;
+            zscan_double2(a, q, sm.dwarp, tile_a, tile_b);
+            if (base == lo && nb > 1) {
+                if (tid == 0) {
+                    g.sum_v[b] = one_tile ? tile_a : ta;
+                    g.sum_v2[b] = one_tile ? tile_b : tb;
+                }
+                if (!barrier(0x60u)) return;
+                for (unsigned int k = lane; k < b; k += 32) {
+                    carry_a = __dadd_rn(carry_a, __ldcg(&g.sum_v[k]));
+                    carry_b = __dadd_rn(carry_b, __ldcg(&g.sum_v2[k]));
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    carry_a = __dadd_rn(carry_a, __shfl_xor_sync(0xFFFFFFFFu, carry_a, o));
+                    carry_b = __dadd_rn(carry_b, __shfl_xor_sync(0xFFFFFFFFu, carry_b, o));
+                }
+            }
+            a = __dadd_rn(carry_a, a);
+            q = __dadd_rn(carry_b, q);
+#pragma unroll
+            for (int j = 0; j < Z_KPT; ++j) {
+                a = __dadd_rn(a, (double)v[j]);
+                q = __dadd_rn(q, __dmul_rn((double)v[j], (double)v[j]));
+                if (i0 + j < hi) {
+                    z.r[i0 + j] = a;
+                    z.t[i0 + j] = q;
+                    z.idx_a[i0 + j] = (int)(i0 + j);
+                }
+            }
+            carry_a = __dadd_rn(carry_a, tile_a);
+            carry_b = __dadd_rn(carry_b, tile_b);
+        }
+        if (nb > 1 && !barrier(0x61u)) return;
     }
     __syncthreads();
     int* idx = z.idx_a;
@@ -185,112 +381,91 @@ zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_m
     unsigned int split_num = n, rounds = 0;
     while (split_num > (unsigned int)bin_num) {
         const unsigned int pairs = split_num / 2, odd = split_num & 1u;
+        const bool alone = nb == 1 || pairs <= Z_ALONE;
+        if (alone && b != 0) return;   // block 0 goes on by itself
+        if (split_num <= (unsigned int)Z_TAIL) break;   // and its first warp finishes
         int want = bin_num / 2 - (int)odd;
         if (want < 1) want = 1;
         const unsigned int thr_num = min((unsigned int)want, pairs);
-        // squared error of merging every adjacent pair of candidates
-        for (unsigned int i = tid; i < pairs; i += ZT) {
-            const unsigned int L = (unsigned int)idx[2 * i];
-            const unsigned int R = (2 * i + 2 >= split_num ? n : (unsigned int)idx[2 * i + 2]) - 1u;
-            const double l1 = __dadd_rn(z.r[R], L ? -z.r[L - 1] : 0.0);
-            const double l2 = __dadd_rn(z.t[R], L ? -z.t[L - 1] : 0.0);
-            const double cnt = (double)(R - L + 1u), mean = __ddiv_rn(l1, cnt);
-            const double e = __dadd_rn(__dadd_rn(l2, __dmul_rn(__dmul_rn(mean, mean), cnt)), -__dmul_rn(__dmul_rn(2.0, mean), l1));
-            z.err[i] = zkey(e);
-        }
+        // this block's pairs; their errors stay in shared memory where they fit
+        const unsigned int per = alone ? pairs : (pairs + nb - 1) / nb;
+        const unsigned int p0 = alone ? 0u : min(pairs, per * b), p1 = alone ? pairs : min(pairs, p0 + per), mine = p1 - p0;
+        unsigned long long* const key = per <= (unsigned int)Z_ALONE ? sm.key : z.err + p0;
+        for (unsigned int i = tid; i < mine; i += ZT) key[i] = pair_error(z, idx, p0 + i, split_num, n);
         __syncthreads();
-        // the thr_num-th largest error: radix select, most significant digit first; once the digit that
-        // holds it has at most ZT members they are gathered and ranked directly
-        unsigned long long prefix = 0, mask = 0;
-        unsigned int k = thr_num;
-        bool found = false;
-        for (int shift = 64 - ZDIGIT; shift > -ZDIGIT && !found; shift -= ZDIGIT) {
-            const int sh = shift < 0 ? 0 : shift;
-            const int bits = shift < 0 ? ZDIGIT + shift : ZDIGIT;
-            const unsigned int dm = (1u << bits) - 1u;
-            for (int i = tid; i < ZBINS; i += ZT) hist[i] = 0;
+        // keys of the slice at or above `thr` stay split (the first thr_num of the round's, in index order)
+        unsigned long long thr = 1;
+        bool exact = thr_num >= mine;   // no more than thr_num keys of the slice reach thr
+        if (!exact) thr = select_largest(sm, key, mine, thr_num, exact);
+        unsigned int before = 0;   // pairs at or above the round's threshold in the blocks before this one
+        if (!alone) {
+            // publish the slice's largest keys (at most thr_num: with more equal ones than that it does not
+            // matter which), then select among everybody's
+            if (tid == 0) sm.fill = 0;
             __syncthreads();
-            for (unsigned int i = tid; i < pairs; i += ZT) {
-                const unsigned long long key = z.err[i];
-                if ((key & mask) == prefix) atomicAdd(&hist[(unsigned int)(key >> sh) & dm], 1u);
-            }
-            __syncthreads();
-            // thread t owns digits [4t, 4t + 4) counted from the top
-            unsigned int c[4], mine = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                c[j] = hist[ZBINS - 1 - (4 * tid + j)];
-                mine += c[j];
-            }
-            unsigned int total;
-            unsigned int above = zscan(mine, sh_warp, total);
-            if (above < k && k <= above + mine) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (above < k && k <= above + c[j]) {
-                        sh_digit = (unsigned int)(ZBINS - 1 - (4 * tid + j));
-                        sh_above = above;
-                        sh_ncand = c[j];
+            for (int pass = exact ? 1 : 0; pass < 2; ++pass) {   // first those above thr, then those equal to it
+                const unsigned long long lo = pass ? thr : thr + 1, hi = pass && !exact ? thr : ~0ull;
+                for (unsigned int i = tid; i < mine; i += ZT) {
+                    const unsigned long long k = key[i];
+                    if (k >= lo && k <= hi) {
+                        const unsigned int at = atomicAdd(&sm.fill, 1u);
+                        if (at < thr_num) g.cand[b * thr_num + at] = k;
                     }
-                    above += c[j];
-                }
-            }
-            __syncthreads();
-            prefix |= (unsigned long long)sh_digit << sh;
-            mask |= (unsigned long long)dm << sh;
-            k -= sh_above;
-            const unsigned int ncand = sh_ncand;
-            __syncthreads();
-            if (sh == 0) {
-                found = true;   // every bit is fixed
-                if (tid == 0) sh_thr = prefix;
-            } else if (ncand <= ZT) {
-                if (tid == 0) sh_ncand = 0;
-                __syncthreads();
-                for (unsigned int i = tid; i < pairs; i += ZT) {
-                    const unsigned long long key = z.err[i];
-                    if ((key & mask) == prefix) cand[atomicAdd(&sh_ncand, 1u)] = key;
                 }
                 __syncthreads();
-                if ((unsigned int)tid < ncand) {
-                    const unsigned long long mk = cand[tid];
-                    unsigned int greater = 0, equal = 0;
-                    for (unsigned int j = 0; j < ncand; ++j) {
-                        greater += cand[j] > mk ? 1u : 0u;
-                        equal += cand[j] == mk ? 1u : 0u;
-                    }
-                    if (greater < k && k <= greater + equal) sh_thr = mk;  // every such thread writes the same key
-                }
-                found = true;
             }
+            // slots without a key hold none (a block with fewer pairs than thr_num)
+            for (unsigned int at = min(sm.fill, thr_num) + tid; at < thr_num; at += ZT) g.cand[b * thr_num + at] = 0ull;
+            if (!barrier(0x62u)) return;
+            for (unsigned int q = tid; q < nb * thr_num; q += ZT) sm.all[q] = __ldcg(&g.cand[q]);   // blocks x thr_num <= Z_ALONE
             __syncthreads();
+            thr = select_largest(sm, sm.all, nb * thr_num, thr_num, exact);
+            unsigned int cnt = 0;
+            for (unsigned int q = tid; q < b * thr_num; q += ZT) cnt += sm.all[q] >= thr ? 1u : 0u;
+            zscan(cnt, sh_warp, before);
         }
-        const unsigned long long thr = sh_thr;
-        // ordered compaction, one tile of ZT pairs at a time: the first thr_num pairs at or above the
-        // threshold keep their second candidate
-        unsigned int flagged_before = 0;
-        for (unsigned int base = 0; base < pairs; base += ZT) {
-            const unsigned int i = base + tid;
-            const bool f = i < pairs && z.err[i] >= thr;
+        // ordered compaction, a tile of ZT pairs at a time: the first thr_num pairs at or above the threshold keep
+        // their second candidate
+        unsigned int flagged = before;
+        for (unsigned int base = 0; base < mine; base += ZT) {
+            const unsigned int i = p0 + base + tid;
+            const bool in = base + tid < mine;
+            const int first = in ? __ldcg(idx + 2 * i) : 0, second = in ? __ldcg(idx + 2 * i + 1) : 0;   // on their way during the scan
+            const bool f = in && key[base + tid] >= thr;
             unsigned int tile_total;
-            const unsigned int before = flagged_before + zscan(f ? 1u : 0u, sh_warp, tile_total);
-            if (i < pairs) {
-                const unsigned int pos = i + min(before, thr_num);
-                nxt[pos] = idx[2 * i];
-                if (f && before < thr_num) nxt[pos + 1] = idx[2 * i + 1];
+            const unsigned int at = flagged + zscan(f ? 1u : 0u, sh_warp, tile_total);
+            if (in) {
+                const unsigned int pos = i + min(at, thr_num);
+                nxt[pos] = first;
+                if (f && at < thr_num) nxt[pos + 1] = second;
             }
-            flagged_before += tile_total;
+            flagged += tile_total;
         }
-        const unsigned int kept_total = min(flagged_before, thr_num);
+        // all blocks together keep thr_num second candidates: at least that many keys reach the threshold
+        const unsigned int kept_total = alone ? min(flagged, thr_num) : thr_num;
         const unsigned int m = pairs + kept_total + odd;
-        if (m >= split_num) break;  // no progress: stop with the current set (uniform for the block)
-        if (odd && tid == 0) nxt[pairs + kept_total] = idx[split_num - 1];
-        __syncthreads();
+        if (m >= split_num) break;  // no progress: stop with the current set (uniform for the block; never while several work)
+        if (odd && tid == 0 && b == 0) nxt[pairs + kept_total] = __ldcg(idx + split_num - 1);
+        if (alone) __syncthreads();
+        else if (!barrier(0x63u)) return;
         int* sw = idx;
         idx = nxt;
         nxt = sw;
         split_num = m;
         ++rounds;
+    }
+    if (b != 0) return;
+    if (split_num > (unsigned int)bin_num && split_num <= (unsigned int)Z_TAIL) {
+        for (unsigned int i = tid; i < split_num; i += ZT) {
+            const int at = __ldcg(idx + i);
+            sm.tail[0].pos[i] = at;
+            sm.tail[0].sum_v[i] = at ? z.r[at - 1] : 0.0;
+            sm.tail[0].sum_v2[i] = at ? z.t[at - 1] : 0.0;
+        }
+        __syncthreads();
+        unsigned int which = 0;
+        tail_rounds(sm, bin_num, z.r[n - 1], z.t[n - 1], (int)n, split_num, rounds, which);
+        for (unsigned int i = tid; i < split_num; i += ZT) idx[i] = sm.tail[which].pos[i];
     }
     __syncthreads();
     // split values (duplicates dropped), bucket midpoints, zero bucket
@@ -314,21 +489,20 @@ zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_m
         total_distinct += tile_total;
     }
     __syncthreads();
-    const unsigned int nb = total_distinct + 1u;
-    for (unsigned int i = tid; i < nb; i += ZT) {
+    const unsigned int buckets = total_distinct + 1u;
+    for (unsigned int i = tid; i < buckets; i += ZT) {
         const double left = i == 0 ? (double)vmin : (double)splits_out[i - 1];
-        const double right = i + 1 == nb ? (double)vmax : (double)splits_out[i];
+        const double right = i + 1 == buckets ? (double)vmax : (double)splits_out[i];
         mids_out[i] = (float)(0.5 * (left + right));
     }
+    int negs = 0;   // the splits ascend: the zero bucket is the number of negative ones
+    for (unsigned int base = 0; base + 1 < buckets; base += ZT) {
+        const unsigned int i = base + tid;
+        negs += __syncthreads_count(i + 1 < buckets && splits_out[i] < 0.f);
+    }
     if (tid == 0) {
-        int zero = 0;
-        if (vmin > 0.f) zero = 0;
-        else if (vmax < 0.f) zero = (int)nb - 1;
-        else {
-            while (zero < (int)nb - 1 && splits_out[zero] < 0.f) ++zero;
-        }
-        meta_out[0] = (int)nb;
-        meta_out[1] = zero;
+        meta_out[0] = (int)buckets;
+        meta_out[1] = vmin > 0.f ? 0 : (vmax < 0.f ? (int)buckets - 1 : negs);
         meta_out[2] = (int)rounds;
         range_out[0] = vmin;
         range_out[1] = vmax;
@@ -408,10 +582,25 @@ extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long l
     ZScratch z;
     if ((long long)carve(reinterpret_cast<unsigned char*>(scratch), n_max, &z) > scratch_bytes) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
-    zip_pad_kernel<<<zip_sm_count() * 4, 256, 0, s>>>(vals, n_ptr, n_max, z.sorted_in);
+    zip_pad_kernel<<<zip_sm_count() * 4, 256, 0, s>>>(vals, n_ptr, n_max, z.sorted_in, z.shared);
     cudaError_t e = cub::DeviceRadixSort::SortKeys(z.cub_temp, z.cub_bytes, z.sorted_in, z.sorted, (int)n_max, 0, 32, s);
     if (e != cudaSuccess) return (int)e;
-    zip_splits_kernel<<<1, ZT, 0, s>>>(z, n_ptr, n_max, bin_num, splits, mids, meta, range);
+    // a block per slice of about 2048 values, as many as their lists of kept pairs have room for
+    long long blocks = (n_max + 2047) / 2048;
+    const int keep = bin_num / 2 > 1 ? bin_num / 2 : 1;
+    if (blocks > Z_ALONE / keep) blocks = Z_ALONE / keep;
+    if (blocks > Z_MAX_BLOCKS) blocks = Z_MAX_BLOCKS;
+    if (blocks > zip_sm_count()) blocks = zip_sm_count();
+    if (blocks < 1 || n_max <= 2 * Z_ALONE) blocks = 1;
+    static bool ready = false;
+    if (!ready) {
+        e = cudaFuncSetAttribute(zip_splits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ZSmem));
+        if (e != cudaSuccess) return (int)e;
+        ready = true;
+    }
+    void* args[] = {&z, &n_ptr, &n_max, &bin_num, &splits, &mids, &meta, &range};
+    e = cudaLaunchCooperativeKernel((const void*)zip_splits_kernel, dim3((unsigned)blocks), dim3(ZT), args, sizeof(ZSmem), s);
+    if (e != cudaSuccess) return (int)e;
     const int cb = skml_zipml_code_bytes(bin_num);
     zip_code_kernel<<<zip_sm_count() * 4, 256, sizeof(float) * (size_t)(bin_num + 2), s>>>(vals, n_ptr, n_max, splits, meta, cb, codes);
     return (int)cudaGetLastError();
