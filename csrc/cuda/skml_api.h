@@ -162,20 +162,18 @@ int skml_finalize_compact(float* gc, const float* wc, float lambda, int n, float
                           void* stream);
 int skml_sm_count();
 
-// DeltaAdaptive key encoder, stand-alone (csrc/cuda/keys_kernels.cu). The caller computes the
-// inclusive prefix sums of the width arrays between the calls. Word buffers are 32-bit views of
-// the 64-bit BitSet words, zero-filled by the caller, with one spare word at the end.
-int skml_da_analyze(const int* keys, long long n, unsigned int* hist32, unsigned int* params, unsigned int* status,
-                    void* stream);   // params[0] = interval count, params[1] = 1 for unary flags; status bit 0 = unsorted keys
-int skml_da_widths(const int* keys, long long n, const unsigned int* params, int* flag_w, int* delta_w, void* stream);
-int skml_da_pack(const int* keys, long long n, const unsigned int* params, const long long* flag_incl,
-                 const long long* delta_incl, unsigned int* flag_words, unsigned int* delta_words, void* stream);
-int skml_da_fixed_iv(const unsigned int* flag_words, long long n, int flag_bits_per_key, int* iv, void* stream);
-int skml_da_zero_count(const unsigned int* flag_words, long long flag_bits, int* zeros, void* stream);
-int skml_da_zero_pos(const unsigned int* flag_words, long long flag_bits, const long long* zeros_incl, long long n,
-                     long long* pos, void* stream);
-int skml_da_extract(const unsigned int* delta_words, long long n, const int* delta_w, const long long* delta_incl,
-                    long long* deltas, void* stream);
+// DeltaAdaptive key codec, stand-alone (csrc/cuda/keys_kernels.cu). skml_da_plan decides the mode and the stream
+// lengths and returns once they are known, in `done` (8 pinned host words): done[1] = interval count | (1 for
+// unary flags) << 32, done[2] / done[3] = flag / delta bits; *status_out bit 0 = keys not strictly increasing
+// or negative. skml_da_pack then writes the streams, ceil(bits / 64) words each (clears them first), with the
+// plan's workspace. skml_da_decode inverts them; zero_pos: n entries of scratch, unary flags only.
+long long skml_da_workspace_bytes();
+int skml_da_plan(const int* keys, long long n, void* workspace, unsigned long long* done, unsigned int* status_out, void* stream);
+int skml_da_pack(const int* keys, long long n, const void* workspace, unsigned long long* flag_words, long long n_flag_words,
+                 unsigned long long* delta_words, long long n_delta_words, void* stream);
+int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,
+                   long long n_delta_words, long long n, int num_intervals, int unary, long long flag_bits, void* workspace,
+                   long long* zero_pos, int* keys, void* stream);
 
 // Expands a minibatch from its transport form (bit-packed column indices, 32-bit row pointers,
 // 8-bit labels; the latter two optional = null) into CSR arrays. `packed` must end with two

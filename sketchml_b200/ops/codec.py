@@ -35,9 +35,9 @@ class ExchangeRegionView:
         return FLAG_BYTES + 2 * world * slot_capacity
 
 
-class _DoneWords:
+class DoneWords:
     """Pinned host words for checked calls: one page for the process (pinning memory takes milliseconds), a word per
-    codec object, given back with it; an object that finds the page full pins a word of its own."""
+    codec object (its 64-byte line, eight words), given back with it; an object that finds the page full pins its own."""
     _WORDS = 512
     _lock = threading.Lock()
     _page: Optional[torch.Tensor] = None
@@ -50,10 +50,10 @@ class _DoneWords:
                 cls._page = torch.zeros(cls._WORDS * 8, dtype=torch.int64).pin_memory()
                 cls._free = list(range(cls._WORDS))
             if not cls._free:
-                return torch.zeros(1, dtype=torch.int64).pin_memory()
+                return torch.zeros(8, dtype=torch.int64).pin_memory()
             i = cls._free.pop()
         weakref.finalize(owner, cls._give_back, i)
-        return cls._page[8 * i:8 * i + 1]     # 64 bytes apart
+        return cls._page[8 * i:8 * i + 8]
 
     @classmethod
     def _give_back(cls, i: int) -> None:
@@ -67,7 +67,7 @@ class _Checked:
 
     def __init__(self, device):
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
-        self.word = _DoneWords.take(self)
+        self.word = DoneWords.take(self)
         self.out = C.c_uint(0)
         self.out_ref = C.byref(self.out)
 

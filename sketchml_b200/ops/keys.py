@@ -6,17 +6,20 @@ variable-width bit code for sorted keys. The training step does not come through
 themselves, chunk by chunk, without leaving the device (csrc/cuda/compress_kernels.cu,
 decode_common.cuh). This module is the library form of the codec, `encode(keys) -> AdaptiveKeys`
 and back, bit for bit equal to the CPU oracle (`oracle.delta_adaptive_encode`). It returns tensors
-of exactly the encoded size, which depends on the data, so `encode` reads the status, the chosen
-mode and the two bit counts back to the host in one copy; the kernels are maps over keys or words
-(csrc/cuda/keys_kernels.cu) with `torch.cumsum` between them.
+of exactly the encoded size, which depends on the data, so `encode` waits once, for the mode and the
+two bit counts (they come through a pinned host word); csrc/cuda/keys_kernels.cu has the kernels.
 """
 from __future__ import annotations
 
+import ctypes as C
+import threading
 from dataclasses import dataclass
+from typing import Optional
 
 import torch
 
 from . import lib as L
+from .codec import DoneWords
 
 
 @dataclass
@@ -40,9 +43,25 @@ class AdaptiveKeys:
         return 4 + 4 + 1 + 4 + 8 * self.flag_words.numel() + 4 + 8 * self.delta_words.numel()
 
 
-def _words(bits: int, device) -> torch.Tensor:
-    # 64-bit words plus one spare: readers fetch the 32-bit word after the one a value starts in
-    return torch.zeros((bits + 63) // 64 + 1, dtype=torch.int64, device=device)
+class _CallState(threading.local):
+    """Per thread: the pinned words a call's plan comes back in."""
+
+    def __init__(self):
+        self.words = DoneWords.take(self)
+        self.status = C.c_uint(0)
+        self.status_ref = C.byref(self.status)
+
+
+_call: Optional[_CallState] = None
+_workspace_bytes = 0
+
+
+def _call_state() -> _CallState:
+    global _call, _workspace_bytes
+    if _call is None:
+        _workspace_bytes = int(L.lib().skml_da_workspace_bytes())
+        _call = _CallState()
+    return _call
 
 
 def encode(keys: torch.Tensor) -> AdaptiveKeys:
@@ -50,27 +69,19 @@ def encode(keys: torch.Tensor) -> AdaptiveKeys:
     if keys.dtype != torch.int32 or not keys.is_cuda:
         raise ValueError("keys must be a CUDA int32 tensor")
     keys = keys.contiguous()
-    n, dev, lib = keys.numel(), keys.device, L.lib()
-    hist = torch.zeros(32, dtype=torch.int32, device=dev)
-    params = torch.zeros(2, dtype=torch.int32, device=dev)
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
-    L.check(lib.skml_da_analyze(L.ptr(keys), n, L.ptr(hist), L.ptr(params), L.ptr(status), L.stream()), "skml_da_analyze")
-    flag_w = torch.zeros(max(n, 1), dtype=torch.int32, device=dev)
-    delta_w = torch.zeros(max(n, 1), dtype=torch.int32, device=dev)
-    L.check(lib.skml_da_widths(L.ptr(keys), n, L.ptr(params), L.ptr(flag_w), L.ptr(delta_w), L.stream()), "skml_da_widths")
-    flag_incl = torch.cumsum(flag_w[:n], 0, dtype=torch.int64) if n else torch.zeros(0, dtype=torch.int64, device=dev)
-    delta_incl = torch.cumsum(delta_w[:n], 0, dtype=torch.int64) if n else torch.zeros(0, dtype=torch.int64, device=dev)
-    # the one read-back of the call: status, mode and the two stream lengths together
-    zero = torch.zeros(1, dtype=torch.int64, device=dev)
-    st, m, kind, flag_bits, delta_bits = (int(x) for x in torch.cat(
-        [status.long(), params.long(), flag_incl[-1:] if n else zero, delta_incl[-1:] if n else zero]).tolist())
-    if st & 1:
+    n, dev, lib, cs = keys.numel(), keys.device, L.lib(), _call_state()
+    stream = L.stream()
+    work = torch.empty(_workspace_bytes, dtype=torch.uint8, device=dev)
+    L.check(lib.skml_da_plan(keys.data_ptr(), n, work.data_ptr(), cs.words.data_ptr(), cs.status_ref, stream), "skml_da_plan")
+    if cs.status.value & 1:
         raise ValueError("keys must be non-negative and strictly increasing")
-    fw, dw = _words(flag_bits, dev), _words(delta_bits, dev)
-    L.check(lib.skml_da_pack(L.ptr(keys), n, L.ptr(params), L.ptr(flag_incl), L.ptr(delta_incl), L.ptr(fw), L.ptr(dw),
-                             L.stream()), "skml_da_pack")
-    L.count_launches(4 if n else 1)
-    return AdaptiveKeys(n, m, kind, flag_bits, delta_bits, fw[:(flag_bits + 63) // 64], dw[:(delta_bits + 63) // 64])
+    _, mode, flag_bits, delta_bits = cs.words[:4].tolist()
+    nf, nd = (flag_bits + 63) // 64, (delta_bits + 63) // 64
+    words = torch.empty(nf + nd, dtype=torch.int64, device=dev)
+    fw, dw = words[:nf], words[nf:]
+    L.check(lib.skml_da_pack(keys.data_ptr(), n, work.data_ptr(), fw.data_ptr(), nf, dw.data_ptr(), nd, stream), "skml_da_pack")
+    L.count_launches(2 if n else 1)
+    return AdaptiveKeys(n, mode & 0xFFFFFFFF, mode >> 32, flag_bits, delta_bits, fw, dw)
 
 
 def decode(e: AdaptiveKeys) -> torch.Tensor:
@@ -78,28 +89,12 @@ def decode(e: AdaptiveKeys) -> torch.Tensor:
     dev, lib, n = e.delta_words.device, L.lib(), e.size
     if n == 0:
         return torch.zeros(0, dtype=torch.int32, device=dev)
-    pad = torch.zeros(1, dtype=torch.int64, device=dev)
-    fw = torch.cat([e.flag_words.to(torch.int64), pad]).contiguous()
-    dw = torch.cat([e.delta_words.to(torch.int64), pad]).contiguous()
-    b = 32 // e.num_intervals
-    if e.flag_kind == 0:
-        fb = e.num_intervals.bit_length() - 1
-        iv = torch.zeros(n, dtype=torch.int32, device=dev)
-        L.check(lib.skml_da_fixed_iv(L.ptr(fw), n, fb, L.ptr(iv), L.stream()), "skml_da_fixed_iv")
-        L.count_launches(1)
-    else:
-        nw = (e.flag_bits + 31) // 32
-        zeros = torch.zeros(max(nw, 1), dtype=torch.int32, device=dev)
-        L.check(lib.skml_da_zero_count(L.ptr(fw), e.flag_bits, L.ptr(zeros), L.stream()), "skml_da_zero_count")
-        zeros_incl = torch.cumsum(zeros, 0, dtype=torch.int64)
-        pos = torch.full((n,), -1, dtype=torch.int64, device=dev)
-        L.check(lib.skml_da_zero_pos(L.ptr(fw), e.flag_bits, L.ptr(zeros_incl), n, L.ptr(pos), L.stream()), "skml_da_zero_pos")
-        L.count_launches(2)
-        prev = torch.cat([pos.new_full((1,), -1), pos[:-1]])
-        iv = (pos - prev - 1).to(torch.int32)
-    delta_w = (iv * b).contiguous()
-    delta_incl = torch.cumsum(delta_w, 0, dtype=torch.int64)
-    deltas = torch.zeros(n, dtype=torch.int64, device=dev)
-    L.check(lib.skml_da_extract(L.ptr(dw), n, L.ptr(delta_w), L.ptr(delta_incl), L.ptr(deltas), L.stream()), "skml_da_extract")
-    L.count_launches(1)
-    return torch.cumsum(deltas, 0).to(torch.int32)
+    _call_state()
+    fw, dw = e.flag_words.to(torch.int64).contiguous(), e.delta_words.to(torch.int64).contiguous()
+    keys = torch.empty(n, dtype=torch.int32, device=dev)
+    work = torch.empty(_workspace_bytes, dtype=torch.uint8, device=dev)
+    pos = torch.empty(n, dtype=torch.int64, device=dev) if e.flag_kind else None
+    L.check(lib.skml_da_decode(fw.data_ptr(), fw.numel(), dw.data_ptr(), dw.numel(), n, e.num_intervals, e.flag_kind, e.flag_bits,
+                               work.data_ptr(), L.ptr(pos), keys.data_ptr(), L.stream()), "skml_da_decode")
+    L.count_launches(5 if e.flag_kind else 3)
+    return keys

@@ -546,3 +546,56 @@ def test_sampled_splits_are_the_sample_s_order_statistics(n, q):
         pr = oracle.parse(ref)
         for a, b in zip(_sections(p), _sections(pr)):
             assert a == b
+
+
+@pytest.mark.parametrize("n,bins,spread", [
+    (16384, 256, 2000), (16385, 257, 2000), (20000, 256, 1), (40000, 8190, 2000), (40000, 4097, 3), (700001, 64, 2000),
+    (2500000, 16, 50), (1300001, 2, 2000)])
+def test_zipml_split_search_over_its_splits_of_the_work(n, bins, spread):
+    """Edges of the split search: the largest search of one block and the smallest of several, keys in registers
+    and in memory, few blocks (many kept pairs) and many, and inputs where most errors tie."""
+    from sketchml_b200.compress import oracle
+    rng = np.random.default_rng(n + bins)
+    vals = (rng.integers(-spread, spread + 1, n) / 1024.0).astype(np.float32)   # exact sums, as above
+    ref = oracle.zipml_quantize(vals.astype(np.float64), bins)
+    zc, v, cnt, nb, zero, rounds, splits, mids, codes = _zip_pack(vals, bins)
+    assert nb == ref["bin_num"] and zero == ref["zero_idx"]
+    assert np.array_equal(splits.astype(np.float64), ref["splits"])
+    assert np.array_equal(mids, ref["values"].astype(np.float32))
+    assert np.array_equal(codes, ref["bins"])
+    zc.pack(v, cnt)    # the words the blocks share are ready for the next call
+    assert int(zc.meta[0]) == nb
+
+
+@pytest.mark.parametrize("n,bins", [(5000, 16), (16000, 256), (20000, 256), (40000, 16), (120000, 256), (120000, 1000)])
+def test_zipml_split_search_on_distinct_errors(n, bins):
+    """Continuous values: no two errors of a round tie, and all the largest ones differ by far more than the
+    rounding of the prefix sums, so the first rounds must keep exactly the oracle's pairs; later ones may differ
+    where a choice hangs on that rounding."""
+    from sketchml_b200.compress import oracle
+    vals = (np.random.default_rng(n).standard_t(3, n) * 1e-3).astype(np.float32)
+    ref = oracle.zipml_quantize(vals.astype(np.float64), bins)
+    zc, v, cnt, nb, zero, rounds, splits, mids, codes = _zip_pack(vals, bins)
+    same = len(np.intersect1d(splits.astype(np.float64), ref["splits"]))
+    assert same >= 0.95 * len(ref["splits"]), (same, len(ref["splits"]))
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 592 * 1024, 592 * 1024 + 1, 1_300_000])
+@pytest.mark.parametrize("gaps", ["ones", "mixed", "wide"])
+def test_delta_adaptive_device_codec_over_its_runs(n, gaps):
+    """Edges of the runs of tiles: less than a tile, exactly one, one run per block full, the first size with two
+    tiles a run; fixed and unary flags."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import keys as K
+    rng = np.random.default_rng(n)
+    d = {"ones": np.ones(n, np.int64), "mixed": np.where(rng.random(n) < 0.9, 1, rng.integers(1, 9000, n)),
+         "wide": rng.integers(1, max(2, (2 ** 31 - 2) // n), n)}[gaps]
+    keys = np.cumsum(d).astype(np.int32)
+    ref = oracle.delta_adaptive_encode(keys)
+    got = K.encode(torch.from_numpy(keys).cuda())
+    assert (got.num_intervals, got.flag_kind, got.flag_bits, got.delta_bits) == (
+        ref["num_intervals"], ref["flag_kind"], ref["flag_bits"], ref["delta_bits"])
+    o = got.to_oracle_dict()
+    assert np.array_equal(o["flag_words"], np.asarray(ref["flag_words"], dtype=np.uint64))
+    assert np.array_equal(o["delta_words"], np.asarray(ref["delta_words"], dtype=np.uint64))
+    assert np.array_equal(K.decode(got).cpu().numpy(), keys)
