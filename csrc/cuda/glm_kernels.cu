@@ -68,15 +68,13 @@ struct GradSmem {
     uint64_t bar[2];
 };
 
-// MODE 0: training (scatter), MODE 1: validation (loss + confusion counts only),
-// MODE 2: per-row coefficients only (the scatter is done by the transposed-index kernels)
-template <int MODE>
+// Training with a scatter: margin, loss, coefficient, coefficient * feature into the accumulator.
 __global__ void __launch_bounds__(GRAD_THREADS)
 glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
                 const float* __restrict__ labels, long long row_lo, long long row_cnt, int rows_per_tile,
                 long long nnz_padded, const float* __restrict__ w, float* __restrict__ g,
                 unsigned int* __restrict__ bitmap, int loss_id, float inv_batch, int hot, double* __restrict__ acc,
-                float* __restrict__ margins, unsigned int* status, long long budget) {
+                unsigned int* status, long long budget) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // layout: [2 stages x cols][2 stages x vals, only if the shard stores values][hot floats]
     __shared__ GradSmem sb;
@@ -90,10 +88,8 @@ glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ co
     const int priv = hot < GRAD_PRIV ? hot : GRAD_PRIV;  // columns [0, priv): per-warp private sums
     float* s_priv = s_hot + hot;
 
-    if (MODE == 0) {
-        for (int i = threadIdx.x; i < hot; i += blockDim.x) s_hot[i] = 0.f;
-        for (int i = threadIdx.x; i < priv * GRAD_WARPS; i += blockDim.x) s_priv[i] = 0.f;
-    }
+    for (int i = threadIdx.x; i < hot; i += blockDim.x) s_hot[i] = 0.f;
+    for (int i = threadIdx.x; i < priv * GRAD_WARPS; i += blockDim.x) s_priv[i] = 0.f;
     if (threadIdx.x == 0) {
         mbar_init(&sb.bar[0], 1);
         mbar_init(&sb.bar[1], 1);
@@ -103,7 +99,6 @@ glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ co
 
     const long long ntiles = (row_cnt + rows_per_tile - 1) / rows_per_tile;
     double loss_sum = 0.0;
-    unsigned int tp = 0, tn = 0, fp = 0, fn = 0;
     unsigned int phase[2] = {0, 0};
 
     // Issues the bulk copies of one tile into `stage`; returns false when the tile does
@@ -187,7 +182,7 @@ glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ co
                 for (int u = 0; u < GRAD_RPI; ++u) sum[u] += __shfl_xor_sync(0xFFFFFFFFu, sum[u], o);
             }
             // Loss and coefficient of the GRAD_RPI rows are evaluated once, by lanes 0..GRAD_RPI-1 in
-            // parallel (lane u owns row rb + u); the scatter mode then broadcasts the coefficients.
+            // parallel (lane u owns row rb + u) and then broadcast.
             float pre_mine = sum[0];
 #pragma unroll
             for (int u = 1; u < GRAD_RPI; ++u) pre_mine = lane == u ? sum[u] : pre_mine;
@@ -195,75 +190,150 @@ glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ co
             if (lane < GRAD_RPI && rb + lane < nrows) {
                 const float y = s_lab[rb + lane];
                 loss_sum += (double)glm_loss(loss_id, pre_mine, y);
-                if (MODE == 0 || MODE == 2) {
-                    coef_mine = -glm_grad(loss_id, pre_mine, y) * inv_batch;
-                    if (MODE == 2) margins[r0 - row_lo + rb + lane] = coef_mine;  // coefficient per row, no scatter
-                } else {
-                    const float z = pre_mine * y;
-                    if (z > 0.f) {
-                        if (pre_mine > 0.f) ++tp; else ++tn;
-                    } else if (z < 0.f) {
-                        if (pre_mine > 0.f) ++fp; else ++fn;
-                    }
-                    if (margins) margins[r0 - row_lo + rb + lane] = pre_mine;
-                }
+                coef_mine = -glm_grad(loss_id, pre_mine, y) * inv_batch;
             }
             float coef[GRAD_RPI];
 #pragma unroll
-            for (int u = 0; u < GRAD_RPI; ++u) coef[u] = MODE == 0 ? __shfl_sync(0xFFFFFFFFu, coef_mine, u) : 0.f;
-            if (MODE == 0) {
-                for (int off = lane; off - lane < maxlen; off += 32) {
-                    int c[GRAD_RPI];
-                    float contrib[GRAD_RPI];
-                    unsigned int seen[GRAD_RPI];
+            for (int u = 0; u < GRAD_RPI; ++u) coef[u] = __shfl_sync(0xFFFFFFFFu, coef_mine, u);
+            for (int off = lane; off - lane < maxlen; off += 32) {
+                int c[GRAD_RPI];
+                float contrib[GRAD_RPI];
+                unsigned int seen[GRAD_RPI];
 #pragma unroll
-                    for (int u = 0; u < GRAD_RPI; ++u) {
-                        const bool ok = off < len[u] && coef[u] != 0.f;
-                        c[u] = ok ? cp[e0[u] + off] : -1;
-                        contrib[u] = ok ? coef[u] * (vp ? vp[e0[u] + off] : 1.f) : 0.f;
-                    }
-                    // cold columns: read the bitmap words first (independent L2 loads), so that
-                    // the atomicOr is only issued for bits that are not set yet
-#pragma unroll
-                    for (int u = 0; u < GRAD_RPI; ++u)
-                        seen[u] = (bitmap && c[u] >= hot) ? *(volatile unsigned int*)(bitmap + (c[u] >> 5)) : ~0u;  // no bitmap: nothing to mark
-#pragma unroll
-                    for (int u = 0; u < GRAD_RPI; ++u) {
-                        if (c[u] < 0) continue;
-                        if (c[u] < priv) {
-                            // the hottest columns: one private copy per warp. The lanes of a row hold
-                            // distinct columns and a warp's shared-memory accesses are ordered, so a
-                            // plain read-modify-write is exact and free of atomics.
-                            s_priv[warp * priv + c[u]] += contrib[u];
-                        } else if (c[u] < hot) {
-                            atomicAdd(&s_hot[c[u]], contrib[u]);
-                        } else {
-                            red_add_f32(g + c[u], contrib[u]);
-                            const unsigned int bit = 1u << (c[u] & 31);
-                            if (!(seen[u] & bit)) atomicOr(bitmap + (c[u] >> 5), bit);
-                        }
-                    }
-                    __syncwarp();
+                for (int u = 0; u < GRAD_RPI; ++u) {
+                    const bool ok = off < len[u] && coef[u] != 0.f;
+                    c[u] = ok ? cp[e0[u] + off] : -1;
+                    contrib[u] = ok ? coef[u] * (vp ? vp[e0[u] + off] : 1.f) : 0.f;
                 }
+                // cold columns: read the bitmap words first (independent L2 loads), so that
+                // the atomicOr is only issued for bits that are not set yet
+#pragma unroll
+                for (int u = 0; u < GRAD_RPI; ++u)
+                    seen[u] = (bitmap && c[u] >= hot) ? *(volatile unsigned int*)(bitmap + (c[u] >> 5)) : ~0u;  // no bitmap: nothing to mark
+#pragma unroll
+                for (int u = 0; u < GRAD_RPI; ++u) {
+                    if (c[u] < 0) continue;
+                    if (c[u] < priv) {
+                        // the hottest columns: one private copy per warp. The lanes of a row hold
+                        // distinct columns and a warp's shared-memory accesses are ordered, so a
+                        // plain read-modify-write is exact and free of atomics.
+                        s_priv[warp * priv + c[u]] += contrib[u];
+                    } else if (c[u] < hot) {
+                        atomicAdd(&s_hot[c[u]], contrib[u]);
+                    } else {
+                        red_add_f32(g + c[u], contrib[u]);
+                        const unsigned int bit = 1u << (c[u] & 31);
+                        if (!(seen[u] & bit)) atomicOr(bitmap + (c[u] >> 5), bit);
+                    }
+                }
+                __syncwarp();
             }
         }
         __syncthreads();  // everyone is done with `stage` (and s_rp / s_lab) before it is refilled
     }
 
-    if (MODE == 0) {
-        for (int i = threadIdx.x; i < priv; i += blockDim.x) {
-            float t = s_hot[i];
-            for (int w2 = 0; w2 < GRAD_WARPS; ++w2) t += s_priv[w2 * priv + i];
-            s_hot[i] = t;
-        }
-        __syncthreads();
-        // flush the hot columns: one red.add per non-zero entry, one atomicOr per 32 columns
-        for (int base = warp * 32; base < hot; base += GRAD_WARPS * 32) {
-            int i = base + lane;
-            float v = i < hot ? s_hot[i] : 0.f;
-            unsigned int m = __ballot_sync(0xFFFFFFFFu, v != 0.f);
-            if (v != 0.f) red_add_f32(g + i, v);
-            if (bitmap && lane == 0 && m) atomicOr(bitmap + (base >> 5), m);
+    for (int i = threadIdx.x; i < priv; i += blockDim.x) {
+        float t = s_hot[i];
+        for (int w2 = 0; w2 < GRAD_WARPS; ++w2) t += s_priv[w2 * priv + i];
+        s_hot[i] = t;
+    }
+    __syncthreads();
+    // flush the hot columns: one red.add per non-zero entry, one atomicOr per 32 columns
+    for (int base = warp * 32; base < hot; base += GRAD_WARPS * 32) {
+        int i = base + lane;
+        float v = i < hot ? s_hot[i] : 0.f;
+        unsigned int m = __ballot_sync(0xFFFFFFFFu, v != 0.f);
+        if (v != 0.f) red_add_f32(g + i, v);
+        if (bitmap && lane == 0 && m) atomicOr(bitmap + (base >> 5), m);
+    }
+    double tot = block_sum_double(loss_sum);
+    if (threadIdx.x == 0 && tot != 0.0) atomicAdd(&acc[0], tot);
+}
+
+// Margins without a scatter. MODE 1: validation (loss + confusion counts), MODE 2: per-row coefficients (the
+// gradient is summed per column by the transposed-index kernels).
+// A warp takes up to 32 consecutive rows, 32 >> GL of them at a time (`iters` times) with 1 << GL lanes each; every
+// row's sum ends up in the lane that owns the row, so loss and coefficient are evaluated for all of them at once.
+// What bounds it is the number of gathers of w: a fully divergent load takes a cycle of the L1 per lane even when
+// it hits and an L1 line while it misses, so the weights of the first `hot` columns (the frequent ones where
+// indices are assigned by frequency) are kept in shared memory, which serves some ten lanes a cycle, and nothing
+// is staged that would take L1 away. 500,000 rows of 30: 80 -> 73 us; 1M rows of 30 with values: 208 -> 109 us
+// (before: a warp per row, tiles staged by bulk copies, 103 warp instructions per 32 entries).
+#define MARGIN_THREADS 512
+template <int MODE, int GL, bool HAS_VALS>
+__global__ void __launch_bounds__(MARGIN_THREADS, 3)
+glm_margin_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
+                  const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
+                  int hot, int loss_id, float inv_batch, double* __restrict__ acc, float* __restrict__ out) {
+    extern __shared__ __align__(16) float s_w[];
+    constexpr int LANES = 1 << GL, ROWS = 32 >> GL, PER = 4;   // rows of an iteration, entries of a lane in flight
+    const int lane = threadIdx.x & 31, sub = lane & (LANES - 1), grp = lane >> GL;
+    for (int i = threadIdx.x; i < hot / 4; i += blockDim.x) reinterpret_cast<float4*>(s_w)[i] = __ldg(reinterpret_cast<const float4*>(w) + i);
+    __syncthreads();
+    const int bundle = ROWS * iters;   // rows of a warp's turn
+    const long long bundles = (row_cnt + bundle - 1) / bundle, stride = (long long)gridDim.x * (blockDim.x / 32);
+    double loss_sum = 0.0;
+    unsigned int tp = 0, tn = 0, fp = 0, fn = 0;
+    for (long long b = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); b < bundles; b += stride) {
+        const long long r0 = b * bundle;   // within the batch
+        const int nrows = row_cnt - r0 < bundle ? (int)(row_cnt - r0) : bundle;
+        const long long e_mine = rowptr[row_lo + r0 + (lane < nrows ? lane : nrows)];
+        const long long e_end = rowptr[row_lo + r0 + nrows];
+        const int my_row = sub * ROWS + grp;   // the row this lane evaluates
+        const float y = my_row < nrows ? labels[row_lo + r0 + my_row] : 0.f;
+        const long long base = __shfl_sync(0xFFFFFFFFu, e_mine, 0);
+        const long long span = e_end - base;
+        float pre = 0.f;
+        auto row_sums = [&](auto off_of) {   // offsets inside the bundle in 32 bits where they fit
+            using T = decltype(off_of(0ll));
+            const T mine = off_of(e_mine - base), last = off_of(span);
+            const int* __restrict__ cp = cols + base;
+            const float* __restrict__ vp = HAS_VALS ? vals + base : nullptr;
+#pragma unroll 2
+            for (int i = 0; i < iters; ++i) {
+                const int row = i * ROWS + grp;
+                const T lo = __shfl_sync(0xFFFFFFFFu, mine, row), nx = __shfl_sync(0xFFFFFFFFu, mine, (row + 1) & 31);
+                const T hi = row + 1 < 32 ? nx : last;   // rows from nrows on are empty: every later offset is the end
+                float sum = 0.f;
+                for (T k = lo + sub; k < hi; k += PER * LANES) {
+                    int c[PER];
+                    float x[PER], wv[PER];
+#pragma unroll
+                    for (int u = 0; u < PER; ++u) {
+                        const bool ok = k + u * LANES < hi;
+                        c[u] = ok ? __ldcs(cp + k + u * LANES) : -1;
+                        x[u] = HAS_VALS ? (ok ? __ldcs(vp + k + u * LANES) : 0.f) : 1.f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < PER; ++u) {
+                        wv[u] = 0.f;
+                        if (c[u] >= hot) wv[u] = __ldg(w + c[u]);
+                        else if (c[u] >= 0) wv[u] = s_w[c[u]];
+                    }
+#pragma unroll
+                    for (int u = 0; u < PER; ++u) sum = fmaf(wv[u], x[u], sum);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+                if (sub == i) pre = sum;
+            }
+        };
+        if (span < (1ll << 30)) row_sums([](long long v) { return (int)v; });
+        else row_sums([](long long v) { return v; });
+        if (my_row < nrows) {
+            loss_sum += (double)glm_loss(loss_id, pre, y);
+            if (MODE == 2) {
+                out[r0 + my_row] = -glm_grad(loss_id, pre, y) * inv_batch;
+            } else {
+                const float z = pre * y;
+                if (z > 0.f) {
+                    if (pre > 0.f) ++tp; else ++tn;
+                } else if (z < 0.f) {
+                    if (pre > 0.f) ++fp; else ++fn;
+                }
+                if (out) out[r0 + my_row] = pre;
+            }
         }
     }
     double tot = block_sum_double(loss_sum);
@@ -291,15 +361,61 @@ static int sm_count() {
     return g_sm_count;
 }
 
-static int grad_launch(int mode, const long long* rowptr, const int* cols, const float* vals, const float* labels,
+// Columns [0, margin_hot) of w in shared memory: at most 8192 (32 KB, three blocks an SM keep 128 KB of L1), no more
+// than a block has entries to look up (reading them in is then an eighth of the sectors of the gathers at most),
+// whole 16-byte units. Below 1024 the copy is not worth its barrier.
+static int margin_hot(long long entries, long long blocks, long long dim, const float* w) {
+    long long hot = entries / (blocks > 0 ? blocks : 1);
+    if (hot > 8192) hot = 8192;
+    if (hot > dim) hot = dim;
+    hot &= ~255ll;
+    return hot < 1024 || ((uintptr_t)w & 15) ? 0 : (int)hot;
+}
+
+template <int MODE, int GL>
+static int margin_launch_gl(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
+                            long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
+                            float* out, cudaStream_t stream) {
+    // rows of a warp's turn: as many as leave every warp slot of the chip (three blocks of 16 warps an SM) a turn,
+    // down to one trip; then blocks of as many warps as spread the turns over all SMs
+    const long long slots = 3ll * sm_count() * (MARGIN_THREADS / 32), rows = 32 >> GL;
+    long long iters = row_cnt / (rows * slots);
+    if (iters < 1) iters = 1;
+    if (iters > (1 << GL)) iters = 1 << GL;
+    const long long bundles = (row_cnt + rows * iters - 1) / (rows * iters);
+    long long warps = (bundles + 3ll * sm_count() - 1) / (3ll * sm_count());
+    if (warps > MARGIN_THREADS / 32) warps = MARGIN_THREADS / 32;
+    long long grid = (bundles + warps - 1) / warps;
+    if (grid > 3ll * sm_count()) grid = 3ll * sm_count();
+    const int hot = margin_hot((long long)(row_cnt * avg_nnz), grid, dim, w);
+    if (vals)
+        glm_margin_kernel<MODE, GL, true><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
+            rowptr, cols, vals, labels, row_lo, row_cnt, (int)iters, w, hot, loss_id, inv_batch, acc, out);
+    else
+        glm_margin_kernel<MODE, GL, false><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
+            rowptr, cols, vals, labels, row_lo, row_cnt, (int)iters, w, hot, loss_id, inv_batch, acc, out);
+    return (int)cudaGetLastError();
+}
+
+// Lanes per row: four entries of a lane are in flight at a time, so a row of the average length takes one trip.
+template <int MODE>
+static int margin_launch(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
+                         long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
+                         float* out, cudaStream_t stream) {
+    if (row_cnt <= 0) return 0;
+    auto go = avg_nnz <= 16.0 ? margin_launch_gl<MODE, 2> : avg_nnz <= 40.0 ? margin_launch_gl<MODE, 3>
+            : avg_nnz <= 96.0 ? margin_launch_gl<MODE, 4> : margin_launch_gl<MODE, 5>;
+    return go(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, inv_batch, acc, out, stream);
+}
+
+static int grad_launch(const long long* rowptr, const int* cols, const float* vals, const float* labels,
                        long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz, const float* w,
                        float* g, unsigned int* bitmap, int loss_id, float inv_batch, int hot, double* acc,
-                       float* margins, unsigned int* status, long long budget, cudaStream_t stream) {
+                       unsigned int* status, long long budget, cudaStream_t stream) {
     if (row_cnt <= 0) return 0;
     if (hot < 0) hot = 0;
     if (hot > 16384) hot = 16384;
     hot &= ~31;
-    if (mode != 0) hot = 0;
     int rpt = (int)(GRAD_TILE_CAP * 0.8 / (avg_nnz > 1.0 ? avg_nnz : 1.0));
     if (rpt < 1) rpt = 1;
     if (rpt > GRAD_MAX_RPT) rpt = GRAD_MAX_RPT;
@@ -309,25 +425,13 @@ static int grad_launch(int mode, const long long* rowptr, const int* cols, const
     int per_sm = smem > 100 * 1024 ? 1 : (smem > 70 * 1024 ? 2 : 3);
     long long grid = (long long)sm_count() * per_sm;
     if (grid > ntiles) grid = ntiles;
-    static bool attr_set[2] = {false, false};
-    if (!attr_set[0]) {
-        cudaFuncSetAttribute(glm_rows_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(glm_rows_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(glm_rows_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_set[0] = attr_set[1] = true;
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaFuncSetAttribute(glm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        attr_set = true;
     }
-    if (mode == 0)
-        glm_rows_kernel<0><<<(unsigned)grid, GRAD_THREADS, smem, stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, rpt, nnz_padded, w, g, bitmap, loss_id, inv_batch, hot, acc,
-            margins, status, budget);
-    else if (mode == 1)
-        glm_rows_kernel<1><<<(unsigned)grid, GRAD_THREADS, smem, stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, rpt, nnz_padded, w, g, bitmap, loss_id, inv_batch, hot, acc,
-            margins, status, budget);
-    else
-        glm_rows_kernel<2><<<(unsigned)grid, GRAD_THREADS, smem, stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, rpt, nnz_padded, w, g, bitmap, loss_id, inv_batch, hot, acc,
-            margins, status, budget);
+    glm_rows_kernel<<<(unsigned)grid, GRAD_THREADS, smem, stream>>>(
+        rowptr, cols, vals, labels, row_lo, row_cnt, rpt, nnz_padded, w, g, bitmap, loss_id, inv_batch, hot, acc, status, budget);
     return (int)cudaGetLastError();
 }
 
@@ -335,16 +439,18 @@ extern "C" int skml_glm_grad(const long long* rowptr, const int* cols, const flo
                              long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz,
                              const float* w, float* g, unsigned int* bitmap, int loss_id, float inv_batch, int hot,
                              double* loss_acc, unsigned int* status, long long budget, void* stream) {
-    return grad_launch(0, rowptr, cols, vals, labels, row_lo, row_cnt, nnz_padded, avg_nnz, w, g, bitmap, loss_id,
-                       inv_batch, hot, loss_acc, nullptr, status, budget, (cudaStream_t)stream);
+    return grad_launch(rowptr, cols, vals, labels, row_lo, row_cnt, nnz_padded, avg_nnz, w, g, bitmap, loss_id,
+                       inv_batch, hot, loss_acc, status, budget, (cudaStream_t)stream);
 }
 
 extern "C" int skml_glm_validate(const long long* rowptr, const int* cols, const float* vals, const float* labels,
                                  long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz,
-                                 const float* w, int loss_id, double* acc5, float* margins, unsigned int* status,
+                                 const float* w, long long dim, int loss_id, double* acc5, float* margins, unsigned int* status,
                                  long long budget, void* stream) {
-    return grad_launch(1, rowptr, cols, vals, labels, row_lo, row_cnt, nnz_padded, avg_nnz, w, nullptr, nullptr,
-                       loss_id, 1.f, 0, acc5, margins, status, budget, (cudaStream_t)stream);
+    (void)nnz_padded;
+    (void)status;
+    (void)budget;   // nothing in it waits
+    return margin_launch<1>(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, 1.f, acc5, margins, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -1010,10 +1116,13 @@ colsum_kernel(const int* __restrict__ colptr, const int* __restrict__ rowidx, co
 
 extern "C" int skml_glm_coef(const long long* rowptr, const int* cols, const float* vals, const float* labels,
                              long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz,
-                             const float* w, int loss_id, float inv_batch, double* loss_acc, float* coef_out,
+                             const float* w, long long dim, int loss_id, float inv_batch, double* loss_acc, float* coef_out,
                              unsigned int* status, long long budget, void* stream) {
-    return grad_launch(2, rowptr, cols, vals, labels, row_lo, row_cnt, nnz_padded, avg_nnz, w, nullptr, nullptr, loss_id,
-                       inv_batch, 0, loss_acc, coef_out, status, budget, (cudaStream_t)stream);
+    (void)nnz_padded;
+    (void)status;
+    (void)budget;   // nothing in it waits
+    return margin_launch<2>(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, inv_batch, loss_acc, coef_out,
+                            (cudaStream_t)stream);
 }
 
 // Local-id batches (streamed minibatches whose column indices were replaced on the host by their

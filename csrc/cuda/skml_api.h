@@ -111,7 +111,7 @@ int skml_glm_grad(const long long* rowptr, const int* cols, const float* vals, c
                   unsigned int* bitmap, int loss_id, float inv_batch, int hot, double* loss_acc, unsigned int* status,
                   long long budget, void* stream);
 int skml_glm_validate(const long long* rowptr, const int* cols, const float* vals, const float* labels,
-                      long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz, const float* w,
+                      long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz, const float* w, long long dim,
                       int loss_id, double* acc5, float* margins, unsigned int* status, long long budget, void* stream);
 int skml_compact(float* g, const float* w, unsigned int* bitmap, int dim, float lambda, unsigned int* block_counts,
                  long long* meta, int* keys, float* vals, float* dense_vals, long long capacity, unsigned int* status,
@@ -145,7 +145,7 @@ int skml_gen_rows(int* cols, float* vals, float* labels, long long row_offset, l
                   double s, int value_kind, int task, float noise, const float* wstar, unsigned long long seed,
                   void* stream);
 int skml_glm_coef(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
-                  long long row_cnt, long long nnz_padded, double avg_nnz, const float* w, int loss_id,
+                  long long row_cnt, long long nnz_padded, double avg_nnz, const float* w, long long dim, int loss_id,
                   float inv_batch, double* loss_acc, float* coef_out, unsigned int* status, long long budget,
                   void* stream);
 int skml_colsum(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,

@@ -23,7 +23,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         int rc = skml_step_prep(a->partials, a->partials_template, a->gvals, a->t_long_col, tiled ? 0 : (int)a->t_long, stream_);
         if (rc) return rc;
         rc = skml_glm_coef(a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->seg_cnt[0], a->nnz_padded,
-                               a->avg_nnz, a->w, (int)a->loss_id, (float)a->inv_batch, a->partials + 1, a->coef,
+                               a->avg_nnz, a->w, a->dim, (int)a->loss_id, (float)a->inv_batch, a->partials + 1, a->coef,
                                a->status, a->budget_cycles, stream_);
         if (rc) return rc;
         if (tiled)

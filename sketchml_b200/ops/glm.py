@@ -97,7 +97,7 @@ def glm_validate(csr: DeviceCSR, w: torch.Tensor, loss_id: int, status: torch.Te
     acc = torch.zeros(6, dtype=torch.float64, device=w.device)
     if csr.rows:
         L.check(L.lib().skml_glm_validate(L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), L.ptr(csr.labels), 0,
-                                          csr.rows, csr.nnz_padded, float(csr.avg_nnz), L.ptr(w), loss_id, L.ptr(acc),
+                                          csr.rows, csr.nnz_padded, float(csr.avg_nnz), L.ptr(w), w.numel(), loss_id, L.ptr(acc),
                                           L.ptr(margins), L.ptr(status), L.budget_cycles(budget_s), L.stream()),
                 "skml_glm_validate")
         L.count_launches(1)

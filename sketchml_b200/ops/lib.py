@@ -84,7 +84,7 @@ _SIGS = {
     "skml_decode_update": (c_int, [C.POINTER(DecodeArgs), c_vp]),
     "skml_glm_grad": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_vp, c_vp, c_int, c_f, c_int,
                               c_vp, c_vp, c_ll, c_vp]),
-    "skml_glm_validate": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_int, c_vp, c_vp, c_vp,
+    "skml_glm_validate": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_ll, c_int, c_vp, c_vp, c_vp,
                                   c_ll, c_vp]),
     "skml_compact": (c_int, [c_vp, c_vp, c_vp, c_int, c_f, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_vp, c_vp]),
     "skml_compact_blocks": (c_ll, [c_int]),
@@ -98,7 +98,7 @@ _SIGS = {
     "skml_update_gathered": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_int, c_f, c_int, c_f, c_f, c_int, c_vp]),
     "skml_gen_wstar": (c_int, [c_vp, c_ll, c_d, c_ull, c_vp]),
     "skml_gen_rows": (c_int, [c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_d, c_int, c_int, c_f, c_vp, c_ull, c_vp]),
-    "skml_glm_coef": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_int, c_f, c_vp, c_vp, c_vp, c_ll, c_vp]),
+    "skml_glm_coef": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_ll, c_int, c_f, c_vp, c_vp, c_vp, c_ll, c_vp]),
     "skml_colsum": (c_int, [c_vp] * 8 + [c_int] * 4 + [c_vp, c_vp, c_f, c_vp, c_vp]),
     "skml_sm_count": (c_int, []),
     "skml_da_workspace_bytes": (c_ll, []),

@@ -143,7 +143,7 @@ def glm_grad_transposed(csr: DeviceCSR, bi: BatchIndex, w: torch.Tensor, coef: t
     the objective loss sum is added into partials[1]."""
     lib = L.lib()
     L.check(lib.skml_glm_coef(L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), L.ptr(csr.labels), bi.lo, bi.rows,
-                              csr.nnz_padded, float(csr.avg_nnz), L.ptr(w), loss_id, 1.0 / max(1, bi.rows),
+                              csr.nnz_padded, float(csr.avg_nnz), L.ptr(w), w.numel(), loss_id, 1.0 / max(1, bi.rows),
                               partials.data_ptr() + 8, L.ptr(coef), L.ptr(status), L.budget_cycles(budget_s), L.stream()),
             "skml_glm_coef")
     if bi.tiled is not None:

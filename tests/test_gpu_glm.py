@@ -255,3 +255,49 @@ def test_compaction_over_its_splits(dim, density):
             assert torch.equal(st.keys[:n].cpu().long(), idx)
             assert torch.allclose(st.vals[:n].cpu(), v[idx], rtol=3e-7, atol=3e-7)
         assert float(st.g.abs().max()) == 0.0 and int(st.bitmap.abs().max()) == 0
+
+
+@pytest.mark.parametrize("rows", [1, 3, 31, 33, 1000, 30011])
+@pytest.mark.parametrize("nnz", [(0, 5), (1, 30), (20, 60), (90, 300)])
+@pytest.mark.parametrize("binary", [True, False])
+def test_margins_over_their_row_shapes(rows, nnz, binary):
+    """Lanes per row (by the average length), turns per warp (by the row count), empty rows, rows longer than a trip,
+    columns on both sides of the ones kept in shared memory: coefficients, loss and counts against fp64."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.models.loss import L2LogLoss
+    from sketchml_b200.ops import DeviceCSR, glm_validate
+    from sketchml_b200.ops import lib as L
+    dev, dim = torch.device("cuda"), 20000
+    gen = torch.Generator().manual_seed(rows + nnz[1])
+    cnt = torch.randint(nnz[0], nnz[1] + 1, (rows,), generator=gen)
+    rowptr = torch.zeros(rows + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(cnt, 0)
+    n = int(rowptr[-1])
+    cols = (torch.rand(n, generator=gen) ** 4 * dim).int().clamp_max(dim - 1)   # frequent low columns; repeats do no harm here
+    vals = None if binary else torch.randn(n, generator=gen)
+    labels = torch.where(torch.rand(rows, generator=gen) < 0.5, -1.0, 1.0)
+    m = CSRMatrix(rowptr, cols, vals, labels, dim)
+    w = torch.randn(dim, generator=gen) * 0.2
+    csr, wd = DeviceCSR(m, dev), w.to(dev)
+    loss = L2LogLoss(0.0)
+    pre = loss.predict(w.double(), m)
+    # a margin is a sum of k <= 300 fp32 products in some order: error <= k eps sum |products| <= 300 * 6e-8 * (300 * 4)
+    # in the worst case; the bound below takes the batch's largest row sum of |products|
+    prod = w.abs().double()[cols.long()] * (1.0 if binary else vals.abs().double())
+    row_abs = torch.zeros(rows, dtype=torch.float64).index_add_(0, torch.repeat_interleave(torch.arange(rows), cnt), prod)
+    tol = 300 * 6e-8 * float(row_abs.max()) + 1e-6
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    out = torch.empty(rows, device=dev)
+    acc = glm_validate(csr, wd, loss.loss_id, status, margins=out).cpu()
+    assert float((out.cpu().double() - pre).abs().max()) <= tol
+    assert abs(float(acc[0]) - float(loss.loss(pre, labels.double()).sum())) <= (tol + 1e-5) * rows
+    assert float(acc[1] + acc[2] + acc[3] + acc[4]) == rows - int((out == 0).sum()) and float(acc[5]) == rows
+    lo = min(rows - 1, 7)    # a batch that starts inside the shard
+    coef = torch.empty(rows, device=dev)
+    part = torch.zeros(1, dtype=torch.float64, device=dev)
+    L.check(L.lib().skml_glm_coef(L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), L.ptr(csr.labels), lo, rows - lo,
+                                  csr.nnz_padded, float(csr.avg_nnz), L.ptr(wd), dim, loss.loss_id, 0.5, L.ptr(part), L.ptr(coef),
+                                  L.ptr(status), L.budget_cycles(1.0), L.stream()), "coef")
+    want = -0.5 * loss.grad(pre, labels.double())[lo:]
+    assert float((coef[:rows - lo].cpu().double() - want).abs().max()) <= tol + 1e-6    # slope <= 1/4; __expf: a few ulp
+    assert abs(float(part) - float(loss.loss(pre, labels.double())[lo:].sum())) <= (tol + 1e-5) * rows
