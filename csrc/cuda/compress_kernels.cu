@@ -196,12 +196,13 @@ extern "C" long long skml_payload_capacity(long long n_max, long long dim, long 
 // ---------------------------------------------------------------------------
 // Per-warp scratch of the Huffman code construction.
 struct HufScratch {
-    unsigned int w[HUF_MAX_SYMS];         // leaf weights, ascending
-    unsigned int iw[HUF_MAX_SYMS];        // weights of the internal nodes, in creation order (ascending)
+    unsigned int cnt[HUF_MAX_SYMS];       // cells per symbol
+    unsigned int w[HUF_MAX_SYMS + 2];     // leaf weights, ascending; two more that are never the smaller ones
+    unsigned int iw[HUF_MAX_SYMS + 2];    // weights of the internal nodes, in creation order (ascending), likewise
     unsigned short ord[HUF_MAX_SYMS];     // symbol of the i-th lightest leaf
     unsigned short pl[HUF_MAX_SYMS];      // parent (internal node) of every leaf
     unsigned short pi[HUF_MAX_SYMS];      // parent of every internal node
-    unsigned char di[HUF_MAX_SYMS];       // depth of every internal node
+    unsigned int next[34];                // symbols per code length, then the next code word of every length
 };
 
 // The quantile stages (S1, S2) and the coding stage (S5) never hold data at the same time, so their
@@ -1418,38 +1419,6 @@ __device__ void push_bytes(const CP& p, unsigned long long lo, unsigned long lon
 
 __device__ __forceinline__ int da_bits_needed(unsigned int d) { return d == 0u ? 1 : 32 - __clz(d); }
 
-// The reference's mode search in the same double arithmetic, operation by operation (explicit
-// round-to-nearest intrinsics keep the compiler from fusing multiply-adds); hist[k] = keys needing k bits.
-__device__ void da_choose(const unsigned int* hist, unsigned int n, unsigned int& num, unsigned int& kind) {
-    double prob[32];
-    const double dn = (double)(n > 0 ? n : 1);
-    for (int k = 0; k < 32; ++k) prob[k] = __ddiv_rn((double)hist[k], dn);
-    double best = 32.0;
-    num = 1;
-    kind = 0;
-    for (int m = 2, lg = 1; m <= 16; m *= 2, ++lg) {
-        const int b = 32 / m;
-        double sum = 0.0;
-        for (int i = 0; i < m; ++i) {
-            double ip = 0.0;
-            for (int j = 0; j < b; ++j) ip = __dadd_rn(ip, prob[i * b + j]);
-            sum = __dadd_rn(sum, __dmul_rn((double)(i + 1), ip));
-        }
-        const double t1 = __dadd_rn(__dmul_rn(sum, (double)b), (double)lg);
-        if (t1 < best) {
-            best = t1;
-            num = (unsigned int)m;
-            kind = 0;
-        }
-        const double t2 = __dadd_rn(__dmul_rn(sum, (double)(b + 1)), 1.0);
-        if (t2 < best) {
-            best = t2;
-            num = (unsigned int)m;
-            kind = 1;
-        }
-    }
-}
-
 // Pass 0: histogram of the delta widths of this block's chunks, per group, added to the global one.
 __device__ void apack_histogram(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
     const Layout& L = s.lay;
@@ -1477,38 +1446,71 @@ __device__ __forceinline__ unsigned long long stream_bytes(unsigned long long bi
 // whole layout of the key sections is known here, before a single key is coded.
 __device__ void apack_choose(const CP& p, Smem& s) {
     Layout& L = s.lay;
-    if (threadIdx.x < p.G) {
-        const int g = threadIdx.x;
-        unsigned int h[32];
-        for (int k = 0; k < 32; ++k) h[k] = __ldcg(&p.key_hist[g * 32 + k]);
-        unsigned int num = 1, kind = 0;
-        da_choose(h, L.n_g[g], num, kind);
-        L.num_iv[g] = num;
-        L.flag_kind[g] = kind;
-        const unsigned int b = 32u / num, fb = 31u - (unsigned int)__clz(num);
-        unsigned long long fbits = 0, dbits = 0;
-        for (unsigned int k = 0; k < 32; ++k) {
-            const unsigned int need = k ? k : 32u;   // bin 0 holds the 32-bit deltas (need & 31)
-            const unsigned long long iv = (need + b - 1) / b;
-            fbits += (unsigned long long)h[k] * (kind ? iv + 1 : fb);
-            dbits += (unsigned long long)h[k] * b * iv;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < p.G) {   // a warp per group, lane = delta width
+        const int g = warp;
+        double* prob = reinterpret_cast<double*>(s.cs.stage_d) + 32 * g;   // (the staging area is idle until pass 2)
+        const unsigned int h = __ldcg(&p.key_hist[g * 32 + lane]), n = L.n_g[g];
+        prob[lane] = __ddiv_rn((double)h, (double)(n > 0 ? n : 1));
+        __syncwarp();
+        // the reference's estimates in the same double arithmetic, operation by operation (explicit round-to-nearest
+        // intrinsics keep the compiler from fusing multiply-adds), one lane per interval count m
+        double t1 = 0.0, t2 = 0.0;
+        if (lane < 4) {
+            const int m = 2 << lane, b = 32 / m;
+            double sum = 0.0;
+            for (int i = 0; i < m; ++i) {
+                double ip = 0.0;
+                for (int j = 0; j < b; ++j) ip = __dadd_rn(ip, prob[i * b + j]);
+                sum = __dadd_rn(sum, __dmul_rn((double)(i + 1), ip));
+            }
+            t1 = __dadd_rn(__dmul_rn(sum, (double)b), (double)(lane + 1));
+            t2 = __dadd_rn(__dmul_rn(sum, (double)(b + 1)), 1.0);
         }
-        L.flag_bits[g] = fbits;
-        L.delta_bits[g] = dbits;
+        double best = 32.0;
+        unsigned int num = 1, kind = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double a = __shfl_sync(0xFFFFFFFFu, t1, q), c = __shfl_sync(0xFFFFFFFFu, t2, q);
+            if (a < best) {
+                best = a;
+                num = 2u << q;
+                kind = 0;
+            }
+            if (c < best) {
+                best = c;
+                num = 2u << q;
+                kind = 1;
+            }
+        }
+        const unsigned int b = 32u / num, fb = 31u - (unsigned int)__clz(num);
+        const unsigned int need = lane ? (unsigned int)lane : 32u;   // bin 0 holds the 32-bit deltas (need & 31)
+        const unsigned long long iv = (need + b - 1) / b;
+        const unsigned long long fbits = warp_sum((unsigned long long)h * (kind ? iv + 1 : fb));
+        const unsigned long long dbits = warp_sum((unsigned long long)h * b * iv);
+        if (lane == 0) {
+            L.num_iv[g] = num;
+            L.flag_kind[g] = kind;
+            L.flag_bits[g] = fbits;
+            L.delta_bits[g] = dbits;
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long o = L.off_keys;
-        for (int g = 0; g < p.G; ++g) {
-            L.flag_off[g] = o;
-            if (L.n_g[g]) o += stream_bytes(L.flag_bits[g]);
-            L.delta_off[g] = o;
-            if (L.n_g[g]) o += stream_bytes(L.delta_bits[g]);
+    if (warp == 0) {
+        const bool any = lane < p.G && L.n_g[lane];
+        const unsigned long long f = any ? stream_bytes(L.flag_bits[lane]) : 0ull, d = any ? stream_bytes(L.delta_bits[lane]) : 0ull;
+        unsigned long long all;
+        const unsigned long long o = L.off_keys + warp_prefix(f + d, all);
+        if (lane < p.G) {
+            L.flag_off[lane] = o;
+            L.delta_off[lane] = o + f;
         }
-        L.total_bytes = o;
-        if (o > (unsigned long long)p.slot_capacity) {
-            L.overflow = 1;
-            skml_set_status(p.status, SKML_CAPACITY, 0x37u);
+        if (lane == 0) {
+            L.total_bytes = L.off_keys + all;
+            if (L.total_bytes > (unsigned long long)p.slot_capacity) {
+                L.overflow = 1;
+                skml_set_status(p.status, SKML_CAPACITY, 0x37u);
+            }
         }
     }
     __syncthreads();
@@ -1801,6 +1803,9 @@ __device__ void huf_histogram(const CP& p, Smem& s, unsigned int t_begin, unsign
 
 // Optimal prefix code of every group from the complete histogram (every block; one warp per group,
 // eight groups at a time), canonical code words, section sizes and the layout that follows the tables.
+// Only the merges are a chain (one lane, the two candidates of either queue read side by side); sorting,
+// code lengths (a walk to the root per leaf) and code words are the whole warp's. (One lane for all of it,
+// reading the histogram from L2, was some 35 us of a launch.)
 __device__ void huf_build(const CP& p, Smem& s) {
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1821,71 +1826,79 @@ __device__ void huf_build(const CP& p, Smem& s) {
                 }
                 continue;
             }
-            // rank sort of the present symbols by (count, symbol): every lane ranks its symbols
-            unsigned int m = 0;
-            for (unsigned int a = lane; a < n; a += 32) m += __ldcg(&p.cell_hist[base + a]) ? 1u : 0u;
-            m = warp_sum(m);
+            unsigned int m = 0;   // symbols that occur
             for (unsigned int a = lane; a < n; a += 32) {
-                const unsigned int ca = __ldcg(&p.cell_hist[base + a]);
+                const unsigned int c = __ldcg(&p.cell_hist[base + a]);
+                h.cnt[a] = c;
+                m += c ? 1u : 0u;
+            }
+            m = __reduce_add_sync(0xFFFFFFFFu, m);
+            h.next[lane] = 0;
+            if (lane < 2) h.next[32 + lane] = 0;
+            __syncwarp();
+            // rank sort of the present symbols by (count, symbol): every lane ranks its symbols
+            for (unsigned int a = lane; a < n; a += 32) {
+                const unsigned int ca = h.cnt[a];
                 if (!ca) continue;
                 unsigned int r = 0;
                 for (unsigned int b = 0; b < n; ++b) {
-                    const unsigned int cb = __ldcg(&p.cell_hist[base + b]);
+                    const unsigned int cb = h.cnt[b];
                     if (cb && (cb < ca || (cb == ca && b < a))) ++r;
                 }
                 h.ord[r] = (unsigned short)a;
                 h.w[r] = ca;
             }
+            if (lane < 2) h.w[m + lane] = 0xFFFFFFFFu;
             __syncwarp();
+            if (lane == 0 && m > 1) {
+                // two-queue construction: leaves and internal nodes are both consumed in ascending weight, leaves first
+                unsigned int li = 0, ii = 0;
+                h.iw[0] = h.iw[1] = 0xFFFFFFFFu;
+                for (unsigned int ni = 0; ni + 1 < m; ++ni) {
+                    const unsigned int l0 = h.w[li], l1 = h.w[li + 1], i0 = h.iw[ii], i1 = h.iw[ii + 1];
+                    const bool leaf_a = l0 <= i0;
+                    const bool leaf_b = (leaf_a ? l1 : l0) <= (leaf_a ? i0 : i1);
+                    h.iw[ni] = (leaf_a ? l0 : i0) + (leaf_b ? (leaf_a ? l1 : l0) : (leaf_a ? i0 : i1));
+                    h.iw[ni + 1] = h.iw[ni + 2] = 0xFFFFFFFFu;
+                    if (leaf_a) h.pl[li++] = (unsigned short)ni;
+                    else h.pi[ii++] = (unsigned short)ni;
+                    if (leaf_b) h.pl[li++] = (unsigned short)ni;
+                    else h.pi[ii++] = (unsigned short)ni;
+                }
+            }
+            __syncwarp();
+            unsigned long long bits = 0;
+            unsigned int longest = 0;
+            for (unsigned int i = lane; i < m; i += 32) {
+                unsigned int len = 1;   // (a single symbol gets the one-bit code 0)
+                if (m > 1)
+                    for (unsigned int j = h.pl[i]; j != m - 2; j = h.pi[j]) ++len;   // node m - 2 is the root
+                s.cs.huf_len[base + h.ord[i]] = (unsigned char)(len < 32 ? len : 32);
+                if (len < 32) atomicAdd(&h.next[len], 1u);
+                longest = max(longest, len);
+                bits += (unsigned long long)h.w[i] * len;
+            }
+            bits = warp_sum(bits);
+            longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+            __syncwarp();
+            // canonical code words: lengths ascending, symbols ascending inside a length
+            unsigned int first = 0;
+            for (int k = 1; k < lane; ++k) first = (first + h.next[k]) << 1;
+            __syncwarp();
+            h.next[lane] = first;
+            __syncwarp();
+            for (unsigned int a0 = 0; a0 < n; a0 += 32) {
+                const unsigned int a = a0 + lane, len = a < n ? s.cs.huf_len[base + a] : 0u;
+                const unsigned int same = __match_any_sync(0xFFFFFFFFu, len);
+                if (len && len < 32) s.cs.huf_code[base + a] = h.next[len] + (unsigned int)__popc(same & lanemask_lt());
+                __syncwarp();
+                if (len && len < 32 && (same & lanemask_lt()) == 0) h.next[len] += (unsigned int)__popc(same);
+                __syncwarp();
+            }
             if (lane == 0) {
-                unsigned long long bits = 0;
-                if (m == 1) {
-                    s.cs.huf_len[base + h.ord[0]] = 1;   // a single symbol gets the one-bit code 0
-                    s.cs.huf_code[base + h.ord[0]] = 0;
-                    bits = h.w[0];
-                } else {
-                    // two-queue construction: leaves and internal nodes are both consumed in ascending weight
-                    unsigned int li = 0, ii = 0, ni = 0;
-                    while (ni + 1 < m) {
-                        unsigned int wsum = 0;
-                        for (int k = 0; k < 2; ++k) {
-                            const bool take_leaf = li < m && (ii >= ni || h.w[li] <= h.iw[ii]);
-                            if (take_leaf) {
-                                wsum += h.w[li];
-                                h.pl[li++] = (unsigned short)ni;
-                            } else {
-                                wsum += h.iw[ii];
-                                h.pi[ii++] = (unsigned short)ni;
-                            }
-                        }
-                        h.iw[ni++] = wsum;
-                    }
-                    h.di[ni - 1] = 0;  // the root
-                    for (int j = (int)ni - 2; j >= 0; --j) h.di[j] = (unsigned char)(h.di[h.pi[j]] + 1);
-                    unsigned int per_len[33];
-                    for (int k = 0; k < 33; ++k) per_len[k] = 0;
-                    unsigned int longest = 0;
-                    for (unsigned int i = 0; i < m; ++i) {
-                        const unsigned int len = (unsigned int)h.di[h.pl[i]] + 1u;
-                        s.cs.huf_len[base + h.ord[i]] = (unsigned char)(len < 32 ? len : 32);
-                        if (len < 33) ++per_len[len];
-                        longest = max(longest, len);
-                        bits += (unsigned long long)h.w[i] * len;
-                    }
-                    if (longest > 31) {
-                        L.overflow = 1;
-                        skml_set_status(p.status, SKML_BAD_INPUT, 0x39u);
-                    }
-                    // canonical code words: lengths ascending, symbols ascending inside a length
-                    unsigned int next[33], code = 0;
-                    for (int k = 1; k < 33; ++k) {
-                        next[k] = code;
-                        code = (code + per_len[k]) << 1;
-                    }
-                    for (unsigned int a = 0; a < n; ++a) {
-                        const unsigned int len = s.cs.huf_len[base + a];
-                        if (len && len < 32) s.cs.huf_code[base + a] = next[len]++;
-                    }
+                if (longest > 31) {
+                    L.overflow = 1;
+                    skml_set_status(p.status, SKML_BAD_INPUT, 0x39u);
                 }
                 L.items[g] = m;
                 L.tbits[g] = bits;
@@ -1894,26 +1907,30 @@ __device__ void huf_build(const CP& p, Smem& s) {
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long o = L.off_tables;
-        for (int g = 0; g < p.G; ++g) {
-            L.table_off[g] = o;
-            if (L.n_g[g]) {
-                const unsigned long long stream = o + 16ull + 12ull * L.items[g];
-                L.tstream_off[g] = stream;
-                L.trestart_off[g] = skml_align16(stream + 8ull * ((L.tbits[g] + 63) / 64));
-                o = skml_align16(L.trestart_off[g] + 4ull * ((L.cells[g] + HUF_RESTART - 1) / HUF_RESTART));
+    if (warp == 0) {   // sections start at multiples of 16, so their sizes do not depend on where
+        const unsigned int n = lane < p.G ? L.n_g[lane] : 0u;
+        unsigned long long stream = 0, restart = 0, size = 0, all, worst;
+        if (n) {
+            stream = 16ull + 12ull * L.items[lane];
+            restart = skml_align16(stream + 8ull * ((L.tbits[lane] + 63) / 64));
+            size = skml_align16(restart + 4ull * ((L.cells[lane] + HUF_RESTART - 1) / HUF_RESTART));
+        }
+        const unsigned long long o = L.off_tables + warp_prefix(size, all);
+        const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE;
+        warp_prefix(lane < p.G ? skml_align16(4ull * n + 8) + (adaptive ? skml_align16(17ull * n / 8 + 8) : 0ull) : 0ull, worst);
+        if (lane < p.G) {
+            L.table_off[lane] = o;
+            if (n) {
+                L.tstream_off[lane] = o + stream;
+                L.trestart_off[lane] = o + restart;
             }
         }
-        L.off_deltas = o;
-        L.off_keys = o;
-        unsigned long long worst = o;
-        const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE;
-        for (int g = 0; g < p.G; ++g)
-            worst += skml_align16(4ull * L.n_g[g] + 8) + (adaptive ? skml_align16(17ull * L.n_g[g] / 8 + 8) : 0ull);
-        if (worst > (unsigned long long)p.slot_capacity && !L.overflow) {
-            L.overflow = 1;
-            skml_set_status(p.status, SKML_CAPACITY, 0x3Au);
+        if (lane == 0) {
+            L.off_deltas = L.off_keys = L.off_tables + all;
+            if (L.off_deltas + worst > (unsigned long long)p.slot_capacity && !L.overflow) {
+                L.overflow = 1;
+                skml_set_status(p.status, SKML_CAPACITY, 0x3Au);
+            }
         }
     }
     __syncthreads();

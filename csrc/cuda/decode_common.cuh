@@ -23,6 +23,8 @@
 #define DEC_BLOCKS_PER_SM 3
 #endif
 #define DEC_HUF_MAX_ITEMS 513  // code words of one Huffman-coded table the expander accepts
+#define DEC_HUF_LUT 10         // code lengths the expander looks up instead of searching
+#define DEC_HUF_STAGE 896      // stream words a warp of the expander stages (16 stretches of 128 cells at 14 bits)
 // Most key ranges a block takes in the key-range-owned apply (dealt in snake order; sizes the slice
 // table in shared memory). Measured at eight payloads of 433k keys: two ranges per block even out the
 // blocks' finishing times (last block 38 us -> 7 us after the first) but not the SGD launch (175 us either

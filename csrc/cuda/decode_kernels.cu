@@ -277,12 +277,23 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
 // largest one not above them). A block works on one item at a time; its threads each decode a stretch
 // of cells from a restart offset (every `head[3]` cells; a table without restart offsets is decoded by
 // one thread). Never-written cells (Integer.MAX_VALUE) become the zero bucket, as in the narrow form.
+// What bounds it is the chain of a stretch's 128 cells, some 60 cycles each: the next stream bits wait in a 64-bit
+// window, words of up to DEC_HUF_LUT bits are looked up in a table of all prefixes, and a warp takes as few
+// stretches (16 at most) as keep all warps busy, with their part of the stream staged in shared memory first:
+// the lanes refill their windows at different cells, so every load from L2 would hold up all of them.
+// (Two L2 loads and a search per cell took 80 us for 200,000 keys' tables.)
 __device__ void expand_tables(const DP& p, DecSmem& s) {
     if (s.nhuf == 0) return;
     unsigned char* area = reinterpret_cast<unsigned char*>(&s) + p.tab_off;
     unsigned int* la = reinterpret_cast<unsigned int*>(area);                       // left-aligned code words, ascending
     unsigned short* sym = reinterpret_cast<unsigned short*>(la + DEC_HUF_MAX_ITEMS);  // their symbols (0xFFFF = never written)
     unsigned char* len = reinterpret_cast<unsigned char*>(sym + DEC_HUF_MAX_ITEMS);
+    // [prefix of DEC_HUF_LUT bits]: symbol | code length << 16, 0 = longer code; the records as they arrived
+    unsigned int* lut = reinterpret_cast<unsigned int*>(area + 7 * DEC_HUF_MAX_ITEMS + 1);   // 7 x 513 + 1 is a multiple of 8
+    int* recs = reinterpret_cast<int*>(lut + (1 << DEC_HUF_LUT));
+    static_assert((7 * DEC_HUF_MAX_ITEMS + 1) % 4 == 0 && 7 * DEC_HUF_MAX_ITEMS + 1 + (4 << DEC_HUF_LUT) + 12 * DEC_HUF_MAX_ITEMS <= DEC_TAB_SMEM &&
+                  7 * DEC_HUF_MAX_ITEMS + 1 + (4 << DEC_HUF_LUT) + DEC_THREADS / 8 * DEC_HUF_STAGE <= DEC_TAB_SMEM,
+                  "the expander's tables fit the staged-table area");
     __shared__ unsigned int s_head[4];
     __shared__ int s_bad;
     // blocks are dealt to the Huffman items round-robin; the blocks of one item share its stretches
@@ -317,9 +328,10 @@ __device__ void expand_tables(const DP& p, DecSmem& s) {
             continue;
         }
         // code words: rank sort by the left-aligned word
+        for (unsigned int a = threadIdx.x; a < 3 * nitems; a += blockDim.x) recs[a] = __ldcg(reinterpret_cast<const int*>(sec + 16) + a);
+        __syncthreads();
         for (unsigned int a = threadIdx.x; a < nitems; a += blockDim.x) {
-            const int* rec = reinterpret_cast<const int*>(sec + 16) + 3 * a;
-            const int value = __ldcg(rec), bits = __ldcg(rec + 1), nb = __ldcg(rec + 2);
+            const int value = recs[3 * a], bits = recs[3 * a + 1], nb = recs[3 * a + 2];
             if (nb < 1 || nb > 32) {
                 s_bad = 1;
                 continue;
@@ -327,43 +339,98 @@ __device__ void expand_tables(const DP& p, DecSmem& s) {
             const unsigned int mine_la = (unsigned int)bits << (32 - nb);
             unsigned int r = 0;
             for (unsigned int b = 0; b < nitems; ++b) {
-                const int* rb = reinterpret_cast<const int*>(sec + 16) + 3 * b;
-                const int nbb = __ldcg(rb + 2);
-                const unsigned int other = (nbb >= 1 && nbb <= 32) ? (unsigned int)__ldcg(rb + 1) << (32 - nbb) : 0u;
+                const int nbb = recs[3 * b + 2];
+                const unsigned int other = (nbb >= 1 && nbb <= 32) ? (unsigned int)recs[3 * b + 1] << (32 - nbb) : 0u;
                 if (other < mine_la || (other == mine_la && b < a)) ++r;
             }
             la[r] = mine_la;
             len[r] = (unsigned char)nb;
-            sym[r] = value == 0x7FFFFFFF ? (unsigned short)0xFFFFu : (unsigned short)value;
+            sym[r] = value == 0x7FFFFFFF ? (unsigned short)it.zero : (unsigned short)value;
         }
         __syncthreads();
         if (s_bad) {
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_HEADER, 0x700u | (unsigned int)(i & 0xFF));
             continue;
         }
+        auto search = [&](unsigned int x) {   // largest word <= x
+            unsigned int a = 0, b = nitems;
+            while (b - a > 1) {
+                const unsigned int mid = (a + b) >> 1;
+                if (la[mid] <= x) a = mid;
+                else b = mid;
+            }
+            return a;
+        };
+        for (unsigned int e = threadIdx.x; e < (1u << DEC_HUF_LUT); e += blockDim.x) {
+            const unsigned int a = search(e << (32 - DEC_HUF_LUT));
+            lut[e] = len[a] <= DEC_HUF_LUT ? (unsigned int)sym[a] | ((unsigned int)len[a] << 16) : 0u;
+        }
+        __syncthreads();
         const unsigned int* words = reinterpret_cast<const unsigned int*>(it.base + stream_off);
-        const unsigned long long wlim = 2ull * nwords;
+        const unsigned int wlim = 2u * nwords;
         const unsigned int* restart = reinterpret_cast<const unsigned int*>(it.base + restart_off);
         unsigned char* out = const_cast<unsigned char*>(it.tab);
-        const unsigned int zero = it.zero;
-        for (unsigned int sg = (unsigned int)helper * blockDim.x + threadIdx.x; sg < nseg; sg += (unsigned int)nhelp * blockDim.x) {
-            unsigned long long pos = interval ? __ldcg(restart + sg) : 0ull;
-            const unsigned int c0 = interval ? sg * interval : 0u, c1 = interval ? min(cells, c0 + interval) : cells;
-            for (unsigned int c = c0; c < c1; ++c) {
-                const unsigned long long w0 = pos >> 5;
-                const unsigned int lo = w0 < wlim ? __ldcg(words + w0) : 0u, hi = w0 + 1 < wlim ? __ldcg(words + w0 + 1) : 0u;
-                const unsigned int x = __brev(__funnelshift_r(lo, hi, (unsigned int)(pos & 31ull)));
-                unsigned int a = 0, b = nitems;   // largest word <= x
-                while (b - a > 1) {
-                    const unsigned int mid = (a + b) >> 1;
-                    if (la[mid] <= x) a = mid;
-                    else b = mid;
+        // one stretch by one thread; word(w): stream word w with its most significant bit first
+        auto stretch = [&](unsigned int pos, unsigned int c0, unsigned int c1, auto word) {
+            unsigned int w = pos >> 5;
+            unsigned long long win = (((unsigned long long)word(w) << 32) | word(w + 1)) << (pos & 31u);   // next bit on top
+            int have = 64 - (int)(pos & 31u);
+            w += 2;
+            auto next = [&]() {
+                const unsigned int x = (unsigned int)(win >> 32);
+                unsigned int v = lut[x >> (32 - DEC_HUF_LUT)], n = v >> 16;
+                if (n == 0) {
+                    const unsigned int a = search(x);
+                    v = sym[a];
+                    n = len[a];
                 }
-                unsigned int v = sym[a] == 0xFFFFu ? zero : sym[a];
-                if (it.cell_bits == 8) out[c] = (unsigned char)v;
-                else reinterpret_cast<unsigned short*>(out)[c] = (unsigned short)v;
-                pos += len[a];
+                win <<= n;
+                have -= (int)n;
+                if (have <= 32) {
+                    win |= (unsigned long long)word(w++) << (32 - have);
+                    have += 32;
+                }
+                return v & 0xFFFFu;
+            };
+            unsigned int c = c0;
+            if (it.cell_bits == 8) {
+                for (; c + 4 <= c1 && (c & 3u) == 0; c += 4) {   // whole words
+                    unsigned int v = next();
+                    v |= next() << 8;
+                    v |= next() << 16;
+                    v |= next() << 24;
+                    *reinterpret_cast<unsigned int*>(out + c) = v;
+                }
+                for (; c < c1; ++c) out[c] = (unsigned char)next();
+            } else {
+                for (; c < c1; ++c) reinterpret_cast<unsigned short*>(out)[c] = (unsigned short)next();
             }
+        };
+        auto from_payload = [&](unsigned int w) { return w < wlim ? __brev(__ldcg(words + w)) : 0u; };
+        if (!interval) {
+            if (helper == 0 && threadIdx.x == 0) stretch(0u, 0u, cells, from_payload);
+            continue;
+        }
+        const unsigned int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (unsigned int)nhelp * (DEC_THREADS / 32);
+        const unsigned int per = min(16u, (nseg + warps - 1) / warps);
+        unsigned int* const stage = reinterpret_cast<unsigned int*>(recs) + warp * DEC_HUF_STAGE;   // (the records are sorted by now)
+        for (unsigned int s0 = ((unsigned int)helper * (DEC_THREADS / 32) + warp) * per; s0 < nseg; s0 += warps * per) {
+            const unsigned int sg = s0 + lane;
+            const bool mine = lane < per && sg < nseg;
+            const unsigned int pos = sg < nseg ? __ldcg(restart + sg) : 32u * wlim;   // lane `per`: where the turn's stretches end
+            const unsigned int first = __shfl_sync(0xFFFFFFFFu, pos, 0) >> 5, last = __shfl_sync(0xFFFFFFFFu, pos, (int)per) >> 5;
+            const unsigned int nw = last - first + 1;
+            __syncwarp();
+            const bool staged = last >= first && nw <= DEC_HUF_STAGE;
+            if (staged)
+                for (unsigned int w = lane; w < nw; w += 32) stage[w] = from_payload(first + w);
+            __syncwarp();
+            if (mine) {
+                const unsigned int c0 = sg * interval, c1 = min(cells, c0 + interval);
+                if (staged) stretch(pos, c0, c1, [&](unsigned int w) { return w - first < nw ? stage[w - first] : 0u; });
+                else stretch(pos, c0, c1, from_payload);
+            }
+            __syncwarp();
         }
     }
     __syncthreads();
