@@ -18,6 +18,7 @@
 //   objective/GradientDescent.scala:89-132.
 #include <math.h>
 
+#include "glm_loss.cuh"
 #include "skml_api.h"
 #include "skml_device.cuh"
 
@@ -28,33 +29,6 @@
 #define GRAD_MAX_RPT 256   // rows of one tile at most
 #define GRAD_RPI 4         // rows per warp and iteration
 #define GRAD_PRIV 256      // hottest columns kept once per warp
-
-__device__ __forceinline__ float glm_loss(int loss_id, float pre, float y) {
-    if (loss_id == 0) {
-        float z = pre * y;
-        if (z > 18.f) return __expf(-z);
-        if (z < -18.f) return -z;
-        return log1pf(__expf(-z));
-    } else if (loss_id == 1) {
-        float z = pre * y;
-        return z < 1.f ? 1.f - z : 0.f;
-    }
-    float d = pre - y;
-    return 0.5f * d * d;
-}
-
-// negative derivative of the loss with respect to the prediction
-__device__ __forceinline__ float glm_grad(int loss_id, float pre, float y) {
-    if (loss_id == 0) {
-        float z = pre * y;
-        if (z > 18.f) return y * __expf(-z);
-        if (z < -18.f) return y;
-        return y / (1.f + __expf(z));
-    } else if (loss_id == 1) {
-        return pre * y <= 1.f ? y : 0.f;
-    }
-    return y - pre;
-}
 
 __device__ __forceinline__ void red_add_f32(float* p, float v) {
     asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");

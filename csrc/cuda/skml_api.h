@@ -138,6 +138,36 @@ int skml_weight_norm(const float* w, long long dim, double lambda, double* sumsq
 int skml_colsum_tiled(const int* tile_pair_ptr, const int* pair_ptr, const unsigned short* lrow, const float* svals,
                       const int* pair_dst, const int* col_pair_ptr, const int* ucols, int rows, int tile_rows, int n_tiles,
                       int n_cols, const float* coef, const float* w, float lambda, float* partial, float* out, void* stream);
+// Tiled copies of the entries of a batch whose gradient is near dense (csrc/cuda/tiled_kernels.cu): per (row tile,
+// column) list c_ptr (in quads of four entries, row_tiles * dim + 1 of them), the tile-local rows c_loc and values
+// c_val (null: all one) in that order, padded with c_loc = tile_rows, c_val = 0; the same per (column tile, row) in
+// r_* with tile-local columns (r_ptr null: margins are taken from the CSR rows). `touched`: one bit per column with
+// an entry. `partial`: scratch of max(row_tiles * dim, col_tiles * rows) floats; `coef`: one float per row.
+#define SKML_DT_TILE_MAX 49152   // floats of a vector tile in shared memory (192 KB)
+typedef struct SkmlDenseIndex {
+    long long rows, dim, row_tiles, tile_rows, col_tiles, tile_cols;
+    const int* c_ptr;
+    unsigned short* c_loc;
+    float* c_val;
+    const int* r_ptr;
+    unsigned short* r_loc;
+    float* r_val;
+    const unsigned int* touched;
+    float* partial;
+    float* coef;
+} SkmlDenseIndex;
+// Entries per list (cnt_cols: row_tiles * dim zeros, cnt_rows: col_tiles * rows, or null); then the entries to
+// their lists (`entries` of them; `cursor`: row_tiles * dim zeros).
+int skml_dt_count(const SkmlDenseIndex* index, const long long* rowptr, const int* cols, long long row_lo, int* cnt_cols,
+                  int* cnt_rows, void* stream);
+int skml_dt_fill(const SkmlDenseIndex* index, const long long* rowptr, const int* cols, const float* vals, long long row_lo,
+                 long long entries, int* cursor, void* stream);
+// Batch gradient into the (zero) accumulator g and the touched bitmap, objective loss added into *loss_acc: what
+// skml_glm_grad leaves for skml_compact.
+int skml_dt_gradient(const SkmlDenseIndex* index, const long long* rowptr, const int* cols, const float* vals,
+                     const float* labels, long long row_lo, long long nnz_padded, double avg_nnz, const float* w, int loss_id,
+                     float inv_batch, double* loss_acc, float* g, unsigned int* bitmap, unsigned int* status, long long budget,
+                     void* stream);
 int skml_scatter_kv(float* acc, const int* keys, const float* vals, const long long* counts, long long stride,
                     int lists, void* stream);
 int skml_gen_wstar(float* w, long long dim, double density, unsigned long long seed, void* stream);
@@ -299,6 +329,7 @@ typedef struct SkmlStepArgs {
     const int* tt_col_pair_ptr;        // [t_cols + 1] partial-sum ranges of the columns
     float* tt_partial;                 // device scratch [>= pairs]
     long long tt_tiles, tt_tile_rows, tt_rows;
+    const SkmlDenseIndex* dense_index; // near-dense batch (null = not one): the gradient comes from its tiled copies
 } SkmlStepArgs;
 
 int skml_train_step(SkmlStepArgs* args, void* stream);

@@ -79,7 +79,13 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         a->decode->loss_out = a->loss_out;
         return skml_decode_update(a->decode, stream_);
     }
-    for (int s = 0; s < 2; ++s) {
+    if (a->dense_index) {
+        int rc = skml_dt_gradient(a->dense_index, a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->nnz_padded, a->avg_nnz, a->w,
+                                  (int)a->loss_id, (float)a->inv_batch, a->partials + 1, a->g, a->bitmap, a->status,
+                                  a->budget_cycles, stream_);
+        if (rc) return rc;
+    }
+    for (int s = 0; s < 2 && !a->dense_index; ++s) {
         if (a->seg_cnt[s] <= 0) continue;
         int rc = skml_glm_grad(a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[s], a->seg_cnt[s], a->nnz_padded,
                                a->avg_nnz, a->w, a->g, a->bitmap, (int)a->loss_id, (float)a->inv_batch, (int)a->hot,

@@ -1,0 +1,354 @@
+// Gradient of a batch that touches most coordinates (the dense kind), over two tiled copies of its entries.
+//
+// A near-dense batch has many entries per column and per row, so both halves of the gradient are products of
+// a sparse matrix with a vector that does not fit L1: margins gather w, column sums gather the coefficients,
+// and every gather is a random 32-byte sector of L2 (155 G/s). The scatter form adds one float atomic per
+// entry on top. Here the vector is cut into tiles that fit shared memory, and the batch's entries are laid
+// out once, when the index is built, by (vector tile, row) for the margins and by (vector tile, column) for
+// the column sums, with 16-bit tile-local positions. A block keeps one tile and sums its share of the (tile,
+// item) lists, one lane per list; the partial sums, tile-major, are added up by a second kernel with
+// consecutive reads. Lists are padded to four entries so that a lane reads them 8 and 16 bytes at a time; the
+// padding points at a slot that holds zero.
+// 500,000 rows x 200 values over 1M columns (100M entries, 1.3 GB of tiled copies read): see the measured
+// figures at dt_partial_kernel.
+//
+// Reference behaviour restated (ml module): objective/GradientDescent.scala:23-51 (margins, coefficients,
+// scatter-add); the kind is still decided by the compaction, as in gradient/DenseDoubleGradient.scala:64-94.
+#include "glm_loss.cuh"
+#include "skml_api.h"
+#include "skml_device.cuh"
+
+namespace {
+
+constexpr int DT_THREADS = 1024;
+constexpr int DT_LONG = 16;          // lists of more quads are summed by the whole warp
+constexpr int DT_BATCH = 4;          // quads of a lane in flight
+constexpr int DT_ROW_WARPS = 8;
+constexpr int DT_MAX_COL_TILES = 256;
+constexpr int DT_ROW_STAGE = 256;    // entries of a row that the fill puts in order in shared memory
+
+// Entries per (row tile, column) and per (column tile, row); one warp per row.
+__global__ void __launch_bounds__(DT_ROW_WARPS * 32)
+dt_count_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, long long row_lo, int rows, int tile_rows,
+                int tile_cols, int col_tiles, int dim, int* __restrict__ cnt_cols, int* __restrict__ cnt_rows) {
+    __shared__ int s_cnt[DT_ROW_WARPS][DT_MAX_COL_TILES];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int r = blockIdx.x * DT_ROW_WARPS + warp; r < rows; r += gridDim.x * DT_ROW_WARPS) {
+        if (cnt_rows)
+            for (int t = lane; t < col_tiles; t += 32) s_cnt[warp][t] = 0;
+        __syncwarp();
+        const long long e0 = rowptr[row_lo + r], e1 = rowptr[row_lo + r + 1];
+        int* const cc = cnt_cols + (long long)(r / tile_rows) * dim;
+        for (long long e = e0 + lane; e < e1; e += 32) {
+            const int c = cols[e];
+            atomicAdd(cc + c, 1);
+            if (cnt_rows) atomicAdd(&s_cnt[warp][c / tile_cols], 1);
+        }
+        __syncwarp();
+        if (cnt_rows)
+            for (int t = lane; t < col_tiles; t += 32) cnt_rows[(long long)t * rows + r] = s_cnt[warp][t];
+        __syncwarp();
+    }
+}
+
+// The entries to their lists. The column lists fill up entry by entry at random places, so they have to stay in L2
+// until they are full: the rows of a tile are walked `parts` times, each time for one range of columns whose lists
+// take some 16 MB, and the walks are dealt to the warps in order. (One walk over 70 MB of lists ran at the rate of
+// random DRAM sectors: 10 ms for 100M entries.) Everything else is read and written as a stream: a warp puts a row's
+// entries in the order of its row lists in shared memory first (rows of up to DT_ROW_STAGE entries).
+__global__ void __launch_bounds__(DT_ROW_WARPS * 32)
+dt_fill_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals, long long row_lo,
+               int rows, int tile_rows, int row_tiles, int tile_cols, int col_tiles, int dim, int parts, const int* __restrict__ c_ptr, int* __restrict__ cursor,
+               unsigned short* __restrict__ c_loc, float* __restrict__ c_val, const int* __restrict__ r_ptr,
+               unsigned short* __restrict__ r_loc, float* __restrict__ r_val) {
+    __shared__ int s_at[DT_ROW_WARPS][DT_MAX_COL_TILES];
+    __shared__ int s_dst[DT_ROW_WARPS][DT_MAX_COL_TILES];   // position of a tile's first staged entry
+    __shared__ unsigned short s_loc[DT_ROW_WARPS][DT_ROW_STAGE];
+    __shared__ unsigned char s_tile[DT_ROW_WARPS][DT_ROW_STAGE];
+    __shared__ float s_val[DT_ROW_WARPS][DT_ROW_STAGE];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int width = (dim + parts - 1) / parts;   // columns of a walk
+    const long long walks = (long long)row_tiles * parts * tile_rows;
+    for (long long q = (long long)blockIdx.x * DT_ROW_WARPS + warp; q < walks; q += (long long)gridDim.x * DT_ROW_WARPS) {
+        const long long walk = q / tile_rows;
+        const int rt = (int)(walk / parts), part = (int)(walk % parts), r = rt * tile_rows + (int)(q % tile_rows);
+        if (r >= rows) continue;
+        const int c_lo = part * width, c_hi = dim - c_lo < width ? dim : c_lo + width;
+        const long long e0 = rowptr[row_lo + r], e1 = rowptr[row_lo + r + 1];
+        const long long cbase = (long long)rt * dim;
+        const unsigned short lr = (unsigned short)(r - rt * tile_rows);
+        const bool by_row = r_ptr && part == 0, stage = by_row && e1 - e0 <= DT_ROW_STAGE;
+        if (by_row) {
+            for (int t = lane; t < col_tiles; t += 32) s_at[warp][t] = 0;
+            __syncwarp();
+        }
+        if (stage) {   // entries per tile, then their first positions
+            for (long long e = e0 + lane; e < e1; e += 32) atomicAdd(&s_at[warp][cols[e] / tile_cols], 1);
+            __syncwarp();
+            int before = 0;
+            for (int t0 = 0; t0 < col_tiles; t0 += 32) {
+                const int n = t0 + lane < col_tiles ? s_at[warp][t0 + lane] : 0;
+                int inc = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                    if (lane >= o) inc += x;
+                }
+                if (t0 + lane < col_tiles) {
+                    s_dst[warp][t0 + lane] = before + inc - n;
+                    s_at[warp][t0 + lane] = before + inc - n;
+                }
+                before += __shfl_sync(0xFFFFFFFFu, inc, 31);
+            }
+            __syncwarp();
+        }
+        for (long long e = e0 + lane; e < e1; e += 32) {
+            const int c = __ldcs(cols + e);
+            const bool here = c >= c_lo && c < c_hi;
+            const float v = vals && (here || by_row) ? __ldcs(vals + e) : 1.f;
+            if (here) {
+                const long long at = 4ll * c_ptr[cbase + c] + atomicAdd(cursor + cbase + c, 1);
+                c_loc[at] = lr;
+                if (vals) c_val[at] = v;
+            }
+            if (by_row) {
+                const int ct = c / tile_cols;
+                const int k = atomicAdd(&s_at[warp][ct], 1);
+                if (stage) {
+                    s_loc[warp][k] = (unsigned short)(c - ct * tile_cols);
+                    s_tile[warp][k] = (unsigned char)ct;
+                    if (vals) s_val[warp][k] = v;
+                } else {
+                    const long long ar = 4ll * r_ptr[(long long)ct * rows + r] + k;
+                    r_loc[ar] = (unsigned short)(c - ct * tile_cols);
+                    if (vals) r_val[ar] = v;
+                }
+            }
+        }
+        __syncwarp();
+        if (stage) {
+            for (int k = lane; k < (int)(e1 - e0); k += 32) {
+                const int ct = s_tile[warp][k];
+                const long long ar = 4ll * r_ptr[(long long)ct * rows + r] + (k - s_dst[warp][ct]);
+                __stcs(r_loc + ar, s_loc[warp][k]);
+                if (vals) __stcs(r_val + ar, s_val[warp][k]);
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// First list p in [lo, hi) whose quads and lists before it reach `target`; a whole warp, 32 probes a round.
+__device__ __forceinline__ int weighted_bound(const int* __restrict__ ptr, int lo, int hi, long long base, long long target) {
+    const int lane = threadIdx.x & 31, first = lo;
+    while (hi > lo) {
+        const int step = (hi - lo + 32) / 33;   // probes lo + step - 1, lo + 2 step - 1, ... below hi
+        const long long at = (long long)lo + (long long)(lane + 1) * step - 1;
+        const bool less = at < hi && (long long)ptr[at] + (at - first) - base < target;
+        const int n = __popc(__ballot_sync(0xFFFFFFFFu, less));   // probes that lie before the answer: the first n
+        const long long nlo = (long long)lo + (long long)n * step, nhi = n == 32 ? (long long)hi : nlo + step - 1;
+        lo = nlo < hi ? (int)nlo : hi;
+        hi = nhi < hi ? (int)nhi : hi;
+    }
+    return lo;
+}
+
+// partial[tile * items + item] = sum over the list of x[tile * T + loc] * val.
+// Blocks of a tile, and the warps of a block, share its lists by quads + lists.
+// What bounds it: reading the lists (7 bytes an entry with padding), about two thirds of the copy rate.
+template <bool HAS_VALS>
+__global__ void __launch_bounds__(DT_THREADS, 1)
+dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, int blocks_per_tile, const int* __restrict__ ptr,
+                  const ushort4* __restrict__ loc, const float4* __restrict__ val, float* __restrict__ partial) {
+    extern __shared__ __align__(16) float s_x[];
+    __shared__ int s_cut[DT_THREADS / 32 + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = DT_THREADS / 32;
+    const int tile = blockIdx.x / blocks_per_tile, sub = blockIdx.x % blocks_per_tile;
+    const long long x0 = (long long)tile * T;
+    const int nx = n - x0 < T ? (int)(n - x0) : T;
+    for (int i = threadIdx.x; i < nx; i += DT_THREADS) s_x[i] = __ldg(x + x0 + i);
+    if (threadIdx.x == 0) s_x[T] = 0.f;   // the padding's slot
+    const int p0 = tile * items, p1 = p0 + items;
+    {
+        const long long base = ptr[p0], all = (long long)ptr[p1] - base + items;
+        const long long share = (long long)sub * warps + warp, shares = (long long)blocks_per_tile * warps;
+        const int cut = weighted_bound(ptr, p0, p1, base, all * share / shares);
+        if (lane == 0) s_cut[warp] = cut;
+        if (warp == warps - 1) {
+            const int end = sub + 1 == blocks_per_tile ? p1 : weighted_bound(ptr, p0, p1, base, all * (share + 1) / shares);
+            if (lane == 0) s_cut[warps] = end;
+        }
+    }
+    __syncthreads();
+    const int w0 = s_cut[warp], w1 = s_cut[warp + 1];
+    auto quad = [&](const ushort4 l, const float4 v) {
+        return HAS_VALS ? fmaf(s_x[l.x], v.x, fmaf(s_x[l.y], v.y, fmaf(s_x[l.z], v.z, s_x[l.w] * v.w)))
+                        : (s_x[l.x] + s_x[l.y]) + (s_x[l.z] + s_x[l.w]);
+    };
+    const ushort4 none = make_ushort4(T, T, T, T);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    int nq0 = 0, nq1 = 0;   // one round of list bounds ahead
+    if (w0 + lane < w1) {
+        nq0 = ptr[w0 + lane];
+        nq1 = ptr[w0 + lane + 1];
+    }
+    for (int b = w0; b < w1; b += 32) {
+        const int p = b + lane;
+        const int q0 = nq0, q1 = nq1;
+        nq0 = nq1 = 0;
+        if (p + 32 < w1) {
+            nq0 = ptr[p + 32];
+            nq1 = ptr[p + 33];
+        }
+        float acc = 0.f;
+        if (q1 - q0 <= DT_LONG)
+            for (int q = q0; q < q1; q += DT_BATCH) {
+                ushort4 l[DT_BATCH];
+                float4 v[DT_BATCH];
+#pragma unroll
+                for (int u = 0; u < DT_BATCH; ++u) {
+                    l[u] = q + u < q1 ? __ldg(loc + q + u) : none;
+                    v[u] = HAS_VALS && q + u < q1 ? __ldg(val + q + u) : zero;
+                }
+#pragma unroll
+                for (int u = 0; u < DT_BATCH; ++u)
+                    if (q + u < q1) acc += quad(l[u], v[u]);
+            }
+        unsigned int longs = __ballot_sync(0xFFFFFFFFu, q1 - q0 > DT_LONG);
+        while (longs) {   // frequent items: the warp sums one list at a time
+            const int src = __ffs(longs) - 1;
+            longs &= longs - 1;
+            const int s0 = __shfl_sync(0xFFFFFFFFu, q0, src), s1 = __shfl_sync(0xFFFFFFFFu, q1, src);
+            float part = 0.f;
+            for (int q = s0 + lane; q < s1; q += 32 * DT_BATCH) {
+                ushort4 l[DT_BATCH];
+                float4 v[DT_BATCH];
+#pragma unroll
+                for (int u = 0; u < DT_BATCH; ++u) {
+                    l[u] = q + 32 * u < s1 ? __ldg(loc + q + 32 * u) : none;
+                    v[u] = HAS_VALS && q + 32 * u < s1 ? __ldg(val + q + 32 * u) : zero;
+                }
+#pragma unroll
+                for (int u = 0; u < DT_BATCH; ++u) part += quad(l[u], v[u]);
+            }
+            part = warp_sum(part);
+            if (lane == src) acc = part;
+        }
+        if (p < w1) partial[p] = acc;
+    }
+}
+
+// Margins of the rows from their partial sums, loss and coefficient.
+__global__ void __launch_bounds__(256)
+dt_coef_kernel(const float* __restrict__ partial, int rows, int tiles, const float* __restrict__ labels, int loss_id, float inv_batch,
+               double* __restrict__ acc, float* __restrict__ coef) {
+    double loss = 0.0;
+    for (int r = blockIdx.x * 256 + threadIdx.x; r < rows; r += gridDim.x * 256) {
+        float pre = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < tiles; ++t) pre += partial[(long long)t * rows + r];
+        const float y = labels[r];
+        loss += (double)glm_loss(loss_id, pre, y);
+        coef[r] = -glm_grad(loss_id, pre, y) * inv_batch;
+    }
+    const double total = block_sum_double(loss);
+    if (threadIdx.x == 0 && total != 0.0) atomicAdd(acc, total);
+}
+
+// Column sums from their partial sums into the (cleared) accumulator, and the columns that the batch touches.
+__global__ void __launch_bounds__(256)
+dt_sum_kernel(const float* __restrict__ partial, int dim, int tiles, const unsigned int* __restrict__ touched, float* __restrict__ g,
+              unsigned int* __restrict__ bitmap) {
+    for (int c = blockIdx.x * 256 + threadIdx.x; c < dim; c += gridDim.x * 256) {
+        float v = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < tiles; ++t) v += partial[(long long)t * dim + c];
+        g[c] = v;
+        if ((c & 31) == 0) bitmap[c >> 5] = touched[c >> 5];
+    }
+}
+
+int dt_sms() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return n;
+}
+
+unsigned blocks_for(long long n, int per, int most_per_sm) {
+    const long long b = (n + per - 1) / per, most = (long long)dt_sms() * most_per_sm;
+    return (unsigned)(b < 1 ? 1 : b > most ? most : b);
+}
+
+int dt_partial(const float* x, long long n, int T, int tiles, int items, const int* ptr, const unsigned short* loc, const float* val,
+               float* partial, cudaStream_t stream) {
+    static bool ready = false;
+    if (!ready) {
+        cudaError_t e = cudaFuncSetAttribute(dt_partial_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (SKML_DT_TILE_MAX + 4));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(dt_partial_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (SKML_DT_TILE_MAX + 4));
+        if (e != cudaSuccess) return (int)e;
+        ready = true;
+    }
+    int bpt = dt_sms() / tiles;
+    if (bpt < 1) bpt = 1;
+    const size_t smem = 4 * ((size_t)T + 4);
+    const ushort4* l = reinterpret_cast<const ushort4*>(loc);
+    const float4* v = reinterpret_cast<const float4*>(val);
+    if (val) dt_partial_kernel<true><<<tiles * bpt, DT_THREADS, smem, stream>>>(x, n, T, items, bpt, ptr, l, v, partial);
+    else dt_partial_kernel<false><<<tiles * bpt, DT_THREADS, smem, stream>>>(x, n, T, items, bpt, ptr, l, v, partial);
+    return (int)cudaGetLastError();
+}
+
+bool dt_valid(const SkmlDenseIndex* d) {
+    return d && d->rows > 0 && d->dim > 0 && d->rows < (1ll << 31) && d->dim < (1ll << 31) && d->tile_rows > 0 && d->tile_cols > 0 &&
+           d->tile_rows <= SKML_DT_TILE_MAX && d->tile_cols <= SKML_DT_TILE_MAX && d->row_tiles * d->tile_rows >= d->rows &&
+           d->col_tiles * d->tile_cols >= d->dim && d->row_tiles * d->dim < (1ll << 31) - 64 && d->col_tiles * d->rows < (1ll << 31) - 64;
+}
+
+}  // namespace
+
+extern "C" int skml_dt_count(const SkmlDenseIndex* d, const long long* rowptr, const int* cols, long long row_lo, int* cnt_cols,
+                             int* cnt_rows, void* stream) {
+    if (!dt_valid(d) || !cnt_cols || (cnt_rows && d->col_tiles > DT_MAX_COL_TILES)) return (int)cudaErrorInvalidValue;
+    dt_count_kernel<<<blocks_for(d->rows, DT_ROW_WARPS, 8), DT_ROW_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        rowptr, cols, row_lo, (int)d->rows, (int)d->tile_rows, (int)d->tile_cols, (int)d->col_tiles, (int)d->dim, cnt_cols, cnt_rows);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int skml_dt_fill(const SkmlDenseIndex* d, const long long* rowptr, const int* cols, const float* vals, long long row_lo,
+                            long long entries, int* cursor, void* stream) {
+    if (!dt_valid(d) || !d->c_ptr || !d->c_loc || !cursor || (d->r_ptr && d->col_tiles > DT_MAX_COL_TILES)) return (int)cudaErrorInvalidValue;
+    long long parts = entries / d->row_tiles * (vals ? 7 : 2) / (16 << 20) + 1;
+    if (parts > d->dim) parts = d->dim;
+    dt_fill_kernel<<<blocks_for(d->rows, DT_ROW_WARPS, 8), DT_ROW_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        rowptr, cols, vals, row_lo, (int)d->rows, (int)d->tile_rows, (int)d->row_tiles, (int)d->tile_cols, (int)d->col_tiles, (int)d->dim,
+        (int)parts, d->c_ptr, cursor,
+        d->c_loc, d->c_val, d->r_ptr, d->r_loc, d->r_val);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int skml_dt_gradient(const SkmlDenseIndex* d, const long long* rowptr, const int* cols, const float* vals, const float* labels,
+                                long long row_lo, long long nnz_padded, double avg_nnz, const float* w, int loss_id, float inv_batch,
+                                double* loss_acc, float* g, unsigned int* bitmap, unsigned int* status, long long budget, void* stream_) {
+    if (!dt_valid(d) || !d->c_ptr || !d->partial || !d->coef || !d->touched) return (int)cudaErrorInvalidValue;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    int rc;
+    if (d->r_ptr) {
+        rc = dt_partial(w, d->dim, (int)d->tile_cols, (int)d->col_tiles, (int)d->rows, d->r_ptr, d->r_loc, d->r_val, d->partial, stream);
+        if (rc) return rc;
+        dt_coef_kernel<<<blocks_for(d->rows, 256, 8), 256, 0, stream>>>(d->partial, (int)d->rows, (int)d->col_tiles, labels + row_lo, loss_id,
+                                                                       inv_batch, loss_acc, d->coef);
+        rc = (int)cudaGetLastError();
+    } else {
+        rc = skml_glm_coef(rowptr, cols, vals, labels, row_lo, d->rows, nnz_padded, avg_nnz, w, d->dim, loss_id, inv_batch, loss_acc, d->coef,
+                           status, budget, stream_);
+    }
+    if (rc) return rc;
+    rc = dt_partial(d->coef, d->rows, (int)d->tile_rows, (int)d->row_tiles, (int)d->dim, d->c_ptr, d->c_loc, d->c_val, d->partial, stream);
+    if (rc) return rc;
+    dt_sum_kernel<<<blocks_for(d->dim, 256, 8), 256, 0, stream>>>(d->partial, (int)d->dim, (int)d->row_tiles, d->touched, g, bitmap);
+    return (int)cudaGetLastError();
+}

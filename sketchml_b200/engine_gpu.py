@@ -186,6 +186,7 @@ class GpuEngine:
         self._step_fn = L.lib().skml_train_step
         self._byref = CT.byref
         import ctypes
+        self._ctypes = ctypes
         self._ca_ptr = [ctypes.pointer(x) for x in self._ca]
         self._da_ptr = [ctypes.pointer(x) for x in self._da]
         self._pending = None
@@ -193,31 +194,50 @@ class GpuEngine:
     def _build_transposed_index(self) -> None:
         """Column-major index of every minibatch, when the batches are fixed row slices (shard size a
         multiple of the batch size) and the index fits beside the data."""
-        from .ops.transposed import build_batch_index
+        from .ops.transposed import build_batch_index, build_dense_index
         import time
         self.tindex = None
+        self.dense_index = False
         self.index_build_s, self.index_bytes = 0.0, 0   # what the one-time preparation cost (reported by the benchmarks)
         conf, csr, B = self.conf, self.csr, self.batch_rows
         if not conf.extras.get("transposed_index", True) or self.depth != 0 or B <= 0 or csr.rows % B != 0:
             return
-        need = csr.nnz * (8 if csr.values is not None else 4) * 1.1 + 16 * B * max(1, csr.max_row_nnz)
         free, _ = torch.cuda.mem_get_info(self.device)
-        if need > 0.8 * free:
-            return
         idx = []
         torch.cuda.synchronize(self.device)
         t0 = time.perf_counter()
+        # near-dense batches: two tiled copies of the entries, lists padded to four entries, and their bounds
+        need = (csr.nnz * (12 if csr.values is not None else 4) * 1.5 + 16 * csr.dim * (B // 49152 + 1) +
+                16 * B * (csr.dim // 49152 + 1))
+        dense = self.st.dense_vals is not None and need <= 0.8 * free
+        for b in range(csr.rows // B if dense else 0):
+            di = build_dense_index(csr, b * B, (b + 1) * B)
+            if di is None:
+                if b:
+                    return
+                dense = False
+                break
+            idx.append(di)
+        need = csr.nnz * (8 if csr.values is not None else 4) * 1.1 + 16 * B * max(1, csr.max_row_nnz)
+        if not dense and need > 0.8 * free:
+            return
         # extras["tiled_index"]: the row-tiled form (a row tile's coefficients in shared memory, no atomics at all,
         # strictly bit-reproducible). Off by default: measured on the headline batch it is slower (partial sums
         # 176 us + combine 92 us against 103 us), because the frequent columns, which hold most entries, already
         # gather near-sequential coefficients in the per-column form, and a 192 KB tile allows one block per SM.
         tiled = bool(conf.extras.get("tiled_index", False))
-        for b in range(csr.rows // B):
+        for b in range(csr.rows // B if not dense else 0):
             bi = build_batch_index(csr, b * B, (b + 1) * B, tiled=tiled)
             if bi.n_cols > self.st.dim * 2 // 3 or bi.n_cols > self.st.n_max:
-                return  # near-dense gradients take the dense kind: keep the scatter path
+                return  # near-dense without a tiled form (see build_dense_index): keep the scatter path
             idx.append(bi)
-        if tiled:
+        coef = torch.zeros((B + 3) // 4 * 4, dtype=torch.float32, device=self.device)
+        if dense:
+            shared = torch.empty(max(di.partial_floats for di in idx), dtype=torch.float32, device=self.device)
+            for di in idx:
+                di.bind(shared, coef)
+            self._dense_partial = shared
+        elif tiled:
             # one scratch for the partial sums of all batches (a step uses one batch's index at a time)
             shared = torch.zeros(max([bi.tiled.n_pairs for bi in idx if bi.tiled is not None] + [1]), dtype=torch.float32,
                                  device=self.device)
@@ -227,7 +247,7 @@ class GpuEngine:
         torch.cuda.synchronize(self.device)
         self.index_build_s, self.index_bytes = time.perf_counter() - t0, sum(bi.nbytes() for bi in idx)
         self.tindex = idx
-        self.coef = torch.zeros((B + 3) // 4 * 4, dtype=torch.float32, device=self.device)
+        self.coef, self.dense_index = coef, dense
 
     def _launch_fast_step(self, step: int, lr: float, adam_scale: float, ring_ptr: int) -> None:
         csr, segs, rows, done_event = self._pending
@@ -240,7 +260,10 @@ class GpuEngine:
             lo, hi = segs[i] if i < len(segs) else (0, 0)
             a.seg_lo[i], a.seg_cnt[i] = lo, hi - lo
         a.inv_batch = 1.0 / max(1, rows)
-        bi = self._index_of(csr, segs)
+        bi, di = self._index_of(csr, segs), None
+        if bi is not None and self.dense_index:
+            bi, di = None, bi
+        a.dense_index = self._ctypes.pointer(di.args) if di is not None else None
         if bi is not None and bi.tiled is not None:
             tp = bi.tiled
             a.t_colptr, a.t_vals, a.t_ucols, a.t_cols = None, L.ptr(bi.svals), L.ptr(bi.ucols), bi.n_cols
@@ -280,7 +303,7 @@ class GpuEngine:
         if lid is not None:
             L.count_launches(len(segs) + 2 + 2)  # gather, gradient segment(s), finalize, compress, decode
         else:
-            L.count_launches((3 if bi is not None else len(segs) + 2) + 1 + 1)
+            L.count_launches((3 if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + 1 + 1)
 
     # ----------------------------------------------------------------- steps
     def _segments(self, count: int):
@@ -326,7 +349,12 @@ class GpuEngine:
                 self.stream_g.wait_event(self.ev_applied[par])
                 st.partials.copy_(self.partials_template)
                 bi = self._index_of(csr, segs)
-                if bi is not None:
+                if bi is not None and self.dense_index:
+                    from .ops.transposed import glm_grad_dense
+                    glm_grad_dense(csr, bi, m.weights, st.g, st.bitmap, st.partials, st.status, m.loss.loss_id,
+                                   self.conf.step_timeout_s)
+                    compact_gradient(st, m.weights, lam)
+                elif bi is not None:
                     from .ops.transposed import glm_grad_transposed
                     glm_grad_transposed(csr, bi, m.weights, self.coef, st.vals, st.partials, st.status, m.loss.loss_id, lam,
                                         self.conf.step_timeout_s)
@@ -340,7 +368,11 @@ class GpuEngine:
             return _BatchHandle(rows, self.batch_index), None, None
         st.partials.copy_(self.partials_template)
         bi = self._index_of(csr, segs)
-        if bi is not None:
+        if bi is not None and self.dense_index:
+            from .ops.transposed import glm_grad_dense
+            glm_grad_dense(csr, bi, m.weights, st.g, st.bitmap, st.partials, st.status, m.loss.loss_id, self.conf.step_timeout_s)
+            compact_gradient(st, m.weights, lam)
+        elif bi is not None:
             # prepared batch: coefficients per row, then one gather-sum per distinct column; the keys are the index's
             from .ops.transposed import glm_grad_transposed
             glm_grad_transposed(csr, bi, m.weights, self.coef, st.vals, st.partials, st.status, m.loss.loss_id, lam,

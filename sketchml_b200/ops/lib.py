@@ -53,6 +53,17 @@ class DecodeArgs(C.Structure):
     ]
 
 
+DT_TILE_MAX = 49152
+
+
+class DenseIndexArgs(C.Structure):
+    _fields_ = [
+        ("rows", c_ll), ("dim", c_ll), ("row_tiles", c_ll), ("tile_rows", c_ll), ("col_tiles", c_ll), ("tile_cols", c_ll),
+        ("c_ptr", c_vp), ("c_loc", c_vp), ("c_val", c_vp), ("r_ptr", c_vp), ("r_loc", c_vp), ("r_val", c_vp),
+        ("touched", c_vp), ("partial", c_vp), ("coef", c_vp),
+    ]
+
+
 class StepArgs(C.Structure):
     _fields_ = [
         ("rowptr", c_vp), ("cols", c_vp), ("vals", c_vp), ("labels", c_vp), ("seg_lo", c_ll * 2), ("seg_cnt", c_ll * 2),
@@ -68,6 +79,7 @@ class StepArgs(C.Structure):
         ("grad_done_event", c_vp),
         ("tt_tile_pair_ptr", c_vp), ("tt_pair_ptr", c_vp), ("tt_lrow", c_vp), ("tt_pair_dst", c_vp),
         ("tt_col_pair_ptr", c_vp), ("tt_partial", c_vp), ("tt_tiles", c_ll), ("tt_tile_rows", c_ll), ("tt_rows", c_ll),
+        ("dense_index", C.POINTER(DenseIndexArgs)),
     ]
 
 
@@ -95,6 +107,10 @@ _SIGS = {
     "skml_weight_norm": (c_int, [c_vp, c_ll, c_d, c_vp, c_vp, c_vp, c_vp]),
     "skml_colsum_tiled": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_vp, c_vp, c_f,
                                   c_vp, c_vp, c_vp]),
+    "skml_dt_count": (c_int, [C.POINTER(DenseIndexArgs), c_vp, c_vp, c_ll, c_vp, c_vp, c_vp]),
+    "skml_dt_fill": (c_int, [C.POINTER(DenseIndexArgs), c_vp, c_vp, c_vp, c_ll, c_ll, c_vp, c_vp]),
+    "skml_dt_gradient": (c_int, [C.POINTER(DenseIndexArgs), c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_d, c_vp, c_int, c_f, c_vp, c_vp, c_vp,
+                                 c_vp, c_ll, c_vp]),
     "skml_update_gathered": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_int, c_f, c_int, c_f, c_f, c_int, c_vp]),
     "skml_gen_wstar": (c_int, [c_vp, c_ll, c_d, c_ull, c_vp]),
     "skml_gen_rows": (c_int, [c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_d, c_int, c_int, c_f, c_vp, c_ull, c_vp]),

@@ -8,8 +8,9 @@ dim-sized accumulator, the touched bitmap and the compaction (see csrc/cuda/glm_
 """
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass
-from typing import Optional
+from typing import List, Optional
 
 import torch
 
@@ -134,6 +135,88 @@ def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False) -> 
                       le0.to(torch.int32).contiguous(), le1.to(torch.int32).contiguous(), int(short.numel()),
                       int(medium.numel()), int(long_col.numel()),
                       torch.tensor([n, 1 if n else 0, 0, 0], dtype=torch.int64, device=dev))
+
+
+@dataclass
+class DenseIndex:
+    """Tiled copies of the entries of a batch that touches most coordinates (csrc/cuda/tiled_kernels.cu)."""
+    lo: int
+    rows: int
+    args: L.DenseIndexArgs
+    tensors: List[torch.Tensor]    # what `args` points into
+    partial_floats: int            # scratch it needs
+
+    def nbytes(self) -> int:
+        return sum(t.numel() * t.element_size() for t in self.tensors)
+
+    def bind(self, partial: torch.Tensor, coef: torch.Tensor) -> None:
+        """Scratch of a step; batches that run one after another share it."""
+        self.args.partial, self.args.coef = partial.data_ptr(), coef.data_ptr()
+
+
+def _tiles(n: int, tile_max: int):
+    tiles = max(1, -(-n // tile_max))
+    return tiles, ((-(-n // tiles)) + 7) // 8 * 8
+
+
+def build_dense_index(csr: DeviceCSR, lo: int, hi: int) -> Optional[DenseIndex]:
+    """None where the batch touches no more than two thirds of the columns, or where the lists would be too short to be
+    worth it (fewer than one entry per row tile and column): partial sums and list bounds then cost more than the
+    scatter's atomics. The margins take the tiled form from six entries per
+    row and column tile on; below, the padding and the partial sums cost more than gathers of w."""
+    dev, lib, rows, dim = csr.cols.device, L.lib(), hi - lo, csr.dim
+    e0, e1 = int(csr.rowptr[lo]), int(csr.rowptr[hi])
+    nnz = e1 - e0
+    a = L.DenseIndexArgs()
+    a.rows, a.dim = rows, dim
+    a.row_tiles, a.tile_rows = _tiles(rows, TILE_ROWS_MAX)
+    a.col_tiles, a.tile_cols = _tiles(dim, TILE_ROWS_MAX)
+    if nnz < a.row_tiles * dim or 3 * nnz <= 2 * dim or a.row_tiles * dim >= 2 ** 31 - 64:
+        return None
+    margins = nnz >= 6 * rows * a.col_tiles and a.col_tiles <= 256 and a.col_tiles * rows < 2 ** 31 - 64
+    cnt_c = torch.zeros(a.row_tiles * dim, dtype=torch.int32, device=dev)
+    cnt_r = torch.empty(a.col_tiles * rows, dtype=torch.int32, device=dev) if margins else None
+    L.check(lib.skml_dt_count(C.byref(a), L.ptr(csr.rowptr), L.ptr(csr.cols), lo, L.ptr(cnt_c), L.ptr(cnt_r), L.stream()), "skml_dt_count")
+
+    any_c = torch.zeros((dim + 31) // 32 * 32, dtype=torch.bool, device=dev)
+    any_c[:dim] = cnt_c.view(a.row_tiles, dim).amax(0) > 0 if a.row_tiles > 1 else cnt_c > 0
+    if int(any_c.sum()) <= dim * 2 // 3:
+        return None
+
+    def lists(cnt, pad):
+        quads = (cnt + 3) >> 2
+        ptr = torch.zeros(cnt.numel() + 1, dtype=torch.int32, device=dev)
+        torch.cumsum(quads, 0, dtype=torch.int32, out=ptr[1:])
+        n = -(-4 * int(ptr[-1]) // 2 ** 20) * 2 ** 20   # whole megabytes: batches of one data set get buffers of one size
+        loc = torch.full((n,), pad if pad < 32768 else pad - 65536, dtype=torch.int16, device=dev)   # unsigned 16-bit patterns
+        val = None if csr.values is None else torch.zeros(n, dtype=torch.float32, device=dev)
+        return ptr, loc, val
+
+    weights = (1 << torch.arange(32, device=dev, dtype=torch.int64))
+    words = (any_c.view(-1, 32) * weights).sum(1)
+    touched = torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32)
+    c_ptr, c_loc, c_val = lists(cnt_c, int(a.tile_rows))
+    tensors = [c_ptr, c_loc, touched] + ([c_val] if c_val is not None else [])
+    a.c_ptr, a.c_loc, a.c_val, a.touched = L.ptr(c_ptr), L.ptr(c_loc), L.ptr(c_val), L.ptr(touched)
+    if margins:
+        r_ptr, r_loc, r_val = lists(cnt_r, int(a.tile_cols))
+        tensors += [r_ptr, r_loc] + ([r_val] if r_val is not None else [])
+        a.r_ptr, a.r_loc, a.r_val = L.ptr(r_ptr), L.ptr(r_loc), L.ptr(r_val)
+    cursor = cnt_c.zero_()
+    L.check(lib.skml_dt_fill(C.byref(a), L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), lo, nnz, L.ptr(cursor), L.stream()),
+            "skml_dt_fill")
+    return DenseIndex(lo, rows, a, tensors, int(max(a.row_tiles * dim, a.col_tiles * rows if margins else 0)))
+
+
+def glm_grad_dense(csr: DeviceCSR, di: DenseIndex, w: torch.Tensor, g: torch.Tensor, bitmap: torch.Tensor, partials: torch.Tensor,
+                   status: torch.Tensor, loss_id: int, budget_s: float = 1.0) -> None:
+    """The batch gradient (mean over the batch) in the zero accumulator ``g`` and its touched bitmap, for
+    `compact_gradient`; the objective loss sum is added into partials[1]."""
+    L.check(L.lib().skml_dt_gradient(C.byref(di.args), L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), L.ptr(csr.labels), di.lo,
+                                     csr.nnz_padded, float(csr.avg_nnz), L.ptr(w), loss_id, 1.0 / max(1, di.rows),
+                                     partials.data_ptr() + 8, L.ptr(g), L.ptr(bitmap), L.ptr(status), L.budget_cycles(budget_s),
+                                     L.stream()), "skml_dt_gradient")
+    L.count_launches(4 if di.args.r_ptr else 3)
 
 
 def glm_grad_transposed(csr: DeviceCSR, bi: BatchIndex, w: torch.Tensor, coef: torch.Tensor, out_vals: torch.Tensor,

@@ -301,3 +301,68 @@ def test_margins_over_their_row_shapes(rows, nnz, binary):
     want = -0.5 * loss.grad(pre, labels.double())[lo:]
     assert float((coef[:rows - lo].cpu().double() - want).abs().max()) <= tol + 1e-6    # slope <= 1/4; __expf: a few ulp
     assert abs(float(part) - float(loss.loss(pre, labels.double())[lo:].sum())) <= (tol + 1e-5) * rows
+
+
+@pytest.mark.parametrize("rows,dim,nnz,tile", [
+    (1, 40, 40, 49152), (33, 300, (250, 300), 49152), (2000, 5000, (20, 90), 49152), (2000, 5000, (20, 90), 256),
+    (50000, 700, (10, 30), 49152), (3001, 1003, (60, 200), 1000)])
+@pytest.mark.parametrize("binary", [True, False])
+@pytest.mark.parametrize("zipf", [True, False])
+def test_near_dense_index_matches_the_scatter_path(rows, dim, nnz, tile, binary, zipf, monkeypatch):
+    """Tiled lists of a near-dense batch: one tile and several, ragged last tiles, lists of no entry, of a few quads
+    and longer than a warp sums at once (frequent columns), margins with and without the tiled form; the batch starts
+    inside the shard."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.models.loss import L2SquareLoss
+    from sketchml_b200.ops import DeviceCSR, GlmState, compact_gradient, glm_grad
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T, "TILE_ROWS_MAX", tile)
+    dev, loss = torch.device("cuda"), L2SquareLoss(1e-2)
+    gen = torch.Generator().manual_seed(rows + dim)
+    lead = 5
+    lo_n, hi_n = nnz if isinstance(nnz, tuple) else (nnz, nnz)
+    cnt = torch.randint(lo_n, hi_n + 1, (rows + lead,), generator=gen)
+    rowptr = torch.zeros(rows + lead + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(cnt, 0)
+    n = int(rowptr[-1])
+    u = torch.rand(n, generator=gen)
+    cols = ((u ** 3 if zipf else u) * dim).int().clamp_max(dim - 1)   # a column may repeat in a row: its products just add up
+    vals = None if binary else torch.randn(n, generator=gen)
+    m = CSRMatrix(rowptr, cols, vals, torch.randn(rows + lead, generator=gen), dim)
+    csr = DeviceCSR(m, dev)
+    w = (torch.randn(dim, generator=gen) * 0.1).to(dev)
+    di = T.build_dense_index(csr, lead, rows + lead)
+    distinct = int(torch.unique(cols[int(rowptr[lead]):]).numel())
+    short = int(rowptr[-1] - rowptr[lead]) < T._tiles(rows, tile)[0] * dim
+    assert (di is None) == (short or distinct <= dim * 2 // 3)
+    if di is None:
+        return
+    st = GlmState.create(dim, dim, dev, allow_dense=True)
+    di.bind(torch.empty(di.partial_floats, device=dev), torch.empty(rows, device=dev))
+    T.glm_grad_dense(csr, di, w, st.g, st.bitmap, st.partials, st.status, loss.loss_id)
+    # fp64 gradient; a margin sums k products in fp32, a column up to n of them: error <= 2 k eps sum |products|
+    c64, e0 = cols.long(), int(rowptr[lead])
+    x = (torch.ones(n) if binary else vals).double()
+    rid = torch.repeat_interleave(torch.arange(rows + lead), cnt)
+    pre = torch.zeros(rows + lead, dtype=torch.float64).index_add_(0, rid, w.cpu().double()[c64] * x)
+    coef = (pre - m.labels.double()) / rows
+    want = torch.zeros(dim, dtype=torch.float64).index_add_(0, c64[e0:], coef[rid[e0:]] * x[e0:])
+    mag = torch.zeros(dim, dtype=torch.float64).index_add_(0, c64[e0:], coef[rid[e0:]].abs() * x[e0:].abs())
+    row_abs = torch.zeros(rows + lead, dtype=torch.float64).index_add_(0, rid, (w.cpu().double()[c64] * x).abs())
+    col_abs = torch.zeros(dim, dtype=torch.float64).index_add_(0, c64[e0:], x[e0:].abs())
+    eps = 6e-8
+    tol = 2 * eps * (torch.bincount(c64, minlength=dim).double().sqrt() + 20) * mag + 2 * eps * hi_n * float(row_abs.max()) / rows * col_abs + 1e-12
+    assert bool(((st.g.cpu().double() - want).abs() <= tol).all())
+    want_loss = 0.5 * (pre - m.labels.double())[lead:].square().sum()
+    assert abs(float(st.partials[1]) - float(want_loss)) <= 1e-5 * float(want_loss)
+    seen = torch.zeros(dim, dtype=torch.bool)
+    seen[c64[e0:]] = True
+    words = st.bitmap.cpu().long() & 0xFFFFFFFF
+    got = ((words[:, None] >> torch.arange(32)) & 1).flatten()[:dim].bool()
+    assert torch.equal(got, seen)
+    compact_gradient(st, w, loss.lam)
+    kinds = [int(st.meta[0]), int(st.meta[1])]
+    assert float(st.g.abs().max()) == 0.0 and int(st.bitmap.abs().max()) == 0
+    glm_grad(csr, [(lead, rows + lead)], w, st, loss.loss_id, rows, hot=256)
+    compact_gradient(st, w, loss.lam)
+    assert kinds == [int(st.meta[0]), int(st.meta[1])] and int(st.status.item()) == 0
