@@ -10,7 +10,7 @@
 //   S4  group sizes -> payload layout; every key goes to its group's contiguous (still key-sorted)
 //       staging list; grouped MinMaxSketch insert (atomicMin on packed cells)
 //   S5  the groups' key lists are coded in 1024-key chunks like a plain array: delta widths, byte
-//       offsets by a block scan, flag bytes, delta bytes, one restart point per chunk. A block owns a
+//       offsets, flag bytes, delta bytes staged per warp, one restart point per chunk. A block owns a
 //       contiguous run of chunks and learns its byte offset from the blocks before it (their
 //       published byte counts), so no grid barrier sits inside this stage
 //   S6  header and group table; sketch tables narrowed to 8/16-bit bucket codes; the finished
@@ -66,6 +66,7 @@ struct CP {
     unsigned int* blk_cnt;           // [grid][SKML_MAX_GROUPS]: the same per block
     unsigned long long* blk_bytes;   // [grid][SKML_MAX_GROUPS]: delta bytes of the chunks every block owns, per group
     unsigned int* blk_flag;          // [grid]: epoch in which blk_bytes was published
+    unsigned short* chunk_part;      // [8 * chunks]: delta bytes of a chunk's eighths (128 keys)
     unsigned int* chunk_off;         // [2 * chunks]: delta-byte offset of a chunk inside its owner's part of the group
                                      // (delta_adaptive: flag-bit and delta-bit offsets)
     unsigned long long* blk_bits;    // delta_adaptive: [grid][2 * SKML_MAX_GROUPS] flag bits / delta bits per block and group
@@ -128,7 +129,7 @@ struct Layout {
 };
 
 struct WsLayout {
-    long long ctrl, run_vals, run_cnt, run_w, splits_raw, warp_cnt, blk_cnt, blk_bytes, blk_flag, chunk_off, blk_bits, blk_done, key_hist, cell_hist, blk_tbits, tchunk_off, bins, gkeys, tables,
+    long long ctrl, run_vals, run_cnt, run_w, splits_raw, warp_cnt, blk_cnt, blk_bytes, blk_flag, chunk_off, chunk_part, blk_bits, blk_done, key_hist, cell_hist, blk_tbits, tchunk_off, bins, gkeys, tables,
         total;
     long long tables_cap;
 };
@@ -148,6 +149,7 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
     L.blk_bytes = o; o += al256(grid * SKML_MAX_GROUPS * 8);
     L.blk_flag = o; o += al256(grid * 4);
     L.chunk_off = o; o += al256((n_max / SKML_RESTART_INTERVAL + SKML_MAX_GROUPS + 8) * 8);
+    L.chunk_part = o; o += al256((n_max / SKML_RESTART_INTERVAL + SKML_MAX_GROUPS + 8) * 16);
     L.blk_bits = o; o += al256(grid * 2 * SKML_MAX_GROUPS * 8);
     L.blk_done = o; o += al256(grid * 4);
     L.key_hist = o; o += al256(SKML_MAX_GROUPS * 32 * 4);
@@ -227,10 +229,27 @@ struct SmemCoding {
     HufScratch huf_scratch[8];
 };
 
+// S3's copy of the split points, laid out for upper_bounds_f (the quantile stages are over, coding has not begun).
+struct SmemSearch {
+    float a[SKML_GPU_MAX_BINS + SKML_GPU_MAX_BINS / 32];
+};
+
+// S5, plain key code: byte counts of a run of chunks (measuring), then every warp's delta bytes on their way out.
+#define MEASURE_CHUNKS 2048  // chunks whose byte counts are kept in shared memory at a time
+struct SmemPack {
+    union {
+        uint4 stage[SKML_WARPS][34];   // 128 keys of at most 4 bytes, at any offset in the first unit
+        unsigned int tot[MEASURE_CHUNKS];
+    };
+};
+static_assert(sizeof(SmemPack) <= offsetof(SmemCoding, huf_len), "the Huffman code tables outlive the key code's staging");
+
 struct Smem {
     union {
         SmemQuantile qs;
         SmemCoding cs;
+        SmemSearch ss;
+        SmemPack ps;
     };
     // stages S3..S6
     float splits[SKML_GPU_MAX_BINS];
@@ -903,54 +922,78 @@ __device__ __forceinline__ long long vslice_size(long long n) {
     return (c + 31) / 32 * 32;
 }
 
-__device__ __forceinline__ void clear_warp_counts(Smem& s) {
-    for (int t = threadIdx.x; t < SKML_WARPS * SKML_MAX_GROUPS; t += blockDim.x) (&s.wcnt[0][0])[t] = 0;
-}
-
 __device__ __forceinline__ void build_group_lut(const CP& p, Smem& s) {
     for (int b = threadIdx.x; b < s.qi.bin_num; b += blockDim.x) {
         int g = 0;   // the edges ascend: the group is the number of edges at or below the bucket
         for (int e = 0; e < p.G - 1; ++e) g += s.qi.edges[e] <= b ? 1 : 0;
         s.grp_lut[b] = (unsigned char)g;
     }
-    clear_warp_counts(s);
     __syncthreads();
 }
 
-// S3: bucket of every value; keys of every group in every warp slice.
-// `first_val`: the value of this lane's first element where the caller has it in flight already; returns that
-// element's bucket.
+// The split points into s.ss; the caller's barrier follows. Returns the search's first step.
+__device__ __forceinline__ int build_search(Smem& s) {
+    const int n = s.qi.nsplits, top = search_top(n);
+    for (int i = threadIdx.x; i < 2 * top - 1; i += blockDim.x) s.ss.a[search_slot(i)] = i < n ? s.splits[i] : __int_as_float(0x7FC00000);
+    return top;
+}
+
+// Group lists keep the keys' order, so a warp ranks its elements by group: one ballot per bit of the group number
+// gives every lane the mask of its own group, and lane g that of group g. (__match_any_sync and counters in shared
+// memory took twice the instructions.)
+template <int BITS>
+__device__ __forceinline__ void group_masks(bool valid, int g, unsigned int& own, unsigned int& of_lane) {
+    const int lane = threadIdx.x & 31;
+    own = of_lane = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+    for (int k = 0; k < BITS; ++k) {
+        const unsigned int b = __ballot_sync(0xFFFFFFFFu, (g >> k) & 1);
+        own &= b ^ (((unsigned int)g >> k & 1u) - 1u);
+        of_lane &= b ^ (((unsigned int)lane >> k & 1u) - 1u);
+    }
+}
+
+// S3: bucket of every value; keys of every group in every warp slice, 64 values a turn (two searches side by side).
+// Bound by instruction issue: a conflict-free search unrolled for up to 255 splits, 32-bit positions inside the slice
+// and shared-memory counts instead of a match of the warp took it from 58 to 31 us at 10M values.
+// `first_val`: the values of this lane's first two elements where the caller has them in flight already; their
+// buckets are left in `first_bin`.
 template <bool FUSED>
-__device__ int stage_count(const CP& p, Smem& s, long long n, bool track_minmax, float first_val) {
+__device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax, const float (&first_val)[2], int (&first_bin)[2]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
+    const int top = build_search(s);
     build_group_lut(p, s);
     const long long sub = vslice_size(n);
     const long long vb = (long long)blockIdx.x * SKML_WARPS + warp;
     long long lo = vb * sub, hi = lo + sub;
     if (lo > n) lo = n;
     if (hi > n) hi = n;
-    int first_bin = 0;
-    float nval = first_val;  // one iteration ahead: the load latency stays off the chain
-    for (long long i0 = lo; i0 < hi; i0 += 32) {
-        const long long i = i0 + lane;
-        const bool valid = i < hi;
-        const float val = nval;
-        if (i + 32 < hi) nval = p.vals[i + 32];
-        int g = 63;
-        if (valid) {
-            const int bin = upper_bound_f(s.splits, s.qi.nsplits, val);
-            p.bins[i] = (unsigned short)bin;
-            if (i0 == lo) first_bin = bin;
-            g = s.grp_lut[bin];
-            const unsigned int k = f2ord(val);
+    s.wcnt[warp][lane] = 0;
+    __syncwarp();
+    const int rem = (int)(hi - lo) - lane;   // this lane's elements: 0, 32, ... below it
+    const float* const vals = p.vals + lo + lane;
+    unsigned short* const bins = p.bins + lo + lane;
+    float nval[2] = {first_val[0], first_val[1]};  // one turn ahead: the load latency stays off the chain
+    for (int i0 = 0; i0 < rem; i0 += 64) {
+        const float val[2] = {nval[0], nval[1]};
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (i0 + 64 + 32 * u < rem) nval[u] = vals[i0 + 64 + 32 * u];
+        int bin[2];
+        upper_bounds_f(s.ss.a, top, val, bin);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (i0 + 32 * u >= rem) break;
+            bins[i0 + 32 * u] = (unsigned short)bin[u];
+            if (i0 == 0) first_bin[u] = bin[u];
+            atomicAdd(&s.wcnt[warp][s.grp_lut[bin[u]]], 1u);
+            const unsigned int k = f2ord(val[u]);
             kmin = min(kmin, k);
             kmax = max(kmax, k);
         }
-        const unsigned int peers = __match_any_sync(0xFFFFFFFFu, g);
-        if (valid && (peers & lanemask_lt()) == 0) s.wcnt[warp][g] += (unsigned int)__popc(peers);  // one leader per group
-        __syncwarp();
     }
+    __syncwarp();
     // (one launch for all stages: the slices' counts stay in shared memory)
     if (!FUSED && lane < p.G) p.warp_cnt[vb * SKML_MAX_GROUPS + lane] = s.wcnt[warp][lane];
     __syncthreads();
@@ -984,7 +1027,6 @@ __device__ int stage_count(const CP& p, Smem& s, long long n, bool track_minmax,
             }
         }
     }
-    return first_bin;
 }
 
 // S4 prelude: group sizes, table sizes, hash rows and every section offset that does not depend on
@@ -1095,19 +1137,15 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
 
 // S4: every key goes to its group's staging list (stable, so the lists stay sorted);
 // grouped MinMaxSketch insert.
-// `nkey`, `nbin`: key and bucket of this lane's first element (one launch for all stages).
+// `nkey`, `nbin`: keys and buckets of this lane's first two elements (one launch for all stages). What bounds it is
+// the rate of atomics in L2: three a key, 121 G/s at 10M keys; a plain count of 100M random keys reaches 156 G/s.
 template <bool FUSED>
-__device__ void stage_scatter(const CP& p, Smem& s, long long n, int nkey, int nbin) {
+__device__ void stage_scatter(const CP& p, Smem& s, long long n, int (&nkey)[2], int (&nbin)[2]) {
     const int G = p.G;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Layout& L = s.lay;
     if (L.overflow) return;
-    if (FUSED) {
-        clear_warp_counts(s);   // the group table is the count stage's
-        __syncthreads();
-    } else {
-        build_group_lut(p, s);
-    }
+    if (!FUSED) build_group_lut(p, s);   // (otherwise the group table is the count stage's)
     const long long sub = vslice_size(n);
     const long long vb = (long long)blockIdx.x * SKML_WARPS + warp;
     long long lo = vb * sub, hi = lo + sub;
@@ -1116,51 +1154,58 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n, int nkey, int n
     const int zero = s.qi.zero_idx;
     unsigned int run = 0;   // lane g: staging position of the next key of group g in this slice
     if (lane < G) run = L.goff[lane] + L.base_rank[lane] + s.wbase[warp][lane];
-    if (!FUSED && lo + lane < hi) {
-        nkey = p.keys[lo + lane];
-        nbin = p.bins[lo + lane];
+    const int len = (int)(hi - lo), rem = len - lane;   // this lane's elements: 0, 32, ... below rem
+    const int* const keys = p.keys + lo + lane;
+    const unsigned short* const bins = p.bins + lo + lane;
+    if (!FUSED) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (32 * u < rem) {
+                nkey[u] = keys[32 * u];
+                nbin[u] = bins[32 * u];
+            }
     }
-    for (long long i0 = lo; i0 < hi; i0 += 32) {
-        const long long i = i0 + lane;
-        const bool valid = i < hi;
-        const int key = nkey, bin = nbin;
-        if (i + 32 < hi) {
-            nkey = p.keys[i + 32];
-            nbin = p.bins[i + 32];
+    for (int i0 = 0; i0 < len; i0 += 64) {
+        const int key[2] = {nkey[0], nkey[1]}, bin[2] = {nbin[0], nbin[1]};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = i0 + 64 + 32 * u;
+            if (i < rem) {
+                nkey[u] = keys[i];
+                nbin[u] = bins[i];
+            }
         }
-        const int g = valid ? (int)s.grp_lut[bin] : 63;
-        const unsigned int peers = __match_any_sync(0xFFFFFFFFu, g);
-        const unsigned int lower = peers & lanemask_lt();
-        const unsigned int base = __shfl_sync(0xFFFFFFFFu, run, valid ? g : 0);
-        if (valid) {
-            if (lower == 0) s.wcnt[warp][g] = (unsigned int)__popc(peers);
-            const unsigned int dst = base + (unsigned int)__popc(lower);
-            p.gkeys[dst] = key;
-            const unsigned int cell = skml_pack_cell(bin, zero);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const bool valid = i0 + 32 * u < rem;
+            const int g = valid ? (int)s.grp_lut[bin[u]] : 0;
+            unsigned int own, of_lane;
+            if (G <= 8) group_masks<3>(valid, g, own, of_lane);
+            else group_masks<5>(valid, g, own, of_lane);
+            const unsigned int base = __shfl_sync(0xFFFFFFFFu, run, g);
+            run += (unsigned int)__popc(of_lane);   // (lanes beyond the last group find nothing)
+            if (!valid) continue;
+            p.gkeys[base + (unsigned int)__popc(own & lanemask_lt())] = key[u];
+            const unsigned int cell = skml_pack_cell(bin[u], zero);
             const int col = (int)L.col[g];
             unsigned int* tab = p.tables + L.tab32_off[g];
             int pos[SKML_MAX_ROWS];
             if (p.mixers) {
-                skml_hash_rows_mixers<3>(L.hash_ids[g], p.rows, key, (unsigned int)col, L.recip[g], pos);
+                skml_hash_rows_mixers<3>(L.hash_ids[g], p.rows, key[u], (unsigned int)col, L.recip[g], pos);
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
                     if (r < p.rows) atomicMin(tab + (long long)r * col + pos[r], cell);
             } else if (p.rows <= 4) {
-                skml_hash_rows<4>(L.hash_ids[g], p.rows, key, col, L.col_magic[g], pos);
+                skml_hash_rows<4>(L.hash_ids[g], p.rows, key[u], col, L.col_magic[g], pos);
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
                     if (r < p.rows) atomicMin(tab + (long long)r * col + pos[r], cell);
             } else {
-                skml_hash_rows<SKML_MAX_ROWS>(L.hash_ids[g], p.rows, key, col, L.col_magic[g], pos);
+                skml_hash_rows<SKML_MAX_ROWS>(L.hash_ids[g], p.rows, key[u], col, L.col_magic[g], pos);
 #pragma unroll
                 for (int r = 0; r < SKML_MAX_ROWS; ++r)
                     if (r < p.rows) atomicMin(tab + (long long)r * col + pos[r], cell);
             }
-        }
-        __syncwarp();
-        if (lane < G) {
-            run += s.wcnt[warp][lane];
-            s.wcnt[warp][lane] = 0;
         }
         __syncwarp();
     }
@@ -1182,44 +1227,61 @@ struct ChunkWork {
     int prev0;              // key before the chunk's first key (0 at the start of a group)
 };
 
-__device__ __forceinline__ void load_chunk(const CP& p, const Layout& L, unsigned int ch, unsigned int ch_end, int G, ChunkWork& c) {
-    const int t = threadIdx.x & 255, lane = threadIdx.x & 31;
-    c.g = -1;
-    c.wsum = 0;
-    c.cnt = 0;
-    c.j = 0;
-    c.prev0 = 0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        c.w[u] = 0;
-        c.d[u] = 0;
-        c.k[u] = 0;
-    }
-    if (ch >= ch_end) return;
-    int g = 0;
+// A chunk's keys on their way from memory.
+struct ChunkFetch {
+    int g;
+    unsigned int j, cnt;
+    int4 k;
+    int before;   // a warp's first lane: the key before its first one
+};
+
+// `g`: a group at or before the chunk's.
+__device__ __forceinline__ ChunkFetch fetch_chunk(const CP& p, const Layout& L, unsigned int ch, unsigned int ch_end, int G, int g) {
+    const unsigned int i0 = 4u * (threadIdx.x & 255);
+    ChunkFetch f;
+    f.g = -1;
+    f.j = f.cnt = 0;
+    f.k = make_int4(0, 0, 0, 0);
+    f.before = 0;
+    if (ch >= ch_end) return f;
     while (g + 1 < G && ch >= L.chunk_prefix[g + 1]) ++g;
-    c.g = g;
-    c.j = ch - L.chunk_prefix[g];
-    const unsigned int first = c.j * SKML_RESTART_INTERVAL;
-    c.cnt = min((unsigned int)SKML_RESTART_INTERVAL, L.n_g[g] - first);
-    const int* list = p.gkeys + L.goff[g];
-    const unsigned int i0 = 4u * t;
-    int4 kk = make_int4(0, 0, 0, 0);
-    if (i0 < c.cnt) kk = *reinterpret_cast<const int4*>(list + first + i0);  // goff and first are multiples of 4
-    c.k[0] = kk.x; c.k[1] = kk.y; c.k[2] = kk.z; c.k[3] = kk.w;
+    f.g = g;
+    f.j = ch - L.chunk_prefix[g];
+    const unsigned int first = f.j * SKML_RESTART_INTERVAL;
+    f.cnt = min((unsigned int)SKML_RESTART_INTERVAL, L.n_g[g] - first);
+    const int* list = p.gkeys + L.goff[g] + first;
+    if (i0 < f.cnt) {
+        f.k = *reinterpret_cast<const int4*>(list + i0);  // goff and first are multiples of 4
+        if ((threadIdx.x & 31) == 0 && first + i0 > 0) f.before = list[(int)i0 - 1];
+    }
+    return f;
+}
+
+__device__ __forceinline__ void expand_chunk(const ChunkFetch& f, ChunkWork& c) {
+    const unsigned int i0 = 4u * (threadIdx.x & 255);
+    c.g = f.g;
+    c.j = f.j;
+    c.cnt = f.cnt;
+    c.wsum = 0;
+    c.k[0] = f.k.x; c.k[1] = f.k.y; c.k[2] = f.k.z; c.k[3] = f.k.w;
     // the key before this thread's first key: the lane below holds it, except at a warp's start
     int prev = __shfl_up_sync(0xFFFFFFFFu, c.k[3], 1);
-    if (lane == 0) prev = (first + i0 > 0 && i0 < c.cnt) ? list[first + i0 - 1] : 0;
-    if (t == 0) c.prev0 = first > 0 ? list[first - 1] : 0;
+    if ((threadIdx.x & 31) == 0) prev = f.before;
+    c.prev0 = f.before;   // (meant for the sub-block's first thread)
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-        if (i0 + u < c.cnt) {
+        c.w[u] = c.d[u] = 0;
+        if (i0 + u < f.cnt) {
             c.d[u] = (unsigned int)(c.k[u] - prev);
             c.w[u] = (unsigned int)skml_delta_bytes(c.d[u]);
             c.wsum += c.w[u];
             prev = c.k[u];
         }
     }
+}
+
+__device__ __forceinline__ void load_chunk(const CP& p, const Layout& L, unsigned int ch, unsigned int ch_end, int G, ChunkWork& c) {
+    expand_chunk(fetch_chunk(p, L, ch, ch_end, G, 0), c);
 }
 
 // Exclusive scan of `v` over the 256 threads of this thread's sub-block; `total` = the sub-block's sum.
@@ -1253,39 +1315,73 @@ __device__ __forceinline__ int group_of_chunk(const unsigned int* prefix, int G,
     return g;
 }
 
-// Byte counts of one round's four chunks (s.sub_total) -> their offsets inside the block's part of their
-// groups (s.sub_off), the block's running totals. Warp 0, one chunk per lane; the caller has a barrier before.
-__device__ __forceinline__ void round_offsets(const CP& p, Smem& s, unsigned int c0, unsigned int my_end) {
-    if (threadIdx.x >= 32) return;
-    const unsigned int q = threadIdx.x;
-    const bool mine = q < 4 && c0 + q < my_end;
-    const Layout& L = s.lay;
-    int g = 0;
-    if (mine) {
-        g = group_of_chunk(L.chunk_prefix, p.G, c0 + q);
-        unsigned int off = (unsigned int)s.my_bytes[g];
-        for (unsigned int k = 0; k < q; ++k)
-            if (c0 + k >= L.chunk_prefix[g]) off += s.sub_total[k];
-        s.sub_off[q] = off;
-    }
-    __syncwarp();
-    if (mine) atomicAdd(&s.my_bytes[g], (unsigned long long)s.sub_total[q]);
-    __syncwarp();
-}
-
 // Pass A: byte counts of this block's chunks -> chunk offsets inside the block's part of each group,
-// the block's byte totals per group (published for the blocks after it). `c`, `boff` and `total` are the
-// last round's: a block with one round of chunks goes on with them and does not read its keys again.
+// the block's byte totals per group (published for the blocks after it). A block with one round of chunks keeps
+// them (`c`, `boff`, `total`; offsets in s.sub_off) and does not read its keys again. Longer runs need the totals
+// only: every warp adds up eighths of chunks on its own, the next one's keys on their way, without a barrier
+// per chunk (a scan and three barriers per round took 31 us at 66 chunks a block).
 __device__ void pack_measure(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end, ChunkWork& c, unsigned int& boff,
                              unsigned int& total) {
+    const Layout& L = s.lay;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x < SKML_MAX_GROUPS) s.my_bytes[threadIdx.x] = 0;
-    for (unsigned int c0 = my_begin; c0 < my_end; c0 += 4) {
-        load_chunk(p, s.lay, c0 + (threadIdx.x >> 8), my_end, p.G, c);
+    if (my_end - my_begin <= 4) {
+        load_chunk(p, L, my_begin + (threadIdx.x >> 8), my_end, p.G, c);
         boff = sub_scan(s, c.wsum, total);
         if ((threadIdx.x & 255) == 0) s.sub_total[threadIdx.x >> 8] = total;
         __syncthreads();
-        round_offsets(p, s, c0, my_end);
-        if (my_end - my_begin > 4 && threadIdx.x < 4 && c0 + threadIdx.x < my_end) p.chunk_off[c0 + threadIdx.x] = s.sub_off[threadIdx.x];
+        const unsigned int q = threadIdx.x;
+        if (q < 4 && my_begin + q < my_end) {
+            const int g = group_of_chunk(L.chunk_prefix, p.G, my_begin + q);
+            unsigned int off = 0;
+            for (unsigned int k = 0; k < q; ++k)
+                if (my_begin + k >= L.chunk_prefix[g]) off += s.sub_total[k];
+            s.sub_off[q] = off;
+            atomicAdd(&s.my_bytes[g], (unsigned long long)s.sub_total[q]);
+        }
+    } else {
+        unsigned int* const tot = s.ps.tot;
+        for (unsigned int b0 = my_begin; b0 < my_end; b0 += MEASURE_CHUNKS) {
+            const unsigned int nb = min((unsigned int)MEASURE_CHUNKS, my_end - b0);
+            for (unsigned int i = threadIdx.x; i < nb; i += blockDim.x) tot[i] = 0;
+            __syncthreads();
+            // warp w: eighth w % 8 of the chunks w / 8, w / 8 + 4, ... (the lanes of a fetch take their keys by thread number)
+            ChunkFetch f = fetch_chunk(p, L, b0 + (warp >> 3), b0 + nb, p.G, 0);
+            for (unsigned int ch = warp >> 3; ch < nb; ch += 4) {
+                const ChunkFetch nf = fetch_chunk(p, L, b0 + ch + 4, b0 + nb, p.G, f.g < 0 ? 0 : f.g);
+                ChunkWork x;
+                expand_chunk(f, x);
+                const unsigned int bytes = __reduce_add_sync(0xFFFFFFFFu, x.wsum);
+                if (lane == 0) {
+                    p.chunk_part[8ull * (b0 + ch) + (warp & 7)] = (unsigned short)bytes;
+                    if (bytes) atomicAdd(&tot[ch], bytes);
+                }
+                f = nf;
+            }
+            __syncthreads();
+            if (warp == 0) {   // running offsets per group, 32 chunks a turn
+                for (unsigned int i0 = 0; i0 < nb; i0 += 32) {
+                    const unsigned int i = i0 + lane;
+                    const unsigned int t = i < nb ? tot[i] : 0u;
+                    const int g = i < nb ? group_of_chunk(L.chunk_prefix, p.G, b0 + i) : -1;
+                    unsigned int inc = t;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned int x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                        if (lane >= o) inc += x;
+                    }
+                    // the chunks of a group are neighbours: subtract what lies before the group's first lane
+                    const unsigned int same = __match_any_sync(0xFFFFFFFFu, g);
+                    const int head = __ffs(same) - 1, tail = 31 - __clz(same);
+                    const unsigned int before = __shfl_sync(0xFFFFFFFFu, inc - t, head), upto = __shfl_sync(0xFFFFFFFFu, inc, tail);
+                    if (i < nb) p.chunk_off[b0 + i] = (unsigned int)s.my_bytes[g] + inc - t - before;
+                    __syncwarp();
+                    if (g >= 0 && lane == head) s.my_bytes[g] += upto - before;
+                    __syncwarp();
+                }
+            }
+            __syncthreads();
+        }
     }
     __syncthreads();
     if (threadIdx.x < SKML_MAX_GROUPS) p.blk_bytes[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x] = s.my_bytes[threadIdx.x];
@@ -1335,18 +1431,21 @@ __device__ void pack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch)
     __syncthreads();
 }
 
-// Flag bytes, delta bytes and restart point of one chunk (256 threads, four adjacent keys each).
-__device__ __forceinline__ void pack_emit(const CP& p, const Smem& s, const ChunkWork& c, unsigned int boff, unsigned int total,
-                                          unsigned int off_in_block) {
+// Flag bytes, delta bytes and restart point of one eighth of a chunk (a warp, four adjacent keys a lane). `at`: byte
+// offset of the chunk in its group's deltas; `before`: the chunk's bytes before this warp's; `lane_off`: this warp's
+// bytes before this lane's; `bytes`: this warp's. The delta bytes are put together in shared memory at the alignment
+// they have in the payload and leave in 16-byte units (bytes at the two ends, which neighbours share); byte stores
+// from every lane, and scans and barriers of 256 threads per chunk, took 48 us of 10M keys.
+__device__ __forceinline__ void pack_emit(const CP& p, Smem& s, const ChunkWork& c, unsigned long long at, unsigned int before,
+                                          unsigned int lane_off, unsigned int bytes) {
     const Layout& L = s.lay;
-    const int t = threadIdx.x & 255, g = c.g;
+    const int t = threadIdx.x & 255, lane = threadIdx.x & 31, g = c.g;
     const unsigned int first = c.j * SKML_RESTART_INTERVAL, i0 = 4u * t;
-    const unsigned long long chunk_off = s.pre_bytes[g] + off_in_block;
     // flags: (w - 1) most significant bit first at stream bits 2i, 2i+1 -> one byte per four keys
     // (a group's last chunk also writes the zero padding up to the section's 16-byte end: there the
     // threads beyond the last key hold widths of zero)
-    const unsigned long long flag_bytes = skml_align16(8ull * ((2ull * L.n_g[g] + 63) / 64));
-    const unsigned long long fbyte = first / 4 + t;
+    const unsigned int flag_bytes = (L.n_g[g] + 63u) / 64u * 16u;
+    const unsigned int fbyte = first / 4 + t;
     if (fbyte < flag_bytes) {
         unsigned int fb = 0;
 #pragma unroll
@@ -1356,51 +1455,89 @@ __device__ __forceinline__ void pack_emit(const CP& p, const Smem& s, const Chun
         }
         p.payload[L.flag_off[g] + fbyte] = (unsigned char)fb;
     }
+    const unsigned long long to = L.delta_off[g] + at + before;
+    const unsigned int sh = (unsigned int)(to & 15ull), end = sh + bytes;
+    uint4* const units = s.ps.stage[threadIdx.x >> 5];
+    unsigned char* const stage = reinterpret_cast<unsigned char*>(units);
+    __syncwarp();   // the previous bytes have left
     if (i0 < c.cnt) {
-        unsigned char* dst = p.payload + L.delta_off[g] + chunk_off + boff;
+        unsigned char* dst = stage + sh + lane_off;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            for (unsigned int j = 0; j < c.w[u]; ++j) dst[j] = skml_delta_stream_byte(c.d[u], (int)c.w[u], (int)j);
+            // the delta's bytes, most significant first and each bit-reversed: the reversed word's bytes in memory order
+            const unsigned int x = c.w[u] ? __brev(c.d[u]) >> (32u - 8u * c.w[u]) : 0u;
+            if (c.w[u] > 0) dst[0] = (unsigned char)x;
+            if (c.w[u] > 1) dst[1] = (unsigned char)(x >> 8);
+            if (c.w[u] > 2) {
+                dst[2] = (unsigned char)(x >> 16);
+                dst[3] = (unsigned char)(x >> 24);
+            }
             dst += c.w[u];
         }
     }
-    if (t == 0 && c.j + 1 == (L.n_g[g] + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL) {
+    __syncwarp();
+    unsigned char* const out = p.payload + (to - sh);
+    const unsigned int u0 = (sh + 15u) / 16u, u1 = end / 16u;   // whole units
+    for (unsigned int u = u0 + lane; u < u1; u += 32) st_v4(reinterpret_cast<uint4*>(out) + u, units[u]);
+    // lanes 0 - 15: the unit the bytes start in, where they do not fill it from its start; lanes 16 - 31: the one they end in
+    const unsigned int b = (lane & 16 ? 16u * u1 : 0u) + (lane & 15);
+    if ((lane & 16 ? u1 >= u0 : sh != 0u) && b >= sh && b < end) out[b] = stage[b];
+    if (t == 224 && c.j + 1 == (L.n_g[g] + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL) {
         // the group's last chunk: clear the padding between the last delta byte and the section's end
-        const unsigned long long endb = chunk_off + total;
+        const unsigned long long endb = at + before + bytes;
         for (unsigned long long a = endb; a < skml_align16(8ull * ((endb + 7) / 8)); ++a) p.payload[L.delta_off[g] + a] = 0;
     }
     if (t == 0) {
         SkmlRestart r;
         r.prev_key = (unsigned int)c.prev0;
         r.flag_bit_off = 2u * first;
-        r.delta_bit_off = 8ull * chunk_off;
+        r.delta_bit_off = 8ull * at;
         *reinterpret_cast<SkmlRestart*>(p.payload + L.restart_off[g] + (unsigned long long)c.j * sizeof(SkmlRestart)) = r;
     }
 }
 
-// Pass B: the key code of this block's chunks. `c`, `boff`, `total`: pass A's only round, where it had one.
+// Pass B: the key code of this block's chunks. `c`, `boff`, `total`: pass A's only round, where it had one (`kept`).
+// Of longer runs every warp takes its eighths on its own, the next one's keys on their way.
 __device__ void pack_write(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end, bool kept, ChunkWork& c, unsigned int boff,
                            unsigned int total) {
     if (s.lay.overflow) return;
-    if (kept) {
-        if (c.g >= 0) pack_emit(p, s, c, boff, total, s.sub_off[threadIdx.x >> 8]);
-    } else {
-        const bool one_round = my_end - my_begin <= 4;
-        for (unsigned int c0 = my_begin; c0 < my_end; c0 += 4) {
-            const unsigned int ch = c0 + (threadIdx.x >> 8);
-            load_chunk(p, s.lay, ch, my_end, p.G, c);
+    const unsigned int sb = threadIdx.x >> 8, lane = threadIdx.x & 31, eighth = (threadIdx.x >> 5) & 7;
+    if (my_end - my_begin <= 4) {
+        unsigned int off = s.sub_off[sb];
+        if (!kept) {   // staged launches: pass A's counts were in another launch's registers and shared memory
+            load_chunk(p, s.lay, my_begin + sb, my_end, p.G, c);
             boff = sub_scan(s, c.wsum, total);
-            if (one_round) {   // staged launches: pass A's offsets were in another launch's shared memory
-                if ((threadIdx.x & 255) == 0) s.sub_total[threadIdx.x >> 8] = total;
-                __syncthreads();
-                unsigned int off = 0;
-                if (c.g >= 0)
-                    for (unsigned int k = c0; k < ch; ++k)
-                        if (k >= s.lay.chunk_prefix[c.g]) off += s.sub_total[k - c0];
-                if (c.g >= 0) pack_emit(p, s, c, boff, total, off);
-            } else if (c.g >= 0) {
-                pack_emit(p, s, c, boff, total, __ldcg(&p.chunk_off[ch]));
+            if ((threadIdx.x & 255) == 0) s.sub_total[sb] = total;
+            __syncthreads();
+            off = 0;
+            for (unsigned int k = 0; k < sb && c.g >= 0; ++k)
+                if (my_begin + k >= s.lay.chunk_prefix[c.g]) off += s.sub_total[k];
+        }
+        const unsigned int before = __shfl_sync(0xFFFFFFFFu, boff, 0);
+        const unsigned int bytes = __shfl_sync(0xFFFFFFFFu, boff + c.wsum, 31) - before;
+        if (c.g >= 0) pack_emit(p, s, c, s.pre_bytes[c.g] + off, before, boff - before, bytes);
+    } else {
+        const unsigned int ch0 = my_begin + sb;
+        ChunkFetch f = fetch_chunk(p, s.lay, ch0, my_end, p.G, 0);
+        // lane k < 8: bytes of the chunk's eighth k; all lanes: the chunk's offset
+        auto part_of = [&](unsigned int ch) { return ch < my_end && lane < eighth ? (unsigned int)__ldcg(&p.chunk_part[8ull * ch + lane]) : 0u; };
+        unsigned int part = part_of(ch0), off = ch0 < my_end ? __ldcg(&p.chunk_off[ch0]) : 0u;
+        for (unsigned int ch = ch0; ch < my_end; ch += 4) {
+            const ChunkFetch nf = fetch_chunk(p, s.lay, ch + 4, my_end, p.G, f.g);
+            const unsigned int npart = part_of(ch + 4), noff = ch + 4 < my_end ? __ldcg(&p.chunk_off[ch + 4]) : 0u;
+            ChunkWork x;
+            expand_chunk(f, x);
+            unsigned int inc = x.wsum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= (unsigned int)o) inc += t;
             }
+            pack_emit(p, s, x, s.pre_bytes[x.g] + off, __reduce_add_sync(0xFFFFFFFFu, part), inc - x.wsum,
+                      __shfl_sync(0xFFFFFFFFu, inc, 31));
+            f = nf;
+            part = npart;
+            off = noff;
         }
     }
     __syncthreads();
@@ -2434,7 +2571,7 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
         }
         if (threadIdx.x == 0) s.lay.overflow = 0;
         __syncthreads();
-        const int cb = s.qi.cell_bits, per = 16 / (cb / 8);
+        const int cb = s.qi.cell_bits;
         const unsigned long long off_codes = SKML_HEADER_BYTES + skml_align16(4ull * p.q);
         const unsigned long long total = skml_align16(off_codes + (unsigned long long)n * (cb / 8));
         if (total > (unsigned long long)p.slot_capacity) {
@@ -2443,27 +2580,47 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
         }
         if (!sample && blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
         unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
-        const long long units = (n + per - 1) / per;
+        // Four adjacent values per thread: one vector load, four searches side by side, one store. (Sixteen values a
+        // thread, searched one after another, left two thirds of the threads idle at 1M coordinates: 25 us.)
+        const long long units = (long long)((total - off_codes) / (cb / 2));   // with the section's zero padding
+        const int top = build_search(s);
+        __syncthreads();
+        const bool vec = (reinterpret_cast<uintptr_t>(vals) & 15) == 0;
         const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
         for (long long u = gid; u < units; u += gsz) {
-            unsigned int words[4] = {0, 0, 0, 0};
-            for (int t = 0; t < per; ++t) {
-                long long i = u * per + t;
-                unsigned int code = 0;
-                if (i < n) {
-                    const float val = vals[i];
-                    code = (unsigned int)upper_bound_f(s.splits, s.qi.nsplits, val);
-                    const unsigned int k = f2ord(val);
+            const long long i0 = 4 * u;
+            float x[4] = {0.f, 0.f, 0.f, 0.f};
+            if (vec && i0 + 4 <= n) {
+                const float4 q = __ldg(reinterpret_cast<const float4*>(vals) + u);
+                x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+            } else {
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (i0 + t < n) x[t] = vals[i0 + t];
+            }
+            int code[4];
+            upper_bounds_f(s.ss.a, top, x, code);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if (i0 + t < n) {
+                    const unsigned int k = f2ord(x[t]);
                     kmin = min(kmin, k);
                     kmax = max(kmax, k);
+                } else {
+                    code[t] = 0;
                 }
-                if (cb == 8) words[t >> 2] |= (code & 0xFFu) << (8 * (t & 3));
-                else words[t >> 1] |= (code & 0xFFFFu) << (16 * (t & 1));
             }
-            uint4 v = make_uint4(words[0], words[1], words[2], words[3]);
-            st_v4(reinterpret_cast<uint4*>(p.payload + off_codes) + u, v);
+            auto put = [&](unsigned char* at) {
+                if (cb == 8)
+                    reinterpret_cast<unsigned int*>(at)[u] =
+                        (unsigned int)code[0] | ((unsigned int)code[1] << 8) | ((unsigned int)code[2] << 16) | ((unsigned int)code[3] << 24);
+                else
+                    reinterpret_cast<uint2*>(at)[u] =
+                        make_uint2((unsigned int)code[0] | ((unsigned int)code[1] << 16), (unsigned int)code[2] | ((unsigned int)code[3] << 16));
+            };
+            put(p.payload + off_codes);
             for (unsigned int r = 0; r < p.world; ++r)
-                if (r != p.rank && p.peer_payload[r]) st_v4(reinterpret_cast<uint4*>(p.peer_payload[r] + off_codes) + u, v);
+                if (r != p.rank && p.peer_payload[r]) put(p.peer_payload[r] + off_codes);
         }
         if (sample) {   // one pair of atomics per warp
 #pragma unroll
@@ -2535,13 +2692,19 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     if (FUSED) stage_stamp(p.ctrl, 0);
     // sample form of the split search: S1 ends with the splits in every block, S2 and two grid barriers drop out
     const bool sample = p.sample_splits != 0 && !given;
-    // this lane's first element: its value is wanted after S1, its key after S3, both loads start here
-    const long long first_i = vslice_size(n) * ((long long)blockIdx.x * SKML_WARPS + (threadIdx.x >> 5)) + (threadIdx.x & 31);
-    float first_val = 0.f;
-    int first_key = 0, first_bin = 0;
-    if (first_i < n && (FUSED || stage == 3)) {
-        first_val = p.vals[first_i];
-        if (FUSED) first_key = p.keys[first_i];
+    // this lane's first two elements: their values are wanted after S1, their keys after S3, the loads start here
+    float first_val[2] = {0.f, 0.f};
+    int first_key[2] = {0, 0}, first_bin[2] = {0, 0};
+    if (FUSED || stage == 3) {
+        const long long sub = vslice_size(n), lo = sub * ((long long)blockIdx.x * SKML_WARPS + (threadIdx.x >> 5));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const long long k = 32 * u + (threadIdx.x & 31);
+            if (k < sub && lo + k < n) {
+                first_val[u] = p.vals[lo + k];
+                if (FUSED) first_key[u] = p.keys[lo + k];
+            }
+        }
     }
     if (FUSED || stage == 1) {
         stage_prepare(p, n);
@@ -2566,7 +2729,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x32u);
             return;
         }
-        first_bin = stage_count<FUSED>(p, s, n, sample, first_val);
+        stage_count<FUSED>(p, s, n, sample, first_val, first_bin);
     }
     STAGE_BARRIER(3)
     if (FUSED || stage == 4) {
@@ -2737,6 +2900,7 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     p.blk_cnt = reinterpret_cast<unsigned int*>(ws + L.blk_cnt);
     p.blk_bytes = reinterpret_cast<unsigned long long*>(ws + L.blk_bytes);
     p.blk_flag = reinterpret_cast<unsigned int*>(ws + L.blk_flag);
+    p.chunk_part = reinterpret_cast<unsigned short*>(ws + L.chunk_part);
     p.chunk_off = reinterpret_cast<unsigned int*>(ws + L.chunk_off);
     p.blk_bits = reinterpret_cast<unsigned long long*>(ws + L.blk_bits);
     p.blk_done = reinterpret_cast<unsigned int*>(ws + L.blk_done);

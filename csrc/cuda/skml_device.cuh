@@ -339,6 +339,33 @@ __device__ __forceinline__ void block_sort_2048(unsigned int* s, unsigned int* t
     merge_round<1024>(tmp, s);
 }
 
+// Upper bounds of K values side by side in an ascending array of n floats: element i lies at a[i + i / 32], and
+// NaNs (below nothing) fill up to 2 top - 1 elements, top = search_top(n). The elements a halving step may read
+// are powers of two apart, in two or four banks of a plain array (37 passes of shared memory per warp at 255
+// elements, half of what bounded S3); with the gaps they lie in different banks.
+__device__ __forceinline__ int search_top(int n) { return n > 255 ? 1 << (31 - __clz(n)) : 128; }
+__device__ __forceinline__ int search_slot(int i) { return i + (i >> 5); }
+template <int K>
+__device__ __forceinline__ void upper_bounds_f(const float* a, int top, const float (&x)[K], int (&pos)[K]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) pos[k] = 0;   // search_slot of the position so far
+    for (int step = top; step > 128; step >>= 1) {
+        const int inc = search_slot(step);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (a[pos[k] + inc - 2] <= x[k]) pos[k] += inc;
+    }
+#pragma unroll
+    for (int step = 128; step > 0; step >>= 1) {
+        const int inc = search_slot(step), at = step >= 32 ? inc - 2 : inc - 1;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (a[pos[k] + at] <= x[k]) pos[k] += inc;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) pos[k] -= pos[k] / 33;
+}
+
 // Number of elements of the ascending array a[0..n) that are <= x (upper bound).
 __device__ __forceinline__ int upper_bound_f(const float* a, int n, float x) {
     int lo = 0, hi = n;

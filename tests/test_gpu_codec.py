@@ -599,3 +599,48 @@ def test_delta_adaptive_device_codec_over_its_runs(n, gaps):
     assert np.array_equal(o["flag_words"], np.asarray(ref["flag_words"], dtype=np.uint64))
     assert np.array_equal(o["delta_words"], np.asarray(ref["delta_words"], dtype=np.uint64))
     assert np.array_equal(K.decode(got).cpu().numpy(), keys)
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("q,G", [(256, 8), (1500, 20)])
+@pytest.mark.parametrize("n", [65, 8 * 1024, 9 * 1024 + 127, 40001])
+def test_payload_of_few_blocks_with_long_runs_of_chunks(n, q, G, fused):
+    """Two blocks code everything: runs on both sides of four chunks a block, deltas of all widths, more groups than
+    three ballots tell apart, more split points than the unrolled part of the search covers."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import GpuCompressor
+    rng = np.random.default_rng(n + q)
+    keys = (np.cumsum(rng.choice([1, 2, 255, 256, 300, 70000], n, p=[.3, .2, .1, .1, .25, .05])) - 1).astype(np.int32)
+    dim = int(keys[-1]) + 1
+    vals = rng.laplace(0, 1e-3, n).astype(np.float32)
+    qz = oracle.quantile_quantize(vals, q, 128, 1, 2, False)
+    splits = qz["splits"].astype(np.float32)
+    ref = oracle.compress_sparse(keys, vals, dim, dict(bin_num=q, group_num=G, row_num=2, col_ratio=0.3, seed=3, step=1, rank=0,
+                                                       world=1, tie_mode=1, key_encoder=0),
+                                 splits, float(qz["min"]), float(qz["max"]))
+    comp = GpuCompressor(dim, n, q, G, 2, 0.3, seed=3, fused=fused, grid=2)
+    buf = comp.compress_local(torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda(), step=1, rank=0, world=1,
+                              given=(torch.from_numpy(splits).cuda(), qz["min"], qz["max"]))
+    got = comp.payload_bytes(buf)
+    assert _sections(oracle.parse(got)) == _sections(oracle.parse(ref))
+    assert np.array_equal(oracle.decompress(got)[2], oracle.decompress(ref)[2])
+
+
+@pytest.mark.parametrize("q", [2, 256, 300])
+@pytest.mark.parametrize("dim", [1, 3, 4, 5, 4099, 50002])
+def test_dense_kind_at_ragged_dimensions(dim, q):
+    """Codes of one and of two bytes, dimensions on all sides of a multiple of four, against the oracle: whole numbers
+    out of the compressor, and a decode of one payload that adds nothing to the bucket values."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import GpuCompressor, GpuDecoder
+    dense = np.random.default_rng(dim).normal(0, 1e-2, dim).astype(np.float32)
+    qz = oracle.quantile_quantize(dense, q, 128, 1, 2, False)
+    splits = qz["splits"].astype(np.float32)
+    comp = GpuCompressor(dim, dim, q, 8, 2, 0.3, seed=1)
+    buf = comp.compress_local(None, torch.from_numpy(dense).cuda(), step=2, rank=0, world=1, dense=True,
+                              given=(torch.from_numpy(splits).cuda(), qz["min"], qz["max"])).clone()
+    ref = oracle.compress_dense(dense, dict(bin_num=q, step=2, rank=0, world=1, seed=1), splits, float(qz["min"]),
+                                float(qz["max"]))
+    want = oracle.decompress(ref)[2].astype(np.float32)
+    assert np.array_equal(oracle.decompress(comp.payload_bytes(buf))[2].astype(np.float32), want)
+    assert np.array_equal(GpuDecoder(dim, dim).decode_sum([buf], step=2).cpu().numpy(), want)
