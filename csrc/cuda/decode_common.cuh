@@ -78,7 +78,8 @@ struct DecItem {  // one (rank, group) key stream
     unsigned int recip;       // floor(2^32 / col_num) for the mixer-only hash path
     unsigned long long off_bv;
     unsigned long long col_magic;
-    int mixers;               // every row uses one of the three integer mixers (at most three rows)
+    unsigned char mixers;     // every row uses one of the three integer mixers, each once (at most three rows)
+    unsigned char row_of[3];  // the mixers' rows (3: not used)
     unsigned int enc;         // key encoder of the item's payload (SkmlKeyEncoder)
     const unsigned char* tab; // the sketch table as 8/16-bit bucket codes: inside the payload, or expanded from its Huffman form
     unsigned int huffman;     // the payload carries the table Huffman-coded (expanded into the scratch before the decode)
@@ -90,25 +91,31 @@ __device__ __forceinline__ double from_fixed(long long a, int shift) { return ld
 
 // Both return new^2 - old^2 of the weight they changed (0 when they write the plain sum instead): the
 // callers add these up so that the squared norm of the model is kept current without a pass over it.
-__device__ __forceinline__ float apply_one(const DP& p, long long k, float g) {
+// The weight, and its moments where there are any, as loaded by the caller.
+__device__ __forceinline__ float apply_loaded(const DP& p, long long k, float g, float old, float m, float v) {
     if (p.out_sum) {
         p.out_sum[k] = g;
         return 0.f;
     }
-    const float old = p.w[k];
     float nw;
     if (!p.adam_v) {
         nw = old - p.lr * g;
     } else {
         const long long q = k * p.adam_stride;
-        float mt = 0.9f * p.adam_m[q] + 0.1f * g;
-        float vt = 0.999f * p.adam_v[q] + 0.001f * g * g;
+        float mt = 0.9f * m + 0.1f * g;
+        float vt = 0.999f * v + 0.001f * g * g;
         nw = old - p.lr * p.adam_scale * mt / (sqrtf(vt) + 1e-8f);
         p.adam_m[q] = mt;
         p.adam_v[q] = vt;
     }
     p.w[k] = nw;
     return (nw - old) * (nw + old);
+}
+
+__device__ __forceinline__ float apply_one(const DP& p, long long k, float g) {
+    const float old = p.out_sum ? 0.f : p.w[k];
+    const bool adam = p.adam_v && !p.out_sum;
+    return apply_loaded(p, k, g, old, adam ? p.adam_m[k * p.adam_stride] : 0.f, adam ? p.adam_v[k * p.adam_stride] : 0.f);
 }
 
 // Linear modes: SGD step on w, or accumulation of the plain mean into out_sum.
@@ -122,16 +129,15 @@ __device__ __forceinline__ float apply_direct(const DP& p, long long k, float g)
     return (nw - old) * (nw + old);
 }
 
-// Query of one key in its group's sketch: the bucket value of the cell farthest from the zero bucket.
+// Query of one key in its group's sketch: the bucket of the cell farthest from the zero bucket. Any hash rows.
 template <int MAXR>
-__device__ __forceinline__ float query_one(const DP& p, const DecItem& it, unsigned int key, const unsigned char* stab) {
+__device__ __forceinline__ int query_one(const DecItem& it, unsigned int key, const unsigned char* stab) {
     const int col = (int)it.e.col_num;
     const int zero = (int)it.zero;
     int cells[MAXR];
     int pos[MAXR];
     const int rows = (int)it.rows;
-    if (it.mixers) skml_hash_rows_mixers<(MAXR < 3 ? MAXR : 3)>(it.e.hash_ids, rows, (int)key, (unsigned int)col, it.recip, pos);
-    else skml_hash_rows<MAXR>(it.e.hash_ids, rows, (int)key, col, it.col_magic, pos);
+    skml_hash_rows<MAXR>(it.e.hash_ids, rows, (int)key, col, it.col_magic, pos);
 #pragma unroll
     for (int r = 0; r < MAXR; ++r) {  // independent loads first
         cells[r] = zero;
@@ -157,10 +163,81 @@ __device__ __forceinline__ float query_one(const DP& p, const DecItem& it, unsig
             res = cells[r];
         }
     }
+    return res;
+}
+
+// The same for a thread's keys at once where every row uses one of the integer mixers (at most three rows), hash by
+// hash: each of the three functions serves one row at most, and unused ones cost nothing. The cells compete as
+// distance << 16 | 3 - row << 14 | cell, so that the first row wins among equal distances. (Row by row, with the
+// function looked up per key and row, a key took 120 instructions more, which bound the decode of short payloads.)
+static_assert(SKML_GPU_MAX_BINS <= 4096, "a cell fits 14 bits and a distance 15");
+template <bool STAGED, typename CELL>
+__device__ __forceinline__ void query_mixers(const DecItem& it, const unsigned char* stab, const unsigned int (&keys)[DEC_KPT],
+                                             int (&res)[DEC_KPT]) {
+    const CELL* const tab = reinterpret_cast<const CELL*>(STAGED ? stab : it.tab);
+    const unsigned int col = it.e.col_num, recip = it.recip;
+    const int zero = (int)it.zero;
+    unsigned int cell[3][DEC_KPT];
+    unsigned int tag[3];
+#pragma unroll
+    for (int h = 0; h < 3; ++h) {
+        const int row = it.row_of[h];
+        tag[h] = (unsigned int)(3 - row) << 14;
+#pragma unroll
+        for (int u = 0; u < DEC_KPT; ++u) cell[h][u] = (unsigned int)zero;
+        if (row >= 3) continue;
+        const CELL* const at = tab + (unsigned int)row * col;   // rows * col < 2^31 (checked in prepare)
+#pragma unroll
+        for (int u = 0; u < DEC_KPT; ++u) {
+            const unsigned int x = h == 0 ? skml_mix_bj(keys[u]) : (h == 1 ? skml_mix_64(keys[u]) : skml_mix_tw(keys[u]));
+            const unsigned int pos = (unsigned int)skml_java_mod(x, col, recip);
+            cell[h][u] = STAGED ? (unsigned int)at[pos] : (unsigned int)__ldcg(at + pos);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < DEC_KPT; ++u) {
+        unsigned int best = (unsigned int)zero;
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+            const int d = (int)cell[h][u] - zero;
+            best = max(best, ((unsigned int)(d < 0 ? -d : d) << 16) + tag[h] + cell[h][u]);
+        }
+        res[u] = (int)(best & 0x3FFFu);
+    }
+}
+
+// Dequantized values (not yet divided by the world size) of a thread's keys. `stab`: the item's staged table or
+// null. Where there is no key the number is asked for like any other (every position lies inside the table): without
+// branches the four keys' chains run side by side.
+__device__ __forceinline__ void query_keys(const DecItem& it, const unsigned char* stab, const unsigned int (&keys)[DEC_KPT],
+                                           float (&bv)[DEC_KPT]) {
+    int b[DEC_KPT];
+    if (it.mixers) {
+        if (it.cell_bits == 8) {
+            if (stab) query_mixers<true, unsigned char>(it, stab, keys, b);
+            else query_mixers<false, unsigned char>(it, stab, keys, b);
+        } else {
+            if (stab) query_mixers<true, unsigned short>(it, stab, keys, b);
+            else query_mixers<false, unsigned short>(it, stab, keys, b);
+        }
+    } else {
+#pragma unroll 1
+        for (int u = 0; u < DEC_KPT; ++u) {
+            const unsigned int key = u == 0 ? keys[0] : (u == 1 ? keys[1] : (u == 2 ? keys[2] : keys[3]));
+            const int x = key == 0xFFFFFFFFu ? (int)it.zero : (it.rows <= 4 ? query_one<4>(it, key, stab) : query_one<SKML_MAX_ROWS>(it, key, stab));
+            b[0] = u == 0 ? x : b[0];
+            b[1] = u == 1 ? x : b[1];
+            b[2] = u == 2 ? x : b[2];
+            b[3] = u == 3 ? x : b[3];
+        }
+    }
+    static_assert(DEC_KPT == 4, "four keys a thread");
     // Bucket values (<= 16 KB per payload, read by every key) go through L1: the SM cannot hold a stale
     // line of them, because it first touches a payload after the arrival flag was acquired and L1 is
     // invalidated between dependent grids. Everything else of the payload is read once: L2 only.
-    return reinterpret_cast<const float*>(it.base + it.off_bv)[res];
+    const float* const values = reinterpret_cast<const float*>(it.base + it.off_bv);
+#pragma unroll
+    for (int u = 0; u < DEC_KPT; ++u) bv[u] = values[b[u]];
 }
 
 // Exclusive prefix sum over the block with ONE barrier: every warp publishes its total, every
@@ -176,35 +253,54 @@ __device__ __forceinline__ unsigned int dec_scan(unsigned int v, unsigned int* p
     }
     if (lane == 31) part[warp] = inc;
     __syncthreads();
-    unsigned int base = 0;
-#pragma unroll
-    for (int w = 0; w < DEC_THREADS / 32; ++w)
-        if (w < warp) base += part[w];
-    return base + inc - v;
+    return __reduce_add_sync(0xFFFFFFFFu, lane < warp ? part[lane] : 0u) + inc - v;
+}
+
+// What the decode of a chunk starts from: its restart point and, for the plain key code, its 1024 two-bit flags,
+// eight bytes (32 keys) to a lane of every warp. Loaded one chunk ahead.
+struct ChunkHead {
+    SkmlRestart rs;
+    uint2 flags;
+};
+
+__device__ __forceinline__ ChunkHead fetch_head(const DecItem& it, unsigned int j) {
+    ChunkHead h;
+    const uint4 r = ld_cg_v4(reinterpret_cast<const uint4*>(it.base + it.e.restart_off) + j);
+    h.rs.prev_key = r.x;
+    h.rs.flag_bit_off = r.y;
+    h.rs.delta_bit_off = (unsigned long long)r.z | ((unsigned long long)r.w << 32);
+    const unsigned int at = j * (SKML_RESTART_INTERVAL / 32) + (threadIdx.x & 31);
+    h.flags = make_uint2(0u, 0u);
+    if (it.enc == SKML_KEYS_DELTA_BINARY && at < it.e.n_flag_words) h.flags = __ldcg(reinterpret_cast<const uint2*>(it.base + it.e.flag_off) + at);
+    return h;
+}
+
+// Sum of the flag values (hi and lo bit) of the keys in a mask of their flag bits.
+__device__ __forceinline__ unsigned int flag_sum(uint2 f) {
+    return 2u * (unsigned int)(__popc(f.x & 0x55555555u) + __popc(f.y & 0x55555555u)) +
+           (unsigned int)(__popc(f.x & 0xAAAAAAAAu) + __popc(f.y & 0xAAAAAAAAu));   // stream order: most significant bit first
 }
 
 // Decode of one 1024-key chunk of a (rank, group) key stream by the whole block (DEC_THREADS
 // threads, DEC_KPT adjacent keys each; restart points make chunks independent): flag bits -> delta
-// widths -> block scan -> delta bytes gathered from aligned words -> block scan -> keys; then the
-// sketch query and the bucket value of every key. `part_a` / `part_b` are two scan scratch rows
-// (DEC_THREADS / 32 words each) that the caller alternates between consecutive chunks, so that no
-// extra barrier is needed between chunks. All threads of the block must call this together.
+// widths -> scan -> delta bytes gathered from aligned words -> block scan -> keys. Every warp scans the
+// plain code's flags of the whole chunk by itself, so the block meets once per chunk (adaptive code: twice,
+// unary flags four times). `part_a` / `part_b` / `part_c` are scan scratch rows (DEC_THREADS / 32 words
+// each) that the caller alternates between consecutive chunks, so that no extra barrier is needed between
+// chunks. All threads of the block must call this together.
 struct ChunkKeys {
     unsigned int i0;              // index inside the chunk of this thread's first key
     unsigned int cnt;             // keys in the chunk
     unsigned int first;           // index inside the list of the chunk's first key
-    unsigned int keys[DEC_KPT];
-    unsigned int d0;              // delta of keys[0]: keys[0] - d0 is the key before it in the list
-    float bv[DEC_KPT];            // dequantized values (not yet divided by the world size)
-    bool live[DEC_KPT];           // key exists and is inside [0, dim)
+    unsigned int keys[DEC_KPT];   // 0xFFFFFFFF: no key, or outside [0, dim)
 };
 
-__device__ __forceinline__ void decode_chunk(const DP& p, const DecItem& it, unsigned int j, const unsigned char* stab,
-                                             unsigned int* part_a, unsigned int* part_b, unsigned int* part_c,
-                                             unsigned short* s_pos, ChunkKeys& o) {
+__device__ __forceinline__ void decode_keys(const DP& p, const DecItem& it, unsigned int j, const ChunkHead& head,
+                                            unsigned int* part_a, unsigned int* part_b, unsigned int* part_c,
+                                            unsigned short* s_pos, ChunkKeys& o) {
     const unsigned int first = j * SKML_RESTART_INTERVAL;
     const unsigned int cnt = min((unsigned int)SKML_RESTART_INTERVAL, it.e.n - first);
-    const SkmlRestart rs = *reinterpret_cast<const SkmlRestart*>(it.base + it.e.restart_off + 16ull * j);
+    const SkmlRestart& rs = head.rs;
     const unsigned int i0 = DEC_KPT * threadIdx.x;
     o.i0 = i0;
     o.cnt = cnt;
@@ -213,46 +309,60 @@ __device__ __forceinline__ void decode_chunk(const DP& p, const DecItem& it, uns
 #pragma unroll
     for (int u = 0; u < DEC_KPT; ++u) d[u] = 0;
     if (it.enc == SKML_KEYS_DELTA_BINARY) {
+        const unsigned int lane = threadIdx.x & 31;
+        // bytes before every 32 keys: lane l adds up keys 32 l ... (a key takes its flag's value + 1; none beyond the last key)
+        const unsigned int mine = cnt > 32u * lane ? min(cnt - 32u * lane, 32u) : 0u;
+        const unsigned long long all = (unsigned long long)head.flags.x | ((unsigned long long)head.flags.y << 32);
+        const unsigned long long have = mine >= 32u ? all : (all & ((1ull << (2u * mine)) - 1ull));
+        const unsigned int own = mine + flag_sum(make_uint2((unsigned int)have, (unsigned int)(have >> 32)));
+        unsigned int inc = own;
+#pragma unroll
+        for (int q = 1; q < 32; q <<= 1) {
+            const unsigned int t = __shfl_up_sync(0xFFFFFFFFu, inc, q);
+            if (lane >= (unsigned int)q) inc += t;
+        }
+        // this thread's keys are four of the 32 that lane 4 * warp + lane / 8 added up
+        const unsigned int from = 4u * (threadIdx.x >> 5) + (lane >> 3), sub = 8u * (lane & 7u);
+        unsigned int boff = __shfl_sync(0xFFFFFFFFu, inc - own, (int)from);
+        const unsigned int fx = __shfl_sync(0xFFFFFFFFu, head.flags.x, (int)from), fy = __shfl_sync(0xFFFFFFFFu, head.flags.y, (int)from);
         unsigned int w[DEC_KPT];
         unsigned int wsum = 0;
-    #pragma unroll
+#pragma unroll
         for (int u = 0; u < DEC_KPT; ++u) w[u] = 0;
         if (i0 < cnt) {
-            // the flags of DEC_KPT adjacent keys are 2 * DEC_KPT adjacent bits of one 32-bit word
-            const unsigned long long fb = (unsigned long long)rs.flag_bit_off + 2ull * i0;
-            const unsigned int word = __ldcg(reinterpret_cast<const unsigned int*>(it.base + it.e.flag_off) + (fb >> 5));
-            const unsigned int b = word >> (fb & 31);
-    #pragma unroll
+            const unsigned int bx = sub < 32u ? (1u << sub) - 1u : 0xFFFFFFFFu, by = sub < 32u ? 0u : (1u << (sub - 32u)) - 1u;
+            boff += sub / 2u + flag_sum(make_uint2(fx & bx, fy & by));
+            const unsigned int b = (sub < 32u ? fx : fy) >> (sub & 31u);
+#pragma unroll
             for (int u = 0; u < DEC_KPT; ++u) {
                 if (i0 + u < cnt) {
                     const unsigned int bb = (b >> (2 * u)) & 3u;
-                    unsigned int wu = (((bb & 1u) << 1) | (bb >> 1)) + 1u;  // stream order is most significant bit first
+                    unsigned int wu = (((bb & 1u) << 1) | (bb >> 1)) + 1u;
                     if (wu == 3) wu = 4;                                     // flag value 2 is never written
                     w[u] = wu;
                     wsum += wu;
                 }
             }
         }
-        const unsigned int boff = dec_scan(wsum, part_a);
         if (i0 < cnt) {
             const unsigned long long byte0 = (rs.delta_bit_off >> 3) + boff;
             if (byte0 + wsum <= 8ull * it.e.n_delta_words) {
                 // The thread's <= 4 * DEC_KPT delta bytes sit in at most DEC_KPT + 1 aligned words.
                 // Bit-reversing a little-endian word yields its four stream bytes in most-significant-
                 // first order (java.util.BitSet order), so a delta is a funnel shift away.
-                const unsigned int* src = reinterpret_cast<const unsigned int*>(it.base + it.e.delta_off);
-                const unsigned long long w0 = byte0 >> 2, wlim = 2ull * it.e.n_delta_words;
+                const unsigned int* src = reinterpret_cast<const unsigned int*>(it.base + it.e.delta_off) + (byte0 >> 2);
+                const unsigned int left = (unsigned int)min(2ull * it.e.n_delta_words - (byte0 >> 2), 8ull);   // words from there on
                 unsigned int W[DEC_KPT + 1];
-    #pragma unroll
-                for (int t = 0; t <= DEC_KPT; ++t) W[t] = (w0 + t < wlim) ? __brev(__ldcg(src + w0 + t)) : 0u;
+#pragma unroll
+                for (int t = 0; t <= DEC_KPT; ++t) W[t] = (unsigned int)t < left ? __brev(__ldcg(src + t)) : 0u;
                 unsigned int start = (unsigned int)(byte0 & 3);
-    #pragma unroll
+#pragma unroll
                 for (int u = 0; u < DEC_KPT; ++u) {
                     const unsigned int wi = start >> 2, sh = 8u * (start & 3u);
                     unsigned int hi = W[0], lo = W[1];
-    #pragma unroll
+#pragma unroll
                     for (int t = 1; t < DEC_KPT; ++t)
-                        if (wi == (unsigned int)t) { hi = W[t]; lo = W[t + 1]; }
+                        if (t <= u && wi == (unsigned int)t) { hi = W[t]; lo = W[t + 1]; }   // (key u starts in word u at most)
                     const unsigned int v = __funnelshift_l(lo, hi, sh);
                     d[u] = w[u] ? v >> (32u - 8u * w[u]) : 0u;
                     start += w[u];
@@ -342,33 +452,14 @@ __device__ __forceinline__ void decode_chunk(const DP& p, const DecItem& it, uns
     unsigned int dsum = 0;
 #pragma unroll
     for (int u = 0; u < DEC_KPT; ++u) dsum += d[u];
-    const unsigned int dex = dec_scan(dsum, part_b);
-    o.d0 = d[0];
+    unsigned int key = rs.prev_key + dec_scan(dsum, part_b);
 #pragma unroll
     for (int u = 0; u < DEC_KPT; ++u) {
-        o.keys[u] = 0xFFFFFFFFu;
-        o.live[u] = false;
-        o.bv[u] = 0.f;
-    }
-    if (i0 < cnt) {
-        unsigned int key = rs.prev_key + dex;
-#pragma unroll
-        for (int u = 0; u < DEC_KPT; ++u) {
-            key += d[u];
-            o.keys[u] = key;
-            o.live[u] = i0 + u < cnt;
-            if (o.live[u] && key >= (unsigned long long)p.dim) {
-                skml_set_status(p.status, SKML_BAD_HEADER, 0x200u);
-                o.live[u] = false;
-                o.keys[u] = 0xFFFFFFFFu;
-            }
-        }
-        if (it.rows <= 4) {
-#pragma unroll
-            for (int u = 0; u < DEC_KPT; ++u) o.bv[u] = o.live[u] ? query_one<4>(p, it, o.keys[u], stab) : 0.f;
-        } else {
-#pragma unroll
-            for (int u = 0; u < DEC_KPT; ++u) o.bv[u] = o.live[u] ? query_one<SKML_MAX_ROWS>(p, it, o.keys[u], stab) : 0.f;
+        key += d[u];
+        o.keys[u] = i0 + u < cnt ? key : 0xFFFFFFFFu;
+        if (i0 + u < cnt && key >= (unsigned long long)p.dim) {
+            skml_set_status(p.status, SKML_BAD_HEADER, 0x200u);
+            o.keys[u] = 0xFFFFFFFFu;
         }
     }
 }

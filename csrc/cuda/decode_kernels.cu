@@ -39,7 +39,6 @@ struct DecSmem {
     unsigned long long total_chunks, total_keys;
     int any_dense;
     int direct;      // linear update (SGD / plain sum): payloads applied in rank order, no accumulators
-    unsigned long long rank_chunk_begin[SKML_MAX_PEERS + 1];
     unsigned long long rank_key_begin[SKML_MAX_PEERS + 1];
     int rank_item_begin[SKML_MAX_PEERS + 1];
     int ref_item;    // the (rank, group) list with the most keys: its quantiles are the blocks' key-range bounds
@@ -118,7 +117,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
                 const unsigned long long lim = h.total_bytes;
                 const bool good = it.e.col_num > 0 && (unsigned long long)h.row_num * it.e.col_num < (1ull << 31) &&
                                   it.e.table_off + (h.cell_bits ? (unsigned long long)h.row_num * it.e.col_num * (h.cell_bits / 8) : 16ull) <= lim &&
-                                  it.e.flag_off + 8ull * it.e.n_flag_words <= lim && it.e.delta_off + 8ull * it.e.n_delta_words <= lim &&
+                                  (it.e.flag_off & 7ull) == 0 && (it.e.restart_off & 15ull) == 0 && it.e.flag_off + 8ull * it.e.n_flag_words <= lim && it.e.delta_off + 8ull * it.e.n_delta_words <= lim &&
                                   it.e.restart_off + 16ull * ((it.e.n + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL) <= lim &&
                                   (h.key_encoder == SKML_KEYS_DELTA_BINARY
                                        ? 2ull * it.e.n <= 64ull * it.e.n_flag_words
@@ -135,7 +134,17 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
                 it.off_bv = h.off_bucket_values;
                 it.col_magic = good ? skml_fastmod_magic(it.e.col_num) : 0ull;
                 it.recip = skml_recip32(it.e.col_num);
-                it.mixers = (h.row_num <= 3 && skml_rows_are_mixers(it.e.hash_ids, (int)h.row_num)) ? 1 : 0;
+                it.mixers = 0;
+                if (h.row_num <= 3) {
+                    unsigned int seen = 0;
+                    it.row_of[0] = it.row_of[1] = it.row_of[2] = 3;
+                    for (unsigned int q = 0; q < h.row_num; ++q)
+                        if (it.e.hash_ids[q] < 3) {
+                            it.row_of[it.e.hash_ids[q]] = (unsigned char)q;
+                            seen |= 1u << it.e.hash_ids[q];
+                        }
+                    it.mixers = __popc(seen) == (int)h.row_num ? 1 : 0;
+                }
                 it.chunk_prefix = good ? 0ull : 1ull;  // scratch use until the compaction below: 1 = failed validation
             }
         }
@@ -149,7 +158,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
         int ni = 0, nhuf = 0;
         unsigned long long chunks = 0, keys = 0, tab_used = 0;
         int dense = 0, ref = 0;
-        unsigned int ref_n = 0;
+        unsigned int ref_n = 0, key_pad = 0;
         double mx = 0.0;
         if (lane == 0) {
             for (int r = 0; r < p.world; ++r) {
@@ -174,7 +183,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
             const unsigned int n = v ? it.e.n : 0u;
             const bool failed = v && it.chunk_prefix != 0ull;
             const bool huf = v && it.huffman != 0u;
-            unsigned long long c_inc = (n + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL, k_inc = n;
+            unsigned long long c_inc = (n + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL, k_inc = (n + 3ull) & ~3ull;   // (stashed four at a time)
             unsigned long long b_inc = huf ? skml_align16((unsigned long long)it.rows * it.e.col_num * (it.cell_bits / 8)) : 0ull;
             const unsigned long long c_own = c_inc, k_own = k_inc, b_own = b_inc;
 #pragma unroll
@@ -190,7 +199,6 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
             const unsigned int vm = __ballot_sync(0xFFFFFFFFu, v);
             const int pos = ni + __popc(vm & ((1u << lane) - 1u));
             if (in && g == 0) {   // what lies in front of rank r's first slot
-                s.rank_chunk_begin[r] = chunks + c_inc - c_own;
                 s.rank_key_begin[r] = keys + k_inc - k_own;
                 s.rank_item_begin[r] = pos;
             }
@@ -227,6 +235,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
             }
             chunks += __shfl_sync(0xFFFFFFFFu, c_inc, 31);
             keys += __shfl_sync(0xFFFFFFFFu, k_inc, 31);
+            key_pad += __reduce_add_sync(0xFFFFFFFFu, (unsigned int)(k_own - n));
             tab_used += __shfl_sync(0xFFFFFFFFu, b_inc, 31);
             ni += __popc(vm);
             nhuf += __popc(__ballot_sync(0xFFFFFFFFu, huf));
@@ -237,12 +246,11 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
             skml_set_status(p.status, SKML_CAPACITY, 0x41u);
             s.ok = 0;
         }
-        if (keys > (unsigned long long)p.key_capacity) {
+        if (keys - key_pad > (unsigned long long)p.key_capacity) {
             skml_set_status(p.status, SKML_CAPACITY, 0x40u);
             s.ok = 0;
         }
         for (int r = p.world; r <= SKML_MAX_PEERS; ++r) {
-            s.rank_chunk_begin[r] = chunks;
             s.rank_key_begin[r] = keys;
             s.rank_item_begin[r] = ni;
         }
@@ -439,57 +447,92 @@ __device__ void expand_tables(const DP& p, DecSmem& s) {
 // D1 for sparse payloads: one 1024-key chunk per block iteration, DEC_KPT adjacent keys per
 // thread (256 threads), so that every thread has several independent load chains in flight and
 // several blocks share an SM.
-__device__ void decode_accumulate(const DP& p, DecSmem& s, unsigned long long ch_begin, unsigned long long ch_end, float& dsq) {
+__device__ void decode_accumulate(const DP& p, DecSmem& s, int i_begin, int i_end, float& dsq) {
     __shared__ unsigned int s_part[6][DEC_THREADS / 32];  // [3 scans x chunk parity]
     __shared__ unsigned short s_pos[SKML_RESTART_INTERVAL];  // delta_adaptive with unary flags: where every key's flag ends
     int par = 0;
     // Every block takes a contiguous run of chunks, so that consecutive chunks belong to the same
     // (rank, group) list and its sketch table, when it fits, is staged in shared memory once and
     // then queried there: three random L2 sectors per key become one coalesced read of the table.
-    const unsigned long long per = (ch_end - ch_begin + gridDim.x - 1) / gridDim.x;
-    const unsigned long long my_begin = ch_begin + per * blockIdx.x;
-    const unsigned long long my_end = my_begin + per < ch_end ? my_begin + per : ch_end;
+    // Runs differ by one chunk at most: with equal runs (6 where 5.06 is the mean) a sixth of the blocks had none.
+    // (One range of the model per block, a share of every list, was tried for single payloads: an update alone is
+    // faster in key order, 59 against 81 us for 2.2M keys of 50M, but the shares come out uneven, 0 to 2 chunks where
+    // one is the mean, and the launch took 89 instead of 81 us, 41 instead of 25 at 0.4M keys.)
+    const unsigned long long run0 = i_begin < i_end ? s.items[i_begin].chunk_prefix : 0ull;
+    const unsigned long long run_n = (i_end < s.nitems ? s.items[i_end].chunk_prefix : s.total_chunks) - run0;
+    const unsigned int run_end = (unsigned int)(run0 + run_n * (blockIdx.x + 1) / gridDim.x);
+    unsigned int ch = (unsigned int)(run0 + run_n * blockIdx.x / gridDim.x);
+    int item = i_begin;
     unsigned char* tab_area = p.tab_off ? reinterpret_cast<unsigned char*>(&s) + p.tab_off : nullptr;
-    int staged = -1, it_i = 0;
+    int staged = -1;
     const unsigned char* stab = nullptr;
-    for (unsigned long long ch = my_begin; ch < my_end; ++ch, par ^= 1) {
-        while (it_i + 1 < s.nitems && ch >= s.items[it_i + 1].chunk_prefix) ++it_i;
-        const DecItem& it = s.items[it_i];
-        if (it_i != staged) {
-            staged = it_i;
+    const bool sums = p.out_sum != nullptr, two_phase = s.two_phase != 0, direct = s.direct != 0, adam = !direct && s.adam_plain != 0;
+    const float iw = (float)s.inv_world;
+    float* const dst = sums ? p.out_sum : p.w;
+    ChunkHead head;
+    auto fetch = [&]() {   // the head of chunk `ch`
+        while (item + 1 < i_end && ch >= s.items[item + 1].chunk_prefix) ++item;
+        head = fetch_head(s.items[item], ch - (unsigned int)s.items[item].chunk_prefix);
+    };
+    if (ch < run_end) fetch();
+    while (ch < run_end) {
+        const DecItem& it = s.items[item];
+        const unsigned int j = ch - (unsigned int)it.chunk_prefix;
+        if (item != staged) {
+            staged = item;
             stab = stage_table(it, tab_area);
         }
+        const ChunkHead now = head;
+        if (++ch < run_end) fetch();
         ChunkKeys c;
-        decode_chunk(p, it, (unsigned int)(ch - it.chunk_prefix), stab, s_part[par], s_part[2 + par], s_part[4 + par], s_pos, c);
+        decode_keys(p, it, j, now, s_part[par], s_part[2 + par], s_part[4 + par], s_pos, c);
         if (c.i0 < c.cnt) {
-            int* ks = p.key_scratch + it.key_prefix + c.first;
-            if (s.two_phase) {
+            // What the update reads does not depend on the sketch: its loads (random sectors of the model) start before
+            // the queries, for all keys of the thread at once. Keys are unique inside a payload, so no store below
+            // touches what another key of the thread loads.
+            float old[DEC_KPT], mom[DEC_KPT], vel[DEC_KPT];
+#pragma unroll
+            for (int u = 0; u < DEC_KPT; ++u) {
+                old[u] = mom[u] = vel[u] = 0.f;
+                if (c.keys[u] == 0xFFFFFFFFu) continue;
+                if (two_phase) continue;
+                if (direct) {
+                    old[u] = dst[c.keys[u]];
+                } else if (adam && !sums) {
+                    old[u] = p.w[c.keys[u]];
+                    mom[u] = p.adam_m[c.keys[u] * p.adam_stride];
+                    vel[u] = p.adam_v[c.keys[u] * p.adam_stride];
+                }
+            }
+            float bv[DEC_KPT];
+            query_keys(it, stab, c.keys, bv);
+            const unsigned long long at = it.key_prefix + c.first + c.i0;   // a multiple of four, as every list's start
+            if (two_phase) {
                 // stash (key, value): the ordered apply passes read them back coalesced
-                float* vs = p.val_scratch + it.key_prefix + c.first;
-#pragma unroll
-                for (int u = 0; u < DEC_KPT; ++u)
-                    if (c.i0 + u < c.cnt) {
-                        ks[c.i0 + u] = (int)c.keys[u];
-                        vs[c.i0 + u] = c.bv[u] * (float)s.inv_world;
-                    }
-            } else if (s.direct) {  // single payload: keys are unique inside it, plain read-modify-write
-#pragma unroll
-                for (int u = 0; u < DEC_KPT; ++u)
-                    if (c.live[u]) dsq += apply_direct(p, c.keys[u], c.bv[u] * (float)s.inv_world);
-            } else if (s.adam_plain) {  // single payload: the decoded value is the whole gradient of its key
-#pragma unroll
-                for (int u = 0; u < DEC_KPT; ++u)
-                    if (c.live[u] && c.bv[u] != 0.f) dsq += apply_one(p, c.keys[u], c.bv[u] * (float)s.inv_world);
-            } else {
+                *reinterpret_cast<int4*>(p.key_scratch + at) = make_int4((int)c.keys[0], (int)c.keys[1], (int)c.keys[2], (int)c.keys[3]);
+                *reinterpret_cast<float4*>(p.val_scratch + at) = make_float4(bv[0] * iw, bv[1] * iw, bv[2] * iw, bv[3] * iw);
+            } else if (direct) {  // single payload: keys are unique inside it, plain read-modify-write
 #pragma unroll
                 for (int u = 0; u < DEC_KPT; ++u) {
-                    if (c.i0 + u < c.cnt) ks[c.i0 + u] = (int)c.keys[u];
-                    const long long fx = c.live[u] ? to_fixed((double)c.bv[u] * s.inv_world, s.shift) : 0ll;
+                    if (c.keys[u] == 0xFFFFFFFFu) continue;
+                    const float g = bv[u] * iw, nw = sums ? old[u] + g : old[u] - p.lr * g;
+                    dst[c.keys[u]] = nw;
+                    if (!sums) dsq += (nw - old[u]) * (nw + old[u]);
+                }
+            } else if (adam) {  // single payload: the decoded value is the whole gradient of its key
+#pragma unroll
+                for (int u = 0; u < DEC_KPT; ++u)
+                    if (c.keys[u] != 0xFFFFFFFFu && bv[u] != 0.f) dsq += apply_loaded(p, c.keys[u], bv[u] * iw, old[u], mom[u], vel[u]);
+            } else {
+                *reinterpret_cast<int4*>(p.key_scratch + at) = make_int4((int)c.keys[0], (int)c.keys[1], (int)c.keys[2], (int)c.keys[3]);
+#pragma unroll
+                for (int u = 0; u < DEC_KPT; ++u) {
+                    const long long fx = c.keys[u] != 0xFFFFFFFFu ? to_fixed((double)bv[u] * s.inv_world, s.shift) : 0ll;
                     if (fx) atomicAdd(reinterpret_cast<unsigned long long*>(p.acc + c.keys[u]), (unsigned long long)fx);
                 }
             }
         }
-        // no barrier here: the next chunk's scans use the other parity of s_part
+        par ^= 1;   // no barrier here: the next chunk's scans use the other parity of s_part
     }
     __syncthreads();
 }
@@ -783,10 +826,20 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         reinterpret_cast<unsigned long long*>(p.ctrl)[9 + 4 * (int)(p.step & 1)] = t;
     }
-    if (s.direct || s.adam_plain) {
+    // Payloads applied one after the other take a pass per rank (un-fused: pass `stage - 1`), the rest one over all
+    // lists. One call for every form: the passes are most of the kernel's code.
+    const bool ordered = s.direct || s.adam_plain, per_rank = ordered && !s.two_phase;
+    for (int r = 0; r < (per_rank ? p.world : 1); ++r) {
+        if (FUSED || stage == r + 1) {
+            decode_accumulate(p, s, per_rank ? s.rank_item_begin[r] : 0, per_rank ? s.rank_item_begin[r + 1] : s.nitems, dsq);
+            if (s.any_dense && !s.two_phase) decode_accumulate_dense(p, s, per_rank ? r : 0, per_rank ? r + 1 : p.world, dsq);
+        }
+        if (FUSED && per_rank && r + 1 < p.world) {
+            if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r, passed)) return;
+        }
+    }
+    if (ordered) {
         if (s.two_phase) {
-            // Phase 1 (un-fused: stage 1): every payload's keys and values, no ordering needed.
-            if (FUSED || stage == 1) decode_accumulate(p, s, 0, s.total_chunks, dsq);
             if (FUSED) {
                 if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x2Fu, passed)) return;
                 if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -803,17 +856,6 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
             for (int r = 0; r < p.world; ++r) {
                 if (FUSED || stage == r + 2) {
                     apply_stashed(p, s.rank_key_begin[r], s.rank_key_begin[r + 1], dsq);
-                    if (s.any_dense) decode_accumulate_dense(p, s, r, r + 1, dsq);
-                }
-                if (FUSED && r + 1 < p.world) {
-                    if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r, passed)) return;
-                }
-            }
-        } else {
-            // one pass per rank; un-fused launches run pass `stage - 1` each
-            for (int r = 0; r < p.world; ++r) {
-                if (FUSED || stage == r + 1) {
-                    decode_accumulate(p, s, s.rank_chunk_begin[r], s.rank_chunk_begin[r + 1], dsq);
                     if (s.any_dense) decode_accumulate_dense(p, s, r, r + 1, dsq);
                 }
                 if (FUSED && r + 1 < p.world) {
@@ -851,10 +893,6 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
             }
         }
         return;
-    }
-    if (FUSED || stage == 1) {
-        decode_accumulate(p, s, 0, s.total_chunks, dsq);
-        if (s.any_dense) decode_accumulate_dense(p, s, 0, p.world, dsq);
     }
     if (FUSED) {
         if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x21u, passed)) return;

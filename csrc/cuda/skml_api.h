@@ -77,7 +77,7 @@ typedef struct SkmlDecodeArgs {
     float* adam_v;             // null for SGD
     double lr, adam_scale;     // Adam: scale = sqrt(1 - beta2^t) / (1 - beta1^t)
     long long* acc;            // dim fixed-point accumulators, all zero between calls
-    int* key_scratch;          // decoded keys, capacity key_capacity
+    int* key_scratch;          // decoded keys: key_capacity + 3 per (payload, group) entries (lists start at multiples of 4)
     long long key_capacity;
     double* loss_out;          // device, 4 doubles: sum over ranks of the payloads' loss partials
     float* out_sum;            // optional dense fp32 [dim]: receives the averaged decoded sum instead of updating w
@@ -87,7 +87,7 @@ typedef struct SkmlDecodeArgs {
     long long fused;
     long long grid;
     long long max_groups;      // upper bound of the payloads' group count (0 = 32): sizes the work table
-    float* val_scratch;        // decoded values, capacity key_capacity (null: SGD applies payload by payload)
+    float* val_scratch;        // decoded values, as many (null: SGD applies payload by payload)
     unsigned char* table_scratch;  // room for the sketch tables of payloads that carry them Huffman-coded (null: refused)
     long long table_capacity;      // its size in bytes
     double* weight_sumsq;          // optional device double: sum of w^2, kept current by the update (see skml_weight_norm)

@@ -238,8 +238,9 @@ class GpuDecoder:
         self.device = torch.device(device)
         self.fused, self.grid, self.budget_s = fused, grid, budget_s
         self.acc = torch.zeros(self.dim, dtype=torch.int64, device=self.device)
-        self.key_scratch = torch.zeros(self.key_capacity, dtype=torch.int32, device=self.device)
-        self.val_scratch = torch.zeros(self.key_capacity, dtype=torch.float32, device=self.device)
+        scratch = self.key_capacity + 3 * L.MAX_PEERS * max(self.max_groups, 32)   # every (payload, group) list starts at a multiple of four
+        self.key_scratch = torch.zeros(scratch, dtype=torch.int32, device=self.device)
+        self.val_scratch = torch.zeros(scratch, dtype=torch.float32, device=self.device)
         self.workspace = torch.zeros(256, dtype=torch.uint8, device=self.device)
         self.table_capacity = int(table_capacity) if table_capacity > 0 else 2 * self.key_capacity + 4096
         self.table_scratch = torch.zeros(self.table_capacity, dtype=torch.uint8, device=self.device)

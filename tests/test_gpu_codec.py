@@ -644,3 +644,28 @@ def test_dense_kind_at_ragged_dimensions(dim, q):
     want = oracle.decompress(ref)[2].astype(np.float32)
     assert np.array_equal(oracle.decompress(comp.payload_bytes(buf))[2].astype(np.float32), want)
     assert np.array_equal(GpuDecoder(dim, dim).decode_sum([buf], step=2).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("grid", [0, 2])
+@pytest.mark.parametrize("ns", [(1,), (2, 3, 7), (1023, 1025), (9001, 31, 5000, 4098)])
+def test_decode_with_exactly_the_keys_it_was_built_for(ns, grid):
+    """Lists of every remainder of four at a key capacity of their sum, one chunk to many per block: SGD against the
+    oracle's mean (fp32 sums of at most four terms of at most 1e-1: 4 * 2^-24 each, below 1e-7)."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import GpuCompressor, GpuDecoder
+    dim, P = 30011, len(ns)
+    comp = GpuCompressor(dim, max(ns), 64, 8, 3, 0.3, seed=5)
+    bufs, g = [], np.zeros(dim)
+    for r, n in enumerate(ns):
+        keys, vals = _sparse_grad(n, dim, seed=r + n, scale=1e-2)
+        vals = np.clip(vals, -0.1, 0.1)
+        b = comp.compress_local(torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda(), step=7, rank=r, world=P).clone()
+        _, k, v = oracle.decompress(comp.payload_bytes(b))
+        g[k] += v.astype(np.float32).astype(np.float64) / P
+        bufs.append(b)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(dim, device="cuda")
+    dec = GpuDecoder(dim, sum(ns), max_groups=8, grid=grid)
+    dec.decode_update([b.data_ptr() for b in bufs], [None] * P, min(b.numel() for b in bufs), 7, status, out_sum=out)
+    assert int(status.item()) == 0
+    assert np.abs(out.cpu().numpy() - g).max() < 1e-7
