@@ -1,9 +1,8 @@
 // Sparse generalized-linear-model numerics for sm_100a:
 //   * skml_glm_grad      : per-row margin, loss and coefficient, fused with the scatter of
 //                          coefficient * feature into the dense gradient accumulator
-//                          (row tiles staged into shared memory by 1-D bulk TMA copies,
-//                          one warp per row, shuffle reductions, hot columns kept in
-//                          shared memory, touched-coordinate bitmap)
+//                          (a few lanes per row, shuffle reductions, hot columns summed
+//                          in shared memory, touched-coordinate bitmap)
 //   * skml_compact_*     : touched bitmap -> sorted (key, value) list with L2 term and
 //                          the |v| > 1e-8 filter; decides sparse vs dense kind
 //   * skml_glm_validate  : margin, loss and confusion counts over a validation shard
@@ -22,205 +21,174 @@
 #include "skml_api.h"
 #include "skml_device.cuh"
 
-#define GRAD_THREADS 512
-#define GRAD_WARPS (GRAD_THREADS / 32)
-#define GRAD_TILE_CAP 4096  // elements of one staged tile (cols and values each)
+#define GRAD_THREADS 1024
 #define SKML_EPS 1e-8f
-#define GRAD_MAX_RPT 256   // rows of one tile at most
-#define GRAD_RPI 4         // rows per warp and iteration
+#define GRAD_RPI 4         // rows a warp scatters at a time
 #define GRAD_PRIV 256      // hottest columns kept once per warp
 
 __device__ __forceinline__ void red_add_f32(float* p, float v) {
     asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 
+__device__ __forceinline__ void red_add_v4(float* p, float4 v) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
 __device__ __forceinline__ void red_or_u32(unsigned int* p, unsigned int v) {
     asm volatile("red.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-struct GradSmem {
-    uint64_t bar[2];
-};
-
-// Training with a scatter: margin, loss, coefficient, coefficient * feature into the accumulator.
-__global__ void __launch_bounds__(GRAD_THREADS)
-glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
-                const float* __restrict__ labels, long long row_lo, long long row_cnt, int rows_per_tile,
-                long long nnz_padded, const float* __restrict__ w, float* __restrict__ g,
-                unsigned int* __restrict__ bitmap, int loss_id, float inv_batch, int hot, double* __restrict__ acc,
-                unsigned int* status, long long budget) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    // layout: [2 stages x cols][2 stages x vals, only if the shard stores values][hot floats]
-    __shared__ GradSmem sb;
-    __shared__ long long s_rp[GRAD_MAX_RPT + 1];
-    __shared__ float s_lab[GRAD_MAX_RPT];
-    int* s_cols = reinterpret_cast<int*>(smem_raw);
-    float* s_vals = reinterpret_cast<float*>(smem_raw + 2 * GRAD_TILE_CAP * sizeof(int));
-    const bool has_vals = vals != nullptr;
-    float* s_hot = reinterpret_cast<float*>(smem_raw + (has_vals ? 4 : 2) * GRAD_TILE_CAP * sizeof(int));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int priv = hot < GRAD_PRIV ? hot : GRAD_PRIV;  // columns [0, priv): per-warp private sums
-    float* s_priv = s_hot + hot;
-
-    for (int i = threadIdx.x; i < hot; i += blockDim.x) s_hot[i] = 0.f;
-    for (int i = threadIdx.x; i < priv * GRAD_WARPS; i += blockDim.x) s_priv[i] = 0.f;
-    if (threadIdx.x == 0) {
-        mbar_init(&sb.bar[0], 1);
-        mbar_init(&sb.bar[1], 1);
-        mbar_fence_init();
-    }
+// Training with a scatter: margin, loss, coefficient, coefficient * feature into the accumulator. Margins are taken as
+// in glm_margin_kernel below (a warp's turn is up to 32 consecutive rows, 1 << GL lanes a row); the scatter then walks
+// the same rows one warp per row, GRAD_RPI rows in flight, so that the columns a warp handles at a time are distinct
+// inside each row and the hottest `priv` of them can live in a private copy per warp, without atomics. Columns up to
+// `hot` meet in one copy per block, the rest go to L2.
+// What bounds it is same-sector traffic in L2, some 4 ns each: with a tenth of the hot columns the adds took 217 us,
+// and reading the touched bitmap (256 columns a sector) before every OR took 40. So a column is marked by the add that
+// finds it zero, one of many (whoever comes first does; a sum that passes through zero again only repeats the OR), and
+// there is one block per SM: every block flushes its hot columns to the same sectors.
+// 100,000 rows of 30: 85 -> 43 us; 50,000: 48 -> 22 us; 7,500 rows of 20: 14.4 -> 9.2 us (before: tiles staged by bulk
+// copies with two block barriers each, two blocks an SM).
+template <int GL, bool HAS_VALS>
+__global__ void __launch_bounds__(GRAD_THREADS, 1)
+glm_scatter_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
+                   const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
+                   float* __restrict__ g, unsigned int* __restrict__ bitmap, int loss_id, float inv_batch, int hot, int priv,
+                   double* __restrict__ acc) {
+    extern __shared__ __align__(16) float s_hot[];   // [hot], then [warps][priv]
+    constexpr int LANES = 1 << GL, ROWS = 32 >> GL, PER = 4;
+    const int lane = threadIdx.x & 31, sub = lane & (LANES - 1), grp = lane >> GL, nwarps = blockDim.x / 32;
+    float* const s_priv = s_hot + hot + (threadIdx.x >> 5) * priv;
+    for (int i = threadIdx.x; i < hot + nwarps * priv; i += blockDim.x) s_hot[i] = 0.f;
     __syncthreads();
-
-    const long long ntiles = (row_cnt + rows_per_tile - 1) / rows_per_tile;
+    const int bundle = ROWS * iters;
+    const long long bundles = (row_cnt + bundle - 1) / bundle, stride = (long long)gridDim.x * nwarps;
     double loss_sum = 0.0;
-    unsigned int phase[2] = {0, 0};
-
-    // Issues the bulk copies of one tile into `stage`; returns false when the tile does
-    // not fit the staging buffer (it is then read with plain loads).
-    auto tile_span = [&](long long tile, long long& a0, long long& a1) -> bool {
-        long long r0 = row_lo + tile * rows_per_tile;
-        long long r1 = r0 + rows_per_tile;
-        if (r1 > row_lo + row_cnt) r1 = row_lo + row_cnt;
-        long long e0 = rowptr[r0], e1 = rowptr[r1];
-        a0 = e0 & ~3ll;
-        a1 = (e1 + 3ll) & ~3ll;
-        if (a1 > nnz_padded) a1 = nnz_padded;
-        return (a1 - a0) <= GRAD_TILE_CAP && a1 > a0;
-    };
-    auto issue = [&](long long tile, int stage) {
-        long long a0, a1;
-        if (!tile_span(tile, a0, a1)) return;
-        unsigned int bytes = (unsigned int)(a1 - a0) * 4u;
-        mbar_expect_tx(&sb.bar[stage], has_vals ? 2 * bytes : bytes);
-        bulk_g2s(s_cols + stage * GRAD_TILE_CAP, cols + a0, bytes, &sb.bar[stage]);
-        if (has_vals) bulk_g2s(s_vals + stage * GRAD_TILE_CAP, vals + a0, bytes, &sb.bar[stage]);
-    };
-
-    long long tile = blockIdx.x;
-    if (tile < ntiles && threadIdx.x == 0) issue(tile, 0);
-    int stage = 0;
-    for (; tile < ntiles; tile += gridDim.x, stage ^= 1) {
-        long long next = tile + gridDim.x;
-        if (next < ntiles && threadIdx.x == 0) issue(next, stage ^ 1);
-        long long a0, a1;
-        bool staged = tile_span(tile, a0, a1);
-        if (staged) {
-            if (!mbar_wait(&sb.bar[stage], phase[stage], budget)) {
-                staged = false;  // never expected; read from global memory instead
-                if (threadIdx.x == 0) skml_set_status(status, SKML_TIMEOUT_BARRIER, 0x10u);
-            }
-            phase[stage] ^= 1;
-        }
-        const int* cp = staged ? (s_cols + stage * GRAD_TILE_CAP) - a0 : cols;
-        const float* vp = has_vals ? (staged ? (s_vals + stage * GRAD_TILE_CAP) - a0 : vals) : nullptr;
-        long long r0 = row_lo + tile * rows_per_tile;
-        long long r1 = r0 + rows_per_tile;
-        if (r1 > row_lo + row_cnt) r1 = row_lo + row_cnt;
-        const int nrows = (int)(r1 - r0);
-        for (int t = threadIdx.x; t <= nrows; t += blockDim.x) s_rp[t] = rowptr[r0 + t];
-        for (int t = threadIdx.x; t < nrows; t += blockDim.x) s_lab[t] = labels[r0 + t];
-        __syncthreads();
-        // GRAD_RPI rows per warp and iteration. All loads of one 32-element slice of the
-        // GRAD_RPI rows are issued before any of them is consumed, so their L2 round trips overlap.
-        for (int rb = warp * GRAD_RPI; rb < nrows; rb += GRAD_WARPS * GRAD_RPI) {
-            long long e0[GRAD_RPI];
-            int len[GRAD_RPI];
-            float sum[GRAD_RPI];
-            int maxlen = 0;
+    for (long long b = (long long)blockIdx.x * nwarps + (threadIdx.x >> 5); b < bundles; b += stride) {
+        const long long r0 = b * bundle;   // within the batch
+        const int nrows = row_cnt - r0 < bundle ? (int)(row_cnt - r0) : bundle;
+        const long long e_mine = rowptr[row_lo + r0 + (lane < nrows ? lane : nrows)];
+        const long long e_end = rowptr[row_lo + r0 + nrows];
+        const int my_row = sub * ROWS + grp;   // the row this lane evaluates
+        const float y = my_row < nrows ? labels[row_lo + r0 + my_row] : 0.f;
+        const long long base = __shfl_sync(0xFFFFFFFFu, e_mine, 0);
+        auto turn = [&](auto off_of) {   // offsets inside the bundle in 32 bits where they fit
+            using T = decltype(off_of(0ll));
+            const T mine = off_of(e_mine - base), last = off_of(e_end - base);
+            const int* __restrict__ cp = cols + base;
+            const float* __restrict__ vp = HAS_VALS ? vals + base : nullptr;
+            auto start = [&](int row) { return __shfl_sync(0xFFFFFFFFu, mine, row & 31); };
+            float pre = 0.f;
+#pragma unroll 2
+            for (int i = 0; i < iters; ++i) {
+                const int row = i * ROWS + grp;
+                const T lo = start(row), nx = start(row + 1), hi = row + 1 < 32 ? nx : last;
+                float sum = 0.f;
+                for (T k = lo + sub; k < hi; k += PER * LANES) {
+                    int c[PER];
+                    float x[PER], wv[PER];
 #pragma unroll
-            for (int u = 0; u < GRAD_RPI; ++u) {
-                const int rr = rb + u < nrows ? rb + u : nrows - 1;
-                e0[u] = s_rp[rr];
-                len[u] = rb + u < nrows ? (int)(s_rp[rr + 1] - e0[u]) : 0;
-                maxlen = max(maxlen, len[u]);
-                sum[u] = 0.f;
-            }
-            for (int off = lane; off < maxlen + lane; off += 32) {
-                if (off - lane >= maxlen) break;
-                int c[GRAD_RPI];
-                float wv[GRAD_RPI], xv[GRAD_RPI];
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u) {
-                    const bool ok = off < len[u];
-                    c[u] = ok ? cp[e0[u] + off] : -1;
-                    xv[u] = (ok && vp) ? vp[e0[u] + off] : 1.f;
-                }
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u) wv[u] = c[u] >= 0 ? __ldg(w + c[u]) : 0.f;
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u) sum[u] = fmaf(wv[u], xv[u], sum[u]);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u) sum[u] += __shfl_xor_sync(0xFFFFFFFFu, sum[u], o);
-            }
-            // Loss and coefficient of the GRAD_RPI rows are evaluated once, by lanes 0..GRAD_RPI-1 in
-            // parallel (lane u owns row rb + u) and then broadcast.
-            float pre_mine = sum[0];
-#pragma unroll
-            for (int u = 1; u < GRAD_RPI; ++u) pre_mine = lane == u ? sum[u] : pre_mine;
-            float coef_mine = 0.f;
-            if (lane < GRAD_RPI && rb + lane < nrows) {
-                const float y = s_lab[rb + lane];
-                loss_sum += (double)glm_loss(loss_id, pre_mine, y);
-                coef_mine = -glm_grad(loss_id, pre_mine, y) * inv_batch;
-            }
-            float coef[GRAD_RPI];
-#pragma unroll
-            for (int u = 0; u < GRAD_RPI; ++u) coef[u] = __shfl_sync(0xFFFFFFFFu, coef_mine, u);
-            for (int off = lane; off - lane < maxlen; off += 32) {
-                int c[GRAD_RPI];
-                float contrib[GRAD_RPI];
-                unsigned int seen[GRAD_RPI];
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u) {
-                    const bool ok = off < len[u] && coef[u] != 0.f;
-                    c[u] = ok ? cp[e0[u] + off] : -1;
-                    contrib[u] = ok ? coef[u] * (vp ? vp[e0[u] + off] : 1.f) : 0.f;
-                }
-                // cold columns: read the bitmap words first (independent L2 loads), so that
-                // the atomicOr is only issued for bits that are not set yet
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u)
-                    seen[u] = (bitmap && c[u] >= hot) ? *(volatile unsigned int*)(bitmap + (c[u] >> 5)) : ~0u;  // no bitmap: nothing to mark
-#pragma unroll
-                for (int u = 0; u < GRAD_RPI; ++u) {
-                    if (c[u] < 0) continue;
-                    if (c[u] < priv) {
-                        // the hottest columns: one private copy per warp. The lanes of a row hold
-                        // distinct columns and a warp's shared-memory accesses are ordered, so a
-                        // plain read-modify-write is exact and free of atomics.
-                        s_priv[warp * priv + c[u]] += contrib[u];
-                    } else if (c[u] < hot) {
-                        atomicAdd(&s_hot[c[u]], contrib[u]);
-                    } else {
-                        red_add_f32(g + c[u], contrib[u]);
-                        const unsigned int bit = 1u << (c[u] & 31);
-                        if (!(seen[u] & bit)) atomicOr(bitmap + (c[u] >> 5), bit);
+                    for (int u = 0; u < PER; ++u) {
+                        const bool ok = k + u * LANES < hi;
+                        c[u] = ok ? __ldg(cp + k + u * LANES) : -1;
+                        x[u] = HAS_VALS ? (ok ? __ldg(vp + k + u * LANES) : 0.f) : 1.f;
                     }
+#pragma unroll
+                    for (int u = 0; u < PER; ++u) wv[u] = c[u] >= 0 ? __ldg(w + c[u]) : 0.f;
+#pragma unroll
+                    for (int u = 0; u < PER; ++u) sum = fmaf(wv[u], x[u], sum);
                 }
                 __syncwarp();
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+                if (sub == i) pre = sum;
             }
-        }
-        __syncthreads();  // everyone is done with `stage` (and s_rp / s_lab) before it is refilled
+            float mine_coef = 0.f;
+            if (my_row < nrows) {
+                loss_sum += (double)glm_loss(loss_id, pre, y);
+                mine_coef = -glm_grad(loss_id, pre, y) * inv_batch;
+            }
+            for (int r = 0; r < nrows; r += GRAD_RPI) {
+                T lo[GRAD_RPI], hi[GRAD_RPI], longest = 0;
+                float coef[GRAD_RPI];
+#pragma unroll
+                for (int u = 0; u < GRAD_RPI; ++u) {   // rows from nrows on are empty
+                    const int row = r + u;
+                    lo[u] = start(row);
+                    const T nx = start(row + 1);
+                    hi[u] = row + 1 < 32 ? nx : last;
+                    coef[u] = __shfl_sync(0xFFFFFFFFu, mine_coef, (((row & (ROWS - 1)) << GL) | (row / ROWS)) & 31);
+                    if (row >= 32 || coef[u] == 0.f) hi[u] = lo[u];
+                    longest = max(longest, hi[u] - lo[u]);
+                }
+                for (T off = lane; off - lane < longest; off += 32) {
+                    int c[GRAD_RPI];
+                    float add[GRAD_RPI];
+                    float old[GRAD_RPI];
+#pragma unroll
+                    for (int u = 0; u < GRAD_RPI; ++u) {
+                        const bool ok = lo[u] + off < hi[u];
+                        c[u] = ok ? __ldg(cp + lo[u] + off) : -1;
+                        add[u] = HAS_VALS ? (ok ? coef[u] * __ldg(vp + lo[u] + off) : 0.f) : coef[u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < GRAD_RPI; ++u) {   // the adds first: their old values come back side by side
+                        old[u] = 1.f;
+                        if (c[u] < hot || c[u] < 0) continue;
+                        if (bitmap) old[u] = atomicAdd(g + c[u], add[u]);
+                        else red_add_f32(g + c[u], add[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < GRAD_RPI; ++u) {
+                        if (c[u] >= hot && c[u] >= 0) {
+                            if (old[u] == 0.f) red_or_u32(bitmap + (c[u] >> 5), 1u << (c[u] & 31));
+                        } else if (c[u] >= priv) {
+                            atomicAdd(&s_hot[c[u]], add[u]);
+                        }
+                        // one row's columns are distinct and a warp's accesses to shared memory are ordered: a plain
+                        // read-modify-write is exact
+                        if (c[u] >= 0 && c[u] < priv) s_priv[c[u]] += add[u];
+                        __syncwarp();
+                    }
+                }
+            }
+        };
+        if (e_end - base < (1ll << 30)) turn([](long long v) { return (int)v; });
+        else turn([](long long v) { return v; });
     }
-
+    __syncthreads();
     for (int i = threadIdx.x; i < priv; i += blockDim.x) {
         float t = s_hot[i];
-        for (int w2 = 0; w2 < GRAD_WARPS; ++w2) t += s_priv[w2 * priv + i];
+        for (int k = 0; k < nwarps; ++k) t += s_hot[hot + k * priv + i];
         s_hot[i] = t;
     }
     __syncthreads();
-    // flush the hot columns: one red.add per non-zero entry, one atomicOr per 32 columns
-    for (int base = warp * 32; base < hot; base += GRAD_WARPS * 32) {
-        int i = base + lane;
-        float v = i < hot ? s_hot[i] : 0.f;
-        unsigned int m = __ballot_sync(0xFFFFFFFFu, v != 0.f);
-        if (v != 0.f) red_add_f32(g + i, v);
-        if (bitmap && lane == 0 && m) atomicOr(bitmap + (base >> 5), m);
+    // flush the hot columns: an add per four columns with a non-zero sum (g is 16-byte aligned, or hot is 0), an OR per
+    // 32 columns where a bit is missing
+    constexpr int FLUSH = 2;
+    for (int i0 = 4 * (threadIdx.x - lane); i0 < hot; i0 += 4 * FLUSH * blockDim.x) {
+        unsigned int mark[FLUSH], word[FLUSH];
+#pragma unroll
+        for (int u = 0; u < FLUSH; ++u) {
+            const int i = i0 + u * 4 * (int)blockDim.x + 4 * lane;
+            mark[u] = 0u;
+            word[u] = ~0u;
+            if (i < hot) {
+                if (bitmap) word[u] = __ldcg(bitmap + (i >> 5));
+                const float4 v = *reinterpret_cast<const float4*>(s_hot + i);
+                mark[u] = (v.x != 0.f ? 1u : 0u) | (v.y != 0.f ? 2u : 0u) | (v.z != 0.f ? 4u : 0u) | (v.w != 0.f ? 8u : 0u);
+                if (mark[u]) red_add_v4(g + i, v);
+            }
+            mark[u] <<= 4 * (lane & 7);
+        }
+#pragma unroll
+        for (int u = 0; u < FLUSH; ++u) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) mark[u] |= __shfl_xor_sync(0xFFFFFFFFu, mark[u], o);
+            if ((lane & 7) == 0 && (mark[u] & ~word[u])) red_or_u32(bitmap + ((i0 + u * 4 * (int)blockDim.x + 4 * lane) >> 5), mark[u]);
+        }
     }
-    double tot = block_sum_double(loss_sum);
+    const double tot = block_sum_double(loss_sum);
     if (threadIdx.x == 0 && tot != 0.0) atomicAdd(&acc[0], tot);
 }
 
@@ -231,7 +199,7 @@ glm_rows_kernel(const long long* __restrict__ rowptr, const int* __restrict__ co
 // What bounds it is the number of gathers of w: a fully divergent load takes a cycle of the L1 per lane even when
 // it hits and an L1 line while it misses, so the weights of the first `hot` columns (the frequent ones where
 // indices are assigned by frequency) are kept in shared memory, which serves some ten lanes a cycle, and nothing
-// is staged that would take L1 away. 500,000 rows of 30: 80 -> 73 us; 1M rows of 30 with values: 208 -> 109 us
+// is staged that would take L1 away. 500,000 rows of 30: 80 -> 61 us; 1M rows of 30 with values: 208 -> 102 us
 // (before: a warp per row, tiles staged by bulk copies, 103 warp instructions per 32 entries).
 #define MARGIN_THREADS 512
 template <int MODE, int GL, bool HAS_VALS>
@@ -346,28 +314,53 @@ static int margin_hot(long long entries, long long blocks, long long dim, const 
     return hot < 1024 || ((uintptr_t)w & 15) ? 0 : (int)hot;
 }
 
+// Rows of a warp's turn (iterations of 32 >> gl rows, 1 << gl at most), warps per block and blocks, for blocks of at
+// most `max_warps` warps, `per_sm` of them on an SM. Few rows: one turn for every warp slot of the chip, down to one
+// iteration, in blocks of as many warps as spread the turns over all SMs. Many: of the turn lengths from half the
+// maximum on, the one whose last round of turns is fullest (500,000 rows in turns of 32 are 2.2 rounds, of 24 are 2.93).
+struct TurnShape {
+    int iters, warps, grid;
+};
+static TurnShape turn_shape(long long row_cnt, int gl, int max_warps, int per_sm) {
+    const long long blocks = (long long)per_sm * sm_count(), slots = blocks * max_warps, rows = 32 >> gl;
+    const int most = 1 << gl;
+    auto turns = [&](long long iters) { return (row_cnt + rows * iters - 1) / (rows * iters); };
+    TurnShape t;
+    const long long even = (row_cnt + rows * slots - 1) / (rows * slots);   // iterations in a single round
+    t.iters = even < 1 ? 1 : (int)(even < most ? even : most);
+    if (even > most) {
+        double best = 0.0;
+        for (int it = most; it >= (most + 1) / 2; --it) {
+            const long long n = turns(it);
+            const double fill = (double)n / (double)((n + slots - 1) / slots * slots);
+            if (fill > best + 0.02) {
+                best = fill;
+                t.iters = it;
+            }
+        }
+    }
+    const long long n = turns(t.iters);
+    long long warps = (n + blocks - 1) / blocks;
+    if (warps > max_warps) warps = max_warps;
+    t.warps = (int)warps;
+    const long long grid = (n + warps - 1) / warps;
+    t.grid = (int)(grid < blocks ? grid : blocks);
+    return t;
+}
+
 template <int MODE, int GL>
 static int margin_launch_gl(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
                             long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
                             float* out, cudaStream_t stream) {
-    // rows of a warp's turn: as many as leave every warp slot of the chip (three blocks of 16 warps an SM) a turn,
-    // down to one trip; then blocks of as many warps as spread the turns over all SMs
-    const long long slots = 3ll * sm_count() * (MARGIN_THREADS / 32), rows = 32 >> GL;
-    long long iters = row_cnt / (rows * slots);
-    if (iters < 1) iters = 1;
-    if (iters > (1 << GL)) iters = 1 << GL;
-    const long long bundles = (row_cnt + rows * iters - 1) / (rows * iters);
-    long long warps = (bundles + 3ll * sm_count() - 1) / (3ll * sm_count());
-    if (warps > MARGIN_THREADS / 32) warps = MARGIN_THREADS / 32;
-    long long grid = (bundles + warps - 1) / warps;
-    if (grid > 3ll * sm_count()) grid = 3ll * sm_count();
+    const TurnShape t = turn_shape(row_cnt, GL, MARGIN_THREADS / 32, 3);
+    const int iters = t.iters, warps = t.warps, grid = t.grid;
     const int hot = margin_hot((long long)(row_cnt * avg_nnz), grid, dim, w);
     if (vals)
         glm_margin_kernel<MODE, GL, true><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, (int)iters, w, hot, loss_id, inv_batch, acc, out);
+            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out);
     else
         glm_margin_kernel<MODE, GL, false><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, (int)iters, w, hot, loss_id, inv_batch, acc, out);
+            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out);
     return (int)cudaGetLastError();
 }
 
@@ -382,30 +375,37 @@ static int margin_launch(const long long* rowptr, const int* cols, const float* 
     return go(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, inv_batch, acc, out, stream);
 }
 
-static int grad_launch(const long long* rowptr, const int* cols, const float* vals, const float* labels,
-                       long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz, const float* w,
-                       float* g, unsigned int* bitmap, int loss_id, float inv_batch, int hot, double* acc,
-                       unsigned int* status, long long budget, cudaStream_t stream) {
-    if (row_cnt <= 0) return 0;
-    if (hot < 0) hot = 0;
+// Columns summed per block: no more than the caller allows, and only those whose adds would queue up in L2: with
+// frequencies falling like 1 / rank, rank r of E entries gets about E / (9 r), so a sector of eight columns is busy
+// for a microsecond (10 ns an add) down to rank E / 110. The others would only lengthen the flush (7,500 rows of 20:
+// 15 us with 8192 columns). Hot columns leave in 16-byte units.
+static int grad_hot(long long entries, int limit, const float* g) {
+    long long hot = entries / 128;
+    if (hot < GRAD_PRIV) hot = GRAD_PRIV;
     if (hot > 16384) hot = 16384;
-    hot &= ~31;
-    int rpt = (int)(GRAD_TILE_CAP * 0.8 / (avg_nnz > 1.0 ? avg_nnz : 1.0));
-    if (rpt < 1) rpt = 1;
-    if (rpt > GRAD_MAX_RPT) rpt = GRAD_MAX_RPT;
-    long long ntiles = (row_cnt + rpt - 1) / rpt;
-    size_t smem = (vals ? 4 : 2) * GRAD_TILE_CAP * sizeof(int) + (size_t)hot * sizeof(float) +
-                  (size_t)(hot < GRAD_PRIV ? hot : GRAD_PRIV) * GRAD_WARPS * sizeof(float);
-    int per_sm = smem > 100 * 1024 ? 1 : (smem > 70 * 1024 ? 2 : 3);
-    long long grid = (long long)sm_count() * per_sm;
-    if (grid > ntiles) grid = ntiles;
+    if (hot > limit) hot = limit;
+    return hot < 0 || ((uintptr_t)g & 15) ? 0 : (int)(hot & ~31ll);
+}
+
+template <int GL>
+static int grad_launch_gl(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
+                          long long row_cnt, double avg_nnz, const float* w, float* g, unsigned int* bitmap, int loss_id,
+                          float inv_batch, int hot_limit, double* acc, cudaStream_t stream) {
+    const TurnShape t = turn_shape(row_cnt, GL, GRAD_THREADS / 32, 1);
+    const int hot = grad_hot((long long)(row_cnt * avg_nnz), hot_limit, g), priv = hot < GRAD_PRIV ? hot : GRAD_PRIV;
+    const size_t smem = ((size_t)hot + (size_t)priv * t.warps) * sizeof(float);
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(glm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(glm_scatter_kernel<GL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        cudaFuncSetAttribute(glm_scatter_kernel<GL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
         attr_set = true;
     }
-    glm_rows_kernel<<<(unsigned)grid, GRAD_THREADS, smem, stream>>>(
-        rowptr, cols, vals, labels, row_lo, row_cnt, rpt, nnz_padded, w, g, bitmap, loss_id, inv_batch, hot, acc, status, budget);
+    if (vals)
+        glm_scatter_kernel<GL, true><<<t.grid, 32 * t.warps, smem, stream>>>(rowptr, cols, vals, labels, row_lo, row_cnt, t.iters, w, g,
+                                                                            bitmap, loss_id, inv_batch, hot, priv, acc);
+    else
+        glm_scatter_kernel<GL, false><<<t.grid, 32 * t.warps, smem, stream>>>(rowptr, cols, vals, labels, row_lo, row_cnt, t.iters, w, g,
+                                                                             bitmap, loss_id, inv_batch, hot, priv, acc);
     return (int)cudaGetLastError();
 }
 
@@ -413,8 +413,12 @@ extern "C" int skml_glm_grad(const long long* rowptr, const int* cols, const flo
                              long long row_lo, long long row_cnt, long long nnz_padded, double avg_nnz,
                              const float* w, float* g, unsigned int* bitmap, int loss_id, float inv_batch, int hot,
                              double* loss_acc, unsigned int* status, long long budget, void* stream) {
-    return grad_launch(rowptr, cols, vals, labels, row_lo, row_cnt, nnz_padded, avg_nnz, w, g, bitmap, loss_id,
-                       inv_batch, hot, loss_acc, status, budget, (cudaStream_t)stream);
+    (void)nnz_padded;
+    (void)status;
+    (void)budget;   // nothing in it waits
+    if (row_cnt <= 0) return 0;
+    auto go = avg_nnz <= 16.0 ? grad_launch_gl<2> : avg_nnz <= 40.0 ? grad_launch_gl<3> : avg_nnz <= 96.0 ? grad_launch_gl<4> : grad_launch_gl<5>;
+    return go(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, g, bitmap, loss_id, inv_batch, hot, loss_acc, (cudaStream_t)stream);
 }
 
 extern "C" int skml_glm_validate(const long long* rowptr, const int* cols, const float* vals, const float* labels,
@@ -429,24 +433,24 @@ extern "C" int skml_glm_validate(const long long* rowptr, const int* cols, const
 
 // ---------------------------------------------------------------------------
 // Compaction of the touched bitmap into a sorted sparse gradient. A warp owns `wpw` consecutive bitmap
-// words, walked 32 at a time; the count pass leaves one count per warp, and every block of the write
-// pass adds up the counts before its own, so there is no scan launch in between.
+// words, walked 32 at a time; the count pass leaves one count per warp and one per block, and every block of
+// the write pass adds up the blocks before its own, so there is no scan launch in between.
 // What bounds it is the chain bitmap word -> g and w -> stores of each group of 32 words, so the split is
-// by latency: as few words per warp as the count array allows (wpw = 8 up to 1M coordinates), which spreads
-// 100k coordinates over 49 blocks. (One 1024-thread block per 131,072 coordinates, the split before, put
-// them on one SM: 39 + 2 + 30 us; 1M coordinates on eight: 55 + 2 + 31 us.)
+// by latency: as few words per warp as the count array allows (wpw = 8 up to 4M coordinates, one group of 32 up
+// to 16M), which spreads 100k coordinates over 49 blocks. (One 1024-thread block per 131,072 coordinates put
+// them on one SM: 39 + 2 + 30 us; 1M coordinates on eight: 55 + 2 + 31 us. Four groups a warp at 10M: 29 + 23 us.)
 // meta[0] = nnz, meta[1] = kind (1 sparse, 2 dense, 0 empty)
 // ---------------------------------------------------------------------------
 #define COMPACT_THREADS 256
 #define COMPACT_WARPS (COMPACT_THREADS / 32)
 #define COMPACT_MIN_WPW 8
-#define COMPACT_MAX_COUNTS 4096  // warps at most: every block of the write pass reads all counts (16 KB)
+#define COMPACT_MAX_BLOCKS 2048  // every block of the write pass reads the totals of all (8 KB)
 #define COMPACT_SPARSE_BITS 4    // words with at most this many bits are walked by one lane
 #define COMPACT_DENSE_BATCH 8    // dense words whose loads are in flight together
 
 struct CompactShape {
     int wpw;      // bitmap words per warp: the smallest power of two from COMPACT_MIN_WPW that needs no more than
-                  // COMPACT_MAX_COUNTS warps
+                  // COMPACT_MAX_BLOCKS blocks
     int nwarps, nblocks;
 };
 
@@ -454,7 +458,7 @@ static CompactShape compact_shape(long long dim) {
     const long long nwords = (dim + 31) / 32;
     CompactShape c;
     c.wpw = COMPACT_MIN_WPW;
-    while (nwords > (long long)c.wpw * COMPACT_MAX_COUNTS) c.wpw *= 2;
+    while (nwords > (long long)c.wpw * COMPACT_WARPS * COMPACT_MAX_BLOCKS) c.wpw *= 2;
     c.nwarps = (int)((nwords + c.wpw - 1) / c.wpw);
     c.nblocks = (c.nwarps + COMPACT_WARPS - 1) / COMPACT_WARPS;
     return c;
@@ -469,10 +473,10 @@ compact_count_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
     // The filtered value g + lambda * w is stored back into g so that the write pass reads one
     // array only.
     const int lane = threadIdx.x & 31;
+    __shared__ unsigned int s_cnt[COMPACT_WARPS];
     const int gw = blockIdx.x * COMPACT_WARPS + (threadIdx.x >> 5);
-    if (gw >= nwarps) return;
     const long long wbase = (long long)gw * wpw;
-    const long long wend = wbase + wpw < nwords ? wbase + wpw : nwords;
+    const long long wend = gw >= nwarps ? wbase : (wbase + wpw < nwords ? wbase + wpw : nwords);
     unsigned int cnt = 0;
     unsigned int next = wbase + lane < wend ? bitmap[wbase + lane] : 0u;
     for (long long gbase = wbase; gbase < wend; gbase += 32) {
@@ -547,7 +551,17 @@ compact_count_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
         cnt += __popc(keep);
     }
     cnt = warp_sum(cnt);
-    if (lane == 0) warp_counts[gw] = cnt;
+    if (lane == 0) {
+        s_cnt[threadIdx.x >> 5] = cnt;
+        if (gw < nwarps) warp_counts[gw] = cnt;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned int t = 0;
+#pragma unroll
+        for (int i = 0; i < COMPACT_WARPS; ++i) t += s_cnt[i];
+        warp_counts[nwarps + blockIdx.x] = t;
+    }
 }
 
 __global__ void __launch_bounds__(COMPACT_THREADS)
@@ -562,10 +576,10 @@ compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
     const long long wend = gw >= nwarps ? wbase : (wbase + wpw < nwords ? wbase + wpw : nwords);
     unsigned int next = wbase + lane < wend ? bitmap[wbase + lane] : 0u;   // in flight while the counts are added up
     unsigned int before = 0, total = 0;
-    for (int i = threadIdx.x; i < nwarps; i += COMPACT_THREADS) {
-        const unsigned int c = warp_counts[i];
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += COMPACT_THREADS) {
+        const unsigned int c = warp_counts[nwarps + i];
         total += c;
-        if (i < gw0) before += c;
+        if (i < (int)blockIdx.x) before += c;
     }
     before = warp_sum(before);
     total = warp_sum(total);
@@ -711,7 +725,10 @@ extern "C" int skml_compact(float* g, const float* w, unsigned int* bitmap, int 
 }
 
 // Entries of the caller's count array.
-extern "C" long long skml_compact_blocks(int dim) { return compact_shape(dim).nwarps; }
+extern "C" long long skml_compact_blocks(int dim) {
+    const CompactShape c = compact_shape(dim);
+    return c.nwarps + c.nblocks;
+}
 
 // ---------------------------------------------------------------------------
 // Updates for the uncompressed baselines (the compressed path updates inside the
@@ -1018,7 +1035,7 @@ extern "C" int skml_sm_count() { return sm_count(); }
 // ---------------------------------------------------------------------------
 // Transposed-index gradient. For a shard whose minibatches are fixed row slices, the batch's
 // column-major index (distinct columns, their row lists) is built once. A step then needs the
-// per-row coefficients (glm_rows_kernel<2>) and, per distinct column c of the batch,
+// per-row coefficients (glm_margin_kernel<2>) and, per distinct column c of the batch,
 //     value[c] = sum over the batch rows r that contain c of coef[r] * x[r][c]  +  lambda * w[c],
 // which is a gather of coefficients (an L2-resident array of batch-size floats) instead of a
 // scatter into the dim-sized accumulator: no atomics, no touched bitmap, no compaction, and the
@@ -1332,7 +1349,7 @@ extern "C" int skml_colsum_tiled(const int* tile_pair_ptr, const int* pair_ptr, 
 // skml_compact_noalloc: the compaction above for callers that must not allocate.
 // (Declared and documented in skml_noalloc.h; it has no counterpart in the reference.)
 //
-// The only scratch memory of the compaction is the per-block count / offset array. Here
+// The only scratch memory of the compaction is the array of counts. Here
 // it lives in a file-scope device array instead of a caller-supplied buffer, so the call
 // needs no cudaMalloc, no cudaFree and no allocating library routine.
 // ---------------------------------------------------------------------------
@@ -1342,7 +1359,8 @@ extern "C" int skml_colsum_tiled(const int* tile_pair_ptr, const int* pair_ptr, 
 
 #include "skml_noalloc.h"
 
-static __device__ __align__(256) unsigned int g_noalloc_block_counts[SKML_NOALLOC_MAX_BLOCKS + 64];
+// one count per warp and one per block of the largest shape
+static __device__ __align__(256) unsigned int g_noalloc_block_counts[(COMPACT_WARPS + 1) * COMPACT_MAX_BLOCKS];
 
 #define NOALLOC_MAX_DEVICES 64
 static unsigned int* g_noalloc_scratch_ptr[NOALLOC_MAX_DEVICES];  // device address of the array, per device
@@ -1381,8 +1399,7 @@ extern "C" int skml_compact_noalloc(float* g, const float* w, unsigned int* bitm
     unsigned int* scratch = nullptr;
     int rc = noalloc_scratch(&scratch);
     if (rc) return rc;
-    // every entry of the scratch that is read (one per warp, at most COMPACT_MAX_COUNTS) is rewritten by the count
-    // kernel of this call, so nothing of an earlier call has to be cleared
-    static_assert(COMPACT_MAX_COUNTS <= SKML_NOALLOC_MAX_BLOCKS + 64, "the built-in scratch holds one count per warp");
+    // every entry of the scratch that is read (one per warp and block) is rewritten by the count kernel of this
+    // call, so nothing of an earlier call has to be cleared
     return compact_launch(g, w, bitmap, dim, lambda, scratch, meta, keys, vals, nullptr, capacity, status, (cudaStream_t)stream_);
 }

@@ -17,7 +17,7 @@
 // kind is never chosen here). Inputs and outputs are still the caller's buffers.
 //
 // Where the scratch lives: in a device array compiled into the library
-// (SKML_NOALLOC_MAX_BLOCKS + 64 unsigned ints, about 16 KB). Every GPU that loads the
+// (one count per warp and block of the launch, 72 KB). Every GPU that loads the
 // library holds that array until the process exits.
 //
 // Limits and rules:

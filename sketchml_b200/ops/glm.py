@@ -12,7 +12,7 @@ from . import lib as L
 
 class DeviceCSR:
     """A CSR shard in device memory, with ``cols`` / ``values`` padded to a multiple of 4
-    elements so that 16-byte bulk copies of row tiles never read past the allocation."""
+    elements so that 16-byte loads never read past the allocation."""
 
     def __init__(self, m: CSRMatrix, device):
         dev = torch.device(device)

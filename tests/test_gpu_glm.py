@@ -366,3 +366,36 @@ def test_near_dense_index_matches_the_scatter_path(rows, dim, nnz, tile, binary,
     glm_grad(csr, [(lead, rows + lead)], w, st, loss.loss_id, rows, hot=256)
     compact_gradient(st, w, loss.lam)
     assert kinds == [int(st.meta[0]), int(st.meta[1])] and int(st.status.item()) == 0
+
+
+@pytest.mark.parametrize("binary", [True, False])
+@pytest.mark.parametrize("hot", [0, 32, 8192])
+@pytest.mark.parametrize("rows,nnz,dim", [(1, (1, 1), 64), (3, (0, 5), 400), (33, (0, 40), 3000), (700, (90, 300), 9001),
+                                          (5000, (0, 45), 9001)])
+def test_scatter_gradient_is_exact_on_whole_numbers(rows, nnz, dim, hot, binary):
+    """Square loss on weights, values and labels of -1, 0, 1: every sum is a whole number below 2^24, so fp32 adds in
+    any order give the fp64 gradient itself. Empty rows, rows longer than a warp, ragged last turns, no shared columns,
+    private ones only, and more than the batch is worth."""
+    from sketchml_b200.models.loss import L2SquareLoss
+    from sketchml_b200.ops import DeviceCSR, GlmState, compact_gradient, glm_grad
+    rng = np.random.default_rng(rows)
+    m = _random_csr(rows, dim, nnz[0], nnz[1], seed=rows + 1, binary=True, zipf=False)
+    if not binary:
+        m.values = torch.from_numpy(rng.integers(-1, 2, m.cols.numel()).astype(np.float32))
+    x = torch.ones(m.cols.numel(), dtype=torch.float64) if binary else m.values.double()
+    w = torch.from_numpy(rng.integers(-1, 2, dim).astype(np.float32))
+    dev = torch.device("cuda")
+    st = GlmState.create(dim, dim, dev)
+    st.partials.zero_()
+    loss = L2SquareLoss(0.0)
+    glm_grad(DeviceCSR(m, dev), [(0, rows)], w.to(dev), st, loss.loss_id, 1, hot=hot)
+    rid = torch.repeat_interleave(torch.arange(rows), m.rowptr[1:] - m.rowptr[:-1])
+    pre = torch.zeros(rows, dtype=torch.float64).index_add_(0, rid, w.double()[m.cols.long()] * x)
+    want = torch.zeros(dim, dtype=torch.float64).index_add_(0, m.cols.long(), (pre - m.labels.double())[rid] * x)
+    assert torch.equal(st.g.cpu().double(), want)
+    assert float(st.partials[1]) == float(0.5 * (pre - m.labels.double()).square().sum())
+    compact_gradient(st, w.to(dev), 0.0)
+    n = int(st.meta[0])
+    assert torch.equal(st.keys[:n].cpu().long(), torch.nonzero(want).flatten())
+    assert torch.equal(st.vals[:n].cpu().double(), want[want != 0])
+    assert float(st.g.abs().max()) == 0.0 and int(st.bitmap.abs().max()) == 0 and int(st.status.item()) == 0
