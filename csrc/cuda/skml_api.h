@@ -268,6 +268,26 @@ int skml_enable_peer_access(int peer_device);
 #ifdef __cplusplus
 extern "C" {
 #endif
+// What a step does with its sparse gradient instead of compress + decode where one process trains with a baseline
+// compressor: the values become what their codes decode to, then the touched coordinates are updated.
+typedef struct SkmlCodedArgs {
+    long long kind;                    // 0: values as they are, 1: FixedPoint codes, 2: ZipML codes
+    long long bits;                    // FixedPoint: bits of a code; ZipML: buckets
+    unsigned long long seed;           // FixedPoint: of this step
+    void* scratch;
+    long long scratch_bytes;
+    unsigned char* codes;
+    long long code_stride;
+    double* norm;                      // FixedPoint
+    float* splits;                     // ZipML, as in skml_zipml_pack
+    float* mids;
+    int* zip_meta;
+    float* range;
+    float* adam_m;                     // null: SGD
+    float* adam_v;
+    long long adam_stride;
+} SkmlCodedArgs;
+
 // One training step (gradient -> compaction -> fused compress -> fused decode + update) as a
 // single call, so that the host spends one library call per step instead of five.
 typedef struct SkmlStepArgs {
@@ -330,6 +350,7 @@ typedef struct SkmlStepArgs {
     float* tt_partial;                 // device scratch [>= pairs]
     long long tt_tiles, tt_tile_rows, tt_rows;
     const SkmlDenseIndex* dense_index; // near-dense batch (null = not one): the gradient comes from its tiled copies
+    const SkmlCodedArgs* coded;        // baseline compressor (null = compress and decode above)
 } SkmlStepArgs;
 
 int skml_train_step(SkmlStepArgs* args, void* stream);

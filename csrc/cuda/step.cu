@@ -14,8 +14,44 @@ static int batch_consumed(const SkmlStepArgs* a, cudaStream_t stream) {
     return (int)cudaEventRecord((cudaEvent_t)a->grad_done_event, stream);
 }
 
+// The gradient's way into the model: through the fused compress and decode kernels, or through a baseline's codes.
+// `batch_keys`: keys and count lie in the batch's own buffers, which are the feeder's again once they are read.
+static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* meta, float* vals, float* dense_vals, bool batch_keys,
+                          void* stream) {
+    if (a->coded) {
+        const SkmlCodedArgs& c = *a->coded;
+        int rc = 0;
+        if (c.kind == 1) {
+            rc = skml_fixedpoint_pack(vals, meta, a->n_max, (int)c.bits, c.seed, (double*)c.scratch, c.codes, c.norm, stream);
+            if (!rc) rc = skml_fixedpoint_unpack_scatter(nullptr, keys, c.codes, c.norm, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals, stream);
+        } else if (c.kind == 2) {
+            rc = skml_zipml_pack(vals, meta, a->n_max, (int)c.bits, c.scratch, c.scratch_bytes, c.splits, c.mids, c.zip_meta, c.range, c.codes, stream);
+            if (!rc) rc = skml_zipml_unpack_scatter(nullptr, keys, c.codes, c.mids, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals, stream);
+        }
+        if (rc) return rc;
+        rc = skml_update_sparse(a->w, c.adam_m, c.adam_v, keys, vals, meta, a->n_max, 1.f, c.adam_v != nullptr, (float)a->lr,
+                                (float)a->adam_scale, (int)c.adam_stride, stream);
+        if (!rc && batch_keys) rc = batch_consumed(a, (cudaStream_t)stream);
+        if (rc) return rc;
+        return (int)cudaMemcpyAsync(a->loss_out, a->partials, 4 * sizeof(double), cudaMemcpyDeviceToDevice, (cudaStream_t)stream);
+    }
+    a->compress->step = a->step;
+    a->compress->keys = keys;
+    a->compress->meta = meta;
+    a->compress->vals = vals;
+    if (dense_vals) a->compress->dense_vals = dense_vals;   // one launch serves both kinds
+    int rc = skml_compress_sparse(a->compress, stream);
+    if (!rc && batch_keys) rc = batch_consumed(a, (cudaStream_t)stream);
+    if (rc) return rc;
+    a->decode->step = a->step;
+    a->decode->lr = a->lr;
+    a->decode->adam_scale = a->adam_scale;
+    a->decode->loss_out = a->loss_out;
+    return skml_decode_update(a->decode, stream);
+}
+
 extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
-    if (!a || !a->compress || !a->decode) return (int)cudaErrorInvalidValue;
+    if (!a || (!a->coded && (!a->compress || !a->decode))) return (int)cudaErrorInvalidValue;
     cudaStream_t stream = (cudaStream_t)stream_;
     if (a->t_colptr || a->tt_pair_ptr) {
         // transposed index: coefficients per row, then one gather-sum per distinct column
@@ -37,17 +73,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         if (rc) return rc;
         rc = batch_consumed(a, stream);
         if (rc) return rc;
-        a->compress->step = a->step;
-        a->compress->keys = a->t_ucols;
-        a->compress->meta = a->t_meta;
-        a->compress->vals = a->gvals;
-        rc = skml_compress_sparse(a->compress, stream_);
-        if (rc) return rc;
-        a->decode->step = a->step;
-        a->decode->lr = a->lr;
-        a->decode->adam_scale = a->adam_scale;
-        a->decode->loss_out = a->loss_out;
-        return skml_decode_update(a->decode, stream_);
+        return apply_gradient(a, a->t_ucols, a->t_meta, a->gvals, nullptr, false, stream_);
     }
     cudaError_t e = cudaMemcpyAsync(a->partials, a->partials_template, 4 * sizeof(double), cudaMemcpyDeviceToDevice, stream);
     if (e != cudaSuccess) return (int)e;
@@ -65,19 +91,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         }
         rc = skml_finalize_compact(a->gc, a->wc, (float)a->lambda, n, a->gvals, nullptr, stream_);  // no touched bitmap: every slot is a key
         if (rc) return rc;
-        a->compress->step = a->step;
-        a->compress->keys = a->l_ucols;
-        a->compress->meta = a->l_meta;
-        a->compress->vals = a->gvals;
-        rc = skml_compress_sparse(a->compress, stream_);
-        if (rc) return rc;
-        rc = batch_consumed(a, stream);  // the compress kernel still reads the batch's column list and count
-        if (rc) return rc;
-        a->decode->step = a->step;
-        a->decode->lr = a->lr;
-        a->decode->adam_scale = a->adam_scale;
-        a->decode->loss_out = a->loss_out;
-        return skml_decode_update(a->decode, stream_);
+        return apply_gradient(a, a->l_ucols, a->l_meta, a->gvals, nullptr, true, stream_);
     }
     if (a->dense_index) {
         int rc = skml_dt_gradient(a->dense_index, a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->nnz_padded, a->avg_nnz, a->w,
@@ -97,16 +111,5 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
     rc = skml_compact(a->g, a->w, a->bitmap, (int)a->dim, (float)a->lambda, a->block_counts, a->meta, a->keys,
                           a->gvals, a->dense_vals, a->n_max, a->status, stream_);
     if (rc) return rc;
-    a->compress->step = a->step;
-    a->compress->keys = a->keys;
-    a->compress->meta = a->meta;
-    a->compress->vals = a->gvals;
-    a->compress->dense_vals = a->dense_vals;   // one launch serves both kinds
-    rc = skml_compress_sparse(a->compress, stream_);
-    if (rc) return rc;
-    a->decode->step = a->step;
-    a->decode->lr = a->lr;
-    a->decode->adam_scale = a->adam_scale;
-    a->decode->loss_out = a->loss_out;
-    return skml_decode_update(a->decode, stream_);
+    return apply_gradient(a, a->keys, a->meta, a->gvals, a->dense_vals, false, stream_);
 }

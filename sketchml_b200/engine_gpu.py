@@ -154,6 +154,7 @@ class GpuEngine:
             elif self.value_quant == C.COMPRESSOR_ZIP:
                 from .ops.baseline_quant import ZipCodec
                 self.zip_codec = ZipCodec(bound, conf.quant_bin_num, comm.world, self.device)
+            self._prepare_fast_step()
         else:
             self.dense_sum = torch.zeros(dim, dtype=torch.float32, device=self.device)
         # the prepared gradient path serves every arm alike (the uncompressed baselines too)
@@ -161,13 +162,13 @@ class GpuEngine:
         self._build_transposed_index()
 
     def _prepare_fast_step(self) -> None:
-        """Argument blocks of the single-call step (`skml_train_step`), one per slot parity."""
+        """Argument blocks of the single-call step (`skml_train_step`): one per slot parity, or a baseline codec's."""
         import ctypes as CT
         m, st, comm, conf = self.t.model, self.st, self.t.comm, self.conf
         opt = m.optimizer
         am, av = (opt.m, opt.v) if self.adam else (None, None)
-        self._ca, self._da = [], []
-        for par in (0, 1):
+        self._ca, self._da, self._coded = [], [], None
+        for par in (0, 1) if self.mode == "sketch" else ():
             sp, sf = self.xchg.send_ptrs(par)
             rp, rf = self.xchg.recv_ptrs(par)
             self._ca.append(self.comp.make_args(st.keys, st.vals, st.meta, 0, comm.rank, comm.world, sp[comm.rank],
@@ -182,6 +183,13 @@ class GpuEngine:
         a.lam = m.loss.get_reg_param() if m.loss.is_l2_reg else 0.0
         a.block_counts, a.meta, a.keys, a.gvals = L.ptr(st.block_counts), L.ptr(st.meta), L.ptr(st.keys), L.ptr(st.vals)
         a.dense_vals, a.n_max, a.dim = L.ptr(st.dense_vals), st.n_max, st.dim
+        if self.mode != "sketch":
+            codec = self.fp_codec or self.zip_codec
+            self._coded = L.CodedArgs() if codec is None else codec.coded_args()
+            if self.adam:
+                from .ops.glm import moment_stride
+                self._coded.adam_m, self._coded.adam_v, self._coded.adam_stride = L.ptr(am), L.ptr(av), moment_stride(am, av)
+            a.coded = CT.pointer(self._coded)
         self._sa = a
         self._step_fn = L.lib().skml_train_step
         self._byref = CT.byref
@@ -295,15 +303,20 @@ class GpuEngine:
         else:
             a.l_ucols = None
         self._last_index = bi
-        par = step & 1
-        a.compress = self._ca_ptr[par]
-        a.decode = self._da_ptr[par]
+        coded = self._coded
+        if coded is None:
+            par = step & 1
+            a.compress = self._ca_ptr[par]
+            a.decode = self._da_ptr[par]
+        elif coded.kind == 1:
+            coded.seed = self._fp_seed(step) & (2 ** 64 - 1)
         a.step, a.lr, a.adam_scale, a.loss_out = step, lr, adam_scale, ring_ptr
         L.check(self._step_fn(self._byref(a), L.stream()), "skml_train_step")
+        tail = 2 if coded is None else (1, 4, 6)[coded.kind]   # compress, decode; or pack, unpack, update
         if lid is not None:
-            L.count_launches(len(segs) + 2 + 2)  # gather, gradient segment(s), finalize, compress, decode
+            L.count_launches(len(segs) + 2 + tail)  # gather, gradient segment(s), finalize
         else:
-            L.count_launches((3 if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + 1 + 1)
+            L.count_launches((3 if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + tail)
 
     # ----------------------------------------------------------------- steps
     def _segments(self, count: int):
@@ -425,7 +438,8 @@ class GpuEngine:
         return self._fast_ok()
 
     def _fast_ok(self) -> bool:
-        return (self.mode == "sketch" and getattr(self, "depth", 0) == 0 and bool(self.conf.extras.get("single_call_step", True)) and
+        one_call = self.mode == "sketch" or (self.mode == "nccl_kv" and self.t.comm.world == 1)
+        return (one_call and getattr(self, "depth", 0) == 0 and bool(self.conf.extras.get("single_call_step", True)) and
                 bool(self.conf.extras.get("fused", True)) and
                 not (self.t.injector is not None and self.t.injector.skip_publish_steps))
 
@@ -442,6 +456,10 @@ class GpuEngine:
         opt = m.optimizer
         am, av = (opt.m, opt.v) if self.adam else (None, None)
         ring = self.loss_ring[self.batch_index % self.loss_ring.shape[0]]
+        if self.mode == "nccl_kv" and getattr(self, "_pending", None) is not None:
+            self._launch_fast_step(step, lr, adam_scale, ring.data_ptr())
+            self.batch_index += 1
+            return
         if self.mode == "sketch" and getattr(self, "_pending", None) is not None:
             self._launch_fast_step(step, lr, adam_scale, ring.data_ptr())
             if self.conf.extras.get("check_status_every_step", False):
@@ -629,7 +647,8 @@ class GpuEngine:
     def payload_stats(self, step: int):
         """(nnz, payload bytes) of this rank's last payload (synchronises)."""
         if self.mode != "sketch":
-            n = int(self.st.meta[0])
+            index = getattr(self, "_last_index", None)
+            n = index.n_cols if index is not None else int(self.st.meta[0])
             return n, 8 * n
         buf = self.xchg.local_slot(step, self.t.comm.rank)
         head = buf[:256].cpu().numpy()

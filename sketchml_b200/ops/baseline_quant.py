@@ -52,6 +52,13 @@ class FixedPointCodec:
                                                         L.stream()), "skml_fixedpoint_unpack_scatter")
         L.count_launches(lists)  # one launch per list: the lists reach a coordinate in list order on every rank
 
+    def coded_args(self) -> L.CodedArgs:
+        """What `skml_train_step` needs to run pack and unpack itself (the seed is the step's)."""
+        a = L.CodedArgs()
+        a.kind, a.bits, a.code_stride = 1, self.bits, self.code_stride
+        a.scratch, a.codes, a.norm = L.ptr(self.scratch), L.ptr(self.codes), L.ptr(self.norm)
+        return a
+
     def wire_bytes(self, n: int) -> int:
         """Bytes one rank contributes for n non-zeros: raw keys, codes, count and norm."""
         return 4 * n + (n + 7) // 8 * self.bits + 16
@@ -112,6 +119,14 @@ class ZipCodec:
                                                    self.n_max, self.code_stride, lists, self.bin_num, L.ptr(vals_out),
                                                    L.stream()), "skml_zipml_unpack_scatter")
         L.count_launches(lists)
+
+    def coded_args(self) -> L.CodedArgs:
+        """What `skml_train_step` needs to run pack and unpack itself."""
+        a = L.CodedArgs()
+        a.kind, a.bits, a.code_stride, a.scratch_bytes = 2, self.bin_num, self.code_stride, self.scratch_bytes
+        a.scratch, a.codes, a.splits, a.mids = L.ptr(self.scratch), L.ptr(self.codes), L.ptr(self.splits), L.ptr(self.mids)
+        a.zip_meta, a.range = L.ptr(self.meta), L.ptr(self.range)
+        return a
 
     def roundtrip(self, vals: torch.Tensor, n: torch.Tensor) -> None:
         """In place on vals[:n]: every value is replaced by the midpoint of its bucket."""

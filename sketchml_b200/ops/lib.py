@@ -64,6 +64,14 @@ class DenseIndexArgs(C.Structure):
     ]
 
 
+class CodedArgs(C.Structure):
+    _fields_ = [
+        ("kind", c_ll), ("bits", c_ll), ("seed", c_ull), ("scratch", c_vp), ("scratch_bytes", c_ll), ("codes", c_vp),
+        ("code_stride", c_ll), ("norm", c_vp), ("splits", c_vp), ("mids", c_vp), ("zip_meta", c_vp), ("range", c_vp),
+        ("adam_m", c_vp), ("adam_v", c_vp), ("adam_stride", c_ll),
+    ]
+
+
 class StepArgs(C.Structure):
     _fields_ = [
         ("rowptr", c_vp), ("cols", c_vp), ("vals", c_vp), ("labels", c_vp), ("seg_lo", c_ll * 2), ("seg_cnt", c_ll * 2),
@@ -79,7 +87,7 @@ class StepArgs(C.Structure):
         ("grad_done_event", c_vp),
         ("tt_tile_pair_ptr", c_vp), ("tt_pair_ptr", c_vp), ("tt_lrow", c_vp), ("tt_pair_dst", c_vp),
         ("tt_col_pair_ptr", c_vp), ("tt_partial", c_vp), ("tt_tiles", c_ll), ("tt_tile_rows", c_ll), ("tt_rows", c_ll),
-        ("dense_index", C.POINTER(DenseIndexArgs)),
+        ("dense_index", C.POINTER(DenseIndexArgs)), ("coded", C.POINTER(CodedArgs)),
     ]
 
 
