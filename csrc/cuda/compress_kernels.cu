@@ -2304,7 +2304,8 @@ __device__ void stage_prepare(const CP& p, long long n) {
         if (bound > p.slot_capacity) bound = p.slot_capacity;
         uint4 z = make_uint4(0, 0, 0, 0);
         uint4* z4 = reinterpret_cast<uint4*>(p.payload);
-        for (long long i = gid + SKML_HEADER_BYTES / 16; i < bound / 16; i += gsz) z4[i] = z;
+        if (!p.zero_slot)
+            for (long long i = gid + SKML_HEADER_BYTES / 16; i < bound / 16; i += gsz) z4[i] = z;
         for (long long i = gid; i < SKML_MAX_GROUPS * 32; i += gsz) p.key_hist[i] = 0;
         for (long long i = gid; i < SKML_GPU_MAX_BINS + SKML_MAX_GROUPS; i += gsz) p.cell_hist[i] = 0;
     }

@@ -95,16 +95,17 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
         l.off_bucket_values = h.off_bucket_values;
         for (int i = 0; i < 4; ++i) l.loss_partials[i] = h.loss_partials[i];
     }
-    __syncthreads();
-    if (!s.ok) return false;
-    // group entries: one thread per (rank, group) fetches its 64-byte entry (independent loads)
+    // group entries: one thread per (rank, group) fetches its 64-byte entry (independent loads), while the header is
+    // still being checked: only the offsets the fetch itself needs are looked at first
     const int gcap = p.max_items / p.world;
     for (int t = threadIdx.x; t < p.world * gcap; t += blockDim.x) {
         const int r = t / gcap, g = t % gcap;
         const SkmlHeader& h = full[r];
         DecItem& it = s.items[t];
         it.e.n = 0;
-        if (h.kind == SKML_KIND_SPARSE && g < (int)h.group_num) {
+        if (h.kind == SKML_KIND_SPARSE && g < (int)h.group_num && h.group_num <= SKML_MAX_GROUPS && (h.off_group_table & 15ull) == 0 &&
+            h.off_group_table <= (unsigned long long)p.slot_capacity && h.row_num <= SKML_MAX_ROWS &&
+            h.off_group_table + sizeof(SkmlGroupEntry) * h.group_num <= (unsigned long long)p.slot_capacity) {
             const uint4* src = reinterpret_cast<const uint4*>(p.payload[r] + h.off_group_table + g * sizeof(SkmlGroupEntry));
             unsigned long long* dst = reinterpret_cast<unsigned long long*>(&it.e);  // 8-byte aligned in DecItem
 #pragma unroll
@@ -132,7 +133,6 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
                 it.zero = h.zero_idx;
                 it.rows = h.row_num;
                 it.off_bv = h.off_bucket_values;
-                it.col_magic = good ? skml_fastmod_magic(it.e.col_num) : 0ull;
                 it.recip = skml_recip32(it.e.col_num);
                 it.mixers = 0;
                 if (h.row_num <= 3) {
@@ -145,11 +145,13 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
                         }
                     it.mixers = __popc(seen) == (int)h.row_num ? 1 : 0;
                 }
+                it.col_magic = good && !it.mixers ? skml_fastmod_magic(it.e.col_num) : 0ull;   // (a 64-bit division)
                 it.chunk_prefix = good ? 0ull : 1ull;  // scratch use until the compaction below: 1 = failed validation
             }
         }
     }
     __syncthreads();
+    if (!s.ok) return false;
     // The work table: the non-empty (rank, group) lists moved to the front in (rank, group) order, each
     // with the number of chunks and keys in front of it. Warp 0 does it 32 slots at a time (ballot for the
     // positions, shuffle scans for the prefixes); thread 0 first looks at the per-rank header facts.
@@ -634,8 +636,9 @@ __device__ void apply_owned(const DP& p, DecSmem& s, float& dsq) {
     __shared__ unsigned long long s_bound[2 * DEC_OWN_RANGES];
     // SGD: one range per block (more ranges even out the blocks but do not shorten the launch: the random
     // DRAM sectors bound it in total); lazy Adam sweeps a range 2 x ranks times, and smaller ranges keep
-    // its sectors in L2 between the sweeps
-    const int rounds = p.adam_v ? DEC_OWN_RANGES : 1;
+    // its sectors in L2
+    // between the sweeps (where a block has fewer than 2048 keys, the sweeps' latency is what counts)
+    const int rounds = p.adam_v && s.total_keys >= 2048ull * gridDim.x ? DEC_OWN_RANGES : 1;
     if (threadIdx.x < 2 * rounds) {
         const DecItem& ref = s.items[s.ref_item];
         const unsigned long long B = gridDim.x, total = (unsigned long long)rounds * B;

@@ -62,7 +62,9 @@ __device__ __forceinline__ void st_v4(uint4* p, uint4 v) {
 // less). Java semantics: the remainder keeps the sign of the dividend and is then moved up by size.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned int skml_recip32(unsigned int size) {
-    return size <= 1u ? 0xFFFFFFFFu : (unsigned int)((1ull << 32) / size);
+    if (size <= 1u) return 0xFFFFFFFFu;
+    const unsigned int q = 0xFFFFFFFFu / size;   // floor(2^32 / size) is one more where size divides 2^32
+    return q + (0xFFFFFFFFu - q * size == size - 1u ? 1u : 0u);
 }
 __device__ __forceinline__ bool skml_rows_are_mixers(const unsigned char* ids, int rows) {
     bool ok = true;

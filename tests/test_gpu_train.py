@@ -254,3 +254,16 @@ def test_local_id_batches_train_like_plain_streamed_batches():
     # float atomics order differs between the two scatters: bucket edges may move a value, as between two runs
     assert np.allclose(losses[0], losses[1], rtol=2e-3)
     assert float((ws[0] - ws[1]).abs().mean()) < 2e-3
+
+
+@pytest.mark.parametrize("opt", ["sgd", "adam"])
+@pytest.mark.parametrize("name", ["Float", "FixedPoint", "Zip"])
+def test_baseline_step_behind_one_call_equals_its_separate_calls(name, opt):
+    """Batches of 400 rows keep every column below the length that is summed with atomics, so both forms of the step
+    run the same sums in the same order: the same weights, bit for bit."""
+    kw = dict(compressor=name, optimizer=opt, epoch_num=2, valid_ratio=0.0, syn_rows=2000, batch_sample_ratio=0.2, quant_bin_num=64,
+              learn_rate=0.5 if opt == "sgd" else 0.01)
+    h1, w1, _ = _train(_conf(**kw))
+    h2, w2, _ = _train(_conf(extras={"single_call_step": False}, **kw))
+    assert torch.equal(w1, w2)
+    assert np.allclose(h1["train_loss"], h2["train_loss"], rtol=1e-12)
