@@ -202,12 +202,19 @@ glm_scatter_kernel(const long long* __restrict__ rowptr, const int* __restrict__
 // is staged that would take L1 away. 500,000 rows of 30: 80 -> 61 us; 1M rows of 30 with values: 208 -> 102 us
 // (before: a warp per row, tiles staged by bulk copies, 103 warp instructions per 32 entries).
 #define MARGIN_THREADS 512
+struct ClearSlots {   // out[slot[0 .. n)] = 0
+    float* out;
+    const int* slot;
+    int n;
+};
 template <int MODE, int GL, bool HAS_VALS>
 __global__ void __launch_bounds__(MARGIN_THREADS, 3)
 glm_margin_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
                   const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
-                  int hot, int loss_id, float inv_batch, double* __restrict__ acc, float* __restrict__ out) {
+                  int hot, int loss_id, float inv_batch, double* __restrict__ acc, float* __restrict__ out, ClearSlots clear) {
     extern __shared__ __align__(16) float s_w[];
+    if (MODE == 2)   // what the column sums behind this launch add to
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < clear.n; i += gridDim.x * blockDim.x) clear.out[clear.slot[i]] = 0.f;
     constexpr int LANES = 1 << GL, ROWS = 32 >> GL, PER = 4;   // rows of an iteration, entries of a lane in flight
     const int lane = threadIdx.x & 31, sub = lane & (LANES - 1), grp = lane >> GL;
     for (int i = threadIdx.x; i < hot / 4; i += blockDim.x) reinterpret_cast<float4*>(s_w)[i] = __ldg(reinterpret_cast<const float4*>(w) + i);
@@ -351,16 +358,16 @@ static TurnShape turn_shape(long long row_cnt, int gl, int max_warps, int per_sm
 template <int MODE, int GL>
 static int margin_launch_gl(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
                             long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
-                            float* out, cudaStream_t stream) {
+                            float* out, const ClearSlots& clear, cudaStream_t stream) {
     const TurnShape t = turn_shape(row_cnt, GL, MARGIN_THREADS / 32, 3);
     const int iters = t.iters, warps = t.warps, grid = t.grid;
     const int hot = margin_hot((long long)(row_cnt * avg_nnz), grid, dim, w);
     if (vals)
         glm_margin_kernel<MODE, GL, true><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out);
+            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
     else
         glm_margin_kernel<MODE, GL, false><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out);
+            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
     return (int)cudaGetLastError();
 }
 
@@ -368,11 +375,11 @@ static int margin_launch_gl(const long long* rowptr, const int* cols, const floa
 template <int MODE>
 static int margin_launch(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
                          long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
-                         float* out, cudaStream_t stream) {
+                         float* out, cudaStream_t stream, const ClearSlots& clear = {nullptr, nullptr, 0}) {
     if (row_cnt <= 0) return 0;
     auto go = avg_nnz <= 16.0 ? margin_launch_gl<MODE, 2> : avg_nnz <= 40.0 ? margin_launch_gl<MODE, 3>
             : avg_nnz <= 96.0 ? margin_launch_gl<MODE, 4> : margin_launch_gl<MODE, 5>;
-    return go(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, inv_batch, acc, out, stream);
+    return go(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, inv_batch, acc, out, clear, stream);
 }
 
 // Columns summed per block: no more than the caller allows, and only those whose adds would queue up in L2: with
@@ -430,6 +437,22 @@ extern "C" int skml_glm_validate(const long long* rowptr, const int* cols, const
     (void)budget;   // nothing in it waits
     return margin_launch<1>(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, 1.f, acc5, margins, (cudaStream_t)stream);
 }
+
+// The loss partials of a step, {rows, loss sum, regularisation, -}: the gradient kernels add the loss to the spare word
+// of the template that holds the rest, and a kernel behind them puts both together for the step and clears the word, so
+// that neither needs a launch (a copy of 32 bytes cost 1.5 us and the gap before the next kernel 2 us).
+struct StepLoss {
+    double* partials;   // null: the caller sees to it
+    double* tmpl;
+    __device__ __forceinline__ void settle() const {
+        if (!partials) return;
+        partials[0] = tmpl[0];
+        partials[1] = tmpl[1] + tmpl[3];
+        partials[2] = tmpl[2];
+        partials[3] = 0.0;
+        tmpl[3] = 0.0;
+    }
+};
 
 // ---------------------------------------------------------------------------
 // Compaction of the touched bitmap into a sorted sparse gradient. A warp owns `wpw` consecutive bitmap
@@ -568,7 +591,7 @@ __global__ void __launch_bounds__(COMPACT_THREADS)
 compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigned int* __restrict__ bitmap,
                      long long nwords, int dim, float lambda, int wpw, int nwarps,
                      const unsigned int* __restrict__ warp_counts, long long* __restrict__ meta, int* __restrict__ keys,
-                     float* __restrict__ vals, float* __restrict__ dense_vals, long long capacity, unsigned int* status) {
+                     float* __restrict__ vals, float* __restrict__ dense_vals, long long capacity, unsigned int* status, StepLoss loss) {
     __shared__ unsigned int s_before[COMPACT_WARPS], s_total[COMPACT_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gw0 = blockIdx.x * COMPACT_WARPS, gw = gw0 + warp;
@@ -598,6 +621,7 @@ compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         meta[0] = total;
         meta[1] = kind;
+        loss.settle();
     }
     if (gw >= nwarps) return;
     if (kind == 2) {
@@ -708,13 +732,21 @@ compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
 
 static int compact_launch(float* g, const float* w, unsigned int* bitmap, int dim, float lambda, unsigned int* warp_counts,
                           long long* meta, int* keys, float* vals, float* dense_vals, long long capacity, unsigned int* status,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, const StepLoss& loss = {nullptr, nullptr}) {
     const long long nwords = ((long long)dim + 31) / 32;
     const CompactShape c = compact_shape(dim);
     compact_count_kernel<<<c.nblocks, COMPACT_THREADS, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts);
     compact_write_kernel<<<c.nblocks, COMPACT_THREADS, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts,
-                                                                    meta, keys, vals, dense_vals, capacity, status);
+                                                                    meta, keys, vals, dense_vals, capacity, status, loss);
     return (int)cudaGetLastError();
+}
+
+// skml_compact that also settles the step's loss partials.
+extern "C" int skml_compact_settle(float* g, const float* w, unsigned int* bitmap, int dim, float lambda, unsigned int* block_counts, long long* meta,
+                   int* keys, float* vals, float* dense_vals, long long capacity, unsigned int* status, double* partials, double* tmpl,
+                   void* stream) {
+    return compact_launch(g, w, bitmap, dim, lambda, block_counts, meta, keys, vals, dense_vals, capacity, status, (cudaStream_t)stream,
+                          StepLoss{partials, tmpl});
 }
 
 extern "C" int skml_compact(float* g, const float* w, unsigned int* bitmap, int dim, float lambda,
@@ -1063,9 +1095,10 @@ colsum_kernel(const int* __restrict__ colptr, const int* __restrict__ rowidx, co
               const int* __restrict__ ucols, const int* __restrict__ bins, const int* __restrict__ long_col,
               const int* __restrict__ long_e0, const int* __restrict__ long_e1, int n_short, int n_medium, int n_long,
               int short_blocks, int medium_blocks, const float* __restrict__ coef, const float* __restrict__ w,
-              float lambda, float* __restrict__ out) {
+              float lambda, float* __restrict__ out, StepLoss loss) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int b = blockIdx.x;
+    if (b == 0 && threadIdx.x == 0) loss.settle();
     if (b < short_blocks) {
         const int t = b * 256 + threadIdx.x;
         if (t < n_short) {
@@ -1103,6 +1136,14 @@ colsum_kernel(const int* __restrict__ colptr, const int* __restrict__ rowidx, co
             atomicAdd(out + i, t);
         }
     }
+}
+
+// skml_glm_coef that also zeroes out[slot[0 .. n_slots)], for the column sums that add to them.
+extern "C" int skml_glm_coef_clear(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo, long long row_cnt,
+                   double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* loss_acc, float* coef_out,
+                   float* out, const int* slot, int n_slots, void* stream) {
+    return margin_launch<2>(rowptr, cols, vals, labels, row_lo, row_cnt, avg_nnz, w, dim, loss_id, inv_batch, loss_acc, coef_out,
+                            (cudaStream_t)stream, ClearSlots{out, slot, n_slots});
 }
 
 extern "C" int skml_glm_coef(const long long* rowptr, const int* cols, const float* vals, const float* labels,
@@ -1148,54 +1189,34 @@ extern "C" int skml_finalize_compact(float* gc, const float* wc, float lambda, i
     return (int)cudaGetLastError();
 }
 
-// Start-of-step housekeeping in one small launch: the loss partials are reset from their template
-// and the output slots of the long columns (the only ones the column-sum kernel accumulates into
-// with atomics) are cleared.
-__global__ void step_prep_kernel(double* __restrict__ partials, const double* __restrict__ partials_template,
-                                 float* __restrict__ out, const int* __restrict__ long_col, int n_long) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < 4) partials[t] = partials_template[t];
-    for (int i = t; i < n_long; i += gridDim.x * blockDim.x) out[long_col[i]] = 0.f;  // duplicates store the same zero
-}
-
-extern "C" int skml_step_prep(double* partials, const double* partials_template, float* out, const int* long_col,
-                              int n_long, void* stream) {
-    int blocks = (n_long + 255) / 256;
-    if (blocks < 1) blocks = 1;
-    if (blocks > 1024) blocks = 1024;
-    step_prep_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(partials, partials_template, out, long_col, n_long);
+static int colsum_launch(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins, const int* long_col,
+                         const int* long_e0, const int* long_e1, int n_short, int n_medium, int n_long, const float* coef, const float* w,
+                         float lambda, float* out, const StepLoss& loss, cudaStream_t stream) {
+    const int short_blocks = (n_short + 255) / 256, medium_blocks = (n_medium + 7) / 8;
+    const long long blocks = (long long)short_blocks + medium_blocks + n_long;
+    if (blocks <= 0 && !loss.partials) return 0;
+    colsum_kernel<<<(unsigned)(blocks > 0 ? blocks : 1), 256, 0, stream>>>(colptr, rowidx, svals, ucols, bins, long_col, long_e0, long_e1,
+                                                                          n_short, n_medium, n_long, short_blocks, medium_blocks, coef, w,
+                                                                          lambda, out, loss);
     return (int)cudaGetLastError();
 }
 
-// `out_is_prepared` != 0: the long columns' slots are already zero (skml_step_prep), skip the full clear.
-extern "C" int skml_colsum_ex(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,
-                              const int* long_col, const int* long_e0, const int* long_e1, int n_short, int n_medium,
-                              int n_long, int n_cols, const float* coef, const float* w, float lambda, float* out,
-                              int out_is_prepared, void* stream);
+// The long columns' slots are zero already (skml_glm_coef_clear); also settles the step's loss partials.
+extern "C" int skml_colsum_settle(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins, const int* long_col,
+                  const int* long_e0, const int* long_e1, int n_short, int n_medium, int n_long, const float* coef, const float* w,
+                  float lambda, float* out, double* partials, double* tmpl, void* stream) {
+    return colsum_launch(colptr, rowidx, svals, ucols, bins, long_col, long_e0, long_e1, n_short, n_medium, n_long, coef, w, lambda, out,
+                         StepLoss{partials, tmpl}, (cudaStream_t)stream);
+}
 
 extern "C" int skml_colsum(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,
                            const int* long_col, const int* long_e0, const int* long_e1, int n_short, int n_medium,
                            int n_long, int n_cols, const float* coef, const float* w, float lambda, float* out,
                            void* stream) {
-    return skml_colsum_ex(colptr, rowidx, svals, ucols, bins, long_col, long_e0, long_e1, n_short, n_medium, n_long,
-                          n_cols, coef, w, lambda, out, 0, stream);
-}
-
-extern "C" int skml_colsum_ex(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,
-                              const int* long_col, const int* long_e0, const int* long_e1, int n_short, int n_medium,
-                              int n_long, int n_cols, const float* coef, const float* w, float lambda, float* out,
-                              int out_is_prepared, void* stream) {
-    if (!out_is_prepared) {
-        cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_cols * sizeof(float), (cudaStream_t)stream);
-        if (e != cudaSuccess) return (int)e;
-    }
-    const int short_blocks = (n_short + 255) / 256, medium_blocks = (n_medium + 7) / 8;
-    const long long blocks = (long long)short_blocks + medium_blocks + n_long;
-    if (blocks <= 0) return 0;
-    colsum_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(colptr, rowidx, svals, ucols, bins, long_col, long_e0,
-                                                                     long_e1, n_short, n_medium, n_long, short_blocks,
-                                                                     medium_blocks, coef, w, lambda, out);
-    return (int)cudaGetLastError();
+    const cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_cols * sizeof(float), (cudaStream_t)stream);
+    if (e != cudaSuccess) return (int)e;
+    return colsum_launch(colptr, rowidx, svals, ucols, bins, long_col, long_e0, long_e1, n_short, n_medium, n_long, coef, w, lambda, out,
+                         StepLoss{nullptr, nullptr}, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -181,12 +181,18 @@ int skml_glm_coef(const long long* rowptr, const int* cols, const float* vals, c
 int skml_colsum(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,
                 const int* long_col, const int* long_e0, const int* long_e1, int n_short, int n_medium, int n_long,
                 int n_cols, const float* coef, const float* w, float lambda, float* out, void* stream);
-int skml_colsum_ex(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,
-                   const int* long_col, const int* long_e0, const int* long_e1, int n_short, int n_medium, int n_long,
-                   int n_cols, const float* coef, const float* w, float lambda, float* out, int out_is_prepared,
-                   void* stream);
-int skml_step_prep(double* partials, const double* partials_template, float* out, const int* long_col, int n_long,
-                   void* stream);
+// The step's forms of the three calls around the gradient: skml_glm_coef also zeroes out[slot[0 .. n_slots)], the
+// slots skml_colsum_settle adds to; the other two also put the step's loss partials together from `tmpl`, whose spare
+// last word the gradient kernels have added the loss to, and clear that word.
+int skml_glm_coef_clear(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
+                        long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch,
+                        double* loss_acc, float* coef_out, float* out, const int* slot, int n_slots, void* stream);
+int skml_colsum_settle(const int* colptr, const int* rowidx, const float* svals, const int* ucols, const int* bins,
+                       const int* long_col, const int* long_e0, const int* long_e1, int n_short, int n_medium, int n_long,
+                       const float* coef, const float* w, float lambda, float* out, double* partials, double* tmpl, void* stream);
+int skml_compact_settle(float* g, const float* w, unsigned int* bitmap, int dim, float lambda, unsigned int* block_counts,
+                        long long* meta, int* keys, float* vals, float* dense_vals, long long capacity, unsigned int* status,
+                        double* partials, double* tmpl, void* stream);
 int skml_gather_compact(const float* w, const int* ucols, int n, float* wc, void* stream);
 int skml_finalize_compact(float* gc, const float* wc, float lambda, int n, float* vals, unsigned int* bitmap,
                           void* stream);
@@ -305,7 +311,7 @@ typedef struct SkmlStepArgs {
     double inv_batch;
     long long hot;
     double* partials;                  // device, 4 doubles: batch size, loss sum, reg loss, spare
-    const double* partials_template;   // device, copied into `partials` before the gradient kernel
+    double* partials_template;         // device, what `partials` holds beside the loss; its last word is zero between steps
     unsigned int* status;
     long long budget_cycles;
     double lambda;

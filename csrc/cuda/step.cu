@@ -1,7 +1,7 @@
 // skml_train_step: the launch sequence of one training step behind a single C call.
 // Reference: ml/algorithm/GeneralizedLinearModel.scala:116-123 (trainOneIteration =
-// computeGradient + aggregateAndUpdate); here the whole iteration is five kernel launches
-// (housekeeping, coefficients, column sums, fused compress, fused decode + update) issued back to
+// computeGradient + aggregateAndUpdate); here the whole iteration is four kernel launches
+// (coefficients, column sums, fused compress, fused decode + update) issued back to
 // back on one stream with no host round trip.
 #include <cuda_runtime.h>
 
@@ -53,31 +53,37 @@ static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* met
 extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
     if (!a || (!a->coded && (!a->compress || !a->decode))) return (int)cudaErrorInvalidValue;
     cudaStream_t stream = (cudaStream_t)stream_;
+    double* const loss = a->partials_template + 3;   // (settled behind the gradient)
     if (a->t_colptr || a->tt_pair_ptr) {
         // transposed index: coefficients per row, then one gather-sum per distinct column
-        const bool tiled = a->tt_pair_ptr != nullptr;
-        int rc = skml_step_prep(a->partials, a->partials_template, a->gvals, a->t_long_col, tiled ? 0 : (int)a->t_long, stream_);
-        if (rc) return rc;
-        rc = skml_glm_coef(a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->seg_cnt[0], a->nnz_padded,
+        int rc;
+        if (a->tt_pair_ptr) {
+            const cudaError_t e = cudaMemcpyAsync(a->partials, a->partials_template, 4 * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+            if (e != cudaSuccess) return (int)e;
+            rc = skml_glm_coef(a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->seg_cnt[0], a->nnz_padded,
                                a->avg_nnz, a->w, a->dim, (int)a->loss_id, (float)a->inv_batch, a->partials + 1, a->coef,
                                a->status, a->budget_cycles, stream_);
-        if (rc) return rc;
-        if (tiled)
+            if (rc) return rc;
             rc = skml_colsum_tiled(a->tt_tile_pair_ptr, a->tt_pair_ptr, a->tt_lrow, a->t_vals, a->tt_pair_dst, a->tt_col_pair_ptr,
                                    a->t_ucols, (int)a->tt_rows, (int)a->tt_tile_rows, (int)a->tt_tiles, (int)a->t_cols, a->coef,
                                    a->w, (float)a->lambda, a->tt_partial, a->gvals, stream_);
-        else
-            rc = skml_colsum_ex(a->t_colptr, a->t_rowidx, a->t_vals, a->t_ucols, a->t_bins, a->t_long_col, a->t_long_e0,
-                                a->t_long_e1, (int)a->t_short, (int)a->t_medium, (int)a->t_long, (int)a->t_cols, a->coef, a->w,
-                                (float)a->lambda, a->gvals, 1, stream_);
+        } else {
+            rc = skml_glm_coef_clear(a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->seg_cnt[0], a->avg_nnz, a->w, a->dim,
+                                     (int)a->loss_id, (float)a->inv_batch, loss, a->coef, a->gvals, a->t_long_col, (int)a->t_long,
+                                     stream_);
+            if (rc) return rc;
+            rc = skml_colsum_settle(a->t_colptr, a->t_rowidx, a->t_vals, a->t_ucols, a->t_bins, a->t_long_col, a->t_long_e0,
+                                    a->t_long_e1, (int)a->t_short, (int)a->t_medium, (int)a->t_long, a->coef, a->w,
+                                    (float)a->lambda, a->gvals, a->partials, a->partials_template, stream_);
+        }
         if (rc) return rc;
         rc = batch_consumed(a, stream);
         if (rc) return rc;
         return apply_gradient(a, a->t_ucols, a->t_meta, a->gvals, nullptr, false, stream_);
     }
-    cudaError_t e = cudaMemcpyAsync(a->partials, a->partials_template, 4 * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-    if (e != cudaSuccess) return (int)e;
     if (a->l_ucols) {
+        const cudaError_t e = cudaMemcpyAsync(a->partials, a->partials_template, 4 * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        if (e != cudaSuccess) return (int)e;
         // local-id batch: compact weights in, scatter into the compact accumulator, values out in key order
         const int n = (int)a->l_ncols;
         int rc = skml_gather_compact(a->w, a->l_ucols, n, a->wc, stream_);
@@ -95,7 +101,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
     }
     if (a->dense_index) {
         int rc = skml_dt_gradient(a->dense_index, a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->nnz_padded, a->avg_nnz, a->w,
-                                  (int)a->loss_id, (float)a->inv_batch, a->partials + 1, a->g, a->bitmap, a->status,
+                                  (int)a->loss_id, (float)a->inv_batch, loss, a->g, a->bitmap, a->status,
                                   a->budget_cycles, stream_);
         if (rc) return rc;
     }
@@ -103,13 +109,13 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         if (a->seg_cnt[s] <= 0) continue;
         int rc = skml_glm_grad(a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[s], a->seg_cnt[s], a->nnz_padded,
                                a->avg_nnz, a->w, a->g, a->bitmap, (int)a->loss_id, (float)a->inv_batch, (int)a->hot,
-                               a->partials + 1, a->status, a->budget_cycles, stream_);
+                               loss, a->status, a->budget_cycles, stream_);
         if (rc) return rc;
     }
     int rc = batch_consumed(a, stream);
     if (rc) return rc;
-    rc = skml_compact(a->g, a->w, a->bitmap, (int)a->dim, (float)a->lambda, a->block_counts, a->meta, a->keys,
-                          a->gvals, a->dense_vals, a->n_max, a->status, stream_);
+    rc = skml_compact_settle(a->g, a->w, a->bitmap, (int)a->dim, (float)a->lambda, a->block_counts, a->meta, a->keys,
+                          a->gvals, a->dense_vals, a->n_max, a->status, a->partials, a->partials_template, stream_);
     if (rc) return rc;
     return apply_gradient(a, a->keys, a->meta, a->gvals, a->dense_vals, false, stream_);
 }

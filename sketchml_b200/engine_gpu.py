@@ -316,7 +316,7 @@ class GpuEngine:
         if lid is not None:
             L.count_launches(len(segs) + 2 + tail)  # gather, gradient segment(s), finalize
         else:
-            L.count_launches((3 if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + tail)
+            L.count_launches(((2 if bi.tiled is None else 3) if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + tail)
 
     # ----------------------------------------------------------------- steps
     def _segments(self, count: int):
@@ -607,6 +607,7 @@ class GpuEngine:
         if not s and getattr(self, "depth", 0) == 1:
             s = read_status(self.sts[1].status)
         if s:
+            self.partials_template[3:].zero_()   # the loss of a step that did not get as far as settling it
             if self.mode == "sketch":
                 self.comp.reset()
                 self.dec.reset()

@@ -94,14 +94,17 @@ def glm_grad(csr: DeviceCSR, segments: List[Tuple[int, int]], w: torch.Tensor, s
 def glm_validate(csr: DeviceCSR, w: torch.Tensor, loss_id: int, status: torch.Tensor,
                  margins: Optional[torch.Tensor] = None, budget_s: float = 1.0) -> torch.Tensor:
     """Returns a device fp64 tensor [sum loss, TP, TN, FP, FN, n]."""
-    acc = torch.zeros(6, dtype=torch.float64, device=w.device)
+    rows, start = getattr(csr, "_validation_start", (None, None))   # [0, 0, 0, 0, 0, rows] on the device
+    if rows != csr.rows or start.device != w.device:
+        start = torch.tensor([0.0] * 5 + [float(csr.rows)], dtype=torch.float64, device=w.device)
+        csr._validation_start = (csr.rows, start)
+    acc = start.clone()
     if csr.rows:
         L.check(L.lib().skml_glm_validate(L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), L.ptr(csr.labels), 0,
                                           csr.rows, csr.nnz_padded, float(csr.avg_nnz), L.ptr(w), w.numel(), loss_id, L.ptr(acc),
                                           L.ptr(margins), L.ptr(status), L.budget_cycles(budget_s), L.stream()),
                 "skml_glm_validate")
         L.count_launches(1)
-    acc[5:].fill_(float(csr.rows))
     return acc
 
 
