@@ -138,6 +138,45 @@ dt_fill_kernel(const long long* __restrict__ rowptr, const int* __restrict__ col
     }
 }
 
+// Puts the quads of every 32 neighbouring lists of a tile in the order dt_partial_kernel reads them: the first quads of
+// all lists, then the second quads of those that have one, and so on, so that a warp's loads are consecutive. The 32
+// lists keep their place in memory. Groups with a list of more than DT_LONG quads stay list by list. One warp a group.
+constexpr int DT_TURN_WARPS = 4;
+template <bool HAS_VALS>
+__global__ void __launch_bounds__(DT_TURN_WARPS * 32)
+dt_interleave_kernel(const int* __restrict__ ptr, int tiles, int items, ushort4* __restrict__ loc, float4* __restrict__ val) {
+    __shared__ float4 s_val[HAS_VALS ? DT_TURN_WARPS : 1][HAS_VALS ? 32 * DT_LONG : 1];
+    __shared__ ushort4 s_loc[DT_TURN_WARPS][32 * DT_LONG];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned int below = (1u << lane) - 1u;
+    const int per_tile = (items + 31) / 32;
+    const long long groups = (long long)tiles * per_tile;
+    for (long long g = (long long)blockIdx.x * DT_TURN_WARPS + warp; g < groups; g += (long long)gridDim.x * DT_TURN_WARPS) {
+        const int tile = (int)(g / per_tile), i = (int)(g % per_tile) * 32 + lane;
+        const long long p = (long long)tile * items + i;
+        const int q0 = i < items ? ptr[p] : 0, len = i < items ? ptr[p + 1] - q0 : 0;
+        const int most = __reduce_max_sync(0xFFFFFFFFu, len);
+        if (most > DT_LONG || most < 2) continue;
+        const int first = __shfl_sync(0xFFFFFFFFu, q0, 0), total = __reduce_add_sync(0xFFFFFFFFu, len);
+        for (int k = lane; k < total; k += 32) {
+            s_loc[warp][k] = loc[first + k];
+            if (HAS_VALS) s_val[warp][k] = val[first + k];
+        }
+        __syncwarp();
+        int at = first;
+        for (int j = 0; j < most; ++j) {
+            const unsigned int have = __ballot_sync(0xFFFFFFFFu, len > j);
+            if (len > j) {
+                const int dst = at + __popc(have & below);
+                loc[dst] = s_loc[warp][q0 - first + j];
+                if (HAS_VALS) val[dst] = s_val[warp][q0 - first + j];
+            }
+            at += __popc(have);
+        }
+        __syncwarp();
+    }
+}
+
 // First list p in [lo, hi) whose quads and lists before it reach `target`; a whole warp, 32 probes a round.
 __device__ __forceinline__ int weighted_bound(const int* __restrict__ ptr, int lo, int hi, long long base, long long target) {
     const int lane = threadIdx.x & 31, first = lo;
@@ -154,8 +193,10 @@ __device__ __forceinline__ int weighted_bound(const int* __restrict__ ptr, int l
 }
 
 // partial[tile * items + item] = sum over the list of x[tile * T + loc] * val.
-// Blocks of a tile, and the warps of a block, share its lists by quads + lists.
-// What bounds it: reading the lists (7 bytes an entry with padding), about two thirds of the copy rate.
+// Blocks of a tile, and the warps of a block, share its lists by quads + lists, cut at whole groups of 32.
+// What bounds it: reading the lists (7 bytes an entry with padding). List by list a lane's loads were 20 and 40 bytes
+// from its neighbour's, and the passes they took through L1 were the limit: 160 us for 100M entries, 149 with the next
+// round's lists on their way into L2, 144 us (4.9 TB/s) with the lists interleaved (dt_interleave_kernel).
 template <bool HAS_VALS>
 __global__ void __launch_bounds__(DT_THREADS, 1)
 dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, int blocks_per_tile, const int* __restrict__ ptr,
@@ -172,10 +213,11 @@ dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, in
     {
         const long long base = ptr[p0], all = (long long)ptr[p1] - base + items;
         const long long share = (long long)sub * warps + warp, shares = (long long)blocks_per_tile * warps;
-        const int cut = weighted_bound(ptr, p0, p1, base, all * share / shares);
+        auto group_start = [&](int p) { return p0 + ((p - p0) & ~31); };
+        const int cut = group_start(weighted_bound(ptr, p0, p1, base, all * share / shares));
         if (lane == 0) s_cut[warp] = cut;
         if (warp == warps - 1) {
-            const int end = sub + 1 == blocks_per_tile ? p1 : weighted_bound(ptr, p0, p1, base, all * (share + 1) / shares);
+            const int end = sub + 1 == blocks_per_tile ? p1 : group_start(weighted_bound(ptr, p0, p1, base, all * (share + 1) / shares));
             if (lane == 0) s_cut[warps] = end;
         }
     }
@@ -187,34 +229,53 @@ dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, in
     };
     const ushort4 none = make_ushort4(T, T, T, T);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    int nq0 = 0, nq1 = 0;   // one round of list bounds ahead
-    if (w0 + lane < w1) {
-        nq0 = ptr[w0 + lane];
-        nq1 = ptr[w0 + lane + 1];
-    }
+    // list bounds two rounds ahead, entries one round ahead as far as L2
+    int nq0 = 0, nq1 = 0, mq0 = 0, mq1 = 0;
+    auto bounds = [&](int p, int& a, int& e) {
+        a = e = 0;
+        if (p < w1) {
+            a = ptr[p];
+            e = ptr[p + 1];
+        }
+    };
+    bounds(w0 + lane, nq0, nq1);
+    bounds(w0 + 32 + lane, mq0, mq1);
     for (int b = w0; b < w1; b += 32) {
         const int p = b + lane;
         const int q0 = nq0, q1 = nq1;
-        nq0 = nq1 = 0;
-        if (p + 32 < w1) {
-            nq0 = ptr[p + 32];
-            nq1 = ptr[p + 33];
+        nq0 = mq0;
+        nq1 = mq1;
+        bounds(p + 64, mq0, mq1);
+        {   // the next round's lists are neighbours: a line of 128 bytes a lane
+            const int f = __shfl_sync(0xFFFFFFFFu, nq0, 0), l = __reduce_max_sync(0xFFFFFFFFu, nq1);
+            if (HAS_VALS && f + 8 * lane < l) asm volatile("prefetch.global.L2 [%0];" ::"l"(val + f + 8 * lane));
+            if (f + 16 * lane < l) asm volatile("prefetch.global.L2 [%0];" ::"l"(loc + f + 16 * lane));
         }
         float acc = 0.f;
-        if (q1 - q0 <= DT_LONG)
-            for (int q = q0; q < q1; q += DT_BATCH) {
+        const int len = q1 - q0, most = __reduce_max_sync(0xFFFFFFFFu, len);
+        if (most <= DT_LONG) {   // interleaved
+            int at = __shfl_sync(0xFFFFFFFFu, q0, 0);
+            for (int k = 0; k < most; k += DT_BATCH) {
                 ushort4 l[DT_BATCH];
                 float4 v[DT_BATCH];
 #pragma unroll
                 for (int u = 0; u < DT_BATCH; ++u) {
-                    l[u] = q + u < q1 ? __ldg(loc + q + u) : none;
-                    v[u] = HAS_VALS && q + u < q1 ? __ldg(val + q + u) : zero;
+                    const unsigned int have = __ballot_sync(0xFFFFFFFFu, len > k + u);
+                    const int q = at + __popc(have & ((1u << lane) - 1u));
+                    at += __popc(have);
+                    l[u] = len > k + u ? __ldg(loc + q) : none;
+                    v[u] = HAS_VALS && len > k + u ? __ldg(val + q) : zero;
                 }
 #pragma unroll
                 for (int u = 0; u < DT_BATCH; ++u)
-                    if (q + u < q1) acc += quad(l[u], v[u]);
+                    if (len > k + u) acc += quad(l[u], v[u]);
             }
-        unsigned int longs = __ballot_sync(0xFFFFFFFFu, q1 - q0 > DT_LONG);
+            if (p < w1) partial[p] = acc;
+            continue;
+        }
+        if (len <= DT_LONG)
+            for (int q = q0; q < q1; ++q) acc += quad(__ldg(loc + q), HAS_VALS ? __ldg(val + q) : zero);
+        unsigned int longs = __ballot_sync(0xFFFFFFFFu, len > DT_LONG);
         while (longs) {   // frequent items: the warp sums one list at a time
             const int src = __ffs(longs) - 1;
             longs &= longs - 1;
@@ -327,6 +388,15 @@ extern "C" int skml_dt_fill(const SkmlDenseIndex* d, const long long* rowptr, co
         rowptr, cols, vals, row_lo, (int)d->rows, (int)d->tile_rows, (int)d->row_tiles, (int)d->tile_cols, (int)d->col_tiles, (int)d->dim,
         (int)parts, d->c_ptr, cursor,
         d->c_loc, d->c_val, d->r_ptr, d->r_loc, d->r_val);
+    auto interleave = [&](const int* ptr, long long tiles, long long items, unsigned short* loc, float* val) {
+        const unsigned blocks = blocks_for(tiles * ((items + 31) / 32), DT_TURN_WARPS, 16);
+        ushort4* const l = reinterpret_cast<ushort4*>(loc);
+        float4* const v = reinterpret_cast<float4*>(val);
+        if (val) dt_interleave_kernel<true><<<blocks, DT_TURN_WARPS * 32, 0, (cudaStream_t)stream>>>(ptr, (int)tiles, (int)items, l, v);
+        else dt_interleave_kernel<false><<<blocks, DT_TURN_WARPS * 32, 0, (cudaStream_t)stream>>>(ptr, (int)tiles, (int)items, l, v);
+    };
+    interleave(d->c_ptr, d->row_tiles, d->dim, d->c_loc, d->c_val);
+    if (d->r_ptr) interleave(d->r_ptr, d->col_tiles, d->rows, d->r_loc, d->r_val);
     return (int)cudaGetLastError();
 }
 
