@@ -373,9 +373,8 @@ SKML_HD uint32_t skml_pack_cell(int bin, int zero_idx) {
 // Width in bytes of one delta in the delta-binary key code: 1, 2 or 4.
 SKML_HD int skml_delta_bytes(uint32_t delta) { return delta < 256u ? 1 : (delta < 65536u ? 2 : 4); }
 
-// Byte j (in stream order) of a `w`-byte delta. The stream stores the value most
-// significant bit first at increasing java.util.BitSet indices, and BitSet index i is
-// bit (i & 63) of word (i >> 6), so each stream byte is a bit-reversed value byte.
+// The stream stores a delta most significant bit first at increasing java.util.BitSet indices, and BitSet
+// index i is bit (i & 63) of word (i >> 6), so each stream byte is a bit-reversed value byte.
 SKML_HD uint8_t skml_brev8(uint8_t b) {
 #if defined(__CUDA_ARCH__)
     return (uint8_t)(__brev((unsigned int)b) >> 24);
@@ -384,7 +383,4 @@ SKML_HD uint8_t skml_brev8(uint8_t b) {
     b = (uint8_t)(((b & 0xCCu) >> 2) | ((b & 0x33u) << 2));
     b = (uint8_t)(((b & 0xAAu) >> 1) | ((b & 0x55u) << 1));
     return b;
-}
-SKML_HD uint8_t skml_delta_stream_byte(uint32_t delta, int w, int j) {
-    return skml_brev8((uint8_t)(delta >> (8 * (w - 1 - j))));
 }

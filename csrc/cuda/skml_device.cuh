@@ -66,11 +66,6 @@ __device__ __forceinline__ unsigned int skml_recip32(unsigned int size) {
     const unsigned int q = 0xFFFFFFFFu / size;   // floor(2^32 / size) is one more where size divides 2^32
     return q + (0xFFFFFFFFu - q * size == size - 1u ? 1u : 0u);
 }
-__device__ __forceinline__ bool skml_rows_are_mixers(const unsigned char* ids, int rows) {
-    bool ok = true;
-    for (int r = 0; r < rows; ++r) ok = ok && ids[r] < 3;
-    return ok;
-}
 __device__ __forceinline__ int skml_java_mod(unsigned int code, unsigned int size, unsigned int recip) {
     const bool neg = (int)code < 0;
     const unsigned int a = neg ? 0u - code : code;
@@ -329,15 +324,6 @@ __device__ __forceinline__ void upper_bounds_f(const float* a, int top, const fl
 }
 
 // Number of elements of the ascending array a[0..n) that are <= x (upper bound).
-__device__ __forceinline__ int upper_bound_f(const float* a, int n, float x) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (a[mid] <= x) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
 __device__ __forceinline__ int upper_bound_u(const unsigned int* a, int n, unsigned int x) {
     int lo = 0, hi = n;
     while (lo < hi) {
