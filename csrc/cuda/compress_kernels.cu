@@ -293,10 +293,12 @@ __device__ __forceinline__ void stage_stamp(unsigned int* ctrl, int i) {
     }
 }
 
-// Clears the local slot (16-byte units; a capacity that is no multiple of 16 keeps its last bytes to the tail).
-__device__ void clear_slot(const CP& p, long long gid, long long gsz) {
+// Clears the local slot from byte `from` (a multiple of 16) on, in 16-byte units; a capacity that is no multiple of 16
+// keeps its last bytes to the tail. Nothing orders the callers' stores against those of other blocks: bytes that
+// another block writes in the same launch need a grid barrier in between.
+__device__ void clear_slot(const CP& p, long long from, long long gid, long long gsz) {
     uint4* z4 = reinterpret_cast<uint4*>(p.payload);
-    for (long long i = gid; i < p.slot_capacity / 16; i += gsz) __stcs(z4 + i, make_uint4(0, 0, 0, 0));
+    for (long long i = from / 16 + gid; i < p.slot_capacity / 16; i += gsz) __stcs(z4 + i, make_uint4(0, 0, 0, 0));
     if (gid < (p.slot_capacity & 15)) p.payload[(p.slot_capacity & ~15ll) + gid] = 0;
 }
 
@@ -2297,7 +2299,7 @@ __device__ void stage_prepare(const CP& p, long long n) {
     uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
     uint4* t4 = reinterpret_cast<uint4*>(p.tables);
     for (long long i = gid; i < (cells + 3) / 4; i += gsz) t4[i] = ones;
-    if (p.zero_slot) clear_slot(p, gid, gsz);
+    if (p.zero_slot) clear_slot(p, 0, gid, gsz);   // (two grid barriers lie before the first byte of the payload)
     if (p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE || p.huffman) {
         // the bit streams are completed with atomic ORs where chunks meet: they start from zero
         long long bound = payload_bound(n, 0, p.q, p.G, p.rows, p.col_ratio);
@@ -2555,7 +2557,6 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
     // values in the header only) are collected by the code pass, and the header is written after it
     const bool sample = p.sample_splits != 0 && !given;
     if (FUSED || stage == 1) {
-        if (p.zero_slot) clear_slot(p, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
         if (sample) stage_sample_splits(p, s, vals, n);
         else if (!given) stage_summary(p, s, vals, n);
     }
@@ -2580,6 +2581,11 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
             return;
         }
         if (!sample && blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
+        const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        // What lies before the end of the codes is written whole (header and bucket values by block 0, the code section
+        // with its padding below) and not cleared: with sampled splits no grid barrier lies in between, so a late block
+        // would clear codes that another one has written.
+        if (p.zero_slot) clear_slot(p, (long long)total, gid, gsz);
         unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
         // Four adjacent values per thread: one vector load, four searches side by side, one store. (Sixteen values a
         // thread, searched one after another, left two thirds of the threads idle at 1M coordinates: 25 us.)
@@ -2587,7 +2593,6 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
         const int top = build_search(s);
         __syncthreads();
         const bool vec = (reinterpret_cast<uintptr_t>(vals) & 15) == 0;
-        const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
         for (long long u = gid; u < units; u += gsz) {
             const long long i0 = 4 * u;
             float x[4] = {0.f, 0.f, 0.f, 0.f};
@@ -2680,7 +2685,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             __syncthreads();
             if (blockIdx.x == 0) {
                 if (p.zero_slot) {   // by this block alone, before its own header
-                    clear_slot(p, threadIdx.x, blockDim.x);
+                    clear_slot(p, 0, threadIdx.x, blockDim.x);
                     __syncthreads();
                 }
                 write_header(p, s, 0, SKML_KIND_EMPTY);   // locally and into the peers' slots

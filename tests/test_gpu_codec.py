@@ -669,3 +669,24 @@ def test_decode_with_exactly_the_keys_it_was_built_for(ns, grid):
     dec.decode_update([b.data_ptr() for b in bufs], [None] * P, min(b.numel() for b in bufs), 7, status, out_sum=out)
     assert int(status.item()) == 0
     assert np.abs(out.cpu().numpy() - g).max() < 1e-7
+
+
+@pytest.mark.parametrize("q", [2, 256, 300])
+@pytest.mark.parametrize("dim", [1, 5, 4099, 1_000_003, 20_000_001])
+def test_dense_kind_with_sampled_splits_into_a_fresh_slot(dim, q):
+    """Splits from the kernel's own sample, a buffer that is not zero when it is handed out: every code is the number
+    of split points at or below its value, and what lies behind the payload is zero. (A slot cleared beside the code
+    pass, without a grid barrier in between, can lose codes of other blocks.)"""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import GpuCompressor
+    vals = np.random.default_rng(dim).normal(0, 1e-2, dim).astype(np.float32)
+    comp = GpuCompressor(dim, dim, q, 8, 2, 0.3, seed=1)
+    v = torch.from_numpy(vals).cuda()
+    for _ in range(3):
+        torch.full((comp.capacity,), 0xA5, dtype=torch.uint8, device="cuda")   # back to the allocator, for the call below
+        buf = comp.compress_local(None, v, dense=True)
+        p = oracle.parse(comp.payload_bytes(buf))
+        want = np.searchsorted(comp.last_splits(), vals, side="right")
+        assert p["bin_num"] == len(comp.last_splits()) + 1
+        assert np.array_equal(np.asarray(p["dense_codes"][:dim]).astype(np.int64), want)
+        assert int(torch.count_nonzero(buf[p["total_bytes"]:])) == 0
