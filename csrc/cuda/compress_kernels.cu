@@ -2428,12 +2428,14 @@ __device__ void copy_range_to_peers(const CP& p, unsigned long long lo, unsigned
 
 // The block barrier orders every thread's stores before thread 0's fence, and the fence before the count, so one
 // thread fences for the block (1024 threads fencing at system scope took 7 us); peers' memory needs system scope.
+// A checked call returns on the last block's word, before the kernel has ended: that word must carry the other blocks'
+// stores (and statuses) too. Only a launch alone, without flag and word, leaves its readers to the end of the kernel.
 __device__ void finish_publish(const CP& p) {
     __shared__ int s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
         if (p.world > 1) __threadfence_system();
-        else if (p.peer_flag[0]) __threadfence();   // (alone and without a flag the end of the kernel orders the readers)
+        else if (p.peer_flag[0] || p.done_word) __threadfence();
         unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
         s_last = prev == gridDim.x - 1;
         if (s_last) {       // nobody is in a grid barrier any more

@@ -883,6 +883,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
             // the last block to finish leaves the kernel's true end time (block 0's stamp above is its own)
             __syncthreads();
             if (threadIdx.x == 0) {
+                if (p.done_word) __threadfence();   // a checked call returns before the kernel ends (see skml_store_done)
                 const unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
                 if (prev == gridDim.x - 1) {
                     p.ctrl[2] = 0;
@@ -914,11 +915,14 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
     finish_norm(p, dsq);
     if (FUSED) {
         __syncthreads();
-        if (threadIdx.x == 0 && atomicAdd(&p.ctrl[2], 1u) == gridDim.x - 1) {
-            p.ctrl[2] = 0;
-            p.ctrl[0] = 0;
-            __threadfence();
-            skml_store_done(p.done_word, p.done_seq, p.status);
+        if (threadIdx.x == 0) {
+            if (p.done_word) __threadfence();
+            if (atomicAdd(&p.ctrl[2], 1u) == gridDim.x - 1) {
+                p.ctrl[2] = 0;
+                p.ctrl[0] = 0;
+                __threadfence();
+                skml_store_done(p.done_word, p.done_seq, p.status);
+            }
         }
     }
 }

@@ -45,7 +45,7 @@ typedef struct SkmlCompressArgs {
     const float* dense_vals;       // values of the dense kind: the sparse entry point then serves both kinds in one launch
                                    // (meta[1] chooses on the device); null = it leaves the dense kind alone
     long long n_value, kind_value; // count and kind when `meta` is null
-    long long zero_slot;           // 1 = the local slot is cleared up to slot_capacity first
+    long long zero_slot;           // 1 = bytes of the local slot that the payload does not cover are zero afterwards
     unsigned long long* done_word; // pinned host word of the checked call (skml_compress_checked sets done_seq itself)
     unsigned long long done_seq;
 } SkmlCompressArgs;
@@ -61,7 +61,8 @@ int skml_compress_sparse(const SkmlCompressArgs* args, void* stream);
 int skml_compress_cluster_size();
 int skml_compress_dense(const SkmlCompressArgs* args, void* stream);
 // skml_compress_sparse that returns once the kernel's status word is known (*status_out; nothing is read back through
-// the stream: the kernel's last block stores it into args->done_word, which the call polls).
+// the stream: the kernel's last block stores it into args->done_word, which the call polls). The payload is complete
+// then: any stream may read it, and the inputs may be written again, although the kernel may not have left the device.
 int skml_compress_checked(SkmlCompressArgs* args, unsigned int* status_out, void* stream);
 
 // Arguments of the fused decode + aggregate + update kernel.
@@ -102,7 +103,8 @@ typedef struct SkmlDecodeArgs {
 
 long long skml_decode_workspace_bytes(long long world, long long group_num);
 int skml_decode_update(const SkmlDecodeArgs* args, void* stream);
-// Clears out_sum, decodes into it and returns once the kernel's status word is known (see skml_compress_checked).
+// Clears out_sum, decodes into it and returns once the kernel's status word is known; out_sum is complete then, for any
+// stream (see skml_compress_checked).
 int skml_decode_sum_checked(SkmlDecodeArgs* args, unsigned int* status_out, void* stream);
 
 // GLM numerics

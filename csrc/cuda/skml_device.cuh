@@ -348,6 +348,9 @@ __device__ __forceinline__ int lower_bound_u(const unsigned int* a, int n, unsig
 // the caller polls that word, instead of a device-to-host copy and a stream synchronisation (15 us and more
 // on top of a 35 us kernel). A kernel that reported an error may end without the store: the stream is
 // queried now and then, and once it has drained the status word is read the plain way.
+// The caller goes on while the kernel's blocks are still leaving, so every block fences after its last store and
+// before it counts itself, and the last one fences after it has counted and before it reads the status here: whoever
+// has seen the word sees every block's outputs, on any stream.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void skml_store_done(unsigned long long* word, unsigned long long seq, const unsigned int* status) {
     if (word) st_release_sys(word, (seq << 32) | ld_relaxed_gpu(status));
@@ -358,6 +361,7 @@ static inline int skml_wait_done(volatile unsigned long long* word, unsigned lon
     for (unsigned long long spins = 1;; ++spins) {
         const unsigned long long v = *word;
         if ((v >> 32) == (seq & 0xFFFFFFFFull)) {
+            __atomic_thread_fence(__ATOMIC_ACQUIRE);   // what the kernel left beside the word is read after it
             *status_out = (unsigned int)v;
             return 0;
         }

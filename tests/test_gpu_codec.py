@@ -690,3 +690,28 @@ def test_dense_kind_with_sampled_splits_into_a_fresh_slot(dim, q):
         assert p["bin_num"] == len(comp.last_splits()) + 1
         assert np.array_equal(np.asarray(p["dense_codes"][:dim]).astype(np.int64), want)
         assert int(torch.count_nonzero(buf[p["total_bytes"]:])) == 0
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_checked_calls_leave_their_results_to_any_stream(dense):
+    """`compress_local` and `decode_sum` return when the kernel's last block has reported, not when the kernel has left
+    the device: a second stream that waits for nothing reads what the first call's stream would read."""
+    from sketchml_b200.ops import GpuCompressor, GpuDecoder
+    dim, n = 6_000_000, 6_000_000 if dense else 700_000
+    keys, vals = (None, np.random.default_rng(3).normal(0, 1e-2, dim).astype(np.float32)) if dense else _sparse_grad(n, dim, seed=3)
+    k, v = None if dense else torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda()
+    comp, dec = GpuCompressor(dim, n, 256, 8, 3, 0.2, seed=2), GpuDecoder(dim, n, max_groups=8)
+    want = comp.compress_local(k, v, dense=dense)
+    torch.cuda.synchronize()
+    want_sum = dec.decode_sum([want]).clone()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for _ in range(20):
+        buf = comp.compress_local(k, v, dense=dense)
+        with torch.cuda.stream(side):
+            got = buf.clone()
+        out = dec.decode_sum([buf])
+        with torch.cuda.stream(side):
+            got_sum = out.clone()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and torch.equal(got_sum, want_sum)
