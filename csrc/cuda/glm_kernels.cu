@@ -794,7 +794,8 @@ __global__ void update_dense_kernel(float* w, float* m, float* v, const float* g
 
 __global__ void update_sparse_kernel(float* w, float* m, float* v, const int* keys, const float* vals,
                                      const long long* n_ptr, long long n_max, float scale, int adam, float lr,
-                                     float adam_scale, long long ms) {
+                                     float adam_scale, long long ms, const unsigned int* status) {
+    if (skml_failed(status)) return;
     long long n = n_ptr ? *n_ptr : n_max;
     if (n > n_max) n = n_max;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -811,10 +812,10 @@ extern "C" int skml_update_dense(float* w, float* m, float* v, const float* g, l
 
 extern "C" int skml_update_sparse(float* w, float* m, float* v, const int* keys, const float* vals,
                                   const long long* n_ptr, long long n_max, float scale, int adam, float lr,
-                                  float adam_scale, int adam_stride, void* stream) {
+                                  float adam_scale, int adam_stride, const unsigned int* status, void* stream) {
     int grid = sm_count() * 8;
     update_sparse_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(w, m, v, keys, vals, n_ptr, n_max, scale, adam, lr,
-                                                                 adam_scale, adam_stride > 1 ? adam_stride : 1);
+                                                                 adam_scale, adam_stride > 1 ? adam_stride : 1, status);
     return (int)cudaGetLastError();
 }
 
@@ -885,7 +886,9 @@ extern "C" int skml_weight_norm(const float* w, long long dim, double lambda, do
 // (exactly zero, skipped) by the later ones. A sum that is exactly zero is a no-op, as in the
 // `sparse_only` dense update.
 __global__ void update_gathered_kernel(float* w, float* m, float* v, float* acc, const int* keys, const long long* count,
-                                       long long stride, float scale, int adam, float lr, float adam_scale, long long ms) {
+                                       long long stride, float scale, int adam, float lr, float adam_scale, long long ms,
+                                       const unsigned int* status) {
+    if (skml_failed(status)) return;
     long long n = *count;
     if (n > stride) n = stride;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -899,11 +902,11 @@ __global__ void update_gathered_kernel(float* w, float* m, float* v, float* acc,
 
 extern "C" int skml_update_gathered(float* w, float* m, float* v, float* acc, const int* keys, const long long* counts,
                                     long long stride, int lists, float scale, int adam, float lr, float adam_scale,
-                                    int adam_stride, void* stream) {
+                                    int adam_stride, const unsigned int* status, void* stream) {
     for (int l = 0; l < lists; ++l) {
         update_gathered_kernel<<<sm_count() * 8, 256, 0, (cudaStream_t)stream>>>(w, m, v, acc, keys + (long long)l * stride,
                                                                                  counts + l, stride, scale, adam, lr, adam_scale,
-                                                                                 adam_stride > 1 ? adam_stride : 1);
+                                                                                 adam_stride > 1 ? adam_stride : 1, status);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }

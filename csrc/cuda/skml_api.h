@@ -120,16 +120,18 @@ int skml_compact(float* g, const float* w, unsigned int* bitmap, int dim, float 
                  void* stream);
 long long skml_compact_blocks(int dim);
 // The update entry points take `adam_stride`: elements between the moments of neighbouring coordinates (1: plain
-// arrays, 4: packed quads, see SkmlDecodeArgs).
+// arrays, 4: packed quads, see SkmlDecodeArgs). With a `status` word given, the updates that follow a coded exchange do
+// nothing once it reports an error.
 int skml_update_dense(float* w, float* m, float* v, const float* g, long long dim, float scale, int adam, float lr,
                       float adam_scale, int sparse_only, int adam_stride, void* stream);
 int skml_update_sparse(float* w, float* m, float* v, const int* keys, const float* vals, const long long* n_ptr,
-                       long long n_max, float scale, int adam, float lr, float adam_scale, int adam_stride, void* stream);
+                       long long n_max, float scale, int adam, float lr, float adam_scale, int adam_stride,
+                       const unsigned int* status, void* stream);
 // Applies acc[key] * scale to the model on the coordinates of `lists` gathered key lists (list l at
 // keys + l * stride, counts[l] entries) and clears those accumulator words.
 int skml_update_gathered(float* w, float* m, float* v, float* acc, const int* keys, const long long* counts,
                          long long stride, int lists, float scale, int adam, float lr, float adam_scale, int adam_stride,
-                         void* stream);
+                         const unsigned int* status, void* stream);
 // sumsq_out[0] = sum of w^2 (double, fixed summation order), reg_out[0] = lambda * sqrt of it; one
 // launch, `scratch` holds skml_weight_norm_scratch_bytes() bytes that are zero before the first call.
 long long skml_weight_norm_scratch_bytes();
@@ -246,19 +248,20 @@ int skml_fixedpoint_unpack_scatter(float* acc, const int* keys, const unsigned c
 // Zip baseline compressor: ZipML split search on the device (no value is read back to the host), one
 // bucket code per value (skml_zipml_code_bytes(bin_num) bytes each) and a table of
 // skml_zipml_table_len(bin_num) bucket midpoints per list. `scratch`: skml_zipml_scratch_bytes(n_max)
-// bytes; meta: buckets, zero bucket, halving rounds; range: min, max. 2 <= bin_num <= 8190.
+// bytes; meta: buckets, zero bucket, halving rounds; range: min, max. 2 <= bin_num <= 8190. `status` receives a grid
+// barrier of the search that gave up; while it reports an error nothing is coded, and nothing decoded where it is given.
 long long skml_zipml_scratch_bytes(long long n_max);
 int skml_zipml_code_bytes(int bin_num);
 int skml_zipml_table_len(int bin_num);
 int skml_zipml_pack(const float* vals, const long long* n_ptr, long long n_max, int bin_num, void* scratch,
                     long long scratch_bytes, float* splits, float* mids, int* meta, float* range, unsigned char* codes,
-                    void* stream);
+                    unsigned int* status, void* stream);
 // Decodes `lists` code arrays (list l at codes + l * code_stride, keys + l * key_stride, its table at
 // mids + l * table_len, counts[l] entries); adds into acc[key] when acc is given, stores the values to
 // vals_out[l * key_stride + i] when vals_out is given (keys may then be null).
 int skml_zipml_unpack_scatter(float* acc, const int* keys, const unsigned char* codes, const float* mids,
                               const long long* counts, long long key_stride, long long code_stride, int lists,
-                              int bin_num, float* vals_out, void* stream);
+                              int bin_num, float* vals_out, const unsigned int* status, void* stream);
 
 // Peer memory (one process per GPU): CUDA IPC handles of a cudaMalloc'ed region.
 int skml_ipc_get_handle(void* dev_ptr, unsigned char* handle64);

@@ -28,6 +28,9 @@ __device__ __forceinline__ void skml_set_status(unsigned int* status, unsigned i
     atomicCAS(status, 0u, code | (detail << 8));
 }
 
+// Whether an earlier launch has reported an error (null: nobody asks).
+__device__ __forceinline__ bool skml_failed(const unsigned int* status) { return status && (*status & 0xFFu) != SKML_OK; }
+
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -25,12 +25,14 @@ static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* met
             rc = skml_fixedpoint_pack(vals, meta, a->n_max, (int)c.bits, c.seed, (double*)c.scratch, c.codes, c.norm, stream);
             if (!rc) rc = skml_fixedpoint_unpack_scatter(nullptr, keys, c.codes, c.norm, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals, stream);
         } else if (c.kind == 2) {
-            rc = skml_zipml_pack(vals, meta, a->n_max, (int)c.bits, c.scratch, c.scratch_bytes, c.splits, c.mids, c.zip_meta, c.range, c.codes, stream);
-            if (!rc) rc = skml_zipml_unpack_scatter(nullptr, keys, c.codes, c.mids, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals, stream);
+            rc = skml_zipml_pack(vals, meta, a->n_max, (int)c.bits, c.scratch, c.scratch_bytes, c.splits, c.mids, c.zip_meta, c.range, c.codes,
+                                 a->status, stream);
+            if (!rc) rc = skml_zipml_unpack_scatter(nullptr, keys, c.codes, c.mids, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals,
+                                                    a->status, stream);
         }
         if (rc) return rc;
         rc = skml_update_sparse(a->w, c.adam_m, c.adam_v, keys, vals, meta, a->n_max, 1.f, c.adam_v != nullptr, (float)a->lr,
-                                (float)a->adam_scale, (int)c.adam_stride, stream);
+                                (float)a->adam_scale, (int)c.adam_stride, a->status, stream);
         if (!rc && batch_keys) rc = batch_consumed(a, (cudaStream_t)stream);
         if (rc) return rc;
         return (int)cudaMemcpyAsync(a->loss_out, a->partials, 4 * sizeof(double), cudaMemcpyDeviceToDevice, (cudaStream_t)stream);

@@ -18,6 +18,8 @@
 // be among the round's largest, publishes them, and after a grid barrier selects among all blocks' lists,
 // which also tells it how many pairs the blocks before it keep split. The rest is block 0's alone, about
 // 2 us a round. (One block for all rounds took 822 us for 330,000 values.)
+// A barrier that gives up reports to the caller's status word; the tables are then those of an earlier call, so the
+// kernels behind the search, and the update behind them, do nothing once the word is set.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -37,7 +39,7 @@ constexpr int Z_TAIL = 512;             // candidates one warp handles in shared
 
 // What the blocks of the split search share (cleared by the pad kernel).
 struct ZShared {
-    unsigned int bar, status, pad[14];
+    unsigned int bar, pad[15];
     double sum_v[Z_MAX_BLOCKS], sum_v2[Z_MAX_BLOCKS];     // sums over the blocks' slices of values
     unsigned long long cand[Z_ALONE];                     // blocks x kept pairs of a round at most
 };
@@ -89,7 +91,7 @@ __global__ void zip_pad_kernel(const float* __restrict__ vals, const long long* 
                                float* __restrict__ out, ZShared* __restrict__ shared) {
     long long n = *n_ptr;
     if (n > n_max) n = n_max;
-    if (blockIdx.x == 0 && threadIdx.x == 0) shared->bar = shared->status = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) shared->bar = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_max; i += (long long)gridDim.x * blockDim.x)
         out[i] = i < n ? vals[i] : __int_as_float(0x7F800000);
 }
@@ -293,7 +295,7 @@ __device__ void tail_rounds(ZSmem& sm, int bin_num, double end_v, double end_v2,
 __global__ void __launch_bounds__(ZT, 1)
 zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_max, int bin_num,
                   float* __restrict__ splits_out, float* __restrict__ mids_out, int* __restrict__ meta_out,
-                  float* __restrict__ range_out) {
+                  float* __restrict__ range_out, unsigned int* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ZSmem& sm = *reinterpret_cast<ZSmem*>(smem_raw);
     unsigned int* const sh_warp = sm.warp;
@@ -301,7 +303,7 @@ zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_m
     const int tid = threadIdx.x, lane = tid & 31;
     const unsigned int nb = gridDim.x, b = blockIdx.x;
     unsigned int passed = 0;
-    auto barrier = [&](unsigned int stage) { return skml_grid_barrier(&g.bar, nb, &g.status, 2000000000ll, stage, passed); };
+    auto barrier = [&](unsigned int stage) { return skml_grid_barrier(&g.bar, nb, status, 2000000000ll, stage, passed); };
     long long n64 = *n_ptr;
     if (n64 > n_max) n64 = n_max;
     const unsigned int n = (unsigned int)n64;
@@ -513,8 +515,9 @@ zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_m
 __global__ void __launch_bounds__(256)
 zip_code_kernel(const float* __restrict__ vals, const long long* __restrict__ n_ptr, long long n_max,
                 const float* __restrict__ splits, const int* __restrict__ meta, int code_bytes,
-                unsigned char* __restrict__ codes) {
+                unsigned char* __restrict__ codes, const unsigned int* __restrict__ status) {
     extern __shared__ float sh_splits[];
+    if (skml_failed(status)) return;
     const int nb = meta[0], ns = nb > 0 ? nb - 1 : 0;
     for (int i = threadIdx.x; i < ns; i += blockDim.x) sh_splits[i] = splits[i];
     __syncthreads();
@@ -536,8 +539,9 @@ zip_code_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
 __global__ void __launch_bounds__(256)
 zip_unpack_scatter_kernel(float* __restrict__ acc, const int* __restrict__ keys, const unsigned char* __restrict__ codes,
                           const float* __restrict__ mids, const long long* __restrict__ count, long long key_stride,
-                          int code_bytes, int table_len, float* __restrict__ vals_out) {
+                          int code_bytes, int table_len, float* __restrict__ vals_out, const unsigned int* __restrict__ status) {
     extern __shared__ float sh_mids[];
+    if (skml_failed(status)) return;
     for (int i = threadIdx.x; i < table_len; i += blockDim.x) sh_mids[i] = mids[i];
     __syncthreads();
     long long n = *count;
@@ -577,8 +581,8 @@ extern "C" int skml_zipml_table_len(int bin_num) { return bin_num + 2; }
 // meta[3] (buckets, zero bucket, rounds), range[2]. splits: bin_num + 2 floats for the split points.
 extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long long n_max, int bin_num, void* scratch,
                                long long scratch_bytes, float* splits, float* mids, int* meta, float* range,
-                               unsigned char* codes, void* stream) {
-    if (bin_num < 2 || bin_num + 2 > Z_MAX_BUCKETS || n_max < 1 || n_max > 0x7FFFFFFFll) return (int)cudaErrorInvalidValue;
+                               unsigned char* codes, unsigned int* status, void* stream) {
+    if (!status || bin_num < 2 || bin_num + 2 > Z_MAX_BUCKETS || n_max < 1 || n_max > 0x7FFFFFFFll) return (int)cudaErrorInvalidValue;
     ZScratch z;
     if ((long long)carve(reinterpret_cast<unsigned char*>(scratch), n_max, &z) > scratch_bytes) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
@@ -598,11 +602,11 @@ extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long l
         if (e != cudaSuccess) return (int)e;
         ready = true;
     }
-    void* args[] = {&z, &n_ptr, &n_max, &bin_num, &splits, &mids, &meta, &range};
+    void* args[] = {&z, &n_ptr, &n_max, &bin_num, &splits, &mids, &meta, &range, &status};
     e = cudaLaunchCooperativeKernel((const void*)zip_splits_kernel, dim3((unsigned)blocks), dim3(ZT), args, sizeof(ZSmem), s);
     if (e != cudaSuccess) return (int)e;
     const int cb = skml_zipml_code_bytes(bin_num);
-    zip_code_kernel<<<zip_sm_count() * 4, 256, sizeof(float) * (size_t)(bin_num + 2), s>>>(vals, n_ptr, n_max, splits, meta, cb, codes);
+    zip_code_kernel<<<zip_sm_count() * 4, 256, sizeof(float) * (size_t)(bin_num + 2), s>>>(vals, n_ptr, n_max, splits, meta, cb, codes, status);
     return (int)cudaGetLastError();
 }
 
@@ -610,14 +614,14 @@ extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long l
 // mids: `lists` tables of bin_num + 2 floats; codes: `lists` arrays code_stride bytes apart.
 extern "C" int skml_zipml_unpack_scatter(float* acc, const int* keys, const unsigned char* codes, const float* mids,
                                          const long long* counts, long long key_stride, long long code_stride,
-                                         int lists, int bin_num, float* vals_out, void* stream) {
+                                         int lists, int bin_num, float* vals_out, const unsigned int* status, void* stream) {
     if (bin_num < 2 || bin_num + 2 > Z_MAX_BUCKETS) return (int)cudaErrorInvalidValue;
     const int cb = skml_zipml_code_bytes(bin_num);
     for (int l = 0; l < lists; ++l) {
         const int tl = bin_num + 2;
         zip_unpack_scatter_kernel<<<zip_sm_count() * 4, 256, sizeof(float) * (size_t)tl, (cudaStream_t)stream>>>(
             acc, keys ? keys + (long long)l * key_stride : nullptr, codes + (long long)l * code_stride,
-            mids + (long long)l * tl, counts + l, key_stride, cb, tl, vals_out ? vals_out + (long long)l * key_stride : nullptr);
+            mids + (long long)l * tl, counts + l, key_stride, cb, tl, vals_out ? vals_out + (long long)l * key_stride : nullptr, status);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }

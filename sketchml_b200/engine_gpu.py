@@ -153,7 +153,7 @@ class GpuEngine:
                 self.fp_codec = FixedPointCodec(bound, conf.fixed_point_bit_num, comm.world, self.device)
             elif self.value_quant == C.COMPRESSOR_ZIP:
                 from .ops.baseline_quant import ZipCodec
-                self.zip_codec = ZipCodec(bound, conf.quant_bin_num, comm.world, self.device)
+                self.zip_codec = ZipCodec(bound, conf.quant_bin_num, comm.world, self.device, self.st.status)
             self._prepare_fast_step()
         else:
             self.dense_sum = torch.zeros(dim, dtype=torch.float32, device=self.device)
@@ -511,9 +511,9 @@ class GpuEngine:
                                                 L.ptr(self.kv_counts), self.n_max, comm.world, L.stream()), "scatter_kv")
                 # update and clear on the gathered coordinates only: nothing here is proportional to dim
                 update_gathered(m.weights, self.kv_acc, self.kv_keys, self.kv_counts, self.n_max, comm.world,
-                                1.0 / comm.world, lr, am, av, adam_scale)
+                                1.0 / comm.world, lr, am, av, adam_scale, st.status)
             else:
-                update_sparse(m.weights, st.keys, st.vals, st.meta, self.n_max, 1.0, lr, am, av, adam_scale)
+                update_sparse(m.weights, st.keys, st.vals, st.meta, self.n_max, 1.0, lr, am, av, adam_scale, st.status)
             ring.copy_(st.partials)
         self.batch_index += 1
 
@@ -559,10 +559,10 @@ class GpuEngine:
             dist.all_reduce(st.partials)
             codec.unpack(self.kv_keys, all_codes, all_side, self.kv_counts, comm.world, acc=self.kv_acc)
             update_gathered(m.weights, self.kv_acc, self.kv_keys, self.kv_counts, self.n_max, comm.world,
-                            1.0 / comm.world, lr, am, av, adam_scale)
+                            1.0 / comm.world, lr, am, av, adam_scale, st.status)
         else:
             codec.unpack(st.keys, codes, side, st.meta[:1], 1, vals_out=st.vals)
-            update_sparse(m.weights, st.keys, st.vals, st.meta, self.n_max, 1.0, lr, am, av, adam_scale)
+            update_sparse(m.weights, st.keys, st.vals, st.meta, self.n_max, 1.0, lr, am, av, adam_scale, st.status)
         ring.copy_(st.partials)
 
     def _fp_seed(self, step: int) -> int:
@@ -586,7 +586,7 @@ class GpuEngine:
                 cache = self.__dict__.setdefault("_zip_roundtrip", {})
                 zc = cache.get(vals.numel())
                 if zc is None:
-                    zc = cache[vals.numel()] = ZipCodec(vals.numel(), conf.quant_bin_num, 1, self.device)
+                    zc = cache[vals.numel()] = ZipCodec(vals.numel(), conf.quant_bin_num, 1, self.device, st.status)
                 zc.roundtrip(vals, n.reshape(1))
 
     def _densify(self) -> None:
@@ -608,6 +608,8 @@ class GpuEngine:
             s = read_status(self.sts[1].status)
         if s:
             self.partials_template[3:].zero_()   # the loss of a step that did not get as far as settling it
+            if self.mode == "nccl_kv":
+                self.kv_acc.zero_()   # sums that a skipped update has left behind
             if self.mode == "sketch":
                 self.comp.reset()
                 self.dec.reset()

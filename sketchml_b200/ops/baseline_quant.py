@@ -16,6 +16,8 @@ bin_num/2 adjacent pairs with the largest squared error, bucket midpoints as dec
 """
 from __future__ import annotations
 
+from typing import Optional
+
 import torch
 
 from . import lib as L
@@ -83,9 +85,10 @@ def fixed_point_roundtrip(vals: torch.Tensor, n: torch.Tensor, num_bits: int, se
 class ZipCodec:
     """ZipML quantizer on the device for up to ``n_max`` values: ``pack`` leaves one bucket code per value
     (``code_bytes`` each) and the table of bucket midpoints; these and the raw keys are what travels
-    between ranks. No step of it reads anything back to the host."""
+    between ranks. No step of it reads anything back to the host: an error (a grid barrier of the split search that
+    gave up) goes to ``status``, and nothing is coded or decoded from then on until the word is cleared."""
 
-    def __init__(self, n_max: int, bin_num: int, world: int, device):
+    def __init__(self, n_max: int, bin_num: int, world: int, device, status: Optional[torch.Tensor] = None):
         self.lib = L.lib()
         self.n_max, self.bin_num, self.world = int(n_max), int(bin_num), int(world)
         if not 2 <= self.bin_num <= 8190:
@@ -102,6 +105,7 @@ class ZipCodec:
         self.mids = torch.zeros(self.table_len, dtype=torch.float32, device=device)
         self.meta = torch.zeros(4, dtype=torch.int32, device=device)
         self.range = torch.zeros(2, dtype=torch.float32, device=device)
+        self.status = status if status is not None else torch.zeros(1, dtype=torch.int32, device=device)
         if world > 1:
             self.all_codes = torch.zeros((world, self.code_stride), dtype=torch.uint8, device=device)
             self.all_mids = torch.zeros((world, self.table_len), dtype=torch.float32, device=device)
@@ -110,14 +114,14 @@ class ZipCodec:
         """vals[:n] -> self.codes, self.mids, self.meta (n: device int64 scalar / 1-element view)."""
         L.check(self.lib.skml_zipml_pack(L.ptr(vals), L.ptr(n), self.n_max, self.bin_num, L.ptr(self.scratch),
                                          self.scratch_bytes, L.ptr(self.splits), L.ptr(self.mids), L.ptr(self.meta),
-                                         L.ptr(self.range), L.ptr(self.codes), L.stream()), "skml_zipml_pack")
+                                         L.ptr(self.range), L.ptr(self.codes), L.ptr(self.status), L.stream()), "skml_zipml_pack")
         L.count_launches(4)
 
     def unpack(self, keys, codes: torch.Tensor, mids: torch.Tensor, counts: torch.Tensor, lists: int,
                acc: torch.Tensor = None, vals_out: torch.Tensor = None) -> None:
         L.check(self.lib.skml_zipml_unpack_scatter(L.ptr(acc), L.ptr(keys), L.ptr(codes), L.ptr(mids), L.ptr(counts),
                                                    self.n_max, self.code_stride, lists, self.bin_num, L.ptr(vals_out),
-                                                   L.stream()), "skml_zipml_unpack_scatter")
+                                                   L.ptr(self.status), L.stream()), "skml_zipml_unpack_scatter")
         L.count_launches(lists)
 
     def coded_args(self) -> L.CodedArgs:

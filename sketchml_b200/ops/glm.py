@@ -134,16 +134,18 @@ def update_dense(w, g, scale: float, lr: float, m=None, v=None, adam_scale: floa
 
 
 def update_gathered(w, acc, keys, counts, stride: int, lists: int, scale: float, lr: float, m=None, v=None,
-                    adam_scale: float = 1.0):
-    """Applies ``acc[key] * scale`` on the coordinates of the gathered key lists and clears them."""
+                    adam_scale: float = 1.0, status: Optional[torch.Tensor] = None):
+    """Applies ``acc[key] * scale`` on the coordinates of the gathered key lists and clears them (not at all once
+    ``status`` reports an error)."""
     L.check(L.lib().skml_update_gathered(L.ptr(w), L.ptr(m), L.ptr(v), L.ptr(acc), L.ptr(keys), L.ptr(counts), stride,
-                                         lists, scale, int(v is not None), lr, adam_scale, moment_stride(m, v), L.stream()),
-            "skml_update_gathered")
+                                         lists, scale, int(v is not None), lr, adam_scale, moment_stride(m, v), L.ptr(status),
+                                         L.stream()), "skml_update_gathered")
     L.count_launches(lists)
 
 
 def update_sparse(w, keys, vals, n_ptr: Optional[torch.Tensor], n_max: int, scale: float, lr: float, m=None, v=None,
-                  adam_scale: float = 1.0):
+                  adam_scale: float = 1.0, status: Optional[torch.Tensor] = None):
+    """``vals * scale`` on the listed coordinates (not at all once ``status`` reports an error)."""
     L.check(L.lib().skml_update_sparse(L.ptr(w), L.ptr(m), L.ptr(v), L.ptr(keys), L.ptr(vals), L.ptr(n_ptr), n_max,
-                                       scale, int(v is not None), lr, adam_scale, moment_stride(m, v), L.stream()),
+                                       scale, int(v is not None), lr, adam_scale, moment_stride(m, v), L.ptr(status), L.stream()),
             "skml_update_sparse")

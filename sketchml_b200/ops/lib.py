@@ -109,7 +109,7 @@ _SIGS = {
     "skml_compact": (c_int, [c_vp, c_vp, c_vp, c_int, c_f, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_vp, c_vp]),
     "skml_compact_blocks": (c_ll, [c_int]),
     "skml_update_dense": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_f, c_int, c_f, c_f, c_int, c_int, c_vp]),
-    "skml_update_sparse": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_f, c_int, c_f, c_f, c_int, c_vp]),
+    "skml_update_sparse": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_f, c_int, c_f, c_f, c_int, c_vp, c_vp]),
     "skml_scatter_kv": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_int, c_vp]),
     "skml_weight_norm_scratch_bytes": (c_ll, []),
     "skml_weight_norm": (c_int, [c_vp, c_ll, c_d, c_vp, c_vp, c_vp, c_vp]),
@@ -119,7 +119,7 @@ _SIGS = {
     "skml_dt_fill": (c_int, [C.POINTER(DenseIndexArgs), c_vp, c_vp, c_vp, c_ll, c_ll, c_vp, c_vp]),
     "skml_dt_gradient": (c_int, [C.POINTER(DenseIndexArgs), c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_d, c_vp, c_int, c_f, c_vp, c_vp, c_vp,
                                  c_vp, c_ll, c_vp]),
-    "skml_update_gathered": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_int, c_f, c_int, c_f, c_f, c_int, c_vp]),
+    "skml_update_gathered": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_int, c_f, c_int, c_f, c_f, c_int, c_vp, c_vp]),
     "skml_gen_wstar": (c_int, [c_vp, c_ll, c_d, c_ull, c_vp]),
     "skml_gen_rows": (c_int, [c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_d, c_int, c_int, c_f, c_vp, c_ull, c_vp]),
     "skml_glm_coef": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_ll, c_int, c_f, c_vp, c_vp, c_vp, c_ll, c_vp]),
@@ -139,8 +139,8 @@ _SIGS = {
     "skml_zipml_scratch_bytes": (c_ll, [c_ll]),
     "skml_zipml_code_bytes": (c_int, [c_int]),
     "skml_zipml_table_len": (c_int, [c_int]),
-    "skml_zipml_pack": (c_int, [c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
-    "skml_zipml_unpack_scatter": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_vp, c_vp]),
+    "skml_zipml_pack": (c_int, [c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "skml_zipml_unpack_scatter": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_vp, c_vp, c_vp]),
     "skml_fixedpoint_unpack_scatter": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_vp, c_vp]),
     "skml_train_step": (c_int, [C.POINTER(StepArgs), c_vp]),
     "skml_ipc_get_handle": (c_int, [c_vp, c_vp]),

@@ -267,3 +267,31 @@ def test_baseline_step_behind_one_call_equals_its_separate_calls(name, opt):
     h2, w2, _ = _train(_conf(extras={"single_call_step": False}, **kw))
     assert torch.equal(w1, w2)
     assert np.allclose(h1["train_loss"], h2["train_loss"], rtol=1e-12)
+
+
+@pytest.mark.parametrize("single_call", [True, False])
+@pytest.mark.parametrize("opt", ["sgd", "adam"])
+@pytest.mark.parametrize("rows", [1000, 60000])
+def test_zip_step_after_a_reported_error_changes_nothing_and_is_raised(rows, opt, single_call):
+    """A split search that gives up at a grid barrier leaves the tables of an earlier step. Its status word (set here on
+    the host, as such a search would) keeps codes, values, weights and moments as they are and reaches the engine's
+    check; search by one block and by several."""
+    from sketchml_b200.parallel.failure import STATUS_TIMEOUT_BARRIER, StepTimeout
+    from sketchml_b200.trainer import Trainer
+    t = Trainer(_conf(compressor="Zip", optimizer=opt, valid_ratio=0.0, syn_rows=rows, feature_num=2000000, batch_sample_ratio=0.5,
+                      quant_bin_num=64, learn_rate=0.5 if opt == "sgd" else 0.01, extras={"single_call_step": single_call}))
+    t.load_data()
+    t.train_one_iteration(0, 0)
+    eng = t.engine
+    state = [t.model.weights] + ([t.model.optimizer.m, t.model.optimizer.v] if opt == "adam" else []) + [eng.zip_codec.codes]
+    before = [x.clone() for x in state]
+    eng.st.status.fill_(STATUS_TIMEOUT_BARRIER | 0x6200)
+    t.train_one_iteration(0, 1)
+    assert all(torch.equal(a, b) for a, b in zip(before[:-1], state[:-1]))
+    assert torch.equal(before[-1], state[-1])
+    with pytest.raises(StepTimeout):
+        eng.check()
+    t.train_one_iteration(0, 2)    # the word is clear again: the next step counts
+    eng.check()
+    assert not torch.equal(before[0], state[0])
+    t.close()
