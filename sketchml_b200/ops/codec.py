@@ -4,6 +4,7 @@ from __future__ import annotations
 import ctypes as C
 import threading
 import weakref
+from collections import deque
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -37,28 +38,25 @@ class ExchangeRegionView:
 
 class DoneWords:
     """Pinned host words for checked calls: one page for the process (pinning memory takes milliseconds), a word per
-    codec object (its 64-byte line, eight words), given back with it; an object that finds the page full pins its own."""
+    owner (its 64-byte line, eight words), given back with it; an owner that finds the page full pins its own.
+    Giving back takes no lock: a collection may do it inside `take` of the same thread."""
     _WORDS = 512
     _lock = threading.Lock()
     _page: Optional[torch.Tensor] = None
-    _free: List[int] = []
+    _free: deque = deque()
 
     @classmethod
     def take(cls, owner) -> torch.Tensor:
         with cls._lock:
             if cls._page is None:
                 cls._page = torch.zeros(cls._WORDS * 8, dtype=torch.int64).pin_memory()
-                cls._free = list(range(cls._WORDS))
-            if not cls._free:
-                return torch.zeros(8, dtype=torch.int64).pin_memory()
+                cls._free.extend(range(cls._WORDS))
+        try:
             i = cls._free.pop()
-        weakref.finalize(owner, cls._give_back, i)
+        except IndexError:
+            return torch.zeros(8, dtype=torch.int64).pin_memory()
+        weakref.finalize(owner, cls._free.append, i)
         return cls._page[8 * i:8 * i + 8]
-
-    @classmethod
-    def _give_back(cls, i: int) -> None:
-        with cls._lock:
-            cls._free.append(i)
 
 
 class _Checked:

@@ -43,8 +43,9 @@ class AdaptiveKeys:
         return 4 + 4 + 1 + 4 + 8 * self.flag_words.numel() + 4 + 8 * self.delta_words.numel()
 
 
-class _CallState(threading.local):
-    """Per thread: the pinned words a call's plan comes back in."""
+class _CallState:
+    """What one thread's calls need: the pinned words a plan comes back in. They go back when the thread ends, with this
+    object (the thread-local around it is one object for all threads and outlives them)."""
 
     def __init__(self):
         self.words = DoneWords.take(self)
@@ -52,16 +53,17 @@ class _CallState(threading.local):
         self.status_ref = C.byref(self.status)
 
 
-_call: Optional[_CallState] = None
+_call = threading.local()
 _workspace_bytes = 0
 
 
 def _call_state() -> _CallState:
-    global _call, _workspace_bytes
-    if _call is None:
+    global _workspace_bytes
+    state: Optional[_CallState] = getattr(_call, "state", None)
+    if state is None:
         _workspace_bytes = int(L.lib().skml_da_workspace_bytes())
-        _call = _CallState()
-    return _call
+        state = _call.state = _CallState()
+    return state
 
 
 def encode(keys: torch.Tensor) -> AdaptiveKeys:

@@ -383,3 +383,40 @@ def test_adam_moment_layouts_are_checked():
     with pytest.raises(ValueError):
         moment_stride(torch.zeros(10), quad[:, 1])
 
+
+
+def test_pinned_words_of_ended_threads_are_free_again(monkeypatch):
+    """Every thread that codes keys takes one of the process's pinned words and gives it back when it ends, also where a
+    collection does that while the same thread is taking one."""
+    import gc
+    import threading
+    from collections import deque
+    from sketchml_b200.ops import codec, keys
+    monkeypatch.setattr(codec.DoneWords, "_page", torch.zeros(8 * 4, dtype=torch.int64))   # (a page that is not pinned)
+    monkeypatch.setattr(codec.DoneWords, "_free", deque(range(4)))
+    seen = []
+
+    def work():
+        seen.append(int(keys._call_state().words.data_ptr()))
+        assert keys._call_state().words.data_ptr() == seen[-1]   # one word a thread
+
+    for _ in range(12):   # three times as many threads as words, one after another
+        th = threading.Thread(target=work)
+        th.start()
+        th.join()
+    gc.collect()
+    assert len(seen) == 12 and len(codec.DoneWords._free) == 4
+
+    class Owner:
+        pass
+
+    def give_back_inside_take():
+        owner = Owner()
+        codec.DoneWords.take(owner)
+        with codec.DoneWords._lock:
+            del owner       # its finalizer runs here
+
+    th = threading.Thread(target=give_back_inside_take, daemon=True)
+    th.start()
+    th.join(5.0)
+    assert not th.is_alive() and len(codec.DoneWords._free) == 4
