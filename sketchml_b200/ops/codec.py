@@ -59,6 +59,16 @@ class DoneWords:
         return cls._page[8 * i:8 * i + 8]
 
 
+class _KeepsArgs:
+    """An argument block kept between calls holds the object's settings: setting any of them drops it."""
+    _kept_args = None
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if not name.startswith("_"):
+            object.__setattr__(self, "_kept_args", None)
+
+
 class _Checked:
     """What a checked call needs besides its arguments: a status word, the pinned host word the kernel reports its
     end in, and room for the status."""
@@ -86,7 +96,7 @@ def read_status(status: torch.Tensor, reset: bool = True) -> int:
     return v
 
 
-class GpuCompressor:
+class GpuCompressor(_KeepsArgs):
     """Owns the scratch memory of the fused compress kernel for gradients of up to
     ``n_max`` non-zeros (sparse kind) or ``dim`` coordinates (dense kind)."""
 
@@ -119,7 +129,6 @@ class GpuCompressor:
         self.capacity = int(self.lib.skml_payload_capacity(self.n_max, self.dim if self.dense_possible else 0, bin_num,
                                                            group_num, row_num, self.col_ratio))
         self._checked: Optional[_Checked] = None
-        self._local_args = None      # argument block of compress_local, kept between calls
 
     def reset(self) -> None:
         """Clears barrier words, counters and publication marks (needed only after a kernel reported an error)."""
@@ -177,10 +186,10 @@ class GpuCompressor:
         if self.fused:   # one launch that also clears the slot; its end and its status come through a host word
             buf = out if out is not None else torch.empty(self.capacity, dtype=torch.uint8, device=self.device)
             ptr = buf.data_ptr()
-            a = self._local_args
+            a = self._kept_args
             if a is None or given is not None or a.n_given or a.rank != rank or a.world != world:
                 ptrs = [None] * world
-                a = self._local_args = self._args(keys, vals, None, step, rank, world, ptr, buf.numel(), ptrs, ptrs, ck.status,
+                a = self._kept_args = self._args(keys, vals, None, step, rank, world, ptr, buf.numel(), ptrs, ptrs, ck.status,
                                                   None, given)
                 a.done_word = ck.word.data_ptr()
             a.keys, a.vals, a.step, a.seed = L.ptr(keys), vals.data_ptr(), step, self.seed
@@ -222,7 +231,7 @@ class GpuCompressor:
         return buf[:total].cpu().numpy().tobytes()
 
 
-class GpuDecoder:
+class GpuDecoder(_KeepsArgs):
     """Owns the scratch memory of the fused decode + aggregate + update kernel."""
 
     def __init__(self, dim: int, key_capacity: int, device="cuda", fused: bool = True, grid: int = 0,
@@ -243,7 +252,6 @@ class GpuDecoder:
         self.table_capacity = int(table_capacity) if table_capacity > 0 else 2 * self.key_capacity + 4096
         self.table_scratch = torch.zeros(self.table_capacity, dtype=torch.uint8, device=self.device)
         self._checked: Optional[_Checked] = None
-        self._sum_args = None        # argument block of decode_sum, kept between calls
         self.norm_track = None  # (sum of w^2, where lambda * ||w|| goes, lambda): see track_norm
 
     def track_norm(self, sumsq: torch.Tensor, reg_out: torch.Tensor, lam: float) -> None:
@@ -303,9 +311,9 @@ class GpuDecoder:
         ptrs, flags = [p.data_ptr() for p in payloads], [None] * len(payloads)
         if self.fused:
             out = torch.empty(self.dim, dtype=torch.float32, device=self.device)
-            a = self._sum_args
+            a = self._kept_args
             if a is None or a.world != len(ptrs):
-                a = self._sum_args = self.make_args(ptrs, flags, cap, step, ck.status, out_sum=out)
+                a = self._kept_args = self.make_args(ptrs, flags, cap, step, ck.status, out_sum=out)
                 a.done_word = ck.word.data_ptr()
             for r, p in enumerate(ptrs):
                 a.payload[r] = p

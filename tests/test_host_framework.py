@@ -420,3 +420,40 @@ def test_pinned_words_of_ended_threads_are_free_again(monkeypatch):
     th.start()
     th.join(5.0)
     assert not th.is_alive() and len(codec.DoneWords._free) == 4
+
+
+def test_settings_of_a_codec_object_count_from_the_call_after_they_change(monkeypatch):
+    """`compress_local` and `decode_sum` keep their argument block between calls: what the launch is given follows the
+    object's attributes all the same (a stand-in records it)."""
+    import ctypes
+    from collections import deque
+    from types import SimpleNamespace
+    from sketchml_b200.ops import codec
+    monkeypatch.setattr(codec.DoneWords, "_page", torch.zeros(8 * 4, dtype=torch.int64))
+    monkeypatch.setattr(codec.DoneWords, "_free", deque(range(4)))
+    monkeypatch.setattr(codec.L, "stream", lambda: 0)
+    seen = []
+
+    def launch(ref, out, stream):
+        seen.append({n: getattr(ref._obj, n) for n, _ in ref._obj._fields_})
+        return 0
+
+    comp, dec = codec.GpuCompressor(1000, 100, device="cpu"), codec.GpuDecoder(1000, 100, device="cpu")
+    keys, vals = torch.arange(50, dtype=torch.int32), torch.ones(50)
+    comp.lib = dec.lib = SimpleNamespace(skml_compress_checked=launch, skml_decode_sum_checked=launch)
+    buf = comp.compress_local(keys, vals)
+    comp.compress_local(keys, vals, given=(torch.zeros(3), -1.0, 1.0))
+    comp.budget_s, comp.grid, comp.key_encoder, comp.quantile_summary, comp.col_ratio, comp.seed = 0.5, 6, 1, 1, 0.25, 9
+    comp.compress_local(keys, vals)
+    first, given, second = seen
+    assert (first["budget_cycles"], first["grid"], first["key_encoder"], first["quantile_summary"], first["col_ratio"], first["seed"]) == (
+        codec.L.budget_cycles(1.0), 0, 0, 0, 0.3, 0)
+    assert given["n_given"] == 3 and second["n_given"] == 0 and not second["given_splits"]
+    assert (second["budget_cycles"], second["grid"], second["key_encoder"], second["quantile_summary"], second["col_ratio"],
+            second["seed"]) == (codec.L.budget_cycles(0.5), 6, 1, 1, 0.25, 9)
+    seen.clear()
+    dec.decode_sum([buf])
+    dec.budget_s, dec.grid, dec.max_groups = 0.5, 6, 16
+    dec.decode_sum([buf])
+    assert [(s["budget_cycles"], s["grid"], s["max_groups"]) for s in seen] == [
+        (codec.L.budget_cycles(1.0), 0, 32), (codec.L.budget_cycles(0.5), 6, 16)]
