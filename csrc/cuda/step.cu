@@ -33,7 +33,6 @@ static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* met
         if (rc) return rc;
         rc = skml_update_sparse(a->w, c.adam_m, c.adam_v, keys, vals, meta, a->n_max, 1.f, c.adam_v != nullptr, (float)a->lr,
                                 (float)a->adam_scale, (int)c.adam_stride, a->status, stream);
-        if (!rc && batch_keys) rc = batch_consumed(a, (cudaStream_t)stream);
         if (rc) return rc;
         return (int)cudaMemcpyAsync(a->loss_out, a->partials, 4 * sizeof(double), cudaMemcpyDeviceToDevice, (cudaStream_t)stream);
     }
@@ -84,6 +83,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         return apply_gradient(a, a->t_ucols, a->t_meta, a->gvals, nullptr, false, stream_);
     }
     if (a->l_ucols) {
+        if (a->coded) return (int)cudaErrorInvalidValue;   // the sketch arm's alone
         const cudaError_t e = cudaMemcpyAsync(a->partials, a->partials_template, 4 * sizeof(double), cudaMemcpyDeviceToDevice, stream);
         if (e != cudaSuccess) return (int)e;
         // local-id batch: compact weights in, scatter into the compact accumulator, values out in key order

@@ -338,7 +338,10 @@ class GpuEngine:
         csr = csr or self.csr
         rows = self.batch_rows if batch_rows is None else batch_rows
         segs = self._segments(rows) if segments is None else segments
-        if self._fast_ok() and len(segs) <= 2:
+        one_call = self._fast_ok() and len(segs) <= 2
+        if getattr(csr, "lid", None) is not None and not (one_call and self.mode == "sketch"):
+            raise NotImplementedError("local-id batches need the fused sketch engine's single-call step")
+        if one_call:
             if rows != self._template_rows:
                 self.partials_template[0] = float(rows)
                 self._template_rows = rows
@@ -347,8 +350,6 @@ class GpuEngine:
             self.deferred_release = done_event is not None
             m.optimizer.advance()
             return _BatchHandle(rows, self.batch_index), None, None
-        if getattr(csr, "lid", None) is not None:
-            raise NotImplementedError("local-id batches need the fused sketch engine's single-call step")
         if rows != self._template_rows:
             self.partials_template[0] = float(rows)
             self._template_rows = rows

@@ -457,3 +457,24 @@ def test_settings_of_a_codec_object_count_from_the_call_after_they_change(monkey
     dec.decode_sum([buf])
     assert [(s["budget_cycles"], s["grid"], s["max_groups"]) for s in seen] == [
         (codec.L.budget_cycles(1.0), 0, 32), (codec.L.budget_cycles(0.5), 6, 16)]
+
+
+@pytest.mark.parametrize("mode,extras,taken", [("sketch", {}, True), ("sketch", {"single_call_step": False}, False),
+                                               ("nccl_kv", {}, False), ("nccl_dense", {}, False)])
+def test_local_id_batches_are_the_sketch_engine_s_alone(mode, extras, taken):
+    """The baselines' single-call step does not take batches of local column ids, as their separate calls never did."""
+    from types import SimpleNamespace
+    from sketchml_b200.engine_gpu import GpuEngine
+    eng = GpuEngine.__new__(GpuEngine)
+    model = SimpleNamespace(optimizer=SimpleNamespace(advance=lambda: None), loss=SimpleNamespace(is_l2_reg=False))
+    eng.t = SimpleNamespace(comm=SimpleNamespace(world=1), injector=None, model=model)
+    eng.conf, eng.mode, eng.st, eng.depth = SimpleNamespace(extras=extras, batch_num=1), mode, None, 0
+    eng.reg_every_step, eng.batch_index, eng._template_rows = False, 0, 10
+    csr = SimpleNamespace(lid=(None, 5, 0))
+    call = lambda: eng.compute_gradient(csr=csr, segments=[(0, 10)], batch_rows=10)
+    if taken:
+        call()
+        assert eng._pending[0] is csr
+    else:
+        with pytest.raises(NotImplementedError):
+            call()
