@@ -171,9 +171,9 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int) -> Optional[DenseIndex]:
     a.rows, a.dim = rows, dim
     a.row_tiles, a.tile_rows = _tiles(rows, TILE_ROWS_MAX)
     a.col_tiles, a.tile_cols = _tiles(dim, TILE_ROWS_MAX)
-    if nnz < a.row_tiles * dim or 3 * nnz <= 2 * dim or a.row_tiles * dim >= 2 ** 31 - 64:
-        return None
-    margins = nnz >= 6 * rows * a.col_tiles and a.col_tiles <= 256 and a.col_tiles * rows < 2 ** 31 - 64
+    if nnz < a.row_tiles * dim or 3 * nnz <= 2 * dim or max(a.row_tiles * dim, a.col_tiles * rows) >= 2 ** 31 - 64:
+        return None   # (lists are numbered in 32 bits)
+    margins = nnz >= 6 * rows * a.col_tiles and a.col_tiles <= 256
     cnt_c = torch.zeros(a.row_tiles * dim, dtype=torch.int32, device=dev)
     cnt_r = torch.empty(a.col_tiles * rows, dtype=torch.int32, device=dev) if margins else None
     L.check(lib.skml_dt_count(C.byref(a), L.ptr(csr.rowptr), L.ptr(csr.cols), lo, L.ptr(cnt_c), L.ptr(cnt_r), L.stream()), "skml_dt_count")

@@ -478,3 +478,19 @@ def test_local_id_batches_are_the_sketch_engine_s_alone(mode, extras, taken):
     else:
         with pytest.raises(NotImplementedError):
             call()
+
+
+def test_a_batch_with_more_lists_than_32_bits_count_has_no_tiled_index(monkeypatch):
+    """Row lists are counted in 32 bits whether or not the margins use them: such a batch keeps the scatter path."""
+    from types import SimpleNamespace
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T.L, "stream", lambda: 0)
+
+    class RowPtr(torch.Tensor):
+        def __getitem__(self, i):
+            return i        # one entry a row
+
+    rows = 2 ** 31 - 32     # one tile of 100 columns: the sizes are refused before anything is read
+    csr = SimpleNamespace(cols=torch.zeros(0, dtype=torch.int32), values=None, rowptr=torch.zeros(1, dtype=torch.int64).as_subclass(RowPtr),
+                          dim=100)
+    assert T.build_dense_index(csr, 0, rows) is None
