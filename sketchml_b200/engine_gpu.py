@@ -214,12 +214,10 @@ class GpuEngine:
         idx = []
         torch.cuda.synchronize(self.device)
         t0 = time.perf_counter()
-        # near-dense batches: two tiled copies of the entries, lists padded to four entries, and their bounds
-        need = (csr.nnz * (12 if csr.values is not None else 4) * 1.5 + 16 * csr.dim * (B // 49152 + 1) +
-                16 * B * (csr.dim // 49152 + 1))
-        dense = self.st.dense_vals is not None and need <= 0.8 * free
+        # near-dense batches: two tiled copies of the entries, as far as there is room for every batch's
+        dense = self.st.dense_vals is not None
         for b in range(csr.rows // B if dense else 0):
-            di = build_dense_index(csr, b * B, (b + 1) * B)
+            di = build_dense_index(csr, b * B, (b + 1) * B, int(0.8 * free) - sum(x.nbytes() for x in idx))
             if di is None:
                 if b:
                     return

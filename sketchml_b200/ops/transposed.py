@@ -159,11 +159,12 @@ def _tiles(n: int, tile_max: int):
     return tiles, ((-(-n // tiles)) + 7) // 8 * 8
 
 
-def build_dense_index(csr: DeviceCSR, lo: int, hi: int) -> Optional[DenseIndex]:
+def build_dense_index(csr: DeviceCSR, lo: int, hi: int, budget: Optional[int] = None) -> Optional[DenseIndex]:
     """None where the batch touches no more than two thirds of the columns, or where the lists would be too short to be
     worth it (fewer than one entry per row tile and column): partial sums and list bounds then cost more than the
     scatter's atomics. The margins take the tiled form from six entries per
-    row and column tile on; below, the padding and the partial sums cost more than gathers of w."""
+    row and column tile on; below, the padding and the partial sums cost more than gathers of w.
+    None too where building it, or the index and its scratch afterwards, would take more than ``budget`` bytes."""
     dev, lib, rows, dim = csr.cols.device, L.lib(), hi - lo, csr.dim
     e0, e1 = int(csr.rowptr[lo]), int(csr.rowptr[hi])
     nnz = e1 - e0
@@ -174,6 +175,11 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int) -> Optional[DenseIndex]:
     if nnz < a.row_tiles * dim or 3 * nnz <= 2 * dim or max(a.row_tiles * dim, a.col_tiles * rows) >= 2 ** 31 - 64:
         return None   # (lists are numbered in 32 bits)
     margins = nnz >= 6 * rows * a.col_tiles and a.col_tiles <= 256
+    # counts and bounds of all lists, the sums in between, the partial sums of a step (the entries are added below)
+    n_lists = (a.row_tiles * dim, a.col_tiles * rows if margins else 0)
+    room = 8 * sum(n_lists) + 12 * max(n_lists) + 24 * dim
+    if budget is not None and room > budget:
+        return None
     cnt_c = torch.zeros(a.row_tiles * dim, dtype=torch.int32, device=dev)
     cnt_r = torch.empty(a.col_tiles * rows, dtype=torch.int32, device=dev) if margins else None
     L.check(lib.skml_dt_count(C.byref(a), L.ptr(csr.rowptr), L.ptr(csr.cols), lo, L.ptr(cnt_c), L.ptr(cnt_r), L.stream()), "skml_dt_count")
@@ -183,23 +189,28 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int) -> Optional[DenseIndex]:
     if int(any_c.sum()) <= dim * 2 // 3:
         return None
 
-    def lists(cnt, pad):
-        quads = (cnt + 3) >> 2
+    def bounds(cnt):
         ptr = torch.zeros(cnt.numel() + 1, dtype=torch.int32, device=dev)
-        torch.cumsum(quads, 0, dtype=torch.int32, out=ptr[1:])
-        n = -(-4 * int(ptr[-1]) // 2 ** 20) * 2 ** 20   # whole megabytes: batches of one data set get buffers of one size
+        torch.cumsum((cnt + 3) >> 2, 0, dtype=torch.int32, out=ptr[1:])
+        return ptr, -(-4 * int(ptr[-1]) // 2 ** 20) * 2 ** 20   # whole megabytes: batches of one data set get buffers of one size
+
+    def entries(n, pad):
         loc = torch.full((n,), pad if pad < 32768 else pad - 65536, dtype=torch.int16, device=dev)   # unsigned 16-bit patterns
-        val = None if csr.values is None else torch.zeros(n, dtype=torch.float32, device=dev)
-        return ptr, loc, val
+        return loc, None if csr.values is None else torch.zeros(n, dtype=torch.float32, device=dev)
+
+    c_ptr, n_c = bounds(cnt_c)
+    r_ptr, n_r = bounds(cnt_r) if margins else (None, 0)
+    if budget is not None and room + (n_c + n_r) * (2 if csr.values is None else 6) > budget:
+        return None
 
     weights = (1 << torch.arange(32, device=dev, dtype=torch.int64))
     words = (any_c.view(-1, 32) * weights).sum(1)
     touched = torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32)
-    c_ptr, c_loc, c_val = lists(cnt_c, int(a.tile_rows))
+    c_loc, c_val = entries(n_c, int(a.tile_rows))
     tensors = [c_ptr, c_loc, touched] + ([c_val] if c_val is not None else [])
     a.c_ptr, a.c_loc, a.c_val, a.touched = L.ptr(c_ptr), L.ptr(c_loc), L.ptr(c_val), L.ptr(touched)
     if margins:
-        r_ptr, r_loc, r_val = lists(cnt_r, int(a.tile_cols))
+        r_loc, r_val = entries(n_r, int(a.tile_cols))
         tensors += [r_ptr, r_loc] + ([r_val] if r_val is not None else [])
         a.r_ptr, a.r_loc, a.r_val = L.ptr(r_ptr), L.ptr(r_loc), L.ptr(r_val)
     cursor = cnt_c.zero_()

@@ -399,3 +399,59 @@ def test_scatter_gradient_is_exact_on_whole_numbers(rows, nnz, dim, hot, binary)
     assert torch.equal(st.keys[:n].cpu().long(), torch.nonzero(want).flatten())
     assert torch.equal(st.vals[:n].cpu().double(), want[want != 0])
     assert float(st.g.abs().max()) == 0.0 and int(st.bitmap.abs().max()) == 0 and int(st.status.item()) == 0
+
+
+@pytest.mark.parametrize("binary", [True, False])
+@pytest.mark.parametrize("rows,dim,nnz", [(20000, 200000, 12), (3001, 20003, 90)])
+def test_near_dense_index_stays_within_its_budget(rows, dim, nnz, binary):
+    """Building it takes no more memory than it was allowed, scratch of a step included; where that is not enough there
+    is no index. Lists of one entry, which padding makes four times as long, and lists for the margins too."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.ops import DeviceCSR
+    from sketchml_b200.ops import transposed as T
+    dev = torch.device("cuda")
+    gen = torch.Generator().manual_seed(rows)
+    cols = torch.randint(0, dim, (rows * nnz,), generator=gen).int()
+    m = CSRMatrix(torch.arange(rows + 1) * nnz, cols, None if binary else torch.randn(rows * nnz, generator=gen), torch.ones(rows), dim)
+    csr = DeviceCSR(m, dev)
+
+    def build(budget):
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        di = T.build_dense_index(csr, 0, rows, budget)
+        scratch = None if di is None else torch.empty(di.partial_floats, device=dev)
+        torch.cuda.synchronize()
+        del scratch
+        return di, torch.cuda.max_memory_allocated() - before
+
+    di, peak = build(None)
+    assert di is not None and di.nbytes() <= peak
+    used = di.nbytes()
+    del di
+    lo, hi = used // 2, 4 * peak
+    while hi - lo > 65536:       # the smallest budget that is enough: what was allowed is never exceeded on the way
+        mid = (lo + hi) // 2
+        di, peak = build(mid)
+        assert peak <= mid + 65536        # (the allocator rounds small tensors up)
+        lo, hi = (lo, mid) if di is not None else (mid, hi)
+        del di
+    assert hi <= 4 * used
+
+
+def test_near_dense_shard_without_room_for_the_index_trains_with_the_scatter(monkeypatch):
+    """Ten binary batches whose lists hold one or two entries, which padding makes four: the index of all batches does
+    not fit what is free, so there is none, and the steps take the scatter path."""
+    from sketchml_b200.config import MLConf
+    from sketchml_b200.trainer import Trainer
+    free = 25_000_000
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a, **k: (free, free))
+    t = Trainer(MLConf(algo="linreg", format="synthetic", feature_num=200_000, syn_rows=200_000, syn_nnz_per_row=12, syn_zipf_s=0.0,
+                       syn_values="binary", valid_ratio=0.0, epoch_num=1, batch_sample_ratio=0.1, learn_rate=0.05, device="cuda"))
+    t.load_data()
+    assert t.engine.tindex is None or t.engine.index_bytes <= 0.8 * free
+    w = t.model.weights.clone()
+    t.train_one_iteration(0, 0)
+    t.engine.check()
+    assert not torch.equal(w, t.model.weights)
+    t.close()
