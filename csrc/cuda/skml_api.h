@@ -145,8 +145,8 @@ int skml_colsum_tiled(const int* tile_pair_ptr, const int* pair_ptr, const unsig
 // Tiled copies of the entries of a batch whose gradient is near dense (csrc/cuda/tiled_kernels.cu): per (row tile,
 // column) list c_ptr (in quads of four entries, row_tiles * dim + 1 of them), the tile-local rows c_loc and values
 // c_val (null: all one) in that order, padded with c_loc = tile_rows, c_val = 0; the same per (column tile, row) in
-// r_* with tile-local columns (r_ptr null: margins are taken from the CSR rows). `touched`: one bit per column with
-// an entry. `partial`: scratch of max(row_tiles * dim, col_tiles * rows) floats; `coef`: one float per row.
+// r_* with tile-local columns (r_ptr null: margins are taken from the CSR rows). `partial`: scratch
+// of max(row_tiles * dim, col_tiles * rows) floats; `coef`: one float per row.
 #define SKML_DT_TILE_MAX 49152   // floats of a vector tile in shared memory (192 KB)
 typedef struct SkmlDenseIndex {
     long long rows, dim, row_tiles, tile_rows, col_tiles, tile_cols;
@@ -156,7 +156,6 @@ typedef struct SkmlDenseIndex {
     const int* r_ptr;
     unsigned short* r_loc;
     float* r_val;
-    const unsigned int* touched;
     float* partial;
     float* coef;
 } SkmlDenseIndex;

@@ -316,16 +316,61 @@ dt_coef_kernel(const float* __restrict__ partial, int rows, int tiles, const flo
     if (threadIdx.x == 0 && total != 0.0) atomicAdd(acc, total);
 }
 
-// Column sums from their partial sums into the (cleared) accumulator, and the columns that the batch touches.
+// Whether this lane's list of a group of 32 holds an x that is not zero (asked by lanes with `mine`; the whole warp).
+__device__ __noinline__ bool holds_nonzero(const float* __restrict__ x, int T, const ushort4* __restrict__ loc, int q0, int len, bool mine) {
+    const int lane = threadIdx.x & 31, most = __reduce_max_sync(0xFFFFFFFFu, len);
+    auto nonzero = [&](int q) {
+        const ushort4 l = __ldg(loc + q);
+        return (l.x != T && x[l.x] != 0.f) || (l.y != T && x[l.y] != 0.f) || (l.z != T && x[l.z] != 0.f) || (l.w != T && x[l.w] != 0.f);
+    };
+    bool some = false;
+    if (most <= DT_LONG) {   // interleaved
+        int at = __shfl_sync(0xFFFFFFFFu, q0, 0);
+        for (int k = 0; k < most; ++k) {
+            const unsigned int have = __ballot_sync(0xFFFFFFFFu, len > k);
+            if (mine && len > k && !some) some = nonzero(at + __popc(have & ((1u << lane) - 1u)));
+            at += __popc(have);
+        }
+    } else {
+        for (unsigned int left = __ballot_sync(0xFFFFFFFFu, mine); left; left &= left - 1) {   // one list after another
+            const int src = __ffs(left) - 1;
+            const int s0 = __shfl_sync(0xFFFFFFFFu, q0, src), n = __shfl_sync(0xFFFFFFFFu, len, src);
+            bool any = false;
+            for (int k = lane; k - lane < n && !any; k += 32) any = __any_sync(0xFFFFFFFFu, k < n && nonzero(s0 + k));
+            if (lane == src) some = any;
+        }
+    }
+    return some;
+}
+
+// Column sums from their partial sums into the (cleared) accumulator, and the columns that the batch touches: those with
+// an entry in a row whose coefficient is not zero, as in the scatter (rows outside the hinge have none, and a logistic
+// slope may underflow). A partial sum other than zero says so; where all are zero the column's lists are looked through.
 __global__ void __launch_bounds__(256)
-dt_sum_kernel(const float* __restrict__ partial, int dim, int tiles, const unsigned int* __restrict__ touched, float* __restrict__ g,
-              unsigned int* __restrict__ bitmap) {
-    for (int c = blockIdx.x * 256 + threadIdx.x; c < dim; c += gridDim.x * 256) {
+dt_sum_kernel(const float* __restrict__ partial, int dim, int tiles, int T, const int* __restrict__ ptr, const ushort4* __restrict__ loc,
+              const float* __restrict__ coef, float* __restrict__ g, unsigned int* __restrict__ bitmap) {
+    const int lane = threadIdx.x & 31;
+    for (int c = blockIdx.x * 256 + threadIdx.x; c - lane < dim; c += gridDim.x * 256) {   // a warp a word of 32 columns
+        const bool in = c < dim;
+        const float* const src = partial + (in ? c : dim - 1);
         float v = 0.f;
+        unsigned int bits = 0;
 #pragma unroll 8
-        for (int t = 0; t < tiles; ++t) v += partial[(long long)t * dim + c];
-        g[c] = v;
-        if ((c & 31) == 0) bitmap[c >> 5] = touched[c >> 5];
+        for (int t = 0; t < tiles; ++t) {
+            const float x = src[(long long)t * dim];
+            bits |= __float_as_uint(x);
+            v += x;
+        }
+        if (in) g[c] = v;
+        bool touched = in && (bits << 1) != 0u;
+        for (int t = 0; t < tiles && !__all_sync(0xFFFFFFFFu, touched || !in); ++t) {
+            const long long p = (long long)t * dim + c;
+            const int q0 = in ? ptr[p] : 0, len = in ? ptr[p + 1] - q0 : 0;
+            const bool mine = !touched && len > 0;
+            if (__any_sync(0xFFFFFFFFu, mine)) touched |= holds_nonzero(coef + (long long)t * T, T, loc, q0, len, mine);
+        }
+        const unsigned int m = __ballot_sync(0xFFFFFFFFu, touched);
+        if (lane == 0) bitmap[c >> 5] = m;
     }
 }
 
@@ -403,7 +448,7 @@ extern "C" int skml_dt_fill(const SkmlDenseIndex* d, const long long* rowptr, co
 extern "C" int skml_dt_gradient(const SkmlDenseIndex* d, const long long* rowptr, const int* cols, const float* vals, const float* labels,
                                 long long row_lo, long long nnz_padded, double avg_nnz, const float* w, int loss_id, float inv_batch,
                                 double* loss_acc, float* g, unsigned int* bitmap, unsigned int* status, long long budget, void* stream_) {
-    if (!dt_valid(d) || !d->c_ptr || !d->partial || !d->coef || !d->touched) return (int)cudaErrorInvalidValue;
+    if (!dt_valid(d) || !d->c_ptr || !d->partial || !d->coef) return (int)cudaErrorInvalidValue;
     cudaStream_t stream = (cudaStream_t)stream_;
     int rc;
     if (d->r_ptr) {
@@ -419,6 +464,7 @@ extern "C" int skml_dt_gradient(const SkmlDenseIndex* d, const long long* rowptr
     if (rc) return rc;
     rc = dt_partial(d->coef, d->rows, (int)d->tile_rows, (int)d->row_tiles, (int)d->dim, d->c_ptr, d->c_loc, d->c_val, d->partial, stream);
     if (rc) return rc;
-    dt_sum_kernel<<<blocks_for(d->dim, 256, 8), 256, 0, stream>>>(d->partial, (int)d->dim, (int)d->row_tiles, d->touched, g, bitmap);
+    dt_sum_kernel<<<blocks_for(d->dim, 256, 8), 256, 0, stream>>>(d->partial, (int)d->dim, (int)d->row_tiles, (int)d->tile_rows, d->c_ptr,
+                                                                  reinterpret_cast<const ushort4*>(d->c_loc), d->coef, g, bitmap);
     return (int)cudaGetLastError();
 }

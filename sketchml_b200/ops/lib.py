@@ -60,7 +60,7 @@ class DenseIndexArgs(C.Structure):
     _fields_ = [
         ("rows", c_ll), ("dim", c_ll), ("row_tiles", c_ll), ("tile_rows", c_ll), ("col_tiles", c_ll), ("tile_cols", c_ll),
         ("c_ptr", c_vp), ("c_loc", c_vp), ("c_val", c_vp), ("r_ptr", c_vp), ("r_loc", c_vp), ("r_val", c_vp),
-        ("touched", c_vp), ("partial", c_vp), ("coef", c_vp),
+        ("partial", c_vp), ("coef", c_vp),
     ]
 
 

@@ -177,16 +177,15 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int, budget: Optional[int] = 
     margins = nnz >= 6 * rows * a.col_tiles and a.col_tiles <= 256
     # counts and bounds of all lists, the sums in between, the partial sums of a step (the entries are added below)
     n_lists = (a.row_tiles * dim, a.col_tiles * rows if margins else 0)
-    room = 8 * sum(n_lists) + 12 * max(n_lists) + 24 * dim
+    room = 8 * sum(n_lists) + 12 * max(n_lists) + 8 * dim
     if budget is not None and room > budget:
         return None
     cnt_c = torch.zeros(a.row_tiles * dim, dtype=torch.int32, device=dev)
     cnt_r = torch.empty(a.col_tiles * rows, dtype=torch.int32, device=dev) if margins else None
     L.check(lib.skml_dt_count(C.byref(a), L.ptr(csr.rowptr), L.ptr(csr.cols), lo, L.ptr(cnt_c), L.ptr(cnt_r), L.stream()), "skml_dt_count")
 
-    any_c = torch.zeros((dim + 31) // 32 * 32, dtype=torch.bool, device=dev)
-    any_c[:dim] = cnt_c.view(a.row_tiles, dim).amax(0) > 0 if a.row_tiles > 1 else cnt_c > 0
-    if int(any_c.sum()) <= dim * 2 // 3:
+    any_c = cnt_c.view(a.row_tiles, dim).amax(0) if a.row_tiles > 1 else cnt_c
+    if int(torch.count_nonzero(any_c)) <= dim * 2 // 3:
         return None
 
     def bounds(cnt):
@@ -203,12 +202,9 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int, budget: Optional[int] = 
     if budget is not None and room + (n_c + n_r) * (2 if csr.values is None else 6) > budget:
         return None
 
-    weights = (1 << torch.arange(32, device=dev, dtype=torch.int64))
-    words = (any_c.view(-1, 32) * weights).sum(1)
-    touched = torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32)
     c_loc, c_val = entries(n_c, int(a.tile_rows))
-    tensors = [c_ptr, c_loc, touched] + ([c_val] if c_val is not None else [])
-    a.c_ptr, a.c_loc, a.c_val, a.touched = L.ptr(c_ptr), L.ptr(c_loc), L.ptr(c_val), L.ptr(touched)
+    tensors = [c_ptr, c_loc] + ([c_val] if c_val is not None else [])
+    a.c_ptr, a.c_loc, a.c_val = L.ptr(c_ptr), L.ptr(c_loc), L.ptr(c_val)
     if margins:
         r_loc, r_val = entries(n_r, int(a.tile_cols))
         tensors += [r_ptr, r_loc] + ([r_val] if r_val is not None else [])
@@ -216,7 +212,7 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int, budget: Optional[int] = 
     cursor = cnt_c.zero_()
     L.check(lib.skml_dt_fill(C.byref(a), L.ptr(csr.rowptr), L.ptr(csr.cols), L.ptr(csr.values), lo, nnz, L.ptr(cursor), L.stream()),
             "skml_dt_fill")
-    return DenseIndex(lo, rows, a, tensors, int(max(a.row_tiles * dim, a.col_tiles * rows if margins else 0)))
+    return DenseIndex(lo, rows, a, tensors, int(max(n_lists)))
 
 
 def glm_grad_dense(csr: DeviceCSR, di: DenseIndex, w: torch.Tensor, g: torch.Tensor, bitmap: torch.Tensor, partials: torch.Tensor,

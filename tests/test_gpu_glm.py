@@ -455,3 +455,52 @@ def test_near_dense_shard_without_room_for_the_index_trains_with_the_scatter(mon
     t.engine.check()
     assert not torch.equal(w, t.model.weights)
     t.close()
+
+
+@pytest.mark.parametrize("loss_name,scale", [("hinge", 1.0), ("log", 60.0)])
+@pytest.mark.parametrize("rows,dim,nnz,tile", [(2000, 5000, (20, 90), 49152), (2000, 5000, (20, 90), 256), (50000, 700, (10, 30), 49152),
+                                               (3001, 1003, (60, 200), 1000)])
+@pytest.mark.parametrize("binary", [True, False])
+def test_near_dense_index_touches_the_columns_the_scatter_touches(rows, dim, nnz, tile, binary, loss_name, scale, monkeypatch):
+    """Rows without a coefficient (outside the hinge, or a logistic slope that underflows) touch no column: the same
+    touched bits, count and kind as the scatter's, also where a column's sum cancels. Whole-numbered weights and values
+    make every margin exact; columns in no list, in short lists and in lists that a warp sums at a time."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.models.loss import L2HingeLoss, L2LogLoss
+    from sketchml_b200.ops import DeviceCSR, GlmState, compact_gradient, glm_grad
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T, "TILE_ROWS_MAX", tile)
+    dev, loss = torch.device("cuda"), (L2HingeLoss if loss_name == "hinge" else L2LogLoss)(1e-3)
+    gen = torch.Generator().manual_seed(rows + dim)
+    cnt = torch.randint(nnz[0], nnz[1] + 1, (rows,), generator=gen)
+    rowptr = torch.zeros(rows + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(cnt, 0)
+    n = int(rowptr[-1])
+    cols = (torch.rand(n, generator=gen) ** (1 if tile == 1000 else 1.3) * dim).int().clamp_max(dim - 1)
+    vals = None if binary else torch.randint(0, 2, (n,), generator=gen).float() * 2 - 1
+    w = (torch.randint(-1, 2, (dim,), generator=gen) * scale).float()
+    rid = torch.repeat_interleave(torch.arange(rows), cnt)
+    pre = torch.zeros(rows, dtype=torch.float64).index_add_(0, rid, (w.double()[cols.long()] * (1.0 if binary else vals.double())))
+    labels = torch.where(pre > 0, 1.0, -1.0)
+    few = torch.randperm(rows, generator=gen)[:max(2, dim // (nnz[0] + nnz[1]))]
+    labels[few] = -labels[few]     # rows on the wrong side: with the ones near the border, those that have a coefficient
+    csr = DeviceCSR(CSRMatrix(rowptr, cols, vals, labels.float(), dim), dev)
+    di = T.build_dense_index(csr, 0, rows)
+    if di is None:
+        assert int(torch.unique(cols).numel()) <= dim * 2 // 3 or n < T._tiles(rows, tile)[0] * dim
+        return
+    wd, got = w.to(dev), []
+    for form in ("index", "scatter"):
+        st = GlmState.create(dim, dim, dev, allow_dense=True)
+        if form == "index":
+            di.bind(torch.empty(di.partial_floats, device=dev), torch.empty(rows, device=dev))
+            T.glm_grad_dense(csr, di, wd, st.g, st.bitmap, st.partials, st.status, loss.loss_id)
+        else:
+            glm_grad(csr, [(0, rows)], wd, st, loss.loss_id, rows, hot=0)
+        bitmap = st.bitmap.clone()
+        compact_gradient(st, wd, loss.lam)
+        got.append((bitmap, int(st.meta[0]), int(st.meta[1])))
+    assert torch.equal(got[0][0], got[1][0])
+    assert 0 < int(torch.count_nonzero(got[0][0])) and got[0][2] == got[1][2]
+    # a value next to the filter's 1e-8 may fall on either side of it: sums of at most n terms in varying order
+    assert abs(got[0][1] - got[1][1]) <= 2
