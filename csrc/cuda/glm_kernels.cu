@@ -795,9 +795,9 @@ __global__ void update_dense_kernel(float* w, float* m, float* v, const float* g
 __global__ void update_sparse_kernel(float* w, float* m, float* v, const int* keys, const float* vals,
                                      const long long* n_ptr, long long n_max, float scale, int adam, float lr,
                                      float adam_scale, long long ms, const unsigned int* status) {
-    if (skml_failed(status)) return;
     long long n = n_ptr ? *n_ptr : n_max;
     if (n > n_max) n = n_max;
+    if (skml_failed(status)) n = 0;   // (read beside the count)
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         apply_update(w, m, v, keys[i], vals[i] * scale, adam, lr, adam_scale, ms);
 }
@@ -888,9 +888,9 @@ extern "C" int skml_weight_norm(const float* w, long long dim, double lambda, do
 __global__ void update_gathered_kernel(float* w, float* m, float* v, float* acc, const int* keys, const long long* count,
                                        long long stride, float scale, int adam, float lr, float adam_scale, long long ms,
                                        const unsigned int* status) {
-    if (skml_failed(status)) return;
     long long n = *count;
     if (n > stride) n = stride;
+    if (skml_failed(status)) n = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const int k = keys[i];
         const float g = acc[k];

@@ -517,12 +517,12 @@ zip_code_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
                 const float* __restrict__ splits, const int* __restrict__ meta, int code_bytes,
                 unsigned char* __restrict__ codes, const unsigned int* __restrict__ status) {
     extern __shared__ float sh_splits[];
-    if (skml_failed(status)) return;
+    long long n = *n_ptr;
+    if (n > n_max) n = n_max;
+    if (skml_failed(status)) n = 0;   // (read beside the counts)
     const int nb = meta[0], ns = nb > 0 ? nb - 1 : 0;
     for (int i = threadIdx.x; i < ns; i += blockDim.x) sh_splits[i] = splits[i];
     __syncthreads();
-    long long n = *n_ptr;
-    if (n > n_max) n = n_max;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float v = vals[i];
         int lo = 0, hi = ns;  // first split > v
@@ -541,11 +541,11 @@ zip_unpack_scatter_kernel(float* __restrict__ acc, const int* __restrict__ keys,
                           const float* __restrict__ mids, const long long* __restrict__ count, long long key_stride,
                           int code_bytes, int table_len, float* __restrict__ vals_out, const unsigned int* __restrict__ status) {
     extern __shared__ float sh_mids[];
-    if (skml_failed(status)) return;
-    for (int i = threadIdx.x; i < table_len; i += blockDim.x) sh_mids[i] = mids[i];
-    __syncthreads();
     long long n = *count;
     if (n > key_stride) n = key_stride;
+    if (skml_failed(status)) n = 0;
+    for (int i = threadIdx.x; i < table_len; i += blockDim.x) sh_mids[i] = mids[i];
+    __syncthreads();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         unsigned int c = code_bytes == 1 ? codes[i] : reinterpret_cast<const unsigned short*>(codes)[i];
         if (c >= (unsigned int)table_len) c = table_len - 1;
