@@ -1185,7 +1185,7 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n, int (&nkey)[2],
             if (G <= 8) group_masks<3>(valid, g, own, of_lane);
             else group_masks<5>(valid, g, own, of_lane);
             const unsigned int base = __shfl_sync(0xFFFFFFFFu, run, g);
-            run += (unsigned int)__popc(of_lane);   // (lanes beyond the last group find nothing)
+            run += (unsigned int)__popc(of_lane);   // (of lanes beyond the last group nobody asks)
             if (!valid) continue;
             p.gkeys[base + (unsigned int)__popc(own & lanemask_lt())] = key[u];
             const unsigned int cell = skml_pack_cell(bin[u], zero);

@@ -635,9 +635,8 @@ __device__ void apply_owned(const DP& p, DecSmem& s, float& dsq) {
     unsigned long long* seg = reinterpret_cast<unsigned long long*>(&s.items[p.max_items]);  // [2 * DEC_OWN_RANGES][max_items]
     __shared__ unsigned long long s_bound[2 * DEC_OWN_RANGES];
     // SGD: one range per block (more ranges even out the blocks but do not shorten the launch: the random
-    // DRAM sectors bound it in total); lazy Adam sweeps a range 2 x ranks times, and smaller ranges keep
-    // its sectors in L2
-    // between the sweeps (where a block has fewer than 2048 keys, the sweeps' latency is what counts)
+    // DRAM sectors bound it in total). Lazy Adam sweeps a range 2 x ranks times, and smaller ranges keep its
+    // sectors in L2 between the sweeps; where a block has fewer than 2048 keys, the sweeps' latency is what counts.
     const int rounds = p.adam_v && s.total_keys >= 2048ull * gridDim.x ? DEC_OWN_RANGES : 1;
     if (threadIdx.x < 2 * rounds) {
         const DecItem& ref = s.items[s.ref_item];

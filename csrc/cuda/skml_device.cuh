@@ -1,7 +1,7 @@
 // Device-side building blocks shared by all sm_100a kernels of this library:
-// status words, bounded waits (grid barrier, flag wait, mbarrier wait), scans,
-// order-preserving float keys, 1-D bulk (TMA) copies into shared memory, and
-// system-scope loads/stores used on peer-mapped memory.
+// status words, bounded waits (grid barrier, flag wait), order-preserving float keys,
+// sorts and searches in shared memory, the end of a checked call, and system-scope
+// loads/stores used on peer-mapped memory.
 //
 // Every wait in this file has a clock64() budget. When it runs out the kernel
 // records a status word and returns normally, so the CUDA context stays usable.
@@ -35,9 +35,6 @@ __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-__device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ unsigned long long ld_acquire_sys(const unsigned long long* p) {
     unsigned long long v;
@@ -174,39 +171,6 @@ __device__ __forceinline__ unsigned int f2ord(float f) {
 }
 __device__ __forceinline__ float ord2f(unsigned int k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
-// ---------------------------------------------------------------------------
-// Block-wide exclusive scan (SKML_BLOCK threads). `total` receives the block sum.
-// ---------------------------------------------------------------------------
-template <class T>
-__device__ __forceinline__ T block_exclusive_scan(T v, T* total) {
-    __shared__ T s_warp[SKML_WARPS];
-    __shared__ T s_total;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        T t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    __syncthreads();  // protects s_warp / s_total against the previous call
-    if (lane == 31) s_warp[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        T w = lane < (int)(blockDim.x >> 5) ? s_warp[lane] : (T)0;
-        T winc = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            T t = __shfl_up_sync(0xFFFFFFFFu, winc, o);
-            if (lane >= o) winc += t;
-        }
-        s_warp[lane] = winc - w;
-        if (lane == 31) s_total = winc;
-    }
-    __syncthreads();
-    if (total) *total = s_total;
-    return s_warp[warp] + inc - v;
 }
 
 template <class T>

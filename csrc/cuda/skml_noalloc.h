@@ -37,8 +37,9 @@
 extern "C" {
 #endif
 
-#define SKML_NOALLOC_MAX_BLOCKS 4096
-#define SKML_NOALLOC_MAX_DIM (4096ll * 4096ll * 32ll) /* blocks x bitmap words per block x bits */
+/* The limit is part of the interface. The built-in array itself serves every dim: warps take longer runs of bitmap words
+   from 16M coordinates on, so there are never more counts than it holds. */
+#define SKML_NOALLOC_MAX_DIM 536870912ll
 #define SKML_NOALLOC_BAD_ARGUMENT (-1)
 #define SKML_NOALLOC_TOO_LARGE (-2)
 
