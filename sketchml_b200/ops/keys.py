@@ -57,11 +57,16 @@ _call = threading.local()
 _workspace_bytes = 0
 
 
-def _call_state() -> _CallState:
+def _workspace(device) -> torch.Tensor:
     global _workspace_bytes
+    if not _workspace_bytes:
+        _workspace_bytes = int(L.lib().skml_da_workspace_bytes())
+    return torch.empty(_workspace_bytes, dtype=torch.uint8, device=device)
+
+
+def _call_state() -> _CallState:
     state: Optional[_CallState] = getattr(_call, "state", None)
     if state is None:
-        _workspace_bytes = int(L.lib().skml_da_workspace_bytes())
         state = _call.state = _CallState()
     return state
 
@@ -73,7 +78,7 @@ def encode(keys: torch.Tensor) -> AdaptiveKeys:
     keys = keys.contiguous()
     n, dev, lib, cs = keys.numel(), keys.device, L.lib(), _call_state()
     stream = L.stream()
-    work = torch.empty(_workspace_bytes, dtype=torch.uint8, device=dev)
+    work = _workspace(dev)
     L.check(lib.skml_da_plan(keys.data_ptr(), n, work.data_ptr(), cs.words.data_ptr(), cs.status_ref, stream), "skml_da_plan")
     if cs.status.value & 1:
         raise ValueError("keys must be non-negative and strictly increasing")
@@ -91,10 +96,9 @@ def decode(e: AdaptiveKeys) -> torch.Tensor:
     dev, lib, n = e.delta_words.device, L.lib(), e.size
     if n == 0:
         return torch.zeros(0, dtype=torch.int32, device=dev)
-    _call_state()
     fw, dw = e.flag_words.to(torch.int64).contiguous(), e.delta_words.to(torch.int64).contiguous()
     keys = torch.empty(n, dtype=torch.int32, device=dev)
-    work = torch.empty(_workspace_bytes, dtype=torch.uint8, device=dev)
+    work = _workspace(dev)
     pos = torch.empty(n, dtype=torch.int64, device=dev) if e.flag_kind else None
     L.check(lib.skml_da_decode(fw.data_ptr(), fw.numel(), dw.data_ptr(), dw.numel(), n, e.num_intervals, e.flag_kind, e.flag_bits,
                                work.data_ptr(), L.ptr(pos), keys.data_ptr(), L.stream()), "skml_da_decode")

@@ -494,3 +494,18 @@ def test_a_batch_with_more_lists_than_32_bits_count_has_no_tiled_index(monkeypat
     csr = SimpleNamespace(cols=torch.zeros(0, dtype=torch.int32), values=None, rowptr=torch.zeros(1, dtype=torch.int64).as_subclass(RowPtr),
                           dim=100)
     assert T.build_dense_index(csr, 0, rows) is None
+
+
+def test_decoding_keys_pins_no_memory(monkeypatch):
+    """Nothing of a decode comes back through host memory: it allocates none, which a stream that is being captured
+    would not allow (the first allocation pins a page)."""
+    from types import SimpleNamespace
+    from sketchml_b200.ops import codec, keys
+    lib = SimpleNamespace(skml_da_workspace_bytes=lambda: 64, skml_da_decode=lambda *a: 0)
+    monkeypatch.setattr(keys, "_workspace_bytes", 0)
+    monkeypatch.setattr(keys.L, "lib", lambda: lib)
+    monkeypatch.setattr(keys.L, "stream", lambda: 0)
+    monkeypatch.setattr(codec.DoneWords, "take", lambda owner: pytest.fail("a pinned word was taken"))
+    words = torch.zeros(4, dtype=torch.int64)
+    for kind in (0, 1):
+        assert keys.decode(keys.AdaptiveKeys(10, 4, kind, 20, 80, words, words)).numel() == 10
