@@ -148,6 +148,7 @@ int skml_colsum_tiled(const int* tile_pair_ptr, const int* pair_ptr, const unsig
 // r_* with tile-local columns (r_ptr null: margins are taken from the CSR rows). `partial`: scratch
 // of max(row_tiles * dim, col_tiles * rows) floats; `coef`: one float per row.
 #define SKML_DT_TILE_MAX 49152   // floats of a vector tile in shared memory (192 KB)
+#define SKML_DT_LISTS_MAX ((1ll << 31) - (1ll << 20))   // lists of either kind: 32-bit counters step past the last by a grid at most
 typedef struct SkmlDenseIndex {
     long long rows, dim, row_tiles, tile_rows, col_tiles, tile_cols;
     const int* c_ptr;

@@ -411,7 +411,7 @@ int dt_partial(const float* x, long long n, int T, int tiles, int items, const i
 bool dt_valid(const SkmlDenseIndex* d) {
     return d && d->rows > 0 && d->dim > 0 && d->rows < (1ll << 31) && d->dim < (1ll << 31) && d->tile_rows > 0 && d->tile_cols > 0 &&
            d->tile_rows <= SKML_DT_TILE_MAX && d->tile_cols <= SKML_DT_TILE_MAX && d->row_tiles * d->tile_rows >= d->rows &&
-           d->col_tiles * d->tile_cols >= d->dim && d->row_tiles * d->dim < (1ll << 31) - 64 && d->col_tiles * d->rows < (1ll << 31) - 64;
+           d->col_tiles * d->tile_cols >= d->dim && d->row_tiles * d->dim < SKML_DT_LISTS_MAX && d->col_tiles * d->rows < SKML_DT_LISTS_MAX;
 }
 
 }  // namespace

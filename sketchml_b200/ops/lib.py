@@ -54,6 +54,7 @@ class DecodeArgs(C.Structure):
 
 
 DT_TILE_MAX = 49152
+DT_LISTS_MAX = 2 ** 31 - 2 ** 20
 
 
 class DenseIndexArgs(C.Structure):

@@ -172,8 +172,10 @@ def build_dense_index(csr: DeviceCSR, lo: int, hi: int, budget: Optional[int] = 
     a.rows, a.dim = rows, dim
     a.row_tiles, a.tile_rows = _tiles(rows, TILE_ROWS_MAX)
     a.col_tiles, a.tile_cols = _tiles(dim, TILE_ROWS_MAX)
-    if nnz < a.row_tiles * dim or 3 * nnz <= 2 * dim or max(a.row_tiles * dim, a.col_tiles * rows) >= 2 ** 31 - 64:
-        return None   # (lists are numbered in 32 bits)
+    if nnz < a.row_tiles * dim or 3 * nnz <= 2 * dim:
+        return None
+    if max(a.row_tiles * dim, a.col_tiles * rows) + nnz // 4 >= L.DT_LISTS_MAX:
+        return None   # (lists and their quads, at most one more than a quarter of the entries each, are numbered in 32 bits)
     margins = nnz >= 6 * rows * a.col_tiles and a.col_tiles <= 256
     # counts and bounds of all lists, the sums in between, the partial sums of a step (the entries are added below)
     n_lists = (a.row_tiles * dim, a.col_tiles * rows if margins else 0)

@@ -480,17 +480,19 @@ def test_local_id_batches_are_the_sketch_engine_s_alone(mode, extras, taken):
             call()
 
 
-def test_a_batch_with_more_lists_than_32_bits_count_has_no_tiled_index(monkeypatch):
-    """Row lists are counted in 32 bits whether or not the margins use them: such a batch keeps the scatter path."""
+@pytest.mark.parametrize("rows,per_row", [(2 ** 31 - 32, 1), (2 ** 31 - 2 ** 19, 1), (49152, 180_000)])
+def test_a_batch_with_more_lists_than_32_bits_count_has_no_tiled_index(rows, per_row, monkeypatch):
+    """Row lists are counted in 32 bits whether or not the margins use them, by counters that step past the last list by
+    a grid, and so are the quads of entries: a batch beyond that keeps the scatter path."""
     from types import SimpleNamespace
     from sketchml_b200.ops import transposed as T
     monkeypatch.setattr(T.L, "stream", lambda: 0)
 
     class RowPtr(torch.Tensor):
         def __getitem__(self, i):
-            return i        # one entry a row
+            return i * per_row
 
-    rows = 2 ** 31 - 32     # one tile of 100 columns: the sizes are refused before anything is read
+    # one tile of 100 columns: the sizes are refused before anything is read
     csr = SimpleNamespace(cols=torch.zeros(0, dtype=torch.int32), values=None, rowptr=torch.zeros(1, dtype=torch.int64).as_subclass(RowPtr),
                           dim=100)
     assert T.build_dense_index(csr, 0, rows) is None
