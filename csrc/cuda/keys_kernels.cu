@@ -7,12 +7,11 @@
 //   first in two separate streams in java.util.BitSet order (stream bit p = bit (p & 31) of 32-bit
 //   word p >> 5).
 //
-// Every kernel cuts the keys into at most KEY_BLOCKS contiguous runs of whole 1024-key tiles, one run per
-// block, so the prefix sums over runs are short enough for every block to add up on its own: encoding is two
-// launches (a run's histogram of delta widths gives its stream lengths for every mode, so one pass decides
-// the mode and every offset), decoding three (five with unary flags). What bounds both at ordinary sizes is
-// launches and the one wait for the stream lengths that the caller allocates by: 1M keys there and back took
-// 35 launches and 300 us as maps over keys with library scans between them.
+// Every kernel cuts the keys into at most KEY_BLOCKS contiguous runs of whole tiles, one run per block, so the prefix
+// sums over runs are short enough for every block to add up on its own: encoding and decoding are one cooperative launch
+// each (two more where flags are unary). What bounds both at ordinary sizes is the chain of trips to L2, two or three
+// grid barriers among them, and the host's calls around the one wait. 1M keys there and back: 72 us, 80 as seven launches
+// (plan, pack, widths, keys, offsets and fills; a device time of 43 us against 40 here), 300 with library scans.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -21,41 +20,44 @@
 
 namespace {
 
-constexpr int KT = 256;
-constexpr int KEY_TILE = 1024;      // four adjacent keys a thread
-constexpr int KEY_BLOCKS = 592;     // four blocks per SM
-constexpr int STAGE_F = 548;        // words of one tile's flag bits (at most 17 a key, plus a word of misalignment)
-constexpr int STAGE_D = 1028;       // the same for its delta bits (at most 32 a key)
+constexpr int KT = 1024;
+constexpr int KPT = 8;              // adjacent keys of a thread
+constexpr int KEY_TILE = KT * KPT;
+constexpr int KEY_BLOCKS = 192;     // at most one block per SM: a grid barrier of 592 small blocks took twice as long
+constexpr int STAGE_F = KEY_TILE * 17 / 32 + 2;   // words of one tile's flag bits (at most 17 a key, plus a word of misalignment)
+constexpr int STAGE_D = KEY_TILE + 2;             // the same for its delta bits (at most 32 a key)
+constexpr int ZT = 256, Z_TILE = 4 * ZT, Z_BLOCKS = 592;   // unary flags: search for the zero bits
+constexpr long long KEY_BUDGET = 2000000000ll;    // cycles a grid barrier waits at most
 
 struct KeyWork {
-    unsigned int ticket, status;    // status bit 0: keys not strictly increasing (or negative)
-    unsigned int m, kind;
-    unsigned int pad[12];
-    unsigned int total[32];         // encode: delta widths of all keys
-    unsigned long long flag_off[KEY_BLOCKS], delta_off[KEY_BLOCKS];   // encode: first bits of the runs
-    alignas(16) unsigned int hist[KEY_BLOCKS][32];                                // encode: delta widths of the runs
-    unsigned long long run_a[KEY_BLOCKS], run_b[KEY_BLOCKS];          // decode: sums over the runs
+    unsigned int bar, ticket, status;   // cleared by the host; status: SkmlStatus (SKML_BAD_INPUT: keys not strictly increasing, or negative)
+    unsigned int pad[13];
+    unsigned int total[32];             // encode: delta widths of all keys; cleared by the host
+    unsigned int hist[KEY_BLOCKS][32];  // encode: delta widths of the runs
+    unsigned long long run_a[KEY_BLOCKS], run_b[KEY_BLOCKS];   // decode: sums over the runs
+    unsigned long long zeros[Z_BLOCKS];
 };
 
 struct Runs {
-    long long tiles_per_run;
+    long long per_run;
     int runs;
 };
 
-Runs runs_for(long long n) {
-    const long long tiles = (n + KEY_TILE - 1) / KEY_TILE;
+Runs runs_for(long long n, long long tile, int blocks) {
+    const long long tiles = (n + tile - 1) / tile;
+    long long per = (tiles + blocks - 1) / blocks;
+    if (per < 1) per = 1;
     Runs r;
-    r.tiles_per_run = (tiles + KEY_BLOCKS - 1) / KEY_BLOCKS;
-    if (r.tiles_per_run < 1) r.tiles_per_run = 1;
-    r.runs = (int)((tiles + r.tiles_per_run - 1) / r.tiles_per_run);
+    r.per_run = per * tile;
+    r.runs = (int)((tiles + per - 1) / per);
     if (r.runs < 1) r.runs = 1;
     return r;
 }
 
 __device__ __forceinline__ int bits_needed(int d) { return d <= 0 ? 1 : 32 - __clz((unsigned int)d); }
 
-// Exclusive sum over the 256 threads of the block; `total` = the block's sum. Two barriers.
-template <class T>
+// Exclusive sum over the block's threads; `total` = the block's sum. Two barriers.
+template <int THREADS, class T>
 __device__ __forceinline__ T block_scan(T v, T* part, T& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T inc = v;
@@ -67,210 +69,292 @@ __device__ __forceinline__ T block_scan(T v, T* part, T& total) {
     __syncthreads();   // the previous call's readers are done
     if (lane == 31) part[warp] = inc;
     __syncthreads();
-    T base = 0, all = 0;
+    const T x = lane < THREADS / 32 ? part[lane] : T(0);
+    total = warp_sum(x);
+    return warp_sum(lane < warp ? x : T(0)) + inc - v;
+}
+
+// Sum of sums[0, count), by every warp for itself.
+__device__ __forceinline__ unsigned long long sum_before(const unsigned long long* sums, int count) {
+    unsigned long long v = 0;
+#pragma unroll 8
+    for (int i = threadIdx.x & 31; i < count; i += 32) v += __ldcg(sums + i);
+    return warp_sum(v);
+}
+
+// Interval counts, widths and flag of a delta under m intervals of b = 1 << lb bits.
+struct Code {
+    unsigned int fv, fw, dw;   // flag value, flag width, delta width
+};
+__device__ __forceinline__ Code code_of(unsigned int delta, unsigned int lb, unsigned int fb, unsigned int kind) {
+    const unsigned int iv = ((unsigned int)bits_needed((int)delta) + (1u << lb) - 1u) >> lb;
+    Code c;
+    c.fw = kind ? iv + 1 : fb;
+    c.fv = kind ? (1u << (iv + 1)) - 2u : iv - 1;
+    c.dw = iv << lb;
+    return c;
+}
+
+// Deltas of a thread's keys i0 .. i0 + KPT (0 beyond hi). `bad`: keys that are negative or do not ascend.
+__device__ __forceinline__ void load_deltas(const int* __restrict__ keys, long long i0, long long hi, unsigned int (&d)[KPT], bool& bad) {
+    const int lane = threadIdx.x & 31;
+    int k[KPT];
+    if (i0 + KPT <= hi && (reinterpret_cast<uintptr_t>(keys) & 15) == 0) {   // (i0 is a multiple of KPT)
 #pragma unroll
-    for (int w = 0; w < KT / 32; ++w) {
-        const T x = part[w];
-        if (w < warp) base += x;
-        all += x;
+        for (int q = 0; q < KPT / 4; ++q) {
+            const int4 v = *reinterpret_cast<const int4*>(keys + i0 + 4 * q);
+            k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < KPT; ++u) k[u] = i0 + u < hi ? keys[i0 + u] : 0;
     }
-    total = all;
-    return base + inc - v;
+    int prev = __shfl_up_sync(0xFFFFFFFFu, k[KPT - 1], 1);
+    if (lane == 0) prev = i0 > 0 && i0 <= hi ? keys[i0 - 1] : 0;
+#pragma unroll
+    for (int u = 0; u < KPT; ++u) {
+        const bool in = i0 + u < hi;
+        if (in && (k[u] < prev || (k[u] == prev && i0 + u > 0) || k[u] < 0)) bad = true;
+        d[u] = in ? (unsigned int)k[u] - (unsigned int)prev : 0u;
+        prev = k[u];
+    }
 }
 
-// Sum of sums[0, count) by the whole block.
-__device__ __forceinline__ unsigned long long sum_before(const unsigned long long* sums, int count, unsigned long long* part) {
-    unsigned long long v = 0, total;
-    for (int i = threadIdx.x; i < count; i += KT) v += __ldcg(sums + i);
-    block_scan(v, part, total);
-    return total;
+// A thread's bits on their way to a zeroed shared-memory word array, most significant bit of every value first (stream
+// bit p = bit (p & 31) of word p >> 5): words between its first and its last are its own, those two it may share.
+struct BitWriter {
+    unsigned int* word;
+    unsigned long long acc;
+    unsigned int have;
+    bool shared;
+    __device__ __forceinline__ BitWriter(unsigned int* words, unsigned int off) : word(words + (off >> 5)), acc(0), have(off & 31u), shared((off & 31u) != 0) {}
+    __device__ __forceinline__ void put(unsigned int value, unsigned int nb) {   // nb <= 32
+        if (nb == 0) return;
+        acc |= (unsigned long long)(__brev(value) >> (32u - nb)) << have;
+        have += nb;
+        if (have >= 32u) {
+            if (shared) atomicOr(word, (unsigned int)acc);
+            else *word = (unsigned int)acc;
+            shared = false;
+            ++word;
+            acc >>= 32;
+            have -= 32u;
+        }
+    }
+    __device__ __forceinline__ void close() {
+        if (have && (unsigned int)acc) atomicOr(word, (unsigned int)acc);
+    }
+};
+
+// Interval count and flag kind of the DeltaAdaptive key code (reference: binary/DeltaAdaptiveEncoder.java:23-112), by one
+// warp: prob[w] (shared memory) = share of the deltas of width w. The reference's estimates in the same double arithmetic,
+// operation by operation (explicit round-to-nearest intrinsics keep the compiler from fusing multiply-adds), but a lane per
+// interval of every interval count: as one lane per count they were a chain of a hundred additions.
+__device__ __forceinline__ void da_mode(const double* prob, unsigned int& num, unsigned int& kind) {
+    const int lane = threadIdx.x & 31, q = lane < 2 ? 0 : (lane < 6 ? 1 : (lane < 14 ? 2 : 3)), i = lane - ((2 << q) - 2);
+    double ip = 0.0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (j < (16 >> q) && lane < 30) ip = __dadd_rn(ip, prob[i * (16 >> q) + j]);
+    const double term = __dmul_rn((double)(i + 1), ip);
+    const int m = 2 << (lane & 3), b = 16 >> (lane & 3);   // lanes 0 to 3: the estimates of 2, 4, 8 and 16 intervals
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const double t = __shfl_sync(0xFFFFFFFFu, term, (m - 2 + k) & 31);
+        if (k < m) sum = __dadd_rn(sum, t);
+    }
+    const double t1 = __dadd_rn(__dmul_rn(sum, (double)b), (double)((lane & 3) + 1)), t2 = __dadd_rn(__dmul_rn(sum, (double)(b + 1)), 1.0);
+    double best = 32.0;
+    num = 1;
+    kind = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double fixed = __shfl_sync(0xFFFFFFFFu, t1, k), unary = __shfl_sync(0xFFFFFFFFu, t2, k);
+        if (fixed < best) {
+            best = fixed;
+            num = 2u << k;
+            kind = 0;
+        }
+        if (unary < best) {
+            best = unary;
+            num = 2u << k;
+            kind = 1;
+        }
+    }
 }
 
-// Pass 1: histogram of the delta widths of every run. The last block adds them up, chooses the mode and turns
-// the runs' histograms into stream offsets.
-__global__ void __launch_bounds__(KT) da_plan_kernel(const int* __restrict__ keys, long long n, long long per_run, KeyWork* __restrict__ wk,
-                                                     unsigned long long* done, unsigned long long seq) {
+// One stream on its way through shared memory. A tile's whole words are stored; the word it ends in goes on to the
+// next tile, the word a run starts in belongs to the run before, and the run's last word is completed with the first
+// bits of the run behind it (write_tails), so that nobody shares a word and nothing has to be cleared first.
+struct Out {
+    unsigned int* words;
+    unsigned long long at;   // stream bit of the next key
+    unsigned int carry;      // bits of the word `at` lies in
+    bool mine;               // whether that word is this run's
+};
+
+__device__ __forceinline__ void open_tile(unsigned int* stage, unsigned int nbits, const Out& o) {
+    const unsigned int words = ((unsigned int)(o.at & 31ull) + nbits) / 32u + 1u;
+    for (unsigned int i = threadIdx.x; i < words; i += KT) stage[i] = i ? 0u : o.carry;
+}
+
+__device__ __forceinline__ void flush_tile(const unsigned int* stage, Out& o, unsigned int nbits) {
+    const unsigned int end = (unsigned int)(o.at & 31ull) + nbits, full = end >> 5;
+    unsigned int* dst = o.words + (o.at >> 5);
+    for (unsigned int w = threadIdx.x; w < full; w += KT)
+        if (w || o.mine) dst[w] = stage[w];
+    o.carry = end & 31u ? stage[full] : 0u;
+    o.mine = o.mine || full;
+    o.at += nbits;
+}
+
+// The words the run ends in, by one warp: up to 32 keys behind the run have bits there.
+__device__ __forceinline__ void write_tails(const int* __restrict__ keys, long long hi, long long n, unsigned int lb, unsigned int fb,
+                                            unsigned int kind, const Out& f, const Out& d) {
+    const unsigned int lane = threadIdx.x & 31;
+    const long long i = hi + lane;
+    Code c{0, 0, 0};
+    unsigned int delta = 0;
+    if (i < n) {
+        delta = (unsigned int)keys[i] - (unsigned int)keys[i - 1];
+        c = code_of(delta, lb, fb, kind);
+    }
+    unsigned int inc = c.fw + (c.dw << 16);   // at most 17 * 32 and 32 * 32
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= (unsigned int)o) inc += t;
+    }
+    const unsigned int fo = (unsigned int)(f.at & 31ull) + (inc & 0xFFFFu) - c.fw, dof = (unsigned int)(d.at & 31ull) + (inc >> 16) - c.dw;
+    const unsigned int fbits = __reduce_or_sync(0xFFFFFFFFu, c.fw && fo < 32u ? (__brev(c.fv) >> (32u - c.fw)) << fo : 0u);
+    const unsigned int dbits = __reduce_or_sync(0xFFFFFFFFu, c.dw && dof < 32u ? (__brev(delta) >> (32u - c.dw)) << dof : 0u);
+    if (lane == 0) {
+        if (f.mine && (f.at & 31ull)) f.words[f.at >> 5] = f.carry | fbits;
+        if (d.mine && (d.at & 31ull)) d.words[d.at >> 5] = d.carry | dbits;
+        if (hi == n) {   // the streams are counted in 64-bit words
+            const unsigned long long fw = (f.at + 31ull) >> 5, dw = (d.at + 31ull) >> 5;
+            if (fw & 1ull) f.words[fw] = 0u;
+            if (dw & 1ull) d.words[dw] = 0u;
+        }
+    }
+}
+
+// Encoding in one cooperative launch: histogram of every run's delta widths and of all, a grid barrier, the mode and
+// the run's first bits from the histograms (every block adds up those of the runs before its own), then the streams.
+// Runs of one tile keep their deltas in registers across the barrier. 20 us at 1M keys, 17 at 10,000: latency.
+__global__ void __launch_bounds__(KT, 1)
+da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, KeyWork* __restrict__ wk, unsigned int* flag_words,
+                 unsigned int* delta_words, unsigned long long* done, unsigned long long seq) {
+    extern __shared__ __align__(16) unsigned int s_stage[];
+    unsigned int* const s_f = s_stage;
+    unsigned int* const s_d = s_stage + STAGE_F;
     __shared__ unsigned int s_h[KT / 32][32];
-    __shared__ bool s_last;
+    __shared__ unsigned long long s_part[KT / 32], s_at[4];
+    __shared__ double s_prob[32];
+    __shared__ unsigned int s_mode[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    s_h[warp][lane] = 0;
-    __syncwarp();
     const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
     bool bad = false;
-    for (long long i0 = lo; i0 < hi; i0 += 4 * KT) {
-        int k[4], p[4];
+    unsigned int x[KPT], count = 0;   // lane w counts width w
+    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
+        const long long i0 = t0 + (long long)KPT * threadIdx.x;
+        load_deltas(keys, i0, hi, x, bad);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const long long i = i0 + u * KT + threadIdx.x;
-            k[u] = i < hi ? keys[i] : 0;
-            p[u] = i < hi && i ? keys[i - 1] : 0;
-        }
+        for (int u = 0; u < KPT; ++u) {   // a ballot per bit of the width: all lanes would meet in a few counters
+            const int width = bits_needed((int)x[u]) & 31;
+            unsigned int of_lane = __ballot_sync(0xFFFFFFFFu, i0 + u < hi);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const long long i = i0 + u * KT + threadIdx.x;
-            if (i >= hi) continue;
-            if (k[u] < p[u] || (k[u] == p[u] && i > 0) || k[u] < 0) bad = true;
-            atomicAdd(&s_h[warp][bits_needed((int)((unsigned int)k[u] - (unsigned int)p[u])) & 31], 1u);
+            for (int k = 0; k < 5; ++k) of_lane &= __ballot_sync(0xFFFFFFFFu, (width >> k) & 1) ^ (((unsigned int)lane >> k & 1u) - 1u);
+            count += (unsigned int)__popc(of_lane);
         }
     }
-    if (bad) atomicOr(&wk->status, 1u);
+    s_h[warp][lane] = count;
+    if (bad) skml_set_status(&wk->status, SKML_BAD_INPUT, 0x70u);
     __syncthreads();
-    if (threadIdx.x < 32) {
+    if (warp == 0) {
         unsigned int t = 0;
         for (int w = 0; w < KT / 32; ++w) t += s_h[w][lane];
         wk->hist[blockIdx.x][lane] = t;
         if (t) red_add_gpu(&wk->total[lane], t);
     }
+    unsigned int passed = 0;
+    if (!skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, KEY_BUDGET, 0x71u, passed)) return;
+    unsigned int total = 0;
+    if (warp == 0) {
+        total = __ldcg(&wk->total[lane]);
+        s_prob[lane] = __ddiv_rn((double)total, (double)(n > 0 ? n : 1));
+        __syncwarp();
+        unsigned int num, mode;
+        da_mode(s_prob, num, mode);
+        if (lane == 0) {
+            s_mode[0] = num;
+            s_mode[1] = mode;
+        }
+    } else {   // the other warps: histogram of the runs before this one, a width per lane
+        unsigned int t = 0;
+        for (int r = warp - 1; r < (int)blockIdx.x; r += KT / 32 - 1) t += __ldcg(&wk->hist[r][lane]);
+        s_h[warp][lane] = t;
+    }
+    __syncthreads();
+    const unsigned int m = s_mode[0], kind = s_mode[1], lb = (unsigned int)__clz(m) - 26u, fb = 5u - lb;   // 32 / m bits an interval
+    if (warp == 0) {
+        unsigned int before = 0;
+        for (int w = 1; w < KT / 32; ++w) before += s_h[w][lane];
+        const unsigned int iv = ((lane ? (unsigned int)lane : 32u) + (1u << lb) - 1u) >> lb, fw = kind ? iv + 1 : fb, dw = iv << lb;
+        const unsigned long long f0 = warp_sum((unsigned long long)before * fw), d0 = warp_sum((unsigned long long)before * dw);
+        const unsigned long long fa = warp_sum((unsigned long long)total * fw), da = warp_sum((unsigned long long)total * dw);
+        if (lane == 0) {
+            s_at[0] = f0;
+            s_at[1] = d0;
+            s_at[2] = fa;
+            s_at[3] = da;
+        }
+    }
+    __syncthreads();
+    Out f{flag_words, s_at[0], 0u, (s_at[0] & 31ull) == 0}, d{delta_words, s_at[1], 0u, (s_at[1] & 31ull) == 0};
+    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
+        const long long i0 = t0 + (long long)KPT * threadIdx.x;
+        if (per_run > KEY_TILE) load_deltas(keys, i0, hi, x, bad);
+        unsigned int fsum = 0, dsum = 0;   // at most 17 and 32 bits a key
+#pragma unroll
+        for (int u = 0; u < KPT; ++u)
+            if (i0 + u < hi) {
+                const Code c = code_of(x[u], lb, fb, kind);
+                fsum += c.fw;
+                dsum += c.dw;
+            }
+        unsigned long long bits;
+        const unsigned long long ex = block_scan<KT>(((unsigned long long)dsum << 32) | fsum, s_part, bits);
+        open_tile(s_f, (unsigned int)bits, f);
+        open_tile(s_d, (unsigned int)(bits >> 32), d);
+        __syncthreads();
+        BitWriter wf(s_f, (unsigned int)(f.at & 31ull) + (unsigned int)ex), wd(s_d, (unsigned int)(d.at & 31ull) + (unsigned int)(ex >> 32));
+#pragma unroll
+        for (int u = 0; u < KPT; ++u)
+            if (i0 + u < hi) {
+                const Code c = code_of(x[u], lb, fb, kind);
+                wf.put(c.fv, c.fw);
+                wd.put(x[u], c.dw);
+            }
+        wf.close();
+        wd.close();
+        __syncthreads();
+        flush_tile(s_f, f, (unsigned int)bits);
+        flush_tile(s_d, d, (unsigned int)(bits >> 32));
+        // (the next tile's words are cleared behind the barriers of its scan)
+    }
+    if (warp == 0) write_tails(keys, hi, n, lb, fb, kind, f, d);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicAdd(&wk->ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const int runs = (int)gridDim.x;
-    __shared__ double s_prob[32], s_t[2][4];
-    __shared__ unsigned int s_mode[2];
-    if (warp == 0) {
-        s_prob[lane] = __ddiv_rn((double)__ldcg(&wk->total[lane]), (double)(n > 0 ? n : 1));
-        __syncwarp();
-        // the reference's estimates in the same double arithmetic, operation by operation (explicit
-        // round-to-nearest intrinsics keep the compiler from fusing multiply-adds), one lane per interval count
-        if (lane < 4) {
-            const int m = 2 << lane, b = 32 / m;
-            double sum = 0.0;
-            for (int i = 0; i < m; ++i) {
-                double ip = 0.0;
-                for (int j = 0; j < b; ++j) ip = __dadd_rn(ip, s_prob[i * b + j]);
-                sum = __dadd_rn(sum, __dmul_rn((double)(i + 1), ip));
-            }
-            s_t[0][lane] = __dadd_rn(__dmul_rn(sum, (double)b), (double)(lane + 1));
-            s_t[1][lane] = __dadd_rn(__dmul_rn(sum, (double)(b + 1)), 1.0);
+        if (atomicAdd(&wk->ticket, 1u) == gridDim.x - 1) {
+            done[1] = (unsigned long long)m | ((unsigned long long)kind << 32);
+            done[2] = s_at[2];
+            done[3] = s_at[3];
+            __threadfence_system();
+            skml_store_done(done, seq, &wk->status);
         }
-        __syncwarp();
-        if (lane == 0) {
-            double best = 32.0;
-            unsigned int num = 1, kind = 0;
-            for (int q = 0; q < 4; ++q)
-                for (unsigned int k = 0; k < 2; ++k)
-                    if (s_t[k][q] < best) {
-                        best = s_t[k][q];
-                        num = 2u << q;
-                        kind = k;
-                    }
-            s_mode[0] = wk->m = num;
-            s_mode[1] = wk->kind = kind;
-        }
-    }
-    __syncthreads();
-    const unsigned int m = s_mode[0], kind = s_mode[1], b = 32u / m, lb = 31u - (unsigned int)__clz(b), fb = 5u - lb;   // powers of two
-    // bits of the streams up to every run
-    __shared__ unsigned long long s_part[KT / 32];
-    unsigned long long base_f = 0, base_d = 0;
-    for (int r0 = 0; r0 < runs; r0 += KT) {
-        const int r = r0 + (int)threadIdx.x;
-        unsigned long long f = 0, d = 0;
-        if (r < runs) {
-            uint4 h[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) h[q] = ld_cg_v4(reinterpret_cast<const uint4*>(wk->hist[r]) + q);
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const unsigned int k = 4u * q + c, cnt = c == 0 ? h[q].x : (c == 1 ? h[q].y : (c == 2 ? h[q].z : h[q].w));
-                    const unsigned int iv = ((k ? k : 32u) + b - 1) >> lb;
-                    f += (unsigned long long)cnt * (kind ? iv + 1 : fb);
-                    d += (unsigned long long)cnt * (b * iv);
-                }
-        }
-        unsigned long long tf, td;
-        const unsigned long long ef = block_scan(f, s_part, tf), ed = block_scan(d, s_part, td);
-        if (r < runs) {
-            wk->flag_off[r] = base_f + ef;
-            wk->delta_off[r] = base_d + ed;
-        }
-        base_f += tf;
-        base_d += td;
-    }
-    if (threadIdx.x == 0) {
-        done[1] = (unsigned long long)m | ((unsigned long long)kind << 32);
-        done[2] = base_f;
-        done[3] = base_d;
-        __threadfence_system();
-        skml_store_done(done, seq, &wk->status);
-    }
-}
-
-// Writes `nb` (<= 32) bits of `value`, most significant first, at bit `off` of a zeroed shared-memory word array.
-__device__ __forceinline__ void put_bits(unsigned int* words, unsigned int off, unsigned int value, unsigned int nb) {
-    if (nb == 0) return;
-    const unsigned int rv = __brev(value) >> (32u - nb);  // stream order: bit j of rv is stream bit off + j
-    const unsigned int sh = off & 31u, w = off >> 5;
-    atomicOr(&words[w], rv << sh);
-    if (sh + nb > 32u) atomicOr(&words[w + 1], rv >> (32u - sh));
-}
-
-// One tile's bits from shared memory to the stream: whole words are stored, the first and last may be shared
-// with the neighbouring tiles and are completed with atomic ORs (the streams start from zero).
-__device__ __forceinline__ void flush_bits(unsigned int* words, const unsigned int* stage, unsigned long long start, unsigned int nbits) {
-    if (nbits == 0) return;
-    const unsigned int sh = (unsigned int)(start & 31ull), nw = (sh + nbits + 31u) >> 5;
-    unsigned int* dst = words + (start >> 5);
-    for (unsigned int w = threadIdx.x; w < nw; w += KT) {
-        const unsigned int v = stage[w];
-        if ((w == 0 && sh != 0) || (w == nw - 1 && ((sh + nbits) & 31u) != 0)) {
-            if (v) atomicOr(dst + w, v);
-        } else {
-            dst[w] = v;
-        }
-    }
-}
-
-// Pass 2: the two streams.
-__global__ void __launch_bounds__(KT) da_pack_kernel(const int* __restrict__ keys, long long n, long long per_run, const KeyWork* __restrict__ wk,
-                                                     unsigned int* flag_words, unsigned int* delta_words) {
-    __shared__ unsigned int s_f[STAGE_F], s_d[STAGE_D], s_part[KT / 32];
-    const unsigned int m = wk->m, kind = wk->kind, b = 32u / m, fb = 31u - (unsigned int)__clz(m);
-    unsigned long long fs = wk->flag_off[blockIdx.x], ds = wk->delta_off[blockIdx.x];
-    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
-    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-        const long long i0 = t0 + 4 * threadIdx.x;
-        int prev = i0 > 0 && i0 < hi ? keys[i0 - 1] : 0;
-        unsigned int d[4], fv[4], fw[4], dw[4], packed = 0;   // flag bits (<= 17408 a tile) low, delta bits (<= 32768) high
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            d[u] = fv[u] = fw[u] = dw[u] = 0;
-            if (i0 + u < hi) {
-                const int k = keys[i0 + u];
-                d[u] = (unsigned int)k - (unsigned int)prev;
-                prev = k;
-                const unsigned int iv = ((unsigned int)bits_needed((int)d[u]) + b - 1) / b;
-                fw[u] = kind ? iv + 1 : fb;
-                fv[u] = kind ? (1u << (iv + 1)) - 2u : iv - 1;
-                dw[u] = b * iv;
-                packed += fw[u] + (dw[u] << 16);
-            }
-        }
-        for (int i = threadIdx.x; i < STAGE_F; i += KT) s_f[i] = 0;
-        for (int i = threadIdx.x; i < STAGE_D; i += KT) s_d[i] = 0;
-        unsigned int total;
-        const unsigned int ex = block_scan(packed, s_part, total);   // its barriers also publish the cleared words
-        unsigned int fo = (unsigned int)(fs & 31ull) + (ex & 0xFFFFu), dof = (unsigned int)(ds & 31ull) + (ex >> 16);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            put_bits(s_f, fo, fv[u], fw[u]);
-            put_bits(s_d, dof, d[u], dw[u]);
-            fo += fw[u];
-            dof += dw[u];
-        }
-        __syncthreads();
-        flush_bits(flag_words, s_f, fs, total & 0xFFFFu);
-        flush_bits(delta_words, s_d, ds, total >> 16);
-        fs += total & 0xFFFFu;
-        ds += total >> 16;
-        __syncthreads();   // the staging words are cleared again by the next tile
     }
 }
 
@@ -283,15 +367,15 @@ struct Streams {
     int unary;
 };
 
-// Interval counts of keys i0..i0+3 (0 beyond `hi`).
-__device__ __forceinline__ void intervals(const Streams& s, long long i0, long long hi, unsigned int (&iv)[4]) {
+// Interval counts of a thread's keys, from i0 on (0 beyond `hi`).
+__device__ __forceinline__ void intervals(const Streams& s, long long i0, long long hi, unsigned int (&iv)[KPT]) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) iv[u] = 0;
+    for (int u = 0; u < KPT; ++u) iv[u] = 0;
     if (i0 >= hi) return;
     if (s.unary) {
         long long before = i0 ? s.zero_pos[i0 - 1] : -1;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < KPT; ++u)
             if (i0 + u < hi) {
                 const long long z = s.zero_pos[i0 + u];
                 iv[u] = (unsigned int)(z - before - 1);
@@ -299,7 +383,7 @@ __device__ __forceinline__ void intervals(const Streams& s, long long i0, long l
             }
         return;
     }
-    const unsigned int fb = 31u - (unsigned int)__clz(s.m);
+    const unsigned int fb = 31u - (unsigned int)__clz(s.m);   // at most 4
     unsigned long long win = 0;
     if (fb) {
         const unsigned long long off = (unsigned long long)i0 * fb;
@@ -308,7 +392,7 @@ __device__ __forceinline__ void intervals(const Streams& s, long long i0, long l
         win = ((unsigned long long)lo | ((unsigned long long)hw << 32)) >> (off & 31ull);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < KPT; ++u)
         if (i0 + u < hi) {
             const unsigned int bits = fb ? (unsigned int)(win >> (fb * u)) & ((1u << fb) - 1u) : 0u;
             iv[u] = (fb ? __brev(bits) >> (32u - fb) : 0u) + 1u;
@@ -316,26 +400,26 @@ __device__ __forceinline__ void intervals(const Streams& s, long long i0, long l
 }
 
 // Unary flags: zero bits of every run of flag words (a key's flag ends at its zero bit).
-__global__ void __launch_bounds__(KT) da_zero_count_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
+__global__ void __launch_bounds__(ZT) da_zero_count_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
                                                            KeyWork* __restrict__ wk) {
-    __shared__ unsigned long long s_part[KT / 32];
+    __shared__ unsigned long long s_part[ZT / 32];
     const long long nw = (flag_bits + 31) >> 5, lo = per_run * blockIdx.x, hi = lo + per_run < nw ? lo + per_run : nw;
     unsigned long long v = 0, total;
-    for (long long w = lo + threadIdx.x; w < hi; w += KT) {
+    for (long long w = lo + threadIdx.x; w < hi; w += ZT) {
         const long long rest = flag_bits - (w << 5);
         v += __popc(~flag_words[w] & (rest >= 32 ? 0xFFFFFFFFu : ((1u << rest) - 1u)));
     }
-    block_scan(v, s_part, total);
-    if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
+    block_scan<ZT>(v, s_part, total);
+    if (threadIdx.x == 0) wk->zeros[blockIdx.x] = total;
 }
 
 // Stream position of the i-th zero bit.
-__global__ void __launch_bounds__(KT) da_zero_pos_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
+__global__ void __launch_bounds__(ZT) da_zero_pos_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
                                                          const KeyWork* __restrict__ wk, long long n, long long* __restrict__ pos) {
-    __shared__ unsigned long long s_part[KT / 32];
+    __shared__ unsigned long long s_part[ZT / 32];
     const long long nw = (flag_bits + 31) >> 5, lo = per_run * blockIdx.x, hi = lo + per_run < nw ? lo + per_run : nw;
-    unsigned long long base = sum_before(wk->run_a, blockIdx.x, s_part);
-    for (long long w0 = lo; w0 < hi; w0 += KT) {
+    unsigned long long base = sum_before(wk->zeros, blockIdx.x);
+    for (long long w0 = lo; w0 < hi; w0 += ZT) {
         const long long w = w0 + threadIdx.x;
         unsigned int z = 0;
         if (w < hi) {
@@ -343,7 +427,7 @@ __global__ void __launch_bounds__(KT) da_zero_pos_kernel(const unsigned int* __r
             z = ~flag_words[w] & (rest >= 32 ? 0xFFFFFFFFu : ((1u << rest) - 1u));
         }
         unsigned long long total;
-        unsigned long long idx = base + block_scan((unsigned long long)__popc(z), s_part, total);
+        unsigned long long idx = base + block_scan<ZT>((unsigned long long)__popc(z), s_part, total);
         while (z) {
             const int bit = __ffs(z) - 1;
             z &= z - 1;
@@ -354,101 +438,129 @@ __global__ void __launch_bounds__(KT) da_zero_pos_kernel(const unsigned int* __r
     }
 }
 
-// Delta bits of every run.
-__global__ void __launch_bounds__(KT) da_width_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk) {
-    __shared__ unsigned long long s_part[KT / 32];
-    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
-    unsigned long long v = 0, total;
-    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-        unsigned int iv[4];
-        intervals(s, t0 + 4 * threadIdx.x, hi, iv);
-        v += (iv[0] + iv[1] + iv[2] + iv[3]) * (32u / s.m);
-    }
-    block_scan(v, s_part, total);
-    if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
-}
-
-// Keys of every run counted from the key before it, and the runs' sums.
-__global__ void __launch_bounds__(KT) da_extract_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk, int* __restrict__ keys) {
+// Decoding in one cooperative launch: delta bits of every run, a grid barrier, the run's keys counted from the key
+// before it, a grid barrier, the sum of the runs before it added. Runs of one tile keep flags and keys in registers.
+__global__ void __launch_bounds__(KT, 1)
+da_decode_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk, int* __restrict__ keys) {
     __shared__ unsigned long long s_part[KT / 32];
     __shared__ unsigned int s_part32[KT / 32];
     const unsigned int b = 32u / s.m;
     const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
-    unsigned long long bit = sum_before(wk->run_a, blockIdx.x, s_part), sum = 0;
-    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-        const long long i0 = t0 + 4 * threadIdx.x;
-        unsigned int iv[4];
-        intervals(s, i0, hi, iv);
-        unsigned int total;
-        unsigned long long off = bit + block_scan((iv[0] + iv[1] + iv[2] + iv[3]) * b, s_part32, total);
-        bit += total;
-        unsigned int d[4], dsum = 0;
+    const bool keep = per_run <= KEY_TILE;
+    unsigned int passed = 0;
+    auto barrier = [&](unsigned int where) {
+        if (skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, KEY_BUDGET, where, passed)) return true;
+        for (long long i = lo + threadIdx.x; i < hi; i += KT) keys[i] = -1;   // nobody takes these for keys
+        return false;
+    };
+    unsigned int iv[KPT], k[KPT];
+    auto bits_of = [&]() {
+        unsigned int t = 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < KPT; ++u) t += iv[u];
+        return t * b;
+    };
+    unsigned long long bit = 0, sum = 0;
+    if (gridDim.x > 1) {   // (one block has nothing to wait for)
+        unsigned long long v = 0, total;
+        for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
+            intervals(s, t0 + (long long)KPT * threadIdx.x, hi, iv);
+            v += bits_of();
+        }
+        block_scan<KT>(v, s_part, total);
+        if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
+        if (!barrier(0x72u)) return;
+        bit = sum_before(wk->run_a, blockIdx.x);
+    }
+    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
+        const long long i0 = t0 + (long long)KPT * threadIdx.x;
+        if (!keep || gridDim.x == 1) intervals(s, i0, hi, iv);
+        unsigned int total;
+        unsigned long long off = bit + block_scan<KT>(bits_of(), s_part32, total);
+        bit += total;
+        unsigned int dsum = 0;
+#pragma unroll
+        for (int u = 0; u < KPT; ++u) {
             const unsigned int dw = b * iv[u];
-            d[u] = 0;
+            unsigned int d = 0;
             if (dw && dw <= 32u) {
                 const long long w = (long long)(off >> 5);
                 const unsigned int x0 = w < s.delta_lim ? s.delta_words[w] : 0u, x1 = w + 1 < s.delta_lim ? s.delta_words[w + 1] : 0u;
-                d[u] = __brev(__funnelshift_r(x0, x1, (unsigned int)(off & 31ull)) << (32u - dw));
+                d = __brev(__funnelshift_r(x0, x1, (unsigned int)(off & 31ull)) << (32u - dw));
             }
             off += dw;
-            dsum += d[u];
+            dsum += d;
+            k[u] = dsum;
         }
         unsigned int tile_sum;
-        unsigned int key = (unsigned int)sum + block_scan(dsum, s_part32, tile_sum);   // keys are below 2^31: 32-bit sums are exact
+        const unsigned int before = (unsigned int)sum + block_scan<KT>(dsum, s_part32, tile_sum);   // keys are below 2^31: 32-bit sums are exact
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            key += d[u];
-            if (i0 + u < hi) keys[i0 + u] = (int)key;
+        for (int u = 0; u < KPT; ++u) {
+            k[u] += before;
+            if (!keep && i0 + u < hi) keys[i0 + u] = (int)k[u];
         }
         sum += tile_sum;
     }
-    if (threadIdx.x == 0) wk->run_b[blockIdx.x] = sum;
+    unsigned int add = 0;
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) wk->run_b[blockIdx.x] = sum;
+        if (!barrier(0x73u)) return;
+        add = (unsigned int)sum_before(wk->run_b, blockIdx.x);
+    }
+    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
+        const long long i0 = t0 + (long long)KPT * threadIdx.x;
+        if (!keep) {   // (what this thread has written itself)
+#pragma unroll
+            for (int u = 0; u < KPT; ++u)
+                if (i0 + u < hi) k[u] = (unsigned int)keys[i0 + u];
+        }
+        if (i0 + KPT <= hi && (reinterpret_cast<uintptr_t>(keys) & 15) == 0) {
+#pragma unroll
+            for (int q = 0; q < KPT / 4; ++q)
+                *reinterpret_cast<uint4*>(keys + i0 + 4 * q) = make_uint4(k[4 * q] + add, k[4 * q + 1] + add, k[4 * q + 2] + add, k[4 * q + 3] + add);
+        } else {
+#pragma unroll
+            for (int u = 0; u < KPT; ++u)
+                if (i0 + u < hi) keys[i0 + u] = (int)(k[u] + add);
+        }
+    }
 }
 
-__global__ void __launch_bounds__(KT) da_offset_kernel(long long n, long long per_run, const KeyWork* __restrict__ wk, int* __restrict__ keys) {
-    __shared__ unsigned long long s_part[KT / 32];
-    if (blockIdx.x == 0) return;
-    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
-    const int add = (int)sum_before(wk->run_b, blockIdx.x, s_part);
-    for (long long i = lo + threadIdx.x; i < hi; i += KT) keys[i] += add;
+constexpr size_t ENCODE_SMEM = 4 * (size_t)(STAGE_F + STAGE_D);
+
+// Blocks of a cooperative launch of `kernel` (0: an error).
+template <class K>
+int resident_blocks(K kernel, size_t smem) {
+    int dev = 0, sms = 0, per_sm = 0;
+    if (smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, KT, smem) != cudaSuccess || per_sm < 1)
+        return 0;
+    return sms < KEY_BLOCKS ? sms : KEY_BLOCKS;
 }
 
 }  // namespace
 
 extern "C" long long skml_da_workspace_bytes() { return (long long)sizeof(KeyWork); }
 
-extern "C" int skml_da_plan(const int* keys, long long n, void* workspace, unsigned long long* done, unsigned int* status_out, void* stream) {
-    if (n < 0 || !workspace || !done || !status_out) return (int)cudaErrorInvalidValue;
+extern "C" int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* flag_words, unsigned long long* delta_words,
+                              unsigned long long* done, unsigned int* status_out, void* stream) {
+    if (n < 0 || !workspace || !done || !status_out || (n && (!keys || !flag_words || !delta_words))) return (int)cudaErrorInvalidValue;
+    static const int blocks = resident_blocks(da_encode_kernel, ENCODE_SMEM);
+    if (blocks < 1) return (int)cudaErrorLaunchOutOfResources;
     cudaStream_t s = (cudaStream_t)stream;
     KeyWork* wk = reinterpret_cast<KeyWork*>(workspace);
-    cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, flag_off), s);
+    cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, hist), s);
     if (e != cudaSuccess) return (int)e;
-    const Runs r = runs_for(n);
-    const unsigned long long seq = ((*done >> 32) + 1) & 0xFFFFFFFFull;
-    da_plan_kernel<<<r.runs, KT, 0, s>>>(keys, n, r.tiles_per_run * KEY_TILE, wk, done, seq);
-    e = cudaGetLastError();
+    const Runs r = runs_for(n, KEY_TILE, blocks);
+    unsigned long long seq = ((*done >> 32) + 1) & 0xFFFFFFFFull;
+    long long per_run = r.per_run;
+    unsigned int* f = reinterpret_cast<unsigned int*>(flag_words);
+    unsigned int* d = reinterpret_cast<unsigned int*>(delta_words);
+    void* args[] = {&keys, &n, &per_run, &wk, &f, &d, &done, &seq};
+    e = cudaLaunchCooperativeKernel((const void*)da_encode_kernel, dim3((unsigned)r.runs), dim3(KT), args, ENCODE_SMEM, s);
     if (e != cudaSuccess) return (int)e;
     return skml_wait_done(done, seq, &wk->status, status_out, s);
-}
-
-extern "C" int skml_da_pack(const int* keys, long long n, const void* workspace, unsigned long long* flag_words, long long n_flag_words,
-                            unsigned long long* delta_words, long long n_delta_words, void* stream) {
-    if (n <= 0) return 0;
-    cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaSuccess;
-    if (delta_words == flag_words + n_flag_words) {   // one allocation: one fill
-        e = cudaMemsetAsync(flag_words, 0, 8 * (size_t)(n_flag_words + n_delta_words), s);
-    } else {
-        if (n_flag_words) e = cudaMemsetAsync(flag_words, 0, 8 * (size_t)n_flag_words, s);
-        if (e == cudaSuccess && n_delta_words) e = cudaMemsetAsync(delta_words, 0, 8 * (size_t)n_delta_words, s);
-    }
-    if (e != cudaSuccess) return (int)e;
-    const Runs r = runs_for(n);
-    da_pack_kernel<<<r.runs, KT, 0, s>>>(keys, n, r.tiles_per_run * KEY_TILE, reinterpret_cast<const KeyWork*>(workspace),
-                                         reinterpret_cast<unsigned int*>(flag_words), reinterpret_cast<unsigned int*>(delta_words));
-    return (int)cudaGetLastError();
 }
 
 extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,
@@ -457,6 +569,8 @@ extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_
     if (num_intervals < 1 || num_intervals > 16 || (num_intervals & (num_intervals - 1)) || !workspace || (unary && !zero_pos))
         return (int)cudaErrorInvalidValue;
     if (n <= 0) return 0;
+    static const int blocks = resident_blocks(da_decode_kernel, 0);
+    if (blocks < 1) return (int)cudaErrorLaunchOutOfResources;
     cudaStream_t s = (cudaStream_t)stream;
     KeyWork* wk = reinterpret_cast<KeyWork*>(workspace);
     Streams st;
@@ -470,14 +584,16 @@ extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_
     if (unary) {
         const long long nw = (flag_bits + 31) >> 5;
         if (nw > st.flag_lim) return (int)cudaErrorInvalidValue;
-        const Runs f = runs_for(nw);
-        da_zero_count_kernel<<<f.runs, KT, 0, s>>>(st.flag_words, flag_bits, f.tiles_per_run * KEY_TILE, wk);
-        da_zero_pos_kernel<<<f.runs, KT, 0, s>>>(st.flag_words, flag_bits, f.tiles_per_run * KEY_TILE, wk, n, zero_pos);
+        const Runs f = runs_for(nw, Z_TILE, Z_BLOCKS);
+        da_zero_count_kernel<<<f.runs, ZT, 0, s>>>(st.flag_words, flag_bits, f.per_run, wk);
+        da_zero_pos_kernel<<<f.runs, ZT, 0, s>>>(st.flag_words, flag_bits, f.per_run, wk, n, zero_pos);
     }
-    const Runs r = runs_for(n);
-    const long long per = r.tiles_per_run * KEY_TILE;
-    da_width_kernel<<<r.runs, KT, 0, s>>>(st, n, per, wk);
-    da_extract_kernel<<<r.runs, KT, 0, s>>>(st, n, per, wk, keys);
-    if (r.runs > 1) da_offset_kernel<<<r.runs, KT, 0, s>>>(n, per, wk, keys);
-    return (int)cudaGetLastError();
+    const Runs r = runs_for(n, KEY_TILE, blocks);
+    long long per = r.per_run;
+    if (r.runs > 1) {
+        const cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, total), s);
+        if (e != cudaSuccess) return (int)e;
+    }
+    void* args[] = {&st, &n, &per, &wk, &keys};
+    return (int)cudaLaunchCooperativeKernel((const void*)da_decode_kernel, dim3((unsigned)r.runs), dim3(KT), args, 0, s);
 }

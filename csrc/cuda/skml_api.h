@@ -202,15 +202,14 @@ int skml_finalize_compact(float* gc, const float* wc, float lambda, int n, float
                           void* stream);
 int skml_sm_count();
 
-// DeltaAdaptive key codec, stand-alone (csrc/cuda/keys_kernels.cu). skml_da_plan decides the mode and the stream
-// lengths and returns once they are known, in `done` (8 pinned host words): done[1] = interval count | (1 for
-// unary flags) << 32, done[2] / done[3] = flag / delta bits; *status_out bit 0 = keys not strictly increasing
-// or negative. skml_da_pack then writes the streams, ceil(bits / 64) words each (clears them first), with the
-// plan's workspace. skml_da_decode inverts them; zero_pos: n entries of scratch, unary flags only.
+// DeltaAdaptive key codec, stand-alone (csrc/cuda/keys_kernels.cu). skml_da_encode chooses the mode and writes the two
+// streams (room for 17 and 32 bits a key, whole 64-bit words), waits for the end and leaves {interval count | flag kind
+// << 32, flag bits, delta bits} in done[1..3] (pinned host words). *status_out: 0, SKML_BAD_INPUT (in the low byte) where
+// the keys are not strictly increasing or negative, or another status of a launch that gave up. skml_da_decode inverts
+// the streams; zero_pos: n entries of scratch, unary flags only.
 long long skml_da_workspace_bytes();
-int skml_da_plan(const int* keys, long long n, void* workspace, unsigned long long* done, unsigned int* status_out, void* stream);
-int skml_da_pack(const int* keys, long long n, const void* workspace, unsigned long long* flag_words, long long n_flag_words,
-                 unsigned long long* delta_words, long long n_delta_words, void* stream);
+int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* flag_words, unsigned long long* delta_words,
+                   unsigned long long* done, unsigned int* status_out, void* stream);
 int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,
                    long long n_delta_words, long long n, int num_intervals, int unary, long long flag_bits, void* workspace,
                    long long* zero_pos, int* keys, void* stream);

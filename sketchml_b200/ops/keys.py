@@ -7,7 +7,8 @@ themselves, chunk by chunk, without leaving the device (csrc/cuda/compress_kerne
 decode_common.cuh). This module is the library form of the codec, `encode(keys) -> AdaptiveKeys`
 and back, bit for bit equal to the CPU oracle (`oracle.delta_adaptive_encode`). It returns tensors
 of exactly the encoded size, which depends on the data, so `encode` waits once, for the mode and the
-two bit counts (they come through a pinned host word); csrc/cuda/keys_kernels.cu has the kernels.
+two bit counts (they come through a pinned host word); they are views of one buffer with room for any
+list, copies of their own where that room would be large. csrc/cuda/keys_kernels.cu has the kernels.
 """
 from __future__ import annotations
 
@@ -20,6 +21,10 @@ import torch
 
 from . import lib as L
 from .codec import DoneWords
+
+
+BAD_INPUT = 5            # SkmlStatus
+KEEP_WORDS = 1 << 22     # 32 MB
 
 
 @dataclass
@@ -79,15 +84,20 @@ def encode(keys: torch.Tensor) -> AdaptiveKeys:
     n, dev, lib, cs = keys.numel(), keys.device, L.lib(), _call_state()
     stream = L.stream()
     work = _workspace(dev)
-    L.check(lib.skml_da_plan(keys.data_ptr(), n, work.data_ptr(), cs.words.data_ptr(), cs.status_ref, stream), "skml_da_plan")
-    if cs.status.value & 1:
+    room = (17 * n + 63) // 64   # flags take 17 bits a key at most, deltas 32
+    words = torch.empty(room + (n + 1) // 2, dtype=torch.int64, device=dev)
+    L.check(lib.skml_da_encode(keys.data_ptr(), n, work.data_ptr(), words.data_ptr(), words.data_ptr() + 8 * room, cs.words.data_ptr(),
+                               cs.status_ref, stream), "skml_da_encode")
+    L.count_launches(1)
+    if cs.status.value & 0xFF == BAD_INPUT:
         raise ValueError("keys must be non-negative and strictly increasing")
+    if cs.status.value:
+        raise RuntimeError(f"skml_da_encode reported status {cs.status.value:#x}")
     _, mode, flag_bits, delta_bits = cs.words[:4].tolist()
     nf, nd = (flag_bits + 63) // 64, (delta_bits + 63) // 64
-    words = torch.empty(nf + nd, dtype=torch.int64, device=dev)
-    fw, dw = words[:nf], words[nf:]
-    L.check(lib.skml_da_pack(keys.data_ptr(), n, work.data_ptr(), fw.data_ptr(), nf, dw.data_ptr(), nd, stream), "skml_da_pack")
-    L.count_launches(2 if n else 1)
+    fw, dw = words[:nf], words[room:room + nd]
+    if words.numel() > KEEP_WORDS:   # a long list does not keep the unused room
+        fw, dw = fw.clone(), dw.clone()
     return AdaptiveKeys(n, mode & 0xFFFFFFFF, mode >> 32, flag_bits, delta_bits, fw, dw)
 
 
@@ -102,5 +112,5 @@ def decode(e: AdaptiveKeys) -> torch.Tensor:
     pos = torch.empty(n, dtype=torch.int64, device=dev) if e.flag_kind else None
     L.check(lib.skml_da_decode(fw.data_ptr(), fw.numel(), dw.data_ptr(), dw.numel(), n, e.num_intervals, e.flag_kind, e.flag_bits,
                                work.data_ptr(), L.ptr(pos), keys.data_ptr(), L.stream()), "skml_da_decode")
-    L.count_launches(5 if e.flag_kind else 3)
+    L.count_launches(3 if e.flag_kind else 1)
     return keys

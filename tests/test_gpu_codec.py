@@ -715,3 +715,27 @@ def test_checked_calls_leave_their_results_to_any_stream(dense):
             got_sum = out.clone()
         torch.cuda.synchronize()
         assert torch.equal(got, want) and torch.equal(got_sum, want_sum)
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 148 * 8192, 148 * 8192 + 1, 2_500_003])
+@pytest.mark.parametrize("gaps", ["ones", "mixed", "wide"])
+def test_delta_adaptive_device_codec_over_tiles_and_runs(n, gaps):
+    """Less than a tile, one tile, the first bits of a second run; one tile a run everywhere, then several. A list that
+    does not start on 16 bytes gives the same code."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import keys as K
+    rng = np.random.default_rng(n)
+    d = {"ones": np.ones(n, np.int64), "mixed": np.where(rng.random(n) < 0.9, 1, rng.integers(1, 700, n)),
+         "wide": rng.integers(1, max(2, (2 ** 31 - 2) // n), n)}[gaps]
+    keys = np.cumsum(d).astype(np.int32)
+    ref = oracle.delta_adaptive_encode(keys)
+    room = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    room[1:] = torch.from_numpy(keys).cuda()
+    for t in (torch.from_numpy(keys).cuda(), room[1:]):
+        got = K.encode(t)
+        assert (got.num_intervals, got.flag_kind, got.flag_bits, got.delta_bits) == (
+            ref["num_intervals"], ref["flag_kind"], ref["flag_bits"], ref["delta_bits"])
+        o = got.to_oracle_dict()
+        assert np.array_equal(o["flag_words"], np.asarray(ref["flag_words"], dtype=np.uint64))
+        assert np.array_equal(o["delta_words"], np.asarray(ref["delta_words"], dtype=np.uint64))
+        assert np.array_equal(K.decode(got).cpu().numpy(), keys)
