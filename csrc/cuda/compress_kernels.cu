@@ -82,6 +82,9 @@ struct CP {
     int* gkeys;                      // keys, grouped: group g's list starts at Layout::goff[g]
     unsigned int* tables;
     long long tables_cap;
+    unsigned char* gcodes;           // insert in shared memory: rank codes of the keys, in the order of gkeys
+    long long copies_cap;            // insert in shared memory: bytes of the tables' copies (they lie where `tables` does)
+    int priv;                        // insert in shared memory: the launch's parameters allow it (see priv_layout)
     unsigned int* status;
     long long budget;
     const float* given_splits;
@@ -124,17 +127,37 @@ struct Layout {
     unsigned int recip[SKML_MAX_GROUPS];            // floor(2^32 / col) for the mixer-only hash path
     unsigned char hash_ids[SKML_MAX_GROUPS][SKML_MAX_ROWS];  // CP's, where the lanes of a warp may differ in the group
     unsigned long long unit_prefix[SKML_MAX_GROUPS + 1];  // 16-byte units of the narrow tables of the groups before
+    // insert in shared memory (priv_layout): parts a row's cells are cut into, cells of a part, parts of the groups
+    // before, the groups' first unit of work (four keys against one part), units per block, bytes of a copy
+    unsigned int parts[SKML_MAX_GROUPS], part_len[SKML_MAX_GROUPS], part_prefix[SKML_MAX_GROUPS + 1];
+    unsigned long long work_prefix[SKML_MAX_GROUPS + 1], work_per;
+    unsigned int copy_stride;
+    int priv;
     unsigned long long off_bv, off_gt, off_flags, off_restart, off_tables, off_deltas, total_bytes;
     int overflow;
 };
 
 struct WsLayout {
-    long long ctrl, run_vals, run_cnt, run_w, splits_raw, warp_cnt, blk_cnt, blk_bytes, blk_flag, chunk_off, chunk_part, blk_bits, blk_done, key_hist, cell_hist, blk_tbits, tchunk_off, bins, gkeys, tables,
+    long long ctrl, run_vals, run_cnt, run_w, splits_raw, warp_cnt, blk_cnt, blk_bytes, blk_flag, chunk_off, chunk_part, blk_bits, blk_done, key_hist, cell_hist, blk_tbits, tchunk_off, bins, gkeys, gcodes, tables,
         total;
-    long long tables_cap;
+    long long tables_cap, copies_cap;
 };
 
 static inline long long al256(long long x) { return (x + 255) & ~255ll; }
+
+#define PRIV_MIN_KEYS 1000000    // inserts of fewer keys stay with atomics in L2 (see priv_layout)
+#define PRIV_MAX_PASSES 4        // parts that a key is hashed against per row, on average, at most
+#define PRIV_UNITS 2             // units of four keys a thread inserts per round
+#define PRIV_MAX_PARTS 2048      // parts of all groups' rows (their blocks are listed in shared memory)
+#define PRIV_BYTES (136 * 1024)  // cells that fit a block's shared memory
+
+// Bytes of the copies that blocks make of the parts they have worked on: at most one copy per block and part border.
+static inline long long copies_bytes(long long n_max, long long G, long long rows, double col_ratio, long long grid) {
+    if (n_max < PRIV_MIN_KEYS) return 0;
+    const long long cells = (long long)(col_ratio * (double)n_max) + 2;
+    const long long len = cells < PRIV_BYTES ? cells : PRIV_BYTES;
+    return (grid + rows * (2 * cells / PRIV_BYTES + G)) * (len + 32);
+}
 
 static WsLayout ws_layout(long long n_max, long long q, long long G, long long rows, double col_ratio, long long grid) {
     WsLayout L;
@@ -159,7 +182,10 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
     L.bins = o; o += al256(n_max * 2);
     L.gkeys = o; o += al256((n_max + 4 * SKML_MAX_GROUPS + 8) * 4);
     L.tables_cap = rows * ((long long)(col_ratio * (double)n_max) + 2 + G) + 64 + 4 * G;  // groups' tables start at multiples of 4 cells
-    L.tables = o; o += al256(L.tables_cap * 4);
+    L.gcodes = o; o += al256(n_max + 4 * SKML_MAX_GROUPS + 8);
+    L.copies_cap = copies_bytes(n_max, G, rows, col_ratio, grid);
+    if (L.copies_cap < L.tables_cap * 4) L.copies_cap = L.tables_cap * 4;
+    L.tables = o; o += al256(L.copies_cap);
     L.total = o;
     return L;
 }
@@ -245,15 +271,17 @@ struct SmemPack {
 static_assert(sizeof(SmemPack) <= offsetof(SmemCoding, huf_len), "the Huffman code tables outlive the key code's staging");
 
 struct Smem {
+    float splits[SKML_GPU_MAX_BINS];               // stages S3..S6
     union {
         SmemQuantile qs;
         SmemCoding cs;
         SmemSearch ss;
         SmemPack ps;
+        uint2 priv_blocks[PRIV_MAX_PARTS];         // merge of the copies: a part's first block and its number of blocks
     };
     // stages S3..S6
-    float splits[SKML_GPU_MAX_BINS];
     unsigned char grp_lut[SKML_GPU_MAX_BINS];      // bucket -> group
+    unsigned char rank_lut[256], code_bin[256];    // insert in shared memory: bucket -> rank code, edge + rank code -> bucket
     QInfo qi;
     Layout lay;
     unsigned int wcnt[SKML_WARPS][SKML_MAX_GROUPS];
@@ -276,6 +304,12 @@ struct Smem {
 // 2.3M keys takes 69 us with that L1 and 120 us with the 28 KB that the next step (228 KB) leaves.
 static_assert(offsetof(Smem, hdr) % 16 == 0, "the header is read in 16-byte units");
 static_assert(sizeof(Smem) <= 162 * 1024, "the compress kernels' shared memory must stay below the 164 KB carve-out");
+
+// Insert in shared memory: the cells lie behind the first 256 split points (all there are with codes of a byte) and in
+// the stages' shared region.
+#define PRIV_SPLITS 256
+static_assert(offsetof(Smem, qs) == SKML_GPU_MAX_BINS * 4, "the cells need one piece of shared memory");
+static_assert(offsetof(Smem, grp_lut) - PRIV_SPLITS * 4 >= PRIV_BYTES && PRIV_BYTES % 16 == 0, "room for the cells");
 
 __device__ __forceinline__ unsigned int lanemask_lt() {
     unsigned int m;
@@ -924,11 +958,23 @@ __device__ __forceinline__ long long vslice_size(long long n) {
     return (c + 31) / 32 * 32;
 }
 
+template <bool PRIV>
 __device__ __forceinline__ void build_group_lut(const CP& p, Smem& s) {
     for (int b = threadIdx.x; b < s.qi.bin_num; b += blockDim.x) {
         int g = 0;   // the edges ascend: the group is the number of edges at or below the bucket
         for (int e = 0; e < p.G - 1; ++e) g += s.qi.edges[e] <= b ? 1 : 0;
         s.grp_lut[b] = (unsigned char)g;
+        if (PRIV) {
+            // rank of the bucket's cell among those of its group: by distance from the zero bucket, the lower bucket first
+            const int lo = g ? s.qi.edges[g - 1] : 0, hi = s.qi.edges[g], z = s.qi.zero_idx;
+            const int below = z - lo, above = hi - 1 - z, d = b < z ? z - b : b - z;
+            int rank = d;
+            if (below <= 0) rank = b - lo;
+            else if (above <= 0) rank = hi - 1 - b;
+            else if (d) rank = 1 + min(d - 1, below) + min(d - 1, above) + (b > z && d <= below ? 1 : 0);
+            s.rank_lut[b] = (unsigned char)rank;
+            s.code_bin[lo + rank] = (unsigned char)b;
+        }
     }
     __syncthreads();
 }
@@ -955,17 +1001,47 @@ __device__ __forceinline__ void group_masks(bool valid, int g, unsigned int& own
     }
 }
 
-// S3: bucket of every value; keys of every group in every warp slice, 64 values a turn (two searches side by side).
+// U searches side by side, the next turn's values on their way.
+template <int U>
+__device__ __forceinline__ void count_turns(Smem& s, int top, int rem, const float* __restrict__ vals, unsigned short* __restrict__ bins,
+                                            const float (&first_val)[2], int (&first_bin)[2], unsigned int& kmin, unsigned int& kmax) {
+    const int warp = threadIdx.x >> 5;
+    float nval[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) nval[u] = u < 2 ? first_val[u] : (32 * u < rem ? vals[32 * u] : 0.f);
+    for (int i0 = 0; i0 < rem; i0 += 32 * U) {
+        float val[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            val[u] = nval[u];
+            if (i0 + 32 * (U + u) < rem) nval[u] = vals[i0 + 32 * (U + u)];
+        }
+        int bin[U];
+        upper_bounds_f(s.ss.a, top, val, bin);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + 32 * u >= rem) break;
+            bins[i0 + 32 * u] = (unsigned short)bin[u];
+            if (u < 2 && i0 == 0) first_bin[u] = bin[u];
+            atomicAdd(&s.wcnt[warp][s.grp_lut[bin[u]]], 1u);
+            const unsigned int k = f2ord(val[u]);
+            kmin = min(kmin, k);
+            kmax = max(kmax, k);
+        }
+    }
+}
+
+// S3: bucket of every value; keys of every group in every warp slice.
 // Bound by instruction issue: a conflict-free search unrolled for up to 255 splits, 32-bit positions inside the slice
 // and shared-memory counts instead of a match of the warp took it from 58 to 31 us at 10M values.
 // `first_val`: the values of this lane's first two elements where the caller has them in flight already; their
 // buckets are left in `first_bin`.
-template <bool FUSED>
+template <bool FUSED, bool PRIV>
 __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax, const float (&first_val)[2], int (&first_bin)[2]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
     const int top = build_search(s);
-    build_group_lut(p, s);
+    build_group_lut<PRIV>(p, s);
     const long long sub = vslice_size(n);
     const long long vb = (long long)blockIdx.x * SKML_WARPS + warp;
     long long lo = vb * sub, hi = lo + sub;
@@ -976,25 +1052,10 @@ __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax
     const int rem = (int)(hi - lo) - lane;   // this lane's elements: 0, 32, ... below it
     const float* const vals = p.vals + lo + lane;
     unsigned short* const bins = p.bins + lo + lane;
-    float nval[2] = {first_val[0], first_val[1]};  // one turn ahead: the load latency stays off the chain
-    for (int i0 = 0; i0 < rem; i0 += 64) {
-        const float val[2] = {nval[0], nval[1]};
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-            if (i0 + 64 + 32 * u < rem) nval[u] = vals[i0 + 64 + 32 * u];
-        int bin[2];
-        upper_bounds_f(s.ss.a, top, val, bin);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            if (i0 + 32 * u >= rem) break;
-            bins[i0 + 32 * u] = (unsigned short)bin[u];
-            if (i0 == 0) first_bin[u] = bin[u];
-            atomicAdd(&s.wcnt[warp][s.grp_lut[bin[u]]], 1u);
-            const unsigned int k = f2ord(val[u]);
-            kmin = min(kmin, k);
-            kmax = max(kmax, k);
-        }
-    }
+    // 32 U values a turn: short slices are not worth a second pair of searches, long ones want the loads in flight (2.3M
+    // values: 11.3 -> 10.1 us, 10M: 32 -> 27.6)
+    if (!PRIV || sub <= 64) count_turns<2>(s, top, rem, vals, bins, first_val, first_bin, kmin, kmax);
+    else count_turns<4>(s, top, rem, vals, bins, first_val, first_bin, kmin, kmax);
     __syncwarp();
     // (one launch for all stages: the slices' counts stay in shared memory)
     if (!FUSED && lane < p.G) p.warp_cnt[vb * SKML_MAX_GROUPS + lane] = s.wcnt[warp][lane];
@@ -1137,8 +1198,165 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
     __syncthreads();
 }
 
+// Insert in shared memory (large gradients, plain tables). A cell of the sketch is decided by the rank of its bucket among
+// the buckets of its group, a byte where a group has at most 255 of them, so a row of a group's table is small enough for
+// a block's shared memory, or a few parts of it are. Work is (part of a row, four keys of the group's list); the units of
+// all parts, one part behind the other, are dealt to the blocks in equal runs. A block hashes its keys for one row, keeps
+// the least codes in shared memory and leaves a copy of the part; the copies of a part are merged when the tables are
+// written to the payload. Bound by the hashes' instructions and the latency of the rounds; atomics in L2, three a key, by
+// L2's rate (121 G/s). Insert and all, S4 and S5 of such launches (rows of 0.2 cells a key; atomics / shared memory, us):
+// 0.5M keys 26 / 33, 1M 41 / 38, 2.27M 76 / 63, 5M 158 / 126, 10M 302 / 268, which is why smaller ones keep the atomics.
+// Sets L.priv where it pays: the keys of large groups are hashed once per part, so a group of many parts (few distinct
+// values: one group holds nearly every key) is left to the atomics.
+__device__ void priv_layout(const CP& p, Smem& s) {
+    Layout& L = s.lay;
+    const int lane = threadIdx.x & 31, G = p.G;
+    if (threadIdx.x < 32) {
+        unsigned int parts = 0, len = 0;
+        unsigned long long work = 0;
+        if (lane < G && L.n_g[lane]) {
+            const unsigned int room = PRIV_BYTES - 16u;   // (a part starts at its place in a 16-byte unit)
+            parts = (L.col[lane] + room - 1u) / room;
+            len = (L.col[lane] + parts - 1u) / parts;
+            work = (unsigned long long)p.rows * parts * ((L.n_g[lane] + 3u) / 4u);
+        }
+        unsigned long long nparts, units;
+        const unsigned long long part0 = warp_prefix((unsigned long long)p.rows * parts, nparts), work0 = warp_prefix(work, units);
+        const unsigned int longest = __reduce_max_sync(0xFFFFFFFFu, len);
+        unsigned long long keys;
+        warp_prefix(lane < G ? (unsigned long long)L.n_g[lane] : 0ull, keys);
+        if (lane < G) {
+            L.parts[lane] = parts;
+            L.part_len[lane] = len;
+            L.part_prefix[lane] = (unsigned int)part0;
+            L.work_prefix[lane] = work0;
+        }
+        if (lane == 0) {
+            L.part_prefix[G] = (unsigned int)nparts;
+            L.work_prefix[G] = units;
+            L.work_per = (units + gridDim.x - 1) / gridDim.x;
+            L.copy_stride = (longest + 15u + 15u) & ~15u;
+            L.priv = nparts <= PRIV_MAX_PARTS && 4ull * units <= (unsigned long long)PRIV_MAX_PASSES * p.rows * keys + 4ull * nparts &&
+                     (nparts + gridDim.x) * L.copy_stride <= (unsigned long long)p.copies_cap;
+        }
+    }
+    __syncthreads();
+}
+
+// Units [u0, u1) of one group's keys against one part of one row: cells lo .. lo + len of the row at cells[at ..].
+// Two block barriers per round instead of an atomic per key: codes smaller than the cell's are stored plainly, so where
+// several threads meet in a cell any of them may win; behind the barrier every thread that has stored looks again, and
+// those that find a larger code (few) repeat it with compare-and-swap, while nobody stores plainly.
+template <int MIXER>
+__device__ __forceinline__ void priv_insert(const CP& p, const Layout& L, int g, unsigned int u0, unsigned int u1, unsigned int lo,
+                                            unsigned int len, unsigned int at, unsigned char* cells) {
+    const unsigned int n = L.n_g[g], col = L.col[g], recip = L.recip[g];
+    const int4* const keys = reinterpret_cast<const int4*>(p.gkeys + L.goff[g]);                       // (lists start at multiples of four)
+    const unsigned int* const codes = reinterpret_cast<const unsigned int*>(p.gcodes + L.goff[g]);
+    int4 nk[PRIV_UNITS];
+    unsigned int nc[PRIV_UNITS];
+    auto fetch = [&](unsigned int u) {
+#pragma unroll
+        for (int q = 0; q < PRIV_UNITS; ++q) {
+            nk[q] = make_int4(0, 0, 0, 0);
+            nc[q] = 0;
+            if (u + q * SKML_BLOCK < u1) {
+                nk[q] = __ldcg(keys + u + q * SKML_BLOCK);
+                nc[q] = __ldcg(codes + u + q * SKML_BLOCK);
+            }
+        }
+    };
+    fetch(u0 + threadIdx.x);
+    for (unsigned int base = u0; base < u1; base += PRIV_UNITS * SKML_BLOCK) {
+        const unsigned int u = base + threadIdx.x;
+        unsigned int c[PRIV_UNITS], pos[PRIV_UNITS][4];
+#pragma unroll
+        for (int q = 0; q < PRIV_UNITS; ++q) {
+            const int k[4] = {nk[q].x, nk[q].y, nk[q].z, nk[q].w};
+            const unsigned int uq = u + q * SKML_BLOCK;
+            c[q] = nc[q];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const unsigned int h = MIXER == 0 ? skml_mix_bj((unsigned int)k[i]) : (MIXER == 1 ? skml_mix_64((unsigned int)k[i]) : skml_mix_tw((unsigned int)k[i]));
+                const unsigned int x = (unsigned int)skml_java_mod(h, col, recip) - lo;
+                pos[q][i] = x < len && uq < u1 && 4u * uq + i < n ? x + at : ~0u;
+            }
+        }
+        fetch(u + PRIV_UNITS * SKML_BLOCK);
+        unsigned char old[PRIV_UNITS][4];
+#pragma unroll
+        for (int q = 0; q < PRIV_UNITS; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) old[q][i] = pos[q][i] != ~0u ? *(volatile unsigned char*)(cells + pos[q][i]) : 0;
+#pragma unroll
+        for (int q = 0; q < PRIV_UNITS; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const unsigned int code = (c[q] >> (8 * i)) & 0xFFu;
+                if (code < old[q][i]) *(volatile unsigned char*)(cells + pos[q][i]) = (unsigned char)code;
+                else pos[q][i] = ~0u;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PRIV_UNITS; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) old[q][i] = pos[q][i] != ~0u ? *(volatile unsigned char*)(cells + pos[q][i]) : 0;
+#pragma unroll
+        for (int q = 0; q < PRIV_UNITS; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const unsigned int code = (c[q] >> (8 * i)) & 0xFFu;
+                if (code < old[q][i]) {
+                    unsigned int* const word = reinterpret_cast<unsigned int*>(cells) + (pos[q][i] >> 2);
+                    const unsigned int shift = 8u * (pos[q][i] & 3u);
+                    unsigned int seen = *(volatile unsigned int*)word;
+                    while (((seen >> shift) & 0xFFu) > code) {
+                        const unsigned int was = atomicCAS(word, seen, (seen & ~(0xFFu << shift)) | (code << shift));
+                        if (was == seen) break;
+                        seen = was;
+                    }
+                }
+            }
+        __syncthreads();
+    }
+}
+
+__device__ void stage_insert(const CP& p, Smem& s) {
+    const Layout& L = s.lay;
+    if (L.overflow) return;
+    unsigned char* const cells = reinterpret_cast<unsigned char*>(s.splits + PRIV_SPLITS);
+    unsigned long long w = L.work_per * blockIdx.x;
+    unsigned long long w1 = w + L.work_per;
+    if (w1 > L.work_prefix[p.G]) w1 = L.work_prefix[p.G];
+    int g = 0;
+    while (w < w1) {   // one part of a row after the other
+        while (g + 1 < p.G && w >= L.work_prefix[g + 1]) ++g;
+        const unsigned int per_part = (L.n_g[g] + 3u) / 4u;
+        const unsigned int t = (unsigned int)((w - L.work_prefix[g]) / per_part);
+        const unsigned long long part_w = L.work_prefix[g] + (unsigned long long)t * per_part;
+        const unsigned int u0 = (unsigned int)(w - part_w), u1 = (unsigned int)min((unsigned long long)per_part, w1 - part_w);
+        const unsigned int row = t / L.parts[g], lo = (t - row * L.parts[g]) * L.part_len[g];
+        const unsigned int len = min(L.part_len[g], L.col[g] - lo);
+        const unsigned int at = (unsigned int)(((unsigned long long)row * L.col[g] + lo) & 15ull), units = (at + len + 15u) / 16u;
+        uint4* const cells4 = reinterpret_cast<uint4*>(cells);
+        for (unsigned int i = threadIdx.x; i < units; i += SKML_BLOCK) cells4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        __syncthreads();
+        const int id = L.hash_ids[g][row];
+        if (id == 0) priv_insert<0>(p, L, g, u0, u1, lo, len, at, cells);
+        else if (id == 1) priv_insert<1>(p, L, g, u0, u1, lo, len, at, cells);
+        else priv_insert<2>(p, L, g, u0, u1, lo, len, at, cells);
+        __syncthreads();
+        // the blocks and the parts of a run of work ascend together: block + part names a copy
+        uint4* const out = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(p.tables) +
+                                                    (unsigned long long)(blockIdx.x + L.part_prefix[g] + t) * L.copy_stride);
+        for (unsigned int i = threadIdx.x; i < units; i += SKML_BLOCK) __stcg(out + i, cells4[i]);
+        __syncthreads();
+        w = part_w + u1;
+    }
+}
+
 // S4: every key goes to its group's staging list (stable, so the lists stay sorted);
-// grouped MinMaxSketch insert.
+// grouped MinMaxSketch insert with atomics in L2.
 // `nkey`, `nbin`: keys and buckets of this lane's first two elements (one launch for all stages). What bounds it is
 // the rate of atomics in L2: three a key, 121 G/s at 10M keys; a plain count of 100M random keys reaches 156 G/s.
 template <bool FUSED>
@@ -1147,7 +1365,7 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n, int (&nkey)[2],
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Layout& L = s.lay;
     if (L.overflow) return;
-    if (!FUSED) build_group_lut(p, s);   // (otherwise the group table is the count stage's)
+    if (!FUSED) build_group_lut<false>(p, s);   // (otherwise the group table is the count stage's)
     const long long sub = vslice_size(n);
     const long long vb = (long long)blockIdx.x * SKML_WARPS + warp;
     long long lo = vb * sub, hi = lo + sub;
@@ -1210,6 +1428,60 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n, int (&nkey)[2],
             }
         }
         __syncwarp();
+    }
+}
+
+// S4 where the insert follows in shared memory: the lists get the keys and their rank codes, 128 elements a turn with the
+// next ones on their way.
+__device__ void stage_partition(const CP& p, Smem& s, long long n) {
+    constexpr int U = 4;
+    const int G = p.G, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Layout& L = s.lay;
+    if (L.overflow) return;
+    const long long sub = vslice_size(n);
+    const long long vb = (long long)blockIdx.x * SKML_WARPS + warp;
+    long long lo = vb * sub, hi = lo + sub;
+    if (lo > n) lo = n;
+    if (hi > n) hi = n;
+    unsigned int run = 0;   // lane g: staging position of the next key of group g in this slice
+    if (lane < G) run = L.goff[lane] + L.base_rank[lane] + s.wbase[warp][lane];
+    const int len = (int)(hi - lo), rem = len - lane;   // this lane's elements: 0, 32, ... below rem
+    const int* const keys = p.keys + lo + lane;
+    const unsigned short* const bins = p.bins + lo + lane;
+    int nkey[U], nbin[U];
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            nkey[u] = nbin[u] = 0;
+            if (i0 + 32 * u < rem) {
+                nkey[u] = keys[i0 + 32 * u];
+                nbin[u] = bins[i0 + 32 * u];
+            }
+        }
+    };
+    fetch(0);
+    for (int i0 = 0; i0 < len; i0 += 32 * U) {
+        int key[U], bin[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            key[u] = nkey[u];
+            bin[u] = nbin[u];
+        }
+        fetch(i0 + 32 * U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool valid = i0 + 32 * u < rem;
+            const int g = valid ? (int)s.grp_lut[bin[u]] : 0;
+            unsigned int own, of_lane;
+            if (G <= 8) group_masks<3>(valid, g, own, of_lane);
+            else group_masks<5>(valid, g, own, of_lane);
+            const unsigned int to = __shfl_sync(0xFFFFFFFFu, run, g) + (unsigned int)__popc(own & lanemask_lt());
+            run += (unsigned int)__popc(of_lane);   // (of lanes beyond the last group nobody asks)
+            if (valid) {
+                p.gkeys[to] = key[u];
+                p.gcodes[to] = s.rank_lut[bin[u]];
+            }
+        }
     }
 }
 
@@ -2290,15 +2562,18 @@ __device__ void layout_finish(const CP& p, Smem& s, unsigned int nactive) {
     __syncthreads();
 }
 
-// Fill helpers run inside S1 (they do not depend on the summary).
-__device__ void stage_prepare(const CP& p, long long n) {
+// Fill helpers run inside S1 (they do not depend on the summary). priv: the sketch is not expected to be inserted in
+// p.tables; where it is after all, a second call fills the tables only.
+__device__ void stage_prepare(const CP& p, long long n, bool priv, bool tables_only = false) {
     // working sketch cells start "empty"
     long long cells = (long long)p.rows * ((long long)(p.col_ratio * (double)n) + 2 + p.G) + 4 * p.G;
     if (cells > p.tables_cap - 4) cells = p.tables_cap - 4;
     const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
     uint4* t4 = reinterpret_cast<uint4*>(p.tables);
-    for (long long i = gid; i < (cells + 3) / 4; i += gsz) t4[i] = ones;
+    if (!priv)
+        for (long long i = gid; i < (cells + 3) / 4; i += gsz) t4[i] = ones;
+    if (tables_only) return;
     if (p.zero_slot) clear_slot(p, 0, gid, gsz);   // (two grid barriers lie before the first byte of the payload)
     if (p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE || p.huffman) {
         // the bit streams are completed with atomic ORs where chunks meet: they start from zero
@@ -2495,6 +2770,64 @@ __device__ void narrow_tables(const CP& p, Smem& s) {
     }
 }
 
+// The copies of the sketch's parts (stage_insert) -> bucket codes, stored locally and into the peers' slots.
+__device__ void merge_copies(const CP& p, Smem& s) {
+    const Layout& L = s.lay;
+    if (L.overflow) return;
+    const int G = p.G;
+    for (unsigned int t = threadIdx.x; t < L.part_prefix[G]; t += SKML_BLOCK) {
+        int g = 0;
+        while (g + 1 < G && t >= L.part_prefix[g + 1]) ++g;
+        const unsigned int per_part = (L.n_g[g] + 3u) / 4u;
+        const unsigned long long w0 = L.work_prefix[g] + (unsigned long long)(t - L.part_prefix[g]) * per_part;
+        const unsigned int b0 = (unsigned int)(w0 / L.work_per), b1 = (unsigned int)((w0 + per_part - 1) / L.work_per);
+        s.priv_blocks[t] = make_uint2(b0, b1 - b0 + 1u);
+    }
+    __syncthreads();
+    const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long units = (long long)L.unit_prefix[G];
+    const unsigned int zero = (unsigned int)s.qi.zero_idx;
+    for (long long u = gid; u < units; u += gsz) {
+        int g = 0;
+        while (g + 1 < G && (unsigned long long)u >= L.unit_prefix[g + 1]) ++g;
+        const unsigned long long j = (unsigned long long)u - L.unit_prefix[g];
+        const unsigned int col = L.col[g], parts = L.parts[g], plen = L.part_len[g];
+        const unsigned long long c0 = 16ull * j, c1 = min(c0 + 16ull, (unsigned long long)p.rows * col);   // cells of this unit
+        uint4 m = make_uint4(~0u, ~0u, ~0u, ~0u);
+        for (unsigned long long c = c0; c < c1;) {   // the parts that have cells in it: one, two at a border
+            const unsigned int row = (unsigned int)(c / col), in_row = (unsigned int)(c - (unsigned long long)row * col), part = in_row / plen;
+            const unsigned int t = L.part_prefix[g] + row * parts + part;
+            const unsigned long long first = (unsigned long long)row * col + (unsigned long long)part * plen;
+            const uint2 blocks = s.priv_blocks[t];
+            const unsigned char* src = reinterpret_cast<const unsigned char*>(p.tables) + (unsigned long long)(blocks.x + t) * L.copy_stride +
+                                       16ull * (j - first / 16ull);
+#pragma unroll 4
+            for (unsigned int b = 0; b < blocks.y; ++b) {
+                const uint4 v = ld_cg_v4(reinterpret_cast<const uint4*>(src + (unsigned long long)b * L.copy_stride));
+                m.x = __vminu4(m.x, v.x);
+                m.y = __vminu4(m.y, v.y);
+                m.z = __vminu4(m.z, v.z);
+                m.w = __vminu4(m.w, v.w);
+            }
+            c = min(first + plen, (unsigned long long)(row + 1) * col);
+        }
+        const unsigned int lo = g ? (unsigned int)s.qi.edges[g - 1] : 0u, left = (unsigned int)(c1 - c0);
+        auto bucket = [&](unsigned int code, unsigned int i) {
+            return i >= left ? 0u : (code == 0xFFu ? zero : (unsigned int)s.code_bin[lo + code]);
+        };
+        auto word = [&](unsigned int x, unsigned int i) {
+            return bucket(x & 0xFFu, i) | (bucket((x >> 8) & 0xFFu, i + 1) << 8) | (bucket((x >> 16) & 0xFFu, i + 2) << 16) |
+                   (bucket(x >> 24, i + 3) << 24);
+        };
+        const uint4 v = make_uint4(word(m.x, 0), word(m.y, 4), word(m.z, 8), word(m.w, 12));
+        const unsigned long long off = L.table_off[g] + 16ull * j;
+        st_v4(reinterpret_cast<uint4*>(p.payload + off), v);
+        for (unsigned int r = 0; r < p.world; ++r)
+            if (r != p.rank && p.peer_payload[r]) st_v4(reinterpret_cast<uint4*>(p.peer_payload[r] + off), v);
+    }
+    __syncthreads();
+}
+
 // Bytes [lo, hi) of the local payload -> the same bytes of every peer's slot, by this block alone:
 // 16-byte stores for the aligned interior, byte stores for a ragged head or tail (two blocks that
 // share a 16-byte unit each store only their own bytes of it).
@@ -2660,8 +2993,9 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
 
 // STAGE < 0: all stages in one cooperative launch; otherwise only that stage.
 // ADAPTIVE / HUFFMAN: the key encoder and the table coder are compile-time choices, so that the default
-// path (delta_binary keys, plain tables) carries none of the other coders' registers.
-template <bool FUSED, bool ADAPTIVE, bool HUFFMAN>
+// path (delta_binary keys, plain tables) carries none of the other coders' registers. PRIV: launches that may have enough
+// keys for the insert in shared memory (its code costs the others 2 us).
+template <bool FUSED, bool ADAPTIVE, bool HUFFMAN, bool PRIV>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, int stage) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
@@ -2714,8 +3048,9 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             }
         }
     }
+    bool priv = PRIV && n >= PRIV_MIN_KEYS;   // insert in shared memory
     if (FUSED || stage == 1) {
-        stage_prepare(p, n);
+        stage_prepare(p, n, priv);
         stage_stamp(p.ctrl, 8);
         if (sample) stage_sample_splits(p, s, p.vals, n);
         else if (!given) stage_summary(p, s, p.vals, n);
@@ -2737,15 +3072,28 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x32u);
             return;
         }
-        stage_count<FUSED>(p, s, n, sample, first_val, first_bin);
+        stage_count<FUSED, PRIV>(p, s, n, sample, first_val, first_bin);
     }
     STAGE_BARRIER(3)
     if (FUSED || stage == 4) {
         if (!FUSED) load_quantizer(p, s);
         layout_from_counts<FUSED>(p, s, FUSED && sample);
-        stage_scatter<FUSED>(p, s, n, first_key, first_bin);
+        if (priv) {
+            priv_layout(p, s);
+            priv = s.lay.priv != 0;
+            if (!priv) {   // the same in every block
+                stage_prepare(p, n, false, true);
+                if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x14u, passed)) return;
+            }
+        }
+        if (priv) stage_partition(p, s, n);
+        else stage_scatter<FUSED>(p, s, n, first_key, first_bin);
     }
     STAGE_BARRIER(4)
+    if (priv) {
+        stage_insert(p, s);
+        stage_stamp(p.ctrl, 7);
+    }
     // S5: key code and publication. In one cooperative launch a block waits only for the counts of the
     // blocks before it (they are resident, and never wait for a later block), and the last block for all of
     // them before it writes the header (it has the fewest chunks, none where there are fewer than blocks);
@@ -2767,7 +3115,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     if (FUSED || stage == 5) {
         if (huffman) {
             if (!s.lay.overflow) huf_histogram(p, s, t_begin, t_end);
-        } else if (adaptive) {
+        } else if (adaptive && !priv) {
             narrow_tables(p, s);   // the tables are complete since S4
         }
         if (adaptive && !s.lay.overflow) apack_histogram(p, s, my_begin, my_end);
@@ -2794,7 +3142,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             st_relaxed_gpu(&p.blk_flag[blockIdx.x], epoch);
         }
     }
-    if (!huffman && !adaptive && (FUSED || stage == 6)) narrow_tables(p, s);   // while the publications travel
+    if (!huffman && !adaptive && !priv && (FUSED || stage == 6)) narrow_tables(p, s);   // while the publications travel
     const bool borders = adaptive || huffman;  // stream words shared by two blocks are sent by the last block at the end
     if (FUSED || stage == 7) {
         if (!FUSED) {  // the block's own counts again (shared memory does not survive a launch)
@@ -2822,6 +3170,10 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             huf_prefix(p, s);   // (the key prefix above has waited for the blocks before this one)
             huf_write(p, s, t_begin, t_end);
             huf_push_own(p, s, t_begin, t_end);
+        }
+        if (priv) {   // every block has made its copies before it published its counts
+            if (!wait_published(p, p.blk_flag, gridDim.x, epoch, 0x54u)) return;
+            merge_copies(p, s);
         }
         if (FUSED && borders) {
             __syncthreads();
@@ -2923,6 +3275,8 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     p.bins = reinterpret_cast<unsigned short*>(ws + L.bins);
     p.tables = reinterpret_cast<unsigned int*>(ws + L.tables);
     p.tables_cap = L.tables_cap;
+    p.gcodes = ws + L.gcodes;
+    p.copies_cap = L.copies_cap;
     p.status = a->status;
     p.budget = a->budget_cycles > 0 ? a->budget_cycles : 2000000000ll;
     p.given_splits = a->given_splits;
@@ -2942,6 +3296,11 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
         skml_pick_hashes(p.seed, p.step, p.rank, (unsigned int)g, p.rows, p.hash_ids[g]);
         for (int r = 0; r < p.rows && p.mixers; ++r) p.mixers = p.hash_ids[g][r] < 3;
     }
+    // codes of a byte, 255 meaning "no key": at most 255 buckets in a group (from three groups on a group has at most
+    // half of all buckets and half a group more)
+    const int bins = a->given_splits ? (int)a->n_given + 1 : p.q;
+    const long long n_known = !a->meta ? a->n_value : (a->n_bound > 0 && a->n_bound < a->n_max ? a->n_bound : a->n_max);
+    p.priv = p.mixers && !p.huffman && n_known >= PRIV_MIN_KEYS && (bins <= 255 || (bins == 256 && p.G >= 3));
     return 0;
 }
 
@@ -3060,17 +3419,19 @@ extern "C" int skml_compress_sparse(const SkmlCompressArgs* a, void* stream) {
     int grid = 0;
     int rc = fill_params(a, p, grid);
     if (rc) return rc;
-    static LaunchCache cache[4];
+    static LaunchCache cache[6];
     const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE, huffman = p.huffman != 0;
-    const bool fused = a->fused != 0;
+    const bool fused = a->fused != 0, priv = fused && !huffman && p.priv;
     cudaStream_t st = (cudaStream_t)stream;
     if (adaptive && huffman)
-        return launch_stages(compress_sparse_kernel<true, true, true>, compress_sparse_kernel<false, true, true>, cache[3], p, grid, fused, 8, st);
-    if (adaptive)
-        return launch_stages(compress_sparse_kernel<true, true, false>, compress_sparse_kernel<false, true, false>, cache[2], p, grid, fused, 8, st);
+        return launch_stages(compress_sparse_kernel<true, true, true, false>, compress_sparse_kernel<false, true, true, false>, cache[3], p, grid, fused, 8, st);
     if (huffman)
-        return launch_stages(compress_sparse_kernel<true, false, true>, compress_sparse_kernel<false, false, true>, cache[1], p, grid, fused, 8, st);
-    return launch_stages(compress_sparse_kernel<true, false, false>, compress_sparse_kernel<false, false, false>, cache[0], p, grid, fused, 8, st);
+        return launch_stages(compress_sparse_kernel<true, false, true, false>, compress_sparse_kernel<false, false, true, false>, cache[1], p, grid, fused, 8, st);
+    if (adaptive)
+        return priv ? launch_stages(compress_sparse_kernel<true, true, false, true>, compress_sparse_kernel<false, true, false, false>, cache[5], p, grid, fused, 8, st)
+                    : launch_stages(compress_sparse_kernel<true, true, false, false>, compress_sparse_kernel<false, true, false, false>, cache[2], p, grid, fused, 8, st);
+    return priv ? launch_stages(compress_sparse_kernel<true, false, false, true>, compress_sparse_kernel<false, false, false, false>, cache[4], p, grid, fused, 8, st)
+                : launch_stages(compress_sparse_kernel<true, false, false, false>, compress_sparse_kernel<false, false, false, false>, cache[0], p, grid, fused, 8, st);
 }
 
 extern "C" int skml_compress_dense(const SkmlCompressArgs* a, void* stream) {

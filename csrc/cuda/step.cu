@@ -15,9 +15,9 @@ static int batch_consumed(const SkmlStepArgs* a, cudaStream_t stream) {
 }
 
 // The gradient's way into the model: through the fused compress and decode kernels, or through a baseline's codes.
-// `batch_keys`: keys and count lie in the batch's own buffers, which are the feeder's again once they are read.
-static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* meta, float* vals, float* dense_vals, bool batch_keys,
-                          void* stream) {
+// `n_bound`: as many non-zeros at most. `batch_keys`: keys and count lie in the batch's own buffers, which are the feeder's again once they are read.
+static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* meta, float* vals, float* dense_vals, long long n_bound,
+                          bool batch_keys, void* stream) {
     if (a->coded) {
         const SkmlCodedArgs& c = *a->coded;
         int rc = 0;
@@ -39,6 +39,7 @@ static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* met
     a->compress->step = a->step;
     a->compress->keys = keys;
     a->compress->meta = meta;
+    a->compress->n_bound = n_bound;
     a->compress->vals = vals;
     if (dense_vals) a->compress->dense_vals = dense_vals;   // one launch serves both kinds
     int rc = skml_compress_sparse(a->compress, stream);
@@ -80,7 +81,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         if (rc) return rc;
         rc = batch_consumed(a, stream);
         if (rc) return rc;
-        return apply_gradient(a, a->t_ucols, a->t_meta, a->gvals, nullptr, false, stream_);
+        return apply_gradient(a, a->t_ucols, a->t_meta, a->gvals, nullptr, a->t_cols, false, stream_);
     }
     if (a->l_ucols) {
         if (a->coded) return (int)cudaErrorInvalidValue;   // the sketch arm's alone
@@ -99,7 +100,7 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
         }
         rc = skml_finalize_compact(a->gc, a->wc, (float)a->lambda, n, a->gvals, nullptr, stream_);  // no touched bitmap: every slot is a key
         if (rc) return rc;
-        return apply_gradient(a, a->l_ucols, a->l_meta, a->gvals, nullptr, true, stream_);
+        return apply_gradient(a, a->l_ucols, a->l_meta, a->gvals, nullptr, a->l_ncols, true, stream_);
     }
     if (a->dense_index) {
         int rc = skml_dt_gradient(a->dense_index, a->rowptr, a->cols, a->vals, a->labels, a->seg_lo[0], a->nnz_padded, a->avg_nnz, a->w,
@@ -119,5 +120,5 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
     rc = skml_compact_settle(a->g, a->w, a->bitmap, (int)a->dim, (float)a->lambda, a->block_counts, a->meta, a->keys,
                           a->gvals, a->dense_vals, a->n_max, a->status, a->partials, a->partials_template, stream_);
     if (rc) return rc;
-    return apply_gradient(a, a->keys, a->meta, a->gvals, a->dense_vals, false, stream_);
+    return apply_gradient(a, a->keys, a->meta, a->gvals, a->dense_vals, a->n_max, false, stream_);
 }

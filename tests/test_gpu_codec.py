@@ -717,6 +717,38 @@ def test_checked_calls_leave_their_results_to_any_stream(dense):
         assert torch.equal(got, want) and torch.equal(got_sum, want_sum)
 
 
+@pytest.mark.parametrize("encoder", ["delta_binary", "delta_adaptive"])
+@pytest.mark.parametrize("n,q,G,rows,ratio,levels", [
+    (999_999, 256, 8, 3, 0.2, 0), (1_000_000, 256, 8, 3, 0.2, 0), (1_000_003, 64, 20, 1, 0.05, 0),   # around the smallest size
+    (1_000_001, 255, 1, 3, 0.1, 0), (1_000_001, 256, 2, 2, 0.3, 0),   # most buckets in a group; one too many
+    (1_100_001, 256, 3, 2, 0.001, 0), (1_200_000, 64, 2, 3, 0.45, 0),   # tiny tables; rows of a table in two parts
+    (1_200_000, 64, 1, 2, 0.6, 0),                                     # in six: left to the atomics
+    (1_000_000, 256, 8, 3, 0.2, 3), (1_000_000, 256, 32, 3, 0.2, 1)])   # few distinct values: empty groups
+def test_sketch_inserted_in_shared_memory(n, q, G, rows, ratio, levels, encoder):
+    """Large gradients insert into tables in shared memory; the tables equal the oracle's, and the whole payload that of
+    the staged launches, which insert with atomics."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import GpuCompressor
+    dim = 3 * n
+    keys, vals = _sparse_grad(n, dim, seed=n + q)
+    if levels:
+        vals = (np.arange(n) % levels + 1).astype(np.float32) * np.where(np.arange(n) % 5 < 2, -1, 1).astype(np.float32)
+    kt, vt = torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda()
+    comps = [GpuCompressor(dim, n, q, G, rows, ratio, seed=11, fused=fused, key_encoder=encoder) for fused in (True, False)]
+    own = [c.payload_bytes(c.compress_local(kt, vt, step=3)) for c in comps]
+    assert own[0] == own[1]
+    qz = oracle.quantile_quantize(vals, q, 128, 1, 2, False)
+    splits = qz["splits"].astype(np.float32)
+    opts = dict(bin_num=q, group_num=G, row_num=rows, col_ratio=ratio, seed=11, step=7, rank=0, world=1, tie_mode=1,
+                key_encoder=1 if encoder == "delta_adaptive" else 0)
+    ref = oracle.parse(oracle.compress_sparse(keys, vals, dim, opts, splits, float(qz["min"]), float(qz["max"])))
+    buf = comps[0].compress_local(kt, vt, step=7, given=(torch.from_numpy(splits).cuda(), qz["min"], qz["max"]))
+    got = oracle.parse(comps[0].payload_bytes(buf))
+    for gi, (a, b) in enumerate(zip(_sections(got), _sections(ref))):
+        for fi, (x, y) in enumerate(zip(a, b)):
+            assert x == y, f"group {gi} field {fi} differs"
+
+
 @pytest.mark.parametrize("n", [8191, 8192, 8193, 148 * 8192, 148 * 8192 + 1, 2_500_003])
 @pytest.mark.parametrize("gaps", ["ones", "mixed", "wide"])
 def test_delta_adaptive_device_codec_over_tiles_and_runs(n, gaps):
