@@ -198,6 +198,26 @@ int skml_colsum_settle(const int* colptr, const int* rowidx, const float* svals,
 int skml_compact_settle(float* g, const float* w, unsigned int* bitmap, int dim, float lambda, unsigned int* block_counts,
                         long long* meta, int* keys, float* vals, float* dense_vals, long long capacity, unsigned int* status,
                         double* partials, double* tmpl, void* stream);
+// Frequent columns of a batch with a transposed index, as lists per (row tile, item): `pos` are their positions in the
+// index, column h has the items item0[h] .. item0[h + 1] (64 entries of a tile at most to each), ptr the lists' bounds in
+// quads of four entries (row_tiles * items + 1 of them), loc and val as in SkmlDenseIndex. skml_hot_count counts the entries per (row tile, column), skml_hot_fill puts them into their lists
+// (loc filled with tile_rows, val with 0 before), skml_hot_colsum leaves all column sums as skml_colsum_settle does:
+// the other columns, n_short of at most four entries and n_medium longer ones in `bins`, are summed from the index. `partial`: scratch of row_tiles * items floats.
+typedef struct SkmlHotColumns {
+    long long rows, row_tiles, tile_rows, columns, items, wide;
+    const int* pos;
+    const int* item0;
+    const int* info;        // [columns][4]: place among the index's columns, first item, items, column
+    const int* wide_info;   // [wide][4]: the same of the columns of several items
+    const int* ptr;
+    unsigned short* loc;
+    float* val;
+    float* partial;
+} SkmlHotColumns;
+int skml_hot_count(const SkmlHotColumns* hot, const int* colptr, const int* rowidx, int* cnt, void* stream);
+int skml_hot_fill(const SkmlHotColumns* hot, const int* colptr, const int* rowidx, const float* svals, void* stream);
+int skml_hot_colsum(const SkmlHotColumns* hot, const int* bins, int n_short, int n_medium, const int* colptr, const int* rowidx,
+                    const float* svals, const int* ucols, const float* coef, const float* w, float lambda, float* out, double* partials, double* tmpl, void* stream);
 int skml_gather_compact(const float* w, const int* ucols, int n, float* wc, void* stream);
 int skml_finalize_compact(float* gc, const float* wc, float lambda, int n, float* vals, unsigned int* bitmap,
                           void* stream);
@@ -361,6 +381,7 @@ typedef struct SkmlStepArgs {
     float* tt_partial;                 // device scratch [>= pairs]
     long long tt_tiles, tt_tile_rows, tt_rows;
     const SkmlDenseIndex* dense_index; // near-dense batch (null = not one): the gradient comes from its tiled copies
+    const SkmlHotColumns* hot_columns; // frequent columns of the transposed index (null = all by their lists of rows)
     const SkmlCodedArgs* coded;        // baseline compressor (null = compress and decode above)
 } SkmlStepArgs;
 

@@ -74,9 +74,13 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
                                      (int)a->loss_id, (float)a->inv_batch, loss, a->coef, a->gvals, a->t_long_col, (int)a->t_long,
                                      stream_);
             if (rc) return rc;
-            rc = skml_colsum_settle(a->t_colptr, a->t_rowidx, a->t_vals, a->t_ucols, a->t_bins, a->t_long_col, a->t_long_e0,
-                                    a->t_long_e1, (int)a->t_short, (int)a->t_medium, (int)a->t_long, a->coef, a->w,
-                                    (float)a->lambda, a->gvals, a->partials, a->partials_template, stream_);
+            if (a->hot_columns)
+                rc = skml_hot_colsum(a->hot_columns, a->t_bins, (int)a->t_short, (int)a->t_medium, a->t_colptr, a->t_rowidx,
+                                     a->t_vals, a->t_ucols, a->coef, a->w, (float)a->lambda, a->gvals, a->partials, a->partials_template, stream_);
+            else
+                rc = skml_colsum_settle(a->t_colptr, a->t_rowidx, a->t_vals, a->t_ucols, a->t_bins, a->t_long_col, a->t_long_e0,
+                                        a->t_long_e1, (int)a->t_short, (int)a->t_medium, (int)a->t_long, a->coef, a->w,
+                                        (float)a->lambda, a->gvals, a->partials, a->partials_template, stream_);
         }
         if (rc) return rc;
         rc = batch_consumed(a, stream);

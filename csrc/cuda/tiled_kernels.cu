@@ -192,37 +192,26 @@ __device__ __forceinline__ int weighted_bound(const int* __restrict__ ptr, int l
     return lo;
 }
 
-// partial[tile * items + item] = sum over the list of x[tile * T + loc] * val.
-// Blocks of a tile, and the warps of a block, share its lists by quads + lists, cut at whole groups of 32.
-// What bounds it: reading the lists (7 bytes an entry with padding). List by list a lane's loads were 20 and 40 bytes
-// from its neighbour's, and the passes they took through L1 were the limit: 160 us for 100M entries, 149 with the next
-// round's lists on their way into L2, 144 us (4.9 TB/s) with the lists interleaved (dt_interleave_kernel).
-template <bool HAS_VALS>
-__global__ void __launch_bounds__(DT_THREADS, 1)
-dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, int blocks_per_tile, const int* __restrict__ ptr,
-                  const ushort4* __restrict__ loc, const float4* __restrict__ val, float* __restrict__ partial) {
-    extern __shared__ __align__(16) float s_x[];
-    __shared__ int s_cut[DT_THREADS / 32 + 1];
+// Shares of a tile's lists [p0, p1) of block `sub` of `blocks`, one per warp, by quads + lists, cut at whole groups of 32:
+// warp w sums lists s_cut[w] to s_cut[w + 1].
+__device__ __forceinline__ void dt_cuts(const int* __restrict__ ptr, int p0, int p1, int sub, int blocks, int* s_cut) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = DT_THREADS / 32;
-    const int tile = blockIdx.x / blocks_per_tile, sub = blockIdx.x % blocks_per_tile;
-    const long long x0 = (long long)tile * T;
-    const int nx = n - x0 < T ? (int)(n - x0) : T;
-    for (int i = threadIdx.x; i < nx; i += DT_THREADS) s_x[i] = __ldg(x + x0 + i);
-    if (threadIdx.x == 0) s_x[T] = 0.f;   // the padding's slot
-    const int p0 = tile * items, p1 = p0 + items;
-    {
-        const long long base = ptr[p0], all = (long long)ptr[p1] - base + items;
-        const long long share = (long long)sub * warps + warp, shares = (long long)blocks_per_tile * warps;
-        auto group_start = [&](int p) { return p0 + ((p - p0) & ~31); };
-        const int cut = group_start(weighted_bound(ptr, p0, p1, base, all * share / shares));
-        if (lane == 0) s_cut[warp] = cut;
-        if (warp == warps - 1) {
-            const int end = sub + 1 == blocks_per_tile ? p1 : group_start(weighted_bound(ptr, p0, p1, base, all * (share + 1) / shares));
-            if (lane == 0) s_cut[warps] = end;
-        }
+    const long long base = ptr[p0], all = (long long)ptr[p1] - base + (p1 - p0);
+    const long long share = (long long)sub * warps + warp, shares = (long long)blocks * warps;
+    auto group_start = [&](int p) { return p0 + ((p - p0) & ~31); };
+    const int cut = group_start(weighted_bound(ptr, p0, p1, base, all * share / shares));
+    if (lane == 0) s_cut[warp] = cut;
+    if (warp == warps - 1) {
+        const int end = sub + 1 == blocks ? p1 : group_start(weighted_bound(ptr, p0, p1, base, all * (share + 1) / shares));
+        if (lane == 0) s_cut[warps] = end;
     }
-    __syncthreads();
-    const int w0 = s_cut[warp], w1 = s_cut[warp + 1];
+}
+
+// One warp's lists [w0, w1): partial[p] = sum over list p of s_x[loc] * val.
+template <bool HAS_VALS>
+__device__ __forceinline__ void dt_lists(const float* s_x, int T, int w0, int w1, const int* __restrict__ ptr, const ushort4* __restrict__ loc,
+                                         const float4* __restrict__ val, float* __restrict__ partial) {
+    const int lane = threadIdx.x & 31;
     auto quad = [&](const ushort4 l, const float4 v) {
         return HAS_VALS ? fmaf(s_x[l.x], v.x, fmaf(s_x[l.y], v.y, fmaf(s_x[l.z], v.z, s_x[l.w] * v.w)))
                         : (s_x[l.x] + s_x[l.y]) + (s_x[l.z] + s_x[l.w]);
@@ -296,6 +285,201 @@ dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, in
             if (lane == src) acc = part;
         }
         if (p < w1) partial[p] = acc;
+    }
+}
+
+// partial[tile * items + item] = sum over the list of x[tile * T + loc] * val.
+// Blocks of a tile, and the warps of a block, share its lists by quads + lists, cut at whole groups of 32.
+// What bounds it: reading the lists (7 bytes an entry with padding). List by list a lane's loads were 20 and 40 bytes
+// from its neighbour's, and the passes they took through L1 were the limit: 160 us for 100M entries, 149 with the next
+// round's lists on their way into L2, 144 us (4.9 TB/s) with the lists interleaved (dt_interleave_kernel).
+template <bool HAS_VALS>
+__global__ void __launch_bounds__(DT_THREADS, 1)
+dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, int blocks_per_tile, const int* __restrict__ ptr,
+                  const ushort4* __restrict__ loc, const float4* __restrict__ val, float* __restrict__ partial) {
+    extern __shared__ __align__(16) float s_x[];
+    __shared__ int s_cut[DT_THREADS / 32 + 1];
+    const int tile = blockIdx.x / blocks_per_tile, warp = threadIdx.x >> 5;
+    const long long x0 = (long long)tile * T;
+    const int nx = n - x0 < T ? (int)(n - x0) : T;
+    for (int i = threadIdx.x; i < nx; i += DT_THREADS) s_x[i] = __ldg(x + x0 + i);
+    if (threadIdx.x == 0) s_x[T] = 0.f;   // the padding's slot
+    dt_cuts(ptr, tile * items, (tile + 1) * items, blockIdx.x % blocks_per_tile, blocks_per_tile, s_cut);
+    __syncthreads();
+    dt_lists<HAS_VALS>(s_x, T, s_cut[warp], s_cut[warp + 1], ptr, loc, val, partial);
+}
+
+// ---------------------------------------------------------------------------
+// Column sums of a sparse batch with a transposed index (glm_kernels.cu): the frequent columns, which hold most entries,
+// from lists per (row tile, column) with the tile's coefficients in shared memory, all others one lane each with gathers
+// of the coefficients from L2. A list of the frequent columns holds at most HOT_SEGMENT entries, so that every group of
+// 32 lists is interleaved and no warp has much more than another: a column takes as many items as its fullest tile needs.
+// ---------------------------------------------------------------------------
+constexpr int HOT_SEGMENT = 4 * DT_LONG;
+
+__device__ __forceinline__ int rows_below(const int* __restrict__ rowidx, int e0, int e1, int row) {   // first entry of a row >= row
+    while (e0 < e1) {
+        const int mid = e0 + ((e1 - e0) >> 1);
+        if (rowidx[mid] < row) e0 = mid + 1;
+        else e1 = mid;
+    }
+    return e0;
+}
+
+// Entries per (row tile, frequent column).
+__global__ void __launch_bounds__(256)
+hot_count_kernel(const int* __restrict__ colptr, const int* __restrict__ rowidx, const int* __restrict__ pos, int columns, int T, int tiles,
+                 int* __restrict__ cnt) {
+    const long long all = (long long)tiles * columns;
+    for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < all; p += (long long)gridDim.x * 256) {
+        const int tile = (int)(p / columns), i = pos[p - (long long)tile * columns];
+        const int e0 = colptr[i], e1 = colptr[i + 1];
+        const int lo = rows_below(rowidx, e0, e1, tile * T), hi = tile + 1 == tiles ? e1 : rows_below(rowidx, lo, e1, (tile + 1) * T);
+        cnt[p] = hi - lo;
+    }
+}
+
+// The entries to their lists, a warp per (row tile, column): the rows of a column ascend.
+__global__ void __launch_bounds__(256)
+hot_fill_kernel(const int* __restrict__ colptr, const int* __restrict__ rowidx, const float* __restrict__ svals, const int* __restrict__ pos,
+                const int* __restrict__ item0, int columns, int items, int T, int tiles, const int* __restrict__ ptr,
+                unsigned short* __restrict__ loc, float* __restrict__ val) {
+    const int lane = threadIdx.x & 31;
+    const long long all = (long long)tiles * columns;
+    for (long long p = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); p < all; p += (long long)gridDim.x * 8) {
+        const int tile = (int)(p / columns), h = (int)(p - (long long)tile * columns), i = pos[h];
+        const int e0 = colptr[i], e1 = colptr[i + 1];
+        const int lo = rows_below(rowidx, e0, e1, tile * T), hi = tile + 1 == tiles ? e1 : rows_below(rowidx, lo, e1, (tile + 1) * T);
+        const int* const lists = ptr + (long long)tile * items + item0[h];
+        for (int e = lo + lane; e < hi; e += 32) {
+            const int k = e - lo;
+            const long long at = 4ll * lists[k / HOT_SEGMENT] + k % HOT_SEGMENT;
+            loc[at] = (unsigned short)(rowidx[e] - tile * T);
+            if (svals) val[at] = svals[e];
+        }
+    }
+}
+
+struct ColdColumns {   // columns bins[0 .. n) of the index: the first n_short (at most four entries) one lane each, the others eight
+    const int* bins;
+    int n_short, n;
+    const int* colptr;
+    const int* rowidx;
+    const float* svals;
+    const int* ucols;
+};
+
+// The other columns. Positions two turns ahead, bounds one, up to four gathers of a lane in flight. Eight lanes read the
+// rows (and values) of a longer column together: one lane each, as for the short ones, took 143 instead of 97 us for the
+// launch at 1M rows of 30 values.
+template <bool HAS_VALS, int LANES>
+__device__ __forceinline__ void cold_columns(const ColdColumns& c, int first, int last, const float* __restrict__ coef, const float* __restrict__ w,
+                                             float lambda, float* __restrict__ out) {
+    const int sub = threadIdx.x & (LANES - 1), turn = (int)gridDim.x * (DT_THREADS / LANES), start = ((int)blockIdx.x * DT_THREADS + (int)threadIdx.x) / LANES;
+    int t = first + start;
+    auto position = [&](int k) { return k < last ? c.bins[k] : -1; };
+    int ni = position(t), mi = position(t + turn), n0 = 0, n1 = 0, nu = 0;
+    auto bounds = [&]() {
+        if (ni < 0) return;
+        n0 = c.colptr[ni];
+        n1 = c.colptr[ni + 1];
+        nu = c.ucols[ni];
+    };
+    bounds();
+    for (; t - (int)(threadIdx.x & 31) / LANES < last; t += turn) {   // (the whole warp)
+        const int i = ni, e0 = n0, e1 = i < 0 ? n0 : n1;
+        const float wv = i < 0 || sub ? 0.f : __ldg(w + nu);   // a random sector of the model: issued first
+        ni = mi;
+        mi = position(t + 2 * turn);
+        bounds();
+        float acc = 0.f;
+        for (int e = e0 + sub; e < e1; e += 4 * LANES) {
+            int r[4];
+            float x[4], v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                r[u] = e + u * LANES < e1 ? c.rowidx[e + u * LANES] : -1;
+                x[u] = HAS_VALS && e + u * LANES < e1 ? c.svals[e + u * LANES] : 1.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = r[u] >= 0 ? __ldg(coef + r[u]) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc = fmaf(v[u], x[u], acc);
+        }
+        if (LANES > 1) {
+            __syncwarp();
+#pragma unroll
+            for (int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+        }
+        if (i >= 0 && sub == 0) out[i] = acc + lambda * wv;
+    }
+}
+
+// Both kinds in one launch: the lists are bound by shared memory, the other columns by random sectors (one of the model
+// per column, most of them from DRAM), so half of the warps begin with either. 500,000 rows of 30: 22 us the lists, 54 the
+// others, 57 together; colsum_kernel, whose gathers of coefficients are random sectors for all columns, took 95. With
+// real values, 1M rows of 30: 97 against 141 (and 8 and 13 us for the sums of the partial sums).
+template <bool HAS_VALS>
+__global__ void __launch_bounds__(DT_THREADS, 1)
+hot_colsum_kernel(const float* __restrict__ coef, int rows, int T, int items, int blocks_per_tile, int listed, const int* __restrict__ ptr,
+                  const ushort4* __restrict__ loc, const float4* __restrict__ val, float* __restrict__ partial, ColdColumns cold,
+                  const float* __restrict__ w, float lambda, float* __restrict__ out) {
+    extern __shared__ __align__(16) float s_x[];
+    __shared__ int s_cut[DT_THREADS / 32 + 1];
+    const int tile = blockIdx.x / blocks_per_tile, warp = threadIdx.x >> 5;
+    if ((int)blockIdx.x < listed) {   // (blocks beyond the tiles' shares have cold columns only)
+        const int x0 = tile * T, nx = rows - x0 < T ? rows - x0 : T;
+        for (int i = threadIdx.x; i < nx; i += DT_THREADS) s_x[i] = __ldg(coef + x0 + i);
+        if (threadIdx.x == 0) s_x[T] = 0.f;   // the padding's slot
+        dt_cuts(ptr, tile * items, (tile + 1) * items, blockIdx.x % blocks_per_tile, blocks_per_tile, s_cut);
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int phase = 0; phase < 2; ++phase) {
+        if (phase == (warp & 1)) {
+            if ((int)blockIdx.x < listed) dt_lists<HAS_VALS>(s_x, T, s_cut[warp], s_cut[warp + 1], ptr, loc, val, partial);
+        } else {
+            cold_columns<HAS_VALS, 8>(cold, cold.n_short, cold.n, coef, w, lambda, out);
+            cold_columns<HAS_VALS, 1>(cold, 0, cold.n_short, coef, w, lambda, out);
+        }
+    }
+}
+
+// Frequent columns from their partial sums, info[h] = {place in out, first item, items, column}: a lane per column of one
+// item, a block per column of several (`wide`).
+__global__ void __launch_bounds__(256)
+hot_combine_kernel(const float* __restrict__ partial, int columns, int items, int tiles, const int4* __restrict__ info, const int4* __restrict__ wide,
+                   int lane_blocks, const float* __restrict__ w, float lambda, float* __restrict__ out, StepLoss loss) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) loss.settle();
+    if ((int)blockIdx.x < lane_blocks) {
+        const int h = blockIdx.x * 256 + threadIdx.x;
+        if (h >= columns) return;
+        const int4 q = info[h];
+        if (q.z > 1) return;
+        const float wv = __ldg(w + q.w);
+        float v = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < tiles; ++t) v += partial[(long long)t * items + q.y];
+        out[q.x] = v + lambda * wv;
+        return;
+    }
+    __shared__ float s_part[8];
+    const int4 q = wide[blockIdx.x - lane_blocks];
+    const float wv = threadIdx.x == 0 ? __ldg(w + q.w) : 0.f;
+    float v = 0.f;
+    const int all = tiles * q.z;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < all; k += 256) {
+        const int t = k / q.z;
+        v += partial[(long long)t * items + q.y + (k - t * q.z)];
+    }
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float sum = 0.f;
+        for (int k = 0; k < 8; ++k) sum += s_part[k];
+        out[q.x] = sum + lambda * wv;
     }
 }
 
@@ -408,6 +592,19 @@ int dt_partial(const float* x, long long n, int T, int tiles, int items, const i
     return (int)cudaGetLastError();
 }
 
+void dt_interleave(const int* ptr, long long tiles, long long items, unsigned short* loc, float* val, cudaStream_t stream) {
+    const unsigned blocks = blocks_for(tiles * ((items + 31) / 32), DT_TURN_WARPS, 16);
+    ushort4* const l = reinterpret_cast<ushort4*>(loc);
+    float4* const v = reinterpret_cast<float4*>(val);
+    if (val) dt_interleave_kernel<true><<<blocks, DT_TURN_WARPS * 32, 0, stream>>>(ptr, (int)tiles, (int)items, l, v);
+    else dt_interleave_kernel<false><<<blocks, DT_TURN_WARPS * 32, 0, stream>>>(ptr, (int)tiles, (int)items, l, v);
+}
+
+bool hot_valid(const SkmlHotColumns* h) {
+    return h && h->rows > 0 && h->rows < (1ll << 31) && h->columns > 0 && h->items >= h->columns && h->tile_rows > 0 && h->tile_rows <= SKML_DT_TILE_MAX &&
+           h->row_tiles * h->tile_rows >= h->rows && h->row_tiles * h->items < SKML_DT_LISTS_MAX && h->wide >= 0;
+}
+
 bool dt_valid(const SkmlDenseIndex* d) {
     return d && d->rows > 0 && d->dim > 0 && d->rows < (1ll << 31) && d->dim < (1ll << 31) && d->tile_rows > 0 && d->tile_cols > 0 &&
            d->tile_rows <= SKML_DT_TILE_MAX && d->tile_cols <= SKML_DT_TILE_MAX && d->row_tiles * d->tile_rows >= d->rows &&
@@ -433,15 +630,8 @@ extern "C" int skml_dt_fill(const SkmlDenseIndex* d, const long long* rowptr, co
         rowptr, cols, vals, row_lo, (int)d->rows, (int)d->tile_rows, (int)d->row_tiles, (int)d->tile_cols, (int)d->col_tiles, (int)d->dim,
         (int)parts, d->c_ptr, cursor,
         d->c_loc, d->c_val, d->r_ptr, d->r_loc, d->r_val);
-    auto interleave = [&](const int* ptr, long long tiles, long long items, unsigned short* loc, float* val) {
-        const unsigned blocks = blocks_for(tiles * ((items + 31) / 32), DT_TURN_WARPS, 16);
-        ushort4* const l = reinterpret_cast<ushort4*>(loc);
-        float4* const v = reinterpret_cast<float4*>(val);
-        if (val) dt_interleave_kernel<true><<<blocks, DT_TURN_WARPS * 32, 0, (cudaStream_t)stream>>>(ptr, (int)tiles, (int)items, l, v);
-        else dt_interleave_kernel<false><<<blocks, DT_TURN_WARPS * 32, 0, (cudaStream_t)stream>>>(ptr, (int)tiles, (int)items, l, v);
-    };
-    interleave(d->c_ptr, d->row_tiles, d->dim, d->c_loc, d->c_val);
-    if (d->r_ptr) interleave(d->r_ptr, d->col_tiles, d->rows, d->r_loc, d->r_val);
+    dt_interleave(d->c_ptr, d->row_tiles, d->dim, d->c_loc, d->c_val, (cudaStream_t)stream);
+    if (d->r_ptr) dt_interleave(d->r_ptr, d->col_tiles, d->rows, d->r_loc, d->r_val, (cudaStream_t)stream);
     return (int)cudaGetLastError();
 }
 
@@ -466,5 +656,54 @@ extern "C" int skml_dt_gradient(const SkmlDenseIndex* d, const long long* rowptr
     if (rc) return rc;
     dt_sum_kernel<<<blocks_for(d->dim, 256, 8), 256, 0, stream>>>(d->partial, (int)d->dim, (int)d->row_tiles, (int)d->tile_rows, d->c_ptr,
                                                                   reinterpret_cast<const ushort4*>(d->c_loc), d->coef, g, bitmap);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int skml_hot_count(const SkmlHotColumns* h, const int* colptr, const int* rowidx, int* cnt, void* stream) {
+    if (!hot_valid(h) || !h->pos || !cnt) return (int)cudaErrorInvalidValue;
+    hot_count_kernel<<<blocks_for(h->row_tiles * h->columns, 256, 8), 256, 0, (cudaStream_t)stream>>>(
+        colptr, rowidx, h->pos, (int)h->columns, (int)h->tile_rows, (int)h->row_tiles, cnt);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int skml_hot_fill(const SkmlHotColumns* h, const int* colptr, const int* rowidx, const float* svals, void* stream) {
+    if (!hot_valid(h) || !h->pos || !h->item0 || !h->ptr || !h->loc || (svals != nullptr) != (h->val != nullptr)) return (int)cudaErrorInvalidValue;
+    hot_fill_kernel<<<blocks_for(h->row_tiles * h->columns, 8, 8), 256, 0, (cudaStream_t)stream>>>(
+        colptr, rowidx, svals, h->pos, h->item0, (int)h->columns, (int)h->items, (int)h->tile_rows, (int)h->row_tiles, h->ptr, h->loc, h->val);
+    dt_interleave(h->ptr, h->row_tiles, h->items, h->loc, h->val, (cudaStream_t)stream);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int skml_hot_colsum(const SkmlHotColumns* h, const int* bins, int n_short, int n_medium, const int* colptr, const int* rowidx, const float* svals,
+                               const int* ucols, const float* coef, const float* w, float lambda, float* out, double* partials, double* tmpl,
+                               void* stream_) {
+    if (!hot_valid(h) || !h->ptr || !h->loc || !h->partial || !h->info || n_short < 0 || n_medium < 0 || (svals != nullptr) != (h->val != nullptr)) return (int)cudaErrorInvalidValue;
+    cudaStream_t stream = (cudaStream_t)stream_;
+    static bool ready = false;
+    if (!ready) {
+        cudaError_t e = cudaFuncSetAttribute(hot_colsum_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (SKML_DT_TILE_MAX + 4));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(hot_colsum_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * (SKML_DT_TILE_MAX + 4));
+        if (e != cudaSuccess) return (int)e;
+        ready = true;
+    }
+    int bpt = dt_sms() / (int)h->row_tiles;
+    if (bpt < 1) bpt = 1;
+    const int listed = (int)h->row_tiles * bpt, grid = listed > dt_sms() ? listed : dt_sms();
+    const size_t smem = 4 * ((size_t)h->tile_rows + 4);
+    const ushort4* l = reinterpret_cast<const ushort4*>(h->loc);
+    const float4* v = reinterpret_cast<const float4*>(h->val);
+    const ColdColumns cold{bins, n_short, n_short + n_medium, colptr, rowidx, svals, ucols};
+    if (svals)
+        hot_colsum_kernel<true><<<grid, DT_THREADS, smem, stream>>>(coef, (int)h->rows, (int)h->tile_rows, (int)h->items, bpt, listed, h->ptr, l, v,
+                                                                   h->partial, cold, w, lambda, out);
+    else
+        hot_colsum_kernel<false><<<grid, DT_THREADS, smem, stream>>>(coef, (int)h->rows, (int)h->tile_rows, (int)h->items, bpt, listed, h->ptr, l, v,
+                                                                    h->partial, cold, w, lambda, out);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    const int lane_blocks = (int)((h->columns + 255) / 256);
+    hot_combine_kernel<<<(unsigned)(lane_blocks + h->wide), 256, 0, stream>>>(h->partial, (int)h->columns, (int)h->items, (int)h->row_tiles,
+                                                                           reinterpret_cast<const int4*>(h->info), reinterpret_cast<const int4*>(h->wide_info),
+                                                                           lane_blocks, w, lambda, out, StepLoss{partials, tmpl});
     return (int)cudaGetLastError();
 }

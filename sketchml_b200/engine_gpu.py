@@ -232,8 +232,9 @@ class GpuEngine:
         # 176 us + combine 92 us against 103 us), because the frequent columns, which hold most entries, already
         # gather near-sequential coefficients in the per-column form, and a 192 KB tile allows one block per SM.
         tiled = bool(conf.extras.get("tiled_index", False))
+        hot = need + csr.nnz * (9 if csr.values is not None else 3) <= 0.8 * free   # lists of the frequent columns beside
         for b in range(csr.rows // B if not dense else 0):
-            bi = build_batch_index(csr, b * B, (b + 1) * B, tiled=tiled)
+            bi = build_batch_index(csr, b * B, (b + 1) * B, tiled=tiled, hot=hot)
             if bi.n_cols > self.st.dim * 2 // 3 or bi.n_cols > self.st.n_max:
                 return  # near-dense without a tiled form (see build_dense_index): keep the scatter path
             idx.append(bi)
@@ -243,6 +244,11 @@ class GpuEngine:
             for di in idx:
                 di.bind(shared, coef)
             self._dense_partial = shared
+        elif any(bi.hot is not None for bi in idx):
+            shared = torch.empty(max(bi.hot.partial_floats for bi in idx if bi.hot is not None), dtype=torch.float32, device=self.device)
+            for bi in idx:
+                if bi.hot is not None:
+                    bi.hot.bind(shared)
         elif tiled:
             # one scratch for the partial sums of all batches (a step uses one batch's index at a time)
             shared = torch.zeros(max([bi.tiled.n_pairs for bi in idx if bi.tiled is not None] + [1]), dtype=torch.float32,
@@ -285,6 +291,7 @@ class GpuEngine:
                                                                 L.ptr(bi.long_e1))
             a.t_short, a.t_medium, a.t_long, a.t_cols = bi.n_short, bi.n_medium, bi.n_long, bi.n_cols
             a.t_meta, a.coef = L.ptr(bi.meta), L.ptr(self.coef)
+            a.hot_columns = self._ctypes.pointer(bi.hot.args) if bi.hot is not None else None
         else:
             a.t_colptr = a.tt_pair_ptr = None
         lid = getattr(csr, "lid", None) if bi is None else None
@@ -314,7 +321,7 @@ class GpuEngine:
         if lid is not None:
             L.count_launches(len(segs) + 2 + tail)  # gather, gradient segment(s), finalize
         else:
-            L.count_launches(((2 if bi.tiled is None else 3) if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + tail)
+            L.count_launches(((2 if bi.tiled is None and bi.hot is None else 3) if bi is not None else (len(segs) if di is None else (4 if di.args.r_ptr else 3)) + 2) + tail)
 
     # ----------------------------------------------------------------- steps
     def _segments(self, count: int):

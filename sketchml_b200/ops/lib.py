@@ -65,6 +65,13 @@ class DenseIndexArgs(C.Structure):
     ]
 
 
+class HotColumnsArgs(C.Structure):
+    _fields_ = [
+        ("rows", c_ll), ("row_tiles", c_ll), ("tile_rows", c_ll), ("columns", c_ll), ("items", c_ll), ("wide", c_ll),
+        ("pos", c_vp), ("item0", c_vp), ("info", c_vp), ("wide_info", c_vp), ("ptr", c_vp), ("loc", c_vp), ("val", c_vp), ("partial", c_vp),
+    ]
+
+
 class CodedArgs(C.Structure):
     _fields_ = [
         ("kind", c_ll), ("bits", c_ll), ("seed", c_ull), ("scratch", c_vp), ("scratch_bytes", c_ll), ("codes", c_vp),
@@ -88,7 +95,7 @@ class StepArgs(C.Structure):
         ("grad_done_event", c_vp),
         ("tt_tile_pair_ptr", c_vp), ("tt_pair_ptr", c_vp), ("tt_lrow", c_vp), ("tt_pair_dst", c_vp),
         ("tt_col_pair_ptr", c_vp), ("tt_partial", c_vp), ("tt_tiles", c_ll), ("tt_tile_rows", c_ll), ("tt_rows", c_ll),
-        ("dense_index", C.POINTER(DenseIndexArgs)), ("coded", C.POINTER(CodedArgs)),
+        ("dense_index", C.POINTER(DenseIndexArgs)), ("hot_columns", C.POINTER(HotColumnsArgs)), ("coded", C.POINTER(CodedArgs)),
     ]
 
 
@@ -125,6 +132,9 @@ _SIGS = {
     "skml_gen_rows": (c_int, [c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_d, c_int, c_int, c_f, c_vp, c_ull, c_vp]),
     "skml_glm_coef": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_ll, c_int, c_f, c_vp, c_vp, c_vp, c_ll, c_vp]),
     "skml_colsum": (c_int, [c_vp] * 8 + [c_int] * 4 + [c_vp, c_vp, c_f, c_vp, c_vp]),
+    "skml_hot_count": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_vp, c_vp, c_vp]),
+    "skml_hot_fill": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_vp, c_vp, c_vp]),
+    "skml_hot_colsum": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_f, c_vp, c_vp, c_vp, c_vp]),
     "skml_sm_count": (c_int, []),
     "skml_da_workspace_bytes": (c_ll, []),
     "skml_da_encode": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),

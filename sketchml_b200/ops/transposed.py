@@ -20,6 +20,8 @@ from .glm import DeviceCSR
 SHORT_MAX, MEDIUM_MAX, LONG_SEGMENT = 4, 512, 4096
 TILE_ROWS_MAX = 49152   # coefficients of one row tile in shared memory: 192 KB
 PAIR_SEGMENT = 256      # longest entry list behind one partial sum
+HOT_SEGMENT = 64        # entries of a tile's list of a frequent column
+HOT_MIN_ENTRIES = 8_000_000   # entries of the frequent columns from which on their lists pay (see `_hot_columns`)
 SEG_SLOTS = 256         # >= TILE_ROWS_MAX / PAIR_SEGMENT segments per (tile, column) pair
 
 
@@ -36,6 +38,22 @@ class TiledPart:
     pair_dst: torch.Tensor        # int32 [n_pairs]
     col_pair_ptr: torch.Tensor    # int32 [n_cols + 1]
     partial: Optional[torch.Tensor] = None   # float32 scratch [>= n_pairs]; may be shared between indices
+
+
+@dataclass
+class HotColumns:
+    """Frequent columns of a batch as lists per (row tile, item), with tile-local rows (csrc/cuda/tiled_kernels.cu)."""
+    args: L.HotColumnsArgs
+    tensors: List[torch.Tensor]    # what `args` points into
+    partial_floats: int            # scratch it needs
+
+    def nbytes(self) -> int:
+        return sum(t.numel() * t.element_size() for t in self.tensors)
+
+    def bind(self, partial: torch.Tensor) -> None:
+        """Scratch of a step; batches that run one after another share it."""
+        self.partial = partial
+        self.args.partial = partial.data_ptr()
 
 
 @dataclass
@@ -56,12 +74,14 @@ class BatchIndex:
     n_long: int
     meta: torch.Tensor        # int64 [4] = {n_cols, 1, 0, 0}
     tiled: Optional[TiledPart] = None   # when set, the per-column arrays above are empty
+    hot: Optional[HotColumns] = None    # when set, `bins` holds the other columns only, and no column is long
 
     def nbytes(self) -> int:
         ts = [self.colptr, self.rowidx, self.ucols, self.bins, self.long_col, self.long_e0, self.long_e1]
         if self.tiled is not None:
             ts += [self.tiled.tile_pair_ptr, self.tiled.pair_ptr, self.tiled.lrow, self.tiled.pair_dst, self.tiled.col_pair_ptr]
-        return sum(t.numel() * t.element_size() for t in ts) + (self.svals.numel() * 4 if self.svals is not None else 0)
+        return sum(t.numel() * t.element_size() for t in ts) + (self.svals.numel() * 4 if self.svals is not None else 0) + (
+            self.hot.nbytes() if self.hot is not None else 0)
 
 
 def _build_tiled(csr: DeviceCSR, lo: int, hi: int, e0: int, e1: int, rows: torch.Tensor) -> BatchIndex:
@@ -103,9 +123,48 @@ def _build_tiled(csr: DeviceCSR, lo: int, hi: int, e0: int, e1: int, rows: torch
                       torch.tensor([n, 1 if n else 0, 0, 0], dtype=torch.int64, device=dev), part)
 
 
-def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False) -> BatchIndex:
+def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor, svals: Optional[torch.Tensor], cnt: torch.Tensor, rows: int):
+    """The columns with at least two entries per row tile on average (and more than the short ones'), and which they are;
+    (None, None) where they hold too few entries to pay for tiles, partial sums and one more launch: column sums of 15M
+    entries 95 -> 65 us, of 30M with values 141 -> 110, of 6M with values 21 -> 26, of 1.9M 18 -> 23."""
+    dev, lib = rowidx.device, L.lib()
+    a = L.HotColumnsArgs()
+    a.rows = rows
+    a.row_tiles, a.tile_rows = _tiles(rows, TILE_ROWS_MAX)
+    is_hot = cnt >= max(SHORT_MAX + 1, 2 * a.row_tiles)
+    pos = torch.nonzero(is_hot).flatten().to(torch.int32)
+    a.columns = pos.numel()
+    if int(cnt[pos.long()].sum()) < HOT_MIN_ENTRIES:
+        return None, None
+    a.items = a.columns
+    a.pos = L.ptr(pos)
+    per = torch.empty((a.row_tiles, a.columns), dtype=torch.int32, device=dev)
+    L.check(lib.skml_hot_count(C.byref(a), L.ptr(colptr), L.ptr(rowidx), L.ptr(per), L.stream()), "skml_hot_count")
+    k = (per.amax(0) + HOT_SEGMENT - 1) // HOT_SEGMENT
+    item0 = torch.zeros(a.columns + 1, dtype=torch.int32, device=dev)
+    torch.cumsum(k, 0, dtype=torch.int32, out=item0[1:])
+    info = torch.stack([pos, item0[:-1], k, ucols[pos.long()].to(torch.int32)], 1).contiguous()
+    wide = info[k > 1].contiguous()
+    a.items, a.wide = int(item0[-1]), wide.shape[0]
+    if a.row_tiles * a.items + rowidx.numel() // 4 >= L.DT_LISTS_MAX:
+        return None, None
+    column = torch.repeat_interleave(torch.arange(a.columns, device=dev), k, output_size=a.items)
+    segment = torch.arange(a.items, device=dev, dtype=torch.int32) - item0[column]
+    quads = ((per[:, column] - HOT_SEGMENT * segment).clamp_(0, HOT_SEGMENT) + 3) >> 2
+    ptr = torch.zeros(a.row_tiles * a.items + 1, dtype=torch.int32, device=dev)
+    torch.cumsum(quads.flatten(), 0, dtype=torch.int32, out=ptr[1:])
+    n = 4 * int(ptr[-1])
+    loc = torch.full((n,), a.tile_rows if a.tile_rows < 32768 else a.tile_rows - 65536, dtype=torch.int16, device=dev)   # unsigned 16-bit patterns
+    val = None if svals is None else torch.zeros(n, dtype=torch.float32, device=dev)
+    a.item0, a.info, a.wide_info, a.ptr, a.loc, a.val = L.ptr(item0), L.ptr(info), L.ptr(wide), L.ptr(ptr), L.ptr(loc), L.ptr(val)
+    L.check(lib.skml_hot_fill(C.byref(a), L.ptr(colptr), L.ptr(rowidx), L.ptr(svals), L.stream()), "skml_hot_fill")
+    return HotColumns(a, [pos, item0, info, wide, ptr, loc] + ([val] if val is not None else []), int(a.row_tiles * a.items)), is_hot
+
+
+def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False, hot: bool = False) -> BatchIndex:
     """``tiled``: the row-tiled form (coefficients of a row tile in shared memory, no atomics); needs fewer than
-    2^20 tiles, i.e. any batch that fits a GPU."""
+    2^20 tiles, i.e. any batch that fits a GPU. ``hot``: the frequent columns of the per-column form as lists per row
+    tile, where that pays (see `_hot_columns`)."""
     dev = csr.cols.device
     e0, e1 = int(csr.rowptr[lo]), int(csr.rowptr[hi])
     cols = csr.cols[e0:e1]
@@ -121,6 +180,12 @@ def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False) -> 
     colptr = torch.zeros(n + 1, dtype=torch.int32, device=dev)
     colptr[1:] = torch.cumsum(cnt, 0).to(torch.int32)
     pos = torch.arange(n, device=dev, dtype=torch.int32)
+    frequent, is_hot = _hot_columns(ucols, colptr, rowidx, svals, cnt, hi - lo) if hot and n else (None, None)
+    if frequent is not None:
+        none = torch.zeros(0, dtype=torch.int32, device=dev)
+        short, medium = pos[cnt <= SHORT_MAX], pos[(cnt > SHORT_MAX) & ~is_hot]
+        return BatchIndex(lo, hi - lo, n, colptr, rowidx, svals, ucols.to(torch.int32).contiguous(), torch.cat([short, medium]).contiguous(),
+                          none, none, none, int(short.numel()), int(medium.numel()), 0, torch.tensor([n, 1, 0, 0], dtype=torch.int64, device=dev), hot=frequent)
     short = pos[cnt <= SHORT_MAX]
     medium = pos[(cnt > SHORT_MAX) & (cnt <= MEDIUM_MAX)]
     longs = pos[cnt > MEDIUM_MAX]
@@ -246,6 +311,14 @@ def glm_grad_transposed(csr: DeviceCSR, bi: BatchIndex, w: torch.Tensor, coef: t
                                       L.ptr(tp.pair_dst), L.ptr(tp.col_pair_ptr), L.ptr(bi.ucols), bi.rows, tp.tile_rows,
                                       tp.n_tiles, bi.n_cols, L.ptr(coef), L.ptr(w), float(lam), L.ptr(tp.partial),
                                       L.ptr(out_vals), L.stream()), "skml_colsum_tiled")
+        L.count_launches(3)
+        return
+    if bi.hot is not None:
+        if not bi.hot.args.partial:
+            bi.hot.bind(torch.empty(bi.hot.partial_floats, dtype=torch.float32, device=coef.device))
+        L.check(lib.skml_hot_colsum(C.byref(bi.hot.args), L.ptr(bi.bins), bi.n_short, bi.n_medium, L.ptr(bi.colptr), L.ptr(bi.rowidx),
+                                    L.ptr(bi.svals), L.ptr(bi.ucols), L.ptr(coef), L.ptr(w), float(lam), L.ptr(out_vals), None, None,
+                                    L.stream()), "skml_hot_colsum")
         L.count_launches(3)
         return
     L.check(lib.skml_colsum(L.ptr(bi.colptr), L.ptr(bi.rowidx), L.ptr(bi.svals), L.ptr(bi.ucols), L.ptr(bi.bins),

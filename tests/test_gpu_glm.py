@@ -504,3 +504,51 @@ def test_near_dense_index_touches_the_columns_the_scatter_touches(rows, dim, nnz
     assert 0 < int(torch.count_nonzero(got[0][0])) and got[0][2] == got[1][2]
     # a value next to the filter's 1e-8 may fall on either side of it: sums of at most n terms in varying order
     assert abs(got[0][1] - got[1][1]) <= 2
+
+
+@pytest.mark.parametrize("binary", [True, False])
+@pytest.mark.parametrize("rows,tile_rows_max,zipf", [(300, 64, 1.3), (2000, 512, 1.1), (5003, 1000, 1.1), (9001, 49152, 1.3), (60000, 49152, 1.1)])
+def test_frequent_columns_from_row_tiles_match_the_per_column_form(binary, rows, tile_rows_max, zipf, monkeypatch):
+    """Columns of one item and of many (a column in every row), tiles with ragged ends and lists that end inside a quad;
+    same keys, sums equal up to the order of the adds, the same bits on every repetition."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.models.loss import L2LogLoss
+    from sketchml_b200.ops import DeviceCSR, GlmState
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T, "TILE_ROWS_MAX", tile_rows_max)
+    monkeypatch.setattr(T, "HOT_MIN_ENTRIES", 1)
+    dev = torch.device("cuda")
+    loss = L2LogLoss(1e-3)
+    dim, rng = 30000, np.random.default_rng(rows)
+    per = [np.unique(np.minimum(rng.zipf(zipf, rng.integers(1, 40)) - 1, dim - 1)) for _ in range(rows + 500)]
+    per = [np.unique(np.concatenate([[3], p])) for p in per]      # column 3 is in every row
+    rowptr = np.concatenate([[0], np.cumsum([len(p) for p in per])])
+    cols = np.concatenate(per).astype(np.int32)
+    vals = None if binary else torch.from_numpy(rng.normal(size=len(cols)).astype(np.float32))
+    m = CSRMatrix(torch.from_numpy(rowptr), torch.from_numpy(cols), vals, torch.from_numpy(np.where(rng.random(rows + 500) < 0.5, 1.0, -1.0).astype(np.float32)), dim)
+    csr = DeviceCSR(m, dev)
+    w = (torch.randn(dim) * 0.3).float().to(dev)
+    st = GlmState.create(dim, dim, dev)
+    lo, hi = 250, 250 + rows
+    plain, hot = T.build_batch_index(csr, lo, hi), T.build_batch_index(csr, lo, hi, hot=True)
+    assert hot.hot is not None and (hot.hot.args.wide >= 1 or tile_rows_max <= T.HOT_SEGMENT) and torch.equal(plain.ucols, hot.ucols)
+    assert hot.n_short + hot.n_medium + hot.hot.args.columns == hot.n_cols
+    coef = torch.zeros((rows + 3) // 4 * 4, device=dev)
+    outs = []
+    for bi in (plain, hot, hot):
+        out = torch.full((dim,), 7.0, device=dev)
+        st.partials.zero_()
+        T.glm_grad_transposed(csr, bi, w, coef, out, st.partials, st.status, loss.loss_id, loss.lam)
+        assert int(st.status.item()) == 0
+        outs.append(out[:bi.n_cols].clone())
+    assert torch.equal(outs[1], outs[2])
+    # the coefficients are at most 1 / rows in size: a sum of n products in any order is within n * 2^-24 * sum |terms|
+    r_of = torch.repeat_interleave(torch.arange(rows, device=dev), csr.rowptr[lo + 1:hi + 1] - csr.rowptr[lo:hi])
+    e0, e1 = int(csr.rowptr[lo]), int(csr.rowptr[hi])
+    x = torch.ones(e1 - e0, device=dev, dtype=torch.float64) if binary else csr.values[e0:e1].double()
+    exact = torch.zeros(dim, device=dev, dtype=torch.float64).index_add_(0, csr.cols[e0:e1].long(), coef[r_of].double() * x)
+    size = torch.zeros(dim, device=dev, dtype=torch.float64).index_add_(0, csr.cols[e0:e1].long(), (coef[r_of].double() * x).abs())
+    uc = hot.ucols.long()
+    want = exact[uc] + loss.lam * w[uc].double()
+    bound = 2 ** -20 * (size[uc] + loss.lam * w[uc].double().abs()) + 1e-12
+    assert bool(((outs[1].double() - want).abs() <= bound).all())
