@@ -25,7 +25,7 @@ static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* met
             rc = skml_fixedpoint_pack(vals, meta, a->n_max, (int)c.bits, c.seed, (double*)c.scratch, c.codes, c.norm, stream);
             if (!rc) rc = skml_fixedpoint_unpack_scatter(nullptr, keys, c.codes, c.norm, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals, stream);
         } else if (c.kind == 2) {
-            rc = skml_zipml_pack(vals, meta, a->n_max, (int)c.bits, c.scratch, c.scratch_bytes, c.splits, c.mids, c.zip_meta, c.range, c.codes,
+            rc = skml_zipml_pack(vals, meta, n_bound > 0 && n_bound < a->n_max ? n_bound : a->n_max, (int)c.bits, c.scratch, c.scratch_bytes, c.splits, c.mids, c.zip_meta, c.range, c.codes,
                                  a->status, stream);
             if (!rc) rc = skml_zipml_unpack_scatter(nullptr, keys, c.codes, c.mids, meta, a->n_max, c.code_stride, 1, (int)c.bits, vals,
                                                     a->status, stream);

@@ -771,3 +771,18 @@ def test_delta_adaptive_device_codec_over_tiles_and_runs(n, gaps):
         assert np.array_equal(o["flag_words"], np.asarray(ref["flag_words"], dtype=np.uint64))
         assert np.array_equal(o["delta_words"], np.asarray(ref["delta_words"], dtype=np.uint64))
         assert np.array_equal(K.decode(got).cpu().numpy(), keys)
+
+
+@pytest.mark.parametrize("n", [4059, 4060, 16384 + 5, 148 * 4096 - 37, 148 * 4096 - 36, 148 * 8192 - 37, 148 * 8192 - 36])
+def test_zipml_sort_over_its_blocks(n):
+    """One block, two, a ragged slice, every block with four and then more values a thread, the largest size and the first
+    beyond it (values on a dyadic grid: the search must pick the oracle's very split points; signed zeros among them)."""
+    from sketchml_b200.compress import oracle
+    rng = np.random.default_rng(n)
+    vals = (rng.integers(-30000, 30000, n) / 1024.0).astype(np.float32)
+    vals[rng.random(n) < 0.01] *= 0.0      # both zeros
+    ref = oracle.zipml_quantize(vals.astype(np.float64), 256)
+    _, _, _, nb, zero, _, splits, mids, codes = _zip_pack(vals, 256)
+    assert nb == ref["bin_num"] and zero == ref["zero_idx"]
+    assert np.array_equal(splits.astype(np.float64), ref["splits"])
+    assert np.array_equal(mids, ref["values"].astype(np.float32)) and np.array_equal(codes, ref["bins"])
