@@ -2997,6 +2997,7 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
 // keys for the insert in shared memory (its code costs the others 2 us).
 template <bool FUSED, bool ADAPTIVE, bool HUFFMAN, bool PRIV>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, int stage) {
+    skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     unsigned int passed = 0;   // arrivals of the grid barriers so far
@@ -3199,6 +3200,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
 
 template <bool FUSED>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int stage) {
+    skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if ((p.meta ? p.meta[1] : p.kind_value) != SKML_KIND_DENSE) return;
     dense_stages<FUSED>(p, *reinterpret_cast<Smem*>(smem_raw), p.vals, stage);
@@ -3332,7 +3334,7 @@ static cudaError_t launch_ex(K kernel, int grid, int cluster, bool coop, const C
     cfg.blockDim = dim3(SKML_BLOCK);
     cfg.dynamicSmemBytes = sizeof(Smem);
     cfg.stream = stream;
-    cudaLaunchAttribute attrs[2];
+    cudaLaunchAttribute attrs[3];
     unsigned int na = 0;
     if (coop) {
         attrs[na].id = cudaLaunchAttributeCooperative;
@@ -3346,6 +3348,9 @@ static cudaError_t launch_ex(K kernel, int grid, int cluster, bool coop, const C
         attrs[na].val.clusterDim.z = 1;
         ++na;
     }
+    attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
     cfg.attrs = attrs;
     cfg.numAttrs = na;
     return cudaLaunchKernelEx(&cfg, kernel, p, stage);

@@ -806,6 +806,7 @@ __device__ void finish_norm(const DP& p, float dsq) {
 
 template <bool FUSED>
 __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_kernel(DP p, int stage) {
+    skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DecSmem& s = *reinterpret_cast<DecSmem*>(smem_raw);
     float dsq = 0.f;  // this thread's share of the change of ||w||^2
@@ -1011,10 +1012,7 @@ extern "C" int skml_decode_update(const SkmlDecodeArgs* a, void* stream_) {
     if (a->fused) {
         if (max_grid < 1) return (int)cudaErrorLaunchOutOfResources;
         if (grid > max_grid) grid = max_grid;
-        int stage = -1;
-        void* args[] = {&p, &stage};
-        return (int)cudaLaunchCooperativeKernel((const void*)decode_update_kernel<true>, dim3(grid), dim3(DEC_THREADS), args,
-                                                smem, stream);
+        return (int)skml_launch_as(true, decode_update_kernel<true>, (unsigned)grid, DEC_THREADS, smem, stream, p, -1);
     }
     // stages: Adam = accumulate + claims; SGD over several payloads with a value scratch = decode +
     // one apply pass per rank; otherwise one pass per rank

@@ -57,6 +57,7 @@ glm_scatter_kernel(const long long* __restrict__ rowptr, const int* __restrict__
                    const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
                    float* __restrict__ g, unsigned int* __restrict__ bitmap, int loss_id, float inv_batch, int hot, int priv,
                    double* __restrict__ acc) {
+    skml_after_previous();
     extern __shared__ __align__(16) float s_hot[];   // [hot], then [warps][priv]
     constexpr int LANES = 1 << GL, ROWS = 32 >> GL, PER = 4;
     const int lane = threadIdx.x & 31, sub = lane & (LANES - 1), grp = lane >> GL, nwarps = blockDim.x / 32;
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(MARGIN_THREADS, 3)
 glm_margin_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
                   const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
                   int hot, int loss_id, float inv_batch, double* __restrict__ acc, float* __restrict__ out, ClearSlots clear) {
+    skml_after_previous();
     extern __shared__ __align__(16) float s_w[];
     if (MODE == 2)   // what the column sums behind this launch add to
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < clear.n; i += gridDim.x * blockDim.x) clear.out[clear.slot[i]] = 0.f;
@@ -365,11 +367,11 @@ static int margin_launch_gl(const long long* rowptr, const int* cols, const floa
     const int iters = t.iters, warps = t.warps, grid = t.grid;
     const int hot = margin_hot((long long)(row_cnt * avg_nnz), grid, dim, w);
     if (vals)
-        glm_margin_kernel<MODE, GL, true><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
+        skml_launch(glm_margin_kernel<MODE, GL, true>, (unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream,
+                    rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
     else
-        glm_margin_kernel<MODE, GL, false><<<(unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream>>>(
-            rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
+        skml_launch(glm_margin_kernel<MODE, GL, false>, (unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream,
+                    rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
     return (int)cudaGetLastError();
 }
 
@@ -410,11 +412,11 @@ static int grad_launch_gl(const long long* rowptr, const int* cols, const float*
         attr_set = true;
     }
     if (vals)
-        glm_scatter_kernel<GL, true><<<t.grid, 32 * t.warps, smem, stream>>>(rowptr, cols, vals, labels, row_lo, row_cnt, t.iters, w, g,
-                                                                            bitmap, loss_id, inv_batch, hot, priv, acc);
+        skml_launch(glm_scatter_kernel<GL, true>, t.grid, 32 * t.warps, smem, stream, rowptr, cols, vals, labels, row_lo, row_cnt, t.iters, w, g,
+                    bitmap, loss_id, inv_batch, hot, priv, acc);
     else
-        glm_scatter_kernel<GL, false><<<t.grid, 32 * t.warps, smem, stream>>>(rowptr, cols, vals, labels, row_lo, row_cnt, t.iters, w, g,
-                                                                             bitmap, loss_id, inv_batch, hot, priv, acc);
+        skml_launch(glm_scatter_kernel<GL, false>, t.grid, 32 * t.warps, smem, stream, rowptr, cols, vals, labels, row_lo, row_cnt, t.iters, w, g,
+                    bitmap, loss_id, inv_batch, hot, priv, acc);
     return (int)cudaGetLastError();
 }
 
@@ -476,6 +478,7 @@ static CompactShape compact_shape(long long dim) {
 __global__ void __launch_bounds__(COMPACT_THREADS)
 compact_count_kernel(float* __restrict__ g, const float* __restrict__ w, unsigned int* __restrict__ bitmap,
                      long long nwords, int dim, float lambda, int wpw, int nwarps, unsigned int* __restrict__ warp_counts) {
+    skml_after_previous();
     // Words with few bits are walked by their own lane; words with many bits are walked by the whole
     // warp, one bit per lane, so that the g / w accesses of dense regions are coalesced. Loads are issued
     // in batches before any of them is consumed (several memory round trips in flight per warp).
@@ -578,6 +581,7 @@ compact_write_kernel(float* __restrict__ g, const float* __restrict__ w, unsigne
                      long long nwords, int dim, float lambda, int wpw, int nwarps,
                      const unsigned int* __restrict__ warp_counts, long long* __restrict__ meta, int* __restrict__ keys,
                      float* __restrict__ vals, float* __restrict__ dense_vals, long long capacity, unsigned int* status, StepLoss loss) {
+    skml_after_previous();
     __shared__ unsigned int s_before[COMPACT_WARPS], s_total[COMPACT_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gw0 = blockIdx.x * COMPACT_WARPS, gw = gw0 + warp;
@@ -721,9 +725,9 @@ static int compact_launch(float* g, const float* w, unsigned int* bitmap, int di
                           cudaStream_t stream, const StepLoss& loss = {nullptr, nullptr}) {
     const long long nwords = ((long long)dim + 31) / 32;
     const CompactShape c = compact_shape(dim);
-    compact_count_kernel<<<c.nblocks, COMPACT_THREADS, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts);
-    compact_write_kernel<<<c.nblocks, COMPACT_THREADS, 0, stream>>>(g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts,
-                                                                    meta, keys, vals, dense_vals, capacity, status, loss);
+    skml_launch(compact_count_kernel, c.nblocks, COMPACT_THREADS, 0, stream, g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts);
+    skml_launch(compact_write_kernel, c.nblocks, COMPACT_THREADS, 0, stream, g, w, bitmap, nwords, dim, lambda, c.wpw, c.nwarps, warp_counts,
+                meta, keys, vals, dense_vals, capacity, status, loss);
     return (int)cudaGetLastError();
 }
 
@@ -781,6 +785,7 @@ __global__ void update_dense_kernel(float* w, float* m, float* v, const float* g
 __global__ void update_sparse_kernel(float* w, float* m, float* v, const int* keys, const float* vals,
                                      const long long* n_ptr, long long n_max, float scale, int adam, float lr,
                                      float adam_scale, long long ms, const unsigned int* status) {
+    skml_after_previous();
     long long n = n_ptr ? *n_ptr : n_max;
     if (n > n_max) n = n_max;
     if (skml_failed(status)) n = 0;   // (read beside the count)
@@ -800,8 +805,8 @@ extern "C" int skml_update_sparse(float* w, float* m, float* v, const int* keys,
                                   const long long* n_ptr, long long n_max, float scale, int adam, float lr,
                                   float adam_scale, int adam_stride, const unsigned int* status, void* stream) {
     int grid = sm_count() * 8;
-    update_sparse_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(w, m, v, keys, vals, n_ptr, n_max, scale, adam, lr,
-                                                                 adam_scale, adam_stride > 1 ? adam_stride : 1, status);
+    skml_launch(update_sparse_kernel, grid, 256, 0, (cudaStream_t)stream, w, m, v, keys, vals, n_ptr, n_max, scale, adam, lr,
+                adam_scale, adam_stride > 1 ? adam_stride : 1, status);
     return (int)cudaGetLastError();
 }
 
@@ -812,6 +817,7 @@ constexpr int NORM_BLOCKS = 592;
 __global__ void __launch_bounds__(256) weight_norm_kernel(const float* __restrict__ w, long long dim, double lambda,
                                                           double* __restrict__ sumsq_out, double* __restrict__ reg_out,
                                                           double* __restrict__ partials, unsigned int* __restrict__ counter) {
+    skml_after_previous();
     const long long per = ((dim + gridDim.x - 1) / gridDim.x + 3) & ~3ll;
     const long long lo = per * blockIdx.x, hi = lo + per < dim ? lo + per : dim;
     double acc = 0.0;
@@ -861,7 +867,7 @@ extern "C" int skml_weight_norm(const float* w, long long dim, double lambda, do
     if (!w || !scratch || dim < 0) return (int)cudaErrorInvalidValue;
     double* partials = reinterpret_cast<double*>(scratch);
     unsigned int* counter = reinterpret_cast<unsigned int*>(partials + NORM_BLOCKS);
-    weight_norm_kernel<<<NORM_BLOCKS, 256, 0, (cudaStream_t)stream>>>(w, dim, lambda, sumsq_out, reg_out, partials, counter);
+    skml_launch(weight_norm_kernel, NORM_BLOCKS, 256, 0, (cudaStream_t)stream, w, dim, lambda, sumsq_out, reg_out, partials, counter);
     return (int)cudaGetLastError();
 }
 
@@ -1085,6 +1091,7 @@ colsum_kernel(const int* __restrict__ colptr, const int* __restrict__ rowidx, co
               const int* __restrict__ long_e0, const int* __restrict__ long_e1, int n_short, int n_medium, int n_long,
               int short_blocks, int medium_blocks, const float* __restrict__ coef, const float* __restrict__ w,
               float lambda, float* __restrict__ out, StepLoss loss) {
+    skml_after_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int b = blockIdx.x;
     if (b == 0 && threadIdx.x == 0) loss.settle();
@@ -1184,9 +1191,9 @@ static int colsum_launch(const int* colptr, const int* rowidx, const float* sval
     const int short_blocks = (n_short + 255) / 256, medium_blocks = (n_medium + 7) / 8;
     const long long blocks = (long long)short_blocks + medium_blocks + n_long;
     if (blocks <= 0 && !loss.partials) return 0;
-    colsum_kernel<<<(unsigned)(blocks > 0 ? blocks : 1), 256, 0, stream>>>(colptr, rowidx, svals, ucols, bins, long_col, long_e0, long_e1,
-                                                                          n_short, n_medium, n_long, short_blocks, medium_blocks, coef, w,
-                                                                          lambda, out, loss);
+    skml_launch(colsum_kernel, (unsigned)(blocks > 0 ? blocks : 1), 256, 0, stream, colptr, rowidx, svals, ucols, bins, long_col, long_e0, long_e1,
+                n_short, n_medium, n_long, short_blocks, medium_blocks, coef, w,
+                lambda, out, loss);
     return (int)cudaGetLastError();
 }
 

@@ -14,6 +14,36 @@
 #define SKML_BLOCK 1024
 #define SKML_WARPS (SKML_BLOCK / 32)
 
+// The kernels of a step follow one another on one stream. Launched by skml_launch (programmatic stream serialization) a
+// kernel is set up while the one before it ends, and waits here, before it touches memory, until that one has completed
+// and its stores are visible: 2 us between kernels became about 1 (an epoch of ten small steps 993 -> 936 us). Every kernel
+// launched that way calls this first. No kernel lets the next one start early: what a block would do before it waits is
+// nothing, and the blocks would take the place of others.
+__device__ __forceinline__ void skml_after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+static inline cudaError_t skml_launch_as(bool cooperative, void (*kernel)(P...), unsigned int grid, unsigned int block, size_t smem,
+                                         cudaStream_t stream, A... args) {
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeCooperative;
+    attrs[1].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attrs;
+    cfg.numAttrs = cooperative ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+static inline cudaError_t skml_launch(void (*kernel)(P...), unsigned int grid, unsigned int block, size_t smem, cudaStream_t stream, A... args) {
+    return skml_launch_as(false, kernel, grid, block, smem, stream, args...);
+}
+
 enum SkmlStatus {
     SKML_OK = 0,
     SKML_TIMEOUT_BARRIER = 1,

@@ -297,6 +297,7 @@ template <bool HAS_VALS>
 __global__ void __launch_bounds__(DT_THREADS, 1)
 dt_partial_kernel(const float* __restrict__ x, long long n, int T, int items, int blocks_per_tile, const int* __restrict__ ptr,
                   const ushort4* __restrict__ loc, const float4* __restrict__ val, float* __restrict__ partial) {
+    skml_after_previous();
     extern __shared__ __align__(16) float s_x[];
     __shared__ int s_cut[DT_THREADS / 32 + 1];
     const int tile = blockIdx.x / blocks_per_tile, warp = threadIdx.x >> 5;
@@ -424,6 +425,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
 hot_colsum_kernel(const float* __restrict__ coef, int rows, int T, int items, int blocks_per_tile, int listed, const int* __restrict__ ptr,
                   const ushort4* __restrict__ loc, const float4* __restrict__ val, float* __restrict__ partial, ColdColumns cold,
                   const float* __restrict__ w, float lambda, float* __restrict__ out) {
+    skml_after_previous();
     extern __shared__ __align__(16) float s_x[];
     __shared__ int s_cut[DT_THREADS / 32 + 1];
     const int tile = blockIdx.x / blocks_per_tile, warp = threadIdx.x >> 5;
@@ -450,6 +452,7 @@ hot_colsum_kernel(const float* __restrict__ coef, int rows, int T, int items, in
 __global__ void __launch_bounds__(256)
 hot_combine_kernel(const float* __restrict__ partial, int columns, int items, int tiles, const int4* __restrict__ info, const int4* __restrict__ wide,
                    int lane_blocks, const float* __restrict__ w, float lambda, float* __restrict__ out, StepLoss loss) {
+    skml_after_previous();
     if (blockIdx.x == 0 && threadIdx.x == 0) loss.settle();
     if ((int)blockIdx.x < lane_blocks) {
         const int h = blockIdx.x * 256 + threadIdx.x;
@@ -487,6 +490,7 @@ hot_combine_kernel(const float* __restrict__ partial, int columns, int items, in
 __global__ void __launch_bounds__(256)
 dt_coef_kernel(const float* __restrict__ partial, int rows, int tiles, const float* __restrict__ labels, int loss_id, float inv_batch,
                double* __restrict__ acc, float* __restrict__ coef) {
+    skml_after_previous();
     double loss = 0.0;
     for (int r = blockIdx.x * 256 + threadIdx.x; r < rows; r += gridDim.x * 256) {
         float pre = 0.f;
@@ -533,6 +537,7 @@ __device__ __noinline__ bool holds_nonzero(const float* __restrict__ x, int T, c
 __global__ void __launch_bounds__(256)
 dt_sum_kernel(const float* __restrict__ partial, int dim, int tiles, int T, const int* __restrict__ ptr, const ushort4* __restrict__ loc,
               const float* __restrict__ coef, float* __restrict__ g, unsigned int* __restrict__ bitmap) {
+    skml_after_previous();
     const int lane = threadIdx.x & 31;
     for (int c = blockIdx.x * 256 + threadIdx.x; c - lane < dim; c += gridDim.x * 256) {   // a warp a word of 32 columns
         const bool in = c < dim;
@@ -587,8 +592,8 @@ int dt_partial(const float* x, long long n, int T, int tiles, int items, const i
     const size_t smem = 4 * ((size_t)T + 4);
     const ushort4* l = reinterpret_cast<const ushort4*>(loc);
     const float4* v = reinterpret_cast<const float4*>(val);
-    if (val) dt_partial_kernel<true><<<tiles * bpt, DT_THREADS, smem, stream>>>(x, n, T, items, bpt, ptr, l, v, partial);
-    else dt_partial_kernel<false><<<tiles * bpt, DT_THREADS, smem, stream>>>(x, n, T, items, bpt, ptr, l, v, partial);
+    if (val) skml_launch(dt_partial_kernel<true>, tiles * bpt, DT_THREADS, smem, stream, x, n, T, items, bpt, ptr, l, v, partial);
+    else skml_launch(dt_partial_kernel<false>, tiles * bpt, DT_THREADS, smem, stream, x, n, T, items, bpt, ptr, l, v, partial);
     return (int)cudaGetLastError();
 }
 
@@ -644,8 +649,8 @@ extern "C" int skml_dt_gradient(const SkmlDenseIndex* d, const long long* rowptr
     if (d->r_ptr) {
         rc = dt_partial(w, d->dim, (int)d->tile_cols, (int)d->col_tiles, (int)d->rows, d->r_ptr, d->r_loc, d->r_val, d->partial, stream);
         if (rc) return rc;
-        dt_coef_kernel<<<blocks_for(d->rows, 256, 8), 256, 0, stream>>>(d->partial, (int)d->rows, (int)d->col_tiles, labels + row_lo, loss_id,
-                                                                       inv_batch, loss_acc, d->coef);
+        skml_launch(dt_coef_kernel, blocks_for(d->rows, 256, 8), 256, 0, stream, d->partial, (int)d->rows, (int)d->col_tiles, labels + row_lo, loss_id,
+                    inv_batch, loss_acc, d->coef);
         rc = (int)cudaGetLastError();
     } else {
         rc = skml_glm_coef(rowptr, cols, vals, labels, row_lo, d->rows, nnz_padded, avg_nnz, w, d->dim, loss_id, inv_batch, loss_acc, d->coef,
@@ -654,8 +659,8 @@ extern "C" int skml_dt_gradient(const SkmlDenseIndex* d, const long long* rowptr
     if (rc) return rc;
     rc = dt_partial(d->coef, d->rows, (int)d->tile_rows, (int)d->row_tiles, (int)d->dim, d->c_ptr, d->c_loc, d->c_val, d->partial, stream);
     if (rc) return rc;
-    dt_sum_kernel<<<blocks_for(d->dim, 256, 8), 256, 0, stream>>>(d->partial, (int)d->dim, (int)d->row_tiles, (int)d->tile_rows, d->c_ptr,
-                                                                  reinterpret_cast<const ushort4*>(d->c_loc), d->coef, g, bitmap);
+    skml_launch(dt_sum_kernel, blocks_for(d->dim, 256, 8), 256, 0, stream, d->partial, (int)d->dim, (int)d->row_tiles, (int)d->tile_rows, d->c_ptr,
+                reinterpret_cast<const ushort4*>(d->c_loc), d->coef, g, bitmap);
     return (int)cudaGetLastError();
 }
 
@@ -694,16 +699,16 @@ extern "C" int skml_hot_colsum(const SkmlHotColumns* h, const int* bins, int n_s
     const float4* v = reinterpret_cast<const float4*>(h->val);
     const ColdColumns cold{bins, n_short, n_short + n_medium, colptr, rowidx, svals, ucols};
     if (svals)
-        hot_colsum_kernel<true><<<grid, DT_THREADS, smem, stream>>>(coef, (int)h->rows, (int)h->tile_rows, (int)h->items, bpt, listed, h->ptr, l, v,
-                                                                   h->partial, cold, w, lambda, out);
+        skml_launch(hot_colsum_kernel<true>, grid, DT_THREADS, smem, stream, coef, (int)h->rows, (int)h->tile_rows, (int)h->items, bpt, listed, h->ptr, l, v,
+                    h->partial, cold, w, lambda, out);
     else
-        hot_colsum_kernel<false><<<grid, DT_THREADS, smem, stream>>>(coef, (int)h->rows, (int)h->tile_rows, (int)h->items, bpt, listed, h->ptr, l, v,
-                                                                    h->partial, cold, w, lambda, out);
+        skml_launch(hot_colsum_kernel<false>, grid, DT_THREADS, smem, stream, coef, (int)h->rows, (int)h->tile_rows, (int)h->items, bpt, listed, h->ptr, l, v,
+                    h->partial, cold, w, lambda, out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
     const int lane_blocks = (int)((h->columns + 255) / 256);
-    hot_combine_kernel<<<(unsigned)(lane_blocks + h->wide), 256, 0, stream>>>(h->partial, (int)h->columns, (int)h->items, (int)h->row_tiles,
-                                                                           reinterpret_cast<const int4*>(h->info), reinterpret_cast<const int4*>(h->wide_info),
-                                                                           lane_blocks, w, lambda, out, StepLoss{partials, tmpl});
+    skml_launch(hot_combine_kernel, (unsigned)(lane_blocks + h->wide), 256, 0, stream, h->partial, (int)h->columns, (int)h->items, (int)h->row_tiles,
+                reinterpret_cast<const int4*>(h->info), reinterpret_cast<const int4*>(h->wide_info),
+                lane_blocks, w, lambda, out, StepLoss{partials, tmpl});
     return (int)cudaGetLastError();
 }

@@ -105,6 +105,7 @@ __global__ void zip_pad_kernel(const float* __restrict__ vals, const long long* 
 __global__ void __launch_bounds__(ZT, 1)
 zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_ptr, long long n_max, unsigned int* buf_a, unsigned int* buf_b,
                 ZShared* __restrict__ shared, unsigned int* status) {
+    skml_after_previous();
     __shared__ unsigned int s_cnt[ZT / 32][256], s_tot[4][256], s_bef[4][256], s_base[256], s_warp[8];
     const unsigned int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = gridDim.x, b = blockIdx.x;
     long long n64 = *n_ptr;
@@ -403,6 +404,7 @@ __global__ void __launch_bounds__(ZT, 1)
 zip_splits_kernel(ZScratch z, const long long* __restrict__ n_ptr, long long n_max, int bin_num,
                   float* __restrict__ splits_out, float* __restrict__ mids_out, int* __restrict__ meta_out,
                   float* __restrict__ range_out, unsigned int* status) {
+    skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ZSmem& sm = *reinterpret_cast<ZSmem*>(smem_raw);
     unsigned int* const sh_warp = sm.warp;
@@ -623,6 +625,7 @@ __global__ void __launch_bounds__(256)
 zip_code_kernel(const float* __restrict__ vals, const long long* __restrict__ n_ptr, long long n_max,
                 const float* __restrict__ splits, const int* __restrict__ meta, int code_bytes,
                 unsigned char* __restrict__ codes, const unsigned int* __restrict__ status) {
+    skml_after_previous();
     extern __shared__ float sh_splits[];
     long long n = *n_ptr;
     if (n > n_max) n = n_max;
@@ -647,6 +650,7 @@ __global__ void __launch_bounds__(256)
 zip_unpack_scatter_kernel(float* __restrict__ acc, const int* __restrict__ keys, const unsigned char* __restrict__ codes,
                           const float* __restrict__ mids, const long long* __restrict__ count, long long key_stride,
                           int code_bytes, int table_len, float* __restrict__ vals_out, const unsigned int* __restrict__ status) {
+    skml_after_previous();
     extern __shared__ float sh_mids[];
     long long n = *count;
     if (n > key_stride) n = key_stride;
@@ -701,8 +705,7 @@ extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long l
     if (n_max <= sorters * ZT * Z_SORT_KEYS) {   // (beyond, passes over memory are what a sort costs)
         unsigned int* a = reinterpret_cast<unsigned int*>(z.sorted_in);
         unsigned int* b = reinterpret_cast<unsigned int*>(z.sorted);
-        void* sort_args[] = {&vals, &n_ptr, &n_max, &a, &b, &z.shared, &status};
-        e = cudaLaunchCooperativeKernel((const void*)zip_sort_kernel, dim3((unsigned)sorters), dim3(ZT), sort_args, 0, s);
+        e = skml_launch_as(true, zip_sort_kernel, (unsigned)sorters, ZT, 0, s, vals, n_ptr, n_max, a, b, z.shared, status);
     } else {
         zip_pad_kernel<<<zip_sm_count() * 4, 256, 0, s>>>(vals, n_ptr, n_max, z.sorted_in);
         e = cub::DeviceRadixSort::SortKeys(z.cub_temp, z.cub_bytes, z.sorted_in, z.sorted, (int)n_max, 0, 32, s);
@@ -721,11 +724,10 @@ extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long l
         if (e != cudaSuccess) return (int)e;
         ready = true;
     }
-    void* args[] = {&z, &n_ptr, &n_max, &bin_num, &splits, &mids, &meta, &range, &status};
-    e = cudaLaunchCooperativeKernel((const void*)zip_splits_kernel, dim3((unsigned)blocks), dim3(ZT), args, sizeof(ZSmem), s);
+    e = skml_launch_as(true, zip_splits_kernel, (unsigned)blocks, ZT, sizeof(ZSmem), s, z, n_ptr, n_max, bin_num, splits, mids, meta, range, status);
     if (e != cudaSuccess) return (int)e;
     const int cb = skml_zipml_code_bytes(bin_num);
-    zip_code_kernel<<<zip_sm_count() * 4, 256, sizeof(float) * (size_t)(bin_num + 2), s>>>(vals, n_ptr, n_max, splits, meta, cb, codes, status);
+    skml_launch(zip_code_kernel, zip_sm_count() * 4, 256, sizeof(float) * (size_t)(bin_num + 2), s, vals, n_ptr, n_max, splits, meta, cb, codes, status);
     return (int)cudaGetLastError();
 }
 
@@ -738,9 +740,9 @@ extern "C" int skml_zipml_unpack_scatter(float* acc, const int* keys, const unsi
     const int cb = skml_zipml_code_bytes(bin_num);
     for (int l = 0; l < lists; ++l) {
         const int tl = bin_num + 2;
-        zip_unpack_scatter_kernel<<<zip_sm_count() * 4, 256, sizeof(float) * (size_t)tl, (cudaStream_t)stream>>>(
-            acc, keys ? keys + (long long)l * key_stride : nullptr, codes + (long long)l * code_stride,
-            mids + (long long)l * tl, counts + l, key_stride, cb, tl, vals_out ? vals_out + (long long)l * key_stride : nullptr, status);
+        skml_launch(zip_unpack_scatter_kernel, zip_sm_count() * 4, 256, sizeof(float) * (size_t)tl, (cudaStream_t)stream,
+                    acc, keys ? keys + (long long)l * key_stride : nullptr, codes + (long long)l * code_stride,
+                    mids + (long long)l * tl, counts + l, key_stride, cb, tl, vals_out ? vals_out + (long long)l * key_stride : nullptr, status);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }
