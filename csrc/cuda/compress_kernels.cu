@@ -270,6 +270,12 @@ struct SmemPack {
 };
 static_assert(sizeof(SmemPack) <= offsetof(SmemCoding, huf_len), "the Huffman code tables outlive the key code's staging");
 
+// S4, insert in shared memory: a warp's turn of 128 elements, put in the groups' order (rank code | group << 8).
+struct SmemPart {
+    unsigned int key[SKML_WARPS][128];
+    unsigned short tag[SKML_WARPS][128];
+};
+
 struct Smem {
     float splits[SKML_GPU_MAX_BINS];               // stages S3..S6
     union {
@@ -278,6 +284,7 @@ struct Smem {
         SmemSearch ss;
         SmemPack ps;
         uint2 priv_blocks[PRIV_MAX_PARTS];         // merge of the copies: a part's first block and its number of blocks
+        SmemPart part;
     };
     // stages S3..S6
     unsigned char grp_lut[SKML_GPU_MAX_BINS];      // bucket -> group
@@ -1205,7 +1212,7 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
 // the least codes in shared memory and leaves a copy of the part; the copies of a part are merged when the tables are
 // written to the payload. Bound by the hashes' instructions and the latency of the rounds; atomics in L2, three a key, by
 // L2's rate (121 G/s). Insert and all, S4 and S5 of such launches (rows of 0.2 cells a key; atomics / shared memory, us):
-// 0.5M keys 26 / 33, 1M 41 / 38, 2.27M 76 / 63, 5M 158 / 126, 10M 302 / 268, which is why smaller ones keep the atomics.
+// 0.5M keys 26 / 32, 1M 41 / 38, 2.27M 76 / 59, 10M 302 / 247, which is why smaller ones keep the atomics.
 // Sets L.priv where it pays: the keys of large groups are hashed once per part, so a group of many parts (few distinct
 // values: one group holds nearly every key) is left to the atomics.
 __device__ void priv_layout(const CP& p, Smem& s) {
@@ -1431,8 +1438,88 @@ __device__ void stage_scatter(const CP& p, Smem& s, long long n, int (&nkey)[2],
     }
 }
 
-// S4 where the insert follows in shared memory: the lists get the keys and their rank codes, 128 elements a turn with the
-// next ones on their way.
+// S4 where the insert follows in shared memory: the lists get the keys and their rank codes.
+// Up to eight groups: 128 elements a turn, four adjacent ones a lane. A lane's counts of all groups are the bytes of one
+// word, so that one scan of the warp ranks the turn's elements; they are put in group order in shared memory and leave it
+// in runs. (A ballot per bit of the group number for every 32 elements took four times the instructions: 66 us of 10M keys.)
+__device__ __forceinline__ void partition_turns(const CP& p, Smem& s, int len, unsigned int run, const int* __restrict__ keys,
+                                                const unsigned short* __restrict__ bins) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int* const s_key = s.part.key[warp];
+    unsigned short* const s_tag = s.part.tag[warp];
+    const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;   // (slices start at multiples of 32 elements)
+    int nkey[4], nbin[4];
+    auto fetch = [&](int i0) {
+        const int i = i0 + 4 * lane;
+        if (vec && i + 4 <= len) {
+            const int4 k = __ldg(reinterpret_cast<const int4*>(keys + i));
+            const uint2 b = *reinterpret_cast<const uint2*>(bins + i);
+            nkey[0] = k.x; nkey[1] = k.y; nkey[2] = k.z; nkey[3] = k.w;
+            nbin[0] = (int)(b.x & 0xFFFFu); nbin[1] = (int)(b.x >> 16); nbin[2] = (int)(b.y & 0xFFFFu); nbin[3] = (int)(b.y >> 16);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                nkey[u] = i + u < len ? keys[i + u] : 0;
+                nbin[u] = i + u < len ? (int)bins[i + u] : 0;
+            }
+        }
+    };
+    fetch(0);
+    for (int i0 = 0; i0 < len; i0 += 128) {
+        int key[4], bin[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            key[u] = nkey[u];
+            bin[u] = nbin[u];
+        }
+        fetch(i0 + 128);
+        const int have = len - i0 - 4 * lane;   // this lane's elements
+        unsigned int g[4];
+        unsigned long long own = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            g[u] = u < have ? s.grp_lut[bin[u]] : 0u;
+            if (u < have) own += 1ull << (8 * g[u]);
+        }
+        unsigned long long inc = own;   // (128 elements at most: no byte overflows)
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        const unsigned long long all = __shfl_sync(0xFFFFFFFFu, inc, 31);
+        // bytes of `start`: elements of the groups before (the sum over the lower bytes, below 256 each)
+        const unsigned long long start = (all << 8) * 0x0101010101010101ull;
+        unsigned long long at = start + inc - own;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (u < have) {
+                const unsigned int r = (unsigned int)(at >> (8 * g[u])) & 0xFFu;
+                s_key[r] = (unsigned int)key[u];
+                s_tag[r] = (unsigned short)(s.rank_lut[bin[u]] | (g[u] << 8));
+                at += 1ull << (8 * g[u]);
+            }
+        }
+        __syncwarp();
+        // lane g: where group g's first element of this turn goes, less its place in the turn
+        const unsigned int base = lane < 8 ? run - ((unsigned int)(start >> (8 * lane)) & 0xFFu) : 0u;
+        if (lane < 8) run += (unsigned int)(all >> (8 * lane)) & 0xFFu;
+        const int turn = min(128, len - i0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int q = 32 * u + lane;
+            const unsigned int tag = q < turn ? s_tag[q] : 0u;
+            const unsigned int to = __shfl_sync(0xFFFFFFFFu, base, (int)(tag >> 8)) + (unsigned int)q;
+            if (q < turn) {
+                p.gkeys[to] = (int)s_key[q];
+                p.gcodes[to] = (unsigned char)tag;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// More groups: a ballot per bit of the group number.
 __device__ void stage_partition(const CP& p, Smem& s, long long n) {
     constexpr int U = 4;
     const int G = p.G, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1446,6 +1533,10 @@ __device__ void stage_partition(const CP& p, Smem& s, long long n) {
     unsigned int run = 0;   // lane g: staging position of the next key of group g in this slice
     if (lane < G) run = L.goff[lane] + L.base_rank[lane] + s.wbase[warp][lane];
     const int len = (int)(hi - lo), rem = len - lane;   // this lane's elements: 0, 32, ... below rem
+    if (G <= 8) {
+        partition_turns(p, s, len, run, p.keys + lo, p.bins + lo);
+        return;
+    }
     const int* const keys = p.keys + lo + lane;
     const unsigned short* const bins = p.bins + lo + lane;
     int nkey[U], nbin[U];
@@ -1473,8 +1564,7 @@ __device__ void stage_partition(const CP& p, Smem& s, long long n) {
             const bool valid = i0 + 32 * u < rem;
             const int g = valid ? (int)s.grp_lut[bin[u]] : 0;
             unsigned int own, of_lane;
-            if (G <= 8) group_masks<3>(valid, g, own, of_lane);
-            else group_masks<5>(valid, g, own, of_lane);
+            group_masks<5>(valid, g, own, of_lane);
             const unsigned int to = __shfl_sync(0xFFFFFFFFu, run, g) + (unsigned int)__popc(own & lanemask_lt());
             run += (unsigned int)__popc(of_lane);   // (of lanes beyond the last group nobody asks)
             if (valid) {
