@@ -571,56 +571,74 @@ __device__ void apply_stashed(const DP& p, unsigned long long begin, unsigned lo
     }
 }
 
-// One rank's slice of the block's key range. OP 0: SGD step / plain sum; OP 1: add into the float
-// accumulators; OP 2: Adam update of every coordinate whose accumulated sum is non-zero, then clear it.
-// The groups of one rank hold disjoint keys, so their slices are walked as one concatenated list,
-// four independent entries per thread and iteration; a block barrier ends the pass.
-template <int OP>
-__device__ __forceinline__ void owned_pass(const DP& p, DecSmem& s, const unsigned long long* seg_b,
-                                           const unsigned long long* seg_e, int r, float& dsq) {
-    const int i0 = s.rank_item_begin[r], i1 = s.rank_item_begin[r + 1];
-    float* dst = OP == 0 ? (p.out_sum ? p.out_sum : p.w) : p.fsum;
-    const long long ds = OP == 0 ? 1ll : p.fsum_stride;
-    unsigned int total = 0;
-    for (int i = i0; i < i1; ++i) total += (unsigned int)(seg_e[i] - seg_b[i]);
-    for (unsigned int q = threadIdx.x; q < total; q += 4 * blockDim.x) {
-        unsigned int k[4];
-        float v[4], old[4];
+// One rank's slice of the block's key range. The groups of one rank hold disjoint keys, so their slices are walked as one
+// concatenated list: `ends` are the slices' ends in it, `shift` what an entry's place in it lacks to its place in the
+// scratch. A thread takes four independent entries per iteration.
+struct OwnedEntries {
+    unsigned int k[4];   // 0xFFFFFFFF: none
+    float v[4];
+};
+template <bool VALUES>
+__device__ __forceinline__ void owned_fetch(const DP& p, const DecSmem& s, const unsigned long long* shift, const unsigned long long* ends, int r,
+                                            unsigned int q, OwnedEntries& e) {
+    int i = s.rank_item_begin[r];
+    const int i1 = s.rank_item_begin[r + 1];
+    const unsigned int total = i < i1 ? (unsigned int)ends[i1 - 1] : 0u;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            unsigned int qq = q + u * blockDim.x;
-            k[u] = 0xFFFFFFFFu;
-            v[u] = 0.f;
-            if (qq < total) {
-                int i = i0;
-                unsigned int len = (unsigned int)(seg_e[i] - seg_b[i]);
-                while (qq >= len) {
-                    qq -= len;
-                    ++i;
-                    len = (unsigned int)(seg_e[i] - seg_b[i]);
-                }
-                const unsigned long long pos = seg_b[i] + qq;
-                k[u] = (unsigned int)__ldcg(p.key_scratch + pos);
-                if (OP != 2) v[u] = __ldcg(p.val_scratch + pos);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) old[u] = k[u] < (unsigned long long)p.dim ? dst[k[u] * ds] : 0.f;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (k[u] >= (unsigned long long)p.dim) continue;
-            if (OP == 0) {
-                const float nw = p.out_sum ? old[u] + v[u] : old[u] - p.lr * v[u];
-                dst[k[u]] = nw;
-                if (!p.out_sum) dsq += (nw - old[u]) * (nw + old[u]);
-            } else if (OP == 1) dst[k[u] * ds] = old[u] + v[u];
-            else if (old[u] != 0.f) {
-                dst[k[u] * ds] = 0.f;
-                dsq += apply_one(p, k[u], old[u]);
-            }
+    for (int u = 0; u < 4; ++u) {
+        const unsigned int qq = q + u * DEC_THREADS;
+        e.k[u] = 0xFFFFFFFFu;
+        e.v[u] = 0.f;
+        if (qq < total) {
+            while (qq >= (unsigned int)ends[i]) ++i;
+            const unsigned long long pos = shift[i] + qq;
+            e.k[u] = (unsigned int)__ldcg(p.key_scratch + pos);
+            if (VALUES) e.v[u] = __ldcg(p.val_scratch + pos);
         }
     }
+}
+
+// OP 0: SGD step / plain sum; OP 1: add into the float accumulators; OP 2: Adam update of every coordinate whose
+// accumulated sum is non-zero, then clear it. `e`: the thread's first entries, loaded by the caller; those of rank `next`
+// (negative: none) are on their way when the pass ends. A block barrier ends it.
+template <int OP>
+__device__ __forceinline__ void owned_pass(const DP& p, DecSmem& s, const unsigned long long* shift, const unsigned long long* ends, int r, int next,
+                                           OwnedEntries& e, float& dsq) {
+    const int i1 = s.rank_item_begin[r + 1];
+    const unsigned int total = s.rank_item_begin[r] < i1 ? (unsigned int)ends[i1 - 1] : 0u;
+    float* dst = OP == 0 ? (p.out_sum ? p.out_sum : p.w) : p.fsum;
+    const long long ds = OP == 0 ? 1ll : p.fsum_stride;
+    OwnedEntries ahead;
+    for (unsigned int q = threadIdx.x;; q += 4 * DEC_THREADS) {
+        float old[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) old[u] = e.k[u] < (unsigned long long)p.dim ? dst[e.k[u] * ds] : 0.f;
+        const bool more = q + 4 * DEC_THREADS < total;
+        if (more) owned_fetch<OP != 2>(p, s, shift, ends, r, q + 4 * DEC_THREADS, ahead);
+        else if (next >= 0) owned_fetch<OP != 2>(p, s, shift, ends, next, threadIdx.x, ahead);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (e.k[u] >= (unsigned long long)p.dim) continue;
+            if (OP == 0) {
+                const float nw = p.out_sum ? old[u] + e.v[u] : old[u] - p.lr * e.v[u];
+                dst[e.k[u] * ds] = nw;
+                if (!p.out_sum) dsq += (nw - old[u]) * (nw + old[u]);
+            } else if (OP == 1) dst[e.k[u] * ds] = old[u] + e.v[u];
+            else if (old[u] != 0.f) {
+                dst[e.k[u] * ds] = 0.f;
+                dsq += apply_one(p, e.k[u], old[u]);
+            }
+        }
+        e = ahead;
+        if (!more) break;
+    }
     __syncthreads();
+}
+template <int OP>
+__device__ __forceinline__ void owned_passes(const DP& p, DecSmem& s, const unsigned long long* shift, const unsigned long long* ends, float& dsq) {
+    OwnedEntries e;
+    owned_fetch<OP != 2>(p, s, shift, ends, 0, threadIdx.x, e);
+    for (int r = 0; r < p.world; ++r) owned_pass<OP>(p, s, shift, ends, r, r + 1 < p.world ? r + 1 : -1, e, dsq);
 }
 
 // Barrier-free ordered apply. The key space is cut into DEC_OWN_RANGES x blocks ranges at the quantiles
@@ -665,16 +683,30 @@ __device__ void apply_owned(const DP& p, DecSmem& s, float& dsq) {
         seg[(size_t)which * p.max_items + item] = it.key_prefix + lo;
     }
     __syncthreads();
+    // begin and end of every slice -> end in the rank's concatenated slices, and shift (a warp's lane per rank and range)
+    for (int t = threadIdx.x; t < rounds * p.world; t += blockDim.x) {
+        const int r = t % p.world;
+        unsigned long long* const b = seg + (size_t)(2 * (t / p.world)) * p.max_items;
+        unsigned long long* const e = b + p.max_items;
+        unsigned long long end = 0;
+        for (int i = s.rank_item_begin[r]; i < s.rank_item_begin[r + 1]; ++i) {
+            const unsigned long long before = end;
+            end += e[i] - b[i];
+            b[i] -= before;
+            e[i] = end;
+        }
+    }
+    __syncthreads();
     for (int round = 0; round < rounds; ++round) {
-        const unsigned long long* seg_b = seg + (size_t)(2 * round) * p.max_items;
-        const unsigned long long* seg_e = seg_b + p.max_items;
+        const unsigned long long* shift = seg + (size_t)(2 * round) * p.max_items;
+        const unsigned long long* ends = shift + p.max_items;
         if (p.adam_v) {
             // Adam: sum the ranks' values per coordinate in rank order (plain floats in the zeroed
             // sums), then let the first rank that holds a coordinate apply the update and clear the sum.
-            for (int r = 0; r < p.world; ++r) owned_pass<1>(p, s, seg_b, seg_e, r, dsq);
-            for (int r = 0; r < p.world; ++r) owned_pass<2>(p, s, seg_b, seg_e, r, dsq);
+            owned_passes<1>(p, s, shift, ends, dsq);
+            owned_passes<2>(p, s, shift, ends, dsq);
         } else {
-            for (int r = 0; r < p.world; ++r) owned_pass<0>(p, s, seg_b, seg_e, r, dsq);
+            owned_passes<0>(p, s, shift, ends, dsq);
         }
     }
 }
