@@ -203,7 +203,9 @@ glm_scatter_kernel(const long long* __restrict__ rowptr, const int* __restrict__
 // it hits and an L1 line while it misses, so the weights of the first `hot` columns (the frequent ones where
 // indices are assigned by frequency) are kept in shared memory, which serves some ten lanes a cycle, and nothing
 // is staged that would take L1 away. 500,000 rows of 30: 80 -> 61 us; 1M rows of 30 with values: 208 -> 102 us
-// (before: a warp per row, tiles staged by bulk copies, 103 warp instructions per 32 entries).
+// (before: a warp per row, tiles staged by bulk copies, 103 warp instructions per 32 entries). Four blocks an SM instead of
+// three, at 32 registers with a few spills: 58 and 99 us, 62,500 rows 15 -> 13; one block of 1024 threads with six times
+// the hot columns took 80 and 129: what counts is the gathers in flight.
 #define MARGIN_THREADS 512
 struct ClearSlots {   // out[slot[0 .. n)] = 0
     float* out;
@@ -211,7 +213,7 @@ struct ClearSlots {   // out[slot[0 .. n)] = 0
     int n;
 };
 template <int MODE, int GL, bool HAS_VALS>
-__global__ void __launch_bounds__(MARGIN_THREADS, 3)
+__global__ void __launch_bounds__(MARGIN_THREADS, 4)
 glm_margin_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
                   const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
                   int hot, int loss_id, float inv_batch, double* __restrict__ acc, float* __restrict__ out, ClearSlots clear) {
@@ -314,7 +316,7 @@ static int sm_count() {
     return g_sm_count;
 }
 
-// Columns [0, margin_hot) of w in shared memory: at most 8192 (32 KB, three blocks an SM keep 128 KB of L1), no more
+// Columns [0, margin_hot) of w in shared memory: at most 8192 (32 KB, four blocks an SM keep 92 KB of L1), no more
 // than a block has entries to look up (reading them in is then an eighth of the sectors of the gathers at most),
 // whole 16-byte units. Below 1024 the copy is not worth its barrier.
 static int margin_hot(long long entries, long long blocks, long long dim, const float* w) {
@@ -363,7 +365,7 @@ template <int MODE, int GL>
 static int margin_launch_gl(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
                             long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
                             float* out, const ClearSlots& clear, cudaStream_t stream) {
-    const TurnShape t = turn_shape(row_cnt, GL, MARGIN_THREADS / 32, 3);
+    const TurnShape t = turn_shape(row_cnt, GL, MARGIN_THREADS / 32, 4);
     const int iters = t.iters, warps = t.warps, grid = t.grid;
     const int hot = margin_hot((long long)(row_cnt * avg_nnz), grid, dim, w);
     if (vals)
