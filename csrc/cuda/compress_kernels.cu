@@ -1111,11 +1111,13 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
         const int g = warp;
         // the blocks' totals (before this block / all blocks), lanes striding over the blocks; this
         // block's own 32 slices are scanned over the lanes for the warps' starting ranks
-        unsigned int before = 0, total = 0;
-        for (int b = lane; b < nb; b += 32) {
-            const unsigned int c = __ldcg(&p.blk_cnt[(long long)b * SKML_MAX_GROUPS + g]);
-            total += c;
-            if (b < (int)blockIdx.x) before += c;
+        unsigned int before = 0, total = 0, c[MAX_GRID / 32];
+#pragma unroll
+        for (int k = 0; k < MAX_GRID / 32; ++k) c[k] = lane + 32 * k < nb ? __ldcg(&p.blk_cnt[(long long)(lane + 32 * k) * SKML_MAX_GROUPS + g]) : 0u;
+#pragma unroll
+        for (int k = 0; k < MAX_GRID / 32; ++k) {   // (all loads in flight at once: one after the other they took 2 us)
+            total += c[k];
+            if (lane + 32 * k < (int)blockIdx.x) before += c[k];
         }
         const unsigned int own = FUSED ? s.wcnt[lane][g] : __ldcg(&p.warp_cnt[((long long)blockIdx.x * SKML_WARPS + lane) * SKML_MAX_GROUPS + g]);
         total = __reduce_add_sync(0xFFFFFFFFu, total);
@@ -1770,6 +1772,17 @@ __device__ bool wait_published(const CP& p, const unsigned int* flags, unsigned 
     return __syncthreads_and(ok) != 0;
 }
 
+// Sum of one word of each of the blocks [0, count), by a warp, its loads in flight together.
+__device__ __forceinline__ unsigned long long sum_over_blocks(const unsigned long long* words, int stride, unsigned int count) {
+    const unsigned int lane = threadIdx.x & 31;
+    unsigned long long c[MAX_GRID / 32], v = 0;
+#pragma unroll
+    for (int k = 0; k < MAX_GRID / 32; ++k) c[k] = lane + 32 * k < count ? __ldcg(words + (long long)(lane + 32 * k) * stride) : 0ull;
+#pragma unroll
+    for (int k = 0; k < MAX_GRID / 32; ++k) v += c[k];
+    return warp_sum(v);
+}
+
 // Byte totals of the blocks before this one (they own the chunks before this block's run, so the
 // sums give this block's starting offsets and the sizes of all earlier groups); a warp per group.
 __device__ void pack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch) {
@@ -1777,9 +1790,7 @@ __device__ void pack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch)
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < p.G) {
-        unsigned long long v = 0;
-        for (unsigned int b = lane; b < blockIdx.x; b += 32) v += __ldcg(&p.blk_bytes[(long long)b * SKML_MAX_GROUPS + warp]);
-        v = warp_sum(v);
+        const unsigned long long v = sum_over_blocks(p.blk_bytes + warp, SKML_MAX_GROUPS, blockIdx.x);
         if (lane == 0) s.pre_bytes[warp] = v;
     }
     __syncthreads();
@@ -2082,9 +2093,7 @@ __device__ void apack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch
     const bool ok = !wait || wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x52u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int g = warp; g < 2 * p.G; g += SKML_WARPS) {
-        unsigned long long v = 0;
-        for (unsigned int b = lane; b < blockIdx.x; b += 32) v += __ldcg(&p.blk_bits[(long long)b * 2 * SKML_MAX_GROUPS + g]);
-        v = warp_sum(v);
+        const unsigned long long v = sum_over_blocks(p.blk_bits + g, 2 * SKML_MAX_GROUPS, blockIdx.x);
         if (lane == 0) s.pre_bits[g] = v;
     }
     if (threadIdx.x == 0 && !ok) s.lay.overflow = 1;
@@ -2473,9 +2482,7 @@ __device__ void huf_measure(const CP& p, Smem& s, unsigned int t_begin, unsigned
 __device__ void huf_prefix(const CP& p, Smem& s) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < p.G) {
-        unsigned long long v = 0;
-        for (unsigned int b = lane; b < blockIdx.x; b += 32) v += __ldcg(&p.blk_tbits[(long long)b * SKML_MAX_GROUPS + warp]);
-        v = warp_sum(v);
+        const unsigned long long v = sum_over_blocks(p.blk_tbits + warp, SKML_MAX_GROUPS, blockIdx.x);
         if (lane == 0) s.pre_tbits[warp] = v;
     }
     __syncthreads();
@@ -2630,9 +2637,7 @@ __device__ void layout_finish(const CP& p, Smem& s, unsigned int nactive) {
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < p.G) {
-        unsigned long long v = 0;
-        for (unsigned int b = lane; b < nactive; b += 32) v += __ldcg(&p.blk_bytes[(long long)b * SKML_MAX_GROUPS + warp]);
-        v = warp_sum(v);
+        const unsigned long long v = sum_over_blocks(p.blk_bytes + warp, SKML_MAX_GROUPS, nactive);
         if (lane == 0) L.bytes_g[warp] = v;
     }
     __syncthreads();
