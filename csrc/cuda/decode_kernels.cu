@@ -675,10 +675,21 @@ __device__ void apply_owned(const DP& p, DecSmem& s, float& dsq) {
         const unsigned long long bound = s_bound[which];
         const int* list = p.key_scratch + it.key_prefix;
         unsigned int lo = 0, hi = it.e.n;
-        while (lo < hi) {  // first position whose key is >= bound
-            const unsigned int mid = (lo + hi) >> 1;
-            if ((unsigned long long)(unsigned int)__ldcg(list + mid) < bound) lo = mid + 1;
-            else hi = mid;
+        while (lo < hi) {  // first position whose key is >= bound: three probes a step, half as many trips to L2 as with one
+            const unsigned int len = hi - lo, m1 = lo + len / 4, m2 = lo + len / 2, m3 = m2 + (hi - m2) / 2;
+            const unsigned int k1 = (unsigned int)__ldcg(list + m1), k2 = (unsigned int)__ldcg(list + m2), k3 = (unsigned int)__ldcg(list + m3);
+            if ((unsigned long long)k2 < bound) {
+                if ((unsigned long long)k3 < bound) lo = m3 + 1;
+                else {
+                    lo = m2 + 1;
+                    hi = m3;
+                }
+            } else if ((unsigned long long)k1 < bound) {
+                lo = m1 + 1;
+                hi = m2;
+            } else {
+                hi = m1;
+            }
         }
         seg[(size_t)which * p.max_items + item] = it.key_prefix + lo;
     }
