@@ -8,7 +8,8 @@
 //   S3  dedupe splits, zero bucket, bucket midpoints, group edges; bucketize every value and
 //       count the keys of every bucket group per warp slice
 //   S4  group sizes -> payload layout; every key goes to its group's contiguous (still key-sorted)
-//       staging list; grouped MinMaxSketch insert (atomicMin on packed cells)
+//       staging list; grouped MinMaxSketch insert (atomicMin on packed cells; from 1M keys on, as a stage of its
+//       own, into tables in shared memory whose copies are merged in S6)
 //   S5  the groups' key lists are coded in 1024-key chunks like a plain array: delta widths, byte
 //       offsets, flag bytes, delta bytes staged per warp, one restart point per chunk. A block owns a
 //       contiguous run of chunks and learns its byte offset from the blocks before it (their
