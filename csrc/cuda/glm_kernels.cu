@@ -1075,10 +1075,24 @@ extern "C" int skml_sm_count() { return sm_count(); }
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float colsum_range(const int* __restrict__ rowidx, const float* __restrict__ svals,
                                               const float* __restrict__ coef, int e0, int e1, int start, int stride) {
+    // four entries in flight: one after the other, each is two trips to L2 (1.9M entries 18.3 -> 15.7 us, 7.5M 51 -> 48,
+    // 0.15M 5.7 -> 4.4)
     float acc = 0.f;
-    for (int e = e0 + start; e < e1; e += stride) {
-        const float c = __ldg(coef + rowidx[e]);
-        acc = fmaf(c, svals ? svals[e] : 1.f, acc);
+    const unsigned int end = (unsigned int)e1;   // (steps past the end do not wrap)
+    for (unsigned int e = (unsigned int)(e0 + start); e < end; e += 4u * stride) {
+        int r[4];
+        float x[4], c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned int at = e + (unsigned int)(u * stride);
+            r[u] = at < end ? rowidx[at] : -1;
+            x[u] = svals && at < end ? svals[at] : 1.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = r[u] >= 0 ? __ldg(coef + r[u]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (r[u] >= 0) acc = fmaf(c[u], x[u], acc);
     }
     return acc;
 }
