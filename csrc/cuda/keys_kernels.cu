@@ -438,60 +438,78 @@ __global__ void __launch_bounds__(ZT) da_zero_pos_kernel(const unsigned int* __r
     }
 }
 
+// Keys of a tile, each counted from the tile's first bit on and within its thread only: k[u] = sum of the deltas of this
+// thread's keys up to the u-th. `bit`: the tile's first delta bit, then the next tile's. Returns the thread's sum.
+__device__ __forceinline__ unsigned int tile_keys(const Streams& s, const unsigned int (&iv)[KPT], unsigned long long& bit, unsigned int* part32,
+                                                  unsigned int (&k)[KPT]) {
+    const unsigned int b = 32u / s.m;
+    unsigned int bits = 0, total;
+#pragma unroll
+    for (int u = 0; u < KPT; ++u) bits += b * iv[u];
+    unsigned long long off = bit + block_scan<KT>(bits, part32, total);
+    bit += total;
+    unsigned int dsum = 0;
+#pragma unroll
+    for (int u = 0; u < KPT; ++u) {
+        const unsigned int dw = b * iv[u];
+        unsigned int d = 0;
+        if (dw && dw <= 32u) {
+            const long long w = (long long)(off >> 5);
+            const unsigned int x0 = w < s.delta_lim ? s.delta_words[w] : 0u, x1 = w + 1 < s.delta_lim ? s.delta_words[w + 1] : 0u;
+            d = __brev(__funnelshift_r(x0, x1, (unsigned int)(off & 31ull)) << (32u - dw));
+        }
+        off += dw;
+        dsum += d;
+        k[u] = dsum;
+    }
+    return dsum;
+}
+
+// What the blocks before this one would have told it, found by itself: delta bits and sum of the keys [0, lo).
+__device__ __noinline__ void before_run(Streams s, long long lo, unsigned int* part32, unsigned long long& bit, unsigned int& sum) {
+    bit = 0;
+    sum = 0;
+    for (long long t0 = 0; t0 < lo; t0 += KEY_TILE) {
+        unsigned int iv[KPT], k[KPT], tile_sum;
+        intervals(s, t0 + (long long)KPT * threadIdx.x, lo, iv);
+        block_scan<KT>(tile_keys(s, iv, bit, part32, k), part32, tile_sum);
+        sum += tile_sum;
+    }
+}
+
 // Decoding in one cooperative launch: delta bits of every run, a grid barrier, the run's keys counted from the key
 // before it, a grid barrier, the sum of the runs before it added. Runs of one tile keep flags and keys in registers.
+// The caller is not told how the launch went, so it cannot fail: where a barrier gives up, a block works out for itself
+// what it waited for, and goes to no barrier any more (the others give up with it: the status word says so).
 __global__ void __launch_bounds__(KT, 1)
-da_decode_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk, int* __restrict__ keys) {
+da_decode_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk, int* __restrict__ keys, long long budget) {
     __shared__ unsigned long long s_part[KT / 32];
     __shared__ unsigned int s_part32[KT / 32];
-    const unsigned int b = 32u / s.m;
     const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
     const bool keep = per_run <= KEY_TILE;
     unsigned int passed = 0;
-    auto barrier = [&](unsigned int where) {
-        if (skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, KEY_BUDGET, where, passed)) return true;
-        for (long long i = lo + threadIdx.x; i < hi; i += KT) keys[i] = -1;   // nobody takes these for keys
-        return false;
-    };
-    unsigned int iv[KPT], k[KPT];
-    auto bits_of = [&]() {
-        unsigned int t = 0;
-#pragma unroll
-        for (int u = 0; u < KPT; ++u) t += iv[u];
-        return t * b;
-    };
+    bool together = gridDim.x > 1;   // (one block has nothing to wait for)
+    unsigned int iv[KPT], k[KPT], add = 0;
     unsigned long long bit = 0, sum = 0;
-    if (gridDim.x > 1) {   // (one block has nothing to wait for)
+    if (together) {
         unsigned long long v = 0, total;
         for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
             intervals(s, t0 + (long long)KPT * threadIdx.x, hi, iv);
-            v += bits_of();
+            unsigned int t = 0;
+#pragma unroll
+            for (int u = 0; u < KPT; ++u) t += iv[u];
+            v += t * (32u / s.m);
         }
         block_scan<KT>(v, s_part, total);
         if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
-        if (!barrier(0x72u)) return;
-        bit = sum_before(wk->run_a, blockIdx.x);
+        together = skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, budget, 0x72u, passed);
+        if (together) bit = sum_before(wk->run_a, blockIdx.x);
+        else before_run(s, lo, s_part32, bit, add);
     }
     for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
         const long long i0 = t0 + (long long)KPT * threadIdx.x;
         if (!keep || gridDim.x == 1) intervals(s, i0, hi, iv);
-        unsigned int total;
-        unsigned long long off = bit + block_scan<KT>(bits_of(), s_part32, total);
-        bit += total;
-        unsigned int dsum = 0;
-#pragma unroll
-        for (int u = 0; u < KPT; ++u) {
-            const unsigned int dw = b * iv[u];
-            unsigned int d = 0;
-            if (dw && dw <= 32u) {
-                const long long w = (long long)(off >> 5);
-                const unsigned int x0 = w < s.delta_lim ? s.delta_words[w] : 0u, x1 = w + 1 < s.delta_lim ? s.delta_words[w + 1] : 0u;
-                d = __brev(__funnelshift_r(x0, x1, (unsigned int)(off & 31ull)) << (32u - dw));
-            }
-            off += dw;
-            dsum += d;
-            k[u] = dsum;
-        }
+        const unsigned int dsum = tile_keys(s, iv, bit, s_part32, k);
         unsigned int tile_sum;
         const unsigned int before = (unsigned int)sum + block_scan<KT>(dsum, s_part32, tile_sum);   // keys are below 2^31: 32-bit sums are exact
 #pragma unroll
@@ -501,11 +519,10 @@ da_decode_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict_
         }
         sum += tile_sum;
     }
-    unsigned int add = 0;
-    if (gridDim.x > 1) {
+    if (together) {
         if (threadIdx.x == 0) wk->run_b[blockIdx.x] = sum;
-        if (!barrier(0x73u)) return;
-        add = (unsigned int)sum_before(wk->run_b, blockIdx.x);
+        if (skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, budget, 0x73u, passed)) add = (unsigned int)sum_before(wk->run_b, blockIdx.x);
+        else before_run(s, lo, s_part32, bit, add);
     }
     for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
         const long long i0 = t0 + (long long)KPT * threadIdx.x;
@@ -565,7 +582,7 @@ extern "C" int skml_da_encode(const int* keys, long long n, void* workspace, uns
 
 extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,
                               long long n_delta_words, long long n, int num_intervals, int unary, long long flag_bits, void* workspace,
-                              long long* zero_pos, int* keys, void* stream) {
+                              long long* zero_pos, int* keys, long long budget_cycles, void* stream) {
     if (num_intervals < 1 || num_intervals > 16 || (num_intervals & (num_intervals - 1)) || !workspace || (unary && !zero_pos))
         return (int)cudaErrorInvalidValue;
     if (n <= 0) return 0;
@@ -594,6 +611,7 @@ extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_
         const cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, total), s);
         if (e != cudaSuccess) return (int)e;
     }
-    void* args[] = {&st, &n, &per, &wk, &keys};
+    long long budget = budget_cycles > 0 ? budget_cycles : KEY_BUDGET;
+    void* args[] = {&st, &n, &per, &wk, &keys, &budget};
     return (int)cudaLaunchCooperativeKernel((const void*)da_decode_kernel, dim3((unsigned)r.runs), dim3(KT), args, 0, s);
 }

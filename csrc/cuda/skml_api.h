@@ -227,13 +227,14 @@ int skml_sm_count();
 // streams (room for 17 and 32 bits a key, whole 64-bit words), waits for the end and leaves {interval count | flag kind
 // << 32, flag bits, delta bits} in done[1..3] (pinned host words). *status_out: 0, SKML_BAD_INPUT (in the low byte) where
 // the keys are not strictly increasing or negative, or another status of a launch that gave up. skml_da_decode inverts
-// the streams; zero_pos: n entries of scratch, unary flags only.
+// the streams; zero_pos: n entries of scratch, unary flags only. budget_cycles: how long its blocks wait for one another (0:
+// a second or so) before each of them does what it waited for itself; the keys are the same.
 long long skml_da_workspace_bytes();
 int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* flag_words, unsigned long long* delta_words,
                    unsigned long long* done, unsigned int* status_out, void* stream);
 int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,
                    long long n_delta_words, long long n, int num_intervals, int unary, long long flag_bits, void* workspace,
-                   long long* zero_pos, int* keys, void* stream);
+                   long long* zero_pos, int* keys, long long budget_cycles, void* stream);
 
 // Expands a minibatch from its transport form (bit-packed column indices, 32-bit row pointers,
 // 8-bit labels; the latter two optional = null) into CSR arrays. `packed` must end with two

@@ -111,6 +111,6 @@ def decode(e: AdaptiveKeys) -> torch.Tensor:
     work = _workspace(dev)
     pos = torch.empty(n, dtype=torch.int64, device=dev) if e.flag_kind else None
     L.check(lib.skml_da_decode(fw.data_ptr(), fw.numel(), dw.data_ptr(), dw.numel(), n, e.num_intervals, e.flag_kind, e.flag_bits,
-                               work.data_ptr(), L.ptr(pos), keys.data_ptr(), L.stream()), "skml_da_decode")
+                               work.data_ptr(), L.ptr(pos), keys.data_ptr(), 0, L.stream()), "skml_da_decode")
     L.count_launches(3 if e.flag_kind else 1)
     return keys

@@ -138,7 +138,7 @@ _SIGS = {
     "skml_sm_count": (c_int, []),
     "skml_da_workspace_bytes": (c_ll, []),
     "skml_da_encode": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
-    "skml_da_decode": (c_int, [c_vp, c_ll, c_vp, c_ll, c_ll, c_int, c_int, c_ll, c_vp, c_vp, c_vp, c_vp]),
+    "skml_da_decode": (c_int, [c_vp, c_ll, c_vp, c_ll, c_ll, c_int, c_int, c_ll, c_vp, c_vp, c_vp, c_ll, c_vp]),
     "skml_unpack_batch": (c_int, [c_vp, c_int, c_ll, c_vp, c_vp, c_ll, c_vp, c_vp, c_vp, c_vp]),
     "skml_unpack_batch_varnibbles": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp, c_vp, c_ll, c_vp, c_vp, c_vp, c_vp]),
     "skml_row_prefix": (c_int, [c_vp, c_ll, c_vp, c_vp]),
