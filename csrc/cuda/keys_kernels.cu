@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "skml_api.h"
 #include "skml_device.cuh"
 
@@ -545,15 +547,25 @@ da_decode_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict_
 
 constexpr size_t ENCODE_SMEM = 4 * (size_t)(STAGE_F + STAGE_D);
 
-// Blocks of a cooperative launch of `kernel` (0: an error).
+// Blocks of a cooperative launch of a kernel on the current device (0: an error, asked for again by the next call). Asked
+// for once per device: a kernel's limit of dynamic shared memory is set for one device only.
+constexpr int KEY_DEVICES = 64;
 template <class K>
-int resident_blocks(K kernel, size_t smem) {
+int resident_blocks(K kernel, size_t smem, std::atomic<int> (&known)[KEY_DEVICES]) {
     int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const bool keep = dev >= 0 && dev < KEY_DEVICES;
+    if (keep) {
+        const int have = known[dev].load(std::memory_order_acquire);
+        if (have) return have;
+    }
     if (smem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, KT, smem) != cudaSuccess || per_sm < 1)
         return 0;
-    return sms < KEY_BLOCKS ? sms : KEY_BLOCKS;
+    const int blocks = sms < KEY_BLOCKS ? sms : KEY_BLOCKS;
+    if (keep) known[dev].store(blocks, std::memory_order_release);
+    return blocks;
 }
 
 }  // namespace
@@ -563,7 +575,8 @@ extern "C" long long skml_da_workspace_bytes() { return (long long)sizeof(KeyWor
 extern "C" int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* flag_words, unsigned long long* delta_words,
                               unsigned long long* done, unsigned int* status_out, void* stream) {
     if (n < 0 || !workspace || !done || !status_out || (n && (!keys || !flag_words || !delta_words))) return (int)cudaErrorInvalidValue;
-    static const int blocks = resident_blocks(da_encode_kernel, ENCODE_SMEM);
+    static std::atomic<int> known[KEY_DEVICES];
+    const int blocks = resident_blocks(da_encode_kernel, ENCODE_SMEM, known);
     if (blocks < 1) return (int)cudaErrorLaunchOutOfResources;
     cudaStream_t s = (cudaStream_t)stream;
     KeyWork* wk = reinterpret_cast<KeyWork*>(workspace);
@@ -586,7 +599,8 @@ extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_
     if (num_intervals < 1 || num_intervals > 16 || (num_intervals & (num_intervals - 1)) || !workspace || (unary && !zero_pos))
         return (int)cudaErrorInvalidValue;
     if (n <= 0) return 0;
-    static const int blocks = resident_blocks(da_decode_kernel, 0);
+    static std::atomic<int> known[KEY_DEVICES];
+    const int blocks = resident_blocks(da_decode_kernel, 0, known);
     if (blocks < 1) return (int)cudaErrorLaunchOutOfResources;
     cudaStream_t s = (cudaStream_t)stream;
     KeyWork* wk = reinterpret_cast<KeyWork*>(workspace);

@@ -807,3 +807,14 @@ def test_key_decode_whose_blocks_stop_waiting_gives_the_keys(n, gaps, unary):
                                        e.num_intervals, e.flag_kind, e.flag_bits, work.data_ptr(), pos.data_ptr(), out.data_ptr(), budget,
                                        L.stream()), "skml_da_decode")
         assert torch.equal(out, keys)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_key_codec_on_every_device_of_a_process():
+    """The encoder's shared memory is above what a kernel gets unasked, and the limit is set for one device only."""
+    from sketchml_b200.ops import keys as K
+    keys = torch.arange(0, 60000, 3, dtype=torch.int32)
+    for d in (0, 1, 0):
+        with torch.cuda.device(d):
+            e = K.encode(keys.to(f"cuda:{d}"))
+            assert torch.equal(K.decode(e).cpu(), keys)
