@@ -245,9 +245,13 @@ __device__ __forceinline__ void write_tails(const int* __restrict__ keys, long l
 // Encoding in one cooperative launch: histogram of every run's delta widths and of all, a grid barrier, the mode and
 // the run's first bits from the histograms (every block adds up those of the runs before its own), then the streams.
 // Runs of one tile keep their deltas in registers across the barrier. 20 us at 1M keys, 17 at 10,000: latency.
+// Mode and lengths are reported once every block is past the barrier, where nothing can fail any more: what the host does
+// with them, it does beside the streams.
+// `words`: where the streams go, the flags and, from the next whole 64-bit word on, the deltas; `room` 64-bit words of it.
+// Null: mode and lengths only. `planned`: a launch of that kind has left the histograms of these keys in the workspace.
 __global__ void __launch_bounds__(KT, 1)
-da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, KeyWork* __restrict__ wk, unsigned int* flag_words,
-                 unsigned int* delta_words, unsigned long long* done, unsigned long long seq) {
+da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, KeyWork* __restrict__ wk, unsigned int* words,
+                 unsigned long long room, bool planned, unsigned long long* done, unsigned long long seq) {
     extern __shared__ __align__(16) unsigned int s_stage[];
     unsigned int* const s_f = s_stage;
     unsigned int* const s_d = s_stage + STAGE_F;
@@ -258,30 +262,33 @@ da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, K
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
     bool bad = false;
-    unsigned int x[KPT], count = 0;   // lane w counts width w
-    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-        const long long i0 = t0 + (long long)KPT * threadIdx.x;
-        load_deltas(keys, i0, hi, x, bad);
+    unsigned int x[KPT];
+    if (!planned) {
+        unsigned int count = 0;   // lane w counts width w
+        for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
+            const long long i0 = t0 + (long long)KPT * threadIdx.x;
+            load_deltas(keys, i0, hi, x, bad);
 #pragma unroll
-        for (int u = 0; u < KPT; ++u) {   // a ballot per bit of the width: all lanes would meet in a few counters
-            const int width = bits_needed((int)x[u]) & 31;
-            unsigned int of_lane = __ballot_sync(0xFFFFFFFFu, i0 + u < hi);
+            for (int u = 0; u < KPT; ++u) {   // a ballot per bit of the width: all lanes would meet in a few counters
+                const int width = bits_needed((int)x[u]) & 31;
+                unsigned int of_lane = __ballot_sync(0xFFFFFFFFu, i0 + u < hi);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) of_lane &= __ballot_sync(0xFFFFFFFFu, (width >> k) & 1) ^ (((unsigned int)lane >> k & 1u) - 1u);
-            count += (unsigned int)__popc(of_lane);
+                for (int k = 0; k < 5; ++k) of_lane &= __ballot_sync(0xFFFFFFFFu, (width >> k) & 1) ^ (((unsigned int)lane >> k & 1u) - 1u);
+                count += (unsigned int)__popc(of_lane);
+            }
         }
+        s_h[warp][lane] = count;
+        if (bad) skml_set_status(&wk->status, SKML_BAD_INPUT, 0x70u);
+        __syncthreads();
+        if (warp == 0) {
+            unsigned int t = 0;
+            for (int w = 0; w < KT / 32; ++w) t += s_h[w][lane];
+            wk->hist[blockIdx.x][lane] = t;
+            if (t) red_add_gpu(&wk->total[lane], t);
+        }
+        unsigned int passed = 0;
+        if (!skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, KEY_BUDGET, 0x71u, passed)) return;
     }
-    s_h[warp][lane] = count;
-    if (bad) skml_set_status(&wk->status, SKML_BAD_INPUT, 0x70u);
-    __syncthreads();
-    if (warp == 0) {
-        unsigned int t = 0;
-        for (int w = 0; w < KT / 32; ++w) t += s_h[w][lane];
-        wk->hist[blockIdx.x][lane] = t;
-        if (t) red_add_gpu(&wk->total[lane], t);
-    }
-    unsigned int passed = 0;
-    if (!skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, KEY_BUDGET, 0x71u, passed)) return;
     unsigned int total = 0;
     if (warp == 0) {
         total = __ldcg(&wk->total[lane]);
@@ -314,10 +321,19 @@ da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, K
         }
     }
     __syncthreads();
-    Out f{flag_words, s_at[0], 0u, (s_at[0] & 31ull) == 0}, d{delta_words, s_at[1], 0u, (s_at[1] & 31ull) == 0};
+    const unsigned long long fwords = (s_at[2] + 63ull) >> 6, dwords = (s_at[3] + 63ull) >> 6;
+    if (!planned && threadIdx.x == 0 && atomicAdd(&wk->ticket, 1u) == gridDim.x - 1) {
+        done[1] = (unsigned long long)m | ((unsigned long long)kind << 32);
+        done[2] = s_at[2];
+        done[3] = s_at[3];
+        __threadfence_system();
+        skml_store_done(done, seq, &wk->status);
+    }
+    if (!words || fwords + dwords > room) return;   // (the same in every block; the host compares the lengths too)
+    Out f{words, s_at[0], 0u, (s_at[0] & 31ull) == 0}, d{words + 2 * fwords, s_at[1], 0u, (s_at[1] & 31ull) == 0};
     for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
         const long long i0 = t0 + (long long)KPT * threadIdx.x;
-        if (per_run > KEY_TILE) load_deltas(keys, i0, hi, x, bad);
+        if (planned || per_run > KEY_TILE) load_deltas(keys, i0, hi, x, bad);
         unsigned int fsum = 0, dsum = 0;   // at most 17 and 32 bits a key
 #pragma unroll
         for (int u = 0; u < KPT; ++u)
@@ -347,17 +363,6 @@ da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, K
         // (the next tile's words are cleared behind the barriers of its scan)
     }
     if (warp == 0) write_tails(keys, hi, n, lb, fb, kind, f, d);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&wk->ticket, 1u) == gridDim.x - 1) {
-            done[1] = (unsigned long long)m | ((unsigned long long)kind << 32);
-            done[2] = s_at[2];
-            done[3] = s_at[3];
-            __threadfence_system();
-            skml_store_done(done, seq, &wk->status);
-        }
-    }
 }
 
 struct Streams {
@@ -572,25 +577,43 @@ int resident_blocks(K kernel, size_t smem, std::atomic<int> (&known)[KEY_DEVICES
 
 extern "C" long long skml_da_workspace_bytes() { return (long long)sizeof(KeyWork); }
 
-extern "C" int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* flag_words, unsigned long long* delta_words,
+// The mode's estimate counts floor(w / b) + 1 intervals of b bits for a delta of w bits, at least as many as it takes, so the
+// streams are no longer than the least estimate: 32 bits a key (the fallback's), and no more than that of 16 intervals with
+// fixed flags, w + 2 + 4 bits. The deltas add up to the last key, below 2^31: their w, at most log2(delta) + 1, are
+// log2(2^31 / n) + 1 on average at most. (And each stream's last word.)
+extern "C" long long skml_da_words(long long n) {
+    int log2n = 0;
+    while ((n >> log2n) > 1) ++log2n;
+    const long long bits = 38 - log2n < 32 ? 38 - log2n : 32;
+    return n > 0 ? (bits * n + 63) / 64 + 4 : 0;
+}
+
+extern "C" int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* words, long long n_words, int planned,
                               unsigned long long* done, unsigned int* status_out, void* stream) {
-    if (n < 0 || !workspace || !done || !status_out || (n && (!keys || !flag_words || !delta_words))) return (int)cudaErrorInvalidValue;
+    if (n < 0 || n_words < 0 || !workspace || !done || !status_out || (n && !keys) || (planned && !words)) return (int)cudaErrorInvalidValue;
     static std::atomic<int> known[KEY_DEVICES];
     const int blocks = resident_blocks(da_encode_kernel, ENCODE_SMEM, known);
     if (blocks < 1) return (int)cudaErrorLaunchOutOfResources;
     cudaStream_t s = (cudaStream_t)stream;
     KeyWork* wk = reinterpret_cast<KeyWork*>(workspace);
-    cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, hist), s);
+    cudaError_t e = planned ? cudaSuccess : cudaMemsetAsync(wk, 0, offsetof(KeyWork, hist), s);
     if (e != cudaSuccess) return (int)e;
     const Runs r = runs_for(n, KEY_TILE, blocks);
     unsigned long long seq = ((*done >> 32) + 1) & 0xFFFFFFFFull;
     long long per_run = r.per_run;
-    unsigned int* f = reinterpret_cast<unsigned int*>(flag_words);
-    unsigned int* d = reinterpret_cast<unsigned int*>(delta_words);
-    void* args[] = {&keys, &n, &per_run, &wk, &f, &d, &done, &seq};
+    unsigned int* out = reinterpret_cast<unsigned int*>(words);
+    unsigned long long room = (unsigned long long)n_words;
+    bool have_plan = planned != 0;
+    void* args[] = {&keys, &n, &per_run, &wk, &out, &room, &have_plan, &done, &seq};
     e = cudaLaunchCooperativeKernel((const void*)da_encode_kernel, dim3((unsigned)r.runs), dim3(KT), args, ENCODE_SMEM, s);
     if (e != cudaSuccess) return (int)e;
-    return skml_wait_done(done, seq, &wk->status, status_out, s);
+    *status_out = 0;
+    if (!planned) {
+        const int rc = skml_wait_done(done, seq, &wk->status, status_out, s);
+        if (rc || *status_out) return rc;
+    }
+    if (words && ((done[2] + 63ull) >> 6) + ((done[3] + 63ull) >> 6) > room) *status_out = SKML_CAPACITY;
+    return 0;
 }
 
 extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,

@@ -223,14 +223,18 @@ int skml_finalize_compact(float* gc, const float* wc, float lambda, int n, float
                           void* stream);
 int skml_sm_count();
 
-// DeltaAdaptive key codec, stand-alone (csrc/cuda/keys_kernels.cu). skml_da_encode chooses the mode and writes the two
-// streams (room for 17 and 32 bits a key, whole 64-bit words), waits for the end and leaves {interval count | flag kind
-// << 32, flag bits, delta bits} in done[1..3] (pinned host words). *status_out: 0, SKML_BAD_INPUT (in the low byte) where
-// the keys are not strictly increasing or negative, or another status of a launch that gave up. skml_da_decode inverts
-// the streams; zero_pos: n entries of scratch, unary flags only. budget_cycles: how long its blocks wait for one another (0:
-// a second or so) before each of them does what it waited for itself; the keys are the same.
+// DeltaAdaptive key codec, stand-alone (csrc/cuda/keys_kernels.cu). skml_da_encode chooses the mode, writes the streams to
+// `words` (the flags, then the deltas, each in whole 64-bit words; null: nothing is written) and leaves {interval count | flag
+// kind << 32, flag bits, delta bits} in done[1..3] (pinned host words). It returns when these are known; the streams follow
+// in the order of `stream`. planned: these keys' call without words was the last one with this workspace and these done
+// words; nothing is waited for. *status_out: 0, SKML_BAD_INPUT (in the low byte) where the keys are not strictly increasing
+// or negative, SKML_CAPACITY where n_words words do not hold the streams (skml_da_words words hold those of any n keys;
+// nothing is written then), or another status of a launch that gave up. skml_da_decode inverts the streams; zero_pos: n
+// entries of scratch, unary flags only. budget_cycles: how long its blocks wait for one another (0: a second or so) before
+// each of them does what it waited for itself; the keys are the same.
+long long skml_da_words(long long n);
 long long skml_da_workspace_bytes();
-int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* flag_words, unsigned long long* delta_words,
+int skml_da_encode(const int* keys, long long n, void* workspace, unsigned long long* words, long long n_words, int planned,
                    unsigned long long* done, unsigned int* status_out, void* stream);
 int skml_da_decode(const unsigned long long* flag_words, long long n_flag_words, const unsigned long long* delta_words,
                    long long n_delta_words, long long n, int num_intervals, int unary, long long flag_bits, void* workspace,

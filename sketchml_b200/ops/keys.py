@@ -7,8 +7,10 @@ themselves, chunk by chunk, without leaving the device (csrc/cuda/compress_kerne
 decode_common.cuh). This module is the library form of the codec, `encode(keys) -> AdaptiveKeys`
 and back, bit for bit equal to the CPU oracle (`oracle.delta_adaptive_encode`). It returns tensors
 of exactly the encoded size, which depends on the data, so `encode` waits once, for the mode and the
-two bit counts (they come through a pinned host word); they are views of one buffer with room for any
-list, copies of their own where that room would be large. csrc/cuda/keys_kernels.cu has the kernels.
+two bit counts (they come through a pinned host word while the streams are written, in the order of
+the calling stream). The tensors are views of one buffer, at most twice as long as they are (or 256 KB
+longer): the room that a list of this length may need, or a copy of what was used of it.
+csrc/cuda/keys_kernels.cu has the kernels.
 """
 from __future__ import annotations
 
@@ -24,7 +26,8 @@ from .codec import DoneWords
 
 
 BAD_INPUT = 5            # SkmlStatus
-KEEP_WORDS = 1 << 22     # 32 MB
+SPARE_WORDS = 1 << 15    # 256 KB: the copy takes 4 us of 77 at 100,000 keys, 3 of 87 at 1M
+ROOM_WORDS = 1 << 22     # 32 MB: from here on the length is found first, by a launch of its own, and no room is allocated unused
 
 
 @dataclass
@@ -84,20 +87,28 @@ def encode(keys: torch.Tensor) -> AdaptiveKeys:
     n, dev, lib, cs = keys.numel(), keys.device, L.lib(), _call_state()
     stream = L.stream()
     work = _workspace(dev)
-    room = (17 * n + 63) // 64   # flags take 17 bits a key at most, deltas 32
-    words = torch.empty(room + (n + 1) // 2, dtype=torch.int64, device=dev)
-    L.check(lib.skml_da_encode(keys.data_ptr(), n, work.data_ptr(), words.data_ptr(), words.data_ptr() + 8 * room, cs.words.data_ptr(),
-                               cs.status_ref, stream), "skml_da_encode")
-    L.count_launches(1)
-    if cs.status.value & 0xFF == BAD_INPUT:
-        raise ValueError("keys must be non-negative and strictly increasing")
-    if cs.status.value:
-        raise RuntimeError(f"skml_da_encode reported status {cs.status.value:#x}")
+    room = lib.skml_da_words(n)
+
+    def run(words: Optional[torch.Tensor], planned: bool = False):
+        L.check(lib.skml_da_encode(keys.data_ptr(), n, work.data_ptr(), L.ptr(words), 0 if words is None else words.numel(), planned,
+                                   cs.words.data_ptr(), cs.status_ref, stream), "skml_da_encode")
+        L.count_launches(1)
+        if cs.status.value & 0xFF == BAD_INPUT:
+            raise ValueError("keys must be non-negative and strictly increasing")
+        if cs.status.value:
+            raise RuntimeError(f"skml_da_encode reported status {cs.status.value:#x}")
+
+    known = room > ROOM_WORDS
+    words = None if known else torch.empty(room, dtype=torch.int64, device=dev)
+    run(words)
     _, mode, flag_bits, delta_bits = cs.words[:4].tolist()
     nf, nd = (flag_bits + 63) // 64, (delta_bits + 63) // 64
-    fw, dw = words[:nf], words[room:room + nd]
-    if words.numel() > KEEP_WORDS:   # a long list does not keep the unused room
-        fw, dw = fw.clone(), dw.clone()
+    if known:
+        words = torch.empty(nf + nd, dtype=torch.int64, device=dev)
+        run(words, True)
+    elif room - (nf + nd) > max(nf + nd, SPARE_WORDS):
+        words = words[:nf + nd].clone()
+    fw, dw = words[:nf], words[nf:nf + nd]
     return AdaptiveKeys(n, mode & 0xFFFFFFFF, mode >> 32, flag_bits, delta_bits, fw, dw)
 
 

@@ -137,7 +137,8 @@ _SIGS = {
     "skml_hot_colsum": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_f, c_vp, c_vp, c_vp, c_vp]),
     "skml_sm_count": (c_int, []),
     "skml_da_workspace_bytes": (c_ll, []),
-    "skml_da_encode": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "skml_da_words": (c_ll, [c_ll]),
+    "skml_da_encode": (c_int, [c_vp, c_ll, c_vp, c_vp, c_ll, c_int, c_vp, c_vp, c_vp]),
     "skml_da_decode": (c_int, [c_vp, c_ll, c_vp, c_ll, c_ll, c_int, c_int, c_ll, c_vp, c_vp, c_vp, c_ll, c_vp]),
     "skml_unpack_batch": (c_int, [c_vp, c_int, c_ll, c_vp, c_vp, c_ll, c_vp, c_vp, c_vp, c_vp]),
     "skml_unpack_batch_varnibbles": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp, c_vp, c_ll, c_vp, c_vp, c_vp, c_vp]),

@@ -818,3 +818,38 @@ def test_key_codec_on_every_device_of_a_process():
         with torch.cuda.device(d):
             e = K.encode(keys.to(f"cuda:{d}"))
             assert torch.equal(K.decode(e).cpu(), keys)
+
+
+@pytest.mark.parametrize("n", [1, 40_000, 300_000, 20_000_000])
+@pytest.mark.parametrize("gap", [1, 100])
+def test_key_code_holds_no_more_memory_than_twice_its_length(n, gap):
+    """The streams' buffer is their length, twice that or 256 KB more at most; a long list is never given room that its
+    code does not need, not even for the length of the call."""
+    from sketchml_b200.ops import keys as K
+    keys = torch.arange(0, gap * n, gap, dtype=torch.int32, device="cuda")
+    K.decode(K.encode(keys[:8]))                # (the pinned words)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    e = K.encode(keys)
+    used = 8 * (e.flag_words.numel() + e.delta_words.numel())
+    held = {t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in (e.flag_words, e.delta_words)}
+    assert sum(held.values()) <= max(2 * used, used + (256 << 10))
+    if n > 14_000_000:
+        assert torch.cuda.max_memory_allocated() - before <= used + (1 << 20)
+    assert torch.equal(K.decode(e), keys)
+
+
+def test_key_encode_does_not_leave_its_room():
+    from sketchml_b200.ops import keys as K
+    from sketchml_b200.ops import lib as L
+    keys = torch.arange(0, 300_000, 3, dtype=torch.int32, device="cuda")
+    e = K.encode(keys)
+    cs, need = K._call_state(), e.flag_words.numel() + e.delta_words.numel()
+    for room, ok in ((need, True), (need - 1, False)):
+        out, work = torch.full((need + 8,), -1, dtype=torch.int64, device="cuda"), K._workspace(keys.device)
+        L.check(L.lib().skml_da_encode(keys.data_ptr(), keys.numel(), work.data_ptr(), out.data_ptr(), room, 0, cs.words.data_ptr(), cs.status_ref,
+                                       L.stream()), "skml_da_encode")
+        assert (cs.status.value == 0) == ok and bool((out[need if ok else 0:] == -1).all())
+        if ok:
+            assert torch.equal(out[:need], torch.cat([e.flag_words, e.delta_words]))

@@ -511,3 +511,24 @@ def test_decoding_keys_pins_no_memory(monkeypatch):
     words = torch.zeros(4, dtype=torch.int64)
     for kind in (0, 1):
         assert keys.decode(keys.AdaptiveKeys(10, 4, kind, 20, 80, words, words)).numel() == 10
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 64, 65, 1000, 1 << 14, 100_000])
+def test_room_for_a_key_code_holds_every_list(n):
+    """Lists whose deltas are as wide as n keys below 2^31 allow, one width throughout or two, powers of two and one less,
+    short lists that start at 0: no code is longer than the room its list gets."""
+    from sketchml_b200.compress import oracle
+    from sketchml_b200.ops import lib as L
+    room = L.lib().skml_da_words(n)
+    rng = np.random.default_rng(n)
+    top = (2 ** 31 - 1) // n
+    lists = [np.full(n, top), np.full(n, 1 << (int(top).bit_length() - 1)), np.full(n, max(1, (1 << (int(top).bit_length() - 1)) - 1)),
+             rng.integers(1, top + 1, n), np.where(np.arange(n) % 2, max(1, 2 * top - 1), 1),
+             np.where(np.arange(n) == n // 2, 2 ** 31 - n, 1), (2.0 ** rng.uniform(0, np.log2(top), n)).astype(np.int64)]
+    for d in lists:
+        keys = np.cumsum(d)
+        for first in (0, keys[0]):
+            k = keys.copy() - (keys[0] - first)
+            assert k[-1] < 2 ** 31
+            e = oracle.delta_adaptive_encode(k.astype(np.int32))
+            assert (e["flag_bits"] + 63) // 64 + (e["delta_bits"] + 63) // 64 <= room
