@@ -7,11 +7,12 @@
 //   first in two separate streams in java.util.BitSet order (stream bit p = bit (p & 31) of 32-bit
 //   word p >> 5).
 //
-// Every kernel cuts the keys into at most KEY_BLOCKS contiguous runs of whole tiles, one run per block, so the prefix
-// sums over runs are short enough for every block to add up on its own: encoding and decoding are one cooperative launch
-// each (two more where flags are unary). What bounds both at ordinary sizes is the chain of trips to L2, two or three
-// grid barriers among them, and the host's calls around the one wait. 1M keys there and back: 72 us, 80 as seven launches
-// (plan, pack, widths, keys, offsets and fills; a device time of 43 us against 40 here), 300 with library scans.
+// Every kernel cuts the keys into contiguous runs of whole tiles, one run per block, so the prefix sums over runs are short
+// enough for every block to add up on its own. Encoding is one cooperative launch (two where its output would be large, see
+// skml_da_encode), and so is decoding of fixed-width flags where a tile a block is enough (1.2M keys; otherwise three launches,
+// and two more where flags are unary). What bounds both at ordinary sizes is the chain of trips to L2, two or three grid barriers among them, and the
+// host's calls around the one wait. 1M keys there and back: 68 us, 80 as seven launches (plan, pack, widths, keys, offsets
+// and fills; 43 us of kernels against 36 here), 300 with library scans.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -28,7 +29,7 @@ constexpr int KEY_TILE = KT * KPT;
 constexpr int KEY_BLOCKS = 192;     // at most one block per SM: a grid barrier of 592 small blocks took twice as long
 constexpr int STAGE_F = KEY_TILE * 17 / 32 + 2;   // words of one tile's flag bits (at most 17 a key, plus a word of misalignment)
 constexpr int STAGE_D = KEY_TILE + 2;             // the same for its delta bits (at most 32 a key)
-constexpr int ZT = 256, Z_TILE = 4 * ZT, Z_BLOCKS = 592;   // unary flags: search for the zero bits
+constexpr int LT = 256, LPT = 4, L_TILE = LT * LPT, L_BLOCKS = 592;   // unary flags, long lists: four small blocks per SM
 constexpr long long KEY_BUDGET = 2000000000ll;    // cycles a grid barrier waits at most
 
 struct KeyWork {
@@ -36,8 +37,8 @@ struct KeyWork {
     unsigned int pad[13];
     unsigned int total[32];             // encode: delta widths of all keys; cleared by the host
     unsigned int hist[KEY_BLOCKS][32];  // encode: delta widths of the runs
-    unsigned long long run_a[KEY_BLOCKS], run_b[KEY_BLOCKS];   // decode: sums over the runs
-    unsigned long long zeros[Z_BLOCKS];
+    unsigned long long run_a[L_BLOCKS], run_b[L_BLOCKS];       // decode: sums over the runs
+    unsigned long long zeros[L_BLOCKS];
 };
 
 struct Runs {
@@ -82,6 +83,15 @@ __device__ __forceinline__ unsigned long long sum_before(const unsigned long lon
 #pragma unroll 8
     for (int i = threadIdx.x & 31; i < count; i += 32) v += __ldcg(sums + i);
     return warp_sum(v);
+}
+
+// The same by the whole block: for the many runs of small blocks the trips of one warp would follow one another.
+template <int THREADS>
+__device__ __forceinline__ unsigned long long block_sum_before(const unsigned long long* sums, int count, unsigned long long* part) {
+    unsigned long long v = 0, total;
+    for (int i = threadIdx.x; i < count; i += THREADS) v += __ldcg(sums + i);
+    block_scan<THREADS>(v, part, total);
+    return total;
 }
 
 // Interval counts, widths and flag of a delta under m intervals of b = 1 << lb bits.
@@ -374,15 +384,16 @@ struct Streams {
     int unary;
 };
 
-// Interval counts of a thread's keys, from i0 on (0 beyond `hi`).
-__device__ __forceinline__ void intervals(const Streams& s, long long i0, long long hi, unsigned int (&iv)[KPT]) {
+// Interval counts of a thread's N keys (at most eight), from i0 on (0 beyond `hi`).
+template <int N>
+__device__ __forceinline__ void intervals(const Streams& s, long long i0, long long hi, unsigned int (&iv)[N]) {
 #pragma unroll
-    for (int u = 0; u < KPT; ++u) iv[u] = 0;
+    for (int u = 0; u < N; ++u) iv[u] = 0;
     if (i0 >= hi) return;
     if (s.unary) {
         long long before = i0 ? s.zero_pos[i0 - 1] : -1;
 #pragma unroll
-        for (int u = 0; u < KPT; ++u)
+        for (int u = 0; u < N; ++u)
             if (i0 + u < hi) {
                 const long long z = s.zero_pos[i0 + u];
                 iv[u] = (unsigned int)(z - before - 1);
@@ -399,7 +410,7 @@ __device__ __forceinline__ void intervals(const Streams& s, long long i0, long l
         win = ((unsigned long long)lo | ((unsigned long long)hw << 32)) >> (off & 31ull);
     }
 #pragma unroll
-    for (int u = 0; u < KPT; ++u)
+    for (int u = 0; u < N; ++u)
         if (i0 + u < hi) {
             const unsigned int bits = fb ? (unsigned int)(win >> (fb * u)) & ((1u << fb) - 1u) : 0u;
             iv[u] = (fb ? __brev(bits) >> (32u - fb) : 0u) + 1u;
@@ -407,26 +418,26 @@ __device__ __forceinline__ void intervals(const Streams& s, long long i0, long l
 }
 
 // Unary flags: zero bits of every run of flag words (a key's flag ends at its zero bit).
-__global__ void __launch_bounds__(ZT) da_zero_count_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
+__global__ void __launch_bounds__(LT) da_zero_count_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
                                                            KeyWork* __restrict__ wk) {
-    __shared__ unsigned long long s_part[ZT / 32];
+    __shared__ unsigned long long s_part[LT / 32];
     const long long nw = (flag_bits + 31) >> 5, lo = per_run * blockIdx.x, hi = lo + per_run < nw ? lo + per_run : nw;
     unsigned long long v = 0, total;
-    for (long long w = lo + threadIdx.x; w < hi; w += ZT) {
+    for (long long w = lo + threadIdx.x; w < hi; w += LT) {
         const long long rest = flag_bits - (w << 5);
         v += __popc(~flag_words[w] & (rest >= 32 ? 0xFFFFFFFFu : ((1u << rest) - 1u)));
     }
-    block_scan<ZT>(v, s_part, total);
+    block_scan<LT>(v, s_part, total);
     if (threadIdx.x == 0) wk->zeros[blockIdx.x] = total;
 }
 
 // Stream position of the i-th zero bit.
-__global__ void __launch_bounds__(ZT) da_zero_pos_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
+__global__ void __launch_bounds__(LT) da_zero_pos_kernel(const unsigned int* __restrict__ flag_words, long long flag_bits, long long per_run,
                                                          const KeyWork* __restrict__ wk, long long n, long long* __restrict__ pos) {
-    __shared__ unsigned long long s_part[ZT / 32];
+    __shared__ unsigned long long s_part[LT / 32];
     const long long nw = (flag_bits + 31) >> 5, lo = per_run * blockIdx.x, hi = lo + per_run < nw ? lo + per_run : nw;
-    unsigned long long base = sum_before(wk->zeros, blockIdx.x);
-    for (long long w0 = lo; w0 < hi; w0 += ZT) {
+    unsigned long long base = block_sum_before<LT>(wk->zeros, blockIdx.x, s_part);
+    for (long long w0 = lo; w0 < hi; w0 += LT) {
         const long long w = w0 + threadIdx.x;
         unsigned int z = 0;
         if (w < hi) {
@@ -434,7 +445,7 @@ __global__ void __launch_bounds__(ZT) da_zero_pos_kernel(const unsigned int* __r
             z = ~flag_words[w] & (rest >= 32 ? 0xFFFFFFFFu : ((1u << rest) - 1u));
         }
         unsigned long long total;
-        unsigned long long idx = base + block_scan<ZT>((unsigned long long)__popc(z), s_part, total);
+        unsigned long long idx = base + block_scan<LT>((unsigned long long)__popc(z), s_part, total);
         while (z) {
             const int bit = __ffs(z) - 1;
             z &= z - 1;
@@ -445,19 +456,27 @@ __global__ void __launch_bounds__(ZT) da_zero_pos_kernel(const unsigned int* __r
     }
 }
 
-// Keys of a tile, each counted from the tile's first bit on and within its thread only: k[u] = sum of the deltas of this
-// thread's keys up to the u-th. `bit`: the tile's first delta bit, then the next tile's. Returns the thread's sum.
-__device__ __forceinline__ unsigned int tile_keys(const Streams& s, const unsigned int (&iv)[KPT], unsigned long long& bit, unsigned int* part32,
-                                                  unsigned int (&k)[KPT]) {
-    const unsigned int b = 32u / s.m;
-    unsigned int bits = 0, total;
+// Bits of the deltas of a thread's keys.
+template <int N>
+__device__ __forceinline__ unsigned int delta_bits(const Streams& s, const unsigned int (&iv)[N]) {
+    unsigned int t = 0;
 #pragma unroll
-    for (int u = 0; u < KPT; ++u) bits += b * iv[u];
-    unsigned long long off = bit + block_scan<KT>(bits, part32, total);
+    for (int u = 0; u < N; ++u) t += iv[u];
+    return t * (32u / s.m);
+}
+
+// Keys of a tile, each counted from its thread's first one: k[u] = sum of the deltas up to the thread's u-th. `bit`: the
+// tile's first delta bit, then the next tile's. Returns the thread's sum.
+template <int THREADS, int N>
+__device__ __forceinline__ unsigned int tile_keys(const Streams& s, const unsigned int (&iv)[N], unsigned long long& bit, unsigned int* part32,
+                                                  unsigned int (&k)[N]) {
+    const unsigned int b = 32u / s.m;
+    unsigned int total;
+    unsigned long long off = bit + block_scan<THREADS>(delta_bits(s, iv), part32, total);
     bit += total;
     unsigned int dsum = 0;
 #pragma unroll
-    for (int u = 0; u < KPT; ++u) {
+    for (int u = 0; u < N; ++u) {
         const unsigned int dw = b * iv[u];
         unsigned int d = 0;
         if (dw && dw <= 32u) {
@@ -479,75 +498,95 @@ __device__ __noinline__ void before_run(Streams s, long long lo, unsigned int* p
     for (long long t0 = 0; t0 < lo; t0 += KEY_TILE) {
         unsigned int iv[KPT], k[KPT], tile_sum;
         intervals(s, t0 + (long long)KPT * threadIdx.x, lo, iv);
-        block_scan<KT>(tile_keys(s, iv, bit, part32, k), part32, tile_sum);
+        block_scan<KT>(tile_keys<KT>(s, iv, bit, part32, k), part32, tile_sum);
         sum += tile_sum;
     }
 }
 
-// Decoding in one cooperative launch: delta bits of every run, a grid barrier, the run's keys counted from the key
-// before it, a grid barrier, the sum of the runs before it added. Runs of one tile keep flags and keys in registers.
+// Decoding in one cooperative launch, where a block has one tile: its delta bits, a grid barrier, its keys counted from the
+// key before them, a grid barrier, the sum of the tiles before it added; flags and keys stay in registers.
 // The caller is not told how the launch went, so it cannot fail: where a barrier gives up, a block works out for itself
 // what it waited for, and goes to no barrier any more (the others give up with it: the status word says so).
 __global__ void __launch_bounds__(KT, 1)
-da_decode_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk, int* __restrict__ keys, long long budget) {
+da_decode_kernel(Streams s, long long n, KeyWork* __restrict__ wk, int* __restrict__ keys, long long budget) {
     __shared__ unsigned long long s_part[KT / 32];
     __shared__ unsigned int s_part32[KT / 32];
-    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
-    const bool keep = per_run <= KEY_TILE;
-    unsigned int passed = 0;
+    const long long lo = (long long)KEY_TILE * blockIdx.x, i0 = lo + (long long)KPT * threadIdx.x;
+    unsigned int passed = 0, iv[KPT], k[KPT], sum, add = 0;
     bool together = gridDim.x > 1;   // (one block has nothing to wait for)
-    unsigned int iv[KPT], k[KPT], add = 0;
-    unsigned long long bit = 0, sum = 0;
+    unsigned long long bit = 0;
+    intervals(s, i0, n, iv);
     if (together) {
-        unsigned long long v = 0, total;
-        for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-            intervals(s, t0 + (long long)KPT * threadIdx.x, hi, iv);
-            unsigned int t = 0;
-#pragma unroll
-            for (int u = 0; u < KPT; ++u) t += iv[u];
-            v += t * (32u / s.m);
-        }
-        block_scan<KT>(v, s_part, total);
+        unsigned long long total;
+        block_scan<KT>((unsigned long long)delta_bits(s, iv), s_part, total);
         if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
         together = skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, budget, 0x72u, passed);
         if (together) bit = sum_before(wk->run_a, blockIdx.x);
         else before_run(s, lo, s_part32, bit, add);
     }
-    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-        const long long i0 = t0 + (long long)KPT * threadIdx.x;
-        if (!keep || gridDim.x == 1) intervals(s, i0, hi, iv);
-        const unsigned int dsum = tile_keys(s, iv, bit, s_part32, k);
-        unsigned int tile_sum;
-        const unsigned int before = (unsigned int)sum + block_scan<KT>(dsum, s_part32, tile_sum);   // keys are below 2^31: 32-bit sums are exact
-#pragma unroll
-        for (int u = 0; u < KPT; ++u) {
-            k[u] += before;
-            if (!keep && i0 + u < hi) keys[i0 + u] = (int)k[u];
-        }
-        sum += tile_sum;
-    }
+    const unsigned int before = block_scan<KT>(tile_keys<KT>(s, iv, bit, s_part32, k), s_part32, sum);   // keys are below 2^31: 32-bit sums are exact
     if (together) {
         if (threadIdx.x == 0) wk->run_b[blockIdx.x] = sum;
         if (skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, budget, 0x73u, passed)) add = (unsigned int)sum_before(wk->run_b, blockIdx.x);
         else before_run(s, lo, s_part32, bit, add);
     }
-    for (long long t0 = lo; t0 < hi; t0 += KEY_TILE) {
-        const long long i0 = t0 + (long long)KPT * threadIdx.x;
-        if (!keep) {   // (what this thread has written itself)
+    add += before;
+    if (i0 + KPT <= n && (reinterpret_cast<uintptr_t>(keys) & 15) == 0) {
 #pragma unroll
-            for (int u = 0; u < KPT; ++u)
-                if (i0 + u < hi) k[u] = (unsigned int)keys[i0 + u];
-        }
-        if (i0 + KPT <= hi && (reinterpret_cast<uintptr_t>(keys) & 15) == 0) {
+        for (int q = 0; q < KPT / 4; ++q)
+            *reinterpret_cast<uint4*>(keys + i0 + 4 * q) = make_uint4(k[4 * q] + add, k[4 * q + 1] + add, k[4 * q + 2] + add, k[4 * q + 3] + add);
+    } else {
 #pragma unroll
-            for (int q = 0; q < KPT / 4; ++q)
-                *reinterpret_cast<uint4*>(keys + i0 + 4 * q) = make_uint4(k[4 * q] + add, k[4 * q + 1] + add, k[4 * q + 2] + add, k[4 * q + 3] + add);
-        } else {
-#pragma unroll
-            for (int u = 0; u < KPT; ++u)
-                if (i0 + u < hi) keys[i0 + u] = (int)(k[u] + add);
-        }
+        for (int u = 0; u < KPT; ++u)
+            if (i0 + u < n) keys[i0 + u] = (int)(k[u] + add);
     }
+}
+
+// Longer lists, and unary flags, where two launches have come before and the stream is never idle for the host: three
+// launches, a run of tiles per block and four small blocks per SM, which hide one another's trips to memory. With the runs of
+// tiles in one block of 1024 per SM and grid barriers, 2M keys took 38 us instead of 28, 20M 206 instead of 143 and 100M 1870
+// instead of 1430; 100,000 keys with unary flags 35 instead of 32. (Fixed-width flags, one launch instead of three: 100,000
+// keys 14.7 instead of 17.3, 1M 18.8 instead of 19.3.)
+// Delta bits of every run.
+__global__ void __launch_bounds__(LT) da_width_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk) {
+    __shared__ unsigned long long s_part[LT / 32];
+    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
+    unsigned long long v = 0, total;
+    for (long long t0 = lo; t0 < hi; t0 += L_TILE) {
+        unsigned int iv[LPT];
+        intervals(s, t0 + LPT * (long long)threadIdx.x, hi, iv);
+        v += delta_bits(s, iv);
+    }
+    block_scan<LT>(v, s_part, total);
+    if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
+}
+
+// Keys of every run counted from the key before it, and the runs' sums.
+__global__ void __launch_bounds__(LT) da_extract_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk, int* __restrict__ keys) {
+    __shared__ unsigned long long s_part[LT / 32];
+    __shared__ unsigned int s_part32[LT / 32];
+    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
+    unsigned long long bit = block_sum_before<LT>(wk->run_a, blockIdx.x, s_part);
+    unsigned int sum = 0;
+    for (long long t0 = lo; t0 < hi; t0 += L_TILE) {
+        const long long i0 = t0 + LPT * (long long)threadIdx.x;
+        unsigned int iv[LPT], k[LPT], tile_sum;
+        intervals(s, i0, hi, iv);
+        const unsigned int before = sum + block_scan<LT>(tile_keys<LT>(s, iv, bit, s_part32, k), s_part32, tile_sum);
+#pragma unroll
+        for (int u = 0; u < LPT; ++u)
+            if (i0 + u < hi) keys[i0 + u] = (int)(k[u] + before);
+        sum += tile_sum;
+    }
+    if (threadIdx.x == 0) wk->run_b[blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(LT) da_offset_kernel(long long n, long long per_run, const KeyWork* __restrict__ wk, int* __restrict__ keys) {
+    __shared__ unsigned long long s_part[LT / 32];
+    if (blockIdx.x == 0) return;
+    const long long lo = per_run * blockIdx.x, hi = lo + per_run < n ? lo + per_run : n;
+    const int add = (int)block_sum_before<LT>(wk->run_b, blockIdx.x, s_part);
+    for (long long i = lo + threadIdx.x; i < hi; i += LT) keys[i] += add;
 }
 
 constexpr size_t ENCODE_SMEM = 4 * (size_t)(STAGE_F + STAGE_D);
@@ -638,17 +677,23 @@ extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_
     if (unary) {
         const long long nw = (flag_bits + 31) >> 5;
         if (nw > st.flag_lim) return (int)cudaErrorInvalidValue;
-        const Runs f = runs_for(nw, Z_TILE, Z_BLOCKS);
-        da_zero_count_kernel<<<f.runs, ZT, 0, s>>>(st.flag_words, flag_bits, f.per_run, wk);
-        da_zero_pos_kernel<<<f.runs, ZT, 0, s>>>(st.flag_words, flag_bits, f.per_run, wk, n, zero_pos);
+        const Runs f = runs_for(nw, L_TILE, L_BLOCKS);
+        da_zero_count_kernel<<<f.runs, LT, 0, s>>>(st.flag_words, flag_bits, f.per_run, wk);
+        da_zero_pos_kernel<<<f.runs, LT, 0, s>>>(st.flag_words, flag_bits, f.per_run, wk, n, zero_pos);
     }
     const Runs r = runs_for(n, KEY_TILE, blocks);
-    long long per = r.per_run;
+    if (r.per_run > KEY_TILE || (unary && r.runs > 1)) {
+        const Runs l = runs_for(n, L_TILE, L_BLOCKS);
+        da_width_kernel<<<l.runs, LT, 0, s>>>(st, n, l.per_run, wk);
+        da_extract_kernel<<<l.runs, LT, 0, s>>>(st, n, l.per_run, wk, keys);
+        da_offset_kernel<<<l.runs, LT, 0, s>>>(n, l.per_run, wk, keys);
+        return (int)cudaGetLastError();
+    }
     if (r.runs > 1) {
         const cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, total), s);
         if (e != cudaSuccess) return (int)e;
     }
     long long budget = budget_cycles > 0 ? budget_cycles : KEY_BUDGET;
-    void* args[] = {&st, &n, &per, &wk, &keys, &budget};
+    void* args[] = {&st, &n, &wk, &keys, &budget};
     return (int)cudaLaunchCooperativeKernel((const void*)da_decode_kernel, dim3((unsigned)r.runs), dim3(KT), args, 0, s);
 }

@@ -26,6 +26,7 @@ from .codec import DoneWords
 
 
 BAD_INPUT = 5            # SkmlStatus
+TILE = 8192              # keys of a block where a list is decoded by one launch
 SPARE_WORDS = 1 << 15    # 256 KB: the copy takes 4 us of 77 at 100,000 keys, 3 of 87 at 1M
 ROOM_WORDS = 1 << 22     # 32 MB: from here on the length is found first, by a launch of its own, and no room is allocated unused
 
@@ -123,5 +124,5 @@ def decode(e: AdaptiveKeys) -> torch.Tensor:
     pos = torch.empty(n, dtype=torch.int64, device=dev) if e.flag_kind else None
     L.check(lib.skml_da_decode(fw.data_ptr(), fw.numel(), dw.data_ptr(), dw.numel(), n, e.num_intervals, e.flag_kind, e.flag_bits,
                                work.data_ptr(), L.ptr(pos), keys.data_ptr(), 0, L.stream()), "skml_da_decode")
-    L.count_launches(3 if e.flag_kind else 1)
+    L.count_launches((1 if n <= (TILE if e.flag_kind else 148 * TILE) else 3) + (2 if e.flag_kind else 0))
     return keys
