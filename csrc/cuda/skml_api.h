@@ -200,7 +200,8 @@ int skml_compact_settle(float* g, const float* w, unsigned int* bitmap, int dim,
                         double* partials, double* tmpl, void* stream);
 // Frequent columns of a batch with a transposed index, as lists per (row tile, item): `pos` are their positions in the
 // index, column h has the items item0[h] .. item0[h + 1] (64 entries of a tile at most to each), ptr the lists' bounds in
-// quads of four entries (row_tiles * items + 1 of them), loc and val as in SkmlDenseIndex. skml_hot_count counts the entries per (row tile, column), skml_hot_fill puts them into their lists
+// quads of four entries (row_tiles * items + 1 of them), loc and val as in SkmlDenseIndex. skml_hot_bounds finds where the
+// entries of a column begin in every row tile (bound[row_tiles + 1][columns]), skml_hot_fill puts them into their lists
 // (loc filled with tile_rows, val with 0 before), skml_hot_colsum leaves all column sums as skml_colsum_settle does:
 // the other columns, n_short of at most four entries and n_medium longer ones in `bins`, are summed from the index. `partial`: scratch of row_tiles * items floats.
 typedef struct SkmlHotColumns {
@@ -214,8 +215,8 @@ typedef struct SkmlHotColumns {
     float* val;
     float* partial;
 } SkmlHotColumns;
-int skml_hot_count(const SkmlHotColumns* hot, const int* colptr, const int* rowidx, int* cnt, void* stream);
-int skml_hot_fill(const SkmlHotColumns* hot, const int* colptr, const int* rowidx, const float* svals, void* stream);
+int skml_hot_bounds(const SkmlHotColumns* hot, const int* colptr, const int* rowidx, int* bound, void* stream);
+int skml_hot_fill(const SkmlHotColumns* hot, const int* bound, const int* item_column, const int* rowidx, const float* svals, void* stream);
 int skml_hot_colsum(const SkmlHotColumns* hot, const int* bins, int n_short, int n_medium, const int* colptr, const int* rowidx,
                     const float* svals, const int* ucols, const float* coef, const float* w, float lambda, float* out, double* partials, double* tmpl, void* stream);
 int skml_gather_compact(const float* w, const int* ucols, int n, float* wc, void* stream);

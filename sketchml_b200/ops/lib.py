@@ -132,8 +132,8 @@ _SIGS = {
     "skml_gen_rows": (c_int, [c_vp, c_vp, c_vp, c_ll, c_ll, c_int, c_int, c_d, c_int, c_int, c_f, c_vp, c_ull, c_vp]),
     "skml_glm_coef": (c_int, [c_vp, c_vp, c_vp, c_vp, c_ll, c_ll, c_ll, c_d, c_vp, c_ll, c_int, c_f, c_vp, c_vp, c_vp, c_ll, c_vp]),
     "skml_colsum": (c_int, [c_vp] * 8 + [c_int] * 4 + [c_vp, c_vp, c_f, c_vp, c_vp]),
-    "skml_hot_count": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_vp, c_vp, c_vp]),
-    "skml_hot_fill": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_vp, c_vp, c_vp]),
+    "skml_hot_bounds": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_vp, c_vp, c_vp]),
+    "skml_hot_fill": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_vp, c_vp, c_vp, c_vp]),
     "skml_hot_colsum": (c_int, [C.POINTER(HotColumnsArgs), c_vp, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_f, c_vp, c_vp, c_vp, c_vp]),
     "skml_sm_count": (c_int, []),
     "skml_da_workspace_bytes": (c_ll, []),

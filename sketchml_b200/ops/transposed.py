@@ -127,6 +127,8 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
     """The columns with at least two entries per row tile on average (and more than the short ones'), and which they are;
     (None, None) where they hold too few entries to pay for tiles, partial sums and one more launch: column sums of 15M
     entries 95 -> 65 us, of 30M with values 141 -> 110, of 6M with values 21 -> 26, of 1.9M 18 -> 23."""
+    if rowidx.numel() < HOT_MIN_ENTRIES:
+        return None, None
     dev, lib = rowidx.device, L.lib()
     a = L.HotColumnsArgs()
     a.rows = rows
@@ -138,8 +140,9 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
         return None, None
     a.items = a.columns
     a.pos = L.ptr(pos)
-    per = torch.empty((a.row_tiles, a.columns), dtype=torch.int32, device=dev)
-    L.check(lib.skml_hot_count(C.byref(a), L.ptr(colptr), L.ptr(rowidx), L.ptr(per), L.stream()), "skml_hot_count")
+    bound = torch.empty((a.row_tiles + 1, a.columns), dtype=torch.int32, device=dev)
+    L.check(lib.skml_hot_bounds(C.byref(a), L.ptr(colptr), L.ptr(rowidx), L.ptr(bound), L.stream()), "skml_hot_bounds")
+    per = bound[1:] - bound[:-1]
     k = (per.amax(0) + HOT_SEGMENT - 1) // HOT_SEGMENT
     item0 = torch.zeros(a.columns + 1, dtype=torch.int32, device=dev)
     torch.cumsum(k, 0, dtype=torch.int32, out=item0[1:])
@@ -148,7 +151,7 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
     a.items, a.wide = int(item0[-1]), wide.shape[0]
     if a.row_tiles * a.items + rowidx.numel() // 4 >= L.DT_LISTS_MAX:
         return None, None
-    column = torch.repeat_interleave(torch.arange(a.columns, device=dev), k, output_size=a.items)
+    column = torch.repeat_interleave(torch.arange(a.columns, device=dev, dtype=torch.int32), k, output_size=a.items)
     segment = torch.arange(a.items, device=dev, dtype=torch.int32) - item0[column]
     quads = ((per[:, column] - HOT_SEGMENT * segment).clamp_(0, HOT_SEGMENT) + 3) >> 2
     ptr = torch.zeros(a.row_tiles * a.items + 1, dtype=torch.int32, device=dev)
@@ -157,7 +160,7 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
     loc = torch.full((n,), a.tile_rows if a.tile_rows < 32768 else a.tile_rows - 65536, dtype=torch.int16, device=dev)   # unsigned 16-bit patterns
     val = None if svals is None else torch.zeros(n, dtype=torch.float32, device=dev)
     a.item0, a.info, a.wide_info, a.ptr, a.loc, a.val = L.ptr(item0), L.ptr(info), L.ptr(wide), L.ptr(ptr), L.ptr(loc), L.ptr(val)
-    L.check(lib.skml_hot_fill(C.byref(a), L.ptr(colptr), L.ptr(rowidx), L.ptr(svals), L.stream()), "skml_hot_fill")
+    L.check(lib.skml_hot_fill(C.byref(a), L.ptr(bound), L.ptr(column), L.ptr(rowidx), L.ptr(svals), L.stream()), "skml_hot_fill")
     return HotColumns(a, [pos, item0, info, wide, ptr, loc] + ([val] if val is not None else []), int(a.row_tiles * a.items)), is_hot
 
 

@@ -532,3 +532,13 @@ def test_room_for_a_key_code_holds_every_list(n):
             assert k[-1] < 2 ** 31
             e = oracle.delta_adaptive_encode(k.astype(np.int32))
             assert (e["flag_bits"] + 63) // 64 + (e["delta_bits"] + 63) // 64 <= room
+
+
+def test_batches_too_small_for_frequent_column_lists_cost_nothing(monkeypatch):
+    """A batch with fewer entries than the lists need is not looked through first."""
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T.L, "lib", lambda: pytest.fail("the library was called"))
+    monkeypatch.setattr(torch, "nonzero", lambda *a: pytest.fail("the columns were counted"))
+    cnt = torch.tensor([60, 40])
+    colptr = torch.tensor([0, 60, 100], dtype=torch.int32)
+    assert T._hot_columns(torch.tensor([3, 5]), colptr, torch.zeros(100, dtype=torch.int32), None, cnt, 100) == (None, None)
