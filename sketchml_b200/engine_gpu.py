@@ -232,9 +232,11 @@ class GpuEngine:
         # 176 us + combine 92 us against 103 us), because the frequent columns, which hold most entries, already
         # gather near-sequential coefficients in the per-column form, and a 192 KB tile allows one block per SM.
         tiled = bool(conf.extras.get("tiled_index", False))
-        hot = need + csr.nnz * (9 if csr.values is not None else 3) <= 0.8 * free   # lists of the frequent columns beside
+        hot_left = int(0.8 * free - need)   # lists of the frequent columns, as far as there is room beside the rest
         for b in range(csr.rows // B if not dense else 0):
-            bi = build_batch_index(csr, b * B, (b + 1) * B, tiled=tiled, hot=hot)
+            bi = build_batch_index(csr, b * B, (b + 1) * B, tiled=tiled, hot=True, hot_budget=hot_left)
+            if bi.hot is not None:
+                hot_left -= bi.hot.nbytes()
             if bi.n_cols > self.st.dim * 2 // 3 or bi.n_cols > self.st.n_max:
                 return  # near-dense without a tiled form (see build_dense_index): keep the scatter path
             idx.append(bi)

@@ -123,10 +123,12 @@ def _build_tiled(csr: DeviceCSR, lo: int, hi: int, e0: int, e1: int, rows: torch
                       torch.tensor([n, 1 if n else 0, 0, 0], dtype=torch.int64, device=dev), part)
 
 
-def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor, svals: Optional[torch.Tensor], cnt: torch.Tensor, rows: int):
+def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor, svals: Optional[torch.Tensor], cnt: torch.Tensor, rows: int,
+                 budget: Optional[int] = None):
     """The columns with at least two entries per row tile on average (and more than the short ones'), and which they are;
     (None, None) where they hold too few entries to pay for tiles, partial sums and one more launch: column sums of 15M
-    entries 95 -> 65 us, of 30M with values 141 -> 110, of 6M with values 21 -> 26, of 1.9M 18 -> 23."""
+    entries 95 -> 65 us, of 30M with values 141 -> 110, of 6M with values 21 -> 26, of 1.9M 18 -> 23.
+    None too where building the lists, or the lists and their scratch afterwards, would take more than ``budget`` bytes."""
     if rowidx.numel() < HOT_MIN_ENTRIES:
         return None, None
     dev, lib = rowidx.device, L.lib()
@@ -138,6 +140,9 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
     a.columns = pos.numel()
     if int(cnt[pos.long()].sum()) < HOT_MIN_ENTRIES:
         return None, None
+    room = a.columns * (8 * a.row_tiles + 100)   # bounds and counts per tile; positions, items and places of the columns
+    if budget is not None and room > budget:
+        return None, None
     a.items = a.columns
     a.pos = L.ptr(pos)
     bound = torch.empty((a.row_tiles + 1, a.columns), dtype=torch.int32, device=dev)
@@ -146,17 +151,24 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
     k = (per.amax(0) + HOT_SEGMENT - 1) // HOT_SEGMENT
     item0 = torch.zeros(a.columns + 1, dtype=torch.int32, device=dev)
     torch.cumsum(k, 0, dtype=torch.int32, out=item0[1:])
-    info = torch.stack([pos, item0[:-1], k, ucols[pos.long()].to(torch.int32)], 1).contiguous()
-    wide = info[k > 1].contiguous()
-    a.items, a.wide = int(item0[-1]), wide.shape[0]
+    a.items = int(item0[-1])
     if a.row_tiles * a.items + rowidx.numel() // 4 >= L.DT_LISTS_MAX:
         return None, None
+    room += 12 * a.row_tiles * a.items + 32 * a.items   # the lists' lengths, bounds and partial sums; the items' columns
+    if budget is not None and room > budget:
+        return None, None
+    info = torch.stack([pos, item0[:-1], k, ucols[pos.long()].to(torch.int32)], 1).contiguous()
+    wide = info[k > 1].contiguous()
+    a.wide = wide.shape[0]
     column = torch.repeat_interleave(torch.arange(a.columns, device=dev, dtype=torch.int32), k, output_size=a.items)
     segment = torch.arange(a.items, device=dev, dtype=torch.int32) - item0[column]
-    quads = ((per[:, column] - HOT_SEGMENT * segment).clamp_(0, HOT_SEGMENT) + 3) >> 2
+    quads = per[:, column]
+    quads.sub_(segment.mul_(HOT_SEGMENT)).clamp_(0, HOT_SEGMENT).add_(3).bitwise_right_shift_(2)
     ptr = torch.zeros(a.row_tiles * a.items + 1, dtype=torch.int32, device=dev)
     torch.cumsum(quads.flatten(), 0, dtype=torch.int32, out=ptr[1:])
     n = 4 * int(ptr[-1])
+    if budget is not None and room + n * (2 if svals is None else 6) > budget:
+        return None, None
     loc = torch.full((n,), a.tile_rows if a.tile_rows < 32768 else a.tile_rows - 65536, dtype=torch.int16, device=dev)   # unsigned 16-bit patterns
     val = None if svals is None else torch.zeros(n, dtype=torch.float32, device=dev)
     a.item0, a.info, a.wide_info, a.ptr, a.loc, a.val = L.ptr(item0), L.ptr(info), L.ptr(wide), L.ptr(ptr), L.ptr(loc), L.ptr(val)
@@ -164,10 +176,10 @@ def _hot_columns(ucols: torch.Tensor, colptr: torch.Tensor, rowidx: torch.Tensor
     return HotColumns(a, [pos, item0, info, wide, ptr, loc] + ([val] if val is not None else []), int(a.row_tiles * a.items)), is_hot
 
 
-def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False, hot: bool = False) -> BatchIndex:
+def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False, hot: bool = False, hot_budget: Optional[int] = None) -> BatchIndex:
     """``tiled``: the row-tiled form (coefficients of a row tile in shared memory, no atomics); needs fewer than
     2^20 tiles, i.e. any batch that fits a GPU. ``hot``: the frequent columns of the per-column form as lists per row
-    tile, where that pays (see `_hot_columns`)."""
+    tile, where that pays and takes no more than ``hot_budget`` bytes (see `_hot_columns`)."""
     dev = csr.cols.device
     e0, e1 = int(csr.rowptr[lo]), int(csr.rowptr[hi])
     cols = csr.cols[e0:e1]
@@ -183,7 +195,7 @@ def build_batch_index(csr: DeviceCSR, lo: int, hi: int, tiled: bool = False, hot
     colptr = torch.zeros(n + 1, dtype=torch.int32, device=dev)
     colptr[1:] = torch.cumsum(cnt, 0).to(torch.int32)
     pos = torch.arange(n, device=dev, dtype=torch.int32)
-    frequent, is_hot = _hot_columns(ucols, colptr, rowidx, svals, cnt, hi - lo) if hot and n else (None, None)
+    frequent, is_hot = _hot_columns(ucols, colptr, rowidx, svals, cnt, hi - lo, hot_budget) if hot and n else (None, None)
     if frequent is not None:
         none = torch.zeros(0, dtype=torch.int32, device=dev)
         short, medium = pos[cnt <= SHORT_MAX], pos[(cnt > SHORT_MAX) & ~is_hot]

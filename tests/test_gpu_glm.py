@@ -1,4 +1,6 @@
 """GPU numerics of the GLM kernels against plain PyTorch fp32/fp64 references."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -552,3 +554,41 @@ def test_frequent_columns_from_row_tiles_match_the_per_column_form(binary, rows,
     want = exact[uc] + loss.lam * w[uc].double()
     bound = 2 ** -20 * (size[uc] + loss.lam * w[uc].double().abs()) + 1e-12
     assert bool(((outs[1].double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("binary", [True, False])
+@pytest.mark.parametrize("rows,tile_rows_max,nnz,dim", [(200_000, 2000, 20, 10_000),   # two to four entries a list: mostly padding and bounds
+                                                      (200_000, 49152, 20, 300), (100_000, 49152, 30, 100_000)])
+def test_frequent_column_lists_keep_to_their_budget(rows, tile_rows_max, nnz, dim, binary, monkeypatch):
+    """A budget below what building them takes is refused before it is exceeded, whatever the lists look like; twice as
+    much is enough."""
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T, "TILE_ROWS_MAX", tile_rows_max)
+    monkeypatch.setattr(T, "HOT_MIN_ENTRIES", 1)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    cols = (dim * torch.rand(rows * nnz, generator=g, device="cuda") ** 1.5).long().clamp_(max=dim - 1)
+    order = torch.argsort(cols, stable=True)
+    rowidx = (order // nnz).to(torch.int32)      # (a column may hold a row twice: the lists do not mind)
+    ucols, cnt = torch.unique_consecutive(cols[order], return_counts=True)
+    colptr = torch.zeros(ucols.numel() + 1, dtype=torch.int32, device="cuda")
+    colptr[1:] = torch.cumsum(cnt, 0)
+    svals = None if binary else torch.rand(rows * nnz, generator=g, device="cuda")
+    args = (ucols, colptr, rowidx, svals, cnt, rows)
+
+    def peak(budget):
+        gc.collect()
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        h, _ = T._hot_columns(*args, budget)
+        scratch = 4 * h.partial_floats if h is not None else 0
+        return h, max(torch.cuda.max_memory_allocated() - before, torch.cuda.memory_allocated() - before + scratch)
+
+    h, need = peak(None)
+    assert h is not None and need >= 4 * cols.numel() / 2
+    del h
+    for budget in (need - (64 << 10), need // 2, need // 8, 0):      # (an allocation is rounded up to 512 bytes)
+        h, took = peak(budget)
+        assert h is None and took <= budget + cnt.numel() * 24 + (64 << 10)   # (which columns are frequent is looked at in any case)
+    h, _ = peak(2 * need)
+    assert h is not None
