@@ -393,13 +393,14 @@ __device__ __forceinline__ void cold_columns(const ColdColumns& c, int first, in
         mi = position(t + 2 * turn);
         bounds();
         float acc = 0.f;
-        for (int e = e0 + sub; e < e1; e += 4 * LANES) {
+        const unsigned int end = (unsigned int)e1;   // (steps past the end do not wrap)
+        for (unsigned int e = (unsigned int)(e0 + sub); e < end; e += 4 * LANES) {
             int r[4];
             float x[4], v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                r[u] = e + u * LANES < e1 ? c.rowidx[e + u * LANES] : -1;
-                x[u] = HAS_VALS && e + u * LANES < e1 ? c.svals[e + u * LANES] : 1.f;
+            for (unsigned int u = 0; u < 4; ++u) {
+                r[u] = e + u * LANES < end ? c.rowidx[e + u * LANES] : -1;
+                x[u] = HAS_VALS && e + u * LANES < end ? c.svals[e + u * LANES] : 1.f;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) v[u] = r[u] >= 0 ? __ldg(coef + r[u]) : 0.f;

@@ -592,3 +592,24 @@ def test_frequent_column_lists_keep_to_their_budget(rows, tile_rows_max, nnz, di
         assert h is None and took <= budget + cnt.numel() * 24 + (64 << 10)   # (which columns are frequent is looked at in any case)
     h, _ = peak(2 * need)
     assert h is not None
+
+
+@pytest.mark.parametrize("count", [3, 20])       # a lane's column, eight lanes' column
+def test_a_column_that_ends_at_the_last_entry_there_can_be(count):
+    """Entries are counted in 32 bits: a lane's steps past the end of a column that ends just below 2^31 do not come back
+    as entries."""
+    import ctypes
+    from sketchml_b200.ops import lib as L
+    last, rows = 2 ** 31 - 1, 64
+    ints = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    rowidx = torch.zeros(last, dtype=torch.int32, device="cuda")
+    rowidx[last - count:] = torch.arange(count, device="cuda", dtype=torch.int32)
+    coef, w, out = torch.rand(rows, device="cuda"), torch.zeros(2, device="cuda"), torch.full((2,), 7.0, device="cuda")
+    bins, colptr, ucols = ints(0), ints(last - count, last), ints(0, 1)
+    ptr, info, loc, partial = ints(0, 0), ints(1, 0, 1, 1), torch.full((4,), rows, dtype=torch.int16, device="cuda"), torch.zeros(1, device="cuda")
+    h = L.HotColumnsArgs(rows=rows, row_tiles=1, tile_rows=rows, columns=1, items=1, wide=0, info=L.ptr(info), ptr=L.ptr(ptr), loc=L.ptr(loc),
+                         partial=L.ptr(partial))
+    L.check(L.lib().skml_hot_colsum(ctypes.byref(h), L.ptr(bins), int(count <= 4), int(count > 4), L.ptr(colptr), L.ptr(rowidx), None, L.ptr(ucols),
+                                    L.ptr(coef), L.ptr(w), 0.0, L.ptr(out), None, None, L.stream()), "skml_hot_colsum")
+    want = float(coef[:count].double().sum())
+    assert abs(float(out[0]) - want) <= 1e-6 * want and float(out[1]) == 0.0
