@@ -147,6 +147,7 @@ struct WsLayout {
 static inline long long al256(long long x) { return (x + 255) & ~255ll; }
 
 #define PRIV_MIN_KEYS 1000000    // inserts of fewer keys stay with atomics in L2 (see priv_layout)
+#define PRIV_MIN_ROOM 4000000    // the same where only room for so many is known, not how many there are (see fill_params)
 #define PRIV_MAX_PASSES 4        // parts that a key is hashed against per row, on average, at most
 #define PRIV_UNITS 2             // units of four keys a thread inserts per round
 #define PRIV_MAX_PARTS 2048      // parts of all groups' rows (their blocks are listed in shared memory)
@@ -3394,11 +3395,17 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
         skml_pick_hashes(p.seed, p.step, p.rank, (unsigned int)g, p.rows, p.hash_ids[g]);
         for (int r = 0; r < p.rows && p.mixers; ++r) p.mixers = p.hash_ids[g][r] < 3;
     }
-    // codes of a byte, 255 meaning "no key": at most 255 buckets in a group (from three groups on a group has at most
-    // half of all buckets and half a group more)
+    // codes of a byte, 255 meaning "no key": at most 255 buckets in a group (of 256 buckets, from three groups on a group has
+    // at most 171)
     const int bins = a->given_splits ? (int)a->n_given + 1 : p.q;
+    // A launch that could insert in shared memory but has too few keys for it is 3 to 4.6 us slower than one of the plain
+    // kernel (247,000 keys 45.1 -> 48.3, 426,000 54.7 -> 59.3, 722,000 68.8 -> 72.2). Where the number is on the device only
+    // (gradients that were scattered and compacted: one key to three to nine entries where columns are frequent and rare, up
+    // to one each where they are alike), n_max says little: 4M keys of 6M alike 149 -> 139, but 247,000 to 722,000 of 1.1M to
+    // 4.5M keys the above.
+    const long long enough = a->meta && a->n_bound <= 0 ? PRIV_MIN_ROOM : PRIV_MIN_KEYS;
     const long long n_known = !a->meta ? a->n_value : (a->n_bound > 0 && a->n_bound < a->n_max ? a->n_bound : a->n_max);
-    p.priv = p.mixers && !p.huffman && n_known >= PRIV_MIN_KEYS && (bins <= 255 || (bins == 256 && p.G >= 3));
+    p.priv = p.mixers && !p.huffman && n_known >= enough && (bins <= 255 || (bins == 256 && p.G >= 3));
     return 0;
 }
 

@@ -48,7 +48,7 @@ typedef struct SkmlCompressArgs {
     long long zero_slot;           // 1 = bytes of the local slot that the payload does not cover are zero afterwards
     unsigned long long* done_word; // pinned host word of the checked call (skml_compress_checked sets done_seq itself)
     unsigned long long done_seq;
-    long long n_bound;               // non-zeros at most where the caller knows better than n_max (0: n_max)
+    long long n_bound;             // number of non-zeros, or hardly more, where the caller knows it (0: n_max at most)
 } SkmlCompressArgs;
 
 long long skml_compress_workspace_bytes(long long n_max, long long bin_num, long long group_num, long long row_num,

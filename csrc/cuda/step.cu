@@ -15,7 +15,7 @@ static int batch_consumed(const SkmlStepArgs* a, cudaStream_t stream) {
 }
 
 // The gradient's way into the model: through the fused compress and decode kernels, or through a baseline's codes.
-// `n_bound`: as many non-zeros at most. `batch_keys`: keys and count lie in the batch's own buffers, which are the feeder's again once they are read.
+// `n_bound`: as many non-zeros there are (0: not known here, n_max at most). `batch_keys`: keys and count lie in the batch's own buffers, which are the feeder's again once they are read.
 static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* meta, float* vals, float* dense_vals, long long n_bound,
                           bool batch_keys, void* stream) {
     if (a->coded) {
@@ -124,5 +124,5 @@ extern "C" int skml_train_step(SkmlStepArgs* a, void* stream_) {
     rc = skml_compact_settle(a->g, a->w, a->bitmap, (int)a->dim, (float)a->lambda, a->block_counts, a->meta, a->keys,
                           a->gvals, a->dense_vals, a->n_max, a->status, a->partials, a->partials_template, stream_);
     if (rc) return rc;
-    return apply_gradient(a, a->keys, a->meta, a->gvals, a->dense_vals, a->n_max, false, stream_);
+    return apply_gradient(a, a->keys, a->meta, a->gvals, a->dense_vals, 0, false, stream_);
 }

@@ -850,3 +850,26 @@ def test_key_encode_does_not_leave_its_room():
         assert (cs.status.value == 0) == ok and bool((out[need if ok else 0:] == -1).all())
         if ok:
             assert torch.equal(out[:need], torch.cat([e.flag_words, e.delta_words]))
+
+
+@pytest.mark.parametrize("n,n_max,bound,in_shared", [
+    (1_200_000, 1_200_000, 0, False), (1_200_000, 3_999_999, 0, False), (1_200_000, 4_000_000, 0, True),   # room alone says little
+    (999_999, 4_000_000, 0, False), (1_200_000, 1_200_000, 1_200_000, True), (1_200_000, 2_000_000, 1_300_000, True)])
+def test_where_the_sketch_is_inserted_when_the_number_of_keys_is_on_the_device(n, n_max, bound, in_shared):
+    """Room for 1M keys does not choose the kernel that inserts in shared memory, which costs launches of fewer keys 3 us
+    and more; a known number does. The payload is the same either way."""
+    import ctypes
+    from sketchml_b200.ops import GpuCompressor
+    from sketchml_b200.ops import lib as L
+    dim = 3 * n
+    keys, vals = _sparse_grad(n, dim, seed=n)
+    kt, vt = torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda()
+    comp, known = (GpuCompressor(dim, m, 256, 8, 3, 0.2, seed=11) for m in (n_max, n))
+    buf = torch.zeros(comp.capacity, dtype=torch.uint8, device="cuda")
+    meta, status = torch.tensor([n, 1, 0, 0], dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    a = comp.make_args(kt, vt, meta, 3, 0, 1, buf.data_ptr(), buf.numel(), [buf.data_ptr()], [None], status, None, None)
+    a.n_bound = bound
+    L.check(L.lib().skml_compress_sparse(ctypes.byref(a), L.stream()), "skml_compress_sparse")
+    assert int(status) == 0
+    assert (int(comp.workspace[:256].view(torch.int64)[15]) != 0) == in_shared       # the stage's time stamp
+    assert comp.payload_bytes(buf) == known.payload_bytes(known.compress_local(kt, vt, step=3))
