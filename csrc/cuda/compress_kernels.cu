@@ -153,15 +153,19 @@ static inline long long al256(long long x) { return (x + 255) & ~255ll; }
 #define PRIV_MAX_PARTS 2048      // parts of all groups' rows (their blocks are listed in shared memory)
 #define PRIV_BYTES (136 * 1024)  // cells that fit a block's shared memory
 
+// Whether launches of these sizes may insert in shared memory: enough keys, rows of integer mixers only, codes of a byte.
+static inline bool priv_sizes(long long n_max, long long q, long long rows) { return n_max >= PRIV_MIN_KEYS && rows <= 3 && q <= 256; }
+
 // Bytes of the copies that blocks make of the parts they have worked on: at most one copy per block and part border.
 static inline long long copies_bytes(long long n_max, long long G, long long rows, double col_ratio, long long grid) {
-    if (n_max < PRIV_MIN_KEYS) return 0;
     const long long cells = (long long)(col_ratio * (double)n_max) + 2;
     const long long len = cells < PRIV_BYTES ? cells : PRIV_BYTES;
     return (grid + rows * (2 * cells / PRIV_BYTES + G)) * (len + 32);
 }
 
-static WsLayout ws_layout(long long n_max, long long q, long long G, long long rows, double col_ratio, long long grid) {
+// `priv`: with what the insert in shared memory takes, a byte a key and the copies. (It lies behind everything else but the
+// tables.)
+static WsLayout ws_layout(long long n_max, long long q, long long G, long long rows, double col_ratio, long long grid, bool priv) {
     WsLayout L;
     long long o = 0;
     L.ctrl = o; o += 256;
@@ -184,8 +188,8 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
     L.bins = o; o += al256(n_max * 2);
     L.gkeys = o; o += al256((n_max + 4 * SKML_MAX_GROUPS + 8) * 4);
     L.tables_cap = rows * ((long long)(col_ratio * (double)n_max) + 2 + G) + 64 + 4 * G;  // groups' tables start at multiples of 4 cells
-    L.gcodes = o; o += al256(n_max + 4 * SKML_MAX_GROUPS + 8);
-    L.copies_cap = copies_bytes(n_max, G, rows, col_ratio, grid);
+    L.gcodes = o; o += priv ? al256(n_max + 4 * SKML_MAX_GROUPS + 8) : 0;
+    L.copies_cap = priv ? copies_bytes(n_max, G, rows, col_ratio, grid) : 0;
     if (L.copies_cap < L.tables_cap * 4) L.copies_cap = L.tables_cap * 4;
     L.tables = o; o += al256(L.copies_cap);
     L.total = o;
@@ -195,7 +199,13 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
 extern "C" long long skml_compress_workspace_bytes(long long n_max, long long bin_num, long long group_num,
                                                    long long row_num, double col_ratio, long long grid) {
     if (grid <= 0 || grid > MAX_GRID) grid = MAX_GRID;
-    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, grid).total;
+    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, grid, priv_sizes(n_max, bin_num, row_num)).total;
+}
+
+extern "C" long long skml_compress_workspace_least(long long n_max, long long bin_num, long long group_num,
+                                                   long long row_num, double col_ratio, long long grid) {
+    if (grid <= 0 || grid > MAX_GRID) grid = MAX_GRID;
+    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, grid, false).total;
 }
 
 // Upper bound of the payload size for n_max non-zeros (sparse kind) or dim codes (dense kind).
@@ -3327,7 +3337,12 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     if (a->key_encoder != SKML_KEYS_DELTA_BINARY && a->key_encoder != SKML_KEYS_DELTA_ADAPTIVE) return (int)cudaErrorInvalidValue;
     grid = a->grid > 0 ? (int)a->grid : device_sms();
     if (grid > MAX_GRID) grid = MAX_GRID;
-    WsLayout L = ws_layout(a->n_max, a->bin_num, a->group_num, a->row_num, a->col_ratio, grid);
+    bool priv_room = priv_sizes(a->n_max, a->bin_num, a->row_num);
+    WsLayout L = ws_layout(a->n_max, a->bin_num, a->group_num, a->row_num, a->col_ratio, grid, priv_room);
+    if (L.total > a->workspace_bytes && priv_room) {   // (a workspace of the least size)
+        priv_room = false;
+        L = ws_layout(a->n_max, a->bin_num, a->group_num, a->row_num, a->col_ratio, grid, false);
+    }
     if (L.total > a->workspace_bytes) return (int)cudaErrorInvalidValue;
     p.keys = a->keys;
     p.vals = a->vals;
@@ -3405,7 +3420,7 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     // 4.5M keys the above.
     const long long enough = a->meta && a->n_bound <= 0 ? PRIV_MIN_ROOM : PRIV_MIN_KEYS;
     const long long n_known = !a->meta ? a->n_value : (a->n_bound > 0 && a->n_bound < a->n_max ? a->n_bound : a->n_max);
-    p.priv = p.mixers && !p.huffman && n_known >= enough && (bins <= 255 || (bins == 256 && p.G >= 3));
+    p.priv = priv_room && p.mixers && !p.huffman && n_known >= enough && (bins <= 255 || (bins == 256 && p.G >= 3));
     return 0;
 }
 
@@ -3416,7 +3431,7 @@ extern "C" long long skml_compress_splits_offset(long long n_max, long long bin_
                                                  long long row_num, double col_ratio, long long grid) {
     long long g = grid > 0 ? grid : device_sms();
     if (g > MAX_GRID) g = MAX_GRID;
-    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, g).splits_raw;
+    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, g, false).splits_raw;   // (in front of all that differs)
 }
 
 // Function attributes and the co-residency limit are looked up once per kernel (one process

@@ -53,6 +53,10 @@ typedef struct SkmlCompressArgs {
 
 long long skml_compress_workspace_bytes(long long n_max, long long bin_num, long long group_num, long long row_num,
                                         double col_ratio, long long grid);
+// The same for launches that never insert in shared memory (Huffman-coded tables, un-fused launches); others with a
+// workspace of this size insert with atomics, too.
+long long skml_compress_workspace_least(long long n_max, long long bin_num, long long group_num, long long row_num,
+                                        double col_ratio, long long grid);
 long long skml_payload_capacity(long long n_max, long long dim, long long bin_num, long long group_num,
                                 long long row_num, double col_ratio);
 long long skml_compress_splits_offset(long long n_max, long long bin_num, long long group_num, long long row_num,

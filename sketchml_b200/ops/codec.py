@@ -122,7 +122,9 @@ class GpuCompressor(_KeepsArgs):
         self.quantile_summary = 1 if quantile_summary == "sketch" else 0
         self.device = torch.device(device)
         ws_n = max(self.n_max, 1)
-        self.ws_bytes = int(self.lib.skml_compress_workspace_bytes(ws_n, bin_num, group_num, row_num, self.col_ratio, 0))
+        # (un-fused launches and Huffman-coded tables never insert in shared memory)
+        room = self.lib.skml_compress_workspace_bytes if fused and self.cell_bits != 0 else self.lib.skml_compress_workspace_least
+        self.ws_bytes = int(room(ws_n, bin_num, group_num, row_num, self.col_ratio, 0))
         self.workspace = torch.zeros(self.ws_bytes, dtype=torch.uint8, device=self.device)
         # the dense kind (one code per coordinate) is only reachable when nnz can exceed 2/3 dim
         self.dense_possible = self.n_max * 3 > self.dim * 2

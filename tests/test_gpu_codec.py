@@ -873,3 +873,17 @@ def test_where_the_sketch_is_inserted_when_the_number_of_keys_is_on_the_device(n
     assert int(status) == 0
     assert (int(comp.workspace[:256].view(torch.int64)[15]) != 0) == in_shared       # the stage's time stamp
     assert comp.payload_bytes(buf) == known.payload_bytes(known.compress_local(kt, vt, step=3))
+
+
+def test_settings_changed_after_a_workspace_of_the_least_size():
+    """A compressor made for Huffman-coded tables has no room for the insert in shared memory: with plain tables set
+    afterwards it inserts with atomics, the payload being the same."""
+    from sketchml_b200.ops import GpuCompressor
+    n, dim = 1_100_000, 4_000_000
+    keys, vals = _sparse_grad(n, dim, seed=5)
+    kt, vt = torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda()
+    c, plain = GpuCompressor(dim, n, 256, 8, 3, 0.2, seed=11, cell_bits=0), GpuCompressor(dim, n, 256, 8, 3, 0.2, seed=11)
+    c.compress_local(kt, vt, step=3)
+    assert c.ws_bytes < plain.ws_bytes - n
+    c.cell_bits = -1
+    assert c.payload_bytes(c.compress_local(kt, vt, step=3)) == plain.payload_bytes(plain.compress_local(kt, vt, step=3))

@@ -542,3 +542,17 @@ def test_batches_too_small_for_frequent_column_lists_cost_nothing(monkeypatch):
     cnt = torch.tensor([60, 40])
     colptr = torch.tensor([0, 60, 100], dtype=torch.int32)
     assert T._hot_columns(torch.tensor([3, 5]), colptr, torch.zeros(100, dtype=torch.int32), None, cnt, 100) == (None, None)
+
+
+def test_compress_workspace_grows_for_the_insert_in_shared_memory_only():
+    """A byte a key and the tables' copies where a launch may insert in shared memory: from 1M keys on, at most three rows,
+    codes of a byte. Elsewhere nothing but buckets, key lists, chunk tables and cells of four bytes."""
+    from sketchml_b200.ops import lib as L
+    least, full = L.lib().skml_compress_workspace_least, L.lib().skml_compress_workspace_bytes
+    for n, q, rows, more in ((999_999, 256, 3, False), (1_000_000, 256, 3, True), (2_000_000, 256, 4, False), (2_000_000, 257, 3, False),
+                             (10_000_000, 64, 2, True)):
+        args = (n, q, 8, rows, 0.2, 148)
+        assert (full(*args) > least(*args) + n) == more and (full(*args) == least(*args)) != more
+        per_key = 2 + 4 + 4 * rows * 0.2 + 24 / 1024 + 4 * rows * 0.2 / 1024
+        fixed = least(1, q, 8, rows, 0.2, 148)
+        assert abs(least(*args) - fixed - per_key * n) < 16384
