@@ -671,19 +671,23 @@ class GpuEngine:
     def stage_times_us(self):
         """Durations of the stages of this rank's last fused compress and decode launches, from the
         `globaltimer` stamps the kernels leave in their workspaces (synchronises). Compress:
-        summary, split query, bucketize + count, scatter + sketch insert, key code, narrow + publish.
-        Decode: prepare (including the wait for the peers' payloads), accumulate, claims."""
+        summary, split query, bucketize + count, scatter + sketch insert, key code, narrow + publish;
+        `sketch_insert`: the share of an insert in shared memory (None where it is atomics of the scatter). Decode: prepare (including the wait for the peers' payloads), accumulate, claims."""
         if self.mode != "sketch":
             return None
         import numpy as np
         last = (self.t.step - 1) & 1  # the decode kernel keeps the stamps of even and odd steps apart
-        c = self.comp.workspace[:256].cpu().numpy().view(np.int64)[8:15]
+        c = self.comp.workspace[:256].cpu().numpy().view(np.int64)[8:16]
         kind = 1 if getattr(self, "_last_index", None) is not None else int(self.st.meta[1])  # index batches are sparse
         if kind != 1 or not all(0 <= int(c[i + 1] - c[i]) < 10**9 for i in range(6)):
             return None   # dense-kind or empty step: the sparse compress kernel left no stamps
+        insert = None
+        if c[4] <= c[7] <= c[5]:   # this launch had a stage of its own for the insert: between scatter and key code
+            insert = float(c[7] - c[4]) / 1e3
+            c[4] = c[7]
         dall = self.dec.workspace[:256].cpu().numpy().view(np.int64)
         d, dprev = dall[8 + 4 * last:12 + 4 * last], dall[8 + 4 * (1 - last):12 + 4 * (1 - last)]
-        return {"compress": [float(c[i + 1] - c[i]) / 1e3 for i in range(6)],
+        return {"compress": [float(c[i + 1] - c[i]) / 1e3 for i in range(6)], "sketch_insert": insert,
                 "decode": [float(d[i + 1] - d[i]) / 1e3 for i in range(3)],
                 # idle time between the end of the compress kernel's last stage and the start of the decode kernel
                 "compress_to_decode_gap": float(d[0] - c[6]) / 1e3,

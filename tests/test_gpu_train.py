@@ -298,3 +298,25 @@ def test_zip_step_after_a_reported_error_changes_nothing_and_is_raised(rows, opt
     eng.check()
     assert not torch.equal(before[0], state[0])
     t.close()
+
+
+def test_a_step_of_over_a_million_columns():
+    """The number of keys comes from the column index and the device: the sketch is inserted in shared memory, which has a
+    stage of its own between scatter and key code; the weights are those of the staged launches, which insert with atomics."""
+    from sketchml_b200.trainer import Trainer
+    ws = []
+    for fused in (True, False):
+        t = Trainer(_conf(feature_num=3_000_000, syn_rows=120_000, syn_nnz_per_row=30, syn_zipf_s=0.0, valid_ratio=0.0, batch_sample_ratio=0.5,
+                          quant_bin_num=256, extras={"fused": fused}))
+        t.load_data()
+        assert all(bi.n_cols > 1_000_000 for bi in t.engine.tindex)
+        for i in range(2):
+            t.train_one_iteration(0, i)
+        if fused:
+            st = t.engine.stage_times_us()
+            total = sum(st["compress"])
+            assert 0 < st["sketch_insert"] < st["compress"][3] < total    # the scatter's stage holds it
+            assert st["sketch_insert"] > st["compress"][4] / 8            # (it was counted as key code)
+        ws.append(t.model.weights.detach().cpu().clone())
+        t.close()
+    assert torch.count_nonzero(ws[0]) > 1_000_000 and torch.equal(ws[0], ws[1])
