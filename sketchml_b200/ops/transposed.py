@@ -51,7 +51,7 @@ class HotColumns:
         return sum(t.numel() * t.element_size() for t in self.tensors)
 
     def bind(self, partial: torch.Tensor) -> None:
-        """Scratch of a step; batches that run one after another share it."""
+        """Scratch of the engine's step; batches that run one after another share it."""
         self.partial = partial
         self.args.partial = partial.data_ptr()
 
@@ -329,9 +329,11 @@ def glm_grad_transposed(csr: DeviceCSR, bi: BatchIndex, w: torch.Tensor, coef: t
         L.count_launches(3)
         return
     if bi.hot is not None:
-        if not bi.hot.args.partial:
-            bi.hot.bind(torch.empty(bi.hot.partial_floats, dtype=torch.float32, device=coef.device))
-        L.check(lib.skml_hot_colsum(C.byref(bi.hot.args), L.ptr(bi.bins), bi.n_short, bi.n_medium, L.ptr(bi.colptr), L.ptr(bi.rowidx),
+        # scratch of this call's own: the same index may be used on another stream or thread at the same time
+        partial = torch.empty(bi.hot.partial_floats, dtype=torch.float32, device=coef.device)
+        args = L.HotColumnsArgs.from_buffer_copy(bi.hot.args)
+        args.partial = partial.data_ptr()
+        L.check(lib.skml_hot_colsum(C.byref(args), L.ptr(bi.bins), bi.n_short, bi.n_medium, L.ptr(bi.colptr), L.ptr(bi.rowidx),
                                     L.ptr(bi.svals), L.ptr(bi.ucols), L.ptr(coef), L.ptr(w), float(lam), L.ptr(out_vals), None, None,
                                     L.stream()), "skml_hot_colsum")
         L.count_launches(3)

@@ -613,3 +613,42 @@ def test_a_column_that_ends_at_the_last_entry_there_can_be(count):
                                     L.ptr(coef), L.ptr(w), 0.0, L.ptr(out), None, None, L.stream()), "skml_hot_colsum")
     want = float(coef[:count].double().sum())
     assert abs(float(out[0]) - want) <= 1e-6 * want and float(out[1]) == 0.0
+
+
+def test_frequent_column_sums_on_two_streams_at_once(monkeypatch):
+    """Two gradients from one batch's index at the same time have scratch of their own; the index keeps none."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.models.loss import L2LogLoss
+    from sketchml_b200.ops import DeviceCSR
+    from sketchml_b200.ops import transposed as T
+    monkeypatch.setattr(T, "TILE_ROWS_MAX", 4096)
+    monkeypatch.setattr(T, "HOT_MIN_ENTRIES", 1)
+    rows, dim, nnz, dev = 120_000, 20_000, 20, torch.device("cuda")
+    g = torch.Generator().manual_seed(4)
+    cols = (dim * torch.rand((rows, nnz), generator=g) ** 3).int().clamp_(max=dim - 1).sort(1).values.flatten()
+    csr = DeviceCSR(CSRMatrix(torch.arange(rows + 1) * nnz, cols, None, torch.sign(torch.rand(rows, generator=g) - 0.5), dim), dev)
+    bi, loss = T.build_batch_index(csr, 0, rows, hot=True), L2LogLoss(1e-3)
+    assert bi.hot is not None
+    ws = [(torch.randn(dim, generator=g) * 0.3).to(dev) for _ in range(2)]
+    state = [(torch.zeros(rows, device=dev), torch.zeros(dim, device=dev), torch.zeros(4, dtype=torch.float64, device=dev),
+              torch.zeros(1, dtype=torch.int32, device=dev)) for _ in range(2)]
+
+    def grad(i):
+        T.glm_grad_transposed(csr, bi, ws[i], *state[i], loss.loss_id, loss.lam)
+
+    want = []
+    for i in range(2):
+        grad(i)
+        torch.cuda.synchronize()
+        want.append(state[i][1].clone())
+    assert not bi.hot.args.partial
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(20):
+        for i in range(2):
+            state[i][1].zero_()
+        torch.cuda.synchronize()
+        for i in range(2):
+            with torch.cuda.stream(streams[i]):
+                grad(i)
+        torch.cuda.synchronize()
+        assert all(torch.equal(state[i][1], want[i]) for i in range(2))
