@@ -320,3 +320,53 @@ def test_a_step_of_over_a_million_columns():
         ws.append(t.model.weights.detach().cpu().clone())
         t.close()
     assert torch.count_nonzero(ws[0]) > 1_000_000 and torch.equal(ws[0], ws[1])
+
+
+@pytest.mark.parametrize("binary", [True, False])
+@pytest.mark.parametrize("compressor", ["Float", "Sketch"])
+def test_steps_with_lists_of_frequent_columns_train_like_steps_without(compressor, binary, monkeypatch):
+    """Three batches of a data set, of which two have lists of frequent columns, of different sizes, and share their
+    scratch: losses (settled by the kernel that adds the partial sums) and weights over two epochs."""
+    from sketchml_b200.data import CSRMatrix
+    from sketchml_b200.ops import transposed as T
+    from sketchml_b200.trainer import Trainer
+    B, nnz, dim = 20000, 20, 1_000_000
+    g = torch.Generator().manual_seed(7)
+    u = torch.rand((3 * B, nnz), generator=g, dtype=torch.float64)
+    u[:B] **= 12                       # batch 0 most frequent, batch 1 every column alike, batch 2 in between
+    u[2 * B:] **= 6
+    cols = (dim * u).int().clamp_(max=dim - 1).sort(1).values
+    keep = torch.ones_like(cols, dtype=torch.bool)
+    keep[:, 1:] = cols[:, 1:] != cols[:, :-1]
+    rowptr = torch.zeros(3 * B + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(keep.sum(1), 0)
+    vals = None if binary else torch.randn(int(rowptr[-1]), generator=g)
+    m = CSRMatrix(rowptr, cols[keep], vals, torch.sign(torch.rand(3 * B, generator=g) - 0.4), dim)
+    monkeypatch.setattr(T, "TILE_ROWS_MAX", 6000)
+    got = []
+    for least in (50_000, 10 ** 12):
+        monkeypatch.setattr(T, "HOT_MIN_ENTRIES", least)
+        t = Trainer(_conf(compressor=compressor, feature_num=dim, valid_ratio=0.0, batch_sample_ratio=1 / 3, quant_bin_num=256))
+        t.load_data(m)
+        hot = [bi.hot for bi in t.engine.tindex]
+        assert [h is not None for h in hot] == [least == 50_000, False, least == 50_000]
+        if least == 50_000:
+            assert hot[0].args.partial == hot[2].args.partial and hot[0].partial_floats != hot[2].partial_floats
+        # weights in the middle of a training: no two coefficients alike, so that no crowd of equal sums lies on a bucket's border
+        t.model.weights.normal_(0.0, 0.01, generator=torch.Generator(device="cuda").manual_seed(3))
+        t.engine.after_resume()
+        start = t.model.weights.detach().cpu().clone()
+        losses = []
+        for epoch in range(2):
+            for i in range(3):
+                t.train_one_iteration(epoch, i)
+            losses.append(t.engine.loss_ring.cpu().clone())
+        got.append((torch.stack(losses), t.model.weights.detach().cpu().clone()))
+        t.close()
+    (l0, w0), (l1, w1) = got
+    assert float(l0[..., 1].abs().min()) > 0
+    if compressor == "Float":     # sums of the same fp32 terms in another order
+        assert torch.allclose(l0, l1, rtol=1e-6) and torch.allclose(w0, w1, rtol=1e-4, atol=1e-8)
+    else:   # a sum within rounding of a bucket's border (some 1e-6 of them) may change its bucket, and the cells it is least in
+        assert torch.allclose(l0[0, 0], l1[0, 0], rtol=1e-9) and torch.allclose(l0, l1, rtol=1e-5)
+        assert float((w0 - w1).norm()) <= 1e-2 * float((w1 - start).norm())
