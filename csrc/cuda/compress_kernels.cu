@@ -8,7 +8,7 @@
 //   S3  dedupe splits, zero bucket, bucket midpoints, group edges; bucketize every value and
 //       count the keys of every bucket group per warp slice
 //   S4  group sizes -> payload layout; every key goes to its group's contiguous (still key-sorted)
-//       staging list; grouped MinMaxSketch insert (atomicMin on packed cells; from 1M keys on, as a stage of its
+//       staging list; grouped MinMaxSketch insert (atomicMin on packed cells; for large gradients, as a stage of its
 //       own, into tables in shared memory whose copies are merged in S6)
 //   S5  the groups' key lists are coded in 1024-key chunks like a plain array: delta widths, byte
 //       offsets, flag bytes, delta bytes staged per warp, one restart point per chunk. A block owns a
@@ -86,6 +86,7 @@ struct CP {
     unsigned char* gcodes;           // insert in shared memory: rank codes of the keys, in the order of gkeys
     long long copies_cap;            // insert in shared memory: bytes of the tables' copies (they lie where `tables` does)
     int priv;                        // insert in shared memory: the launch's parameters allow it (see priv_layout)
+    float priv_least[4], priv_parts; // and where it pays (priv_pays, priv_passes)
     unsigned int* status;
     long long budget;
     const float* given_splits;
@@ -146,15 +147,49 @@ struct WsLayout {
 
 static inline long long al256(long long x) { return (x + 255) & ~255ll; }
 
-#define PRIV_MIN_KEYS 1000000    // inserts of fewer keys stay with atomics in L2 (see priv_layout)
-#define PRIV_MIN_ROOM 4000000    // the same where only room for so many is known, not how many there are (see fill_params)
-#define PRIV_MAX_PASSES 4        // parts that a key is hashed against per row, on average, at most
+#define PRIV_MIN_ROOM 4000000    // insert in shared memory where only room for so many keys is known, not how many there are (see fill_params)
 #define PRIV_UNITS 2             // units of four keys a thread inserts per round
 #define PRIV_MAX_PARTS 2048      // parts of all groups' rows (their blocks are listed in shared memory)
 #define PRIV_BYTES (136 * 1024)  // cells that fit a block's shared memory
 
+// Keys from which on the insert in shared memory pays (priv_layout): it hashes a key once per row and part of the row
+// (`passes`: parts a row on average), where an atomic per row and key has to be saved by it, and puts the keys and their codes
+// into lists first, a fixed price and one per key. Whole calls, atomics / shared memory in us, eight groups of 250 buckets:
+//   three rows: 1M keys 79 / 79, 1.5M 91 / 86, 2M 105 / 95, 4M 187 / 144; in two parts 2.5M 122 / 126, 3M 156 / 139, 10M 371 / 323;
+//               in three 2.5M 130 / 151, 4M 205 / 193, 6M 268 / 255, 10M 383 / 384; in four 4M 215 / 224, 6M 277 / 293; tables of
+//               10 MB, three parts 3M 131 / 153, 4M 160 / 187
+//   two rows:   1M 68 / 73, 2M 91 / 93, 2.5M 103 / 101, 4M 139 / 134; in two parts 4M 136 / 146, 6M 192 / 183, 10M 292 / 274;
+//               in three 10M 296 / 314
+//   one row:    2M 76 / 86, 4M 108 / 122, 6M 151 / 144; in two parts 10M 215 / 227
+// More than eight groups (the lists are made by ballots then): three rows, 1.5M 98 / 100, 2M 112 / 113, 3M 145 / 135; in two
+// parts 4M 201 / 204, 10M 426 / 415. Tables of 32-bit cells that leave L2 make atomics dear: 72 MB 541 / 466, 120 MB 862 / 569.
+// least[k]: keys from which on k + 1 passes pay.
+static void priv_thresholds(long long rows, long long G, double col_ratio, float least[4]) {
+    const double scale = G > 8 ? 1.6 : 1.0, bytes = 4.0 * (double)rows * (col_ratio > 1e-9 ? col_ratio : 1e-9);   // of 32-bit cells, a key
+    const double one = rows >= 3 ? 1.25e6 : (rows == 2 ? 2.5e6 : 6e6), two = rows >= 3 ? 3e6 : 6e6, three = 24e6 / bytes > 4e6 ? 24e6 / bytes : 4e6;
+    const double out = 64e6 / bytes > one * scale ? 64e6 / bytes : one * scale;
+    least[0] = (float)(one * scale);
+    least[1] = (float)(rows >= 2 && two * scale < out ? two * scale : out);
+    least[2] = (float)(rows >= 3 && three * scale < out ? three * scale : out);
+    least[3] = (float)out;
+}
+// `hashed` / `rows`: passes, a little above a whole number counting as that. A launch's start takes the groups to be alike
+// (`slack` 1); once they are known the insert is given up only where it clearly does not pay, since the tables have to be
+// cleared then.
+static __host__ __device__ inline bool priv_pays(const float (&least)[4], float keys, float hashed, float rows, float slack) {
+    const float parts = hashed - 0.25f * slack * rows;
+    if (parts > 4.f * rows) return false;
+    return keys * slack >= (parts <= rows ? least[0] : (parts <= 2.f * rows ? least[1] : (parts <= 3.f * rows ? least[2] : least[3])));
+}
+// Parts of a row if the groups are alike; `parts`: parts of a group that holds one key.
+static __host__ __device__ inline float priv_passes(float keys, float parts) { return fmaxf(ceilf(keys * parts), 1.f); }
+
 // Whether launches of these sizes may insert in shared memory: enough keys, rows of integer mixers only, codes of a byte.
-static inline bool priv_sizes(long long n_max, long long q, long long rows) { return n_max >= PRIV_MIN_KEYS && rows <= 3 && q <= 256; }
+static inline bool priv_sizes(long long n_max, long long q, long long rows, long long G, double col_ratio) {
+    float least[4];
+    priv_thresholds(rows, G, col_ratio, least);
+    return rows <= 3 && q <= 256 && (float)n_max >= least[0];
+}
 
 // Bytes of the copies that blocks make of the parts they have worked on: at most one copy per block and part border.
 static inline long long copies_bytes(long long n_max, long long G, long long rows, double col_ratio, long long grid) {
@@ -199,7 +234,7 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
 extern "C" long long skml_compress_workspace_bytes(long long n_max, long long bin_num, long long group_num,
                                                    long long row_num, double col_ratio, long long grid) {
     if (grid <= 0 || grid > MAX_GRID) grid = MAX_GRID;
-    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, grid, priv_sizes(n_max, bin_num, row_num)).total;
+    return ws_layout(n_max, bin_num, group_num, row_num, col_ratio, grid, priv_sizes(n_max, bin_num, row_num, group_num, col_ratio)).total;
 }
 
 extern "C" long long skml_compress_workspace_least(long long n_max, long long bin_num, long long group_num,
@@ -1225,10 +1260,10 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
 // all parts, one part behind the other, are dealt to the blocks in equal runs. A block hashes its keys for one row, keeps
 // the least codes in shared memory and leaves a copy of the part; the copies of a part are merged when the tables are
 // written to the payload. Bound by the hashes' instructions and the latency of the rounds; atomics in L2, three a key, by
-// L2's rate (121 G/s). Insert and all, S4 and S5 of such launches (rows of 0.2 cells a key; atomics / shared memory, us):
-// 0.5M keys 26 / 32, 1M 41 / 38, 2.27M 76 / 59, 10M 302 / 247, which is why smaller ones keep the atomics.
-// Sets L.priv where it pays: the keys of large groups are hashed once per part, so a group of many parts (few distinct
-// values: one group holds nearly every key) is left to the atomics.
+// L2's rate (121 G/s). Insert and all, S4 and S5 of such launches (three rows of 0.2 cells a key; atomics / shared memory, us):
+// 2.27M keys 76 / 59, 10M 302 / 247.
+// Sets L.priv where it pays (priv_pays): the keys of large groups are hashed once per part, so a group of many parts (few
+// distinct values: one group holds nearly every key) is left to the atomics.
 __device__ void priv_layout(const CP& p, Smem& s) {
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, G = p.G;
@@ -1257,7 +1292,7 @@ __device__ void priv_layout(const CP& p, Smem& s) {
             L.work_prefix[G] = units;
             L.work_per = (units + gridDim.x - 1) / gridDim.x;
             L.copy_stride = (longest + 15u + 15u) & ~15u;
-            L.priv = nparts <= PRIV_MAX_PARTS && 4ull * units <= (unsigned long long)PRIV_MAX_PASSES * p.rows * keys + 4ull * nparts &&
+            L.priv = nparts <= PRIV_MAX_PARTS && priv_pays(p.priv_least, (float)keys, 4.f * (float)units, (float)p.rows * (float)keys, 1.3f) &&
                      (nparts + gridDim.x) * L.copy_stride <= (unsigned long long)p.copies_cap;
         }
     }
@@ -3156,7 +3191,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             }
         }
     }
-    bool priv = PRIV && n >= PRIV_MIN_KEYS;   // insert in shared memory
+    bool priv = PRIV && priv_pays(p.priv_least, (float)n, priv_passes((float)n, p.priv_parts), 1.f, 1.f);   // insert in shared memory
     if (FUSED || stage == 1) {
         stage_prepare(p, n, priv);
         stage_stamp(p.ctrl, 8);
@@ -3337,7 +3372,7 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     if (a->key_encoder != SKML_KEYS_DELTA_BINARY && a->key_encoder != SKML_KEYS_DELTA_ADAPTIVE) return (int)cudaErrorInvalidValue;
     grid = a->grid > 0 ? (int)a->grid : device_sms();
     if (grid > MAX_GRID) grid = MAX_GRID;
-    bool priv_room = priv_sizes(a->n_max, a->bin_num, a->row_num);
+    bool priv_room = priv_sizes(a->n_max, a->bin_num, a->row_num, a->group_num, a->col_ratio);
     WsLayout L = ws_layout(a->n_max, a->bin_num, a->group_num, a->row_num, a->col_ratio, grid, priv_room);
     if (L.total > a->workspace_bytes && priv_room) {   // (a workspace of the least size)
         priv_room = false;
@@ -3418,9 +3453,13 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     // (gradients that were scattered and compacted: one key to three to nine entries where columns are frequent and rare, up
     // to one each where they are alike), n_max says little: 4M keys of 6M alike 149 -> 139, but 247,000 to 722,000 of 1.1M to
     // 4.5M keys the above.
-    const long long enough = a->meta && a->n_bound <= 0 ? PRIV_MIN_ROOM : PRIV_MIN_KEYS;
+    const long long enough = a->meta && a->n_bound <= 0 ? PRIV_MIN_ROOM : 0;
     const long long n_known = !a->meta ? a->n_value : (a->n_bound > 0 && a->n_bound < a->n_max ? a->n_bound : a->n_max);
-    p.priv = priv_room && p.mixers && !p.huffman && n_known >= enough && (bins <= 255 || (bins == 256 && p.G >= 3));
+    priv_thresholds(p.rows, p.G, p.col_ratio, p.priv_least);
+    p.priv_parts = (float)(p.col_ratio / p.G / (PRIV_BYTES - 16));
+    p.priv = priv_room && p.mixers && !p.huffman && n_known >= enough &&
+             priv_pays(p.priv_least, (float)n_known, priv_passes((float)n_known, p.priv_parts), 1.f, 1.f) &&
+             (bins <= 255 || (bins == 256 && p.G >= 3));
     return 0;
 }
 

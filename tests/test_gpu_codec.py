@@ -853,8 +853,8 @@ def test_key_encode_does_not_leave_its_room():
 
 
 @pytest.mark.parametrize("n,n_max,bound,in_shared", [
-    (1_200_000, 1_200_000, 0, False), (1_200_000, 3_999_999, 0, False), (1_200_000, 4_000_000, 0, True),   # room alone says little
-    (999_999, 4_000_000, 0, False), (1_200_000, 1_200_000, 1_200_000, True), (1_200_000, 2_000_000, 1_300_000, True)])
+    (1_300_000, 1_300_000, 0, False), (1_300_000, 3_999_999, 0, False), (1_300_000, 4_000_000, 0, True),   # room alone says little
+    (1_249_999, 4_000_000, 0, False), (1_300_000, 1_400_000, 1_300_000, True), (1_300_000, 2_000_000, 1_400_000, True)])
 def test_where_the_sketch_is_inserted_when_the_number_of_keys_is_on_the_device(n, n_max, bound, in_shared):
     """Room for 1M keys does not choose the kernel that inserts in shared memory, which costs launches of fewer keys 3 us
     and more; a known number does. The payload is the same either way."""
@@ -879,7 +879,7 @@ def test_settings_changed_after_a_workspace_of_the_least_size():
     """A compressor made for Huffman-coded tables has no room for the insert in shared memory: with plain tables set
     afterwards it inserts with atomics, the payload being the same."""
     from sketchml_b200.ops import GpuCompressor
-    n, dim = 1_100_000, 4_000_000
+    n, dim = 1_400_000, 4_000_000
     keys, vals = _sparse_grad(n, dim, seed=5)
     kt, vt = torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda()
     c, plain = GpuCompressor(dim, n, 256, 8, 3, 0.2, seed=11, cell_bits=0), GpuCompressor(dim, n, 256, 8, 3, 0.2, seed=11)
@@ -887,3 +887,28 @@ def test_settings_changed_after_a_workspace_of_the_least_size():
     assert c.ws_bytes < plain.ws_bytes - n
     c.cell_bits = -1
     assert c.payload_bytes(c.compress_local(kt, vt, step=3)) == plain.payload_bytes(plain.compress_local(kt, vt, step=3))
+
+
+@pytest.mark.parametrize("encoder", ["delta_binary", "delta_adaptive"])
+@pytest.mark.parametrize("n,q,G,rows,ratio,levels,in_shared", [
+    (1_249_999, 256, 8, 3, 0.2, 0, False), (1_250_000, 256, 8, 3, 0.2, 0, True), (1_250_003, 64, 20, 3, 0.05, 0, False),   # the fewest keys, more
+    (2_000_003, 64, 20, 3, 0.05, 0, True), (2_499_999, 256, 8, 2, 0.1, 0, False), (2_500_001, 256, 8, 2, 0.1, 0, True),    # for many groups, fewer rows
+    (6_000_001, 255, 8, 1, 0.05, 0, True), (2_600_000, 255, 1, 3, 0.04, 0, True), (2_600_000, 256, 2, 3, 0.08, 0, False),  # most buckets in a group; one too many
+    (1_300_001, 256, 3, 3, 0.001, 0, True), (2_900_000, 128, 8, 3, 0.6, 0, False), (3_100_000, 128, 8, 3, 0.6, 0, True),   # tiny tables; rows in two parts
+    (4_100_001, 128, 8, 3, 0.7, 0, True), (4_100_000, 128, 8, 3, 0.95, 0, False),                                         # in three; in four
+    (1_300_000, 256, 8, 3, 0.2, 3, True), (1_300_000, 256, 32, 3, 0.2, 1, False), (2_100_000, 256, 20, 3, 0.2, 1, False)])  # few distinct values: empty groups, one of many parts
+def test_large_gradients_insert_where_it_pays(n, q, G, rows, ratio, levels, in_shared, encoder):
+    """Where the sketch is inserted (the stage of its own leaves a time stamp), and that the payload is that of the staged
+    launches, which insert with atomics, byte for byte."""
+    from sketchml_b200.ops import GpuCompressor
+    dim = 3 * n
+    g = torch.Generator(device="cuda").manual_seed(n + q)
+    kt = torch.cumsum(torch.randint(1, 4, (n,), generator=g, device="cuda"), 0).to(torch.int32) - 1
+    vt = torch.randn(n, generator=g, device="cuda") * 1e-3
+    if levels:
+        i = torch.arange(n, device="cuda")
+        vt = (i % levels + 1).float() * torch.where(i % 5 < 2, -1.0, 1.0)
+    comps = [GpuCompressor(dim, n, q, G, rows, ratio, seed=11, fused=fused, key_encoder=encoder) for fused in (True, False)]
+    own = [c.payload_bytes(c.compress_local(kt, vt, step=3)) for c in comps]
+    assert own[0] == own[1]
+    assert (int(comps[0].workspace[:256].view(torch.int64)[15]) != 0) == in_shared

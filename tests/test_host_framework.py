@@ -545,12 +545,12 @@ def test_batches_too_small_for_frequent_column_lists_cost_nothing(monkeypatch):
 
 
 def test_compress_workspace_grows_for_the_insert_in_shared_memory_only():
-    """A byte a key and the tables' copies where a launch may insert in shared memory: from 1M keys on, at most three rows,
-    codes of a byte. Elsewhere nothing but buckets, key lists, chunk tables and cells of four bytes."""
+    """A byte a key and the tables' copies where a launch may insert in shared memory: from 1.25M keys on (2.5M with two rows, 6M
+    with one), at most three rows, codes of a byte. Elsewhere nothing but buckets, key lists, chunk tables and cells of four bytes."""
     from sketchml_b200.ops import lib as L
     least, full = L.lib().skml_compress_workspace_least, L.lib().skml_compress_workspace_bytes
-    for n, q, rows, more in ((999_999, 256, 3, False), (1_000_000, 256, 3, True), (2_000_000, 256, 4, False), (2_000_000, 257, 3, False),
-                             (10_000_000, 64, 2, True)):
+    for n, q, rows, more in ((1_249_999, 256, 3, False), (1_250_000, 256, 3, True), (2_000_000, 256, 4, False), (2_000_000, 257, 3, False),
+                             (2_499_999, 64, 2, False), (10_000_000, 64, 2, True), (5_999_999, 64, 1, False), (6_000_000, 64, 1, True)):
         args = (n, q, 8, rows, 0.2, 148)
         assert (full(*args) > least(*args) + n) == more and (full(*args) == least(*args)) != more
         per_key = 2 + 4 + 4 * rows * 0.2 + 24 / 1024 + 4 * rows * 0.2 / 1024
