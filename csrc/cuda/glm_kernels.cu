@@ -204,16 +204,17 @@ glm_scatter_kernel(const long long* __restrict__ rowptr, const int* __restrict__
 // indices are assigned by frequency) are kept in shared memory, which serves some ten lanes a cycle, and nothing
 // is staged that would take L1 away. 500,000 rows of 30: 80 -> 61 us; 1M rows of 30 with values: 208 -> 102 us
 // (before: a warp per row, tiles staged by bulk copies, 103 warp instructions per 32 entries). Four blocks an SM instead of
-// three, at 32 registers with a few spills: 58 and 99 us, 62,500 rows 15 -> 13; one block of 1024 threads with six times
-// the hot columns took 80 and 129: what counts is the gathers in flight.
+// three (PER_SM), at 32 registers with a few spills: 58 and 99 us, 62,500 rows 15 -> 13; one block of 1024 threads with six
+// times the hot columns took 80 and 129: what counts is the gathers in flight. That holds where they go to DRAM; see
+// margin_launch_gl for where three blocks are the better choice.
 #define MARGIN_THREADS 512
 struct ClearSlots {   // out[slot[0 .. n)] = 0
     float* out;
     const int* slot;
     int n;
 };
-template <int MODE, int GL, bool HAS_VALS>
-__global__ void __launch_bounds__(MARGIN_THREADS, 4)
+template <int MODE, int GL, bool HAS_VALS, int PER_SM>
+__global__ void __launch_bounds__(MARGIN_THREADS, PER_SM)
 glm_margin_kernel(const long long* __restrict__ rowptr, const int* __restrict__ cols, const float* __restrict__ vals,
                   const float* __restrict__ labels, long long row_lo, long long row_cnt, int iters, const float* __restrict__ w,
                   int hot, int loss_id, float inv_batch, double* __restrict__ acc, float* __restrict__ out, ClearSlots clear) {
@@ -365,15 +366,25 @@ template <int MODE, int GL>
 static int margin_launch_gl(const long long* rowptr, const int* cols, const float* vals, const float* labels, long long row_lo,
                             long long row_cnt, double avg_nnz, const float* w, long long dim, int loss_id, float inv_batch, double* acc,
                             float* out, const ClearSlots& clear, cudaStream_t stream) {
-    const TurnShape t = turn_shape(row_cnt, GL, MARGIN_THREADS / 32, 4);
+    // Spills cost the validation's counters and the values more than a fourth block brings, unless the gathers miss L2.
+    // Three / four blocks, us: dim 10M, 1M rows of 8 values 35 / 40 (validated 40 / 47, binary and validated 38 / 42), dim 1M,
+    // 100,000 rows of 250 values 51 / 58 (56 / 65); dim 50M, 200,000 rows of 30 values 21.0 / 20.5, dim 100M, 1M rows 93 / 89.
+    const bool four = (MODE == 2 && !vals) || dim > (16ll << 20);
+    const TurnShape t = turn_shape(row_cnt, GL, MARGIN_THREADS / 32, four ? 4 : 3);
     const int iters = t.iters, warps = t.warps, grid = t.grid;
     const int hot = margin_hot((long long)(row_cnt * avg_nnz), grid, dim, w);
-    if (vals)
-        skml_launch(glm_margin_kernel<MODE, GL, true>, (unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream,
+    auto launch = [&](auto kernel) {
+        skml_launch(kernel, (unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream,
                     rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
-    else
-        skml_launch(glm_margin_kernel<MODE, GL, false>, (unsigned)grid, (unsigned)(32 * warps), hot * sizeof(float), stream,
-                    rowptr, cols, vals, labels, row_lo, row_cnt, iters, w, hot, loss_id, inv_batch, acc, out, clear);
+    };
+    if (vals) {
+        if (four) launch(glm_margin_kernel<MODE, GL, true, 4>);
+        else launch(glm_margin_kernel<MODE, GL, true, 3>);
+    } else if (four || MODE == 2) {
+        launch(glm_margin_kernel<MODE, GL, false, 4>);
+    } else {
+        launch(glm_margin_kernel<MODE, GL, false, 3>);
+    }
     return (int)cudaGetLastError();
 }
 
