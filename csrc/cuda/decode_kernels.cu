@@ -600,7 +600,12 @@ __device__ __forceinline__ void owned_fetch(const DP& p, const DecSmem& s, const
 
 // OP 0: SGD step / plain sum; OP 1: add into the float accumulators; OP 2: Adam update of every coordinate whose
 // accumulated sum is non-zero, then clear it. `e`: the thread's first entries, loaded by the caller; those of rank `next`
-// (negative: none) are on their way when the pass ends. A block barrier ends it.
+// (negative: none) are there when the pass ends. A block barrier ends it.
+// Entries are loaded while the weights before them arrive where a pass is an iteration or little more and waits for one trip
+// after the other; longer passes, whose sectors come from DRAM, load them behind the stores: eight payloads of 60,000 keys
+// 42 us (44 with the loads behind the barrier), of 62,500 rows (430,000 keys) 122 (131), of 1M keys of 50M 431 (458 with the
+// loads ahead), two of 4M with Adam 1155 (1229). Adam's sweeps find the sums of shorter slices in L2 already: eight of 600,000
+// keys, slices of 675, 702 (715).
 template <int OP>
 __device__ __forceinline__ void owned_pass(const DP& p, DecSmem& s, const unsigned long long* shift, const unsigned long long* ends, int r, int next,
                                            OwnedEntries& e, float& dsq) {
@@ -608,14 +613,17 @@ __device__ __forceinline__ void owned_pass(const DP& p, DecSmem& s, const unsign
     const unsigned int total = s.rank_item_begin[r] < i1 ? (unsigned int)ends[i1 - 1] : 0u;
     float* dst = OP == 0 ? (p.out_sum ? p.out_sum : p.w) : p.fsum;
     const long long ds = OP == 0 ? 1ll : p.fsum_stride;
+    const bool many = total > (OP == 0 ? 5 : 2) * DEC_THREADS;
     OwnedEntries ahead;
     for (unsigned int q = threadIdx.x;; q += 4 * DEC_THREADS) {
         float old[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) old[u] = e.k[u] < (unsigned long long)p.dim ? dst[e.k[u] * ds] : 0.f;
         const bool more = q + 4 * DEC_THREADS < total;
-        if (more) owned_fetch<OP != 2>(p, s, shift, ends, r, q + 4 * DEC_THREADS, ahead);
-        else if (next >= 0) owned_fetch<OP != 2>(p, s, shift, ends, next, threadIdx.x, ahead);
+        if (!many) {
+            if (more) owned_fetch<OP != 2>(p, s, shift, ends, r, q + 4 * DEC_THREADS, ahead);
+            else if (next >= 0) owned_fetch<OP != 2>(p, s, shift, ends, next, threadIdx.x, ahead);
+        }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             if (e.k[u] >= (unsigned long long)p.dim) continue;
@@ -628,6 +636,10 @@ __device__ __forceinline__ void owned_pass(const DP& p, DecSmem& s, const unsign
                 dst[e.k[u] * ds] = 0.f;
                 dsq += apply_one(p, e.k[u], old[u]);
             }
+        }
+        if (many) {
+            if (more) owned_fetch<OP != 2>(p, s, shift, ends, r, q + 4 * DEC_THREADS, ahead);
+            else if (next >= 0) owned_fetch<OP != 2>(p, s, shift, ends, next, threadIdx.x, ahead);
         }
         e = ahead;
         if (!more) break;

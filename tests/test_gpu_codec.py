@@ -912,3 +912,27 @@ def test_large_gradients_insert_where_it_pays(n, q, G, rows, ratio, levels, in_s
     own = [c.payload_bytes(c.compress_local(kt, vt, step=3)) for c in comps]
     assert own[0] == own[1]
     assert (int(comps[0].workspace[:256].view(torch.int64)[15]) != 0) == in_shared
+
+
+@pytest.mark.parametrize("P,n,blocks", [(2, 1000, 1), (2, 1024, 1), (2, 1025, 1), (2, 1280, 1), (2, 1281, 1), (3, 5000, 2), (3, 9000, 3), (2, 3000, 0)])
+def test_decode_passes_of_one_and_of_several_iterations(P, n, blocks):
+    """A block's slice of a rank's keys in one iteration of 1024 entries, at its edge, in one and a little (up to 1280), and in
+    several: the bits of the staged launches, for SGD and for lazy Adam."""
+    from sketchml_b200.ops import GpuCompressor, GpuDecoder
+    dim = 4 * n
+    comp = GpuCompressor(dim, n, 64, 4, 2, 0.3, seed=9)
+    bufs = []
+    for r in range(P):
+        m = n if r < 2 else n // 5       # the last rank's pass is a short one behind long ones
+        keys, vals = _sparse_grad(m, dim, seed=100 * n + r)
+        bufs.append(comp.compress_local(torch.from_numpy(keys).cuda(), torch.from_numpy(vals).cuda(), step=3, rank=r, world=P).clone())
+    ptrs, cap, status = [b.data_ptr() for b in bufs], min(b.numel() for b in bufs), torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = []
+    for dec in (GpuDecoder(dim, P * n, fused=False), GpuDecoder(dim, P * n, max_groups=4, grid=blocks)):
+        w = torch.ones(dim, device="cuda")
+        dec.decode_update(ptrs, [None] * P, cap, 3, status, w=w, lr=0.5)
+        wa, m, v = torch.ones(dim, device="cuda"), torch.zeros(dim, device="cuda"), torch.zeros(dim, device="cuda")
+        dec.decode_update(ptrs, [None] * P, cap, 3, status, w=wa, lr=0.1, adam_m=m, adam_v=v, adam_scale=0.3)
+        assert int(status.item()) == 0
+        out.append((w, wa, m, v))
+    assert all(torch.equal(a, b) for a, b in zip(*out)) and int((out[0][0] != 1).sum()) > n // 2
