@@ -23,6 +23,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include <cub/device/device_radix_sort.cuh>
 
 #include "skml_api.h"
@@ -38,6 +40,7 @@ constexpr int Z_MAX_BLOCKS = 148;
 constexpr int Z_TAIL = 512;             // candidates one warp handles in shared memory and registers, without a barrier
 
 constexpr int Z_SORT_KEYS = 8;          // values a thread of the sort keeps in registers
+constexpr int Z_SORT_ALONE = 6144;      // values that one block sorts (44 KB of shared memory)
 
 // What the blocks of the sort and of the split search share; the barrier words are cleared before the sort.
 struct ZShared {
@@ -100,11 +103,16 @@ __global__ void zip_pad_kernel(const float* __restrict__ vals, const long long* 
 // launch. A warp owns consecutive values and ranks 32 of them at a time among those of their digit; a block publishes its
 // slice's digit counts, and behind a grid barrier every block adds up those it needs. Bound by the seven barriers and the
 // trips to L2 between them. 330,000 values: 43 us; cub's sort, six kernels and six fills with the gaps between them, took 88.
+// ALONE: one block, whose values stay in shared memory between the passes: a pack of 3,000 values 66 us instead of 72, of 4,097
+// (two blocks otherwise) 72 instead of 85; with cub's sort 64 and 68, of 6,000 87 instead of 97 and 118.
+template <bool ALONE>
 __global__ void __launch_bounds__(ZT, 1)
 zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_ptr, long long n_max, unsigned int* buf_a, unsigned int* buf_b,
                 ZShared* __restrict__ shared, unsigned int* status) {
     skml_after_previous();
-    __shared__ unsigned int s_cnt[ZT / 32][256], s_tot[4][256], s_bef[4][256], s_base[256], s_warp[8];
+    using Count = typename std::conditional<ALONE, unsigned short, unsigned int>::type;
+    __shared__ Count s_cnt[ZT / 32][256];
+    __shared__ unsigned int s_tot[ALONE ? 1 : 4][256], s_bef[ALONE ? 1 : 4][256], s_base[256], s_warp[8], s_buf[ALONE ? Z_SORT_ALONE : 1];
     const unsigned int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = gridDim.x, b = blockIdx.x;
     long long n64 = *n_ptr;
     if (n64 > n_max) n64 = n_max;
@@ -121,7 +129,7 @@ zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
         for (int e = 0; e < Z_SORT_KEYS; ++e) {
             const unsigned int i = lo + 32 * e + lane;
             x[e] = 0;
-            if (i < hi) x[e] = pass ? __ldcg(src + i) : f2ord(vals[i]);
+            if (i < hi) x[e] = pass ? (ALONE ? s_buf[i] : __ldcg(src + i)) : f2ord(vals[i]);
         }
         for (unsigned int d = lane; d < 256; d += 32) s_cnt[warp][d] = 0;
         __syncwarp();
@@ -133,23 +141,22 @@ zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
             same[e] = __ballot_sync(0xFFFFFFFFu, in);   // lanes with this lane's digit (a ballot per bit: faster than a match of the warp)
 #pragma unroll
             for (int k = 0; k < 8; ++k) same[e] &= __ballot_sync(0xFFFFFFFFu, (d >> k) & 1u) ^ ((d >> k & 1u) - 1u);
-            if (in && (int)lane == __ffs(same[e]) - 1) s_cnt[warp][d] += (unsigned int)__popc(same[e]);
+            if (in && (int)lane == __ffs(same[e]) - 1) s_cnt[warp][d] += (Count)__popc(same[e]);
             __syncwarp();
         }
         __syncthreads();
+        unsigned int run = 0;
         if (tid < 256) {   // what the warps before it hold, and the slice's counts
-            unsigned int run = 0;
 #pragma unroll 8
             for (int w = 0; w < ZT / 32; ++w) {
                 const unsigned int c = s_cnt[w][tid];
-                s_cnt[w][tid] = run;
+                s_cnt[w][tid] = (Count)run;
                 run += c;
             }
-            shared->digits[b][tid] = run;
+            if (!ALONE) shared->digits[b][tid] = run;
         }
-        if (nb > 1 && !skml_grid_barrier(&shared->sort_bar, nb, status, 2000000000ll, 0x64u, passed)) return;
-        if (nb == 1) __syncthreads();
-        {
+        if (!ALONE) {
+            if (!skml_grid_barrier(&shared->sort_bar, nb, status, 2000000000ll, 0x64u, passed)) return;
             const unsigned int d = tid & 255, part = tid >> 8;
             unsigned int tot = 0, bef = 0;
 #pragma unroll 8
@@ -160,11 +167,11 @@ zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
             }
             s_tot[part][d] = tot;
             s_bef[part][d] = bef;
+            __syncthreads();
         }
-        __syncthreads();
         unsigned int tot = 0, inc = 0;
         if (tid < 256) {
-            tot = s_tot[0][tid] + s_tot[1][tid] + s_tot[2][tid] + s_tot[3][tid];
+            tot = ALONE ? run : s_tot[0][tid] + s_tot[ALONE ? 0 : 1][tid] + s_tot[ALONE ? 0 : 2][tid] + s_tot[ALONE ? 0 : 3][tid];
             inc = tot;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -175,7 +182,9 @@ zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
         }
         __syncthreads();
         if (tid < 256) {
-            unsigned int before = inc - tot + s_bef[0][tid] + s_bef[1][tid] + s_bef[2][tid] + s_bef[3][tid];
+            unsigned int before = inc - tot;
+            if (!ALONE)
+                for (int part = 0; part < 4; ++part) before += s_bef[ALONE ? 0 : part][tid];
             for (unsigned int w = 0; w < warp; ++w) before += s_warp[w];
             s_base[tid] = before;
         }
@@ -187,18 +196,16 @@ zip_sort_kernel(const float* __restrict__ vals, const long long* __restrict__ n_
             const unsigned int d = (x[e] >> shift) & 255u;
             if (in) {
                 const unsigned int at = s_base[d] + s_cnt[warp][d] + (unsigned int)__popc(same[e] & ((1u << lane) - 1u));
-                dst[at] = pass < 3 ? x[e] : __float_as_uint(ord2f(x[e]));
+                if (ALONE && pass < 3) s_buf[at] = x[e];   // (everyone has read its values of this pass)
+                else dst[at] = pass < 3 ? x[e] : __float_as_uint(ord2f(x[e]));
             }
             __syncwarp();
-            if (in && (int)lane == __ffs(same[e]) - 1) s_cnt[warp][d] += (unsigned int)__popc(same[e]);
+            if (in && (int)lane == __ffs(same[e]) - 1) s_cnt[warp][d] += (Count)__popc(same[e]);
             __syncwarp();
         }
         if (pass == 3) return;
-        if (nb > 1) {
-            if (!skml_grid_barrier(&shared->sort_bar, nb, status, 2000000000ll, 0x65u, passed)) return;
-        } else {
-            __syncthreads();
-        }
+        if (ALONE) __syncthreads();
+        else if (!skml_grid_barrier(&shared->sort_bar, nb, status, 2000000000ll, 0x65u, passed)) return;
     }
 }
 
@@ -720,13 +727,14 @@ extern "C" int skml_zipml_pack(const float* vals, const long long* n_ptr, long l
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaMemsetAsync(z.shared, 0, offsetof(ZShared, digits), s);   // the barriers' words
     if (e != cudaSuccess) return (int)e;
-    long long sorters = (n_max + 4095) / 4096;
+    long long sorters = n_max <= Z_SORT_ALONE ? 1 : (n_max + 4095) / 4096;
     if (sorters > Z_MAX_BLOCKS) sorters = Z_MAX_BLOCKS;
     if (sorters > zip_sm_count()) sorters = zip_sm_count();
     if (n_max <= sorters * ZT * Z_SORT_KEYS) {   // (beyond, passes over memory are what a sort costs)
         unsigned int* a = reinterpret_cast<unsigned int*>(z.sorted_in);
         unsigned int* b = reinterpret_cast<unsigned int*>(z.sorted);
-        e = skml_launch_as(true, zip_sort_kernel, (unsigned)sorters, ZT, 0, s, vals, n_ptr, n_max, a, b, z.shared, status);
+        if (sorters == 1) e = skml_launch(zip_sort_kernel<true>, 1, ZT, 0, s, vals, n_ptr, n_max, a, b, z.shared, status);
+        else e = skml_launch_as(true, zip_sort_kernel<false>, (unsigned)sorters, ZT, 0, s, vals, n_ptr, n_max, a, b, z.shared, status);
     } else {
         zip_pad_kernel<<<zip_sm_count() * 4, 256, 0, s>>>(vals, n_ptr, n_max, z.sorted_in);
         e = cub::DeviceRadixSort::SortKeys(z.cub_temp, z.cub_bytes, z.sorted_in, z.sorted, (int)n_max, 0, 32, s);

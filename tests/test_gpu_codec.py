@@ -936,3 +936,18 @@ def test_decode_passes_of_one_and_of_several_iterations(P, n, blocks):
         assert int(status.item()) == 0
         out.append((w, wa, m, v))
     assert all(torch.equal(a, b) for a, b in zip(*out)) and int((out[0][0] != 1).sum()) > n // 2
+
+
+@pytest.mark.parametrize("n", [700, 1024, 1025, 3000, 6107, 6108])
+def test_zipml_sort_of_one_block(n):
+    """Values that stay in shared memory between the passes, up to the largest size and the first beyond it (37 values of
+    room more than there are): the oracle's split points, both zeros among the values."""
+    from sketchml_b200.compress import oracle
+    rng = np.random.default_rng(n)
+    vals = (rng.integers(-30000, 30000, n) / 1024.0).astype(np.float32)
+    vals[rng.random(n) < 0.01] *= 0.0
+    ref = oracle.zipml_quantize(vals.astype(np.float64), 64)
+    _, _, _, nb, zero, _, splits, mids, codes = _zip_pack(vals, 64)
+    assert nb == ref["bin_num"] and zero == ref["zero_idx"]
+    assert np.array_equal(splits.astype(np.float64), ref["splits"])
+    assert np.array_equal(mids, ref["values"].astype(np.float32)) and np.array_equal(codes, ref["bins"])
