@@ -3239,7 +3239,8 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     }
     // S5: key code and publication. In one cooperative launch a block waits only for the counts of the
     // blocks before it (they are resident, and never wait for a later block), and the last block for all of
-    // them before it writes the header (it has the fewest chunks, none where there are fewer than blocks);
+    // them before it writes the header (it has the fewest chunks, none where there are fewer than blocks); after an
+    // insert in shared memory every block waits for all of them, behind its own keys, before it merges the copies;
     // staged launches split the stage at those points. The delta_adaptive
     // code needs the groups' complete histograms of delta widths first: one more grid barrier.
     unsigned int my_begin = 0, my_end = 0, t_begin = 0, t_end = 0, nactive = 0;

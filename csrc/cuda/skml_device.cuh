@@ -16,7 +16,7 @@
 
 // The kernels of a step follow one another on one stream. Launched by skml_launch (programmatic stream serialization) a
 // kernel is set up while the one before it ends, and waits here, before it touches memory, until that one has completed
-// and its stores are visible: 2 us between kernels became about 1 (an epoch of ten small steps 993 -> 936 us). Every kernel
+// and its stores are visible: 2 us between kernels became about 1 (an epoch of ten small steps 1058 -> 993 us). Every kernel
 // launched that way calls this first. No kernel lets the next one start early: what a block would do before it waits is
 // nothing, and the blocks would take the place of others.
 __device__ __forceinline__ void skml_after_previous() {
