@@ -147,6 +147,7 @@ struct WsLayout {
 
 static inline long long al256(long long x) { return (x + 255) & ~255ll; }
 
+#define PRIV_MIN_KEYS 1250000    // least number of keys of an insert in shared memory (see priv_thresholds)
 #define PRIV_MIN_ROOM 4000000    // insert in shared memory where only room for so many keys is known, not how many there are (see fill_params)
 #define PRIV_UNITS 2             // units of four keys a thread inserts per round
 #define PRIV_MAX_PARTS 2048      // parts of all groups' rows (their blocks are listed in shared memory)
@@ -166,7 +167,7 @@ static inline long long al256(long long x) { return (x + 255) & ~255ll; }
 // least[k]: keys from which on k + 1 passes pay.
 static void priv_thresholds(long long rows, long long G, double col_ratio, float least[4]) {
     const double scale = G > 8 ? 1.6 : 1.0, bytes = 4.0 * (double)rows * (col_ratio > 1e-9 ? col_ratio : 1e-9);   // of 32-bit cells, a key
-    const double one = rows >= 3 ? 1.25e6 : (rows == 2 ? 2.5e6 : 6e6), two = rows >= 3 ? 3e6 : 6e6, three = 24e6 / bytes > 4e6 ? 24e6 / bytes : 4e6;
+    const double one = rows >= 3 ? PRIV_MIN_KEYS : (rows == 2 ? 2.5e6 : 6e6), two = rows >= 3 ? 3e6 : 6e6, three = 24e6 / bytes > 4e6 ? 24e6 / bytes : 4e6;
     const double out = 64e6 / bytes > one * scale ? 64e6 / bytes : one * scale;
     least[0] = (float)(one * scale);
     least[1] = (float)(rows >= 2 && two * scale < out ? two * scale : out);
@@ -186,9 +187,10 @@ static __host__ __device__ inline float priv_passes(float keys, float parts) { r
 
 // Whether launches of these sizes may insert in shared memory: enough keys, rows of integer mixers only, codes of a byte.
 static inline bool priv_sizes(long long n_max, long long q, long long rows, long long G, double col_ratio) {
+    if (n_max < PRIV_MIN_KEYS || rows > 3 || q > 256) return false;
     float least[4];
     priv_thresholds(rows, G, col_ratio, least);
-    return rows <= 3 && q <= 256 && (float)n_max >= least[0];
+    return (float)n_max >= least[0];
 }
 
 // Bytes of the copies that blocks make of the parts they have worked on: at most one copy per block and part border.
@@ -3456,11 +3458,12 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     // 4.5M keys the above.
     const long long enough = a->meta && a->n_bound <= 0 ? PRIV_MIN_ROOM : 0;
     const long long n_known = !a->meta ? a->n_value : (a->n_bound > 0 && a->n_bound < a->n_max ? a->n_bound : a->n_max);
-    priv_thresholds(p.rows, p.G, p.col_ratio, p.priv_least);
-    p.priv_parts = (float)(p.col_ratio / p.G / (PRIV_BYTES - 16));
-    p.priv = priv_room && p.mixers && !p.huffman && n_known >= enough &&
-             priv_pays(p.priv_least, (float)n_known, priv_passes((float)n_known, p.priv_parts), 1.f, 1.f) &&
-             (bins <= 255 || (bins == 256 && p.G >= 3));
+    p.priv = priv_room && p.mixers && !p.huffman && n_known >= enough && n_known >= PRIV_MIN_KEYS && (bins <= 255 || (bins == 256 && p.G >= 3));
+    if (p.priv) {
+        priv_thresholds(p.rows, p.G, p.col_ratio, p.priv_least);
+        p.priv_parts = (float)(p.col_ratio / p.G / (PRIV_BYTES - 16));
+        p.priv = priv_pays(p.priv_least, (float)n_known, priv_passes((float)n_known, p.priv_parts), 1.f, 1.f);
+    }
     return 0;
 }
 
