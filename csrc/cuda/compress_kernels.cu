@@ -64,9 +64,9 @@ struct CP {
     unsigned long long* run_w;
     unsigned int* splits_raw;
     unsigned int* warp_cnt;          // [grid * 32 warps][SKML_MAX_GROUPS]: keys of every group in every warp slice
-    unsigned int* blk_cnt;           // [grid][SKML_MAX_GROUPS]: the same per block
-    unsigned long long* blk_bytes;   // [grid][SKML_MAX_GROUPS]: delta bytes of the chunks every block owns, per group
-    unsigned int* blk_flag;          // [grid]: epoch in which blk_bytes was published
+    unsigned long long* blk_cnt;     // [SKML_MAX_GROUPS + 2][MAX_GRID]: the same per block, and its least and largest value (tagged)
+    unsigned long long* blk_bytes;   // [SKML_MAX_GROUPS][MAX_GRID]: delta bytes of the chunks every block owns, per group (tagged)
+    unsigned int* blk_flag;          // [grid]: epoch in which the block has published all of its counts
     unsigned short* chunk_part;      // [8 * chunks]: delta bytes of a chunk's eighths (128 keys)
     unsigned int* chunk_off;         // [2 * chunks]: delta-byte offset of a chunk inside its owner's part of the group
                                      // (delta_adaptive: flag-bit and delta-bit offsets)
@@ -96,6 +96,7 @@ struct CP {
     long long n_value;                                   // count and kind when meta is null
     int kind_value;
     int zero_slot;                                       // clear the local slot first
+    int decode_follows;                                  // whoever waits for the arrival flag is behind this launch on its stream
     unsigned long long* done_word;                       // pinned host word for the status (checked calls)
     unsigned long long done_seq;
     unsigned long long sample_rand;                      // draw behind the sample's offset (host: seed, step, rank)
@@ -211,8 +212,8 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
     L.run_w = o; o += al256(grid * 8);
     L.splits_raw = o; o += al256(q * 4);
     L.warp_cnt = o; o += al256(grid * SKML_WARPS * SKML_MAX_GROUPS * 4);
-    L.blk_cnt = o; o += al256(grid * SKML_MAX_GROUPS * 4);
-    L.blk_bytes = o; o += al256(grid * SKML_MAX_GROUPS * 8);
+    L.blk_cnt = o; o += al256(MAX_GRID * (SKML_MAX_GROUPS + 2) * 8);
+    L.blk_bytes = o; o += al256(MAX_GRID * SKML_MAX_GROUPS * 8);
     L.blk_flag = o; o += al256(grid * 4);
     L.chunk_off = o; o += al256((n_max / SKML_RESTART_INTERVAL + SKML_MAX_GROUPS + 8) * 8);
     L.chunk_part = o; o += al256((n_max / SKML_RESTART_INTERVAL + SKML_MAX_GROUPS + 8) * 16);
@@ -350,6 +351,7 @@ struct Smem {
     unsigned int sub_total[4], sub_off[4];
     unsigned long long sums[5];                      // layout_from_counts: totals of its five prefix sums
     unsigned int scan[2][SKML_WARPS];                // block_rank scratch, alternating
+    unsigned int row[SKML_MAX_GROUPS + 2];           // S3: the block's counts, least and largest value
     alignas(16) SkmlHeader hdr;                      // copied out in 16-byte units
     int flag;
 };
@@ -371,6 +373,24 @@ __device__ __forceinline__ unsigned int lanemask_lt() {
     unsigned int m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
+}
+
+// Control words (u32): [1] launches so far; [2] blocks that are done (finish_publish); from ctrl_set on, four words of one
+// launch: arrivals of its grid barriers, and the minimum (inverted) and maximum of its values. Launches take one of two
+// sets in turn, and a launch clears the set of the next one, so none has to wait at its end until everyone is done with its own.
+__device__ __forceinline__ unsigned int* ctrl_set(unsigned int* ctrl, unsigned int epoch) { return ctrl + 4 + 4 * (epoch & 1u); }
+enum { CTRL_BAR = 0, CTRL_MIN = 1, CTRL_MAX = 2 };
+
+// A launch's first words: `epoch` names it. The set behind it is nobody's now (its last user has ended).
+template <bool FUSED>
+__device__ __forceinline__ unsigned int ctrl_open(unsigned int* ctrl) {
+    const unsigned int epoch = ld_relaxed_gpu(&ctrl[1]) + 1u;
+    if (FUSED && blockIdx.x == 0 && threadIdx.x < 4) ctrl_set(ctrl, epoch + 1u)[threadIdx.x] = 0u;
+    return epoch;
+}
+// Behind a grid barrier: every block has read the number.
+__device__ __forceinline__ void ctrl_advance(unsigned int* ctrl, unsigned int epoch) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st_relaxed_gpu(&ctrl[1], epoch);
 }
 
 // Block 0 leaves a nanosecond time stamp per stage in the control words (u64 at ctrl[16 + 2 i]);
@@ -436,7 +456,7 @@ __device__ __forceinline__ void carry_run(Smem& s, unsigned int& occupied, int l
 }
 
 // The block's share of the values -> one run of at most SK_K samples in s.qs.tile[0, cnt) with weight w.
-__device__ void summarize_slice(const CP& p, Smem& s, const float* __restrict__ vals, long long n, unsigned int& run_cnt,
+__device__ void summarize_slice(const CP& p, Smem& s, unsigned int* set, const float* __restrict__ vals, long long n, unsigned int& run_cnt,
                                 unsigned long long& run_w) {
     run_cnt = 0;
     run_w = 0;
@@ -558,8 +578,8 @@ __device__ void summarize_slice(const CP& p, Smem& s, const float* __restrict__ 
                 b = max(b, __shfl_xor_sync(0xFFFFFFFFu, b, o));
             }
             if (threadIdx.x == 0) {
-                atomicMax(&p.ctrl[4], ~a);
-                atomicMax(&p.ctrl[5], b);
+                atomicMax(&set[CTRL_MIN], ~a);
+                atomicMax(&set[CTRL_MAX], b);
             }
         }
     }
@@ -690,12 +710,12 @@ __device__ unsigned long long merge_two_runs(Smem& s, unsigned int ca, unsigned 
 // their runs in shared memory (the cluster's first block reads the others' runs through distributed
 // shared memory) and only the merged run goes to global memory, so S2 has 1 / cluster-size as many runs
 // to load and to rank against. Launched without clusters the cluster is the block itself.
-__device__ void stage_summary(const CP& p, Smem& s, const float* __restrict__ vals, long long n) {
+__device__ void stage_summary(const CP& p, Smem& s, unsigned int* set, const float* __restrict__ vals, long long n) {
     __shared__ unsigned int s_pub_cnt;
     __shared__ unsigned long long s_pub_w;
     unsigned int cnt;
     unsigned long long w;
-    summarize_slice(p, s, vals, n, cnt, w);
+    summarize_slice(p, s, set, vals, n, cnt, w);
     const unsigned int cs = cluster_nctarank(), cr = cluster_ctarank();
     if (threadIdx.x == 0) {
         s_pub_cnt = cnt;
@@ -924,8 +944,8 @@ __device__ __forceinline__ unsigned int block_rank(Smem& s, int par, bool keep, 
 // Distinct splits, zero bucket and group edges, in the shared memory of every block.
 // in_smem: the raw split points are in raw_splits(s) (sample form, same launch), otherwise in the workspace.
 // minmax_ready = false: the minimum and maximum of the values are not known yet (sample form before the
-// count stage has run); the zero bucket does not need them (see below), refresh_minmax sets them later.
-__device__ void load_quantizer(const CP& p, Smem& s, bool in_smem = false, bool minmax_ready = true) {
+// count stage has run); the zero bucket does not need them (see below), set_minmax follows later.
+__device__ void load_quantizer(const CP& p, Smem& s, const unsigned int* set, bool in_smem = false, bool minmax_ready = true) {
     const bool given = p.given_splits != nullptr;
     const int nraw = given ? p.n_given : p.q - 1;
     auto raw = [&](int i) { return given ? p.given_splits[i] : ord2f(in_smem ? raw_splits(s)[i] : __ldcg(p.splits_raw + i)); };
@@ -953,8 +973,8 @@ __device__ void load_quantizer(const CP& p, Smem& s, bool in_smem = false, bool 
             minv = p.given_min;
             maxv = p.given_max;
         } else if (minmax_ready) {
-            minv = ord2f(~__ldcg(p.ctrl + 4));
-            maxv = ord2f(__ldcg(p.ctrl + 5));
+            minv = ord2f(~__ldcg(set + CTRL_MIN));
+            maxv = ord2f(__ldcg(set + CTRL_MAX));
         }
         // The splits ascend, so the zero bucket (the first whose upper split is not negative) is their number of
         // negative ones. With splits taken from the data, min > 0 means every split is positive and max < 0 that
@@ -988,12 +1008,51 @@ __device__ void load_quantizer(const CP& p, Smem& s, bool in_smem = false, bool 
     __syncthreads();
 }
 
-// Sample form, after the count stage and its grid barrier: minimum and maximum of all values (one thread; the
-// caller has a block barrier after it).
-__device__ void refresh_minmax(const CP& p, Smem& s) {
-    s.qi.minv = ord2f(~__ldcg(p.ctrl + 4));
-    s.qi.maxv = ord2f(__ldcg(p.ctrl + 5));
-    if (!isfinite(s.qi.minv) || !isfinite(s.qi.maxv)) skml_set_status(p.status, SKML_BAD_INPUT, 0x35u);
+// Sample form, once the values have all been looked at: their minimum or maximum, as order-preserving keys (one thread;
+// the caller has a block barrier after it).
+__device__ __forceinline__ void set_extreme(const CP& p, Smem& s, bool least, unsigned int key) {
+    const float v = ord2f(key);
+    if (least) s.qi.minv = v;
+    else s.qi.maxv = v;
+    if (!isfinite(v)) skml_set_status(p.status, SKML_BAD_INPUT, 0x35u);
+}
+
+// What a block tells the others of its counts: word i of all blocks lies in words[i * MAX_GRID ...], the count below the
+// number of the launch (none in staged launches, where a launch's end is the barrier), so that whoever reads the number has
+// the count with it. By one warp, behind a block barrier; the block's earlier stores come before it.
+template <bool FUSED>
+__device__ __forceinline__ void publish_row(unsigned long long* words, const unsigned int* row, int count, unsigned int epoch) {
+    if (FUSED) __threadfence();
+    for (int i = threadIdx.x & 31; i < count; i += 32) st_relaxed_gpu64(words + i * MAX_GRID + blockIdx.x, ((unsigned long long)(FUSED ? epoch : 0u) << 32) | row[i]);
+}
+
+// One word of the blocks [0, count), lane l those of blocks l, l + 32, ...: c[k] (undefined beyond). Waits for them where `wait`;
+// false where the budget ran out (reported) or, `stop`, where an error has been reported: that block may never come.
+template <bool WAIT>
+__device__ __forceinline__ bool read_row(const CP& p, const unsigned long long* words, unsigned int count, unsigned int epoch, unsigned int where,
+                                         bool stop, unsigned int (&c)[MAX_GRID / 32]) {
+    const unsigned int lane = threadIdx.x & 31;
+    const long long t0 = WAIT ? clock64() : 0;
+    for (unsigned int ns = 0;; ns = min(ns + 20u, 200u)) {
+        if (ns) __nanosleep(ns);
+        unsigned long long v[MAX_GRID / 32];
+#pragma unroll
+        for (int k = 0; k < MAX_GRID / 32; ++k) v[k] = lane + 32 * k < count ? ld_relaxed_gpu64(words + lane + 32 * k) : (unsigned long long)epoch << 32;
+        const unsigned int st = WAIT && stop ? ld_relaxed_gpu(p.status) : 0u;   // (in the same flight)
+        bool here = true;
+#pragma unroll
+        for (int k = 0; k < MAX_GRID / 32; ++k) {
+            here = here && (unsigned int)(v[k] >> 32) == epoch;
+            c[k] = (unsigned int)v[k];
+        }
+        if (!WAIT) return true;
+        if (__any_sync(0xFFFFFFFFu, (st & 0xFFu) != SKML_OK)) return false;
+        if (__all_sync(0xFFFFFFFFu, here)) return true;
+        if (__any_sync(0xFFFFFFFFu, clock64() - t0 > p.budget)) {
+            if (lane == 0) skml_set_status(p.status, SKML_TIMEOUT_BARRIER, where);
+            return false;
+        }
+    }
 }
 
 __device__ __forceinline__ float bucket_value(const Smem& s, int b) {
@@ -1093,7 +1152,8 @@ __device__ __forceinline__ void count_turns(Smem& s, int top, int rem, const flo
 // `first_val`: the values of this lane's first two elements where the caller has them in flight already; their
 // buckets are left in `first_bin`.
 template <bool FUSED, bool PRIV>
-__device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax, const float (&first_val)[2], int (&first_bin)[2]) {
+__device__ void stage_count(const CP& p, Smem& s, unsigned int* set, unsigned int epoch, long long n, bool track_minmax, const float (&first_val)[2],
+                            int (&first_bin)[2]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int kmin = 0xFFFFFFFFu, kmax = 0u;
     const int top = build_search(s);
@@ -1112,60 +1172,60 @@ __device__ void stage_count(const CP& p, Smem& s, long long n, bool track_minmax
     // values: 11.3 -> 10.1 us, 10M: 32 -> 27.6)
     if (!PRIV || sub <= 64) count_turns<2>(s, top, rem, vals, bins, first_val, first_bin, kmin, kmax);
     else count_turns<4>(s, top, rem, vals, bins, first_val, first_bin, kmin, kmax);
-    __syncwarp();
+    kmin = __reduce_min_sync(0xFFFFFFFFu, kmin);
+    kmax = __reduce_max_sync(0xFFFFFFFFu, kmax);
+    if (lane == 0) {
+        s.scan[0][warp] = kmin;
+        s.scan[1][warp] = kmax;
+    }
     // (one launch for all stages: the slices' counts stay in shared memory)
     if (!FUSED && lane < p.G) p.warp_cnt[vb * SKML_MAX_GROUPS + lane] = s.wcnt[warp][lane];
     __syncthreads();
-    if (warp < p.G) {  // the block's totals: warp g adds up group g over the 32 slices
-        const unsigned int tot = warp_sum(s.wcnt[lane][warp]);
-        if (lane == 0) p.blk_cnt[(long long)blockIdx.x * SKML_MAX_GROUPS + warp] = tot;
+    for (int i = warp; i < p.G + 2; i += SKML_WARPS) {   // the block's totals, a warp each
+        const unsigned int v = i < p.G ? __reduce_add_sync(0xFFFFFFFFu, s.wcnt[lane][i])
+                                       : (i == p.G ? __reduce_min_sync(0xFFFFFFFFu, s.scan[0][lane]) : __reduce_max_sync(0xFFFFFFFFu, s.scan[1][lane]));
+        if (lane == 0) s.row[i] = v;
     }
-    if (track_minmax) {   // sample form: the extremes of all values (one pair of atomics per block)
-        __shared__ unsigned int c_mn[SKML_WARPS], c_mx[SKML_WARPS];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            kmin = min(kmin, __shfl_xor_sync(0xFFFFFFFFu, kmin, o));
-            kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, o));
-        }
-        if (lane == 0) {
-            c_mn[warp] = kmin;
-            c_mx[warp] = kmax;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            kmin = c_mn[lane];
-            kmax = c_mx[lane];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                kmin = min(kmin, __shfl_xor_sync(0xFFFFFFFFu, kmin, o));
-                kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, o));
-            }
-            if (lane == 0 && kmin <= kmax) {
-                atomicMax(&p.ctrl[4], ~kmin);
-                atomicMax(&p.ctrl[5], kmax);
-            }
-        }
+    __syncthreads();
+    if (warp == 0) publish_row<FUSED>(p.blk_cnt, s.row, p.G + 2, epoch);
+    if (!FUSED && track_minmax && threadIdx.x == 0 && s.row[p.G] <= s.row[p.G + 1]) {   // staged launches: for the next ones
+        atomicMax(&set[CTRL_MIN], ~s.row[p.G]);
+        atomicMax(&set[CTRL_MAX], s.row[p.G + 1]);
     }
 }
 
 // S4 prelude: group sizes, table sizes, hash rows and every section offset that does not depend on
 // the key code (every block computes the same layout); this block's and its warps' starting ranks.
+// One launch for all stages: waits for every block's row of counts. Whoever has seen them all is behind a grid barrier: a
+// row is stored behind a fence, and nothing is counted in one place first. (An arrival, a poll for the last one and only then
+// the loads of the counts took 4.3 us of every launch. This, the counts of S5 sent likewise, the narrow tables by other blocks
+// than the keys' and the flag without a count, together: 26,000 keys 37.5 -> 29.5 us, 430,000 57.5 -> 48.5, 2.27M 105.5 -> 100.7.)
+// False on every thread where the wait ran out, or on an error.
 template <bool FUSED>
-__device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
+__device__ bool layout_from_counts(const CP& p, Smem& s, unsigned int epoch, bool want_minmax) {
     const int G = p.G, nb = gridDim.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Layout& L = s.lay;
-    if (want_minmax && threadIdx.x == SKML_BLOCK - 1) refresh_minmax(p, s);
-    if (warp < G) {
-        const int g = warp;
+    bool ok = true;
+    for (int i = warp; i < (want_minmax ? G + 2 : G); i += SKML_WARPS) {
         // the blocks' totals (before this block / all blocks), lanes striding over the blocks; this
         // block's own 32 slices are scanned over the lanes for the warps' starting ranks
-        unsigned int before = 0, total = 0, c[MAX_GRID / 32];
+        unsigned int c[MAX_GRID / 32];
+        ok = read_row<FUSED>(p, p.blk_cnt + i * MAX_GRID, nb, epoch, 3u, true, c) && ok;
+        if (i >= G) {   // least and largest value
+            unsigned int v = i == G ? 0xFFFFFFFFu : 0u;
 #pragma unroll
-        for (int k = 0; k < MAX_GRID / 32; ++k) c[k] = lane + 32 * k < nb ? __ldcg(&p.blk_cnt[(long long)(lane + 32 * k) * SKML_MAX_GROUPS + g]) : 0u;
+            for (int k = 0; k < MAX_GRID / 32; ++k)
+                if (lane + 32 * k < nb) v = i == G ? min(v, c[k]) : max(v, c[k]);
+            v = i == G ? __reduce_min_sync(0xFFFFFFFFu, v) : __reduce_max_sync(0xFFFFFFFFu, v);
+            if (lane == 0) set_extreme(p, s, i == G, v);
+            continue;
+        }
+        const int g = i;
+        unsigned int before = 0, total = 0;
 #pragma unroll
-        for (int k = 0; k < MAX_GRID / 32; ++k) {   // (all loads in flight at once: one after the other they took 2 us)
-            total += c[k];
+        for (int k = 0; k < MAX_GRID / 32; ++k) {
+            if (lane + 32 * k < nb) total += c[k];
             if (lane + 32 * k < (int)blockIdx.x) before += c[k];
         }
         const unsigned int own = FUSED ? s.wcnt[lane][g] : __ldcg(&p.warp_cnt[((long long)blockIdx.x * SKML_WARPS + lane) * SKML_MAX_GROUPS + g]);
@@ -1184,7 +1244,8 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
         }
         if (lane < SKML_MAX_ROWS) L.hash_ids[g][lane] = p.hash_ids[g][lane];
     }
-    __syncthreads();
+    if (FUSED && warp == 0) __threadfence();   // the others' stores before their rows, too
+    if (!__syncthreads_and(ok)) return false;
     // One lane per group, one warp per quantity: sizes, then prefix sums over the lanes. (One thread that walked the
     // groups took 3 us of a 62 us launch at 10,000 keys.)
     const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE;
@@ -1254,6 +1315,7 @@ __device__ void layout_from_counts(const CP& p, Smem& s, bool want_minmax) {
         }
     }
     __syncthreads();
+    return true;
 }
 
 // Insert in shared memory (large gradients, plain tables). A cell of the sketch is decided by the rank of its bucket among
@@ -1735,7 +1797,8 @@ __device__ __forceinline__ int group_of_chunk(const unsigned int* prefix, int G,
 // them (`c`, `boff`, `total`; offsets in s.sub_off) and does not read its keys again. Longer runs need the totals
 // only: every warp adds up eighths of chunks on its own, the next one's keys on their way, without a barrier
 // per chunk (a scan and three barriers per round took 31 us at 66 chunks a block).
-__device__ void pack_measure(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end, ChunkWork& c, unsigned int& boff,
+template <bool FUSED>
+__device__ void pack_measure(const CP& p, Smem& s, unsigned int epoch, unsigned int my_begin, unsigned int my_end, ChunkWork& c, unsigned int& boff,
                              unsigned int& total) {
     const Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1799,7 +1862,9 @@ __device__ void pack_measure(const CP& p, Smem& s, unsigned int my_begin, unsign
         }
     }
     __syncthreads();
-    if (threadIdx.x < SKML_MAX_GROUPS) p.blk_bytes[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x] = s.my_bytes[threadIdx.x];
+    // (32 bits: a delta of more than a byte is 256 at least, and those of a group's keys add up to less than 2^31)
+    if ((int)threadIdx.x < p.G)
+        st_relaxed_gpu64(p.blk_bytes + threadIdx.x * MAX_GRID + blockIdx.x, ((unsigned long long)(FUSED ? epoch : 0u) << 32) | (unsigned int)s.my_bytes[threadIdx.x]);
 }
 
 // Bounded wait for the publications (epoch words) of blocks [0, count); false on every thread when one is missing.
@@ -1832,17 +1897,32 @@ __device__ __forceinline__ unsigned long long sum_over_blocks(const unsigned lon
     return warp_sum(v);
 }
 
+// Sum of one word of the blocks [0, count) (see read_row), by a warp.
+template <bool WAIT>
+__device__ __forceinline__ bool sum_row(const CP& p, const unsigned long long* words, unsigned int count, unsigned int epoch, unsigned int where,
+                                        unsigned long long& sum) {
+    unsigned int c[MAX_GRID / 32];
+    const bool ok = read_row<WAIT>(p, words, count, epoch, where, false, c);
+    sum = 0;
+#pragma unroll
+    for (int k = 0; k < MAX_GRID / 32; ++k) sum += (threadIdx.x & 31) + 32 * k < count ? c[k] : 0u;
+    sum = warp_sum(sum);
+    return ok;
+}
+
 // Byte totals of the blocks before this one (they own the chunks before this block's run, so the
 // sums give this block's starting offsets and the sizes of all earlier groups); a warp per group.
-__device__ void pack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch) {
-    const bool ok = !wait || wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x50u);
+template <bool WAIT>
+__device__ void pack_prefix(const CP& p, Smem& s, unsigned int epoch) {
+    bool ok = true;
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < p.G) {
-        const unsigned long long v = sum_over_blocks(p.blk_bytes + warp, SKML_MAX_GROUPS, blockIdx.x);
+        unsigned long long v;
+        ok = sum_row<WAIT>(p, p.blk_bytes + warp * MAX_GRID, blockIdx.x, epoch, 0x50u, v);
         if (lane == 0) s.pre_bytes[warp] = v;
     }
-    __syncthreads();
+    ok = __syncthreads_and(ok) != 0;
     if (warp == 0) {
         // section starts of the groups this block can reach: all earlier groups are complete in pre_bytes
         // (plus this block's own part of the group its run starts in)
@@ -2682,14 +2762,17 @@ __device__ __forceinline__ unsigned int chunk_run(const Layout& L, int G, unsign
 }
 
 // S6 prelude: every group's delta bytes from all blocks' counts -> delta section offsets, total size.
-__device__ void layout_finish(const CP& p, Smem& s, unsigned int nactive) {
+template <bool WAIT>
+__device__ bool layout_finish(const CP& p, Smem& s, unsigned int epoch, unsigned int nactive) {
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool ok = true;
     if (warp < p.G) {
-        const unsigned long long v = sum_over_blocks(p.blk_bytes + warp, SKML_MAX_GROUPS, nactive);
+        unsigned long long v;
+        ok = sum_row<WAIT>(p, p.blk_bytes + warp * MAX_GRID, nactive, epoch, 0x51u, v);
         if (lane == 0) L.bytes_g[warp] = v;
     }
-    __syncthreads();
+    if (!__syncthreads_and(ok)) return false;
     if (warp == 0) {
         unsigned long long size = 0, all;
         if (lane < p.G && L.n_g[lane]) size = skml_align16(8ull * ((L.bytes_g[lane] + 7) / 8));
@@ -2704,6 +2787,7 @@ __device__ void layout_finish(const CP& p, Smem& s, unsigned int nactive) {
         }
     }
     __syncthreads();
+    return true;
 }
 
 // Fill helpers run inside S1 (they do not depend on the summary). priv: the sketch is not expected to be inserted in
@@ -2848,8 +2932,15 @@ __device__ void copy_range_to_peers(const CP& p, unsigned long long lo, unsigned
 // The block barrier orders every thread's stores before thread 0's fence, and the fence before the count, so one
 // thread fences for the block (1024 threads fencing at system scope took 7 us); peers' memory needs system scope.
 // A checked call returns on the last block's word, before the kernel has ended: that word must carry the other blocks'
-// stores (and statuses) too. Only a launch alone, without flag and word, leaves its readers to the end of the kernel.
-__device__ void finish_publish(const CP& p) {
+// stores (and statuses) too. Only a launch alone, without flag and word, leaves its readers to the end of the kernel; so does
+// one whose only reader is behind it on its stream, and the block that writes the header sets the flag then (`header`): fence,
+// count and flag took 3.7 us at the end of every step.
+template <bool FUSED>
+__device__ void finish_publish(const CP& p, unsigned int* set, bool header) {
+    if (FUSED && p.world == 1 && !p.done_word && (p.decode_follows || !p.peer_flag[0])) {
+        if (header && threadIdx.x == 0 && p.peer_flag[0]) *(volatile unsigned long long*)p.peer_flag[0] = p.step + 1;
+        return;
+    }
     __shared__ int s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -2857,12 +2948,9 @@ __device__ void finish_publish(const CP& p) {
         else if (p.peer_flag[0] || p.done_word) __threadfence();
         unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
         s_last = prev == gridDim.x - 1;
-        if (s_last) {       // nobody is in a grid barrier any more
-            p.ctrl[0] = 0;
-            p.ctrl[1] += 1;
+        if (s_last) {
             p.ctrl[2] = 0;
-            p.ctrl[4] = 0;  // the summary's min / max words go back to "nothing yet"
-            p.ctrl[5] = 0;
+            if (!FUSED) set[CTRL_MIN] = set[CTRL_MAX] = 0;   // (a staged launch opens no set of its own)
             __threadfence();
             skml_store_done(p.done_word, p.done_seq, p.status);
         }
@@ -2877,11 +2965,13 @@ __device__ void finish_publish(const CP& p) {
 }
 
 // Sketch tables: 32-bit working cells -> 8/16-bit bucket codes, stored locally and into the peers' slots.
-__device__ void narrow_tables(const CP& p, Smem& s) {
+// `first`: the block that begins, the first one without keys to code where there is one (10,000 keys: 2.2 us less).
+__device__ void narrow_tables(const CP& p, Smem& s, unsigned int first) {
     const Layout& L = s.lay;
     if (L.overflow) return;
     const int G = p.G, cb = s.qi.cell_bits, per = 16 / (cb / 8);  // cells per 16-byte unit
-    const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned int turn = blockIdx.x >= first ? blockIdx.x - first : blockIdx.x + gridDim.x - first;
+    const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)turn * blockDim.x + threadIdx.x;
     const long long units = (long long)L.unit_prefix[G];
     const unsigned int zero = (unsigned int)s.qi.zero_idx;
     auto code_of = [&](unsigned int cell) { return cell == SKML_EMPTY_CELL ? zero : cell; };
@@ -3021,14 +3111,14 @@ __device__ void push_own_chunks(const CP& p, Smem& s, unsigned int my_begin, uns
 // ---------------------------------------------------------------------------
 #define STAGE_BARRIER(stage_id)                                                           \
     if (FUSED) {                                                                          \
-        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, stage_id, passed)) return; \
+        if (!skml_grid_barrier(set + CTRL_BAR, gridDim.x, p.status, p.budget, stage_id, passed)) return; \
         stage_stamp(p.ctrl, stage_id);                                                    \
     }
 
 // Dense kind: one narrow bucket code per coordinate, written straight into the local
 // payload and every peer's slot.
 template <bool FUSED>
-__device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ vals, int stage) {
+__device__ void dense_stages(const CP& p, Smem& s, unsigned int* set, unsigned int epoch, const float* __restrict__ vals, int stage) {
     unsigned int passed = 0;   // arrivals of the grid barriers so far
     const long long n = p.dim;
     const bool given = p.given_splits != nullptr;
@@ -3037,7 +3127,7 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
     const bool sample = p.sample_splits != 0 && !given;
     if (FUSED || stage == 1) {
         if (sample) stage_sample_splits(p, s, vals, n);
-        else if (!given) stage_summary(p, s, vals, n);
+        else if (!given) stage_summary(p, s, set, vals, n);
     }
     if (!sample) {
         STAGE_BARRIER(1)
@@ -3045,7 +3135,7 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
         STAGE_BARRIER(2)
     }
     if (FUSED || stage == 3) {
-        load_quantizer(p, s, FUSED && sample, !sample);
+        load_quantizer(p, s, set, FUSED && sample, !sample);
         if (s.qi.bin_num > SKML_GPU_MAX_BINS) {
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x33u);
             return;
@@ -3114,16 +3204,17 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
                 kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, o));
             }
             if ((threadIdx.x & 31) == 0 && kmin <= kmax) {
-                atomicMax(&p.ctrl[4], ~kmin);
-                atomicMax(&p.ctrl[5], kmax);
+                atomicMax(&set[CTRL_MIN], ~kmin);
+                atomicMax(&set[CTRL_MAX], kmax);
             }
         }
     }
     STAGE_BARRIER(3)
+    if (FUSED) ctrl_advance(p.ctrl, epoch);
     if (FUSED || stage == 4) {
         if (sample) {
-            if (!FUSED) load_quantizer(p, s);   // staged launches: the extremes are complete now
-            else if (threadIdx.x == 0) refresh_minmax(p, s);
+            if (!FUSED) load_quantizer(p, s, set);   // staged launches: the extremes are complete now
+            else if (threadIdx.x < 2) set_extreme(p, s, threadIdx.x == 0, threadIdx.x == 0 ? ~__ldcg(set + CTRL_MIN) : __ldcg(set + CTRL_MAX));
             __syncthreads();
             if (!FUSED) {
                 if (threadIdx.x == 0) s.lay.overflow = 0;
@@ -3131,7 +3222,7 @@ __device__ void dense_stages(const CP& p, Smem& s, const float* __restrict__ val
             }
             if (blockIdx.x == 0) write_header(p, s, n, SKML_KIND_DENSE);
         }
-        finish_publish(p);
+        finish_publish<FUSED>(p, set, blockIdx.x == 0);
     }
 }
 
@@ -3145,14 +3236,17 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     unsigned int passed = 0;   // arrivals of the grid barriers so far
-    // names this launch's publications: one more than the launch before it (see finish_publish)
-    const unsigned int epoch = FUSED ? ld_relaxed_gpu(&p.ctrl[1]) + 1u : 0u;
-    const long long kind = p.meta ? p.meta[1] : p.kind_value;
+    long long n = p.n_value, kind = p.kind_value;
+    if (p.meta) {
+        n = p.meta[0];
+        kind = p.meta[1];
+    }
+    const unsigned int epoch = ctrl_open<FUSED>(p.ctrl);   // names this launch's publications
+    unsigned int* const set = ctrl_set(p.ctrl, epoch);
     if (kind == SKML_KIND_DENSE) {  // un-fused launches leave it to the dense kernel's stages
-        if (FUSED && p.dense_vals) dense_stages<FUSED>(p, s, p.dense_vals, stage);
+        if (FUSED && p.dense_vals) dense_stages<FUSED>(p, s, set, epoch, p.dense_vals, stage);
         return;
     }
-    long long n = p.meta ? p.meta[0] : p.n_value;
     if (n > p.n_max) {
         if (threadIdx.x == 0) skml_set_status(p.status, SKML_CAPACITY, 0x31u);
         n = 0;
@@ -3171,7 +3265,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
                 }
                 write_header(p, s, 0, SKML_KIND_EMPTY);   // locally and into the peers' slots
             }
-            finish_publish(p);
+            finish_publish<FUSED>(p, set, blockIdx.x == 0);
         }
         return;
     }
@@ -3198,7 +3292,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         stage_prepare(p, n, priv);
         stage_stamp(p.ctrl, 8);
         if (sample) stage_sample_splits(p, s, p.vals, n);
-        else if (!given) stage_summary(p, s, p.vals, n);
+        else if (!given) stage_summary(p, s, set, p.vals, n);
         stage_stamp(p.ctrl, 9);
     }
     if (sample) {
@@ -3212,23 +3306,26 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         STAGE_BARRIER(2)
     }
     if (FUSED || stage == 3) {
-        load_quantizer(p, s, FUSED && sample, !sample);
+        load_quantizer(p, s, set, FUSED && sample, !sample);
         if (s.qi.bin_num > SKML_GPU_MAX_BINS) {
             if (threadIdx.x == 0) skml_set_status(p.status, SKML_BAD_INPUT, 0x32u);
             return;
         }
-        stage_count<FUSED, PRIV>(p, s, n, sample, first_val, first_bin);
+        stage_count<FUSED, PRIV>(p, s, set, epoch, n, sample, first_val, first_bin);
     }
-    STAGE_BARRIER(3)
     if (FUSED || stage == 4) {
-        if (!FUSED) load_quantizer(p, s);
-        layout_from_counts<FUSED>(p, s, FUSED && sample);
+        if (!FUSED) load_quantizer(p, s, set);
+        if (!layout_from_counts<FUSED>(p, s, epoch, FUSED && sample)) return;
+        if (FUSED) {
+            ctrl_advance(p.ctrl, epoch);
+            stage_stamp(p.ctrl, 3);
+        }
         if (priv) {
             priv_layout(p, s);
             priv = s.lay.priv != 0;
             if (!priv) {   // the same in every block
                 stage_prepare(p, n, false, true);
-                if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x14u, passed)) return;
+                if (!skml_grid_barrier(set + CTRL_BAR, gridDim.x, p.status, p.budget, 0x14u, passed)) return;
             }
         }
         if (priv) stage_partition(p, s, n);
@@ -3249,8 +3346,8 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     constexpr bool adaptive = ADAPTIVE, huffman = HUFFMAN;
     if (FUSED || stage >= 5) {
         if (!FUSED) {
-            load_quantizer(p, s);
-            layout_from_counts<FUSED>(p, s, false);
+            load_quantizer(p, s, set);
+            layout_from_counts<FUSED>(p, s, epoch, false);
         }
         nactive = chunk_run(s.lay, p.G, my_begin, my_end);
         if (huffman) {
@@ -3262,12 +3359,12 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         if (huffman) {
             if (!s.lay.overflow) huf_histogram(p, s, t_begin, t_end);
         } else if (adaptive && !priv) {
-            narrow_tables(p, s);   // the tables are complete since S4
+            narrow_tables(p, s, nactive);   // the tables are complete since S4
         }
         if (adaptive && !s.lay.overflow) apack_histogram(p, s, my_begin, my_end);
     }
     if (FUSED && (adaptive || huffman)) {
-        if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x15u, passed)) return;
+        if (!skml_grid_barrier(set + CTRL_BAR, gridDim.x, p.status, p.budget, 0x15u, passed)) return;
     }
     if (FUSED || stage >= 6) {
         // code tables and the layout behind the tables (every block; staged launches repeat it per stage)
@@ -3278,22 +3375,22 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     unsigned int boff = 0, btotal = 0;
     if (FUSED || stage == 6) {
         if (adaptive) apack_measure(p, s, my_begin, my_end);
-        else if (my_begin < my_end) pack_measure(p, s, my_begin, my_end, cw, boff, btotal);
+        else if (my_begin < my_end) pack_measure<FUSED>(p, s, epoch, my_begin, my_end, cw, boff, btotal);
         if (huffman) huf_measure(p, s, t_begin, t_end);
     }
-    if (FUSED) {
+    if (FUSED && (adaptive || huffman || priv)) {   // (the plain key code's counts carry the number themselves)
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
             st_relaxed_gpu(&p.blk_flag[blockIdx.x], epoch);
         }
     }
-    if (!huffman && !adaptive && !priv && (FUSED || stage == 6)) narrow_tables(p, s);   // while the publications travel
+    if (!huffman && !adaptive && !priv && (FUSED || stage == 6)) narrow_tables(p, s, nactive);   // while the publications travel
     const bool borders = adaptive || huffman;  // stream words shared by two blocks are sent by the last block at the end
     if (FUSED || stage == 7) {
         if (!FUSED) {  // the block's own counts again (shared memory does not survive a launch)
             if (threadIdx.x < SKML_MAX_GROUPS) {
-                s.my_bytes[threadIdx.x] = p.blk_bytes[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x];
+                s.my_bytes[threadIdx.x] = (unsigned int)p.blk_bytes[threadIdx.x * MAX_GRID + blockIdx.x];
                 s.my_tbits[threadIdx.x] = p.blk_tbits[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x];
             }
             if (threadIdx.x < 2 * SKML_MAX_GROUPS) s.my_bits[threadIdx.x] = p.blk_bits[(long long)blockIdx.x * 2 * SKML_MAX_GROUPS + threadIdx.x];
@@ -3303,17 +3400,19 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
             apack_prefix(p, s, FUSED, epoch);
             apack_write(p, s, my_begin, my_end);
             apush_own_chunks(p, s, my_begin, my_end);
-        } else if (my_begin < my_end) {
-            pack_prefix(p, s, FUSED, epoch);
-            pack_write(p, s, my_begin, my_end, FUSED && my_end - my_begin <= 4, cw, boff, btotal);
-            push_own_chunks(p, s, my_begin, my_end);
-        } else if (FUSED && huffman) {
-            // no keys here, but huf_prefix below reads the same publications
-            if (!wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x53u) && threadIdx.x == 0) s.lay.overflow = 1;
-            __syncthreads();
+        } else {
+            if (FUSED && huffman) {   // what huf_prefix below reads
+                if (!wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x53u) && threadIdx.x == 0) s.lay.overflow = 1;
+                __syncthreads();
+            }
+            if (my_begin < my_end) {
+                pack_prefix<FUSED>(p, s, epoch);
+                pack_write(p, s, my_begin, my_end, FUSED && my_end - my_begin <= 4, cw, boff, btotal);
+                push_own_chunks(p, s, my_begin, my_end);
+            }
         }
         if (huffman) {
-            huf_prefix(p, s);   // (the key prefix above has waited for the blocks before this one)
+            huf_prefix(p, s);   // (the blocks before this one have been waited for)
             huf_write(p, s, t_begin, t_end);
             huf_push_own(p, s, t_begin, t_end);
         }
@@ -3332,13 +3431,13 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     }
     if (FUSED || stage == 8) {
         if (blockIdx.x == gridDim.x - 1) {
-            if (FUSED && !wait_published(p, borders ? p.blk_done : p.blk_flag, borders ? gridDim.x : nactive, epoch, 0x51u)) return;
+            if (FUSED && borders && !wait_published(p, p.blk_done, gridDim.x, epoch, 0x51u)) return;
             if (adaptive) apush_borders(p, s);
-            else layout_finish(p, s, nactive);
+            else if (!layout_finish<FUSED>(p, s, epoch, nactive)) return;
             if (huffman) huf_push_borders(p, s);
             write_header(p, s, n, SKML_KIND_SPARSE);
         }
-        finish_publish(p);
+        finish_publish<FUSED>(p, set, blockIdx.x == gridDim.x - 1);
         if (FUSED) stage_stamp(p.ctrl, 6);
     }
 }
@@ -3348,7 +3447,8 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int
     skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if ((p.meta ? p.meta[1] : p.kind_value) != SKML_KIND_DENSE) return;
-    dense_stages<FUSED>(p, *reinterpret_cast<Smem*>(smem_raw), p.vals, stage);
+    const unsigned int epoch = ctrl_open<FUSED>(p.ctrl);
+    dense_stages<FUSED>(p, *reinterpret_cast<Smem*>(smem_raw), ctrl_set(p.ctrl, epoch), epoch, p.vals, stage);
 }
 
 // ---------------------------------------------------------------------------
@@ -3409,7 +3509,7 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     p.run_w = reinterpret_cast<unsigned long long*>(ws + L.run_w);
     p.splits_raw = reinterpret_cast<unsigned int*>(ws + L.splits_raw);
     p.warp_cnt = reinterpret_cast<unsigned int*>(ws + L.warp_cnt);
-    p.blk_cnt = reinterpret_cast<unsigned int*>(ws + L.blk_cnt);
+    p.blk_cnt = reinterpret_cast<unsigned long long*>(ws + L.blk_cnt);
     p.blk_bytes = reinterpret_cast<unsigned long long*>(ws + L.blk_bytes);
     p.blk_flag = reinterpret_cast<unsigned int*>(ws + L.blk_flag);
     p.chunk_part = reinterpret_cast<unsigned short*>(ws + L.chunk_part);
@@ -3439,6 +3539,7 @@ static int fill_params(const SkmlCompressArgs* a, CP& p, int& grid) {
     p.n_value = a->n_value;
     p.kind_value = (int)a->kind_value;
     p.zero_slot = a->zero_slot != 0;
+    p.decode_follows = a->decode_follows != 0;
     p.done_word = a->done_word;
     p.done_seq = a->done_seq;
     // draws that depend on the launch's parameters only are made here, once, instead of by every block

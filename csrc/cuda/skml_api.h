@@ -49,6 +49,8 @@ typedef struct SkmlCompressArgs {
     unsigned long long* done_word; // pinned host word of the checked call (skml_compress_checked sets done_seq itself)
     unsigned long long done_seq;
     long long n_bound;             // number of non-zeros, or hardly more, where the caller knows it (0: n_max at most)
+    long long decode_follows;      // 1 = whoever waits for the arrival flag is behind this launch on its stream (one rank: the
+                                   // flag is then set without waiting for all blocks' stores, which the launch's end orders)
 } SkmlCompressArgs;
 
 long long skml_compress_workspace_bytes(long long n_max, long long bin_num, long long group_num, long long row_num,

@@ -40,6 +40,7 @@ static int apply_gradient(SkmlStepArgs* a, const int* keys, const long long* met
     a->compress->keys = keys;
     a->compress->meta = meta;
     a->compress->n_bound = n_bound;
+    a->compress->decode_follows = 1;
     a->compress->vals = vals;
     if (dense_vals) a->compress->dense_vals = dense_vals;   // one launch serves both kinds
     int rc = skml_compress_sparse(a->compress, stream);

@@ -37,7 +37,7 @@ class CompressArgs(C.Structure):
         ("budget_cycles", c_ll), ("given_splits", c_vp), ("n_given", c_ll), ("given_min", c_d),
         ("given_max", c_d), ("fused", c_ll), ("grid", c_ll), ("key_encoder", c_ll), ("cell_bits", c_ll), ("quantile_summary", c_ll),
         ("dense_vals", c_vp), ("n_value", c_ll), ("kind_value", c_ll), ("zero_slot", c_ll), ("done_word", c_vp),
-        ("done_seq", c_ull), ("n_bound", c_ll),
+        ("done_seq", c_ull), ("n_bound", c_ll), ("decode_follows", c_ll),
     ]
 
 

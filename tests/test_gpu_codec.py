@@ -951,3 +951,23 @@ def test_zipml_sort_of_one_block(n):
     assert nb == ref["bin_num"] and zero == ref["zero_idx"]
     assert np.array_equal(splits.astype(np.float64), ref["splits"])
     assert np.array_equal(mids, ref["values"].astype(np.float32)) and np.array_equal(codes, ref["bins"])
+
+
+def test_launches_of_all_kinds_share_a_workspace():
+    """A launch takes one of two sets of control words and opens the other for the next one: sparse, dense, empty and staged
+    launches in any order leave what they leave in a fresh workspace."""
+    from sketchml_b200.ops import GpuCompressor
+    dim, n = 60_000, 50_000
+    new = lambda fused=True: GpuCompressor(dim, n, 64, 4, 2, 0.3, seed=9, fused=fused)
+    comp = new()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    for i, what in enumerate(["sparse", "dense", "sparse", "empty", "sparse", "sparse", "staged", "sparse", "staged", "dense", "dense", "empty", "staged", "sparse"]):
+        if what == "dense":
+            keys, vals, kind = None, torch.randn(dim, generator=g, device="cuda"), dict(dense=True)
+        else:
+            m = 0 if what == "empty" else (n if i % 2 else 777)
+            keys = torch.randperm(dim, generator=g, device="cuda")[:m].sort().values.int()
+            vals, kind = torch.randn(m, generator=g, device="cuda") * 10.0 ** -i, {}
+        comp.fused = what != "staged"
+        got = comp.compress_local(keys, vals, step=i, **kind)
+        assert torch.equal(got, new(comp.fused).compress_local(keys, vals, step=i, **kind)), (i, what)
