@@ -287,13 +287,13 @@ struct HufScratch {
 // arrays share one region: the smaller the block's shared memory, the more of the SM's 256 KB is left
 // as L1 for the scatter and coding passes, which keep many loads in flight.
 struct SmemQuantile {
-    unsigned int tile[TILE];
+    alignas(16) unsigned int tile[TILE];
     unsigned int levels[MAX_LEVELS][SK_K];
     unsigned int run[SK_K];
     unsigned int merge[2 * SK_K];
     unsigned int tail[SK_K];
     unsigned long long e_acc[SK_K];
-    unsigned int runs_all[MAX_GRID * SK_K];   // S2: all blocks' runs
+    alignas(16) unsigned int runs_all[MAX_GRID * SK_K];   // S2: all blocks' runs; S1: scratch of the sort
     unsigned int runs_cnt[MAX_GRID];
     unsigned long long runs_w[MAX_GRID];
 };
@@ -360,6 +360,7 @@ struct Smem {
 // 164 KB is a shared-memory carve-out step of the SM: staying under it (with the block's static shared
 // memory and the 1 KB the system reserves) leaves 92 KB of L1; measured, the scatter + insert stage of
 // 2.3M keys takes 69 us with that L1 and 120 us with the 28 KB that the next step (228 KB) leaves.
+static_assert(2 * TILE + SKML_GPU_MAX_BINS <= MAX_GRID * SK_K, "S1: the sort's scratch, the split points, the other half");
 static_assert(offsetof(Smem, hdr) % 16 == 0, "the header is read in 16-byte units");
 static_assert(sizeof(Smem) <= 162 * 1024, "the compress kernels' shared memory must stay below the 164 KB carve-out");
 
@@ -771,50 +772,69 @@ __device__ __forceinline__ unsigned long long warp_prefix(unsigned long long v, 
 // S1, sample form. Every thread-block cluster draws the SAME stratified sample of the values (one value
 // per stride of n / m positions, the offset a function of (seed, step, rank)), so every block ends up with
 // the same split points without a grid barrier and without S2. The two blocks of a cluster sort one half
-// of a 4096-value sample each and read the other half through distributed shared memory: split t is the
+// of a 4096-value sample each and leave it in the other's shared memory, too: split t is the
 // value of rank floor(m (t + 1) / q) in the union of the two sorted halves, found by a merge-path search
-// over the own half and a local copy of the other. Without clusters a block sorts 2048 values alone.
+// over both. Without clusters a block sorts 2048 values alone.
 // The rank error of a split is that of an m-value sample (standard deviation at most 0.8 % of n at
 // m = 4096), the same order as the k = 128 summary's; inputs of up to m values are summarised exactly.
 // Minimum and maximum of ALL values are taken by the count stage, which reads every value anyway.
 // The splits stay in the block's shared memory (raw_splits); block 0 also leaves them in the workspace.
 __device__ __forceinline__ unsigned int* raw_splits(Smem& s) { return s.qs.runs_all + TILE; }
 
-__device__ void stage_sample_splits(const CP& p, Smem& s, const float* __restrict__ vals, long long n) {
-    const unsigned int cs = cluster_nctarank(), cr = cluster_ctarank();
-    const int lh = cs >= 2 ? 1 : 0, halves = 1 << lh;
-    const long long M = (long long)TILE * halves;
-    const long long m = n < M ? n : M;   // sample size
-    __shared__ unsigned long long s_off;
-    if (threadIdx.x == 0) s_off = n > m ? p.sample_rand % (unsigned long long)n : 0ull;
-    __syncthreads();
-    const unsigned long long off = s_off;
-    const int half = (int)cr & (halves - 1);
-    const int mine = (int)((m - half + halves - 1) >> lh);   // samples in this block's half
-    for (int t = threadIdx.x; t < TILE; t += blockDim.x) {
+// x mod n, n < 2^31: the upper half reduced first, then a quotient in double, one off at most.
+__device__ __forceinline__ unsigned int mod_u64(unsigned long long x, unsigned int n) {
+    const unsigned long long y = ((unsigned long long)((unsigned int)(x >> 32) % n) << 32) | (unsigned int)x;   // below n 2^32
+    const unsigned long long q = (unsigned long long)((double)y * __drcp_rn((double)n));
+    long long r = (long long)(y - q * n);
+    if (r < 0) r += n;
+    if (r >= (long long)n) r -= n;
+    return (unsigned int)r;
+}
+
+// Where sample t of this block's half lies (below n), and how large sample and half are.
+struct SamplePlace {
+    int lh, half, m;            // log2 of the halves, which one, sample size
+    unsigned long long off;
+    __device__ __forceinline__ long long at(int t, long long n) const {   // -1: none
         const long long j = ((long long)t << lh) + half;
-        unsigned int key = 0xFFFFFFFFu;
-        if (j < m) {
-            // m is a power of two (TILE * halves) whenever it is not n itself
-            const long long pos = n > m ? (long long)(((unsigned long long)j * (unsigned long long)n + off) >> (11 + lh)) : j;
-            key = f2ord(__ldg(vals + pos));
-        }
-        s.qs.tile[t] = key;
+        if (j >= m) return -1;
+        // m is a power of two (TILE * halves) whenever it is not n itself
+        return n > m ? (long long)(((unsigned long long)j * (unsigned long long)n + off) >> (11 + lh)) : j;
+    }
+};
+__device__ __forceinline__ SamplePlace sample_place(const CP& p, long long n) {
+    SamplePlace f;
+    f.lh = cluster_nctarank() >= 2 ? 1 : 0;
+    f.half = (int)cluster_ctarank() & ((1 << f.lh) - 1);
+    const int M = TILE << f.lh;
+    f.m = n < M ? (int)n : M;
+    f.off = n > f.m ? mod_u64(p.sample_rand, (unsigned int)n) : 0u;
+    return f;
+}
+
+__device__ void stage_sample_splits(const CP& p, Smem& s, const float* __restrict__ vals, long long n) {
+    const SamplePlace f = sample_place(p, n);
+    const int m = f.m, mine = (m - f.half + (1 << f.lh) - 1) >> f.lh, theirs = m - mine;   // samples in this block's half, and the other
+    if (f.lh) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its shared memory may be written
+#pragma unroll
+    for (int t = threadIdx.x; t < TILE; t += SKML_BLOCK) {
+        const long long pos = f.at(t, n);
+        s.qs.tile[t] = pos >= 0 ? f2ord(__ldg(vals + pos)) : 0xFFFFFFFFu;
     }
     __syncthreads();
-    block_sort_2048(s.qs.tile, s.qs.runs_all);
-    const int theirs = (int)(m - mine);
-    unsigned int* const their = s.qs.runs_all;   // local copy of the other block's sorted half
-    if (halves == 2) {
-        cluster_sync_all();   // both halves are sorted and visible in the cluster
-        const unsigned int other = dsmem_addr(s.qs.tile, (unsigned int)half ^ 1u);
-        for (int t = threadIdx.x; t < theirs; t += blockDim.x) their[t] = ld_dsmem_u32(other + 4u * (unsigned int)t);
-        cluster_sync_all();   // nobody reads the other block's shared memory any more; the copy is complete
+    // the other block's sorted half arrives behind the split points, which nothing else uses
+    unsigned int* const their = raw_splits(s) + SKML_GPU_MAX_BINS;
+    unsigned int remote = 0;
+    if (f.lh) {
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        remote = dsmem_addr(their, (unsigned int)f.half ^ 1u);
     }
+    block_sort_2048(s.qs.tile, s.qs.runs_all, remote);
+    if (f.lh) cluster_sync_all();   // both halves are in both blocks
     const double inv_q = 1.0 / (double)p.q;
     for (int t = threadIdx.x; t < p.q - 1; t += blockDim.x) {
         int k = (int)((double)m * ((double)(t + 1) * inv_q));   // target rank in the sample (m <= 4096)
-        if (k > (int)m - 1) k = (int)m - 1;
+        if (k > m - 1) k = m - 1;
         // i = how many of the k values before the answer come from this block's half (ties: this half first)
         int lo = k - theirs > 0 ? k - theirs : 0, hi = k < mine ? k : mine;
         while (lo < hi) {

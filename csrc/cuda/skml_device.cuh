@@ -237,8 +237,9 @@ __device__ __forceinline__ double block_sum_double(double v) {
 // One merge round of sorted runs of LEN keys: an element's place in the merged pair of runs is its place in
 // its own run plus the number of the other run's keys before it (a binary search; the left run wins ties).
 // A warp's 64 elements belong to one run, so its 32 searches run side by side on neighbouring keys.
+// `remote`: where another block of the cluster takes a copy (shared::cluster address; 0: none).
 template <int LEN>
-__device__ __forceinline__ void merge_round(const unsigned int* __restrict__ src, unsigned int* __restrict__ dst) {
+__device__ __forceinline__ void merge_round(const unsigned int* __restrict__ src, unsigned int* __restrict__ dst, unsigned int remote = 0) {
     const int lane = threadIdx.x & 31, i0 = (threadIdx.x >> 5) * 64 + lane;
     const int run = i0 / LEN;
     const unsigned int* other = src + (run ^ 1) * LEN;
@@ -264,41 +265,67 @@ __device__ __forceinline__ void merge_round(const unsigned int* __restrict__ src
     const int base = (run & ~1) * LEN + (i0 & (LEN - 1));
     dst[base + p0] = x0;
     dst[base + 32 + p1] = x1;
+    if (remote) {
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote + 4u * (unsigned int)(base + p0)), "r"(x0) : "memory");
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote + 4u * (unsigned int)(base + 32 + p1)), "r"(x1) : "memory");
+    }
     __syncthreads();
 }
 
-// Ascending sort of 2048 unsigned keys in shared memory by a block of 1024 threads, `tmp` a second array of
-// that size. Every warp sorts 64 keys in registers (bitonic, shuffles only), five merge rounds by binary
-// search follow with one block barrier each. (A full bitonic network, whose steps of distance 64 and more
-// went through shared memory with 20 barriers and 46 shuffle steps, took 6.9 us of every compress launch.)
-__device__ __forceinline__ void block_sort_2048(unsigned int* s, unsigned int* tmp) {
-    const int lane = threadIdx.x & 31, i0 = (threadIdx.x >> 5) * 64 + lane, i1 = i0 + 32;
-    unsigned int a = s[i0], b = s[i1];
+// Ascending order of 256 keys by one warp, eight adjacent ones a lane: a bitonic network whose steps of distance 8 and more
+// are shuffles. Keys of descending stretches are inverted, so that every comparison is a minimum and a maximum.
+__device__ __forceinline__ void warp_sort_256(unsigned int (&a)[8]) {
+    const unsigned int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int k = 2; k <= 64; k <<= 1) {
-        if (k == 64 && a > b) {  // distance 32: both elements live in this thread, ascending
-            const unsigned int t = a;
-            a = b;
-            b = t;
+    for (int k = 2; k <= 256; k <<= 1) {
+        if (k >= 8) {   // stretches of k keys: whole lanes from here on
+            const unsigned int now = k < 256 && (lane & (k / 8)) ? 0xFFFFFFFFu : 0u, before = k > 8 && (lane & (k / 16)) ? 0xFFFFFFFFu : 0u;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) a[e] ^= now ^ before;
         }
 #pragma unroll
-        for (int j = (k >> 1) < 16 ? (k >> 1) : 16; j > 0; j >>= 1) {
-            const unsigned int pa = __shfl_xor_sync(0xFFFFFFFFu, a, j);
-            const unsigned int pb = __shfl_xor_sync(0xFFFFFFFFu, b, j);
-            const bool low = (lane & j) == 0;
-            const bool up0 = (lane & k) == 0 || k == 64, up1 = ((lane + 32) & k) == 0 || k == 64;
-            a = (low == up0) ? min(a, pa) : max(a, pa);
-            b = (low == up1) ? min(b, pb) : max(b, pb);
+        for (int j = k / 2; j >= 8; j >>= 1) {
+            const bool upper = (lane & (j / 8)) != 0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const unsigned int o = __shfl_xor_sync(0xFFFFFFFFu, a[e], j / 8);
+                a[e] = upper ? max(a[e], o) : min(a[e], o);
+            }
+        }
+#pragma unroll
+        for (int j = k / 2 < 4 ? k / 2 : 4; j > 0; j >>= 1) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                if (e & j) continue;
+                const bool down = k < 8 && (e & k);   // (inside a lane)
+                const unsigned int x = a[e], y = a[e + j];
+                a[e] = down ? max(x, y) : min(x, y);
+                a[e + j] = down ? min(x, y) : max(x, y);
+            }
         }
     }
-    tmp[i0] = a;
-    tmp[i1] = b;
+}
+
+// Ascending sort of 2048 unsigned keys in shared memory (16-byte aligned) by a block of 1024 threads, `tmp` a second array of
+// that size. Eight warps sort 256 keys each in registers, three merge rounds by binary search follow with one block barrier each.
+// What bounds it is the chain of dependent steps, and shared memory's passes in the merge rounds. In every block of a compress
+// launch, with its result sent to the other block instead of fetched: 10,000 keys 35.0 -> 33.8 us, 170,000 with coded tables
+// 67.5 -> 65.7, against 32 warps of 64 keys and five merge rounds.
+// `remote`: a copy of the result in another block of the cluster (see merge_round), complete behind a cluster barrier.
+__device__ __forceinline__ void block_sort_2048(unsigned int* s, unsigned int* tmp, unsigned int remote = 0) {
+    if (threadIdx.x < 256) {
+        uint4* const at = reinterpret_cast<uint4*>(s) + 2 * threadIdx.x;
+        const uint4 x = at[0], y = at[1];
+        unsigned int a[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        warp_sort_256(a);
+        uint4* const to = reinterpret_cast<uint4*>(tmp) + 2 * threadIdx.x;
+        to[0] = make_uint4(a[0], a[1], a[2], a[3]);
+        to[1] = make_uint4(a[4], a[5], a[6], a[7]);
+    }
     __syncthreads();
-    merge_round<64>(tmp, s);
-    merge_round<128>(s, tmp);
     merge_round<256>(tmp, s);
     merge_round<512>(s, tmp);
-    merge_round<1024>(tmp, s);
+    merge_round<1024>(tmp, s, remote);
 }
 
 // Upper bounds of K values side by side in an ascending array of n floats: element i lies at a[i + i / 32], and
