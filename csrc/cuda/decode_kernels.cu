@@ -38,12 +38,10 @@ struct DecSmem {
     int nitems;
     unsigned long long total_chunks, total_keys;
     int any_dense;
-    int direct;      // linear update (SGD / plain sum): payloads applied in rank order, no accumulators
     unsigned long long rank_key_begin[SKML_MAX_PEERS + 1];
     int rank_item_begin[SKML_MAX_PEERS + 1];
     int ref_item;    // the (rank, group) list with the most keys: its quantiles are the blocks' key-range bounds
-    int two_phase;   // several payloads: decode everything first, then ordered apply
-    int adam_plain;  // Adam without fixed-point accumulators (no dense payload, and one payload or a value scratch)
+    int small_passes;   // a pass per payload would leave most blocks with one chunk or none
     int shift;       // fixed-point: accumulator = value * 2^shift
     double inv_world;
     int ok;
@@ -51,6 +49,24 @@ struct DecSmem {
     int nhuf;        // items whose table arrives Huffman-coded
     DecItem items[1];  // max_items entries (dynamic shared memory)
 };
+
+// How the payloads are applied.
+struct DecForm {
+    bool direct;       // linear update (SGD / plain sum): payloads applied in rank order, no accumulators
+    bool adam_plain;   // Adam without fixed-point accumulators (no dense payload, and one payload or a value scratch)
+    bool two_phase;    // several payloads: decode everything first, then ordered apply
+};
+// Several payloads are decoded into the scratch first and applied by key range when a per-rank
+// pass would leave most blocks with one chunk or none (the pass latency then dominates). Long
+// payloads keep the blocks busy in per-rank passes and skip the scratch round trip; Adam has no
+// per-rank mode, so it always takes the scratch.
+__device__ __forceinline__ DecForm decode_form(const DP& p, const DecSmem& s) {
+    DecForm f;
+    f.direct = p.adam_v == nullptr;
+    f.adam_plain = !f.direct && !s.any_dense && (p.world == 1 || p.val_scratch != nullptr);
+    f.two_phase = (f.direct || f.adam_plain) && p.world > 1 && p.val_scratch != nullptr && (s.small_passes || f.adam_plain);
+    return f;
+}
 
 // D0: wait, validate, build the work table (identically in every block).
 __device__ bool decode_prepare(const DP& p, DecSmem& s) {
@@ -70,6 +86,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
         reinterpret_cast<uint4*>(&full[r])[i] = ld_cg_v4(reinterpret_cast<const uint4*>(p.payload[r]) + i);
     }
     __syncthreads();
+    bool bad = false;
     if (threadIdx.x < p.world) {
         const SkmlHeader& h = full[threadIdx.x];
         bool good = h.magic == SKML_MAGIC && h.version == SKML_VERSION && h.header_checksum == skml_header_checksum(&h) &&
@@ -84,7 +101,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
                                                     (h.cell_bits == 8 || h.cell_bits == 16 || (h.cell_bits == 0 && p.tab_scratch))));
         if (!good) {
             skml_set_status(p.status, SKML_BAD_HEADER, (unsigned int)threadIdx.x);
-            s.ok = 0;
+            bad = true;
         }
         HdrLite& l = s.hdr[threadIdx.x];
         l.kind = h.kind;
@@ -95,10 +112,10 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
         l.off_bucket_values = h.off_bucket_values;
         for (int i = 0; i < 4; ++i) l.loss_partials[i] = h.loss_partials[i];
     }
-    // group entries: one thread per (rank, group) fetches its 64-byte entry (independent loads), while the header is
-    // still being checked: only the offsets the fetch itself needs are looked at first
+    // group entries: one thread per (rank, group) fetches its 64-byte entry (independent loads), while the first warp is
+    // still checking the headers: only the offsets the fetch itself needs are looked at first
     const int gcap = p.max_items / p.world;
-    for (int t = threadIdx.x; t < p.world * gcap; t += blockDim.x) {
+    for (int t = (threadIdx.x + DEC_THREADS - 32) % DEC_THREADS; t < p.world * gcap; t += DEC_THREADS) {
         const int r = t / gcap, g = t % gcap;
         const SkmlHeader& h = full[r];
         DecItem& it = s.items[t];
@@ -150,43 +167,45 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
             }
         }
     }
-    __syncthreads();
-    if (!s.ok) return false;
+    if (__syncthreads_or(bad)) return false;
+    if (threadIdx.x == 32) {   // the per-rank header facts
+        int dense = 0, e = 0;
+        double mx = 0.0;
+        for (int r = 0; r < p.world; ++r) {
+            const SkmlHeader& h = full[r];
+            if (h.kind == SKML_KIND_EMPTY) continue;
+            mx = fmax(mx, fmax(fabs(h.min_value), fabs(h.max_value)));
+            if (h.kind == SKML_KIND_DENSE) dense = 1;
+            else if ((int)h.group_num > gcap) {
+                skml_set_status(p.status, SKML_BAD_HEADER, 0x300u | (unsigned int)r);
+                s.ok = 0;
+            }
+        }
+        if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
+        s.shift = 60 - e;
+        s.any_dense = dense;
+        s.inv_world = 1.0 / (double)p.world;
+    }
     // The work table: the non-empty (rank, group) lists moved to the front in (rank, group) order, each
     // with the number of chunks and keys in front of it. Warp 0 does it 32 slots at a time (ballot for the
-    // positions, shuffle scans for the prefixes); thread 0 first looks at the per-rank header facts.
+    // positions, shuffle scans for the prefixes).
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         int ni = 0, nhuf = 0;
         unsigned long long chunks = 0, keys = 0, tab_used = 0;
-        int dense = 0, ref = 0;
+        int ref = 0;
         unsigned int ref_n = 0, key_pad = 0;
-        double mx = 0.0;
-        if (lane == 0) {
-            for (int r = 0; r < p.world; ++r) {
-                const SkmlHeader& h = full[r];
-                if (h.kind == SKML_KIND_EMPTY) continue;
-                mx = fmax(mx, fmax(fabs(h.min_value), fabs(h.max_value)));
-                if (h.kind == SKML_KIND_DENSE) dense = 1;
-                else if ((int)h.group_num > gcap) {
-                    skml_set_status(p.status, SKML_BAD_HEADER, 0x300u | (unsigned int)r);
-                    s.ok = 0;
-                }
-            }
-        }
         const int nslots = p.world * gcap;
         for (int base = 0; base < nslots; base += 32) {
             const int t = base + lane;
             const bool in = t < nslots;
             const int r = in ? t / gcap : 0, g = in ? t % gcap : 0;
             const bool v = in && s.items[t].e.n != 0;
-            DecItem it;
-            if (v) it = s.items[t];
-            const unsigned int n = v ? it.e.n : 0u;
-            const bool failed = v && it.chunk_prefix != 0ull;
-            const bool huf = v && it.huffman != 0u;
+            const unsigned int n = v ? s.items[t].e.n : 0u;
+            const bool failed = v && s.items[t].chunk_prefix != 0ull;
+            const bool huf = v && s.items[t].huffman != 0u;
             unsigned long long c_inc = (n + SKML_RESTART_INTERVAL - 1) / SKML_RESTART_INTERVAL, k_inc = (n + 3ull) & ~3ull;   // (stashed four at a time)
-            unsigned long long b_inc = huf ? skml_align16((unsigned long long)it.rows * it.e.col_num * (it.cell_bits / 8)) : 0ull;
+            unsigned long long b_inc = huf ? skml_align16((unsigned long long)s.items[t].rows * s.items[t].e.col_num * (s.items[t].cell_bits / 8)) : 0ull;
             const unsigned long long c_own = c_inc, k_own = k_inc, b_own = b_inc;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -204,12 +223,17 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
                 s.rank_key_begin[r] = keys + k_inc - k_own;
                 s.rank_item_begin[r] = pos;
             }
-            __syncwarp();   // every lane holds its entry in registers: entries may now move forward
+            if (__any_sync(0xFFFFFFFFu, v && pos != t)) {   // some slot before is empty: entries move forward
+                DecItem it;
+                if (v) it = s.items[t];
+                __syncwarp();   // every lane holds its entry in registers
+                if (v) s.items[pos] = it;
+            }
             if (v) {
+                DecItem& it = s.items[pos];
                 it.chunk_prefix = chunks + c_inc - c_own;
                 it.key_prefix = keys + k_inc - k_own;
                 if (huf) it.tab = p.tab_scratch + tab_used + b_inc - b_own;
-                s.items[pos] = it;
             }
             const unsigned int fm = __ballot_sync(0xFFFFFFFFu, failed);
             if (fm) {
@@ -261,20 +285,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
         s.nhuf = nhuf;
         s.total_chunks = chunks;
         s.total_keys = keys;
-        s.any_dense = dense;
-        s.direct = (p.adam_v == nullptr) ? 1 : 0;
-        s.adam_plain = (!s.direct && !dense && (p.world == 1 || p.val_scratch != nullptr)) ? 1 : 0;
-        // Several payloads are decoded into the scratch first and applied by key range when a per-rank
-        // pass would leave most blocks with one chunk or none (the pass latency then dominates). Long
-        // payloads keep the blocks busy in per-rank passes and skip the scratch round trip; Adam has no
-        // per-rank mode, so it always takes the scratch.
-        const bool small_passes = chunks < 4ull * gridDim.x * (unsigned long long)p.world;
-        s.two_phase = ((s.direct || s.adam_plain) && p.world > 1 && p.val_scratch != nullptr &&
-                       (small_passes || s.adam_plain)) ? 1 : 0;
-        int e = 0;
-        if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
-        s.shift = 60 - e;
-        s.inv_world = 1.0 / (double)p.world;
+        s.small_passes = chunks < 4ull * gridDim.x * (unsigned long long)p.world ? 1 : 0;
       }
     }
     __syncthreads();
@@ -468,7 +479,8 @@ __device__ void decode_accumulate(const DP& p, DecSmem& s, int i_begin, int i_en
     unsigned char* tab_area = p.tab_off ? reinterpret_cast<unsigned char*>(&s) + p.tab_off : nullptr;
     int staged = -1;
     const unsigned char* stab = nullptr;
-    const bool sums = p.out_sum != nullptr, two_phase = s.two_phase != 0, direct = s.direct != 0, adam = !direct && s.adam_plain != 0;
+    const DecForm form = decode_form(p, s);
+    const bool sums = p.out_sum != nullptr, two_phase = form.two_phase, direct = form.direct, adam = form.adam_plain;
     const float iw = (float)s.inv_world;
     float* const dst = sums ? p.out_sum : p.w;
     ChunkHead head;
@@ -767,7 +779,7 @@ __device__ void decode_accumulate_dense(const DP& p, DecSmem& s, int r_begin, in
             float v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) v[u] = bv[c[u] < bin_num ? c[u] : zero];
-            if (!s.direct) {
+            if (p.adam_v) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     if (i0 + u >= p.dim) continue;
@@ -833,28 +845,40 @@ __device__ void decode_update(const DP& p, DecSmem& s, float& dsq) {
     }
 }
 
-// Adds the launch's change of the squared weight norm to the running sum; the last block to arrive
+// The launch's end. Adds its change of the squared weight norm to the running sum; the last block to arrive
 // turns the sum into the regularisation loss of the next batch (lambda * ||w||_2, un-squared as in
-// ml/objective/Loss.scala:48-53) so that no step passes over the whole model for it.
-__device__ void finish_norm(const DP& p, float dsq) {
-    if (!p.wsq) return;
+// ml/objective/Loss.scala:48-53) so that no step passes over the whole model for it, and puts the control words back.
+// One count for both: a second one behind the first was another trip to L2 for every block. With that, the work table where it
+// is and a block per SM for few keys: 10,000 keys 16.5 -> 15.0 us, 26,000 with Adam 18.9 -> 17.2, 430,000 20.7 -> 19.5.
+template <bool FUSED>
+__device__ void finish_launch(const DP& p, float dsq) {
+    if (!FUSED && !p.wsq) return;
     __shared__ double s_red[DEC_THREADS / 32];
-    double d = (double)dsq;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xFFFFFFFFu, d, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = d;
+    if (p.wsq) {
+        const double d = warp_sum((double)dsq);
+        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = d;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < DEC_THREADS / 32; ++w) t += s_red[w];
-        if (t != 0.0) atomicAdd(p.wsq, t);
-        __threadfence();
-        const unsigned int prev = atomicAdd(&p.ctrl[3], 1u);
+        if (p.wsq) {
+            double t = 0.0;
+            for (int w = 0; w < DEC_THREADS / 32; ++w) t += s_red[w];
+            if (t != 0.0) atomicAdd(p.wsq, t);
+        }
+        if (p.wsq || p.done_word) __threadfence();   // (a checked call returns before the kernel ends, see skml_store_done)
+        const unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
         if (prev == gridDim.x - 1) {
-            p.ctrl[3] = 0;
-            __threadfence();
-            const double w2 = *reinterpret_cast<volatile double*>(p.wsq);
-            if (p.reg_out) p.reg_out[0] = p.reg_lambda * sqrt(w2 > 0.0 ? w2 : 0.0);
+            p.ctrl[2] = 0;
+            p.ctrl[0] = 0;   // nobody is in a grid barrier any more
+            unsigned long long now;   // the kernel's true end (block 0's stamp is its own)
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (FUSED) reinterpret_cast<unsigned long long*>(p.ctrl)[16 + (int)(p.step & 1)] = now;
+            if (p.wsq || p.done_word) __threadfence();
+            if (p.wsq && p.reg_out) {
+                const double w2 = *reinterpret_cast<volatile double*>(p.wsq);
+                p.reg_out[0] = p.reg_lambda * sqrt(w2 > 0.0 ? w2 : 0.0);
+            }
+            skml_store_done(p.done_word, p.done_seq, p.status);
         }
     }
 }
@@ -886,18 +910,19 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
     }
     // Payloads applied one after the other take a pass per rank (un-fused: pass `stage - 1`), the rest one over all
     // lists. One call for every form: the passes are most of the kernel's code.
-    const bool ordered = s.direct || s.adam_plain, per_rank = ordered && !s.two_phase;
+    const DecForm form = decode_form(p, s);
+    const bool ordered = form.direct || form.adam_plain, per_rank = ordered && !form.two_phase;
     for (int r = 0; r < (per_rank ? p.world : 1); ++r) {
         if (FUSED || stage == r + 1) {
             decode_accumulate(p, s, per_rank ? s.rank_item_begin[r] : 0, per_rank ? s.rank_item_begin[r + 1] : s.nitems, dsq);
-            if (s.any_dense && !s.two_phase) decode_accumulate_dense(p, s, per_rank ? r : 0, per_rank ? r + 1 : p.world, dsq);
+            if (s.any_dense && !form.two_phase) decode_accumulate_dense(p, s, per_rank ? r : 0, per_rank ? r + 1 : p.world, dsq);
         }
         if (FUSED && per_rank && r + 1 < p.world) {
             if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x30u + r, passed)) return;
         }
     }
     if (ordered) {
-        if (s.two_phase) {
+        if (form.two_phase) {
             if (FUSED) {
                 if (!skml_grid_barrier(p.ctrl, gridDim.x, p.status, p.budget, 0x2Fu, passed)) return;
                 if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -930,27 +955,10 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
         if (FUSED && blockIdx.x == 0 && threadIdx.x == 0) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (!s.two_phase) reinterpret_cast<unsigned long long*>(p.ctrl)[10 + 4 * (int)(p.step & 1)] = t;
+            if (!form.two_phase) reinterpret_cast<unsigned long long*>(p.ctrl)[10 + 4 * (int)(p.step & 1)] = t;
             reinterpret_cast<unsigned long long*>(p.ctrl)[11 + 4 * (int)(p.step & 1)] = t;
         }
-        finish_norm(p, dsq);
-        if (FUSED) {
-            // the last block to finish leaves the kernel's true end time (block 0's stamp above is its own)
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                if (p.done_word) __threadfence();   // a checked call returns before the kernel ends (see skml_store_done)
-                const unsigned int prev = atomicAdd(&p.ctrl[2], 1u);
-                if (prev == gridDim.x - 1) {
-                    p.ctrl[2] = 0;
-                    p.ctrl[0] = 0;   // nobody is in a grid barrier any more
-                    unsigned long long t;
-                    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-                    reinterpret_cast<unsigned long long*>(p.ctrl)[16 + (int)(p.step & 1)] = t;
-                    __threadfence();
-                    skml_store_done(p.done_word, p.done_seq, p.status);
-                }
-            }
-        }
+        finish_launch<FUSED>(p, dsq);
         return;
     }
     if (FUSED) {
@@ -967,19 +975,7 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         reinterpret_cast<unsigned long long*>(p.ctrl)[11 + 4 * (int)(p.step & 1)] = t;
     }
-    finish_norm(p, dsq);
-    if (FUSED) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (p.done_word) __threadfence();
-            if (atomicAdd(&p.ctrl[2], 1u) == gridDim.x - 1) {
-                p.ctrl[2] = 0;
-                p.ctrl[0] = 0;
-                __threadfence();
-                skml_store_done(p.done_word, p.done_seq, p.status);
-            }
-        }
-    }
+    finish_launch<FUSED>(p, dsq);
 }
 
 extern "C" long long skml_decode_workspace_bytes(long long world, long long group_num) {
@@ -1062,7 +1058,12 @@ extern "C" int skml_decode_update(const SkmlDecodeArgs* a, void* stream_) {
         max_grid = per_sm * sms;
         cached_smem = smem;
     }
+    // Few keys: a block per SM, where each has a chunk at most (as many as a list's end takes more per group; a dense payload
+    // has a code per coordinate). The other blocks would only stand in line at the launch's end (see finish_launch
+    // for what this and a single count gave).
     int grid = a->grid > 0 ? (int)a->grid : DEC_BLOCKS_PER_SM * sms;
+    const long long few = (long long)sms * SKML_RESTART_INTERVAL;
+    if (a->grid <= 0 && a->world == 1 && a->key_capacity + groups * SKML_RESTART_INTERVAL <= few && (a->slot_capacity < a->dim || a->dim <= few)) grid = sms;
     cudaError_t e;
     if (a->fused) {
         if (max_grid < 1) return (int)cudaErrorLaunchOutOfResources;

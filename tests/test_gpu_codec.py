@@ -971,3 +971,26 @@ def test_launches_of_all_kinds_share_a_workspace():
         comp.fused = what != "staged"
         got = comp.compress_local(keys, vals, step=i, **kind)
         assert torch.equal(got, new(comp.fused).compress_local(keys, vals, step=i, **kind)), (i, what)
+
+
+@pytest.mark.parametrize("n,dim", [(1, 5), (5000, 50_000), (148 * 1024 - 8 * 1024, 1_000_000), (148 * 1024 - 8 * 1024 + 1, 1_000_000), (60_000, 60_000)])
+def test_decode_of_few_keys_by_a_block_per_sm(n, dim):
+    """Either side of the limit (room for a chunk per SM and one per group), a dense payload too: the bits of three blocks an SM."""
+    from sketchml_b200.ops import GpuCompressor, GpuDecoder
+    g = torch.Generator(device="cuda").manual_seed(n)
+    dense = n == dim
+    keys = None if dense else torch.randperm(dim, generator=g, device="cuda")[:n].sort().values.int()
+    vals = torch.randn(n, generator=g, device="cuda")
+    buf = GpuCompressor(dim, n, 64, 8, 2, 0.3, seed=5).compress_local(keys, vals, dense=dense)
+    status, out = torch.zeros(1, dtype=torch.int32, device="cuda"), []
+    for grid in (0, 3 * torch.cuda.get_device_properties(0).multi_processor_count):
+        dec = GpuDecoder(dim, n, max_groups=8, grid=grid)
+        w, sumsq, reg = torch.ones(dim, device="cuda"), torch.full((1,), float(dim), dtype=torch.float64, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+        dec.track_norm(sumsq, reg, 0.5)
+        dec.decode_update([buf.data_ptr()], [None], buf.numel(), 0, status, w=w, lr=0.5)
+        assert int(status.item()) == 0 and int((w != 1).sum()) > n // 2
+        norm = float(w.double().norm())
+        # n changes of a squared weight in fp32, each within 2^-22 of itself
+        assert abs(float(reg) - 0.5 * norm) <= 1e-6 * norm and abs(float(sumsq) - norm * norm) <= 2e-6 * norm * norm
+        out.append((w, dec.decode_sum([buf])))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
