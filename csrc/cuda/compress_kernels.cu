@@ -70,14 +70,14 @@ struct CP {
     unsigned short* chunk_part;      // [8 * chunks]: delta bytes of a chunk's eighths (128 keys)
     unsigned int* chunk_off;         // [2 * chunks]: delta-byte offset of a chunk inside its owner's part of the group
                                      // (delta_adaptive: flag-bit and delta-bit offsets)
-    unsigned long long* blk_bits;    // delta_adaptive: [grid][2 * SKML_MAX_GROUPS] flag bits / delta bits per block and group
-    unsigned int* blk_done;          // delta_adaptive: [grid] epoch in which the block finished writing its chunks
+    unsigned long long* blk_bits;    // delta_adaptive: [2 * SKML_MAX_GROUPS][2][MAX_GRID] flag bits / delta bits per block and group (tagged halves)
+    unsigned int* blk_done;          // bit streams on several ranks: [grid] epoch in which the block finished writing its chunks
     unsigned int* key_hist;          // delta_adaptive: [SKML_MAX_GROUPS][32] keys per delta width, zeroed in S1
     int key_encoder;
     int huffman;                     // sketch tables travel Huffman-coded (cell_bits = 0)
     int sample_splits;               // split points from a sample every cluster draws alike (no S2, two grid barriers fewer)
     unsigned int* cell_hist;         // Huffman: [bin_num + groups] cells per symbol, zeroed in S1
-    unsigned long long* blk_tbits;   // Huffman: [grid][SKML_MAX_GROUPS] code bits per block and group
+    unsigned long long* blk_tbits;   // Huffman: [SKML_MAX_GROUPS][2][MAX_GRID] code bits per block (in the tables' turn) and group (tagged halves)
     unsigned int* tchunk_off;        // Huffman: [table chunks] bit offset of a chunk inside its owner's part of the stream
     unsigned short* bins;
     int* gkeys;                      // keys, grouped: group g's list starts at Layout::goff[g]
@@ -217,11 +217,11 @@ static WsLayout ws_layout(long long n_max, long long q, long long G, long long r
     L.blk_flag = o; o += al256(grid * 4);
     L.chunk_off = o; o += al256((n_max / SKML_RESTART_INTERVAL + SKML_MAX_GROUPS + 8) * 8);
     L.chunk_part = o; o += al256((n_max / SKML_RESTART_INTERVAL + SKML_MAX_GROUPS + 8) * 16);
-    L.blk_bits = o; o += al256(grid * 2 * SKML_MAX_GROUPS * 8);
+    L.blk_bits = o; o += al256(2 * SKML_MAX_GROUPS * 2 * MAX_GRID * 8);
     L.blk_done = o; o += al256(grid * 4);
     L.key_hist = o; o += al256(SKML_MAX_GROUPS * 32 * 4);
     L.cell_hist = o; o += al256((SKML_GPU_MAX_BINS + SKML_MAX_GROUPS) * 4);
-    L.blk_tbits = o; o += al256(grid * SKML_MAX_GROUPS * 8);
+    L.blk_tbits = o; o += al256(SKML_MAX_GROUPS * 2 * MAX_GRID * 8);
     L.tchunk_off = o; o += al256(((rows * ((long long)(col_ratio * (double)n_max) + 2 + G) + 64) / 1024 + SKML_MAX_GROUPS + 8) * 4);
     L.bins = o; o += al256(n_max * 2);
     L.gkeys = o; o += al256((n_max + 4 * SKML_MAX_GROUPS + 8) * 4);
@@ -1906,17 +1906,6 @@ __device__ bool wait_published(const CP& p, const unsigned int* flags, unsigned 
     return __syncthreads_and(ok) != 0;
 }
 
-// Sum of one word of each of the blocks [0, count), by a warp, its loads in flight together.
-__device__ __forceinline__ unsigned long long sum_over_blocks(const unsigned long long* words, int stride, unsigned int count) {
-    const unsigned int lane = threadIdx.x & 31;
-    unsigned long long c[MAX_GRID / 32], v = 0;
-#pragma unroll
-    for (int k = 0; k < MAX_GRID / 32; ++k) c[k] = lane + 32 * k < count ? __ldcg(words + (long long)(lane + 32 * k) * stride) : 0ull;
-#pragma unroll
-    for (int k = 0; k < MAX_GRID / 32; ++k) v += c[k];
-    return warp_sum(v);
-}
-
 // Sum of one word of the blocks [0, count) (see read_row), by a warp.
 template <bool WAIT>
 __device__ __forceinline__ bool sum_row(const CP& p, const unsigned long long* words, unsigned int count, unsigned int epoch, unsigned int where,
@@ -1928,6 +1917,25 @@ __device__ __forceinline__ bool sum_row(const CP& p, const unsigned long long* w
     for (int k = 0; k < MAX_GRID / 32; ++k) sum += (threadIdx.x & 31) + 32 * k < count ? c[k] : 0u;
     sum = warp_sum(sum);
     return ok;
+}
+
+// The same for numbers of 64 bits, whose halves are words of their own: halves 2 i and 2 i + 1 of the i-th number of block `at`.
+template <bool FUSED>
+__device__ __forceinline__ void put_halves(unsigned long long* words, unsigned int i, unsigned int at, unsigned int epoch, unsigned long long v) {
+    const unsigned long long tag = (unsigned long long)(FUSED ? epoch : 0u) << 32;
+    st_relaxed_gpu64(words + (2 * i) * MAX_GRID + at, tag | (v & 0xFFFFFFFFull));
+    st_relaxed_gpu64(words + (2 * i + 1) * MAX_GRID + at, tag | (v >> 32));
+}
+__device__ __forceinline__ unsigned long long get_halves(const unsigned long long* words, unsigned int i, unsigned int at) {
+    return (__ldcg(words + (2 * i) * MAX_GRID + at) & 0xFFFFFFFFull) | (__ldcg(words + (2 * i + 1) * MAX_GRID + at) << 32);
+}
+template <bool WAIT>
+__device__ __forceinline__ bool sum_halves(const CP& p, const unsigned long long* words, unsigned int i, unsigned int count, unsigned int epoch,
+                                           unsigned int where, unsigned long long& sum) {
+    unsigned long long lo, hi;
+    const bool a = sum_row<WAIT>(p, words + (2 * i) * MAX_GRID, count, epoch, where, lo), b = sum_row<WAIT>(p, words + (2 * i + 1) * MAX_GRID, count, epoch, where, hi);
+    sum = lo + (hi << 32);
+    return a && b;
 }
 
 // Byte totals of the blocks before this one (they own the chunks before this block's run, so the
@@ -2105,11 +2113,10 @@ __device__ __forceinline__ unsigned long long stream_bytes(unsigned long long bi
 // Pass 1 prelude (every block): interval count and flag kind of every group from the complete
 // histogram. The histogram also gives the exact lengths of the two bit streams of every group, so the
 // whole layout of the key sections is known here, before a single key is coded.
-__device__ void apack_choose(const CP& p, Smem& s) {
+__device__ __forceinline__ void apack_modes(const CP& p, Smem& s, int first, int step) {   // a warp per group, lane = delta width
     Layout& L = s.lay;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp < p.G) {   // a warp per group, lane = delta width
-        const int g = warp;
+    const int lane = threadIdx.x & 31;
+    for (int g = first; g < p.G; g += step) {
         double* prob = reinterpret_cast<double*>(s.cs.stage_d) + 32 * g;   // (the staging area is idle until pass 2)
         const unsigned int h = __ldcg(&p.key_hist[g * 32 + lane]), n = L.n_g[g];
         prob[lane] = __ddiv_rn((double)h, (double)(n > 0 ? n : 1));
@@ -2156,8 +2163,13 @@ __device__ void apack_choose(const CP& p, Smem& s) {
             L.delta_bits[g] = dbits;
         }
     }
-    __syncthreads();
-    if (warp == 0) {
+}
+
+// And the key sections' places behind what lies before them (one warp).
+__device__ __forceinline__ void apack_places(const CP& p, Smem& s) {
+    Layout& L = s.lay;
+    const int lane = threadIdx.x & 31;
+    {
         const bool any = lane < p.G && L.n_g[lane];
         const unsigned long long f = any ? stream_bytes(L.flag_bits[lane]) : 0ull, d = any ? stream_bytes(L.delta_bits[lane]) : 0ull;
         unsigned long long all;
@@ -2174,8 +2186,15 @@ __device__ void apack_choose(const CP& p, Smem& s) {
             }
         }
     }
+}
+
+__device__ void apack_choose(const CP& p, Smem& s) {
+    apack_modes(p, s, threadIdx.x >> 5, SKML_WARPS);
+    __syncthreads();
+    if (threadIdx.x < 32) apack_places(p, s);
     __syncthreads();
 }
+
 
 struct KeyCode {
     unsigned int fv, fw, dw;  // flag value / width, delta width (the delta value is the delta itself)
@@ -2202,7 +2221,8 @@ __device__ __forceinline__ void put_bits_shared(unsigned int* words, unsigned in
 
 // Pass 1: flag and delta bits of this block's chunks -> chunk bit offsets inside the block's part of
 // each group, the block's bit totals per group (published for the blocks after it).
-__device__ void apack_measure(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
+template <bool FUSED>
+__device__ void apack_measure(const CP& p, Smem& s, unsigned int epoch, unsigned int my_begin, unsigned int my_end) {
     const Layout& L = s.lay;
     if (threadIdx.x < 2 * SKML_MAX_GROUPS) s.my_bits[threadIdx.x] = 0;
     __syncthreads();
@@ -2234,18 +2254,20 @@ __device__ void apack_measure(const CP& p, Smem& s, unsigned int my_begin, unsig
         }
         __syncthreads();
     }
-    if (threadIdx.x < 2 * SKML_MAX_GROUPS) p.blk_bits[(long long)blockIdx.x * 2 * SKML_MAX_GROUPS + threadIdx.x] = s.my_bits[threadIdx.x];
+    if ((int)threadIdx.x < 2 * p.G) put_halves<FUSED>(p.blk_bits, threadIdx.x, blockIdx.x, epoch, s.my_bits[threadIdx.x]);
 }
 
 // Bit totals of the blocks before this one -> this block's starting bit offsets inside the streams.
-__device__ void apack_prefix(const CP& p, Smem& s, bool wait, unsigned int epoch) {
-    const bool ok = !wait || wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x52u);
+template <bool WAIT>
+__device__ void apack_prefix(const CP& p, Smem& s, unsigned int epoch) {
+    bool ok = true;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int g = warp; g < 2 * p.G; g += SKML_WARPS) {
-        const unsigned long long v = sum_over_blocks(p.blk_bits + g, 2 * SKML_MAX_GROUPS, blockIdx.x);
+        unsigned long long v;
+        ok = sum_halves<WAIT>(p, p.blk_bits, g, blockIdx.x, epoch, 0x52u, v) && ok;
         if (lane == 0) s.pre_bits[g] = v;
     }
-    if (threadIdx.x == 0 && !ok) s.lay.overflow = 1;
+    if (!__syncthreads_and(ok) && threadIdx.x == 0) s.lay.overflow = 1;
     __syncthreads();
 }
 
@@ -2355,8 +2377,8 @@ __device__ void apush_borders(const CP& p, Smem& s) {
         if (cs != L.chunk_prefix[g]) {  // the run of block b starts inside group g
             unsigned long long a[2] = {0, 0};
             for (unsigned int q = 0; q < b; ++q) {
-                a[0] += __ldcg(&p.blk_bits[(long long)q * 2 * SKML_MAX_GROUPS + 2 * g]);
-                a[1] += __ldcg(&p.blk_bits[(long long)q * 2 * SKML_MAX_GROUPS + 2 * g + 1]);
+                a[0] += get_halves(p.blk_bits, 2 * g, q);
+                a[1] += get_halves(p.blk_bits, 2 * g + 1, q);
             }
             for (int k = 0; k < 2; ++k) {
                 if ((a[k] & 127ull) == 0) continue;
@@ -2385,12 +2407,12 @@ __device__ __forceinline__ unsigned int huf_slot(const Layout& L, int g, unsigne
     return L.sym_lo[g] + (unsigned int)g + (sidx < L.nsym[g] ? sidx : L.nsym[g] - 1u);
 }
 
-// Table chunks (1024 cells of one group's table, group-major) of this block: a contiguous run.
-__device__ __forceinline__ void tchunk_run(const Layout& L, int G, unsigned int& t_begin, unsigned int& t_end) {
+// Table chunks (1024 cells of one group's table, group-major) of the block whose turn it is: a contiguous run.
+__device__ __forceinline__ void tchunk_run(const Layout& L, int G, unsigned int turn, unsigned int& t_begin, unsigned int& t_end) {
     const unsigned int total = L.tchunk_prefix[G];
     unsigned int per = (total + gridDim.x - 1) / gridDim.x;
     per = (per + 3u) & ~3u;
-    t_begin = min(total, per * blockIdx.x);
+    t_begin = min(total, per * turn);
     t_end = min(total, t_begin + per);
 }
 
@@ -2465,6 +2487,9 @@ __device__ void huf_histogram(const CP& p, Smem& s, unsigned int t_begin, unsign
 // Only the merges are a chain (one lane, the two candidates of either queue read side by side); sorting,
 // code lengths (a walk to the root per leaf) and code words are the whole warp's. (One lane for all of it,
 // reading the histogram from L2, was some 35 us of a launch.)
+// ADAPTIVE: the other warps choose the key code's modes meanwhile, and its places follow (170,000 keys: with the counts sent by themselves and the
+// tables coded by other blocks than the keys, the launch 66 -> 54 us; 560,000 keys 96 -> 84).
+template <bool ADAPTIVE>
 __device__ void huf_build(const CP& p, Smem& s) {
     Layout& L = s.lay;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2564,6 +2589,8 @@ __device__ void huf_build(const CP& p, Smem& s) {
             }
             __syncwarp();
         }
+    } else if (ADAPTIVE && warp >= 8) {
+        apack_modes(p, s, warp - 8, SKML_WARPS - 8);
     }
     __syncthreads();
     if (warp == 0) {   // sections start at multiples of 16, so their sizes do not depend on where
@@ -2591,13 +2618,16 @@ __device__ void huf_build(const CP& p, Smem& s) {
                 skml_set_status(p.status, SKML_CAPACITY, 0x3Au);
             }
         }
+        __syncwarp();
+        if (ADAPTIVE) apack_places(p, s);
     }
     __syncthreads();
 }
 
 // Pass 1: code bits of this block's table chunks -> chunk offsets inside the block's part of each
 // group's stream, the block's bit totals per group (published with the key counts).
-__device__ void huf_measure(const CP& p, Smem& s, unsigned int t_begin, unsigned int t_end) {
+template <bool FUSED>
+__device__ void huf_measure(const CP& p, Smem& s, unsigned int epoch, unsigned int turn, unsigned int t_begin, unsigned int t_end) {
     const Layout& L = s.lay;
     if (threadIdx.x < SKML_MAX_GROUPS) s.my_tbits[threadIdx.x] = 0;
     __syncthreads();
@@ -2624,16 +2654,20 @@ __device__ void huf_measure(const CP& p, Smem& s, unsigned int t_begin, unsigned
         }
         __syncthreads();
     }
-    if (threadIdx.x < SKML_MAX_GROUPS) p.blk_tbits[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x] = s.my_tbits[threadIdx.x];
+    if ((int)threadIdx.x < p.G) put_halves<FUSED>(p.blk_tbits, threadIdx.x, turn, epoch, s.my_tbits[threadIdx.x]);
 }
 
-// Table bits of the blocks before this one (the caller has waited for their publications).
-__device__ void huf_prefix(const CP& p, Smem& s) {
+// Table bits of the blocks whose turn is before this one's.
+template <bool WAIT>
+__device__ void huf_prefix(const CP& p, Smem& s, unsigned int epoch, unsigned int turn) {
+    bool ok = true;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < p.G) {
-        const unsigned long long v = sum_over_blocks(p.blk_tbits + warp, SKML_MAX_GROUPS, blockIdx.x);
+        unsigned long long v;
+        ok = sum_halves<WAIT>(p, p.blk_tbits, warp, turn, epoch, 0x53u, v);
         if (lane == 0) s.pre_tbits[warp] = v;
     }
+    if (!__syncthreads_and(ok) && threadIdx.x == 0) s.lay.overflow = 1;
     __syncthreads();
 }
 
@@ -2758,7 +2792,7 @@ __device__ void huf_push_borders(const CP& p, Smem& s) {
         while (g + 1 < p.G && cs >= L.tchunk_prefix[g + 1]) ++g;
         if (cs != L.tchunk_prefix[g]) {
             unsigned long long a = 0;
-            for (unsigned int q = 0; q < b; ++q) a += __ldcg(&p.blk_tbits[(long long)q * SKML_MAX_GROUPS + g]);
+            for (unsigned int q = 0; q < b; ++q) a += get_halves(p.blk_tbits, g, q);
             const unsigned long long bit = 8ull * L.tstream_off[g] + a;
             if (bit & 127ull) {
                 const unsigned long long off = 16ull * (bit / 128ull);
@@ -3362,7 +3396,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     // insert in shared memory every block waits for all of them, behind its own keys, before it merges the copies;
     // staged launches split the stage at those points. The delta_adaptive
     // code needs the groups' complete histograms of delta widths first: one more grid barrier.
-    unsigned int my_begin = 0, my_end = 0, t_begin = 0, t_end = 0, nactive = 0;
+    unsigned int my_begin = 0, my_end = 0, t_begin = 0, t_end = 0, nactive = 0, turn = 0;
     constexpr bool adaptive = ADAPTIVE, huffman = HUFFMAN;
     if (FUSED || stage >= 5) {
         if (!FUSED) {
@@ -3372,7 +3406,9 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         nactive = chunk_run(s.lay, p.G, my_begin, my_end);
         if (huffman) {
             huf_ranges(p, s);
-            tchunk_run(s.lay, p.G, t_begin, t_end);
+            // the tables' chunks begin behind the blocks that have keys to code
+            turn = blockIdx.x >= nactive ? blockIdx.x - nactive : blockIdx.x + gridDim.x - nactive;
+            tchunk_run(s.lay, p.G, turn, t_begin, t_end);
         }
     }
     if (FUSED || stage == 5) {
@@ -3388,17 +3424,17 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     }
     if (FUSED || stage >= 6) {
         // code tables and the layout behind the tables (every block; staged launches repeat it per stage)
-        if (huffman && (FUSED || stage >= 6)) huf_build(p, s);
-        if (adaptive) apack_choose(p, s);
+        if (huffman) huf_build<ADAPTIVE>(p, s);
+        else if (adaptive) apack_choose(p, s);
     }
     ChunkWork cw;
     unsigned int boff = 0, btotal = 0;
     if (FUSED || stage == 6) {
-        if (adaptive) apack_measure(p, s, my_begin, my_end);
+        if (adaptive) apack_measure<FUSED>(p, s, epoch, my_begin, my_end);
         else if (my_begin < my_end) pack_measure<FUSED>(p, s, epoch, my_begin, my_end, cw, boff, btotal);
-        if (huffman) huf_measure(p, s, t_begin, t_end);
+        if (huffman) huf_measure<FUSED>(p, s, epoch, turn, t_begin, t_end);
     }
-    if (FUSED && (adaptive || huffman || priv)) {   // (the plain key code's counts carry the number themselves)
+    if (FUSED && priv) {   // (counts carry the number themselves, the copies of an insert in shared memory do not)
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
@@ -3406,33 +3442,27 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         }
     }
     if (!huffman && !adaptive && !priv && (FUSED || stage == 6)) narrow_tables(p, s, nactive);   // while the publications travel
-    const bool borders = adaptive || huffman;  // stream words shared by two blocks are sent by the last block at the end
+    const bool borders = (adaptive || huffman) && p.world > 1;  // stream words shared by two blocks are sent by the last block at the end
     if (FUSED || stage == 7) {
         if (!FUSED) {  // the block's own counts again (shared memory does not survive a launch)
             if (threadIdx.x < SKML_MAX_GROUPS) {
                 s.my_bytes[threadIdx.x] = (unsigned int)p.blk_bytes[threadIdx.x * MAX_GRID + blockIdx.x];
-                s.my_tbits[threadIdx.x] = p.blk_tbits[(long long)blockIdx.x * SKML_MAX_GROUPS + threadIdx.x];
+                s.my_tbits[threadIdx.x] = get_halves(p.blk_tbits, threadIdx.x, turn);
             }
-            if (threadIdx.x < 2 * SKML_MAX_GROUPS) s.my_bits[threadIdx.x] = p.blk_bits[(long long)blockIdx.x * 2 * SKML_MAX_GROUPS + threadIdx.x];
+            if (threadIdx.x < 2 * SKML_MAX_GROUPS) s.my_bits[threadIdx.x] = get_halves(p.blk_bits, threadIdx.x, blockIdx.x);
             __syncthreads();
         }
         if (adaptive) {
-            apack_prefix(p, s, FUSED, epoch);
+            apack_prefix<FUSED>(p, s, epoch);
             apack_write(p, s, my_begin, my_end);
             apush_own_chunks(p, s, my_begin, my_end);
-        } else {
-            if (FUSED && huffman) {   // what huf_prefix below reads
-                if (!wait_published(p, p.blk_flag, blockIdx.x, epoch, 0x53u) && threadIdx.x == 0) s.lay.overflow = 1;
-                __syncthreads();
-            }
-            if (my_begin < my_end) {
-                pack_prefix<FUSED>(p, s, epoch);
-                pack_write(p, s, my_begin, my_end, FUSED && my_end - my_begin <= 4, cw, boff, btotal);
-                push_own_chunks(p, s, my_begin, my_end);
-            }
+        } else if (my_begin < my_end) {
+            pack_prefix<FUSED>(p, s, epoch);
+            pack_write(p, s, my_begin, my_end, FUSED && my_end - my_begin <= 4, cw, boff, btotal);
+            push_own_chunks(p, s, my_begin, my_end);
         }
         if (huffman) {
-            huf_prefix(p, s);   // (the blocks before this one have been waited for)
+            huf_prefix<FUSED>(p, s, epoch, turn);
             huf_write(p, s, t_begin, t_end);
             huf_push_own(p, s, t_begin, t_end);
         }
