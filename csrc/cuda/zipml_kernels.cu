@@ -37,8 +37,12 @@ constexpr int Z_MAX_BUCKETS = 8192;     // the split and midpoint tables are sta
 constexpr int Z_KPT = 8;                // values a thread handles per tile of the prefix sums
 constexpr int Z_ALONE = ZT * Z_KPT;     // pairs one block handles in shared memory: below, a barrier costs more than it saves
 constexpr int Z_MAX_BLOCKS = 148;
-constexpr int Z_TAIL = 512;             // candidates one warp handles in shared memory and registers, without a barrier
+// Candidates block 0 keeps in shared memory for the last rounds, a pair a thread: where the blocks' lists were, so that the
+// block stays below the 164 KB that leave 92 KB of L1 (2048 of them in memory of their own: the search of 233,000 values 154 us
+// instead of 139). With two pairs' loads in flight in the rounds before: 233,000 values 145 -> 139 us, 48,000 99 -> 92, 16,000 97 -> 90.
+constexpr int Z_TAIL = 1536;
 
+constexpr int Z_FLIGHT = 2;             // pairs of a thread whose loads are in flight together
 constexpr int Z_SORT_KEYS = 8;          // values a thread of the sort keeps in registers
 constexpr int Z_SORT_ALONE = 6144;      // values that one block sorts (44 KB of shared memory)
 
@@ -299,41 +303,57 @@ __device__ __forceinline__ void pair_errors(const ZScratch& z, const int* idx, u
         int at;
         double2 sum;
     };
-    auto front = [&](unsigned int pair) {   // where a pair begins, and the sums up to there
-        Front f;
-        f.at = 2 * pair >= split_num ? (int)n : __ldcg(idx + 2 * pair);
-        f.sum = f.at ? z.rt[f.at - 1] : make_double2(0.0, 0.0);
-        return f;
-    };
-    for (unsigned int i0 = 0; i0 < count; i0 += ZT) {
-        const unsigned int i = i0 + threadIdx.x;
-        const bool in = i < count;
-        Front lo{0, make_double2(0.0, 0.0)}, hi;
-        if (in) lo = front(p0 + i);
-        hi.at = __shfl_down_sync(0xFFFFFFFFu, lo.at, 1);
-        hi.sum.x = __shfl_down_sync(0xFFFFFFFFu, lo.sum.x, 1);
-        hi.sum.y = __shfl_down_sync(0xFFFFFFFFu, lo.sum.y, 1);
-        if (in && (lane == 31 || i + 1 >= count)) hi = front(p0 + i + 1);
-        if (in) {
-            const double l1 = __dadd_rn(hi.sum.x, lo.at ? -lo.sum.x : 0.0), l2 = __dadd_rn(hi.sum.y, lo.at ? -lo.sum.y : 0.0);
-            key[i] = merge_error(l1, l2, (double)(hi.at - lo.at));
+    auto place = [&](unsigned int pair) { return 2 * pair >= split_num ? (int)n : __ldcg(idx + 2 * pair); };   // where a pair begins
+    auto sum_to = [&](int at) { return at ? z.rt[at - 1] : make_double2(0.0, 0.0); };                          // the sums up to there
+    // Z_FLIGHT pairs of a thread at a time: a pair is two trips to L2, one behind the other (one block alone, 7,400 pairs: 10 us
+    // with one in flight)
+    for (unsigned int i0 = 0; i0 < count; i0 += Z_FLIGHT * ZT) {
+        Front lo[Z_FLIGHT], hi[Z_FLIGHT];
+#pragma unroll
+        for (int u = 0; u < Z_FLIGHT; ++u) {
+            const unsigned int i = i0 + u * ZT + threadIdx.x;
+            lo[u].at = i < count ? place(p0 + i) : 0;
+            hi[u].at = i < count && (lane == 31 || i + 1 >= count) ? place(p0 + i + 1) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < Z_FLIGHT; ++u) {
+            lo[u].sum = sum_to(lo[u].at);
+            hi[u].sum = sum_to(hi[u].at);
+        }
+#pragma unroll
+        for (int u = 0; u < Z_FLIGHT; ++u) {
+            const unsigned int i = i0 + u * ZT + threadIdx.x;
+            const bool last = lane == 31 || i + 1 >= count;
+            Front up;
+            up.at = __shfl_down_sync(0xFFFFFFFFu, lo[u].at, 1);
+            up.sum.x = __shfl_down_sync(0xFFFFFFFFu, lo[u].sum.x, 1);
+            up.sum.y = __shfl_down_sync(0xFFFFFFFFu, lo[u].sum.y, 1);
+            if (last) up = hi[u];
+            if (i < count) {
+                const double l1 = __dadd_rn(up.sum.x, lo[u].at ? -lo[u].sum.x : 0.0), l2 = __dadd_rn(up.sum.y, lo[u].at ? -lo[u].sum.y : 0.0);
+                key[i] = merge_error(l1, l2, (double)(up.at - lo[u].at));
+            }
         }
     }
 }
 
 struct ZSmem {
     unsigned long long key[Z_ALONE];   // errors of the block's slice of a round, where they fit
-    unsigned long long all[Z_ALONE];   // the lists of all blocks
     unsigned int hist[ZT];             // select_largest
     unsigned int warp[33];
     double2 dwarp[32];
     unsigned int digit, above, ncand, fill;
-    // the last rounds (at most Z_TAIL candidates): their positions and the prefix sums in front of them
+    // the last rounds (at most Z_TAIL candidates, of one block): their positions and the prefix sums in front of them
     struct Tail {
         int pos[Z_TAIL];
         double sum_v[Z_TAIL], sum_v2[Z_TAIL];
-    } tail[2];                         // a round reads one and writes the other
+    };
+    union {
+        unsigned long long all[Z_ALONE];   // the lists of all blocks
+        Tail tail[2];                      // a round reads one and writes the other
+    };
 };
+static_assert(Z_TAIL <= 2 * ZT && sizeof(ZSmem) <= 162 * 1024, "a pair a thread; the 164 KB carve-out");
 
 // Threshold for the k largest of keys[0, count), in shared memory or global (0 = no key, k keys at least): the k-th
 // largest, or a value that exactly k keys reach (`exact`). Radix select, ten bits a pass from the top: a
@@ -381,7 +401,7 @@ __device__ __noinline__ unsigned long long select_largest(ZSmem& sm, const unsig
     }
 }
 
-// The last rounds: at most Z_TAIL candidates in shared memory, a pair per thread of the first eight warps; the
+// The last rounds: at most Z_TAIL candidates in shared memory, a pair per thread; the
 // selection is the block's. Every thread keeps count of the set.
 __device__ void tail_rounds(ZSmem& sm, int bin_num, double end_v, double end_v2, int n, unsigned int& split_num, unsigned int& rounds,
                             unsigned int& which) {

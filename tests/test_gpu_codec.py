@@ -994,3 +994,14 @@ def test_decode_of_few_keys_by_a_block_per_sm(n, dim):
         assert abs(float(reg) - 0.5 * norm) <= 1e-6 * norm and abs(float(sumsq) - norm * norm) <= 2e-6 * norm * norm
         out.append((w, dec.decode_sum([buf])))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("n,bins", [(1535, 64), (1536, 64), (1537, 64), (1538, 2), (3071, 256), (3072, 1500), (3073, 1535), (6200, 1537), (16385, 700)])
+def test_zipml_last_rounds_around_their_room(n, bins):
+    """Searches whose rounds reach the 1,536 candidates of the last rounds from the start, exactly, one above, or never; odd numbers."""
+    from sketchml_b200.compress import oracle
+    vals = (np.random.default_rng(n + bins).integers(-3000, 3001, n) / 1024.0).astype(np.float32)   # exact sums
+    ref = oracle.zipml_quantize(vals.astype(np.float64), bins)
+    zc, v, cnt, nb, zero, rounds, splits, mids, codes = _zip_pack(vals, bins)
+    assert nb == ref["bin_num"] and zero == ref["zero_idx"] and np.array_equal(splits.astype(np.float64), ref["splits"])
+    assert np.array_equal(mids, ref["values"].astype(np.float32)) and np.array_equal(codes, ref["bins"])
