@@ -407,7 +407,7 @@ __device__ __forceinline__ void stage_stamp(unsigned int* ctrl, int i) {
 // Clears the local slot from byte `from` (a multiple of 16) on, in 16-byte units; a capacity that is no multiple of 16
 // keeps its last bytes to the tail. Nothing orders the callers' stores against those of other blocks: bytes that
 // another block writes in the same launch need a grid barrier in between.
-__device__ void clear_slot(const CP& p, long long from, long long gid, long long gsz) {
+__device__ __noinline__ void clear_slot(const CP& p, long long from, long long gid, long long gsz) {
     uint4* z4 = reinterpret_cast<uint4*>(p.payload);
     for (long long i = from / 16 + gid; i < p.slot_capacity / 16; i += gsz) __stcs(z4 + i, make_uint4(0, 0, 0, 0));
     if (gid < (p.slot_capacity & 15)) p.payload[(p.slot_capacity & ~15ll) + gid] = 0;
@@ -711,7 +711,7 @@ __device__ unsigned long long merge_two_runs(Smem& s, unsigned int ca, unsigned 
 // their runs in shared memory (the cluster's first block reads the others' runs through distributed
 // shared memory) and only the merged run goes to global memory, so S2 has 1 / cluster-size as many runs
 // to load and to rank against. Launched without clusters the cluster is the block itself.
-__device__ void stage_summary(const CP& p, Smem& s, unsigned int* set, const float* __restrict__ vals, long long n) {
+__device__ __noinline__ void stage_summary(const CP& p, Smem& s, unsigned int* set, const float* __restrict__ vals, long long n) {
     __shared__ unsigned int s_pub_cnt;
     __shared__ unsigned long long s_pub_w;
     unsigned int cnt;
@@ -863,7 +863,7 @@ __device__ __forceinline__ unsigned long long rank_target(long long n, int t, do
     return r << FP_SHIFT;
 }
 
-__device__ void stage_query(const CP& p, Smem& s, long long n) {
+__device__ __noinline__ void stage_query(const CP& p, Smem& s, long long n) {
     if (n <= 0) return;
     const int nb = gridDim.x;
     for (int t = threadIdx.x; t < nb; t += blockDim.x) {
@@ -2084,7 +2084,7 @@ __device__ void pack_write(const CP& p, Smem& s, unsigned int my_begin, unsigned
 // words, and the sections' sizes depend on the data: the two sections of a group follow each other
 // at the end of the payload, and the (pre-zeroed) shared words are completed with atomic ORs.
 // ---------------------------------------------------------------------------
-__device__ void push_bytes(const CP& p, unsigned long long lo, unsigned long long hi);
+__device__ __noinline__ void push_bytes(const CP& p, unsigned long long lo, unsigned long long hi);
 
 __device__ __forceinline__ int da_bits_needed(unsigned int d) { return d == 0u ? 1 : 32 - __clz(d); }
 
@@ -2344,7 +2344,7 @@ __device__ void apack_write(const CP& p, Smem& s, unsigned int my_begin, unsigne
 
 // The restart points and the 16-byte units of the two bit streams that hold bits of this block only
 // -> the peers' slots. Units that hold a block border are sent by the last block once every block is done.
-__device__ void apush_own_chunks(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
+__device__ __noinline__ void apush_own_chunks(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow || my_begin >= my_end) return;
     __syncthreads();
@@ -2363,7 +2363,7 @@ __device__ void apush_own_chunks(const CP& p, Smem& s, unsigned int my_begin, un
 }
 
 // The last block, after every block has written its chunks: the stream units that hold a block border.
-__device__ void apush_borders(const CP& p, Smem& s) {
+__device__ __noinline__ void apush_borders(const CP& p, Smem& s) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow) return;
     const unsigned int total = L.chunk_prefix[p.G];
@@ -2753,7 +2753,7 @@ __device__ __forceinline__ void own_units(unsigned long long base, unsigned long
 
 // The parts of the coded tables this block wrote -> the peers' slots (units that hold a block border
 // are sent by block 0 once every block is done).
-__device__ void huf_push_own(const CP& p, Smem& s, unsigned int t_begin, unsigned int t_end) {
+__device__ __noinline__ void huf_push_own(const CP& p, Smem& s, unsigned int t_begin, unsigned int t_end) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow || t_begin >= t_end) return;
     __syncthreads();
@@ -2779,7 +2779,7 @@ __device__ void huf_push_own(const CP& p, Smem& s, unsigned int t_begin, unsigne
 }
 
 // Block 0, after every block has written: the units of the table streams that hold a block border.
-__device__ void huf_push_borders(const CP& p, Smem& s) {
+__device__ __noinline__ void huf_push_borders(const CP& p, Smem& s) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow) return;
     const unsigned int total = L.tchunk_prefix[p.G];
@@ -3119,7 +3119,7 @@ __device__ void merge_copies(const CP& p, Smem& s) {
 // Bytes [lo, hi) of the local payload -> the same bytes of every peer's slot, by this block alone:
 // 16-byte stores for the aligned interior, byte stores for a ragged head or tail (two blocks that
 // share a 16-byte unit each store only their own bytes of it).
-__device__ void push_bytes(const CP& p, unsigned long long lo, unsigned long long hi) {
+__device__ __noinline__ void push_bytes(const CP& p, unsigned long long lo, unsigned long long hi) {
     if (p.world <= 1 || hi <= lo) return;
     const unsigned long long a0 = (lo + 15ull) & ~15ull, a1 = hi & ~15ull;
     if (a0 < a1) {
@@ -3141,7 +3141,7 @@ __device__ void push_bytes(const CP& p, unsigned long long lo, unsigned long lon
 }
 
 // The flag bytes, restart points and delta bytes this block wrote for its chunks -> the peers' slots.
-__device__ void push_own_chunks(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
+__device__ __noinline__ void push_own_chunks(const CP& p, Smem& s, unsigned int my_begin, unsigned int my_end) {
     const Layout& L = s.lay;
     if (p.world <= 1 || L.overflow || my_begin >= my_end) return;
     __syncthreads();  // this block's own stores are visible to all its threads
@@ -3284,8 +3284,8 @@ __device__ void dense_stages(const CP& p, Smem& s, unsigned int* set, unsigned i
 // ADAPTIVE / HUFFMAN: the key encoder and the table coder are compile-time choices, so that the default
 // path (delta_binary keys, plain tables) carries none of the other coders' registers. PRIV: launches that may have enough
 // keys for the insert in shared memory (its code costs the others 2 us).
-template <bool FUSED, bool ADAPTIVE, bool HUFFMAN, bool PRIV>
-__global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, int stage) {
+template <bool FUSED, bool ADAPTIVE, bool HUFFMAN, bool PRIV, bool DENSE>
+__global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(const __grid_constant__ CP p, int stage) {
     skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
@@ -3298,7 +3298,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     const unsigned int epoch = ctrl_open<FUSED>(p.ctrl);   // names this launch's publications
     unsigned int* const set = ctrl_set(p.ctrl, epoch);
     if (kind == SKML_KIND_DENSE) {  // un-fused launches leave it to the dense kernel's stages
-        if (FUSED && p.dense_vals) dense_stages<FUSED>(p, s, set, epoch, p.dense_vals, stage);
+        if (FUSED && DENSE && p.dense_vals) dense_stages<FUSED>(p, s, set, epoch, p.dense_vals, stage);
         return;
     }
     if (n > p.n_max) {
@@ -3455,16 +3455,16 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
         if (adaptive) {
             apack_prefix<FUSED>(p, s, epoch);
             apack_write(p, s, my_begin, my_end);
-            apush_own_chunks(p, s, my_begin, my_end);
+            if (p.world > 1) apush_own_chunks(p, s, my_begin, my_end);
         } else if (my_begin < my_end) {
             pack_prefix<FUSED>(p, s, epoch);
             pack_write(p, s, my_begin, my_end, FUSED && my_end - my_begin <= 4, cw, boff, btotal);
-            push_own_chunks(p, s, my_begin, my_end);
+            if (p.world > 1) push_own_chunks(p, s, my_begin, my_end);
         }
         if (huffman) {
             huf_prefix<FUSED>(p, s, epoch, turn);
             huf_write(p, s, t_begin, t_end);
-            huf_push_own(p, s, t_begin, t_end);
+            if (p.world > 1) huf_push_own(p, s, t_begin, t_end);
         }
         if (priv) {   // every block has made its copies before it published its counts
             if (!wait_published(p, p.blk_flag, gridDim.x, epoch, 0x54u)) return;
@@ -3482,9 +3482,9 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
     if (FUSED || stage == 8) {
         if (blockIdx.x == gridDim.x - 1) {
             if (FUSED && borders && !wait_published(p, p.blk_done, gridDim.x, epoch, 0x51u)) return;
-            if (adaptive) apush_borders(p, s);
-            else if (!layout_finish<FUSED>(p, s, epoch, nactive)) return;
-            if (huffman) huf_push_borders(p, s);
+            if (adaptive && borders) apush_borders(p, s);
+            if (!adaptive && !layout_finish<FUSED>(p, s, epoch, nactive)) return;
+            if (huffman && borders) huf_push_borders(p, s);
             write_header(p, s, n, SKML_KIND_SPARSE);
         }
         finish_publish<FUSED>(p, set, blockIdx.x == gridDim.x - 1);
@@ -3493,7 +3493,7 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(CP p, in
 }
 
 template <bool FUSED>
-__global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(CP p, int stage) {
+__global__ void __launch_bounds__(SKML_BLOCK, 1) compress_dense_kernel(const __grid_constant__ CP p, int stage) {
     skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if ((p.meta ? p.meta[1] : p.kind_value) != SKML_KIND_DENSE) return;
@@ -3736,19 +3736,18 @@ extern "C" int skml_compress_sparse(const SkmlCompressArgs* a, void* stream) {
     int grid = 0;
     int rc = fill_params(a, p, grid);
     if (rc) return rc;
-    static LaunchCache cache[6];
+    static LaunchCache cache[8];
     const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE, huffman = p.huffman != 0;
-    const bool fused = a->fused != 0, priv = fused && !huffman && p.priv;
+    const bool fused = a->fused != 0, priv = fused && !huffman && p.priv, dense = p.dense_vals != nullptr;
     cudaStream_t st = (cudaStream_t)stream;
-    if (adaptive && huffman)
-        return launch_stages(compress_sparse_kernel<true, true, true, false>, compress_sparse_kernel<false, true, true, false>, cache[3], p, grid, fused, 8, st);
-    if (huffman)
-        return launch_stages(compress_sparse_kernel<true, false, true, false>, compress_sparse_kernel<false, false, true, false>, cache[1], p, grid, fused, 8, st);
-    if (adaptive)
-        return priv ? launch_stages(compress_sparse_kernel<true, true, false, true>, compress_sparse_kernel<false, true, false, false>, cache[5], p, grid, fused, 8, st)
-                    : launch_stages(compress_sparse_kernel<true, true, false, false>, compress_sparse_kernel<false, true, false, false>, cache[2], p, grid, fused, 8, st);
-    return priv ? launch_stages(compress_sparse_kernel<true, false, false, true>, compress_sparse_kernel<false, false, false, false>, cache[4], p, grid, fused, 8, st)
-                : launch_stages(compress_sparse_kernel<true, false, false, false>, compress_sparse_kernel<false, false, false, false>, cache[0], p, grid, fused, 8, st);
+    auto go = [&](auto kernel, auto staged, int which) { return launch_stages(kernel, staged, cache[which], p, grid, fused, 8, st); };
+    if (adaptive && huffman) return go(compress_sparse_kernel<true, true, true, false, true>, compress_sparse_kernel<false, true, true, false, false>, 0);
+    if (huffman) return go(compress_sparse_kernel<true, false, true, false, true>, compress_sparse_kernel<false, false, true, false, false>, 1);
+    if (adaptive && priv) return go(compress_sparse_kernel<true, true, false, true, true>, compress_sparse_kernel<false, true, false, false, false>, 2);
+    if (adaptive) return go(compress_sparse_kernel<true, true, false, false, true>, compress_sparse_kernel<false, true, false, false, false>, 3);
+    const auto plain = compress_sparse_kernel<false, false, false, false, false>;
+    if (priv) return dense ? go(compress_sparse_kernel<true, false, false, true, true>, plain, 4) : go(compress_sparse_kernel<true, false, false, true, false>, plain, 5);
+    return dense ? go(compress_sparse_kernel<true, false, false, false, true>, plain, 6) : go(compress_sparse_kernel<true, false, false, false, false>, plain, 7);
 }
 
 extern "C" int skml_compress_dense(const SkmlCompressArgs* a, void* stream) {

@@ -303,7 +303,7 @@ __device__ bool decode_prepare(const DP& p, DecSmem& s) {
 // stretches (16 at most) as keep all warps busy, with their part of the stream staged in shared memory first:
 // the lanes refill their windows at different cells, so every load from L2 would hold up all of them.
 // (Two L2 loads and a search per cell took 80 us for 200,000 keys' tables.)
-__device__ void expand_tables(const DP& p, DecSmem& s) {
+__device__ __noinline__ void expand_tables(const DP& p, DecSmem& s) {
     if (s.nhuf == 0) return;
     unsigned char* area = reinterpret_cast<unsigned char*>(&s) + p.tab_off;
     unsigned int* la = reinterpret_cast<unsigned int*>(area);                       // left-aligned code words, ascending
@@ -553,7 +553,7 @@ __device__ void decode_accumulate(const DP& p, DecSmem& s, int i_begin, int i_en
 
 // Ordered apply of one rank's stashed (key, value) pairs: keys are unique inside a payload, so the
 // plain read-modify-write needs no atomics; four independent pairs per thread and iteration.
-__device__ void apply_stashed(const DP& p, unsigned long long begin, unsigned long long end, float& dsq) {
+__device__ __noinline__ void apply_stashed(const DP& p, unsigned long long begin, unsigned long long end, float& dsq) {
     const unsigned long long gsz = (unsigned long long)gridDim.x * blockDim.x;
     for (unsigned long long t = begin + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < end; t += 4 * gsz) {
         unsigned int k[4];
@@ -810,7 +810,7 @@ __device__ void decode_accumulate_dense(const DP& p, DecSmem& s, int r_begin, in
 }
 
 // D2: claim and update.
-__device__ void decode_update(const DP& p, DecSmem& s, float& dsq) {
+__device__ __noinline__ void decode_update(const DP& p, DecSmem& s, float& dsq) {
     const long long gsz = (long long)gridDim.x * blockDim.x, gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s.any_dense) {
         for (long long i = gid; i < p.dim; i += gsz) {
@@ -884,7 +884,7 @@ __device__ void finish_launch(const DP& p, float dsq) {
 }
 
 template <bool FUSED>
-__global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_kernel(DP p, int stage) {
+__global__ void __launch_bounds__(DEC_THREADS, DEC_BLOCKS_PER_SM) decode_update_kernel(const __grid_constant__ DP p, int stage) {
     skml_after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DecSmem& s = *reinterpret_cast<DecSmem*>(smem_raw);
