@@ -3280,10 +3280,22 @@ __device__ void dense_stages(const CP& p, Smem& s, unsigned int* set, unsigned i
     }
 }
 
+// As a function of its own, for the launches that rarely need it.
+__device__ __noinline__ void dense_stages_apart(const CP& p, Smem& s, unsigned int* set, unsigned int epoch, const float* __restrict__ vals) {
+    dense_stages<true>(p, s, set, epoch, vals, -1);
+}
+
 // STAGE < 0: all stages in one cooperative launch; otherwise only that stage.
 // ADAPTIVE / HUFFMAN: the key encoder and the table coder are compile-time choices, so that the default
 // path (delta_binary keys, plain tables) carries none of the other coders' registers. PRIV: launches that may have enough
-// keys for the insert in shared memory (its code costs the others 2 us).
+// keys for the insert in shared memory (its code costs the others 2 us). DENSE: launches that may be of the dense kind.
+// A launch runs most of its code once, so what it does not need should not lie between what it does: fetching instructions
+// is a good part of a short stage, and most of it where the step's other kernels have put them out of L2. Without the dense
+// kind's stages, and with the sketch form of S1 and S2 and the stores to peers out of line: 430,000 keys in a step 49.3 -> 43.2 us,
+// 2.27M 100.3 -> 93.3, 26,000 29.1 -> 28.5; a dense launch of 1M coordinates 27.9 -> 22.8. (The stages of the insert in shared
+// memory, the sample, the quantizer or the layout out of line too: 2.27M keys 100 to 102, 10M 323 -> 343 to 346. The dense
+// stages as a function of their own: 27.9 -> 34, but the insert in shared memory compiles the better for it, 2.27M keys 93.3 -> 92.1
+// and 10M 323 -> 313, so launches of PRIV have them so.)
 template <bool FUSED, bool ADAPTIVE, bool HUFFMAN, bool PRIV, bool DENSE>
 __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(const __grid_constant__ CP p, int stage) {
     skml_after_previous();
@@ -3298,7 +3310,10 @@ __global__ void __launch_bounds__(SKML_BLOCK, 1) compress_sparse_kernel(const __
     const unsigned int epoch = ctrl_open<FUSED>(p.ctrl);   // names this launch's publications
     unsigned int* const set = ctrl_set(p.ctrl, epoch);
     if (kind == SKML_KIND_DENSE) {  // un-fused launches leave it to the dense kernel's stages
-        if (FUSED && DENSE && p.dense_vals) dense_stages<FUSED>(p, s, set, epoch, p.dense_vals, stage);
+        if (FUSED && p.dense_vals) {
+            if (PRIV) dense_stages_apart(p, s, set, epoch, p.dense_vals);
+            else if (DENSE) dense_stages<FUSED>(p, s, set, epoch, p.dense_vals, stage);
+        }
         return;
     }
     if (n > p.n_max) {
@@ -3736,18 +3751,18 @@ extern "C" int skml_compress_sparse(const SkmlCompressArgs* a, void* stream) {
     int grid = 0;
     int rc = fill_params(a, p, grid);
     if (rc) return rc;
-    static LaunchCache cache[8];
+    static LaunchCache cache[7];
     const bool adaptive = p.key_encoder == SKML_KEYS_DELTA_ADAPTIVE, huffman = p.huffman != 0;
     const bool fused = a->fused != 0, priv = fused && !huffman && p.priv, dense = p.dense_vals != nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     auto go = [&](auto kernel, auto staged, int which) { return launch_stages(kernel, staged, cache[which], p, grid, fused, 8, st); };
     if (adaptive && huffman) return go(compress_sparse_kernel<true, true, true, false, true>, compress_sparse_kernel<false, true, true, false, false>, 0);
     if (huffman) return go(compress_sparse_kernel<true, false, true, false, true>, compress_sparse_kernel<false, false, true, false, false>, 1);
-    if (adaptive && priv) return go(compress_sparse_kernel<true, true, false, true, true>, compress_sparse_kernel<false, true, false, false, false>, 2);
+    if (adaptive && priv) return go(compress_sparse_kernel<true, true, false, true, false>, compress_sparse_kernel<false, true, false, false, false>, 2);
     if (adaptive) return go(compress_sparse_kernel<true, true, false, false, true>, compress_sparse_kernel<false, true, false, false, false>, 3);
     const auto plain = compress_sparse_kernel<false, false, false, false, false>;
-    if (priv) return dense ? go(compress_sparse_kernel<true, false, false, true, true>, plain, 4) : go(compress_sparse_kernel<true, false, false, true, false>, plain, 5);
-    return dense ? go(compress_sparse_kernel<true, false, false, false, true>, plain, 6) : go(compress_sparse_kernel<true, false, false, false, false>, plain, 7);
+    if (priv) return go(compress_sparse_kernel<true, false, false, true, false>, plain, 4);
+    return dense ? go(compress_sparse_kernel<true, false, false, false, true>, plain, 5) : go(compress_sparse_kernel<true, false, false, false, false>, plain, 6);
 }
 
 extern "C" int skml_compress_dense(const SkmlCompressArgs* a, void* stream) {
