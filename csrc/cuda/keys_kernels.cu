@@ -10,9 +10,9 @@
 // Every kernel cuts the keys into contiguous runs of whole tiles, one run per block, so the prefix sums over runs are short
 // enough for every block to add up on its own. Encoding is one cooperative launch (two where its output would be large, see
 // skml_da_encode), and so is decoding of fixed-width flags where a tile a block is enough (1.2M keys; otherwise three launches,
-// and two more where flags are unary). What bounds both at ordinary sizes is the chain of trips to L2, two or three grid barriers among them, and the
-// host's calls around the one wait. 1M keys there and back: 68 us, 80 as seven launches (plan, pack, widths, keys, offsets
-// and fills; 43 us of kernels against 36 here), 300 with library scans.
+// and two more where flags are unary). What bounds both at ordinary sizes is the chain of trips to L2, two or three from block to block among them, and the
+// host's calls around the one wait. 1M keys there and back: 64 us, 80 as seven launches (plan, pack, widths, keys, offsets
+// and fills; 43 us of kernels against 27 here), 300 with library scans.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -32,12 +32,18 @@ constexpr int STAGE_D = KEY_TILE + 2;             // the same for its delta bits
 constexpr int LT = 256, LPT = 4, L_TILE = LT * LPT, L_BLOCKS = 592;   // unary flags, long lists: four small blocks per SM
 constexpr long long KEY_BUDGET = 2000000000ll;    // cycles a grid barrier waits at most
 
+// What a block tells the others it tells in words that say themselves that they are there, and who needs them polls the
+// words: a grid barrier (fence, count, poll, fence) and the loads behind it are four trips to L2, this is two. 1M keys encoded
+// 18.7 -> 17.3 us, decoded 15.9 -> 9.6; 10,000 keys 16.9 -> 15.4 and 9.8 -> 7.1; 1.2M 18.9 -> 18.4 and 18.1 -> 8.6.
+constexpr unsigned int ROW_HERE = 1u << 31, ROW_BAD = 1u << 30;         // beside a run's count of a width (runs are below 2^30 keys)
+constexpr unsigned long long SUM_HERE = 1ull << 63, SUM_GONE = 1ull << 50;   // beside a tile's sum (192 of them are below 2^40)
+
 struct KeyWork {
-    unsigned int bar, ticket, status;   // cleared by the host; status: SkmlStatus (SKML_BAD_INPUT: keys not strictly increasing, or negative)
-    unsigned int pad[13];
-    unsigned int total[32];             // encode: delta widths of all keys; cleared by the host
-    unsigned int hist[KEY_BLOCKS][32];  // encode: delta widths of the runs
-    unsigned long long run_a[L_BLOCKS], run_b[L_BLOCKS];       // decode: sums over the runs
+    unsigned long long told_a[KEY_BLOCKS], told_b[KEY_BLOCKS];   // decode: sums over the tiles; cleared by the host
+    unsigned int ticket, status;        // encode: cleared by the host; status: SkmlStatus (SKML_BAD_INPUT: keys not strictly increasing, or negative)
+    unsigned int pad[30];
+    unsigned int hist[KEY_BLOCKS][32];  // encode: delta widths of the runs; cleared by the host
+    unsigned long long run_a[L_BLOCKS], run_b[L_BLOCKS];       // decode of long lists: sums over the runs
     unsigned long long zeros[L_BLOCKS];
 };
 
@@ -77,15 +83,41 @@ __device__ __forceinline__ T block_scan(T v, T* part, T& total) {
     return warp_sum(lane < warp ? x : T(0)) + inc - v;
 }
 
-// Sum of sums[0, count), by every warp for itself.
-__device__ __forceinline__ unsigned long long sum_before(const unsigned long long* sums, int count) {
-    unsigned long long v = 0;
-#pragma unroll 8
-    for (int i = threadIdx.x & 31; i < count; i += 32) v += __ldcg(sums + i);
-    return warp_sum(v);
+// Polls a block's word, `v` on, until `here` is set in it; false where that takes more than `budget` cycles. (With sleeps of 10
+// to 200 ns between the polls, 1M keys were decoded in 10.8 us instead of 9.6.)
+template <class T, class Load>
+__device__ __forceinline__ bool await_word(T& v, T here, long long budget, Load load) {
+    const long long t0 = clock64();
+    while (!(v & here)) {
+        if (clock64() - t0 > budget) return false;
+        v = load();
+    }
+    return true;
 }
 
-// The same by the whole block: for the many runs of small blocks the trips of one warp would follow one another.
+// Sum of what the first `count` blocks tell, a thread per block; SUM_GONE or more where one of them has not told it in time.
+// `part`: KEY_BLOCKS / 32 words that nobody else writes. (Not inlined: with the
+// loop twice in the kernel, decoding 1M keys took 16.7 us instead of 10.8.)
+__device__ __noinline__ unsigned long long told_before(const unsigned long long* told, int count, long long budget, unsigned long long* part) {
+    const int warp = threadIdx.x >> 5;
+    if (warp < KEY_BLOCKS / 32) {
+        unsigned long long v = 0;
+        if ((int)threadIdx.x < count) {
+            const unsigned long long* const word = told + threadIdx.x;
+            v = ld_relaxed_gpu64(word);
+            v = await_word(v, SUM_HERE, budget, [=] { return ld_relaxed_gpu64(word); }) ? v & ~SUM_HERE : SUM_GONE;
+        }
+        v = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) part[warp] = v;
+    }
+    __syncthreads();
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int w = 0; w < KEY_BLOCKS / 32; ++w) sum += part[w];
+    return sum;
+}
+
+// Sum of sums[0, count) of a launch before, by the whole block.
 template <int THREADS>
 __device__ __forceinline__ unsigned long long block_sum_before(const unsigned long long* sums, int count, unsigned long long* part) {
     unsigned long long v = 0, total;
@@ -252,10 +284,10 @@ __device__ __forceinline__ void write_tails(const int* __restrict__ keys, long l
     }
 }
 
-// Encoding in one cooperative launch: histogram of every run's delta widths and of all, a grid barrier, the mode and
-// the run's first bits from the histograms (every block adds up those of the runs before its own), then the streams.
-// Runs of one tile keep their deltas in registers across the barrier. 20 us at 1M keys, 17 at 10,000: latency.
-// Mode and lengths are reported once every block is past the barrier, where nothing can fail any more: what the host does
+// Encoding in one cooperative launch: every run's histogram of delta widths, told to all blocks, the mode and the run's
+// first bits from the histograms (every block adds up all, and those of the runs before its own), then the streams.
+// Runs of one tile keep their deltas in registers meanwhile. 17.3 us at 1M keys, 15.4 at 10,000: latency.
+// Mode and lengths are reported once every block has all histograms, where nothing can fail any more: what the host does
 // with them, it does beside the streams.
 // `words`: where the streams go, the flags and, from the next whole 64-bit word on, the deltas; `room` 64-bit words of it.
 // Null: mode and lengths only. `planned`: a launch of that kind has left the histograms of these keys in the workspace.
@@ -265,7 +297,7 @@ da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, K
     extern __shared__ __align__(16) unsigned int s_stage[];
     unsigned int* const s_f = s_stage;
     unsigned int* const s_d = s_stage + STAGE_F;
-    __shared__ unsigned int s_h[KT / 32][32];
+    __shared__ unsigned int s_h[KT / 32][32], s_all[KT / 32][32], s_before[KT / 32][32];
     __shared__ unsigned long long s_part[KT / 32], s_at[4];
     __shared__ double s_prob[32];
     __shared__ unsigned int s_mode[2];
@@ -289,19 +321,42 @@ da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, K
         }
         s_h[warp][lane] = count;
         if (bad) skml_set_status(&wk->status, SKML_BAD_INPUT, 0x70u);
-        __syncthreads();
+        const unsigned int any = __syncthreads_or(bad) ? ROW_BAD : 0u;
         if (warp == 0) {
             unsigned int t = 0;
             for (int w = 0; w < KT / 32; ++w) t += s_h[w][lane];
-            wk->hist[blockIdx.x][lane] = t;
-            if (t) red_add_gpu(&wk->total[lane], t);
+            st_relaxed_gpu(&wk->hist[blockIdx.x][lane], ROW_HERE | any | t);
         }
-        unsigned int passed = 0;
-        if (!skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, KEY_BUDGET, 0x71u, passed)) return;
+    }
+    {   // all runs' histograms, a width per lane, a warp's rows in flight together
+        constexpr int ROWS = KEY_BLOCKS / (KT / 32);
+        unsigned int row[ROWS], all = 0, before = 0;
+        bool stop = false;
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            const int r = warp + j * (KT / 32);
+            row[j] = r < (int)gridDim.x ? ld_relaxed_gpu(&wk->hist[r][lane]) : ROW_HERE;
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            const int r = warp + j * (KT / 32);
+            if (!await_word(row[j], ROW_HERE, KEY_BUDGET, [=] { return ld_relaxed_gpu(&wk->hist[r][lane]); })) {
+                skml_set_status(&wk->status, SKML_TIMEOUT_BARRIER, 0x71u);
+                stop = true;
+                break;
+            }
+            stop = stop || (row[j] & ROW_BAD);
+            const unsigned int t = row[j] & (ROW_BAD - 1u);
+            all += t;
+            if (r < (int)blockIdx.x) before += t;
+        }
+        s_all[warp][lane] = all;
+        s_before[warp][lane] = before;
+        if (__syncthreads_or(stop)) return;   // (the same in every block, but for waits that run out: the status says so)
     }
     unsigned int total = 0;
     if (warp == 0) {
-        total = __ldcg(&wk->total[lane]);
+        for (int w = 0; w < KT / 32; ++w) total += s_all[w][lane];
         s_prob[lane] = __ddiv_rn((double)total, (double)(n > 0 ? n : 1));
         __syncwarp();
         unsigned int num, mode;
@@ -310,16 +365,15 @@ da_encode_kernel(const int* __restrict__ keys, long long n, long long per_run, K
             s_mode[0] = num;
             s_mode[1] = mode;
         }
-    } else {   // the other warps: histogram of the runs before this one, a width per lane
+    } else if (warp == 1) {
         unsigned int t = 0;
-        for (int r = warp - 1; r < (int)blockIdx.x; r += KT / 32 - 1) t += __ldcg(&wk->hist[r][lane]);
-        s_h[warp][lane] = t;
+        for (int w = 0; w < KT / 32; ++w) t += s_before[w][lane];
+        s_before[0][lane] = t;
     }
     __syncthreads();
     const unsigned int m = s_mode[0], kind = s_mode[1], lb = (unsigned int)__clz(m) - 26u, fb = 5u - lb;   // 32 / m bits an interval
     if (warp == 0) {
-        unsigned int before = 0;
-        for (int w = 1; w < KT / 32; ++w) before += s_h[w][lane];
+        const unsigned int before = s_before[0][lane];
         const unsigned int iv = ((lane ? (unsigned int)lane : 32u) + (1u << lb) - 1u) >> lb, fw = kind ? iv + 1 : fb, dw = iv << lb;
         const unsigned long long f0 = warp_sum((unsigned long long)before * fw), d0 = warp_sum((unsigned long long)before * dw);
         const unsigned long long fa = warp_sum((unsigned long long)total * fw), da = warp_sum((unsigned long long)total * dw);
@@ -503,31 +557,32 @@ __device__ __noinline__ void before_run(Streams s, long long lo, unsigned int* p
     }
 }
 
-// Decoding in one cooperative launch, where a block has one tile: its delta bits, a grid barrier, its keys counted from the
-// key before them, a grid barrier, the sum of the tiles before it added; flags and keys stay in registers.
-// The caller is not told how the launch went, so it cannot fail: where a barrier gives up, a block works out for itself
-// what it waited for, and goes to no barrier any more (the others give up with it: the status word says so).
+// Decoding in one cooperative launch, where a block has one tile: its delta bits, told to the blocks behind it, its keys
+// counted from the key before them, their sum told, too, and the sum of the tiles before it added; flags and keys stay in registers.
+// The caller is not told how the launch went, so it cannot fail: where a wait runs out, the block works out for itself
+// what it waited for, and tells the others what they wait for all the same.
 __global__ void __launch_bounds__(KT, 1)
 da_decode_kernel(Streams s, long long n, KeyWork* __restrict__ wk, int* __restrict__ keys, long long budget) {
-    __shared__ unsigned long long s_part[KT / 32];
+    __shared__ unsigned long long s_part[KT / 32], s_told[2][KEY_BLOCKS / 32];
     __shared__ unsigned int s_part32[KT / 32];
     const long long lo = (long long)KEY_TILE * blockIdx.x, i0 = lo + (long long)KPT * threadIdx.x;
-    unsigned int passed = 0, iv[KPT], k[KPT], sum, add = 0;
+    unsigned int iv[KPT], k[KPT], sum, add = 0;
     bool together = gridDim.x > 1;   // (one block has nothing to wait for)
     unsigned long long bit = 0;
     intervals(s, i0, n, iv);
     if (together) {
         unsigned long long total;
         block_scan<KT>((unsigned long long)delta_bits(s, iv), s_part, total);
-        if (threadIdx.x == 0) wk->run_a[blockIdx.x] = total;
-        together = skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, budget, 0x72u, passed);
-        if (together) bit = sum_before(wk->run_a, blockIdx.x);
-        else before_run(s, lo, s_part32, bit, add);
+        if (threadIdx.x == 0) st_relaxed_gpu64(&wk->told_a[blockIdx.x], SUM_HERE | total);
+        bit = told_before(wk->told_a, blockIdx.x, budget, s_told[0]);
+        together = bit < SUM_GONE;
+        if (!together) before_run(s, lo, s_part32, bit, add);
     }
     const unsigned int before = block_scan<KT>(tile_keys<KT>(s, iv, bit, s_part32, k), s_part32, sum);   // keys are below 2^31: 32-bit sums are exact
+    if (gridDim.x > 1 && threadIdx.x == 0) st_relaxed_gpu64(&wk->told_b[blockIdx.x], SUM_HERE | sum);
     if (together) {
-        if (threadIdx.x == 0) wk->run_b[blockIdx.x] = sum;
-        if (skml_grid_barrier(&wk->bar, gridDim.x, &wk->status, budget, 0x73u, passed)) add = (unsigned int)sum_before(wk->run_b, blockIdx.x);
+        const unsigned long long keys_before = told_before(wk->told_b, blockIdx.x, budget, s_told[1]);
+        if (keys_before < SUM_GONE) add = (unsigned int)keys_before;
         else before_run(s, lo, s_part32, bit, add);
     }
     add += before;
@@ -546,7 +601,7 @@ da_decode_kernel(Streams s, long long n, KeyWork* __restrict__ wk, int* __restri
 // launches, a run of tiles per block and four small blocks per SM, which hide one another's trips to memory. With the runs of
 // tiles in one block of 1024 per SM and grid barriers, 2M keys took 38 us instead of 28, 20M 206 instead of 143 and 100M 1870
 // instead of 1430; 100,000 keys with unary flags 35 instead of 32. (Fixed-width flags, one launch instead of three: 100,000
-// keys 14.7 instead of 17.3, 1M 18.8 instead of 19.3.)
+// keys 11.7 instead of 17.3, 1M 13.1 instead of 19.3, fill and gaps with them.)
 // Delta bits of every run.
 __global__ void __launch_bounds__(LT) da_width_kernel(Streams s, long long n, long long per_run, KeyWork* __restrict__ wk) {
     __shared__ unsigned long long s_part[LT / 32];
@@ -635,9 +690,10 @@ extern "C" int skml_da_encode(const int* keys, long long n, void* workspace, uns
     if (blocks < 1) return (int)cudaErrorLaunchOutOfResources;
     cudaStream_t s = (cudaStream_t)stream;
     KeyWork* wk = reinterpret_cast<KeyWork*>(workspace);
-    cudaError_t e = planned ? cudaSuccess : cudaMemsetAsync(wk, 0, offsetof(KeyWork, hist), s);
-    if (e != cudaSuccess) return (int)e;
+    cudaError_t e = cudaSuccess;
     const Runs r = runs_for(n, KEY_TILE, blocks);
+    if (!planned) e = cudaMemsetAsync(&wk->ticket, 0, offsetof(KeyWork, hist) - offsetof(KeyWork, ticket) + r.runs * sizeof(wk->hist[0]), s);
+    if (e != cudaSuccess) return (int)e;
     unsigned long long seq = ((*done >> 32) + 1) & 0xFFFFFFFFull;
     long long per_run = r.per_run;
     unsigned int* out = reinterpret_cast<unsigned int*>(words);
@@ -690,7 +746,7 @@ extern "C" int skml_da_decode(const unsigned long long* flag_words, long long n_
         return (int)cudaGetLastError();
     }
     if (r.runs > 1) {
-        const cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, total), s);
+        const cudaError_t e = cudaMemsetAsync(wk, 0, offsetof(KeyWork, ticket), s);
         if (e != cudaSuccess) return (int)e;
     }
     long long budget = budget_cycles > 0 ? budget_cycles : KEY_BUDGET;

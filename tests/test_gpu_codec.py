@@ -806,6 +806,20 @@ def test_key_decode_whose_blocks_stop_waiting_gives_the_keys(n):
         assert torch.equal(out, keys)
 
 
+@pytest.mark.parametrize("n", [8192, 8193, 100_000, 148 * 8192, 148 * 8192 + 1])
+def test_a_fault_in_any_run_of_keys_is_every_blocks(n):
+    """The fault travels with the run's counts: no block goes on, wherever it lies (borders of runs too), and the call
+    after it, in the same memory, is not touched by it."""
+    from sketchml_b200.ops import keys as K
+    keys = torch.arange(0, 3 * n, 3, dtype=torch.int32, device="cuda")
+    for at in sorted({1, 8191, min(8192, n - 1), n // 2, n - 1}):
+        bad = keys.clone()
+        bad[at] = bad[at - 1]
+        with pytest.raises(ValueError):
+            K.encode(bad)
+        assert torch.equal(K.decode(K.encode(keys)), keys)
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_key_codec_on_every_device_of_a_process():
     """The encoder's shared memory is above what a kernel gets unasked, and the limit is set for one device only."""
