@@ -17,8 +17,10 @@
 //   S6  header and group table; sketch tables narrowed to 8/16-bit bucket codes; the finished
 //       payload is stored into every peer's receive slot with 16-byte peer stores, then the
 //       arrival flags are released (system scope). There is no separate all-gather.
-// Grid-wide dependencies are bounded software barriers (cooperative launch guarantees
-// co-residency). With `fused = 0` the same stage functions run as separate launches.
+// Grid-wide dependencies are bounded software barriers, or, where a block needs only counts of the
+// others, words that carry the launch's number beside the count and are polled with the same bound
+// (a cooperative launch guarantees co-residency). With `fused = 0` the same stage functions run as
+// separate launches.
 //
 // Reference behaviour restated (paths inside the reference project, module `sketch`):
 //   quantization/QuantileQuantizer.java:27-50, sketch/quantile/HeapQuantileSketch.java:73-143,
